@@ -11,6 +11,7 @@
 // B200_COMPUTE_F32 keeps them in f32 and multiplies with FMA on the CUDA cores (no reduced-precision matrix mode).
 #include "layerprog.h"
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -246,239 +247,7 @@ __global__ void __launch_bounds__(256) lp_gemm_kernel(const T* __restrict__ X, i
 }
 
 // ------------------------------------------------------------------------------------------------ GEMM (tcgen05 / TMEM, bf16)
-// Y[t][n] = epi(alpha * sum_k X[t][k] W[n][k]) for many rows: one CTA of 128 threads per (128 weight rows, TN tokens) tile, the f32
-// accumulator in TMEM (TN columns x 128 lanes).  Per K step of 64 elements (128 bytes of bf16 = one row of a 128-byte swizzle
-// atom) the threads copy the weight rows and the activation rows with 16-byte cp.async into K-major SWIZZLE_128B tiles (chunk c of
-// row r lands at chunk c ^ (r & 7)); TC_STAGES such stages are in flight.  When a stage has landed: fence.proxy.async, barrier,
-// and one thread issues 4 x tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = TN, K = 16, bf16 operands) and commits them to the
-// stage's mbarrier; a stage is refilled when that commit has arrived.  Epilogue: warp w reads TMEM lanes 32w .. 32w + 31 (= weight
-// rows) 32 token columns at a time; a warp's stores of one token are 32 consecutive outputs.  Every mbarrier wait is bounded: a
-// wait that gives up sets *err and the CTA drains its copies, frees its TMEM columns and returns.
-// Gated epilogues: the tile's 128 weight rows are 64 units' gate rows and the same units' up rows; the two halves of the CTA exchange half
-// of their tokens' sums through the (drained) stages and each makes the units of the other half.
-constexpr int TC_M = 128, TC_K = 64, TC_STAGES = 4;
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// K-major SWIZZLE_128B shared-memory matrix descriptor: start >> 4, LBO (unused) = 1, SBO = 1024 bytes between 8-row groups,
-// version 1 at bit 46, layout SWIZZLE_128B = 2 at bit 61
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-// instruction descriptor: D = f32 (bits 4-5 = 1), A = B = bf16 (1 at bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-__device__ __forceinline__ uint32_t tc_idesc(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok = 0;
-    const long long t0 = clock64();
-    while (!ok) {
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (!ok && clock64() - t0 > 2000000000LL) return false;
-    }
-    return true;
-}
-__device__ __forceinline__ uint32_t tc_sw128(int r, int c) {
-    return (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u + (uint32_t)((c ^ (r & 7)) << 4);
-}
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {   // bytes = 16, or 0 for a zero chunk
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-
-// 32 columns of this warp's 32 TMEM lanes
-__device__ __forceinline__ void tc_ld32(uint32_t* v, uint32_t taddr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-
-template <int TN, int EPI>
-__global__ void __launch_bounds__(128) lp_gemm_tc_kernel(const bf16* __restrict__ X, int ldx, const bf16* __restrict__ W, int ldw,
-                                                         void* __restrict__ Y, int ldy, int R, int N, int K, float alpha, int* err,
-                                                         const int* __restrict__ seg, size_t w_zstride, ZStride zs, const float* __restrict__ bias,
-                                                         float2 act) {
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
-    if (!seg && gridDim.z > 1) {
-        W += blockIdx.z * w_zstride;
-        X += blockIdx.z * zs.x;
-        Y = seg_rows<bf16, EPI>(Y, blockIdx.z * zs.y);
-    }
-    if (seg) {   // grid.z = group: rows [seg[0], seg[0] + seg[1]) of X and Y, known on the device only, against the group's own weight
-                 // matrix; a CTA beyond the rows leaves before it holds anything
-        seg += 2 * blockIdx.z;
-        W += blockIdx.z * w_zstride;
-        X += (size_t)seg[0] * ldx;
-        Y = seg_rows<bf16, EPI>(Y, (size_t)seg[0] * ldy);
-        R = seg[1];
-        if ((int)blockIdx.y * TN >= R) return;
-    }
-    __shared__ __align__(8) unsigned long long s_bar[TC_STAGES];
-    __shared__ uint32_t s_tmem;
-    constexpr int kStage = (TC_M + TN) * 128;
-    uint8_t* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);   // the swizzle is on absolute address bits
-    const int tid = threadIdx.x, warp = tid >> 5;
-    constexpr bool GLU = epi_is_glu(EPI);
-    const int n0 = blockIdx.x * (GLU ? TC_M / 2 : TC_M), t0 = blockIdx.y * TN;
-    const uint32_t bar = smem_u32(&s_bar[0]);
-    constexpr int kCols = TN < 32 ? 32 : TN;
-    if (tid == 0) {
-#pragma unroll
-        for (int i = 0; i < TC_STAGES; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8u * i) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "n"(kCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem;
-    const uint32_t idesc = tc_idesc(TC_M, TN);
-    const int steps = (K + TC_K - 1) / TC_K;
-    // copies of K step `st` into its stage: 8 chunks per row, (128 + TN) rows, spread over the 128 threads
-    auto load = [&](int st) {
-        uint8_t* tA = base + (st % TC_STAGES) * kStage;
-        uint8_t* tB = tA + TC_M * 128;
-        const int k0 = st * TC_K;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int i = tid + u * 128, r = i >> 3, c = i & 7, n = n0 + (GLU ? r & (TC_M / 2 - 1) : r), k = k0 + 8 * c;
-            const bool in = n < N && k < K;
-            const size_t wrow = GLU && r >= TC_M / 2 ? (size_t)N + n : (size_t)n;
-            cp_async16(smem_u32(tA + tc_sw128(r, c)), in ? (const void*)(W + wrow * ldw + k) : (const void*)W, in ? 16u : 0u);
-        }
-#pragma unroll
-        for (int u = 0; u < TN / 16; u++) {
-            const int i = tid + u * 128, r = i >> 3, c = i & 7, t = t0 + r, k = k0 + 8 * c;
-            const bool in = t < R && k < K;
-            cp_async16(smem_u32(tB + tc_sw128(r, c)), in ? (const void*)(X + (size_t)t * ldx + k) : (const void*)X, in ? 16u : 0u);
-        }
-    };
-    for (int st = 0; st < TC_STAGES - 1; st++) {
-        if (st < steps) load(st);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    bool alive = true;
-    for (int it = 0; it < steps; it++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(TC_STAGES - 2) : "memory");   // this thread's copies of step `it` have landed
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // generic-proxy writes -> visible to the tensor core
-        __syncthreads();
-        if (tid == 0 && alive) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint8_t* tA = base + (it % TC_STAGES) * kStage;
-            const uint64_t da = tc_desc(smem_u32(tA)), db = tc_desc(smem_u32(tA + TC_M * 128));
-#pragma unroll
-            for (int kk = 0; kk < TC_K / 16; kk++) {   // 16 bf16 = 32 bytes along the swizzled row: start address + 2
-                const uint32_t accum = (it > 0 || kk > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(da + (uint64_t)(2 * kk)), "l"(db + (uint64_t)(2 * kk)), "r"(idesc), "r"(accum)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar + 8u * (it % TC_STAGES)) : "memory");
-        }
-        // refill the stage that step it - 1 read: its MMAs must be done (they run while the MMAs of step `it` wait in the queue)
-        const int nx = it + TC_STAGES - 1;
-        if (nx < steps) {
-            if (it >= 1 && alive) {
-                const int ps = (it - 1) % TC_STAGES;
-                if (!tc_wait(bar + 8u * ps, (uint32_t)(((it - 1) / TC_STAGES) & 1))) {
-                    alive = false;
-                    if (err) atomicExch(err, 1);
-                }
-            }
-            if (alive) load(nx);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (alive && steps > 0 && !tc_wait(bar + 8u * ((steps - 1) % TC_STAGES), (uint32_t)(((steps - 1) / TC_STAGES) & 1))) {
-        alive = false;
-        if (err) atomicExch(err, 2);
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int n = n0 + (GLU ? tid & (TC_M / 2 - 1) : tid);
-    const float bn = (bias && n < N) ? bias[n] : 0.0f;
-    if constexpr (GLU) {
-        float* ex = reinterpret_cast<float*>(base);        // [2 halves][16 tokens][64 units]
-        bf16* ob = reinterpret_cast<bf16*>(ex + 2 * 16 * 64);      // [2][32 tokens][64 units]: the units on their way out, 16 bytes per store
-        const bool v8 = N % 8 == 0 && ldy % 8 == 0 && ((uintptr_t)Y & 15) == 0;
-        const bool up = tid >= TC_M / 2;
-        __syncthreads();                                    // every thread's copies have landed, every MMA has read its stage
-#pragma unroll 1
-        for (int c0 = 0; c0 < TN; c0 += 32) {
-            if (t0 + c0 >= R) break;   // CTA-uniform
-            uint32_t v[32];
-#pragma unroll
-            for (int c = 0; c < 32; c++) v[c] = 0u;
-            if (alive) {
-                tc_ld32(v, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            }
-#pragma unroll
-            for (int c = 0; c < 16; c++) ex[(up ? 0 : 16 * 64) + c * 64 + (tid & 63)] = __uint_as_float(v[up ? c : 16 + c]);
-            __syncthreads();
-#pragma unroll
-            for (int c = 0; c < 16; c++) {
-                const float mine = alpha * __uint_as_float(v[up ? 16 + c : c]), other = alpha * ex[(up ? 16 * 64 : 0) + c * 64 + (tid & 63)];
-                ob[(c0 & 32) * 64 + (up ? 16 + c : c) * 64 + (tid & 63)] = __float2bfloat16_rn(glu_fast<EPI>(up ? other : mine, up ? mine : other));
-            }
-            __syncthreads();
-            const bf16* o = ob + (c0 & 32) * 64;
-            bf16* y = reinterpret_cast<bf16*>(Y) + (size_t)(t0 + c0) * ldy + n0;
-            if (alive && v8) {
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int i = tid + u * 128, t = i >> 3, c = (i & 7) * 8;
-                    if (t0 + c0 + t < R && n0 + c < N) *reinterpret_cast<uint4*>(y + (size_t)t * ldy + c) = *reinterpret_cast<const uint4*>(o + t * 64 + c);
-                }
-            } else if (alive) {
-                for (int i = tid; i < 32 * 64; i += 128)
-                    if (t0 + c0 + (i >> 6) < R && n0 + (i & 63) < N) y[(size_t)(i >> 6) * ldy + (i & 63)] = o[i];
-            }
-        }
-    } else if (alive) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < TN; c0 += 32) {
-            if (t0 + c0 >= R) break;   // CTA-uniform
-            uint32_t v[32];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-            tc_ld32(v, taddr);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (EPI == EPI_ADD && n < N) {   // all 32 sums are read before the first one is written
-                float old[32];
-#pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const int t = t0 + c0 + c;
-                    old[c] = t < R ? reinterpret_cast<const float*>(Y)[(size_t)t * ldy + n] : 0.0f;
-                }
-#pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const int t = t0 + c0 + c;
-                    if (t < R) reinterpret_cast<float*>(Y)[(size_t)t * ldy + n] = old[c] + (alpha * __uint_as_float(v[c]) + bn);
-                }
-            } else if (n < N) {
-#pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const int t = t0 + c0 + c;
-                    if (t < R) epi_store<bf16, EPI>(Y, (size_t)t * ldy + n, alpha * __uint_as_float(v[c]) + bn, act);
-                }
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols) : "memory");
-}
+#include "lp_gemm_tc.cuh"
 
 // Few rows (decoding): one warp per output column, the weight row is read once with 16-byte loads and meets up to GV_ROWS
 // activation rows; W streams from HBM at the copy rate, the activations come out of L1/L2.
@@ -1772,9 +1541,21 @@ const Tensor* find(const LpModel* m, const std::string& name) {
     return it == m->tensors.end() ? nullptr : &it->second;
 }
 
+// cluster: CTAs of a cluster along x (1: none)
 template <typename... KArgs, typename... Args>
-void launch(LpModel* m, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
-    kern<<<grid, block, smem, m->stream>>>(std::forward<Args>(args)...);
+void launch_cluster(LpModel* m, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = m->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, KArgs(std::forward<Args>(args))...);
     m->launches++;
     if (m->launch_fail.empty()) {   // the first refused launch is remembered by name, so that the step's error says which kernel it was
         const cudaError_t e = cudaPeekAtLastError();
@@ -1788,53 +1569,65 @@ void launch(LpModel* m, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sm
         }
     }
 }
+template <typename... KArgs, typename... Args>
+void launch(LpModel* m, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+    launch_cluster(m, kern, grid, block, smem, 1, std::forward<Args>(args)...);
+}
 
-// The tensor-core GEMM takes bf16 operands whose rows are 16-byte aligned (K and the row pitches multiples of 8).
-template <int TN>
-bool tc_launch(LpModel* m, const bf16* x, int ldx, const bf16* w, int ldw, int N, int K, void* Y, int ldy, int R, float alpha, int epi, const int* seg,
-               int groups, size_t wz, ZStride zs, const float* bias, float2 act) {
-    const size_t smem = (size_t)TC_STAGES * (TC_M + TN) * 128 + 1024;
-    static bool once[EPI_COUNT][64] = {};
+// One launch of a tensor-core product: the tensor maps are made for the call (about a microsecond of host time each) and travel with it.
+template <int TN, bool PERSISTENT, int EPI>
+bool tc_launch_as(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid) {
+    constexpr size_t smem = tc_smem_bytes<TN, PERSISTENT>(epi_is_glu(EPI));
+    auto kern = PERSISTENT ? lp_gemm_tc_kernel<TN, EPI> : lp_gemm_tc_split_kernel<(TN > 128 ? 128 : TN), EPI>;
+    static bool once[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    auto prep = [&](auto kern, int e) {
-        if (dev >= 0 && dev < 64 && once[e][dev]) return true;
+    if (dev < 0 || dev >= 64 || !once[dev]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
-        if (dev >= 0 && dev < 64) once[e][dev] = true;
-        return true;
-    };
-    const int per_cta = epi_is_glu(epi) ? TC_M / 2 : TC_M;
-    dim3 grid((N + per_cta - 1) / per_cta, (R + TN - 1) / TN, groups), block(128);
-#define LP_TC(E)                                                                                                                       \
-    do {                                                                                                                               \
-        if (!prep(lp_gemm_tc_kernel<TN, E>, E)) return false;                                                                          \
-        launch(m, lp_gemm_tc_kernel<TN, E>, grid, block, smem, x, ldx, w, ldw, Y, ldy, R, N, K, alpha, m->tc_err, seg, wz, zs, bias, act);  \
-    } while (0)
-    if (epi == EPI_STORE) LP_TC(EPI_STORE);
-    else if (epi == EPI_ADD) LP_TC(EPI_ADD);
-    else if (epi == EPI_GELU) LP_TC(EPI_GELU);
-    else if (epi == EPI_XIELU) LP_TC(EPI_XIELU);
-    else if (epi == EPI_RELU_GLU) LP_TC(EPI_RELU_GLU);
-    else if (epi == EPI_SILU_GLU) LP_TC(EPI_SILU_GLU);
-    else LP_TC(EPI_RELU2);
-#undef LP_TC
+        if (dev >= 0 && dev < 64) once[dev] = true;
+    }
+    launch_cluster(m, kern, grid, dim3(TC_THREADS), smem, PERSISTENT ? 1 : a.splits, xm, wm, a);
     return true;
 }
+template <int TN, bool PERSISTENT>
+bool tc_launch(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid, int epi) {
+    switch (epi) {
+        case EPI_STORE: return tc_launch_as<TN, PERSISTENT, EPI_STORE>(m, xm, wm, a, grid);
+        case EPI_ADD: return tc_launch_as<TN, PERSISTENT, EPI_ADD>(m, xm, wm, a, grid);
+        case EPI_GELU: return tc_launch_as<TN, PERSISTENT, EPI_GELU>(m, xm, wm, a, grid);
+        case EPI_XIELU: return tc_launch_as<TN, PERSISTENT, EPI_XIELU>(m, xm, wm, a, grid);
+        case EPI_RELU_GLU: return tc_launch_as<TN, PERSISTENT, EPI_RELU_GLU>(m, xm, wm, a, grid);
+        case EPI_SILU_GLU: return tc_launch_as<TN, PERSISTENT, EPI_SILU_GLU>(m, xm, wm, a, grid);
+        default: return tc_launch_as<TN, PERSISTENT, EPI_RELU2>(m, xm, wm, a, grid);
+    }
+}
+// The tensor-core GEMM takes bf16 operands whose rows are 16-byte aligned (K and the row pitches multiples of 8).
 bool tc_takes(const LpModel* m, const void* X, int ldx, const void* W, int ldw, int K, int R, size_t wz, ZStride zs) {
     if (m->f32 || !m->use_tc || R < m->tc_min_rows) return false;
     return !(K % 8 || ldx % 8 || ldw % 8 || wz % 8 || zs.x % 8 || ((uintptr_t)X & 15) || ((uintptr_t)W & 15));
 }
+// xrows: rows of X in all groups of `seg` together
 bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, void* Y, int ldy, int R, float alpha, int epi, const int* seg,
-             int groups, size_t wz, ZStride zs, const float* bias, float2 act) {
+             int xrows, int groups, size_t wz, ZStride zs, const float* bias, float2 act) {
     if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs)) return false;
-    const bf16* x = (const bf16*)X;
-    const bf16* w = (const bf16*)W;
-    if (R <= 64) return tc_launch<64>(m, x, ldx, w, ldw, N, K, Y, ldy, R, alpha, epi, seg, groups, wz, zs, bias, act);
-    if (R <= 128) return tc_launch<128>(m, x, ldx, w, ldw, N, K, Y, ldy, R, alpha, epi, seg, groups, wz, zs, bias, act);   // (wider token tiles move fewer operand bytes per FLOP: measured 2.5x on a 2048 x 8192 x 2048 product even at 128 CTAs)
-    return tc_launch<256>(m, x, ldx, w, ldw, N, K, Y, ldy, R, alpha, epi, seg, groups, wz, zs, bias, act);
+    const bool glu = epi_is_glu(epi), x_z = !seg && groups > 1 && zs.x > 0;
+    const TcPlan pl = tc_plan(R, N, K, groups, xrows, seg != nullptr, glu);
+    CUtensorMap xm, wm;
+    const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
+    if (!tc_map(&xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, pl.tn, kh) ||
+        !tc_map(&wm, W, K, N, ldw, glu ? 2 : 1, groups, wz, glu ? TC_M / 2 : TC_M, kh)) return false;
+    const TcArgs a{Y, ldy, R, N, K, alpha, m->tc_err, seg, groups, x_z ? 1 : 0, zs.y, bias, act, pl.splits, K % TC_K == 0 ? 1 : 0};
+    const int per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per, n_nt = (R + pl.tn - 1) / pl.tn;
+    if (pl.persistent) {
+        const int most = seg ? n_mt * (xrows / pl.tn + groups) : n_mt * n_nt * groups;
+        const dim3 grid(std::min(most, 148));
+        return pl.tn == 256 ? tc_launch<256, true>(m, xm, wm, a, grid, epi) : tc_launch<128, true>(m, xm, wm, a, grid, epi);
+    }
+    const dim3 grid(n_mt * pl.splits, n_nt, groups);
+    return pl.tn == 128 ? tc_launch<128, false>(m, xm, wm, a, grid, epi) : tc_launch<64, false>(m, xm, wm, a, grid, epi);
 }
 
 // Whether gemm / project_in can end with a gated epilogue for these rows (K: the products' length; few: the input is made by the projection)
@@ -1850,7 +1643,7 @@ bool glu_takes(const LpModel* m, const void* X, const void* W, int K, int R) {
 template <typename T>
 void gemm_t(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, void* Y, int ldy, int R, float alpha, int epi, const int* seg = nullptr,
             int groups = 1, size_t wz = 0, const RowsTail* tail = nullptr, ZStride zs = ZStride{0, 0}, const float* bias = nullptr,
-            float2 act = float2{0.0f, 0.0f}) {
+            float2 act = float2{0.0f, 0.0f}, int xrows = 0) {
     const T* x = (const T*)X;
     const T* w = (const T*)W;
     if (R <= 2 * GV_ROWS && !seg) {
@@ -1907,7 +1700,7 @@ void gemm_t(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, i
 #undef LP_GV
         return;
     }
-    if (tc_gemm(m, X, ldx, W, ldw, N, K, Y, ldy, R, alpha, epi, seg, groups, wz, zs, bias, act)) return;
+    if (tc_gemm(m, X, ldx, W, ldw, N, K, Y, ldy, R, alpha, epi, seg, xrows, groups, wz, zs, bias, act)) return;
     dim3 grid((N + GB - 1) / GB, (R + GB - 1) / GB, groups), block(256);
 #define LP_GM(E) launch(m, lp_gemm_kernel<T, E>, grid, block, 0, x, ldx, w, ldw, Y, ldy, R, N, K, alpha, seg, wz, zs, bias, act)
     if (epi == EPI_STORE) LP_GM(EPI_STORE);
@@ -1924,12 +1717,13 @@ void gemm(LpModel* m, const void* X, int ldx, const void* W, int N, int K, void*
     else gemm_t<bf16>(m, X, ldx, W, K, N, K, Y, ldy, R, alpha, epi, nullptr, 1, 0, tail, ZStride{0, 0}, bias, act);
 }
 // `groups` products in one launch (grid.z): group g multiplies rows [seg[2g], seg[2g] + seg[2g + 1]) of X -- the counts live on the
-// device, R is their upper bound -- with the matrix at Wm + g * zs elements, whose rows are ldw apart (contiguous matrices: ldw = K,
+// device, R is their upper bound, xrows the rows of X -- with the matrix at Wm + g * zs elements, whose rows are ldw apart (contiguous matrices: ldw = K,
 // zs = N K; column blocks of one wide matrix: ldw = its width, zs = K), into the same rows of Y.
 void gemm_grouped(LpModel* m, const void* X, int ldx, const void* Wm, int ldw, size_t zs, int groups, int N, int K, void* Y, int ldy, int R, int epi,
-                  const int* seg) {
-    if (m->f32) gemm_t<float>(m, X, ldx, Wm, ldw, N, K, Y, ldy, R, 1.0f, epi, seg, groups, zs);
-    else gemm_t<bf16>(m, X, ldx, Wm, ldw, N, K, Y, ldy, R, 1.0f, epi, seg, groups, zs);
+                  const int* seg, int xrows) {
+    const float2 none{0.0f, 0.0f};
+    if (m->f32) gemm_t<float>(m, X, ldx, Wm, ldw, N, K, Y, ldy, R, 1.0f, epi, seg, groups, zs, nullptr, ZStride{0, 0}, nullptr, none, xrows);
+    else gemm_t<bf16>(m, X, ldx, Wm, ldw, N, K, Y, ldy, R, 1.0f, epi, seg, groups, zs, nullptr, ZStride{0, 0}, nullptr, none, xrows);
 }
 // One product per head in one launch: Y[r][z yz + n] = sum_k X[r][z xz + k] Wm[z N + n][k], z < heads, all rows of the step (f32 out).
 void gemm_heads(LpModel* m, const void* X, int ldx, size_t xz, const void* Wm, int heads, int N, int K, void* Y, int ldy, size_t yz, int R) {
@@ -3617,7 +3411,7 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
                 uint8_t* act_sh = (uint8_t*)m->act_a + (size_t)pairs * e.expert_ff * es;     // the always-on expert's activations behind the others
                 if (own_act) {
                     // pre-activations in f32 (m->P: its router columns have been read), then the units with the pair's weight
-                    gemm_grouped(m, m->moe_xp, W, up_experts, W, (size_t)per * W, e.experts, per, W, m->P, per, R, EPI_STORE, m->moe_seg);
+                    gemm_grouped(m, m->moe_xp, W, up_experts, W, (size_t)per * W, e.experts, per, W, m->P, per, R, EPI_STORE, m->moe_seg, pairs);
                     const int V = e.expert_ff % 4 ? 1 : 4;
                     const unsigned nb = (unsigned)(((size_t)pairs * (e.expert_ff / V) + 255) / 256);
 #define LP_PA(T, V) launch(m, lp_moe_pair_act_kernel<T, V>, dim3(nb), dim3(256), 0, (const float*)m->P, per, (const int*)m->moe_pos, (const int*)m->moe_sel, (const float*)m->moe_selw, e.experts, e.expert_ff, (T*)m->act_a, pairs, ea)
@@ -3625,9 +3419,9 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
                     else { if (V == 4) LP_PA(bf16, 4); else LP_PA(bf16, 1); }
 #undef LP_PA
                 } else {
-                    gemm_grouped(m, m->moe_xp, W, up_experts, W, (size_t)per * W, e.experts, e.expert_ff, W, m->act_a, e.expert_ff, R, act_epi, m->moe_seg);
+                    gemm_grouped(m, m->moe_xp, W, up_experts, W, (size_t)per * W, e.experts, e.expert_ff, W, m->act_a, e.expert_ff, R, act_epi, m->moe_seg, pairs);
                 }
-                gemm_grouped(m, m->act_a, e.expert_ff, down, L.k_down, (size_t)e.expert_ff, e.experts, W, e.expert_ff, m->moe_yp, W, R, EPI_STORE, m->moe_seg);
+                gemm_grouped(m, m->act_a, e.expert_ff, down, L.k_down, (size_t)e.expert_ff, e.experts, W, e.expert_ff, m->moe_yp, W, R, EPI_STORE, m->moe_seg, pairs);
                 if (e.shared_ff > 0) {
                     const uint8_t* up_sh = up_experts + (size_t)e.experts * per * W * es;
                     if (act_gated(e.act) || shw) {         // (m->P: the pairs' pre-activations have been read)
