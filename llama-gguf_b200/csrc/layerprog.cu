@@ -1308,6 +1308,7 @@ __global__ void lp_argmax_kernel(const float* __restrict__ logits, int vocab, in
 #include "lp_ffn.cuh"
 #include "lp_streams.cuh"
 #include "lp_row_attn.cuh"
+#include "lp_tile_attn.cuh"
 #include "lp_latent_attn.cuh"
 #include "lp_state_space.cuh"
 #include "lp_gated_recurrent.cuh"
@@ -1407,6 +1408,9 @@ struct LpModel {
     std::map<std::string, Tensor> tensors;
     std::vector<LayerPlan> plan;        // per layer
     std::vector<int> runs;              // layer index of every layer run
+    std::vector<int> step_p0, step_len; // the step's runs: first position, tokens
+    uint8_t* keys16 = nullptr;          // lp_tile_attn.cuh: the keys and values of one layer in bf16, kept from call to call
+    size_t keys16_bytes = 0;
     std::vector<int> run_pass;          // pass number t when the run is the first of a pass (step vector t is added), else -1
     std::vector<size_t> run_kv_off, run_rec_off;
     size_t slot_kv_bytes = 0, slot_rec_bytes = 0;
@@ -2705,6 +2709,7 @@ void lp_destroy(LpModel* m) {
     if (m->h_logits) cudaFreeHost(m->h_logits);
     if (m->h_tc_err) cudaFreeHost(m->h_tc_err);
     cudaFree(m->tc_err);
+    cudaFree(m->keys16);
     delete m;
 }
 
@@ -2803,8 +2808,67 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     return B200_OK;
 }
 
-// Tensor-pipe attention for prompt rows: bf16 mode, runs of at least 16 rows, key size a multiple of 16 up to 128, value size a
-// multiple of 8 up to 256 (with 16-byte aligned cache rows); everything else takes the warp kernel.
+// Attention of prompt rows through tcgen05 (lp_tile_attn.cuh): bf16 mode, runs of at least 16 rows, key size a multiple of 16 and value size a
+// multiple of 8, both up to 128 (128-byte swizzled operands, 256 TMEM columns), while the bf16 copies of one layer's keys stay within 1 GB
+// (and the device has room for them); wider heads take the mma.sync kernels below, everything else the warp kernel.
+template <int DKP, int DVP>
+bool attn_tc_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len, int tiles, int out_ld, float out_scale) {
+    const int cols = tiles * KA_K;
+    const size_t k_bytes = (size_t)ag.G * cols * DKP * 2, bytes = k_bytes + (size_t)ag.G * cols * DVP * 2;
+    if (bytes > ((size_t)1 << 30)) return false;
+    if (bytes > m->keys16_bytes) {
+        cudaFree(m->keys16);
+        m->keys16 = nullptr;
+        m->keys16_bytes = 0;
+        if (cudaMalloc((void**)&m->keys16, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            m->keys16 = nullptr;
+            return false;
+        }
+        m->keys16_bytes = bytes;
+    }
+    bf16 *k16 = (bf16*)m->keys16, *vt16 = (bf16*)(m->keys16 + k_bytes);
+    const TcEncodeFn fn = tc_encode_fn();
+    CUtensorMap km, vm;
+    const cuuint64_t kd[3] = {64, (cuuint64_t)ag.G * cols, DKP / 64}, ks[2] = {DKP * 2, 128}, vd[2] = {(cuuint64_t)cols, (cuuint64_t)ag.G * DVP}, vs[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t kb[3] = {64, KA_K, DKP / 64}, vb[2] = {KA_K, DVP}, one[3] = {1, 1, 1};
+    if (!fn ||
+        fn(&km, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, k16, kd, ks, kb, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+        fn(&vm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vt16, vd, vs, vb, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    constexpr int smem = KaSmem<DKP, DVP>::BYTES;
+    static bool once[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !once[dev]) {
+        if (cudaFuncSetAttribute(lp_tile_attn_kernel<DKP, DVP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (dev >= 0 && dev < 64) once[dev] = true;
+    }
+    launch(m, lp_keys16_kernel<DKP, DVP>, dim3(tiles, ag.G), dim3(256), 0, sm, ag, n_runs, cols, k16, vt16);
+    const unsigned blocks = (unsigned)(((size_t)max_len * (ag.H / ag.G) + KA_Q - 1) / KA_Q);
+    launch(m, lp_tile_attn_kernel<DKP, DVP>, dim3(blocks * ag.G, n_runs), dim3(192), smem, km, vm, sm, ag, (const float*)m->qbuf, (const float*)m->P, ldp, cols,
+           (bf16*)m->act_a, out_ld, out_scale, m->tc_err);
+    return true;
+}
+bool attn_tc(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len, int out_ld, float out_scale) {
+    if (ag.dim % 16 || ag.vdim % 8 || ag.dim > 128 || ag.vdim > 128 || ag.H % ag.G || out_ld % 2 || n_runs != (int)m->step_len.size()) return false;
+    long tiles = 0;
+    for (int i = 0; i < n_runs; i++) {
+        int start, kept, t;
+        keys16(ag, m->step_p0[i], m->step_len[i], start, kept, t);
+        tiles += t;
+    }
+    if (tiles > (1 << 20)) return false;
+    if (ag.dim <= 64 && ag.vdim <= 64) return attn_tc_launch<64, 64>(m, sm, ag, ldp, n_runs, max_len, (int)tiles, out_ld, out_scale);
+    return attn_tc_launch<128, 128>(m, sm, ag, ldp, n_runs, max_len, (int)tiles, out_ld, out_scale);
+}
+
+// The same with mma.sync: key size a multiple of 16 up to 128, value size a multiple of 8 up to 256.
 template <int DK, int DV>
 bool attn_tile_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len) {
     const size_t smem = (size_t)(AT_K * (DK + 8) + DV * (AT_K + 8)) * 2;
@@ -2824,9 +2888,8 @@ bool attn_tile_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ld
 }
 bool attn_tile(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len) {
     if (m->f32 || !m->use_attn_tile || max_len < 16) return false;
+    if (attn_tc(m, sm, ag, ldp, n_runs, max_len, ag.out_ld, ag.out_scale)) return true;
     if (ag.dim % 16 || ag.vdim % 8 || ag.dim > 128 || ag.vdim > 256 || ag.out_ld % 2) return false;
-    if (ag.dim <= 64 && ag.vdim <= 64) return attn_tile_launch<64, 64>(m, sm, ag, ldp, n_runs, max_len);
-    if (ag.vdim <= 128) return attn_tile_launch<128, 128>(m, sm, ag, ldp, n_runs, max_len);
     return attn_tile_launch<128, 256>(m, sm, ag, ldp, n_runs, max_len);
 }
 
@@ -2849,8 +2912,9 @@ bool row_tile_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int n_r
 }
 bool row_tile(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int n_runs, int max_len) {
     if (m->f32 || !m->use_attn_tile || max_len < 16 || ag.dim % 16 || ag.vdim % 8 || ag.chunk || ag.keep_first || ag.slope_exp > 0.0f || ag.out_gate) return false;
-    if (ag.dim <= 64 && ag.vdim <= 64) return row_tile_launch<64, 64>(m, sm, ag, n_runs, max_len);
-    if (ag.dim <= 128 && ag.vdim <= 128) return row_tile_launch<128, 128>(m, sm, ag, n_runs, max_len);
+    AttnGeom tg = ag;
+    tg.vrot = nullptr;
+    if (attn_tc(m, sm, tg, 0, n_runs, max_len, ag.H * ag.vdim, 1.0f)) return true;
     if (ag.dim <= 320 && ag.vdim <= 256) return row_tile_launch<320, 256>(m, sm, ag, n_runs, max_len);
     return false;
 }
@@ -3555,6 +3619,8 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         if (want_rows[i] < 0 || want_rows[i] >= R) return lp_fail(err, B200_ERR_INVALID_ARGUMENT, "b200_step: want_rows out of range");
     LCU(cudaSetDevice(m->device));
     int rc;
+    m->step_p0.assign(pos0, pos0 + n_runs);
+    m->step_len.assign(lens, lens + n_runs);
     if ((rc = ensure_scratch(m, R, n_runs, n_want, err))) return rc;
     // slot memory: a slot at position 0 starts from a zeroed state block (out of the pool when one is waiting there)
     for (int i = 0; i < n_runs; i++) {

@@ -1,0 +1,32 @@
+"""The tcgen05 attention of prompt rows (csrc/lp_tile_attn.cuh) against the warp kernel (B200_LP_ATTN_TILE=0), which scores in f32: kept first
+tokens that fill, end inside and pass their tiles of 64, windows that leave tiles out between them and the first visible key, blocks of 128
+(token, head) pairs that end inside a token, portions that continue a cache, scores large enough that the running maximum jumps and
+the sums are rescaled.  Tolerance: bf16 queries, keys and probabilities (2^-8 each) against f32, as in the models' own tests; a wrong key or factor
+is off by the size of the result."""
+import numpy as np
+import pytest
+
+import lazilorn_synth as S
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 128, 128), (3, 1, 64, 64), (5, 1, 48, 72), (2, 2, 80, 8)])
+@pytest.mark.parametrize("window,keep,scale", [(200, 130, 1.0), (40, 64, 1.0), (100, 3, 12.0), (1000, 0, 4.0), (1, 5, 1.0)])
+def test_against_the_warp_kernel(b200, monkeypatch, heads, kv_heads, dim, vdim, window, keep, scale):
+    cfg = S.config([S.parallel_layer(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, window=window, keep_first=keep, scale=scale * dim ** -0.5, left_scale=1.0,
+                                     right_scale=0.0, ff=0)], width=64, vocab=80)
+    w = S.random_weights(cfg, 5)
+    rng = np.random.default_rng(window + keep)
+    a, b, more = ([int(t) for t in rng.integers(0, cfg["vocab"], n)] for n in (450, 131, 97))
+    outs = {}
+    for tile in ("1", "0"):
+        monkeypatch.setenv("B200_LP_ATTN_TILE", tile)
+        gpu = S.gpu_model(cfg, w, "bfloat16", max_seq_len=640)
+        try:
+            first = gpu.step([(0, a), (1, b)], list(range(len(a) + len(b))))
+            second = gpu.step([(1, more[:1]), (0, more)], list(range(1 + len(more))))
+            outs[tile] = np.concatenate([first, second])
+        finally:
+            gpu.close()
+    assert S.rel_err(outs["1"], outs["0"]) < (2e-2 if scale < 8 else 6e-2)      # (scores of tens: a bf16 score error is 2^-8 of them)
