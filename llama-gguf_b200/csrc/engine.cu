@@ -33,6 +33,7 @@
 #include "gemv.cuh"
 #include "gemm_umma.cuh"
 #include "gemm_umma2.cuh"
+#include "prompt_f16.cuh"
 #include "attn_umma.cuh"
 #include "kv_int8.cuh"
 #include "gguf_load.cuh"
@@ -215,6 +216,9 @@ struct b200_ctx {
     float* h_logits = nullptr;
     // GEMM prefill (gemm_umma.cuh + prefill.cuh): activation rows of one chunk of prompt tokens
     bool use_prefill_gemm = true;
+    int prompt_f16_min = 0;       // prompt chunks of at least so many tokens: weights to fp16 rows first, then plain products (0: by type; prompt_f16.cuh)
+    __half* pf_w16 = nullptr;     // their rows, allocated by the first such chunk and kept
+    size_t pf_w16_elems = 0;
     int prefill_gemm_min = 32;
     bool queue_bypass = false;    // (set while a queue is being flushed: its short tail runs token by token)
     bool prefill_queue = false;   // b200_prefill_token queues; the queue runs as ONE GEMM prefill at the next call that needs the state
@@ -352,6 +356,7 @@ extern "C" int b200_ctx_create(const b200_model_desc* desc, const b200_parallel_
     }
     c->prefill_gemm_min = std::max(1, env_int("B200_PREFILL_GEMM_MIN", 32));
     c->prefill_queue = env_int("B200_PREFILL_QUEUE", 0) != 0;
+    c->prompt_f16_min = std::max(0, env_int("B200_PROMPT_F16_MIN", 0));
     c->batch_gemm_min = std::max(2, env_int("B200_BATCH_GEMM_MIN", 8));
     c->batch_graph = env_int("B200_BATCH_GRAPH", 1) != 0;
     c->batch_pdl = env_int("B200_BATCH_PDL", 1) != 0;
@@ -903,6 +908,7 @@ extern "C" void b200_ctx_destroy(b200_ctx* c) {
     for (auto& bg : c->batch_graphs)
         if (bg.exec) cudaGraphExecDestroy(bg.exec);
     cudaFree(c->pf_split);
+    cudaFree(c->pf_w16);
     cudaFree(c->pf_tmaps);
     cudaFree(c->pf_tile_cnt);
     cudaFree(c->attn_q8_part);
@@ -1959,9 +1965,55 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (p.k_split && (p.n_rows + kUmmaM - 1) / kUmmaM <= 8192 && env_int("B200_GEMM2_FUSED_REDUCE", 0)) p.tile_cnt = c->pf_tile_cnt;
         return gemm_dispatch(p, c->n_sm, st, &c->launches);
     };
+    // Two-pass products (prompt_f16.cuh): the rows of `ws` one after the other -> fp16, at most pf_w16_elems at a time, then the product of those
+    // rows.  glu: ws = {gate, up}, the unit silu(gate) up -> fp16 y.
+    auto gemm16 = [&](std::initializer_list<const DevTensor*> ws, int K, const __half* x, int ldx, int T, void* y, int ldy, const float* bias, int epi) -> cudaError_t {
+        const bool glu = epi == tc16::EPI_SILU_GLU;
+        long long total = 0;
+        for (const DevTensor* w : ws) total += glu ? 0 : (long long)w->ne[1];
+        if (glu) total = (long long)(*ws.begin())->ne[1];
+        const long long most = (long long)(c->pf_w16_elems / ((size_t)K * (glu ? 2 : 1))) & ~127LL;
+        for (long long at = 0; at < total; at += most) {
+            const int rows_n = (int)std::min(most, total - at);
+            long long first = 0;
+            size_t put = 0;
+            for (const DevTensor* w : ws) {
+                const long long lo = glu ? at : std::max(at, first), hi = glu ? at + rows_n : std::min(at + rows_n, first + (long long)w->ne[1]);
+                if (lo < hi) {
+                    const int nr = (int)(hi - lo);
+                    rows_to_f16_kernel<<<dim3((K / 8 + 255) / 256, (nr + F16_ROWS - 1) / F16_ROWS), 256, 0, st>>>(w->type, (const uint8_t*)w->d + (lo - (glu ? 0 : first)) * w->row_bytes,
+                                                                                                                w->row_bytes, nr, K, c->pf_w16 + put);
+                    c->launches++;
+                    put += (size_t)nr * K;
+                }
+                if (!glu) first += (long long)w->ne[1];
+            }
+            void* yt = glu ? (void*)((__half*)y + at) : (void*)((float*)y + at);
+            const cudaError_t e = tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, st);
+            if (e != cudaSuccess) return e;
+            c->launches++;
+        }
+        return cudaSuccess;
+    };
+    // Which chunks: above 64 tokens all (two 8B layers, 80 / 333 / 2048 tokens: Q4_K_M 1160 -> 725, 1517 -> 993, 3635 -> 2635 us, Q6_K 1865 -> 822,
+    // 2420 -> 1092, 5873 -> 2730 us; two 2048-wide layers in Q8_0 699 -> 366, 931 -> 470, 1662 -> 1082 us), where the fused kernel's token tile
+    // doubles; down to 32 tokens too unless the wide matrices are Q4_K, whose fused unpacking costs less than the pass over fp16 rows (32 tokens:
+    // Q4_K_M 551 against 674 us, Q6_K 783 against 772, Q8_0 380 against 331).  256 MB of rows at a time at most; a device without room for them
+    // keeps the fused kernel.
+    const int f16_min = c->prompt_f16_min > 0 ? c->prompt_f16_min : c->layers[0].gate.type == T_Q4_K ? 65 : 32;
+    const bool f16_able = !rows && gemm_encode_fn() && std::min(cap, n) >= f16_min;
+    if (f16_able && !c->pf_w16) {
+        const size_t want = std::max(std::min<size_t>((size_t)env_int("B200_PROMPT_F16_KROWS", 128 << 10) << 10, std::max((size_t)2 * I * H, (size_t)QKV * H)), (size_t)256 * std::max(std::max(I, H), A));
+        if (cudaMalloc((void**)&c->pf_w16, want * sizeof(__half)) == cudaSuccess) c->pf_w16_elems = want;
+        else {
+            cudaGetLastError();
+            c->pf_w16 = nullptr;
+        }
+    }
     int last_T = 0;
     for (int done = 0; done < n; done += cap) {
         const int T = std::min(cap, n - done);
+        const bool f16 = f16_able && c->pf_w16 && T >= f16_min;
         const int pos0 = (int)sl.host_pos + done;
         last_T = T;
         if (!use_graph) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -1971,9 +2023,17 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             float* kc = sl.kv + (size_t)l * kv_layer;
             float* vc = kc + kv_layer / 2;
             CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.attn_norm.f32(), d.norm_eps, XNh, H));
-            CU(gemm(L.wq, H, XNh, H, T, Q, QKV, &L.bq, 0));
-            CU(gemm(L.wk, H, XNh, H, T, Q + A, QKV, &L.bk, 0));
-            CU(gemm(L.wv, H, XNh, H, T, Q + A + nkv * hd, QKV, &L.bv, 0));
+            if (f16 && !(L.bq.present() || L.bk.present() || L.bv.present())) {
+                CU(gemm16({&L.wq, &L.wk, &L.wv}, H, XNh, H, T, Q, QKV, nullptr, tc16::EPI_STORE));
+            } else if (f16) {
+                CU(gemm16({&L.wq}, H, XNh, H, T, Q, QKV, L.bq.present() ? L.bq.f32() : nullptr, tc16::EPI_STORE));
+                CU(gemm16({&L.wk}, H, XNh, H, T, Q + A, QKV, L.bk.present() ? L.bk.f32() : nullptr, tc16::EPI_STORE));
+                CU(gemm16({&L.wv}, H, XNh, H, T, Q + A + nkv * hd, QKV, L.bv.present() ? L.bv.f32() : nullptr, tc16::EPI_STORE));
+            } else {
+                CU(gemm(L.wq, H, XNh, H, T, Q, QKV, &L.bq, 0));
+                CU(gemm(L.wk, H, XNh, H, T, Q + A, QKV, &L.bk, 0));
+                CU(gemm(L.wv, H, XNh, H, T, Q + A + nkv * hd, QKV, &L.bv, 0));
+            }
             PrefillRopeParams rp{};
             rp.qkv = Q; rp.ld = QKV; rp.k_cache = kc; rp.v_cache = vc; rp.freq = c->rope_freq; rp.pos0 = pos0;
             rp.n_heads = nh; rp.n_kv = nkv; rp.hd = hd; rp.max_seq = d.max_seq_len; rp.neox = d.rope_neox; rp.rope_scale = d.rope_scale;
@@ -2022,8 +2082,15 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                     CU(launch_on(st, pdl, Gq <= 4 ? prefill_attn_kernel<64, 4> : prefill_attn_kernel<64, 8>, dim3(ablocks), dim3(128), 0, ap));
                 }
             }
-            CU(gemm(L.wo, A, ATh, A, T, X, H, nullptr, 1));                       // X += Wo attn
+            if (f16) CU(gemm16({&L.wo}, A, ATh, A, T, X, H, nullptr, tc16::EPI_ADD));
+            else CU(gemm(L.wo, A, ATh, A, T, X, H, nullptr, 1));                  // X += Wo attn
             CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.ffn_norm.f32(), d.norm_eps, XNh, H));
+            if (f16) {
+                CU(gemm16({&L.gate, &L.up}, H, XNh, H, T, Hh, I, nullptr, tc16::EPI_SILU_GLU));
+                CU(gemm16({&L.down}, I, Hh, I, T, X, H, nullptr, tc16::EPI_ADD));
+                c->launches += 4;
+                continue;
+            }
             CU(gemm(L.gate, H, XNh, H, T, G, I, nullptr, 0));
             CU(gemm(L.up, H, XNh, H, T, U, I, nullptr, 0));
             CU(launch_on(st, pdl, prefill_swiglu_kernel, dim3(std::min(148 * 8, (int)(((long long)T * I + 255) / 256))), dim3(256), 0, (const float*)G, (const float*)U, Hh, (long long)T * I));

@@ -1,7 +1,9 @@
-// lp_gemm_tc.cuh — bf16 products of many rows on the 5th-generation tensor cores.  Included by layerprog.cu inside its anonymous namespace.
+// gemm_tc.cuh — 16-bit products of many rows on the 5th-generation tensor cores.  Included by layerprog.cu (bf16) and engine.cu (fp16), each
+// inside a namespace that has defined: tc_t (the operand type), TC_BF16 (whether it is bfloat16), the epilogues EPI_STORE, EPI_ADD, ... with
+// epi_is_glu, epi_is_act, seg_rows<T, EPI>, epi_store<T, EPI> and glu_fast<EPI>, and from_f<T>.
 //
 // Y[t][n] = epi(alpha * sum_k X[t][k] W[n][k] + bias[n]).  A tile is TC_M = 128 weight rows (the M of tcgen05.mma) by TN tokens (its N); its
-// f32 sums live in TMEM.  A stage holds KH slabs of 64 elements of K (128 bytes of bf16 = one row of a SWIZZLE_128B atom): one thread asks the TMA
+// f32 sums live in TMEM.  A stage holds KH slabs of 64 elements of K (128 bytes = one row of a SWIZZLE_128B atom): one thread asks the TMA
 // unit for the stage's weight rows, a second one for its token rows, ONE copy each; an mbarrier ring of TcRing<TN>::N stages runs between
 // them and the one thread that issues the MMAs, whose tcgen05.commit hands a stage back.  Rows and columns past the end arrive as zeros
 // (a zero-filled box counts its whole size), so ragged shapes need no code in the loop.
@@ -30,9 +32,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// instruction descriptor: D = f32 (bits 4-5 = 1), A = B = bf16 (1 at bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+// instruction descriptor: D = f32 (bits 4-5 = 1), A = B = bf16 (1 at bits 7 and 10) or fp16 (0), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
 __device__ __forceinline__ uint32_t tc_idesc(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+    return (1u << 4) | (TC_BF16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 __device__ __forceinline__ bool tc_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -83,7 +85,7 @@ __device__ __forceinline__ void tc_ld32(uint32_t* v, uint32_t taddr) {
 template <int TN> struct TcRing {
     static constexpr int KH = TN == 256 ? 1 : 2, W_BYTES = KH * TC_M * 128, X_BYTES = KH * TN * 128, STAGE = W_BYTES + X_BYTES, N = 196608 / STAGE, K = KH * TC_K;
 };
-constexpr int TC_EX_BYTES = 32768;      // gated epilogue of the persistent kernel, for each half of its warps: exchanged sums [2][16][64] f32, units [2][32][64] bf16
+constexpr int TC_EX_BYTES = 32768;      // gated epilogue of the persistent kernel, for each half of its warps: exchanged sums [2][16][64] f32, units [2][32][64] of tc_t
 template <int TN, bool PERSISTENT> constexpr size_t tc_smem_bytes(bool glu) {
     return (size_t)TcRing<TN>::N * TcRing<TN>::STAGE + (PERSISTENT && glu ? TC_EX_BYTES : 0) + 1024;
 }
@@ -176,7 +178,7 @@ __device__ __forceinline__ void tc_mma_stage(uint32_t acc, uint32_t stage, uint3
 #pragma unroll
     for (int h = 0; h < Ring::KH; h++) {
 #pragma unroll
-        for (int kk = 0; kk < TC_K / 16; kk++) {   // 16 bf16 = 32 bytes along the swizzled row: start address + 2
+        for (int kk = 0; kk < TC_K / 16; kk++) {   // 16 elements = 32 bytes along the swizzled row: start address + 2
             const uint32_t accum = (!first || h > 0 || kk > 0) ? 1u : 0u;
             asm volatile(
                 "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -242,12 +244,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         for (int item = blockIdx.x; walk.find(a, n_mt, item, t); item += gridDim.x, it++) {
             const uint32_t buf = it & 1u, acc = tmem + buf * TN + ((uint32_t)((warp & 3) * 32) << 16);
             const int n0 = t.m * (GLU ? TC_M / 2 : TC_M), n = n0 + row, rows = t.rows - t.t0;        // rows: tokens of the tile that exist
-            void* Yt = seg_rows<bf16, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
+            void* Yt = seg_rows<tc_t, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
             if constexpr (GLU) {
                 tc_wait(acc_full + 8u * buf, (it >> 1) & 1u, alive, a.err, 4);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 float* ex = reinterpret_cast<float*>(base + NS * STAGE + half * (TC_EX_BYTES / 2));      // [2 halves][16 tokens][64 units]
-                bf16* ob = reinterpret_cast<bf16*>(ex + 2 * 16 * 64);            // [2][32 tokens][64 units]: the units on their way out, 16 bytes per store
+                tc_t* ob = reinterpret_cast<tc_t*>(ex + 2 * 16 * 64);            // [2][32 tokens][64 units]: the units on their way out, 16 bytes per store
                 const bool v8 = a.N % 8 == 0 && a.ldy % 8 == 0 && ((uintptr_t)Yt & 15) == 0, up = row >= TC_M / 2;
 #pragma unroll 1
                 for (int c0 = 32 * half, ph = 0; c0 < TN; c0 += 64, ph ^= 1) {
@@ -260,11 +262,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
                         const float mine = a.alpha * __uint_as_float(v[up ? 16 + c : c]), other = a.alpha * ex[(up ? 16 * 64 : 0) + c * 64 + (row & 63)];
-                        ob[ph * 2048 + (up ? 16 + c : c) * 64 + (row & 63)] = __float2bfloat16_rn(glu_fast<EPI>(up ? other : mine, up ? mine : other));
+                        ob[ph * 2048 + (up ? 16 + c : c) * 64 + (row & 63)] = from_f<tc_t>(glu_fast<EPI>(up ? other : mine, up ? mine : other));
                     }
                     asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
-                    const bf16* o = ob + ph * 2048;
-                    bf16* y = reinterpret_cast<bf16*>(Yt) + (size_t)c0 * a.ldy + n0;
+                    const tc_t* o = ob + ph * 2048;
+                    tc_t* y = reinterpret_cast<tc_t*>(Yt) + (size_t)c0 * a.ldy + n0;
                     if (v8) {
 #pragma unroll
                         for (int u = 0; u < 2; u++) {
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     } else {
 #pragma unroll
                         for (int c = 0; c < 32; c++)
-                            if (live && c0 + c < rows) epi_store<bf16, EPI>(Yt, (size_t)(c0 + c) * a.ldy + n, a.alpha * __uint_as_float(v[c]) + bn, a.act);
+                            if (live && c0 + c < rows) epi_store<tc_t, EPI>(Yt, (size_t)(c0 + c) * a.ldy + n, a.alpha * __uint_as_float(v[c]) + bn, a.act);
                     }
                 }
             }
@@ -396,7 +398,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (warp < TC_EPI_WARPS) {
         const int c_beg = rank * rows / S, c_end = (rank + 1) * rows / S, n0 = t.m * (GLU ? TC_M / 2 : TC_M);
         const uint32_t part_s = smem_u32(part);
-        void* Yt = seg_rows<bf16, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
+        void* Yt = seg_rows<tc_t, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
         auto sum = [&](int c, int row) {
             float p[8];
 #pragma unroll
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll 2
             for (int c = c_beg + (tid >> 6); c < c_end; c += TC_EPI_WARPS / 2) {
                 const float g = a.alpha * sum(c, tid & 63), u = a.alpha * sum(c, (tid & 63) + 64);
-                if (n < a.N) reinterpret_cast<bf16*>(Yt)[(size_t)c * a.ldy + n] = __float2bfloat16_rn(glu_fast<EPI>(g, u));
+                if (n < a.N) reinterpret_cast<tc_t*>(Yt)[(size_t)c * a.ldy + n] = from_f<tc_t>(glu_fast<EPI>(g, u));
             }
         } else {
             const int n = n0 + (tid & (TC_M - 1));
@@ -429,7 +431,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 for (int u = 0; u < 4; u++)
                     if (live && c + u < c_end) {
                         if (EPI == EPI_ADD) reinterpret_cast<float*>(Yt)[(size_t)(c + u) * a.ldy + n] = old[u] + v[u];
-                        else epi_store<bf16, EPI>(Yt, (size_t)(c + u) * a.ldy + n, v[u], a.act);
+                        else epi_store<tc_t, EPI>(Yt, (size_t)(c + u) * a.ldy + n, v[u], a.act);
                     }
             }
         }
@@ -454,7 +456,7 @@ TcEncodeFn tc_encode_fn() {
     }();
     return fn;
 }
-// [groups][parts][rows][K] bf16, rows `ld` elements apart, parts (gate and up of a gated matrix) rows * ld, groups z, in boxes of box rows x 64
+// [groups][parts][rows][K], rows `ld` elements apart, parts (gate and up of a gated matrix) rows * ld, groups z, in boxes of box rows x 64
 // elements x all parts; K % 64 == 0: as [groups][K / 64][parts][rows][64], `kh` slabs of 64 per box
 bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts, int groups, size_t z, int box, int kh) {
     const TcEncodeFn fn = tc_encode_fn();
@@ -463,7 +465,7 @@ bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts,
     const cuuint64_t dims[5] = {(cuuint64_t)(slabs ? TC_K : K), (cuuint64_t)rows, (cuuint64_t)parts, (cuuint64_t)(slabs ? K / TC_K : 1), (cuuint64_t)groups};
     const cuuint64_t strides[4] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * ld * 2, TC_K * 2, (groups > 1 ? (cuuint64_t)z : (cuuint64_t)ld) * 2};
     const cuuint32_t boxes[5] = {(cuuint32_t)TC_K, (cuuint32_t)box, (cuuint32_t)parts, (cuuint32_t)(slabs ? kh : 1), 1}, one[5] = {1, 1, 1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void*)p, dims, strides, boxes, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    return fn(map, TC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, (void*)p, dims, strides, boxes, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

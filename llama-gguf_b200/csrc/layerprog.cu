@@ -247,7 +247,9 @@ __global__ void __launch_bounds__(256) lp_gemm_kernel(const T* __restrict__ X, i
 }
 
 // ------------------------------------------------------------------------------------------------ GEMM (tcgen05 / TMEM, bf16)
-#include "lp_gemm_tc.cuh"
+using tc_t = bf16;
+constexpr bool TC_BF16 = true;
+#include "gemm_tc.cuh"
 
 // Few rows (decoding): one warp per output column, the weight row is read once with 16-byte loads and meets up to GV_ROWS
 // activation rows; W streams from HBM at the copy rate, the activations come out of L1/L2.

@@ -1,4 +1,4 @@
-"""The tensor-core products of the layer-program engine (csrc/lp_gemm_tc.cuh) at the edges of their tiles: row counts around the token tiles
+"""The tensor-core products of the layer-program engine (csrc/gemm_tc.cuh) at the edges of their tiles: row counts around the token tiles
 of 64, 128 and 256, widths that are no multiple of a slab of 64 or of a weight tile of 128, K steps cut over 1 to 8 CTAs, gated units, experts,
 heads.  Same operands through the CUDA-core product (B200_LP_TC=0): f32 sums in another order, so a bf16 activation may round to its
 neighbour (2^-8 of its value) and a close call of a router may turn; a wrong tile is off by the size of the result."""

@@ -1,0 +1,37 @@
+"""The two-pass products of prompts (csrc/prompt_f16.cuh: blocks -> fp16 rows, plain tcgen05 products) against the fused dequant-GEMM on the same
+prompts: every block type, rows that are no multiple of a weight tile, biases, token counts around the token tiles of 64, 128 and 256, matrices
+that need several portions of the scratch rows.
+
+Tolerance: both round the same f32 block values to fp16 and add in f32, in another order; from there an activation near a tie rounds to the other
+fp16 neighbour (2^-11), at three places per layer.  Against the oracle such roundings measure 0.9e-4 .. 5.3e-4 of the largest logit
+(tests/test_gpu_prefill.py); two independent sets of them are at most sqrt(2) times as far apart, 7.5e-4, within the 1e-3 that either path
+holds.  A wrong row, block or portion is off by the size of the logits."""
+import pytest
+
+import synth
+from synth import rel_err
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-3
+
+
+def logits(b200, monkeypatch, desc, tensors, prompt, **env):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    gpu = b200.GpuOnlyInference(desc, tensors)
+    try:
+        return gpu.prefill(prompt)
+    finally:
+        gpu.close()
+
+
+@pytest.mark.parametrize("preset,mix", [("llama-tiny", "Q4_K_M"), ("llama-tiny", "Q5_K_M"), ("llama-tiny", "Q6_K"), ("tinyllama-tiny", "Q8_0"), ("qwen-tiny", "Q8_0")])
+@pytest.mark.parametrize("n", [32, 65, 129, 300])
+def test_two_passes_against_the_fused_product(b200, monkeypatch, preset, mix, n):
+    arch, desc, tensors = synth.synth_model(preset, mix, n + 8)
+    prompt = synth.prompt_tokens(n, desc["vocab"])
+    fused = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="100000")
+    two = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="1")
+    assert rel_err(two, fused) < TOL
+    few = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="1", B200_PROMPT_F16_KROWS="1")     # portions of the least size
+    assert rel_err(few, two) < TOL
