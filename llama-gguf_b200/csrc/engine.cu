@@ -1072,7 +1072,7 @@ static cudaError_t enqueue_token(b200_ctx* c, int slot_i, Mode mode, bool only_g
             rt.x = c->xb; rt.norm_w = L.ffn_norm.f32(); rt.eps = d.norm_eps; rt.w_router = L.router.f32();
             rt.hidden = H; rt.n_experts = d.n_experts; rt.top_k = d.n_experts_used; rt.sel = c->moe_sel; rt.wt = c->moe_wt;
             rt.epoch = c->ep ? c->ep_epoch : nullptr;
-            if (!only_gemv) CK(launch_k(c, moe_route_kernel, dim3(1), dim3(256), 0, rt));
+            if (!only_gemv) CK(launch_k(c, moe_route_kernel, dim3(1), dim3(kRouteThreads), 0, rt));
             for (int s = 0; s < d.n_experts_used; s++) {
                 const int e_base = c->ep ? c->par.rank * c->ep_local : 0, e_count = c->ep ? c->ep_local : 0;
                 GemvParams p{};
