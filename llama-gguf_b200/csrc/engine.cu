@@ -1044,7 +1044,7 @@ static cudaError_t enqueue_token(b200_ctx* c, int slot_i, Mode mode, bool only_g
             ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.n_splits = c->attn_q8_splits; ap.scale = 1.0f / sqrtf((float)hd);
             const dim3 grid(ap.n_splits, nkv);
             CK(launch_k(c, hd == 128 ? attn_q8_split_kernel<128, 4> : attn_q8_split_kernel<64, 4>, grid, dim3(kAttnQ8Warps * 32), 0, ap));
-            CK(launch_k(c, attn_q8_merge_kernel, dim3(nh), dim3(hd), 0, ap, hd));
+            CK(launch_k(c, attn_q8_merge_kernel, dim3(nh), dim3(kAttnQ8MergeThreads), 0, ap, hd));
         }
         if (!only_gemv && c->kv_format == 0) {   // RoPE + KV write
             RopeKvParams rp{};

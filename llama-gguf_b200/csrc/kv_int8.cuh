@@ -303,37 +303,52 @@ __global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(con
     }
 }
 
-// out[head][:] = sum_s acc_s e^(m_s - m) / sum_s l_s e^(m_s - m), splits in order.  grid n_heads, hd threads.  The (m, l) pairs of
-// the splits are fetched by one thread each and the coefficients shared, so the loop over splits has no dependent load in it.
-constexpr int kAttnQ8MaxSplits = 128;
-__global__ void attn_q8_merge_kernel(const AttnQ8Params p, int hd) {
-    __shared__ float sc[kAttnQ8MaxSplits], sm_m[kAttnQ8MaxSplits], sm_l[kAttnQ8MaxSplits];
-    __shared__ float s_m, s_l;
+// out[head][:] = sum_s acc_s e^(m_s - m) / sum_s l_s e^(m_s - m), over the splits that hold positions.  grid n_heads.  Bound by latency: warp 0
+// makes the coefficients of up to 128 splits in registers, then 256 / hd groups of threads add every so-manyth split with 8 loads in flight
+// (groups in order at the end).  9 positions in 128 splits, 14 heads of 64: 21 -> 5 us against one thread per channel that walked all splits after two
+// serial passes of one thread over the maxima and sums.
+constexpr int kAttnQ8MaxSplits = 128, kAttnQ8MergeThreads = 256;
+__global__ void __launch_bounds__(kAttnQ8MergeThreads) attn_q8_merge_kernel(const AttnQ8Params p, int hd) {
+    __shared__ float sc[kAttnQ8MaxSplits], sums[kAttnQ8MergeThreads], s_l;
     pdl_launch_dependents();
     pdl_wait();
-    const int head = blockIdx.x, kh = head / p.G, g = head - kh * p.G, d = threadIdx.x;
+    const int head = blockIdx.x, kh = head / p.G, g = head - kh * p.G, lane = threadIdx.x & 31;
+    const int kv_len = *p.pos + 1, chunk = (kv_len + p.n_splits - 1) / p.n_splits, live = (kv_len + chunk - 1) / chunk;      // (<= n_splits)
     const float* base = p.part + (((size_t)kh * p.n_splits) * p.G + g) * (hd + 2);
     const size_t stride = (size_t)p.G * (hd + 2);
-    for (int s = d; s < p.n_splits; s += blockDim.x) { sm_m[s] = base[s * stride + hd]; sm_l[s] = base[s * stride + hd + 1]; }
-    __syncthreads();
-    if (d == 0) {
-        float m = -INFINITY;
-        for (int s = 0; s < p.n_splits; s++) m = fmaxf(m, sm_m[s]);
-        s_m = m;
+    if (threadIdx.x < 32) {
+        float m[kAttnQ8MaxSplits / 32], l[kAttnQ8MaxSplits / 32], mx = -INFINITY, tot = 0.0f;
+#pragma unroll
+        for (int u = 0; u < kAttnQ8MaxSplits / 32; u++) {
+            const int s = lane + 32 * u;
+            m[u] = s < live ? base[s * stride + hd] : -INFINITY;
+            l[u] = s < live ? base[s * stride + hd + 1] : 0.0f;
+            mx = fmaxf(mx, m[u]);
+        }
+        mx = warp_max(mx);
+#pragma unroll
+        for (int u = 0; u < kAttnQ8MaxSplits / 32; u++) {
+            const float c = m[u] == -INFINITY ? 0.0f : expf(m[u] - mx);
+            sc[lane + 32 * u] = c;
+            tot += c * l[u];
+        }
+        tot = warp_sum(tot);
+        if (lane == 0) s_l = tot;
     }
     __syncthreads();
-    for (int s = d; s < p.n_splits; s += blockDim.x) sc[s] = (sm_m[s] == -INFINITY) ? 0.0f : expf(sm_m[s] - s_m);
-    __syncthreads();
-    if (d == 0) {
-        float l = 0.0f;
-        for (int s = 0; s < p.n_splits; s++) l += sc[s] * sm_l[s];
-        s_l = l;
-    }
+    const int groups = kAttnQ8MergeThreads / hd, grp = threadIdx.x / hd, d = threadIdx.x - grp * hd;
     float a = 0.0f;
+    if (grp < groups) {
 #pragma unroll 8
-    for (int s = 0; s < p.n_splits; s++) a = fmaf(base[s * stride + d], sc[s], a);
+        for (int s = grp; s < live; s += groups) a = fmaf(base[s * stride + d], sc[s], a);
+    }
+    sums[threadIdx.x] = a;
     __syncthreads();
-    p.out[(size_t)head * hd + d] = a / s_l;
+    if (threadIdx.x < hd) {
+        float t = 0.0f;
+        for (int i = 0; i < groups; i++) t += sums[i * hd + threadIdx.x];
+        p.out[(size_t)head * hd + threadIdx.x] = t / s_l;
+    }
 }
 
 }  // namespace b200
