@@ -8,15 +8,18 @@
 // A CTA owns 128 query ROWS = (128 / G tokens) x (the G query heads of one kv head): the rows share every K / V tile.
 //   prep   prefill_kv16_kernel rounds the f32 cache rows 0 .. kv_end-1 of the layer to fp16 once per chunk:
 //          K16[kv][pos][hd] and the transpose Vt16[kv][hd][pos] (both operands of a tcgen05.mma are K-major), pad rows zeroed;
-//   pass 1 per 128-key tile: TMA (SWIZZLE_128B boxes) -> S = Q K^T (hd/16 x tcgen05.mma kind::f16, M = N = 128) into TMEM,
-//          thread r reads row r (tcgen05.ld), scales, masks keys > its query position, keeps the running max and sum;
-//   pass 2 per tile: S again, e = exp(s - max) into a swizzled P tile, O += P V (tcgen05.mma, N = hd) accumulated in TMEM; at the
-//          end O / sum -> fp16 output row.  P and V are carried as fp16 PAIRS (hi + lo, 22 significant bits) and the product as
-//          P_hi V_hi + P_lo V_hi + P_hi V_lo: an attention output is an average with heavy cancellation, so single-fp16 P and V put
-//          2^-12 of relative noise on it — measured: the logits of a 300-token prompt moved from 6e-4 to 1.1e-3 of the oracle's.
-// Two passes instead of an online rescale of O: the softmax is the reference's (global max, then exp, then normalise) and
-// nothing in TMEM is ever rewritten; the price is a second Q K^T, half of which the tensor pipe does while idle anyway.
-// fp16 operands (q, k; v and e as hi + lo pairs), f32 scores / softmax / accumulation.  Every wait is bounded and reports through p.err.
+//   tile   of 64 keys: TMA (SWIZZLE_128B boxes) -> S = Q K^T (tcgen05.mma kind::f16, M = 128, N = 64) into one of two TMEM buffers; two threads
+//          per row (32 keys each) scale, mask keys > the query position, agree on the running maximum, and write e = exp(s - max) into a
+//          swizzled P tile; O += P V (N = hd) accumulates in TMEM.  O is rescaled only when a row's maximum has grown by more than 2^8 since
+//          the last time; the division by the sum comes last.
+// Q, K, P and V are carried as fp16 PAIRS (hi + lo, 22 significant bits) and a product as hi hi + lo hi + hi lo: an attention output is an
+// average with heavy cancellation, so single-fp16 operands put 2^-12 of relative noise on it — measured: the logits of a 300-token prompt
+// moved from 6e-4 to 1.1e-3 of the oracle's.
+// Roles: 8 softmax warps, a loader thread (two stages of K and of V^T), an MMA thread that issues the next tile's scores before it waits for this
+// tile's probabilities.  What bounds it: 6 x 256 clocks of tensor pipe per tile (M = 128, N = 64, K = hd and back), under which the exponentials run;
+// the kernel before made two passes over the keys (maximum and sum, then values) with copy, product and exponentials one after the other: 12000
+// clocks per tile, 358 us per layer of 2048 tokens (32 heads over 8) against 157 us now (one tile at a time through load, maximum, exponentials and store: 5300 clocks).
+// f32 scores / softmax / accumulation.  Every wait is bounded and reports through p.err.
 #pragma once
 #include <cuda.h>
 #include "gemm_umma2.cuh"
@@ -65,252 +68,273 @@ __global__ void __launch_bounds__(256) prefill_kv16_kernel(const float* __restri
 
 constexpr int kAttnTK = 64;   // keys per tile
 
-// 256 threads: threads t and t + 128 share query row t & 127 (TMEM lane t & 127) and split every tile's 64 key columns
-// (and the head dimension in the prologue / epilogue); thread 0 issues the TMA loads and the MMAs.
+__device__ __forceinline__ void au_ld32(uint32_t (&v)[32], uint32_t taddr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void au_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};" ::"r"(v[0]), "r"(v[1]),
+        "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
+        "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ float au_ex2(float z) {      // 2^z by the special-function unit (relative error about 2^-22)
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
+    return r;
+}
+
+template <int HD> struct AttnUmmaSmem {          // Q, two stages of K and of V^T, P: each hi + lo
+    static constexpr int Q = 128 * HD * 2, K = kAttnTK * HD * 2, V = HD * kAttnTK * 2, P = 128 * kAttnTK * 2;
+    static constexpr int K_AT = 2 * Q, V_AT = K_AT + 4 * K, P_AT = V_AT + 4 * V, MX_AT = P_AT + 2 * P, BAR_AT = MX_AT + 2 * 128 * 4, BYTES = BAR_AT + 128;
+};
+constexpr int kAttnTcThreads = 320, kAttnLoader = 8, kAttnMma = 9;
+
 template <int HD>
-__global__ void __launch_bounds__(256, 1) prefill_attn_umma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
-                                                                   const AttnUmmaParams p) {
+__global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
+                                                                            const AttnUmmaParams p) {
     extern __shared__ __align__(1024) uint8_t au_smem[];
-    __shared__ __align__(8) unsigned long long s_bar[4];   // k_full, v_full, s_done, pv_done
-    __shared__ uint32_t s_tmem;
-    __shared__ float s_ml[2][128][2];
+    using SM = AttnUmmaSmem<HD>;
     constexpr int NS = HD / 64;                     // 64-element slabs along hd
-    constexpr int kQBytes = 128 * HD * 2;           // Q tile (hi or lo): NS slabs of [128 rows][128 B]
-    constexpr int kKBytes = kAttnTK * HD * 2;       // K tile (hi or lo): NS slabs of [64 keys][128 B]
-    constexpr int kVBytes = HD * kAttnTK * 2;       // Vt tile (hi or lo): [HD rows][64 keys = 128 B]
-    constexpr int kPBytes = 128 * kAttnTK * 2;      // P tile (hi or lo): [128 rows][64 keys = 128 B]
-    constexpr int kCols = 256;                      // S: columns 0..63, O: columns 128..128+HD-1
-    uint8_t* base = au_smem + ((1024u - (umma_smem_u32(au_smem) & 1023u)) & 1023u);
-    uint8_t* sQ = base;                             // hi, lo
-    uint8_t* sK = sQ + 2 * kQBytes;                 // hi, lo
-    uint8_t* sV = sK + 2 * kKBytes;                 // hi, lo
-    uint8_t* sP = sV + 2 * kVBytes;                 // hi, lo
-    const int tid = threadIdx.x, warp = tid >> 5, half = tid >> 7;
+    const uint32_t base = umma_smem_u32(au_smem);
+    if (base & 1023u) {                             // the swizzle is on absolute address bits (there is no static shared memory in front)
+        if (threadIdx.x == 0 && p.err) atomicExch(p.err, 20);
+        return;
+    }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = p.G, TQ = 128 / G;
     const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;   // heavy (late) query tiles first
     const int kh = blockIdx.y, t0 = qt * TQ;
-    const uint32_t bar = umma_smem_u32(&s_bar[0]);
-    const uint32_t bK = bar, bV = bar + 8u, bS = bar + 16u, bPV = bar + 24u;
+    const uint32_t bars = base + SM::BAR_AT, s_tmem = bars + 120u;
+    const uint32_t k_full = bars, k_empty = bars + 16u, v_full = bars + 32u, v_empty = bars + 48u, s_full = bars + 64u, s_empty = bars + 80u, q_full = bars + 96u,
+                   p_full = bars + 104u, pv_done = bars + 112u;
     if (tid == 0) {
-        for (int i = 0; i < 4; i++) u2_mbar_init(bar + 8u * i, 1);
+        for (int i = 0; i < 2; i++) {
+            u2_mbar_init(k_full + 8u * i, 1);
+            u2_mbar_init(k_empty + 8u * i, 1);
+            u2_mbar_init(v_full + 8u * i, 1);
+            u2_mbar_init(v_empty + 8u * i, 1);
+            u2_mbar_init(s_full + 8u * i, 1);
+            u2_mbar_init(s_empty + 8u * i, 8);      // one arrive per softmax warp
+        }
+        u2_mbar_init(q_full, 8);
+        u2_mbar_init(p_full, 8);
+        u2_mbar_init(pv_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(umma_smem_u32(&s_tmem)), "n"(kCols) : "memory");
+    if (warp == kAttnMma) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(256) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // ---- Q tile: row r = (token t0 + r / G, head kh * G + r % G), f32 -> fp16 hi / lo, swizzled K-major; each thread of the pair
-    //      converts half of the row's 16-byte chunks
-    const int r = tid & 127, tq = t0 + r / G, g = r % G;
-    const bool row_ok = tq < p.T;
-    {
-        const float* qrow = p.qkv + (size_t)min(tq, p.T - 1) * p.ld + (size_t)(kh * G + g) * HD;
-#pragma unroll
-        for (int cc = 0; cc < HD / 16; cc++) {
-            const int c = half * (HD / 16) + cc;    // chunk of 8 elements
-            const float4 a = *reinterpret_cast<const float4*>(qrow + 8 * c), b = *reinterpret_cast<const float4*>(qrow + 8 * c + 4);
-            const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-            uint32_t wh[4], wl[4];
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const float x0 = fminf(fmaxf(f[2 * h], -65504.0f), 65504.0f), x1 = fminf(fmaxf(f[2 * h + 1], -65504.0f), 65504.0f);
-                const __half2 hi = __floats2half2_rn(x0, x1);
-                const float2 hf = __half22float2(hi);
-                wh[h] = *reinterpret_cast<const uint32_t*>(&hi);
-                wl[h] = umma_pack_h2(x0 - hf.x, x1 - hf.y);
-            }
-            const uint32_t off = (uint32_t)(c >> 3) * (128 * 128) + umma_sw128(r, c & 7);
-            *reinterpret_cast<uint4*>(sQ + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-            *reinterpret_cast<uint4*>(sQ + kQBytes + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-        }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem, tS = tmem, tO = tmem + 128u;
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;         // TMEM lanes of this warp = query rows
-    const int pos_q = p.pos0 + min(tq, p.T - 1);                          // this row attends keys 0 .. pos_q
-    const int kv_hi = p.pos0 + min(t0 + TQ, p.T);                         // keys needed by the tile: 0 .. kv_hi - 1
-    const int nt = (kv_hi + kAttnTK - 1) / kAttnTK;
-    const uint32_t idS = umma_idesc(128, kAttnTK), idO = umma_idesc(128, HD);
-    const uint64_t dQh = umma_desc(umma_smem_u32(sQ)), dQl = umma_desc(umma_smem_u32(sQ + kQBytes));
-    const uint64_t dKh = umma_desc(umma_smem_u32(sK)), dKl = umma_desc(umma_smem_u32(sK + kKBytes));
-    const uint64_t dVh = umma_desc(umma_smem_u32(sV)), dVl = umma_desc(umma_smem_u32(sV + kVBytes));
-    const uint64_t dPh = umma_desc(umma_smem_u32(sP)), dPl = umma_desc(umma_smem_u32(sP + kPBytes));
+    uint32_t tmem;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(s_tmem));
+    const uint32_t tO = tmem + 128u;                // S: columns 0..63 and 64..127, O: 128..128+HD-1
+    const int nt = (p.pos0 + min(t0 + TQ, p.T) + kAttnTK - 1) / kAttnTK;     // key tiles that the block's queries see
     bool alive = true;
     long long waited = 0;
-    uint32_t phK = 0u, phV = 0u, phS = 0u, phPV = 0u;
 
-    auto load_k = [&](int j) {   // thread 0: hi and lo K tiles of key tile j (the previous tile's S MMAs have completed)
-        u2_expect_tx(bK, (uint32_t)(2 * kKBytes));
+    if (warp == kAttnLoader) {
+        if (lane == 0) {
+            int asked = 0;
+            for (int j = 0; j < nt; j++) {
+                const uint32_t b = j & 1, ph = ((j >> 1) & 1) ^ 1;
+                u2_wait(k_empty + 8u * b, ph, alive, p.err, 21, waited);
+                if (!alive) break;
+                u2_expect_tx(k_full + 8u * b, (uint32_t)(2 * SM::K));
 #pragma unroll
-        for (int h = 0; h < 2; h++)
+                for (int h = 0; h < 2; h++)
 #pragma unroll
-            for (int s = 0; s < NS; s++)
-                u2_tma_2d(umma_smem_u32(sK + h * kKBytes + s * (kAttnTK * 128)), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, bK);
-    };
-    auto load_v = [&](int j) {   // thread 0: hi and lo V^T tiles of key tile j (the previous tile's PV MMAs have completed)
-        u2_expect_tx(bV, (uint32_t)(2 * kVBytes));
+                    for (int s = 0; s < NS; s++)
+                        u2_tma_2d(base + SM::K_AT + (2 * b + h) * SM::K + s * (kAttnTK * 128), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, k_full + 8u * b);
+                u2_wait(v_empty + 8u * b, ph, alive, p.err, 22, waited);
+                if (!alive) break;
+                u2_expect_tx(v_full + 8u * b, (uint32_t)(2 * SM::V));
 #pragma unroll
-        for (int h = 0; h < 2; h++) u2_tma_2d(umma_smem_u32(sV + h * kVBytes), &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, bV);
-    };
-    auto mma_s = [&]() {         // thread 0: S = Q_hi K_hi^T + Q_lo K_hi^T + Q_hi K_lo^T
-#pragma unroll
-        for (int t = 0; t < 3; t++) {
-            const uint64_t da = t == 1 ? dQl : dQh, db = t == 2 ? dKl : dKh;
-#pragma unroll
-            for (int s = 0; s < NS; s++)
-#pragma unroll
-                for (int kk = 0; kk < 4; kk++)
-                    umma_f16(tS, da + (uint64_t)(s * (128 * 128 / 16) + 2 * kk), db + (uint64_t)(s * (kAttnTK * 128 / 16) + 2 * kk), idS,
-                             (t > 0 || s > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(bS);
-    };
-    // this thread's 32 columns of its row of S
-    auto ld_s32 = [&](uint32_t (&v)[32]) {
-        const uint32_t taddr = tS + lane_base + (uint32_t)(half * 32);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-              "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-              "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-              "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    };
-
-    // ---- pass 1: row maximum and sum of exp (softmax_inplace of ops.rs:1500-1527: max, exp(s - max), sum), per column half
-    float m = -INFINITY, l = 0.0f;
-    if (tid == 0) load_k(0);
-    for (int j = 0; j < nt; j++) {
-        if (tid == 0) {
-            u2_wait(bK, phK, alive, p.err, 21, waited);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            mma_s();
-        }
-        phK ^= 1u;
-        u2_wait(bS, phS, alive, p.err, 22, waited);
-        phS ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (tid == 0 && j + 1 < nt) load_k(j + 1);   // lands while the rows are reduced
-        {
-            uint32_t v[32];
-            ld_s32(v);
-            float mt = m;
-            const int key0 = j * kAttnTK + half * 32;
-#pragma unroll
-            for (int q = 0; q < 32; q++) {
-                const float s = (key0 + q <= pos_q) ? __uint_as_float(v[q]) * p.scale : -INFINITY;
-                v[q] = __float_as_uint(s);
-                mt = fmaxf(mt, s);
+                for (int h = 0; h < 2; h++) u2_tma_2d(base + SM::V_AT + (2 * b + h) * SM::V, &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, v_full + 8u * b);
+                asked = j + 1;
             }
-            if (mt != -INFINITY) {
-                float add = 0.0f;
-#pragma unroll
-                for (int q = 0; q < 32; q++) {
-                    const float s = __uint_as_float(v[q]);
-                    add += (s == -INFINITY) ? 0.0f : __expf(s - mt);
+            if (!alive)                             // gave up: what has been asked for lands first (bounded)
+                for (int j = max(0, asked - 2); j < asked; j++) {
+                    bool w = true;
+                    u2_wait(k_full + 8u * (j & 1), (j >> 1) & 1, w, nullptr, 0, waited);
+                    u2_wait(v_full + 8u * (j & 1), (j >> 1) & 1, w, nullptr, 0, waited);
                 }
-                l = (m == -INFINITY ? 0.0f : l * expf(m - mt)) + add;
-                m = mt;
+        }
+    } else if (warp == kAttnMma) {
+        if (lane == 0) {
+            const uint32_t idS = umma_idesc(128, kAttnTK), idO = umma_idesc(128, HD);
+            const uint64_t dQ = umma_desc(base), dP = umma_desc(base + SM::P_AT);
+            auto scores = [&](int j) {              // S = Q_hi K_hi^T + Q_lo K_hi^T + Q_hi K_lo^T
+                const uint32_t b = j & 1, ph = (j >> 1) & 1;
+                u2_wait(k_full + 8u * b, ph, alive, p.err, 23, waited);
+                u2_wait(s_empty + 8u * b, ph ^ 1u, alive, p.err, 24, waited);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dK = umma_desc(base + SM::K_AT + 2 * b * SM::K);
+                if (alive) {
+#pragma unroll
+                    for (int t = 0; t < 3; t++) {
+                        const uint64_t da = dQ + (t == 1 ? SM::Q / 16 : 0), db = dK + (t == 2 ? SM::K / 16 : 0);
+#pragma unroll
+                        for (int s = 0; s < NS; s++)
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++)
+                                umma_f16(tmem + b * kAttnTK, da + (uint64_t)(s * (128 * 128 / 16) + 2 * kk), db + (uint64_t)(s * (kAttnTK * 128 / 16) + 2 * kk), idS,
+                                         (t > 0 || s > 0 || kk > 0) ? 1u : 0u);
+                    }
+                }
+                umma_commit(k_empty + 8u * b);
+                umma_commit(s_full + 8u * b);
+            };
+            u2_wait(q_full, 0, alive, p.err, 25, waited);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            scores(0);
+            for (int j = 0; j < nt; j++) {
+                const uint32_t b = j & 1;
+                if (j + 1 < nt) scores(j + 1);
+                u2_wait(v_full + 8u * b, (j >> 1) & 1, alive, p.err, 26, waited);
+                u2_wait(p_full, j & 1, alive, p.err, 27, waited);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dV = umma_desc(base + SM::V_AT + 2 * b * SM::V);
+                if (alive) {                        // O += P_hi V_hi + P_lo V_hi + P_hi V_lo
+#pragma unroll
+                    for (int t = 0; t < 3; t++) {
+                        const uint64_t da = dP + (t == 1 ? SM::P / 16 : 0), db = dV + (t == 2 ? SM::V / 16 : 0);
+#pragma unroll
+                        for (int kk = 0; kk < kAttnTK / 16; kk++) umma_f16(tO, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), idO, (j > 0 || t > 0 || kk > 0) ? 1u : 0u);
+                    }
+                }
+                umma_commit(v_empty + 8u * b);
+                umma_commit(pv_done);
             }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();                       // every row of S has been read: the next tile's MMAs may overwrite it
-    }
-    // the two column halves of a row agree on max and sum
-    s_ml[half][r][0] = m;
-    s_ml[half][r][1] = l;
-    __syncthreads();
-    {
-        const float m0 = s_ml[0][r][0], l0 = s_ml[0][r][1], m1 = s_ml[1][r][0], l1 = s_ml[1][r][1];
-        m = fmaxf(m0, m1);
-        l = (m0 == -INFINITY ? 0.0f : l0 * expf(m0 - m)) + (m1 == -INFINITY ? 0.0f : l1 * expf(m1 - m));
-    }
-    // ---- pass 2: O = sum_p exp(s[p] - max) V[p], normalised at the end
-    if (tid == 0) { load_k(0); load_v(0); }
-    for (int j = 0; j < nt; j++) {
-        if (tid == 0) {
-            u2_wait(bK, phK, alive, p.err, 23, waited);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            mma_s();
-        }
-        phK ^= 1u;
-        u2_wait(bS, phS, alive, p.err, 24, waited);
-        phS ^= 1u;
-        if (j > 0) {                           // the PV MMAs of the previous tile have read P and V
-            u2_wait(bPV, phPV, alive, p.err, 25, waited);
-            phPV ^= 1u;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (tid == 0) {                        // both land while the rows are exponentiated
-            if (j + 1 < nt) load_k(j + 1);
-            if (j > 0) load_v(j);
-        }
-        {
-            uint32_t v[32];
-            ld_s32(v);
-            const int key0 = j * kAttnTK + half * 32;
+    } else {
+        // threads t and t + 128 share query row t & 127 (TMEM lane t & 127): row r = (token t0 + r / G, head kh * G + r % G); they split every tile's 64
+        // keys and the head dimension
+        const int r = tid & 127, half = tid >> 7, tq = t0 + r / G, g = r % G;
+        {   // Q row, f32 -> fp16 hi / lo, swizzled K-major; each thread of the pair converts half of the row's 16-byte chunks
+            const float* qrow = p.qkv + (size_t)min(tq, p.T - 1) * p.ld + (size_t)(kh * G + g) * HD;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {      // 8 keys -> one 16-byte chunk of the row, hi and lo
+            for (int cc = 0; cc < HD / 16; cc++) {
+                const int c = half * (HD / 16) + cc;    // chunk of 8 elements
+                const float4 a = *reinterpret_cast<const float4*>(qrow + 8 * c), b = *reinterpret_cast<const float4*>(qrow + 8 * c + 4);
+                const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
                 uint32_t wh[4], wl[4];
 #pragma unroll
                 for (int h = 0; h < 4; h++) {
-                    const int q = 8 * c + 2 * h, key = key0 + q;
-                    const float e0 = (key <= pos_q) ? __expf(__uint_as_float(v[q]) * p.scale - m) : 0.0f;
-                    const float e1 = (key + 1 <= pos_q) ? __expf(__uint_as_float(v[q + 1]) * p.scale - m) : 0.0f;
+                    const float x0 = fminf(fmaxf(f[2 * h], -65504.0f), 65504.0f), x1 = fminf(fmaxf(f[2 * h + 1], -65504.0f), 65504.0f);
+                    const __half2 hi = __floats2half2_rn(x0, x1);
+                    const float2 hf = __half22float2(hi);
+                    wh[h] = *reinterpret_cast<const uint32_t*>(&hi);
+                    wl[h] = umma_pack_h2(x0 - hf.x, x1 - hf.y);
+                }
+                const uint32_t off = (uint32_t)(c >> 3) * (128 * 128) + umma_sw128(r, c & 7);
+                *reinterpret_cast<uint4*>(au_smem + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                *reinterpret_cast<uint4*>(au_smem + SM::Q + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) u2_mbar_arrive(q_full);
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        const int pos_q = p.pos0 + min(tq, p.T - 1);         // this row attends keys 0 .. pos_q
+        const float scale2 = p.scale * 1.4426950408889634f;      // scores in powers of two
+        float* mx_s = reinterpret_cast<float*>(au_smem + SM::MX_AT);     // [2 halves][128 rows]
+        float m = -INFINITY, l = 0.0f;
+        for (int j = 0; j < nt; j++) {
+            const uint32_t b = j & 1;
+            uint32_t v[32];
+            u2_wait(s_full + 8u * b, (j >> 1) & 1, alive, p.err, 28, waited);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            au_ld32(v, tmem + b * kAttnTK + lanes + (uint32_t)(half * 32));
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) u2_mbar_arrive(s_empty + 8u * b);
+            float s[32];
+#pragma unroll
+            for (int q = 0; q < 32; q++) s[q] = __uint_as_float(v[q]) * scale2;
+            const int seen = pos_q - (j * kAttnTK + half * 32);      // keys 0 .. seen of this half
+            if (!__all_sync(0xffffffffu, seen >= 31)) {
+#pragma unroll
+                for (int q = 0; q < 32; q++) s[q] = q <= seen ? s[q] : -INFINITY;
+            }
+            float x0 = s[0], x1 = s[1];
+#pragma unroll
+            for (int q = 2; q < 32; q += 2) {
+                x0 = fmaxf(x0, s[q]);
+                x1 = fmaxf(x1, s[q + 1]);
+            }
+            mx_s[half * 128 + r] = fmaxf(x0, x1);
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const float mx = fmaxf(mx_s[r], mx_s[128 + r]);
+            if (j > 0) {                            // the products of the tile before are done: P is free, O may be rescaled
+                u2_wait(pv_done, (j - 1) & 1, alive, p.err, 29, waited);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            if (__any_sync(0xffffffffu, mx > m + 8.0f)) {          // (the same for both warps of these rows)
+                const float mn = fmaxf(m, mx), c = m == -INFINITY ? 0.0f : au_ex2(m - mn);
+                l *= c;
+                m = mn;
+                if (j > 0) {
+#pragma unroll 1
+                    for (int n = 0; n < HD / 2; n += 32) {
+                        uint32_t o[32];
+                        const uint32_t at = tO + lanes + (uint32_t)(half * (HD / 2) + n);
+                        au_ld32(o, at);
+#pragma unroll
+                        for (int q = 0; q < 32; q++) o[q] = __float_as_uint(__uint_as_float(o[q]) * c);
+                        au_st32(at, o);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) {          // 8 keys -> one 16-byte chunk of the row, hi and lo
+                uint32_t wh[4], wl[4];
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    const float e0 = au_ex2(s[8 * c + 2 * h] - m), e1 = au_ex2(s[8 * c + 2 * h + 1] - m);      // (key 0 is visible to every row: m is finite)
+                    l += e0 + e1;
                     const __half2 hi = __floats2half2_rn(e0, e1);
                     const float2 hf = __half22float2(hi);
                     wh[h] = *reinterpret_cast<const uint32_t*>(&hi);
                     wl[h] = umma_pack_h2(e0 - hf.x, e1 - hf.y);
                 }
-                const uint32_t off = umma_sw128(r, half * 4 + c);   // chunk 0..7 of the 64-key row
-                *reinterpret_cast<uint4*>(sP + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                *reinterpret_cast<uint4*>(sP + kPBytes + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                const uint32_t off = SM::P_AT + umma_sw128(r, half * 4 + c);
+                *reinterpret_cast<uint4*>(au_smem + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                *reinterpret_cast<uint4*>(au_smem + SM::P + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
             }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) u2_mbar_arrive(p_full);
+            asm volatile("bar.sync 1, 256;" ::: "memory");      // (the maxima have been read)
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            u2_wait(bV, phV, alive, p.err, 26, waited);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // O += P_hi V_hi + P_lo V_hi + P_hi V_lo
-#pragma unroll
-            for (int t = 0; t < 3; t++) {
-                const uint64_t da = t == 1 ? dPl : dPh, db = t == 2 ? dVl : dVh;
-#pragma unroll
-                for (int kk = 0; kk < kAttnTK / 16; kk++)
-                    umma_f16(tO, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), idO, (j > 0 || t > 0 || kk > 0) ? 1u : 0u);
-            }
-            umma_commit(bPV);
-        }
-        phV ^= 1u;
-    }
-    u2_wait(bPV, phPV, alive, p.err, 27, waited);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // ---- epilogue: O row / sum -> fp16; each thread of the pair stores half of the head dimension
-    {
-        const float inv = 1.0f / l;
+        mx_s[half * 128 + r] = l;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const float inv = 1.0f / (mx_s[r] + mx_s[128 + r]);
+        u2_wait(pv_done, (nt - 1) & 1, alive, p.err, 30, waited);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // O row / sum -> fp16; each thread of the pair stores half of the head dimension
         __half* orow = p.out + (size_t)min(tq, p.T - 1) * p.ldo + (size_t)(kh * G + g) * HD + half * (HD / 2);
 #pragma unroll
         for (int c0 = 0; c0 < HD / 2; c0 += 32) {
             uint32_t v[32];
-            const uint32_t taddr = tO + lane_base + (uint32_t)(half * (HD / 2) + c0);
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                  "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                  "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                  "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row_ok) {
+            au_ld32(v, tO + lanes + (uint32_t)(half * (HD / 2) + c0));
+            if (tq < p.T) {
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     uint32_t w[4];
@@ -322,13 +346,15 @@ __global__ void __launch_bounds__(256, 1) prefill_attn_umma_kernel(const __grid_
                     *reinterpret_cast<uint4*>(orow + c0 + 8 * c) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
+            __syncwarp();
         }
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
+    if (warp == kAttnMma) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
     }
 }
 
@@ -350,9 +376,6 @@ inline bool attn_umma_encode(Umma2EncodeFn encode, const __half* k16, const __ha
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-inline size_t attn_umma_smem(int hd) {   // Q, K, V^T, P tiles, each hi + lo
-    return (size_t)2 * (128 * hd * 2 + kAttnTK * hd * 2 + hd * kAttnTK * 2 + 128 * kAttnTK * 2) + 1024;
-}
 inline bool attn_umma_ok(int hd, int n_heads, int n_kv) {
     const int G = n_kv > 0 ? n_heads / n_kv : 0;
     return (hd == 64 || hd == 128) && n_kv > 0 && n_heads % n_kv == 0 && (G == 1 || G == 2 || G == 4 || G == 8);
@@ -364,13 +387,13 @@ inline cudaError_t attn_umma_launch_hd(const CUtensorMap& kmap, const CUtensorMa
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !once[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_umma_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_umma_smem(HD));
+        cudaError_t e = cudaFuncSetAttribute(prefill_attn_umma_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnUmmaSmem<HD>::BYTES);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) once[dev] = true;
     }
     const int TQ = 128 / p.G;
     dim3 grid((p.T + TQ - 1) / TQ, p.n_kv);
-    prefill_attn_umma_kernel<HD><<<grid, 256, attn_umma_smem(HD), st>>>(kmap, vmap, p);
+    prefill_attn_umma_kernel<HD><<<grid, kAttnTcThreads, AttnUmmaSmem<HD>::BYTES, st>>>(kmap, vmap, p);
     return cudaGetLastError();
 }
 
