@@ -1,5 +1,5 @@
 // gemm_tc.cuh — 16-bit products of many rows on the 5th-generation tensor cores.  Included by layerprog.cu (bf16) and engine.cu (fp16), each
-// inside a namespace that has defined: tc_t (the operand type), TC_BF16 (whether it is bfloat16), the epilogues EPI_STORE, EPI_ADD, ... with
+// inside a namespace that has defined: next_grid / wait_grid (programmatic launches; empty where there are none), tc_t (the operand type), TC_BF16 (whether it is bfloat16), the epilogues EPI_STORE, EPI_ADD, ... with
 // epi_is_glu, epi_is_act, seg_rows<T, EPI>, epi_store<T, EPI> and glu_fast<EPI>, and from_f<T>.
 //
 // Y[t][n] = epi(alpha * sum_k X[t][k] W[n][k] + bias[n]).  A tile is TC_M = 128 weight rows (the M of tcgen05.mma) by TN tokens (its N); its
@@ -192,6 +192,7 @@ __device__ __forceinline__ void tc_mma_stage(uint32_t acc, uint32_t stage, uint3
 template <int TN, int EPI>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     lp_gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const TcArgs a) {
+    next_grid();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     constexpr int NS = TcRing<TN>::N, STAGE = TcRing<TN>::STAGE, KS = TcRing<TN>::K;
     constexpr bool GLU = epi_is_glu(EPI);
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * NS, acc_full = bar + 16u * NS, acc_empty = acc_full + 16u;
     tc_setup(tid, warp, bar, NS, &s_tmem, 2, 2 * TN);
+    if (a.seg || warp != TC_LOAD_W) wait_grid();          // (weights do not depend on the kernel before)
     const uint32_t tmem = s_tmem, ring = smem_u32(base);
     const int steps = (a.K + KS - 1) / KS, n_mt = (a.N + (GLU ? TC_M / 2 : TC_M) - 1) / (GLU ? TC_M / 2 : TC_M);
     bool alive = true;
@@ -332,6 +334,8 @@ __device__ __forceinline__ float tc_peer_f32(uint32_t addr, uint32_t rank) {
 template <int TN, int EPI>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     lp_gemm_tc_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const TcArgs a) {
+    next_grid();
+    if (a.seg) wait_grid();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     constexpr int NS = TcRing<TN>::N, STAGE = TcRing<TN>::STAGE, KS = TcRing<TN>::K;
     constexpr bool GLU = epi_is_glu(EPI);
@@ -349,6 +353,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * NS, acc_full = bar + 16u * NS;
     tc_setup(tid, warp, bar, NS, &s_tmem, 1, TN);
+    if (!a.seg && warp != TC_LOAD_W) wait_grid();         // (weights do not depend on the kernel before)
     const uint32_t tmem = s_tmem, ring = smem_u32(base);
     const int all = (a.K + KS - 1) / KS, k_beg = rank * all / S, k_end = (rank + 1) * all / S;      // (S <= all)
     bool alive = true;

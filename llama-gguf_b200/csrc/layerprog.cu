@@ -27,6 +27,14 @@ namespace {
 using bf16 = __nv_bfloat16;
 
 // ------------------------------------------------------------------------------------------------ device helpers
+// First statement of every kernel (a few ask for weights before they wait).  Steps are chains of kernels of a few microseconds; `launch` starts each one programmatically, so that its blocks are
+// placed (and may ask for weights) while the kernel before runs out.  Nothing of that kernel's is read or overwritten before this wait.
+__device__ __forceinline__ void next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void prev_grid() {
+    next_grid();
+    wait_grid();
+}
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f<bf16>(bf16 v) { return __bfloat162float(v); }
@@ -68,6 +76,7 @@ struct StepMeta {
 template <typename T>
 __global__ void lp_embed_kernel(StepMeta sm, const T* __restrict__ table, const double* __restrict__ inv_freq, float* __restrict__ x,
                                 int width, float scale, int sinusoid, T* __restrict__ xc) {
+    prev_grid();
     const int r = blockIdx.x;
     const T* row = table + (size_t)sm.tok[r] * width;
     const double p = (double)sm.row_pos[r];
@@ -98,6 +107,7 @@ __global__ void lp_embed_kernel(StepMeta sm, const T* __restrict__ table, const 
 template <typename OutT>
 __global__ void lp_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ add, const float* __restrict__ w, OutT* __restrict__ out,
                                   const int* __restrict__ gather, int width, float eps, int center) {
+    prev_grid();
     const int b = blockIdx.x;
     const int r = gather ? gather[b] : b;
     float* xr = x + (size_t)r * width;
@@ -193,6 +203,7 @@ template <typename T, int EPI>
 __global__ void __launch_bounds__(256) lp_gemm_kernel(const T* __restrict__ X, int ldx, const T* __restrict__ W, int ldw, void* __restrict__ Y,
                                                       int ldy, int R, int N, int K, float alpha, const int* __restrict__ seg, size_t w_zstride, ZStride zs,
                                                       const float* __restrict__ bias, float2 act) {
+    prev_grid();
     __shared__ float As[GK][GB + 4];
     __shared__ float Bs[GK][GB + 4];
     if (!seg && gridDim.z > 1) {
@@ -316,6 +327,7 @@ template <typename T, int EPI, int NR>
 __global__ void __launch_bounds__(256) lp_gemv_kernel(const T* __restrict__ X, int ldx, const T* __restrict__ W, int ldw, void* __restrict__ Y,
                                                       int ldy, int R, int N, int K, float alpha, int vec_ok, int stage, RowsTail tail, int nh,
                                                       ZStride zs, const float* __restrict__ bias, float2 act) {
+    next_grid();
     // nh > 0: the N outputs are heads of nh columns; head z = n / nh reads X `zs.x` elements on and writes column z * zs.y + n % nh
     extern __shared__ __align__(16) uint8_t gv_smem[];
     const T* X0 = X;
@@ -325,6 +337,7 @@ __global__ void __launch_bounds__(256) lp_gemv_kernel(const T* __restrict__ X, i
         const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
         if (stage && n < N) prefetch_row(W + (size_t)n * ldw, K, lane);
     }
+    wait_grid();
     if (stage) {   // the activation rows once per block into shared memory (every warp of the block reads all of them)
         T* xs = reinterpret_cast<T*>(gv_smem);
         const int per_row = K / VN;
@@ -388,6 +401,7 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b
 template <int EPI, int NT>
 __global__ void __launch_bounds__(256) lp_gemv_mma_kernel(const bf16* __restrict__ X, int ldx, const bf16* __restrict__ W, int ldw, void* __restrict__ Y, int ldy,
                                                           int R, int N, int K, float alpha, RowsTail tail, const float* __restrict__ bias, float2 act) {
+    prev_grid();
     __shared__ float red[8][16 * 8 * NT];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
     const bf16* xr[NT];
@@ -446,12 +460,14 @@ template <typename T, int EPI, int NR>
 __global__ void __launch_bounds__(256) lp_gemv_norm_kernel(const float* __restrict__ X, const int* __restrict__ gather, const float* __restrict__ nw,
                                                            float eps, const T* __restrict__ W, void* __restrict__ Y, int ldy, int R, int N, int K,
                                                            float alpha, int center, T* __restrict__ hn_out, float2 act, InConv ic, StepMeta sm, SubNorm sn) {
+    next_grid();
     extern __shared__ __align__(16) uint8_t gn_smem[];
     T* xs = reinterpret_cast<T*>(gn_smem);            // [R][K]
     __shared__ float red[8];
     __shared__ float inv_s, mean_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (blockIdx.x * 8 + warp < N) prefetch_row(W + (size_t)(blockIdx.x * 8 + warp) * K, K, lane);
+    wait_grid();
     for (int r = 0; r < R; r++) {
         if (sn.on) {         // (no gather; block 0 keeps the new stream, in another buffer than the one the blocks read)
             sub_norm_row<T, 256>(sn, r, X + (size_t)r * K, blockIdx.x == 0 ? sn.xout + (size_t)r * K : (float*)nullptr, K, r & 1, xs + (size_t)r * K, (T*)nullptr);
@@ -571,6 +587,7 @@ __device__ __forceinline__ float attn_score(const AttnGeom& a, float s, float sl
 }
 __global__ void lp_attn_prep_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ P, int ldp, const float* __restrict__ qw,
                                     const float* __restrict__ kw, float* __restrict__ qbuf) {
+    prev_grid();
     const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int run = sm.row_run[r], pos = sm.row_pos[r];
     const float* p = P + (size_t)r * ldp;
@@ -604,6 +621,7 @@ template <typename OutT, int VCH>
 __global__ void __launch_bounds__(32 * ATT_WARPS) lp_window_attn_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ qbuf,
                                                                         const float* __restrict__ P, int ldp, const float* __restrict__ qw,
                                                                         const float* __restrict__ kw, OutT* __restrict__ out) {
+    prev_grid();
     extern __shared__ __align__(16) float smem[];
     float* qs = smem;                                  // [dim]
     float* acc_s = smem + ((a.dim + 3) & ~3);          // [ATT_WARPS][vdim]
@@ -792,6 +810,7 @@ constexpr int AT_Q = 64, AT_K = 64;
 template <int DK, int DV>
 __global__ void __launch_bounds__(128) lp_window_attn_tile_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ qbuf,
                                                                   const float* __restrict__ P, int ldp, bf16* __restrict__ out) {
+    prev_grid();
     constexpr int KS = DK + 8, VS = AT_K + 8;          // row pitches in bf16: conflict-free 32-bit fragment loads
     extern __shared__ __align__(16) uint8_t at_smem[];
     bf16* Ks = reinterpret_cast<bf16*>(at_smem);        // [AT_K][KS]
@@ -1014,6 +1033,7 @@ template <int DMAX>
 __global__ void __launch_bounds__(SCAN_BD) lp_matrix_memory_kernel(StepMeta sm, MemGeom g, const float* __restrict__ P, int ldp,
                                                                    const float* __restrict__ ib, const float* __restrict__ fb,
                                                                    float* __restrict__ O, int ldo) {
+    prev_grid();
     constexpr int CH = ScanChunk<DMAX>::N, SPLIT = DMAX / SCAN_DREG, COLS = SCAN_BD / SPLIT;
     __shared__ __align__(16) float qs[CH][DMAX];
     __shared__ __align__(16) float ks[CH][DMAX];
@@ -1122,6 +1142,7 @@ struct DeltaGeom {
 // (the convolved channels are columns in_off .. in_off + C of P; bias: one value per channel added to the sum, or null)
 __global__ void lp_conv_silu_kernel(StepMeta sm, DeltaGeom g, const float* __restrict__ P, int ldp, const float* __restrict__ cw,
                                     const float* __restrict__ bias, float* __restrict__ out, int shift_tail) {
+    prev_grid();
     const int r = blockIdx.x, run = sm.row_run[r];
     const int t = r - sm.run_start[run];
     float* tail = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off) + (size_t)g.H * g.dim * g.vdim;
@@ -1142,6 +1163,7 @@ __global__ void lp_conv_silu_kernel(StepMeta sm, DeltaGeom g, const float* __res
 }
 // After the convolution: the run's tail becomes the last taps - 1 inputs of (old tail ++ new rows).
 __global__ void lp_conv_tail_kernel(StepMeta sm, DeltaGeom g, const float* __restrict__ P, int ldp) {
+    prev_grid();
     const int run = blockIdx.x, r0 = sm.run_start[run], len = sm.run_start[run + 1] - r0;
     float* tail = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off) + (size_t)g.H * g.dim * g.vdim;
     P += g.in_off;
@@ -1159,6 +1181,7 @@ template <int DMAX>
 __global__ void __launch_bounds__(SCAN_BD) lp_gated_delta_kernel(StepMeta sm, DeltaGeom g, const float* __restrict__ QKV, const float* __restrict__ P,
                                                                  int ldp, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                                                                  float* __restrict__ O, int ldo) {
+    prev_grid();
     constexpr int CH = ScanChunk<DMAX>::N, SPLIT = DMAX / SCAN_DREG, COLS = SCAN_BD / SPLIT;
     __shared__ __align__(16) float qs[CH][DMAX];
     __shared__ __align__(16) float ks[CH][DMAX];
@@ -1261,6 +1284,7 @@ template <typename OutT>
 __global__ void lp_headnorm_gate_kernel(const float* __restrict__ O, int ldo, const float* __restrict__ P, int ldp, int g_off,
                                         const float* __restrict__ w, int w_per_head, int H, int vdim, float eps, int act,
                                         OutT* __restrict__ out, int out_ld, float out_scale, int R) {
+    prev_grid();
     const int r = blockIdx.x, lane = threadIdx.x & 31;
     const int h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (h >= H || r >= R) return;
@@ -1279,6 +1303,7 @@ __global__ void lp_headnorm_gate_kernel(const float* __restrict__ O, int ldo, co
 
 // Greedy pick per row, the LAST maximum wins (the rule of the library's other paths).
 __global__ void lp_argmax_kernel(const float* __restrict__ logits, int vocab, int* __restrict__ out) {
+    prev_grid();
     const float* row = logits + (size_t)blockIdx.x * vocab;
     float best = -INFINITY;
     int bi = 0;
@@ -1319,6 +1344,7 @@ __global__ void lp_argmax_kernel(const float* __restrict__ logits, int vocab, in
 // out [H][b][a] = in [H][a][b]: a mixer's per-head matrices turned once at load
 template <typename T>
 __global__ void lp_transpose_heads_kernel(const T* __restrict__ in, T* __restrict__ out, int H, int a, int b) {
+    prev_grid();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)H * a * b) return;
     const int h = (int)(i / ((size_t)a * b)), rem = (int)(i - (size_t)h * a * b), ia = rem / b, ib = rem - ia * b;
@@ -1327,10 +1353,12 @@ __global__ void lp_transpose_heads_kernel(const T* __restrict__ in, T* __restric
 
 // x[r] += v
 __global__ void lp_add_vec_kernel(float* __restrict__ x, const float* __restrict__ v, int width) {
+    prev_grid();
     for (int c = threadIdx.x; c < width; c += blockDim.x) x[(size_t)blockIdx.x * width + c] += v[c];
 }
 
 __global__ void lp_add_scalar_kernel(float* __restrict__ v, int n, float a) {
+    prev_grid();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] += a;
 }
@@ -1416,6 +1444,9 @@ struct LpModel {
     size_t keys16_bytes = 0;
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
     size_t chunk_scan_floats = 0;
+    // Programmatic launches for steps of more than 16 rows (B200_LP_PDL=0: none): three ragged prompts 702 -> 605 us, prompt of 2048 910 -> 863, 32 prompts
+    // and 8 steps of 32 sequences 2717 -> 2530; one row, whose kernels fill the chip with blocks that would only wait, 6275 -> 6404 (24 steps)
+    bool use_pdl = true, pdl_now = false;
     bool use_chunk_scan = true;         // B200_LP_CHUNK_SCAN=0: prompts go token by token
     std::vector<int> run_pass;          // pass number t when the run is the first of a pass (step vector t is added), else -1
     std::vector<size_t> run_kv_off, run_rec_off;
@@ -1559,12 +1590,20 @@ void launch_cluster(LpModel* m, void (*kern)(KArgs...), dim3 grid, dim3 block, s
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = m->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cluster;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (m->pdl_now) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        n++;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    cfg.numAttrs = n;
     cudaLaunchKernelEx(&cfg, kern, KArgs(std::forward<Args>(args))...);
     m->launches++;
     if (m->launch_fail.empty()) {   // the first refused launch is remembered by name, so that the step's error says which kernel it was
@@ -1961,6 +2000,8 @@ int lp_create(const b200_program_desc* prog, const b200_layer_desc* layers, int 
         if (e && *e) m->use_fuse = atoi(e) != 0;
         e = getenv("B200_LP_ATTN_TILE");
         if (e && *e) m->use_attn_tile = atoi(e) != 0;
+        e = getenv("B200_LP_PDL");
+        if (e && *e) m->use_pdl = atoi(e) != 0;
         e = getenv("B200_LP_CHUNK_SCAN");
         if (e && *e) m->use_chunk_scan = atoi(e) != 0;
         e = getenv("B200_LP_GLIN_SEG");
@@ -3022,6 +3063,7 @@ void row_combine(LpModel* m, const AttnGeom& ag, int R, int splits) {
 // Every kernel of one step, in order, on the model's stream: eagerly, or while the stream is being captured into a CUDA graph (a
 // decode step: one row per run, nothing allocated).  head: 0 = no logits, 1 = logits of the wanted rows, 2 = their greedy picks.
 void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want, int head, int taps_len, int max_len) {
+    m->pdl_now = m->use_pdl && R > 2 * GV_ROWS;
     const b200_program_desc& p = m->p;
     const int W = p.width;
     const float* loop_step = p.loop_stop > p.loop_start ? (const float*)find(m, "loop.step")->d : nullptr;
@@ -3814,7 +3856,8 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
                 cudaGetLastError();
                 m->launch_fail.clear();
                 g = LpModel::Graph();
-                m->use_graph = false;          // fall back to eager launches for good
+                if (m->use_pdl) m->use_pdl = false;        // not capturable here: without programmatic edges from now on,
+                else m->use_graph = false;                 // then eager launches for good
                 m->launches = before;
                 enqueue_step(m, sm, R, n_runs, n_want, head, 0, 1);
             } else {

@@ -36,6 +36,7 @@ struct ChunkScan {
 
 template <int MODE, int DM>
 __global__ void __launch_bounds__(CS_THREADS) lp_chunk_prep_kernel(StepMeta sm, ChunkScan g) {
+    prev_grid();
     constexpr int PI = DM + 4;
     extern __shared__ __align__(16) float cp_sm[];
     float* qs = cp_sm;                          // [32][PI]
@@ -210,6 +211,7 @@ template <int DM> constexpr size_t cp_smem_bytes() { return (size_t)(2 * CS * (D
 // blockIdx.x: 8 columns of the state (MEM: 7 and the column of ones, whose state is n)
 template <int MODE, int DM>
 __global__ void __launch_bounds__(CS_THREADS) lp_chunk_scan_kernel(StepMeta sm, ChunkScan g) {
+    prev_grid();
     using L = CsSmem<MODE, DM>;
     constexpr int PI = L::PI, VC = MODE == CS_MEM ? CS_COLS - 1 : CS_COLS;
     constexpr int TILES = MODE == CS_DELTA ? 16 : 8, SL = CS_THREADS / TILES;                // row tiles of 4 of [W; q] (or q), slices of the key channels

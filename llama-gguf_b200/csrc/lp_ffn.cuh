@@ -8,6 +8,7 @@
 template <typename OutT>
 __global__ void lp_postnorm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, OutT* __restrict__ xc, int width,
                                    float alpha, float eps) {
+    prev_grid();
     const int r = blockIdx.x;
     float* xr = x + (size_t)r * width;
     OutT* cr = xc + (size_t)r * width;
@@ -45,6 +46,7 @@ __device__ __forceinline__ float gelu_tanh_f(float z) { return 0.5f * z * (1.0f 
 // out[r][n] = gelu_tanh(P[r][n]) * P[r][ff + n]: the fused projection holds [gate | up]
 template <typename OutT>
 __global__ void lp_gated_gelu_kernel(const float* __restrict__ P, int ldp, OutT* __restrict__ out, int ff, int R) {
+    prev_grid();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * ff) return;
     const int r = (int)(i / ff), n = (int)(i - (size_t)r * ff);
@@ -55,6 +57,7 @@ __global__ void lp_gated_gelu_kernel(const float* __restrict__ P, int ldp, OutT*
 // out[r][n] = relu(P[r][n])^2 (the relu^2 layer when its up projection is part of a wider product)
 template <typename OutT>
 __global__ void lp_relu2_kernel(const float* __restrict__ P, int ldp, OutT* __restrict__ out, int ff, int R) {
+    prev_grid();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * ff) return;
     const int r = (int)(i / ff), n = (int)(i - (size_t)r * ff);
@@ -65,6 +68,7 @@ __global__ void lp_relu2_kernel(const float* __restrict__ P, int ldp, OutT* __re
 // Router: one warp per row of the f32 logits P[r][0 .. E) (route_row, lp_rows_tail.cuh)
 __global__ void lp_moe_route_kernel(const float* __restrict__ P, int ldp, int E, int top, float* __restrict__ wts, int* __restrict__ sel,
                                     float* __restrict__ selw, int R, int mode, float scale, float* __restrict__ shw, const float* __restrict__ corr) {
+    prev_grid();
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= R) return;
     route_row(P + (size_t)r * ldp, E, top, wts + (size_t)r * E, sel + (size_t)r * top, selw + (size_t)r * top, lane, mode, scale, corr);
@@ -110,6 +114,7 @@ __device__ __forceinline__ float shared_unit(float z, float zu, float w, ExpertA
 template <typename OutT>
 __global__ void lp_moe_act_kernel(const float* __restrict__ P, int ldp, int off, const float* __restrict__ wts, int ldw, const float* __restrict__ shw, int E,
                                   int eff, int sff, OutT* __restrict__ out, int R, ExpertAct a) {
+    prev_grid();
     const int total = E * eff + sff;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * total) return;
@@ -135,6 +140,7 @@ __global__ void lp_moe_act_kernel(const float* __restrict__ P, int ldp, int off,
 template <typename OutT, int V>
 __global__ void lp_moe_pair_act_kernel(const float* __restrict__ P, int ldp, const int* __restrict__ pos, const int* __restrict__ sel, const float* __restrict__ selw,
                                        int E, int eff, OutT* __restrict__ out, int n_pairs, ExpertAct a) {
+    prev_grid();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)n_pairs * (eff / V)) return;
     const int pr = (int)(i / (eff / V)), n = (int)(i - (size_t)pr * (eff / V)) * V;
@@ -149,6 +155,7 @@ __global__ void lp_moe_pair_act_kernel(const float* __restrict__ P, int ldp, con
 // and for the always-on expert over all rows: P [R][expert_rows(sff)] -> out [R][sff]
 template <typename OutT, int V>
 __global__ void lp_moe_shared_act_kernel(const float* __restrict__ P, int ldp, const float* __restrict__ shw, int sff, OutT* __restrict__ out, int R, ExpertAct a) {
+    prev_grid();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * (sff / V)) return;
     const int r = (int)(i / (sff / V)), n = (int)(i - (size_t)r * (sff / V)) * V;
@@ -170,6 +177,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) lp_moe_up_sel_kernel(const T* __restrict__ H, const T* __restrict__ up_exp, const int* __restrict__ sel,
                                                             const float* __restrict__ selw, const float* __restrict__ shw, int E, int top, int eff, int sff,
                                                             int width, int R, T* __restrict__ act, ExpertAct a) {
+    prev_grid();
     extern __shared__ __align__(16) uint8_t mu_smem[];
     T* hs = reinterpret_cast<T*>(mu_smem);
     constexpr int VN = Vec8<T>::N;
@@ -218,6 +226,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) lp_moe_down_sel_kernel(const T* __restrict__ act, const T* __restrict__ down_cat, const int* __restrict__ sel,
                                                               int E, int top, int eff, int sff, int width, int R, float* __restrict__ y, RowsTail tail, int accum,
                                                               const float* __restrict__ selw, const T* __restrict__ h, const float* hf, int identity) {
+    prev_grid();
     constexpr int VN = Vec8<T>::N, GROUPS = 8 / MD_SPLIT;
     __shared__ float part[8];
     __shared__ int sel_s[256];
@@ -282,6 +291,7 @@ __global__ void __launch_bounds__(256) lp_moe_down_sel_kernel(const T* __restric
 // One block: counts per expert, their running sum (seg[e] = {first row, rows}), then every pair takes the next free row of its
 // expert (pos[r top + k]).  Which pair of an expert gets which row does not matter: a row's result does not depend on its place.
 __global__ void __launch_bounds__(1024) lp_moe_sort_kernel(const int* __restrict__ sel, int n_pairs, int E, int* __restrict__ seg, int* __restrict__ pos) {
+    prev_grid();
     extern __shared__ int ms[];          // [E] counts, then [E] cursors
     int* cnt = ms;
     int* cur = ms + E;
@@ -305,6 +315,7 @@ __global__ void __launch_bounds__(1024) lp_moe_sort_kernel(const int* __restrict
 // Xp[pos[i]] = H[i / top]: one block per pair (pairs of an identity expert, sel[i] >= E, need no row)
 template <typename T>
 __global__ void lp_moe_gather_kernel(const T* __restrict__ H, const int* __restrict__ pos, const int* __restrict__ sel, int E, int top, int width, T* __restrict__ Xp) {
+    prev_grid();
     const int i = blockIdx.x;
     if (sel[i] >= E) return;
     const T* src = H + (size_t)(i / top) * width;
@@ -338,6 +349,7 @@ __device__ __forceinline__ FloatV<V> moe_sum(const float* __restrict__ Yp, const
 template <typename T>
 __global__ void __launch_bounds__(256) lp_sub_norm_moe_kernel(SubNorm sn, const float* x, int width, T* __restrict__ out, const float* __restrict__ Yp,
                                                               const int* __restrict__ pos, const int* __restrict__ sel, const float* __restrict__ selw, int top, int E) {
+    prev_grid();
     const int r = blockIdx.x;
     const float* xr = x + (size_t)r * width;
     float* xo = sn.xout + (size_t)r * width;
@@ -352,6 +364,7 @@ __global__ void __launch_bounds__(256) lp_sub_norm_moe_kernel(SubNorm sn, const 
 // Identity experts are left out (lp_moe_identity_kernel adds them).
 __global__ void lp_moe_combine_kernel(const float* __restrict__ Yp, const int* __restrict__ pos, const int* __restrict__ sel, const float* __restrict__ selw, int top, int E,
                                       int width, int add, float* __restrict__ y) {
+    prev_grid();
     const int r = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         float acc = add ? y[(size_t)r * width + c] : 0.0f, sum = 0.0f;
@@ -365,6 +378,7 @@ __global__ void lp_moe_combine_kernel(const float* __restrict__ Yp, const int* _
 // y[r] (+)= (sum of the row's weights for identity experts, wts[r][E .. E + n)) * what the feed-forward reads: hf in f32 or, when null, h
 template <typename T>
 __global__ void lp_moe_identity_kernel(const float* __restrict__ wts, int E, int n, const T* __restrict__ h, const float* hf, int width, int add, float* __restrict__ y) {
+    prev_grid();
     const int r = blockIdx.x;
     float w = 0.0f;
     for (int e = 0; e < n; e++) w += wts[(size_t)r * (E + n) + E + e];

@@ -22,6 +22,7 @@ struct GlinGeom {
     size_t rec_off;
 };
 __global__ void lp_glin_gates_kernel(float* __restrict__ P, int ldp, GlinGeom g, const float* __restrict__ fb, const float* __restrict__ lower, int R) {
+    prev_grid();
     const int n = g.H * g.dim;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * n) return;
@@ -34,6 +35,7 @@ __global__ void lp_glin_gates_kernel(float* __restrict__ P, int ldp, GlinGeom g,
 template <int DMAX, int MODE>
 __global__ void __launch_bounds__(SCAN_BD) lp_gated_linear_kernel(StepMeta sm, GlinGeom g, const float* __restrict__ P, int ldp, int vec4,
                                                                   float* __restrict__ O, int ldo, int nseg, float* __restrict__ carry) {
+    prev_grid();
     constexpr int CH = ScanChunk<DMAX>::N, SPLIT = DMAX / SCAN_DREG, COLS = SCAN_BD / SPLIT;
     __shared__ __align__(16) float qs[CH][DMAX];
     __shared__ __align__(16) float fs[CH][DMAX];
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(SCAN_BD) lp_gated_linear_kernel(StepMeta sm, G
 constexpr int GC_CH = 32, GC_TL = 8, GC_SEG_MAX = 16;
 __global__ void __launch_bounds__(GC_CH * GC_TL) lp_glin_carry_kernel(StepMeta sm, GlinGeom g, const float* __restrict__ P, int ldp, int nseg,
                                                                       float* __restrict__ carry) {
+    prev_grid();
     __shared__ float part[GC_TL][GC_CH];
     __shared__ float D[GC_SEG_MAX][GC_CH];
     const int lane = threadIdx.x % GC_CH, tl = threadIdx.x / GC_CH;
@@ -200,6 +203,7 @@ template <typename OutT>
 __global__ void __launch_bounds__(GU_CH * GU_SEG) lp_gated_unit_kernel(StepMeta sm, GunitGeom g, const float* __restrict__ P, int ldp,
                                                                         const float* __restrict__ zb, const float* __restrict__ xb,
                                                                         OutT* __restrict__ out, int out_ld, float out_scale) {
+    prev_grid();
     __shared__ float As[GU_SEG][GU_CH], Bs[GU_SEG][GU_CH];
     const int c = blockIdx.x * GU_CH + threadIdx.x, seg = threadIdx.y, run = blockIdx.y;
     const int r0 = sm.run_start[run], len = sm.run_start[run + 1] - r0;
@@ -275,6 +279,7 @@ __global__ void __launch_bounds__(GU_CH * GU_SEG) lp_gated_unit_kernel(StepMeta 
 __global__ void __launch_bounds__(256) lp_dual_norm_add_kernel(float* __restrict__ x, const float* __restrict__ ya, const float* __restrict__ yb, int ldy,
                                                                const float* __restrict__ wa, const float* __restrict__ wb, int width, float eps,
                                                                float weight) {
+    prev_grid();
     __shared__ float red[2][8];
     const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float* a = ya + (size_t)r * ldy;
@@ -300,6 +305,7 @@ __global__ void __launch_bounds__(256) lp_dual_norm_add_kernel(float* __restrict
 // A thread takes VEC neighbouring units (VEC = 4: 16-byte loads; ff, the row pitch and the column offset multiples of 4).
 template <typename OutT, int VEC>
 __global__ void lp_clamped_glu_kernel(const float* __restrict__ P, int ldp, OutT* __restrict__ out, int ff, int R, float limit, float slope) {
+    prev_grid();
     const int per = ff / VEC;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * per) return;

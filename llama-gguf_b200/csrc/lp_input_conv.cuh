@@ -175,6 +175,7 @@ __device__ __forceinline__ void step_route(const StepRoute& rt, const T* hs, int
 template <typename T>
 __global__ void __launch_bounds__(512) lp_norm_conv_step_kernel(StepMeta sm, InConv ic, const float* __restrict__ x, const float* __restrict__ g, int width,
                                                                 float eps, T* __restrict__ out, StepRoute rt) {
+    prev_grid();
     extern __shared__ __align__(16) uint8_t nc_smem[];
     T* hs = reinterpret_cast<T*>(nc_smem);     // [width] (with routing only)
     const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -194,6 +195,7 @@ constexpr int NC_ROWS = 8;
 template <typename T, int V, int TAPS>
 __global__ void __launch_bounds__(256) lp_norm_conv_rows_kernel(StepMeta sm, InConv ic, const float* __restrict__ x, const float* __restrict__ g, int width,
                                                                 float eps, T* __restrict__ out, int R) {
+    prev_grid();
     extern __shared__ float nc_inv[];      // [NC_ROWS + taps - 1]: row r0 - (taps - 1) + i
     const int taps = TAPS > 0 ? TAPS : ic.taps, back = taps - 1;
     const int r0 = blockIdx.x * NC_ROWS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -270,6 +272,7 @@ __global__ void __launch_bounds__(256) lp_norm_conv_rows_kernel(StepMeta sm, InC
 // where they are).  Block (convolution, run, b): the input b places before the run's last; ring_offs[i]: the ring of convolution i inside
 // a slot's state block; pend [convolutions][runs][taps - 1][width].
 __global__ void __launch_bounds__(256) lp_ring_commit_kernel(StepMeta sm, const size_t* __restrict__ ring_offs, const float* __restrict__ pend, int taps, int width) {
+    prev_grid();
     const int run = blockIdx.y, b = blockIdx.z, r = sm.run_start[run + 1] - 1 - b;
     if (r < sm.run_start[run]) return;
     const float* src = pend + (((size_t)blockIdx.x * gridDim.y + run) * (taps - 1) + b) * width;
@@ -282,6 +285,7 @@ __global__ void __launch_bounds__(256) lp_ring_commit_kernel(StepMeta sm, const 
 template <typename T>
 __global__ void __launch_bounds__(256) lp_embed_norm_kernel(float* __restrict__ x, const float* __restrict__ g, int width, float eps, int norm,
                                                             T* __restrict__ xcat) {
+    prev_grid();
     __shared__ float red[33];
     float* xr = x + (size_t)blockIdx.x * width;
     const float inv = norm ? 1.0f / sqrtf(block_sum_sq(xr, width, red) / (float)width + eps) : 1.0f;
@@ -294,12 +298,14 @@ __global__ void __launch_bounds__(256) lp_embed_norm_kernel(float* __restrict__ 
 // the stream in the compute type, `ld` columns apart; V channels per thread (4: width and ld multiples of 4)
 template <typename T, int V>
 __global__ void lp_cast_rows_kernel(const float* __restrict__ x, int width, T* __restrict__ out, int ld) {
+    prev_grid();
     const int r = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c < width) store_v<V>(out + (size_t)r * ld + c, load_v<V>(x + (size_t)r * width + c));
 }
 
 // v[0 .. n) = s[0]: a norm's single number for every coordinate
 __global__ void lp_fill_kernel(float* __restrict__ v, const float* __restrict__ s, int n) {
+    prev_grid();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] = s[0];
 }

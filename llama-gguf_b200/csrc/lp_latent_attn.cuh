@@ -70,6 +70,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) lp_latent_prep_kernel(StepMeta sm, LatentGeom g, const float* __restrict__ P, int ldp,
                                                              const float* __restrict__ qw, const float* __restrict__ kvw,
                                                              const double* __restrict__ freq, T* __restrict__ cq, T* __restrict__ qn, float* __restrict__ qbuf) {
+    prev_grid();
     extern __shared__ float lp_cs[];     // [rot_n / 2] cos, then sin
     __shared__ float red[2][8];
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(256) lp_latent_prep_kernel(StepMeta sm, Latent
 template <typename T>
 __global__ void __launch_bounds__(256) lp_latent_qprep_kernel(StepMeta sm, LatentGeom g, const float* __restrict__ Q, const double* __restrict__ freq,
                                                               T* __restrict__ qn, float* __restrict__ qbuf) {
+    prev_grid();
     extern __shared__ float lq_cs[];
     const int r = blockIdx.x;
     float* cs = lq_cs;
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(256) lp_latent_qprep_kernel(StepMeta sm, Laten
 // out[r][c] = V[r][c] * gate in the compute type: the operand of W_o.  N channels per thread (4: vdim a multiple of 4)
 template <typename T, int N>
 __global__ void lp_latent_gate_kernel(LatentGeom g, const float* __restrict__ V, const float* __restrict__ P, int ldp, T* __restrict__ out) {
+    prev_grid();
     const int n = g.H * g.vdim, r = blockIdx.x;
     for (int c = threadIdx.x * N; c < n; c += blockDim.x * N) {
         FloatV<N> v = load_v<N>(V + (size_t)r * n + c);
@@ -174,6 +177,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) lp_latent_absorb_kernel(StepMeta sm, LatentGeom g, const float* __restrict__ Q, int ldq, const float* __restrict__ P, int ldp,
                                                                const T* __restrict__ ukT, const float* __restrict__ kvw, const double* __restrict__ freq,
                                                                float* __restrict__ qbuf, int R, int nch) {
+    prev_grid();
     extern __shared__ __align__(16) float la_sm[];     // product blocks: [R][dim] plain queries; [rot_n] angles
     __shared__ float red[33];
     const int per = g.dim + g.rot_dim, D = g.kv_rank + g.rot_dim;
@@ -229,6 +233,7 @@ __global__ void __launch_bounds__(256) lp_latent_absorb_kernel(StepMeta sm, Late
 template <typename T>
 __global__ void __launch_bounds__(256) lp_latent_merge_kernel(LatentGeom g, const float* __restrict__ part_o, const float* __restrict__ part_ml, int splits,
                                                               const T* __restrict__ uv, const float* __restrict__ P, int ldp, T* __restrict__ out, int R, int nch) {
+    prev_grid();
     extern __shared__ __align__(16) float lm_sm[];
     float* lat = lm_sm;                                  // [R][kv_rank]
     float* wgt = lm_sm + (size_t)R * g.kv_rank;          // [R][splits]

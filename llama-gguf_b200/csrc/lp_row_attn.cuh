@@ -10,6 +10,7 @@
 // it is -> the position's cache row, its factor behind the rows.  V channels per lane and load (4: dim and the columns multiples of 4).
 template <int V>
 __global__ void __launch_bounds__(256) lp_row_prep_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ P, int ldp, float* __restrict__ qbuf, int R) {
+    prev_grid();
     const int u = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, r = u / (a.H + a.G), h = u - r * (a.H + a.G);
     if (r >= R) return;
     const bool isq = h < a.H;
@@ -58,6 +59,7 @@ __host__ __device__ inline size_t row_split_smem(int D, int heads) { return (siz
 template <int VCH>
 __global__ void __launch_bounds__(32 * LS_HEADS) lp_row_split_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ qbuf, const float* __restrict__ P, int ldp,
                                                                      float* __restrict__ part_o, float* __restrict__ part_ml) {
+    prev_grid();
     extern __shared__ __align__(16) float ls_sm[];
     const int D = a.dim, pitch = D + 4, nwarp = blockDim.x >> 5, hpg = a.H / a.G, zb = (hpg + nwarp - 1) / nwarp;
     float* qs = ls_sm;                         // [warps][D]
@@ -182,6 +184,7 @@ constexpr int LC_BATCH = 8;
 template <typename T, int V>
 __global__ void __launch_bounds__(256) lp_row_combine_kernel(int H, int vdim, const float* __restrict__ part_o, const float* __restrict__ part_ml, int splits,
                                                              T* __restrict__ out, int out_ld) {
+    prev_grid();
     __shared__ float wgt[64], part[8][32 * V];              // (splits <= 64)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t at = ((size_t)blockIdx.x * H + blockIdx.y) * splits;
@@ -249,6 +252,7 @@ __device__ __forceinline__ void ldsm4_t(uint32_t* r, uint32_t addr) {
 }
 template <int DK, int DV>
 __global__ void __launch_bounds__(256) lp_row_tile_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ qbuf, bf16* __restrict__ out) {
+    prev_grid();
     constexpr int PITCH = DK + 8, NU = LT_KEYS * (DK / 4) / 256;
     constexpr bool AHEAD = DK <= 128;
     extern __shared__ __align__(16) uint8_t lt_sm[];

@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
                                                             const double* __restrict__ inv_freq, const float* __restrict__ lam_p,
                                                             float* __restrict__ vsrc, float* __restrict__ qbuf, int shift_tail,
                                                             const double* __restrict__ v_freq, float* __restrict__ vrot_out) {
+    prev_grid();
     extern __shared__ __align__(16) float ps[];
     float* y = ps;                              // [C]
     float* cs = ps + ((g.C + 3) & ~3);          // [rot_dims / 2] cos, then sin
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
 
 // After the rows of a step have been convolved: the run's tail becomes the last taps - 1 inputs of (old tail ++ new rows + bias).
 __global__ void lp_attn_conv_tail_kernel(StepMeta sm, PrepGeom g, const float* __restrict__ P, int ldp, const float* __restrict__ bias) {
+    prev_grid();
     const int run = blockIdx.x, r0 = sm.run_start[run], len = sm.run_start[run + 1] - r0;
     float* tail = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off);
     for (int c = threadIdx.x; c < g.C; c += blockDim.x) {

@@ -19,6 +19,7 @@ template <int DMAX>
 __global__ void __launch_bounds__(SCAN_BD) lp_ssd_scan_kernel(StepMeta sm, SsdGeom g, const float* __restrict__ XBC, int ldc, const float* __restrict__ P,
                                                               int ldp, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                                                               const float* __restrict__ Dskip, float* __restrict__ O, int ldo) {
+    prev_grid();
     constexpr int DREG = SCAN_DREG, CH = ScanChunk<DMAX>::N, SPLIT = DMAX / DREG, COLS = SCAN_BD / SPLIT;
     __shared__ __align__(16) float cs_[CH][DMAX];
     __shared__ __align__(16) float bs_[CH][DMAX];
@@ -108,6 +109,7 @@ __global__ void __launch_bounds__(SCAN_BD) lp_ssd_scan_kernel(StepMeta sm, SsdGe
 template <typename OutT>
 __global__ void __launch_bounds__(256) lp_gate_groupnorm_kernel(const float* __restrict__ O, int ldo, const float* __restrict__ P, int ldp, int z_off,
                                                                 const float* __restrict__ w, int n, int groups, float eps, OutT* __restrict__ out) {
+    prev_grid();
     __shared__ float red[9];
     const int r = blockIdx.x, gi = blockIdx.y, len = n / groups, c0 = gi * len;
     const float* o = O + (size_t)r * ldo + c0;

@@ -25,6 +25,7 @@ __device__ __forceinline__ void st_store(float* p, const float* o) {
 // (SMAX: compile-time bound of the stream count, 4 or ST_MAX, so that few streams cost few registers)
 template <typename OutT, int VEC, int SMAX>
 __global__ void __launch_bounds__(256) lp_streams_kernel(float* __restrict__ xs, StreamStep st, OutT* __restrict__ hn) {
+    prev_grid();
     extern __shared__ __align__(16) float u_s[];      // [width]
     __shared__ float red[9];
     __shared__ float mix_s[ST_MAX * ST_MAX], out_s[ST_MAX], in_s[ST_MAX];

@@ -115,6 +115,7 @@ __device__ __forceinline__ void sub_norm_row(const SubNorm& sn, int r, const flo
 // One block per row: the new stream (in place) and its copy `out`; before a mixture of experts also the router's logits and the choice.
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS) lp_sub_norm_kernel(SubNorm sn, const float* x, int width, T* __restrict__ out, StepRoute rt) {
+    prev_grid();
     extern __shared__ __align__(16) uint8_t sn_smem[];
     T* hs = reinterpret_cast<T*>(sn_smem);     // [width] (with routing only)
     const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -36,6 +36,7 @@ __device__ __forceinline__ int keys16_tiles(const StepMeta& sm, const AttnGeom& 
 // blockIdx.x: tile of all runs' tiles, blockIdx.y: K/V head.  cols: 64 x all tiles.
 template <int DKP, int DVP>
 __global__ void __launch_bounds__(256) lp_keys16_kernel(StepMeta sm, AttnGeom a, int n_runs, int cols, bf16* __restrict__ K16, bf16* __restrict__ Vt16) {
+    prev_grid();
     __shared__ bf16 sv[DVP][KA_K + 2];
     const int lane = threadIdx.x & 31, g = blockIdx.y, tile = blockIdx.x;
     int run = 0, base = 0;
@@ -119,6 +120,7 @@ template <int DKP, int DVP>
 __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, StepMeta sm, AttnGeom a,
                                                               const float* __restrict__ qbuf, const float* __restrict__ P, int ldp, int cols,
                                                               bf16* __restrict__ out, int out_ld, float out_scale, int* err) {
+    prev_grid();
     extern __shared__ __align__(1024) uint8_t ka_smem[];
     using SM = KaSmem<DKP, DVP>;
     const int run = blockIdx.y, g = blockIdx.x % a.G, bx = blockIdx.x / a.G, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

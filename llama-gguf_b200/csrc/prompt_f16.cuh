@@ -63,6 +63,8 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(int type, const uint8_
 namespace tc16 {
 using tc_t = __half;
 constexpr bool TC_BF16 = false;
+__device__ __forceinline__ void next_grid() {}      // (plain launches)
+__device__ __forceinline__ void wait_grid() {}
 enum { EPI_STORE = 0, EPI_ADD = 1, EPI_SILU_GLU = 2 };
 constexpr bool epi_is_glu(int epi) { return epi == EPI_SILU_GLU; }
 constexpr bool epi_is_act(int epi) { return epi == EPI_SILU_GLU; }
