@@ -52,12 +52,21 @@ __global__ void prefill_rope_kv_kernel(const PrefillRopeParams p) {
     float* row = p.qkv + (size_t)t * p.ld;
     const float* kraw = row + (size_t)p.n_heads * p.hd;
     const float* vraw = kraw + (size_t)p.n_kv * p.hd;
+    // a token's hd / 2 angles once per CTA (every head turns by the same ones; four 2048-wide layers, 333 tokens: 806 -> 798 us)
+    __shared__ float cs_s[64], sn_s[64];
+    const bool once = half <= 64;
+    if (once && (int)threadIdx.x < half) {
+        const float theta = position * p.freq[threadIdx.x];
+        cs_s[threadIdx.x] = cosf(theta);
+        sn_s[threadIdx.x] = sinf(theta);
+    }
+    __syncthreads();
     // gridDim.y CTAs share a token's items (each item is independent: same arithmetic whoever computes it)
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n_pairs + n_v; i += blockDim.x * gridDim.y) {
         if (i < n_pairs) {
             const int head = i / half, pi = i - head * half;
-            const float theta = position * p.freq[pi];
-            const float c = cosf(theta), s = sinf(theta);
+            const float theta = once ? 0.0f : position * p.freq[pi];
+            const float c = once ? cs_s[pi] : cosf(theta), s = once ? sn_s[pi] : sinf(theta);
             const int i0 = p.neox ? pi : 2 * pi, i1 = p.neox ? pi + half : 2 * pi + 1;
             if (head < p.n_heads) {
                 float* d = row + (size_t)head * p.hd;
