@@ -478,11 +478,13 @@ bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts,
 // what each one measured, of a step of 64 elements per CTA (operand bytes at 64 per clock) and of what a CTA adds when it is not overlapped
 // (filling the ring, epilogue, the exchange of a split), on 148 SMs.  Clusters of 8 do not tile the chip's SM groups: 128 of
 // their CTAs already took two waves (12.4 us where 64 CTAs in clusters of 4 took 8.3: 32 x 2048 x 2048).
+// split: K may be cut over a cluster.  Without, every sum adds its products in the order of K, so that a row's result is the same bits whatever the number of
+// rows of the step.
 struct TcPlan {
     bool persistent;
     int tn, splits;
 };
-TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu) {
+TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, bool split) {
     const int n_sm = 148, steps = (K + TC_K - 1) / TC_K, per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per;
     auto tiles = [&](int tn) { return (long long)n_mt * (seg ? xrows / tn + (groups + 1) / 2 : groups * ((R + tn - 1) / tn)); };
     TcPlan best{true, 256, 1};
@@ -498,7 +500,7 @@ TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu) {
     for (int tn : {128, 64}) {
         if (tn == 128 && R <= 64) continue;
         for (int s : {1, 2, 4, 8}) {
-            if (steps < 4 * s && s > 1) break;
+            if (s > 1 && (!split || steps < 4 * s)) break;
             const long long fit = s == 8 ? 112 : s == 4 ? 140 : n_sm, waves = (tiles(tn) * s + fit - 1) / fit;
             offer(false, tn, s, waves * ((steps + s - 1) / s * (tn == 128 ? 470 : 375) + 4500) - 4500 + 18 * tn + (s > 1 ? 1000 : 0));
         }

@@ -1442,6 +1442,11 @@ struct LpModel {
     std::vector<int> step_p0, step_len; // the step's runs: first position, tokens
     uint8_t* keys16 = nullptr;          // lp_tile_attn.cuh: the keys and values of one layer in bf16, kept from call to call
     size_t keys16_bytes = 0;
+    // Whether the products may cut K over a cluster (B200_LP_TC_SPLIT=0 / 1).  Not in programs with experts: another order of the sums is another rounding of the
+    // activations behind them, which after a few layers has changed every activation by its bf16 rounding, and a token whose second and third expert are that
+    // close then takes the other one -- a different row, not a rounding of it.
+    bool tc_split = true;
+    size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
     size_t chunk_scan_floats = 0;
     // Programmatic launches for steps of more than 16 rows (B200_LP_PDL=0: none): three ragged prompts 702 -> 605 us, prompt of 2048 910 -> 863, 32 prompts
@@ -1663,7 +1668,7 @@ bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, 
              int xrows, int groups, size_t wz, ZStride zs, const float* bias, float2 act) {
     if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs)) return false;
     const bool glu = epi_is_glu(epi), x_z = !seg && groups > 1 && zs.x > 0;
-    const TcPlan pl = tc_plan(R, N, K, groups, xrows, seg != nullptr, glu);
+    const TcPlan pl = tc_plan(R, N, K, groups, xrows, seg != nullptr, glu, m->tc_split);
     CUtensorMap xm, wm;
     const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     if (!tc_map(&xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, pl.tn, kh) ||
@@ -2000,6 +2005,8 @@ int lp_create(const b200_program_desc* prog, const b200_layer_desc* layers, int 
         if (e && *e) m->use_fuse = atoi(e) != 0;
         e = getenv("B200_LP_ATTN_TILE");
         if (e && *e) m->use_attn_tile = atoi(e) != 0;
+        e = getenv("B200_LP_KEYS16_MB");
+        if (e && *e) m->keys16_most = (size_t)std::max(0, atoi(e)) << 20;
         e = getenv("B200_LP_PDL");
         if (e && *e) m->use_pdl = atoi(e) != 0;
         e = getenv("B200_LP_CHUNK_SCAN");
@@ -2727,6 +2734,10 @@ int lp_finalize(LpModel* m, std::string* err) {
             LCU(cudaFuncSetAttribute(lp_streams_kernel<bf16, 4, ST_MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb));
         }
     }
+    {
+        const char* e = getenv("B200_LP_TC_SPLIT");
+        m->tc_split = e && *e ? atoi(e) != 0 : m->max_experts == 0;
+    }
     LCU_ALLOC(cudaMalloc((void**)&m->tc_err, 256));
     LCU(cudaMemset(m->tc_err, 0, 256));
     m->tail_counter = (unsigned*)(m->tc_err + 16);
@@ -2865,7 +2876,7 @@ template <int DKP, int DVP>
 bool attn_tc_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len, int tiles, int out_ld, float out_scale) {
     const int cols = tiles * KA_K;
     const size_t k_bytes = (size_t)ag.G * cols * DKP * 2, bytes = k_bytes + (size_t)ag.G * cols * DVP * 2;
-    if (bytes > ((size_t)1 << 30)) return false;
+    if (bytes > m->keys16_most) return false;
     if (bytes > m->keys16_bytes) {
         cudaFree(m->keys16);
         m->keys16 = nullptr;
@@ -2914,11 +2925,13 @@ bool attn_tc(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_
         tiles += t;
     }
     if (tiles > (1 << 20)) return false;
+    if (tiles == n_runs) return false;      // (one tile of keys per run: the copies would cost what the mma.sync kernels take for all of it)
     if (ag.dim <= 64 && ag.vdim <= 64) return attn_tc_launch<64, 64>(m, sm, ag, ldp, n_runs, max_len, (int)tiles, out_ld, out_scale);
     return attn_tc_launch<128, 128>(m, sm, ag, ldp, n_runs, max_len, (int)tiles, out_ld, out_scale);
 }
 
-// The same with mma.sync: key size a multiple of 16 up to 128, value size a multiple of 8 up to 256.
+// The same with mma.sync: key size a multiple of 16 up to 128, value size a multiple of 8 up to 256.  Values wider than 128, and the narrower heads whose
+// bf16 copies would be too large or find no room (instances of their own: a 64-wide head in the 256-wide instance carries four times its accumulators).
 template <int DK, int DV>
 bool attn_tile_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len) {
     const size_t smem = (size_t)(AT_K * (DK + 8) + DV * (AT_K + 8)) * 2;
@@ -2940,6 +2953,8 @@ bool attn_tile(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int 
     if (m->f32 || !m->use_attn_tile || max_len < 16) return false;
     if (attn_tc(m, sm, ag, ldp, n_runs, max_len, ag.out_ld, ag.out_scale)) return true;
     if (ag.dim % 16 || ag.vdim % 8 || ag.dim > 128 || ag.vdim > 256 || ag.out_ld % 2) return false;
+    if (ag.dim <= 64 && ag.vdim <= 64) return attn_tile_launch<64, 64>(m, sm, ag, ldp, n_runs, max_len);
+    if (ag.vdim <= 128) return attn_tile_launch<128, 128>(m, sm, ag, ldp, n_runs, max_len);
     return attn_tile_launch<128, 256>(m, sm, ag, ldp, n_runs, max_len);
 }
 
@@ -2965,6 +2980,8 @@ bool row_tile(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int n_runs, in
     AttnGeom tg = ag;
     tg.vrot = nullptr;
     if (attn_tc(m, sm, tg, 0, n_runs, max_len, ag.H * ag.vdim, 1.0f)) return true;
+    if (ag.dim <= 64 && ag.vdim <= 64) return row_tile_launch<64, 64>(m, sm, ag, n_runs, max_len);
+    if (ag.dim <= 128 && ag.vdim <= 128) return row_tile_launch<128, 128>(m, sm, ag, n_runs, max_len);
     if (ag.dim <= 320 && ag.vdim <= 256) return row_tile_launch<320, 256>(m, sm, ag, n_runs, max_len);
     return false;
 }

@@ -118,7 +118,7 @@ template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& x
 // Y[t][n] = epi(sum_k x[t][k] w[n][k] + bias[n]), T rows, N outputs (EPI_SILU_GLU: N units from the 2 N rows [gate | up] of w, fp16 Y)
 inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, cudaStream_t st) {
     const bool glu = epi_is_glu(epi);
-    const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu);
+    const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu, true);
     const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     CUtensorMap xm, wm;
     if (!tc_map(&xm, x, K, T, ldx, 1, 1, 0, pl.tn, kh) || !tc_map(&wm, w, K, N, K, glu ? 2 : 1, 1, 0, glu ? TC_M / 2 : TC_M, kh)) return cudaErrorInvalidValue;

@@ -75,6 +75,21 @@ def clear_weights(cfg, sequences, seed, margin=0.012):
     raise AssertionError("no clear choices found")
 
 
+def decided_weights(cfg, seed, lean=30.0):
+    """Random weights whose embedding rows lean towards two choices of every mixture (their logits `lean` above the rest before the layers add to the stream,
+    in equal parts, without a correction): rounding moves the two weights a little and never the choice, however many tokens there are"""
+    w, rng = random_weights(cfg, seed), np.random.default_rng(seed + 1)
+    for i, L in enumerate(cfg["layers"]):
+        if L["mlp"]["kind"] == "moe":
+            r = w["l%d.mlp.router" % i]
+            two = np.argsort(rng.random((cfg["vocab"], len(r))), axis=1)[:, :2]
+            step = lean / float((r * r).sum(1).mean()) / cfg["embedding"]["scale"]
+            w["embed"] = w["embed"] + step * (r[two[:, 0]] + r[two[:, 1]])
+            w["l%d.mlp.correction" % i] = np.zeros_like(w["l%d.mlp.correction" % i])
+    w["embed"] = bf16_to_f32(bf16_bits(np.asarray(w["embed"], dtype=np.float32))).reshape(w["embed"].shape)
+    return w
+
+
 def gpu_model(cfg, weights, compute="float32", max_seq_len=256, max_batch=4, taps=False):
     program, layers = gefovik.parse_config(cfg, max_seq_len, max_batch, compute)
     tensors = {n: (B.F32, list(reversed(a.shape)), np.ascontiguousarray(a, dtype=np.float32)) for n, a in weights.items()}

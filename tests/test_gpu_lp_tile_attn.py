@@ -1,4 +1,5 @@
-"""The tcgen05 attention of prompt rows (csrc/lp_tile_attn.cuh) against the warp kernel (B200_LP_ATTN_TILE=0), which scores in f32: kept first
+"""The tcgen05 attention of prompt rows (csrc/lp_tile_attn.cuh), and the mma.sync kernels that stand in for it where the bf16 copies find no room
+(B200_LP_KEYS16_MB=0), against the warp kernel (B200_LP_ATTN_TILE=0), which scores in f32: kept first
 tokens that fill, end inside and pass their tiles of 64, windows that leave tiles out between them and the first visible key, blocks of 128
 (token, head) pairs that end inside a token, portions that continue a cache, scores large enough that the running maximum jumps and
 the sums are rescaled.  Tolerance: bf16 queries, keys and probabilities (2^-8 each) against f32, as in the models' own tests; a wrong key or factor
@@ -6,6 +7,7 @@ is off by the size of the result."""
 import numpy as np
 import pytest
 
+import gefovik_synth as GS
 import lazilorn_synth as S
 
 pytestmark = pytest.mark.gpu
@@ -20,8 +22,9 @@ def test_against_the_warp_kernel(b200, monkeypatch, heads, kv_heads, dim, vdim, 
     rng = np.random.default_rng(window + keep)
     a, b, more = ([int(t) for t in rng.integers(0, cfg["vocab"], n)] for n in (450, 131, 97))
     outs = {}
-    for tile in ("1", "0"):
-        monkeypatch.setenv("B200_LP_ATTN_TILE", tile)
+    for tile, mb in (("1", "1024"), ("0", "1024"), ("mma", "0")):
+        monkeypatch.setenv("B200_LP_ATTN_TILE", "0" if tile == "0" else "1")
+        monkeypatch.setenv("B200_LP_KEYS16_MB", mb)
         gpu = S.gpu_model(cfg, w, "bfloat16", max_seq_len=640)
         try:
             first = gpu.step([(0, a), (1, b)], list(range(len(a) + len(b))))
@@ -29,4 +32,23 @@ def test_against_the_warp_kernel(b200, monkeypatch, heads, kv_heads, dim, vdim, 
             outs[tile] = np.concatenate([first, second])
         finally:
             gpu.close()
-    assert S.rel_err(outs["1"], outs["0"]) < (2e-2 if scale < 8 else 6e-2)      # (scores of tens: a bf16 score error is 2^-8 of them)
+    tol = 2e-2 if scale < 8 else 6e-2      # (scores of tens: a bf16 score error is 2^-8 of them)
+    assert S.rel_err(outs["1"], outs["0"]) < tol and S.rel_err(outs["mma"], outs["0"]) < tol
+
+
+@pytest.mark.parametrize("lens,same", [((48, 64, 17), True), ((48, 65, 17), False)])
+def test_one_tile_of_keys_per_run_keeps_the_mma_kernels(b200, monkeypatch, lens, same):
+    """Steps whose runs see one tile of keys each: bit for bit the mma.sync kernels (B200_LP_KEYS16_MB=0); with one run of 65 keys the other kernel takes the step."""
+    cfg = GS.config([GS.attn(heads=4, kv_heads=2, dim=128, softcap=50.0), GS.latent(heads=3, dim=16, vdim=24, kv_rank=128)], width=256, vocab=80)
+    w = GS.random_weights(cfg, 5)
+    rng = np.random.default_rng(1)
+    runs = [(i, [int(t) for t in rng.integers(0, cfg["vocab"], n)]) for i, n in enumerate(lens)]
+    outs = {}
+    for mb in ("1024", "0"):
+        monkeypatch.setenv("B200_LP_KEYS16_MB", mb)
+        gpu = GS.gpu_model(cfg, w, "bfloat16", max_seq_len=128)
+        try:
+            outs[mb] = gpu.step(runs, list(range(sum(lens))))
+        finally:
+            gpu.close()
+    assert (outs["1024"] == outs["0"]).all() == same
