@@ -2875,7 +2875,7 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
 template <int DKP, int DVP>
 bool attn_tc_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len, int tiles, int out_ld, float out_scale) {
     const int cols = tiles * KA_K;
-    const size_t k_bytes = (size_t)ag.G * cols * DKP * 2, bytes = k_bytes + (size_t)ag.G * cols * DVP * 2;
+    const size_t k_bytes = (size_t)ag.G * cols * DKP * 2, v_bytes = (size_t)ag.G * cols * DVP * 2, bytes = k_bytes + v_bytes + (ag.k_inv ? (size_t)ag.G * cols * 4 : 0);
     if (bytes > m->keys16_most) return false;
     if (bytes > m->keys16_bytes) {
         cudaFree(m->keys16);
@@ -2889,6 +2889,7 @@ bool attn_tc_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp,
         m->keys16_bytes = bytes;
     }
     bf16 *k16 = (bf16*)m->keys16, *vt16 = (bf16*)(m->keys16 + k_bytes);
+    float* factors = (float*)(m->keys16 + k_bytes + v_bytes);
     const TcEncodeFn fn = tc_encode_fn();
     CUtensorMap km, vm;
     const cuuint64_t kd[3] = {64, (cuuint64_t)ag.G * cols, DKP / 64}, ks[2] = {DKP * 2, 128}, vd[2] = {(cuuint64_t)cols, (cuuint64_t)ag.G * DVP}, vs[1] = {(cuuint64_t)cols * 2};
@@ -2910,9 +2911,9 @@ bool attn_tc_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp,
         }
         if (dev >= 0 && dev < 64) once[dev] = true;
     }
-    launch(m, lp_keys16_kernel<DKP, DVP>, dim3(tiles, ag.G), dim3(256), 0, sm, ag, n_runs, cols, k16, vt16);
+    launch(m, lp_keys16_kernel<DKP, DVP>, dim3(tiles, ag.G), dim3(256), 0, sm, ag, n_runs, cols, k16, vt16, factors);
     const unsigned blocks = (unsigned)(((size_t)max_len * (ag.H / ag.G) + KA_Q - 1) / KA_Q);
-    launch(m, lp_tile_attn_kernel<DKP, DVP>, dim3(blocks * ag.G, n_runs), dim3(192), smem, km, vm, sm, ag, (const float*)m->qbuf, (const float*)m->P, ldp, cols,
+    launch(m, lp_tile_attn_kernel<DKP, DVP>, dim3(blocks * ag.G, n_runs), dim3(192), smem, km, vm, sm, ag, (const float*)m->qbuf, (const float*)m->P, ldp, (const float*)factors, cols,
            (bf16*)m->act_a, out_ld, out_scale, m->tc_err);
     return true;
 }

@@ -4,10 +4,12 @@
 // The hpg = H / G heads of K/V head g meet the same cached rows, so their (token, head) pairs are ONE list of query rows, pair f = (token f / hpg,
 // head g hpg + f % hpg); a CTA takes 128 neighbours of the list against tiles of 64 keys:
 //   S = Q K^T (M = 128, N = 64) into one of two TMEM buffers; a thread per row reads its 64 scores, masks, caps, keeps the running maximum, writes
-//   the probabilities as bf16 into a swizzled tile, and O += P V (M = 128, N = DVP) accumulates in TMEM.  O is rescaled only when a row's
-//   maximum has grown by more than 2^8 since the last time (probabilities up to 2^8 lose nothing in bf16); the division comes last.
+//   the probabilities as bf16 into a swizzled tile, and O += P V (M = 128, N = DVP) accumulates in TMEM.  O is rescaled whenever a maximum of
+//   the warp's rows has grown, so that a probability is rounded against the running maximum, as in the mma.sync kernels (rescaling only past a growth of 2^8
+//   is as exact, saves nothing here -- the chain of a tile hides it: 886 against 888 us -- and rounds other values); the division comes last.
 // Both B operands have the contracted index contiguous, so the cached f32 rows are rounded to bf16 once per layer (lp_keys16_kernel): K16[g]
-// [key][DKP] and the transpose Vt16[g][channel][key], the keys of every run from the first one that a query of the step sees, in tiles of 64
+// [key][DKP], as they are stored (their factors, if they have any, go into F[g][key] and meet the f32 score: rounding key x factor moves every score by another
+// 2^-9 of itself and, through the layers behind, the logits), and the transpose Vt16[g][channel][key], the keys of every run from the first one that a query of the step sees, in tiles of 64
 // whose missing keys are zeros; TMA brings the tiles.  Roles: 4 softmax warps, a loader thread, an MMA thread; two CTAs share an SM (112 KB
 // of shared memory and 256 TMEM columns each), so one CTA's products run under the other's exponentials.
 // What bounded the mma.sync kernels (each block converting its own tiles, one tile after the other): 12.5 us per 64-key tile of
@@ -35,7 +37,8 @@ __device__ __forceinline__ int keys16_tiles(const StepMeta& sm, const AttnGeom& 
 
 // blockIdx.x: tile of all runs' tiles, blockIdx.y: K/V head.  cols: 64 x all tiles.
 template <int DKP, int DVP>
-__global__ void __launch_bounds__(256) lp_keys16_kernel(StepMeta sm, AttnGeom a, int n_runs, int cols, bf16* __restrict__ K16, bf16* __restrict__ Vt16) {
+__global__ void __launch_bounds__(256) lp_keys16_kernel(StepMeta sm, AttnGeom a, int n_runs, int cols, bf16* __restrict__ K16, bf16* __restrict__ Vt16,
+                                                        float* __restrict__ F) {
     prev_grid();
     __shared__ bf16 sv[DVP][KA_K + 2];
     const int lane = threadIdx.x & 31, g = blockIdx.y, tile = blockIdx.x;
@@ -68,9 +71,9 @@ __global__ void __launch_bounds__(256) lp_keys16_kernel(StepMeta sm, AttnGeom a,
     for (int i = threadIdx.x; i < KA_K * (DKP / 4); i += 256) {
         const int key = i / (DKP / 4), d = (i - key * (DKP / 4)) * 4, j = j0 + key;
         float4 v = (j < end && d < a.dim) ? *reinterpret_cast<const float4*>(kc + (size_t)j * ldk + g * a.dim + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float f = (kinv && j < end) ? kinv[(size_t)j * a.G] : 1.0f;
-        *reinterpret_cast<uint2*>(K16 + ((size_t)g * cols + (size_t)tile * KA_K + key) * DKP + d) = make_uint2(pack_bf2(v.x * f, v.y * f), pack_bf2(v.z * f, v.w * f));
+        *reinterpret_cast<uint2*>(K16 + ((size_t)g * cols + (size_t)tile * KA_K + key) * DKP + d) = make_uint2(pack_bf2(v.x, v.y), pack_bf2(v.z, v.w));
     }
+    if (kinv && threadIdx.x < KA_K) F[(size_t)g * cols + (size_t)tile * KA_K + threadIdx.x] = j0 + (int)threadIdx.x < end ? kinv[(size_t)(j0 + threadIdx.x) * a.G] : 0.0f;
 #pragma unroll 4
     for (int i = threadIdx.x; i < KA_K * (DVP / 4); i += 256) {
         const int key = i / (DVP / 4), c = (i - key * (DVP / 4)) * 4, j = j0 + key;
@@ -118,7 +121,7 @@ __device__ __forceinline__ void ka_mma(uint32_t acc, uint64_t da, uint64_t db, u
 // blockIdx.x = K/V head + G * (blocks from the last queries on), blockIdx.y = run.  out: rows out_ld apart.
 template <int DKP, int DVP>
 __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, StepMeta sm, AttnGeom a,
-                                                              const float* __restrict__ qbuf, const float* __restrict__ P, int ldp, int cols,
+                                                              const float* __restrict__ qbuf, const float* __restrict__ P, int ldp, const float* __restrict__ F, int cols,
                                                               bf16* __restrict__ out, int out_ld, float out_scale, int* err) {
     prev_grid();
     extern __shared__ __align__(1024) uint8_t ka_smem[];
@@ -246,9 +249,11 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
             if (attn_sink(a, h, &c)) { m = c * L2E; l = 1.0f; }
         }
         const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        const float* Fg = F + (size_t)g * cols + (size_t)before * KA_K;      // the keys' factors
         for (int t = 0; t < n_tiles; t++) {
             const uint32_t b = t & 1;
             const int j0 = position(t);
+            if (a.k_inv && lane < 2) asm volatile("prefetch.global.L1 [%0];" ::"l"(Fg + place(t) * KA_K + 32 * lane));
             uint32_t raw[KA_K];
             float s[KA_K];
             tc_wait(s_full + 8u * b, (t >> 1) & 1, alive, err, 28);
@@ -260,6 +265,14 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) tc_arrive(s_empty + 8u * b);
+            if (a.k_inv) {
+                const float4* f4 = reinterpret_cast<const float4*>(Fg + place(t) * KA_K);
+#pragma unroll
+                for (int e = 0; e < KA_K; e += 4) {
+                    const float4 f = f4[e / 4];
+                    s[e] *= f.x; s[e + 1] *= f.y; s[e + 2] *= f.z; s[e + 3] *= f.w;
+                }
+            }
             if (capped) {
 #pragma unroll
                 for (int e = 0; e < KA_K; e++) s[e] = soft_cap_exp(s[e], cap_in, cap_out);
@@ -291,7 +304,7 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
                 tc_wait(pv_done, (t - 1) & 1, alive, err, 29);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
-            if (__any_sync(0xffffffffu, mx > m + 8.0f)) {
+            if (__any_sync(0xffffffffu, mx > m)) {
                 const float mn = fmaxf(m, mx), c = m == -INFINITY ? 0.0f : ex2_fast(m - mn);
                 l *= c;
                 m = mn;

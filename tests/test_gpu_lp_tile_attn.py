@@ -36,6 +36,28 @@ def test_against_the_warp_kernel(b200, monkeypatch, heads, kv_heads, dim, vdim, 
     assert S.rel_err(outs["1"], outs["0"]) < tol and S.rel_err(outs["mma"], outs["0"]) < tol
 
 
+@pytest.mark.parametrize("layer", [GS.attn(heads=4, kv_heads=2, dim=128, scale=1.0, softcap=50.0), GS.attn(heads=3, kv_heads=1, dim=64, scale=1.0, softcap=1000.0),
+                                   GS.latent(heads=3, dim=16, vdim=24, kv_rank=128, scale=1.0), GS.latent(heads=4, dim=48, vdim=64, kv_rank=64, scale=1.0)])
+@pytest.mark.parametrize("n", [65, 130, 300])
+def test_rounds_what_the_mma_kernels_round(b200, monkeypatch, layer, n):
+    """Queries, keys as they are stored and probabilities against the running maximum of tiles of 64 keys are rounded to bf16, and nothing else: a key row's factor meets
+    the f32 score.  The mma.sync kernels (B200_LP_KEYS16_MB=0) round the same numbers, so both differ by the order of f32 sums: here and there a probability
+    of a row falls on the other side of a bf16 boundary, 2^-8 of itself and at most 4e-3 of the row where it is nearly all of it.  A product of key and factor
+    that is rounded moves scores of some tens (scale 1) by 2^-9 of themselves, the row by 1e-2 and more."""
+    cfg = GS.config([layer], width=256, vocab=80)
+    w = GS.random_weights(cfg, 5)
+    toks = [int(t) for t in np.random.default_rng(n).integers(0, cfg["vocab"], n)]
+    outs = {}
+    for mb in ("1024", "0"):
+        monkeypatch.setenv("B200_LP_KEYS16_MB", mb)
+        gpu = GS.gpu_model(cfg, w, "bfloat16", max_seq_len=320)
+        try:
+            outs[mb] = gpu.step([(0, toks), (1, toks[: n // 2 + 8])], list(range(n + n // 2 + 8)))
+        finally:
+            gpu.close()
+    assert GS.rel_err(outs["1024"], outs["0"]) < 4e-3
+
+
 @pytest.mark.parametrize("lens,same", [((48, 64, 17), True), ((48, 65, 17), False)])
 def test_one_tile_of_keys_per_run_keeps_the_mma_kernels(b200, monkeypatch, lens, same):
     """Steps whose runs see one tile of keys each: bit for bit the mma.sync kernels (B200_LP_KEYS16_MB=0); with one run of 65 keys the other kernel takes the step."""
