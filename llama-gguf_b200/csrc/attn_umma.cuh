@@ -23,6 +23,7 @@
 #pragma once
 #include <cuda.h>
 #include "gemm_umma2.cuh"
+#include "ring.cuh"
 
 namespace b200 {
 
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
 
     if (warp == kAttnLoader) {
         if (lane == 0) {
-            int asked = 0;
+            int asked_k = 0, asked_v = 0;
             for (int j = 0; j < nt; j++) {
                 const uint32_t b = j & 1, ph = ((j >> 1) & 1) ^ 1;
                 u2_wait(k_empty + 8u * b, ph, alive, p.err, 21, waited);
@@ -160,19 +161,24 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
 #pragma unroll
                     for (int s = 0; s < NS; s++)
                         u2_tma_2d(base + SM::K_AT + (2 * b + h) * SM::K + s * (kAttnTK * 128), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, k_full + 8u * b);
+                asked_k = j + 1;
                 u2_wait(v_empty + 8u * b, ph, alive, p.err, 22, waited);
                 if (!alive) break;
                 u2_expect_tx(v_full + 8u * b, (uint32_t)(2 * SM::V));
 #pragma unroll
                 for (int h = 0; h < 2; h++) u2_tma_2d(base + SM::V_AT + (2 * b + h) * SM::V, &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, v_full + 8u * b);
-                asked = j + 1;
+                asked_v = j + 1;
             }
-            if (!alive)                             // gave up: what has been asked for lands first (bounded)
-                for (int j = max(0, asked - 2); j < asked; j++) {
-                    bool w = true;
-                    u2_wait(k_full + 8u * (j & 1), (j >> 1) & 1, w, nullptr, 0, waited);
-                    u2_wait(v_full + 8u * (j & 1), (j >> 1) & 1, w, nullptr, 0, waited);
-                }
+            if (!alive) {                           // gave up: what has been asked for lands first (bounded)
+                auto land = [&](uint32_t full, int asked) {
+                    ring_in_flight<2>(asked, [&](int stage, unsigned parity) {
+                        bool w = true;
+                        u2_wait(full + 8u * stage, parity, w, nullptr, 0, waited);
+                    });
+                };
+                land(k_full, asked_k);
+                land(v_full, asked_v);
+            }
         }
     } else if (warp == kAttnMma) {
         if (lane == 0) {

@@ -10,6 +10,7 @@
 // modes.  B200_COMPUTE_BF16 keeps the matrices and the GEMM operands in bf16 (f32 accumulation, f32 results);
 // B200_COMPUTE_F32 keeps them in f32 and multiplies with FMA on the CUDA cores (no reduced-precision matrix mode).
 #include "layerprog.h"
+#include "ring.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
     auto position = [&](int t) { return t < nA ? t * KA_K : start + (t - nA + t_lo) * KA_K; };
     if (warp == 4) {
         if (lane == 0) {
-            for (int t = 0; t < n_tiles && alive; t++) {
+            int asked_k = 0, asked_v = 0;
+            for (int t = 0; t < n_tiles; t++) {
                 const uint32_t b = t & 1, ph = ((t >> 1) & 1) ^ 1;
                 const int col = (before + place(t)) * KA_K;
                 tc_wait(k_empty + 8u * b, ph, alive, err, 21);
@@ -182,19 +183,25 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
                 asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(base + SM::K_AT + b * SM::K),
                              "l"(&kmap), "r"(0), "r"(g * cols + col), "r"(0), "r"(k_full + 8u * b)
                              : "memory");
+                asked_k = t + 1;
                 tc_wait(v_empty + 8u * b, ph, alive, err, 22);
                 if (!alive) break;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(v_full + 8u * b), "r"((uint32_t)SM::V) : "memory");
                 asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(base + SM::V_AT + b * SM::V),
                              "l"(&vmap), "r"(col), "r"(g * DVP), "r"(v_full + 8u * b)
                              : "memory");
+                asked_v = t + 1;
             }
-            if (!alive)                 // gave up: what has been asked for lands first (bounded)
-                for (int t = max(0, n_tiles - 4); t < n_tiles; t++)
-                    for (uint32_t f : {k_full, v_full}) {
+            if (!alive) {               // gave up: what has been asked for lands first (bounded)
+                auto land = [&](uint32_t full, int asked) {
+                    ring_in_flight<2>(asked, [&](int stage, unsigned parity) {
                         bool w = true;
-                        tc_wait(f + 8u * (t & 1), (t >> 1) & 1, w, nullptr, 0);
-                    }
+                        tc_wait(full + 8u * stage, parity, w, nullptr, 0);
+                    });
+                };
+                land(k_full, asked_k);
+                land(v_full, asked_v);
+            }
         }
     } else if (warp == 5) {
         if (lane == 0) {
