@@ -34,6 +34,7 @@
 #include "gemm_umma.cuh"
 #include "gemm_umma2.cuh"
 #include "prompt_f16.cuh"
+#include "spare.cuh"
 #include "attn_umma.cuh"
 #include "kv_int8.cuh"
 #include "gguf_load.cuh"
@@ -997,6 +998,19 @@ static cudaError_t launch_attn(b200_ctx* c, const AttnParams& ap, int hd, int G)
 }
 
 // Enqueue every kernel of one token for `slot` on c->stream (captured into a graph by the caller).
+// Device memory that a call after loading has to have: the prompts' fp16 weight rows, which the fused products can do without, go first when there is no room
+static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
+    return (cudaError_t)alloc_or_give_back(
+        [&] { return (int)cudaMalloc(p, bytes); },
+        [&] {
+            cudaGetLastError();
+            if (!c->pf_w16) return false;
+            cudaFree(c->pf_w16);
+            c->pf_w16 = nullptr;
+            c->pf_w16_elems = 0;
+            return true;
+        });
+}
 static cudaError_t enqueue_token(b200_ctx* c, int slot_i, Mode mode, bool only_gemv = false) {
     const b200_model_desc& d = c->d;
     Slot& sl = c->slots[slot_i];
@@ -1220,10 +1234,10 @@ static int mega_build(b200_ctx* c) {
     };
 
     if (!c->mega_bar) {
-        CU_ALLOC(cudaMalloc((void**)&c->mega_bar, sizeof(unsigned int)));
-        CU_ALLOC(cudaMalloc((void**)&c->mega_cand_val, c->n_sm * sizeof(float)));
-        CU_ALLOC(cudaMalloc((void**)&c->mega_cand_idx, c->n_sm * sizeof(int)));
-        CU_ALLOC(cudaMalloc((void**)&c->mega_attn_part, (size_t)nkv * c->mega_splits * G * (hd + 2) * sizeof(float)));
+        CU_ALLOC(late_malloc(c, (void**)&c->mega_bar, sizeof(unsigned int)));
+        CU_ALLOC(late_malloc(c, (void**)&c->mega_cand_val, c->n_sm * sizeof(float)));
+        CU_ALLOC(late_malloc(c, (void**)&c->mega_cand_idx, c->n_sm * sizeof(int)));
+        CU_ALLOC(late_malloc(c, (void**)&c->mega_attn_part, (size_t)nkv * c->mega_splits * G * (hd + 2) * sizeof(float)));
     }
     // single GPU: every activation vector that feeds a GEMV is also kept in its staged form, written by the phase
     // that produces it (gemv_mma.cuh: stage_out32), so the consuming GEMV copies it instead of converting it per CTA
@@ -1231,7 +1245,7 @@ static int mega_build(b200_ctx* c) {
     if (staged && !c->mega_stage[0]) {
         const int ks[4] = {H, H, nh * hd, (int)d.ffn};
         for (int i = 0; i < 4; i++) {
-            CU_ALLOC(cudaMalloc((void**)&c->mega_stage[i], x_staged_bytes(ks[i]) + 256));
+            CU_ALLOC(late_malloc(c, (void**)&c->mega_stage[i], x_staged_bytes(ks[i]) + 256));
             CU(cudaMemset(c->mega_stage[i], 0, x_staged_bytes(ks[i]) + 256));
         }
     }
@@ -1314,7 +1328,7 @@ static int mega_build(b200_ctx* c) {
             prog.push_back(ph);
         }
         if (sl.d_phases) cudaFree(sl.d_phases);
-        CU_ALLOC(cudaMalloc((void**)&sl.d_phases, prog.size() * sizeof(MegaPhase)));
+        CU_ALLOC(late_malloc(c, (void**)&sl.d_phases, prog.size() * sizeof(MegaPhase)));
         CU(cudaMemcpy(sl.d_phases, prog.data(), prog.size() * sizeof(MegaPhase), cudaMemcpyHostToDevice));
         c->mega_phases = (int)prog.size();
     }
@@ -1458,7 +1472,7 @@ static int stream_build(b200_ctx* c) {
     if (!s1_ok && env_int("B200_LOG", 0)) fprintf(stderr, "[b200] stream_build: first streamed kernel not eligible (x region %zu of %zu bytes, %d slots)\n", x_region, avail, slots);
     if (c->d_tmaps) cudaFree(c->d_tmaps);
     c->d_tmaps = nullptr;
-    CU_ALLOC(cudaMalloc(&c->d_tmaps, maps.size() * sizeof(CUtensorMap)));
+    CU_ALLOC(late_malloc(c, (void**)&c->d_tmaps, maps.size() * sizeof(CUtensorMap)));
     CU(cudaMemcpy(c->d_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     for (size_t si = 0; si < c->slots.size(); si++) {
         for (MegaPhase& ph : progs[si]) {
@@ -1496,7 +1510,7 @@ static int stream2_build(b200_ctx* c, std::vector<std::vector<MegaPhase>>& progs
         if (P == 1 || d.hidden % 32 || (d.n_heads * hd) % 32 || d.ffn % 32) return B200_OK;
         const int ks[4] = {d.hidden, d.hidden, d.n_heads * hd, (int)d.ffn};
         for (int i = 0; i < 4; i++) {
-            CU_ALLOC(cudaMalloc((void**)&c->mega_stage[i], x_staged_bytes(ks[i]) + 256));
+            CU_ALLOC(late_malloc(c, (void**)&c->mega_stage[i], x_staged_bytes(ks[i]) + 256));
             CU(cudaMemset(c->mega_stage[i], 0, x_staged_bytes(ks[i]) + 256));
         }
     }
@@ -1529,10 +1543,10 @@ static int stream2_build(b200_ctx* c, std::vector<std::vector<MegaPhase>>& progs
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kS2Threads, smem));
     if (per_sm < 1) { if (env_int("B200_LOG", 0)) fprintf(stderr, "[b200] stream2_build: not eligible (occupancy)\n"); return B200_OK; }
     if (!c->s2_ll) {
-        CU_ALLOC(cudaMalloc((void**)&c->s2_ll, (size_t)c->n_sm * 64 * sizeof(uint2)));
+        CU_ALLOC(late_malloc(c, (void**)&c->s2_ll, (size_t)c->n_sm * 64 * sizeof(uint2)));
         CU(cudaMemset(c->s2_ll, 0, (size_t)c->n_sm * 64 * sizeof(uint2)));
-        CU_ALLOC(cudaMalloc((void**)&c->s2_cand_val, (size_t)c->n_sm * kS2Cons * sizeof(float)));
-        CU_ALLOC(cudaMalloc((void**)&c->s2_cand_idx, (size_t)c->n_sm * kS2Cons * sizeof(int)));
+        CU_ALLOC(late_malloc(c, (void**)&c->s2_cand_val, (size_t)c->n_sm * kS2Cons * sizeof(float)));
+        CU_ALLOC(late_malloc(c, (void**)&c->s2_cand_idx, (size_t)c->n_sm * kS2Cons * sizeof(int)));
         CU(cudaMemset(c->s2_cand_idx, 0xff, (size_t)c->n_sm * kS2Cons * sizeof(int)));
         CU(cudaMemset(c->s2_cand_val, 0, (size_t)c->n_sm * kS2Cons * sizeof(float)));
     }
@@ -1648,7 +1662,7 @@ static int stream2_build(b200_ctx* c, std::vector<std::vector<MegaPhase>>& progs
         Slot& sl = c->slots[si];
         if (sl.d_phases2) cudaFree(sl.d_phases2);
         sl.d_phases2 = nullptr;
-        CU_ALLOC(cudaMalloc((void**)&sl.d_phases2, prog2.size() * sizeof(MegaPhase)));
+        CU_ALLOC(late_malloc(c, (void**)&sl.d_phases2, prog2.size() * sizeof(MegaPhase)));
         CU(cudaMemcpy(sl.d_phases2, prog2.data(), prog2.size() * sizeof(MegaPhase), cudaMemcpyHostToDevice));
         c->s2_phases = (int)prog2.size();
     }
@@ -1796,7 +1810,7 @@ static int umma_tmaps_build(b200_ctx* c) {
     for (const Layer& L : c->layers) { add(L.wq); add(L.wk); add(L.wv); add(L.wo); add(L.gate); add(L.up); add(L.down); }
     add(c->output.present() ? c->output : c->token_embd);
     if (maps.empty()) return B200_OK;
-    CU_ALLOC(cudaMalloc(&c->pf_tmaps, maps.size() * sizeof(CUtensorMap)));
+    CU_ALLOC(late_malloc(c, (void**)&c->pf_tmaps, maps.size() * sizeof(CUtensorMap)));
     CU(cudaMemcpy(c->pf_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     return B200_OK;
 }
@@ -1858,15 +1872,15 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     const size_t per_tok = (size_t)H + QKV + 2 * (size_t)I + ((size_t)H + A + I + 1) / 2;   // floats (the fp16 rows count half)
     const int cap = std::min(prefill_chunk(), d.max_seq_len);
     if (!c->pf_buf) {
-        CU_ALLOC(cudaMalloc((void**)&c->pf_buf, per_tok * cap * sizeof(float)));
-        CU_ALLOC(cudaMalloc((void**)&c->pf_tok, cap * sizeof(int)));
-        CU_ALLOC(cudaMalloc((void**)&c->pf_rows, (size_t)cap * 24));
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_buf, per_tok * cap * sizeof(float)));
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_tok, cap * sizeof(int)));
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_rows, (size_t)cap * 24));
     }
     { int rc_t = umma_tmaps_build(c); if (rc_t) return rc_t; }
     if (!c->pf_split) {   // split-K scratch for passes of <= 64 rows: 8 partial tiles of the widest projection
         c->pf_split_floats = (size_t)8 * 64 * std::max(std::max(I, QKV), H);
-        CU_ALLOC(cudaMalloc((void**)&c->pf_split, c->pf_split_floats * sizeof(float)));
-        CU_ALLOC(cudaMalloc((void**)&c->pf_tile_cnt, 8192 * sizeof(int)));
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_split, c->pf_split_floats * sizeof(float)));
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_tile_cnt, 8192 * sizeof(int)));
         CU(cudaMemset(c->pf_tile_cnt, 0, 8192 * sizeof(int)));
     }
     // batched decode: per-row (position, KV base of the slot, SeqState of the slot)
@@ -1875,8 +1889,8 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     bool attn_tc = !rows && c->pf_attn_tc && gemm_encode_fn() && attn_umma_ok(hd, nh, nkv);
     if (attn_tc && !c->pf_k16) {
         const int P = (d.max_seq_len + 127) & ~127;
-        CU_ALLOC(cudaMalloc((void**)&c->pf_k16, (size_t)2 * nkv * P * hd * sizeof(__half)));    // hi rows, then lo rows
-        CU_ALLOC(cudaMalloc((void**)&c->pf_vt16, (size_t)2 * nkv * P * hd * sizeof(__half)));   // hi rows, then lo rows
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_k16, (size_t)2 * nkv * P * hd * sizeof(__half)));    // hi rows, then lo rows
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_vt16, (size_t)2 * nkv * P * hd * sizeof(__half)));   // hi rows, then lo rows
         c->pf_kv16_P = P;
         if (!attn_umma_encode(gemm_encode_fn(), c->pf_k16, c->pf_vt16, nkv, hd, P, &c->pf_kmap, &c->pf_vmap)) {
             c->pf_attn_tc = false;
@@ -1904,7 +1918,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (c->pf_logits_rows < n) {
             cudaFree(c->pf_logits);
             c->pf_logits = nullptr;
-            CU_ALLOC(cudaMalloc((void**)&c->pf_logits, (size_t)n * d.vocab * sizeof(float)));
+            CU_ALLOC(late_malloc(c, (void**)&c->pf_logits, (size_t)n * d.vocab * sizeof(float)));
             c->pf_logits_rows = n;
             for (auto& bg : c->batch_graphs) {   // (the captured head GEMMs write the old buffer)
                 if (bg.exec) cudaGraphExecDestroy(bg.exec);
@@ -3625,7 +3639,7 @@ extern "C" int b200_decode_batch_greedy(b200_ctx* c, const int* seqs, const uint
         if (c->pf_argmax_rows < n) {
             cudaFree(c->pf_argmax);
             c->pf_argmax = nullptr;
-            CU_ALLOC(cudaMalloc((void**)&c->pf_argmax, (size_t)n * sizeof(int)));
+            CU_ALLOC(late_malloc(c, (void**)&c->pf_argmax, (size_t)n * sizeof(int)));
             c->pf_argmax_rows = n;
         }
         if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs))) return rc;

@@ -11,6 +11,7 @@
 // B200_COMPUTE_F32 keeps them in f32 and multiplies with FMA on the CUDA cores (no reduced-precision matrix mode).
 #include "layerprog.h"
 #include "ring.cuh"
+#include "spare.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -2810,11 +2811,27 @@ int lp_get_taps(LpModel* m, float* out, size_t cap_floats, std::string* err) {
 
 // ------------------------------------------------------------------------------------------------ the step
 namespace {
+// Device memory of a step that has to be had (buffers, slots): the bf16 keys and the terms of the chunked scans, up to 1 and 0.5 GB that their kernels can do
+// without, go first when there is no room
+cudaError_t step_malloc(LpModel* m, void** p, size_t bytes) {
+    return (cudaError_t)alloc_or_give_back(
+        [&] { return (int)cudaMalloc(p, bytes); },
+        [&] {
+            cudaGetLastError();
+            if (!m->keys16 && !m->chunk_scan) return false;
+            cudaFree(m->keys16);
+            cudaFree(m->chunk_scan);
+            m->keys16 = nullptr;
+            m->chunk_scan = nullptr;
+            m->keys16_bytes = m->chunk_scan_floats = 0;
+            return true;
+        });
+}
 template <typename P>
-int grow(P** ptr, size_t bytes, std::string* err) {
+int grow(LpModel* m, P** ptr, size_t bytes, std::string* err) {
     cudaFree(*ptr);
     *ptr = nullptr;
-    LCU_ALLOC(cudaMalloc((void**)ptr, up16(bytes)));
+    LCU_ALLOC(step_malloc(m, (void**)ptr, up16(bytes)));
     return B200_OK;
 }
 
@@ -2825,37 +2842,37 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     const int W = m->p.width;
     if (R > m->cap_rows) {
         const int cap = std::max(R, std::min(2 * m->cap_rows, 1 << 20));
-        if ((rc = grow(&m->x, (size_t)cap * W * 4, err))) return rc;
-        if (m->p.post_norm == B200_FORM_NORM_OUTPUT && (rc = grow(&m->x2, (size_t)cap * W * 4, err))) return rc;
-        if ((rc = grow(&m->P, (size_t)cap * m->max_in * 4, err))) return rc;
-        if ((rc = grow(&m->qbuf, (size_t)cap * std::max(m->max_q, 1) * 4, err))) return rc;
-        if ((rc = grow(&m->O, (size_t)cap * std::max(m->max_o, 1) * 4, err))) return rc;
-        if ((rc = grow(&m->conv, (size_t)cap * std::max(m->max_conv, 1) * 4, err))) return rc;
-        if ((rc = grow(&m->hn, (size_t)cap * W * es, err))) return rc;
-        if ((rc = grow(&m->act_a, (size_t)cap * m->max_act * es, err))) return rc;
-        if ((m->p.post_norm || m->max_experts > 0 || m->p.streams > 0 || m->need_y2) && (rc = grow(&m->y, (size_t)cap * W * (m->need_y2 ? 8 : 4), err))) return rc;
-        if (m->max_vrot > 0 && (rc = grow(&m->vrot, (size_t)cap * m->max_vrot * 4, err))) return rc;
-        if (m->p.streams > 0 && (rc = grow(&m->xs, (size_t)cap * m->p.streams * W * 4, err))) return rc;
-        if (m->max_qrank > 0 && (rc = grow(&m->cq, (size_t)cap * m->max_qrank * es, err))) return rc;
-        if (m->p.loop_in && (rc = grow(&m->xcat, (size_t)cap * 2 * W * es, err))) return rc;
-        if (m->max_vsrc > 0 && (rc = grow(&m->vsrc, (size_t)cap * m->max_vsrc * 4, err))) return rc;
+        if ((rc = grow(m, &m->x, (size_t)cap * W * 4, err))) return rc;
+        if (m->p.post_norm == B200_FORM_NORM_OUTPUT && (rc = grow(m, &m->x2, (size_t)cap * W * 4, err))) return rc;
+        if ((rc = grow(m, &m->P, (size_t)cap * m->max_in * 4, err))) return rc;
+        if ((rc = grow(m, &m->qbuf, (size_t)cap * std::max(m->max_q, 1) * 4, err))) return rc;
+        if ((rc = grow(m, &m->O, (size_t)cap * std::max(m->max_o, 1) * 4, err))) return rc;
+        if ((rc = grow(m, &m->conv, (size_t)cap * std::max(m->max_conv, 1) * 4, err))) return rc;
+        if ((rc = grow(m, &m->hn, (size_t)cap * W * es, err))) return rc;
+        if ((rc = grow(m, &m->act_a, (size_t)cap * m->max_act * es, err))) return rc;
+        if ((m->p.post_norm || m->max_experts > 0 || m->p.streams > 0 || m->need_y2) && (rc = grow(m, &m->y, (size_t)cap * W * (m->need_y2 ? 8 : 4), err))) return rc;
+        if (m->max_vrot > 0 && (rc = grow(m, &m->vrot, (size_t)cap * m->max_vrot * 4, err))) return rc;
+        if (m->p.streams > 0 && (rc = grow(m, &m->xs, (size_t)cap * m->p.streams * W * 4, err))) return rc;
+        if (m->max_qrank > 0 && (rc = grow(m, &m->cq, (size_t)cap * m->max_qrank * es, err))) return rc;
+        if (m->p.loop_in && (rc = grow(m, &m->xcat, (size_t)cap * 2 * W * es, err))) return rc;
+        if (m->max_vsrc > 0 && (rc = grow(m, &m->vsrc, (size_t)cap * m->max_vsrc * 4, err))) return rc;
         if (m->max_experts > 0) {
-            if ((rc = grow(&m->moe_shw, (size_t)cap * 4, err))) return rc;
-            if ((rc = grow(&m->moe_w, (size_t)cap * m->max_experts * 4, err))) return rc;
-            if ((rc = grow(&m->moe_selw, (size_t)cap * m->max_top * 4, err))) return rc;
-            if ((rc = grow(&m->moe_sel, (size_t)cap * m->max_top * 4, err))) return rc;
-            if ((rc = grow(&m->moe_pos, (size_t)cap * m->max_top * 4, err))) return rc;
-            if ((rc = grow(&m->moe_seg, (size_t)(2 * m->max_experts + 2) * 4, err))) return rc;
-            if ((rc = grow(&m->moe_xp, (size_t)cap * m->max_top * W * es, err))) return rc;
-            if ((rc = grow(&m->moe_yp, (size_t)cap * m->max_top * W * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_shw, (size_t)cap * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_w, (size_t)cap * m->max_experts * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_selw, (size_t)cap * m->max_top * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_sel, (size_t)cap * m->max_top * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_pos, (size_t)cap * m->max_top * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_seg, (size_t)(2 * m->max_experts + 2) * 4, err))) return rc;
+            if ((rc = grow(m, &m->moe_xp, (size_t)cap * m->max_top * W * es, err))) return rc;
+            if ((rc = grow(m, &m->moe_yp, (size_t)cap * m->max_top * W * 4, err))) return rc;
         }
         m->cap_rows = cap;
     }
     if (n_want > m->cap_want) {
         const int cap = std::max(n_want, 2 * m->cap_want);
-        if ((rc = grow(&m->logits, (size_t)cap * m->p.vocab * 4, err))) return rc;
-        if ((rc = grow(&m->hw, (size_t)cap * W * es, err))) return rc;
-        if ((rc = grow(&m->pick, (size_t)cap * 4, err))) return rc;
+        if ((rc = grow(m, &m->logits, (size_t)cap * m->p.vocab * 4, err))) return rc;
+        if ((rc = grow(m, &m->hw, (size_t)cap * W * es, err))) return rc;
+        if ((rc = grow(m, &m->pick, (size_t)cap * 4, err))) return rc;
         m->cap_want = cap;
     }
     m->cap_runs = std::max(m->cap_runs, n_runs);
@@ -2864,7 +2881,7 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
         if (m->h_meta) cudaFreeHost(m->h_meta);
         m->h_meta = nullptr;
         LCU_ALLOC(cudaHostAlloc((void**)&m->h_meta, meta, cudaHostAllocDefault));
-        if ((rc = grow(&m->d_meta, meta, err))) return rc;
+        if ((rc = grow(m, &m->d_meta, meta, err))) return rc;
         m->meta_bytes = meta;
     }
     return B200_OK;
@@ -3761,8 +3778,8 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
                 s = m->pool.back();
                 m->pool.pop_back();
             } else {
-                LCU_ALLOC(cudaMalloc((void**)&s.kv, m->slot_kv_bytes));
-                cudaError_t e = cudaMalloc((void**)&s.rec, m->slot_rec_bytes);
+                LCU_ALLOC(step_malloc(m, (void**)&s.kv, m->slot_kv_bytes));
+                cudaError_t e = step_malloc(m, (void**)&s.rec, m->slot_rec_bytes);
                 if (e != cudaSuccess) {
                     cudaFree(s.kv);
                     s = SlotMem();
@@ -3814,7 +3831,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
     if (m->taps_on) {
         const size_t need = (size_t)m->runs.size() * lens[0] * W;
         if (need > m->taps_floats) {
-            if ((rc = grow(&m->taps, need * 4, err))) return rc;
+            if ((rc = grow(m, &m->taps, need * 4, err))) return rc;
             m->taps_floats = need;
         }
         m->taps_len = lens[0];
@@ -3830,7 +3847,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
             }
         if (need > m->glin_carry_bytes) {
             m->glin_carry_bytes = 0;
-            if ((rc = grow(&m->glin_carry, need, err))) return rc;
+            if ((rc = grow(m, &m->glin_carry, need, err))) return rc;
             m->glin_carry_bytes = need;
         }
     }
@@ -3838,7 +3855,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         const size_t need = (size_t)m->n_convs * n_runs * (p.in_conv - 1) * W * 4;
         if (need > m->conv_pend_bytes) {
             m->conv_pend_bytes = 0;
-            if ((rc = grow(&m->conv_pend, need, err))) return rc;
+            if ((rc = grow(m, &m->conv_pend, need, err))) return rc;
             m->scratch_epoch++;
             m->conv_pend_bytes = need;
         }

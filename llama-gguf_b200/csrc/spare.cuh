@@ -1,0 +1,11 @@
+// spare.cuh — scratch that a call can do without (it has another way): kept between calls, and given back when something that has no other way finds no
+// room.  Plain arithmetic (compiled by the host compiler in tests/test_spare_host.py).
+#pragma once
+#include <algorithm>
+#include <cstddef>
+
+// alloc(): 0, or an error.  give_back(): frees the scratch, false if there was none.
+template <typename Alloc, typename GiveBack> inline int alloc_or_give_back(Alloc alloc, GiveBack give_back) {
+    const int e = alloc();
+    return e && give_back() ? alloc() : e;
+}
