@@ -1450,7 +1450,7 @@ struct LpModel {
     bool tc_split = true;
     size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
-    size_t chunk_scan_floats = 0;
+    size_t chunk_scan_bytes = 0;
     // Programmatic launches for steps of more than 16 rows (B200_LP_PDL=0: none): three ragged prompts 702 -> 605 us, prompt of 2048 910 -> 863, 32 prompts
     // and 8 steps of 32 sequences 2717 -> 2530; one row, whose kernels fill the chip with blocks that would only wait, 6275 -> 6404 (24 steps)
     bool use_pdl = true, pdl_now = false;
@@ -2823,7 +2823,7 @@ cudaError_t step_malloc(LpModel* m, void** p, size_t bytes) {
             cudaFree(m->chunk_scan);
             m->keys16 = nullptr;
             m->chunk_scan = nullptr;
-            m->keys16_bytes = m->chunk_scan_floats = 0;
+            m->keys16_bytes = m->chunk_scan_bytes = 0;
             return true;
         });
 }
@@ -2887,6 +2887,26 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     return B200_OK;
 }
 
+// `want` bytes of scratch that is kept from call to call (spare.cuh); false: more than `most`, or no room, and none is kept
+template <typename P>
+bool keep_scratch(P*& p, size_t& have, size_t want, size_t most) {
+    if (want > most) return false;
+    if (want <= have) return true;
+    const size_t room = grown(have, want, most);
+    cudaFree(p);
+    p = nullptr;
+    have = 0;
+    for (size_t n : {room, want}) {
+        if (cudaMalloc((void**)&p, n) == cudaSuccess) {
+            have = n;
+            return true;
+        }
+        cudaGetLastError();
+        p = nullptr;
+    }
+    return false;
+}
+
 // Attention of prompt rows through tcgen05 (lp_tile_attn.cuh): bf16 mode, runs of at least 16 rows, key size a multiple of 16 and value size a
 // multiple of 8, both up to 128 (128-byte swizzled operands, 256 TMEM columns), while the bf16 copies of one layer's keys stay within 1 GB
 // (and the device has room for them); wider heads take the mma.sync kernels below, everything else the warp kernel.
@@ -2894,18 +2914,7 @@ template <int DKP, int DVP>
 bool attn_tc_launch(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_runs, int max_len, int tiles, int out_ld, float out_scale) {
     const int cols = tiles * KA_K;
     const size_t k_bytes = (size_t)ag.G * cols * DKP * 2, v_bytes = (size_t)ag.G * cols * DVP * 2, bytes = k_bytes + v_bytes + (ag.k_inv ? (size_t)ag.G * cols * 4 : 0);
-    if (bytes > m->keys16_most) return false;
-    if (bytes > m->keys16_bytes) {
-        cudaFree(m->keys16);
-        m->keys16 = nullptr;
-        m->keys16_bytes = 0;
-        if (cudaMalloc((void**)&m->keys16, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            m->keys16 = nullptr;
-            return false;
-        }
-        m->keys16_bytes = bytes;
-    }
+    if (!keep_scratch(m->keys16, m->keys16_bytes, bytes, m->keys16_most)) return false;
     bf16 *k16 = (bf16*)m->keys16, *vt16 = (bf16*)(m->keys16 + k_bytes);
     float* factors = (float*)(m->keys16 + k_bytes + v_bytes);
     const TcEncodeFn fn = tc_encode_fn();
@@ -3034,19 +3043,8 @@ bool chunk_scan(LpModel* m, const StepMeta& sm, ChunkScan g, int n_runs, int max
     if (!m->use_chunk_scan || max_len < (MODE == CS_SSD ? 128 : 48)) return false;
     if (g.dim % 4 || g.vdim % 4 || g.dim > 128 || g.ldq % 4 || g.ldv % 4 || (((uintptr_t)g.Q | (uintptr_t)g.K | (uintptr_t)g.V) & 15)) return false;
     const size_t hr = (size_t)g.H * g.R, nm = MODE == CS_MEM ? (size_t)n_runs * g.H * (g.dim + 1) : 0;
-    const size_t want = hr * (3 + CS) + 8 + (MODE == CS_DELTA ? hr * (g.dim + g.vdim) : 0) + nm;
-    if (want > ((size_t)128 << 20)) return false;
-    if (want > m->chunk_scan_floats) {
-        cudaFree(m->chunk_scan);
-        m->chunk_scan = nullptr;
-        m->chunk_scan_floats = 0;
-        if (cudaMalloc((void**)&m->chunk_scan, want * 4) != cudaSuccess) {
-            cudaGetLastError();
-            m->chunk_scan = nullptr;
-            return false;
-        }
-        m->chunk_scan_floats = want;
-    }
+    const size_t want = (hr * (3 + CS) + 8 + (MODE == CS_DELTA ? hr * (g.dim + g.vdim) : 0) + nm) * 4;
+    if (!keep_scratch(m->chunk_scan, m->chunk_scan_bytes, want, (size_t)512 << 20)) return false;
     g.M = m->chunk_scan;                               // (16-byte rows first)
     g.W = g.M + hr * CS;
     g.U0 = g.W + (MODE == CS_DELTA ? hr * g.dim : 0);

@@ -9,3 +9,7 @@ template <typename Alloc, typename GiveBack> inline int alloc_or_give_back(Alloc
     const int e = alloc();
     return e && give_back() ? alloc() : e;
 }
+
+// What scratch of `have` bytes grows to for `want` (have < want <= most): at least twice what it was, so that a conversation whose portions ask for a little
+// more each time allocates (and waits for the device) a few times in all; never above `most`.
+inline size_t grown(size_t have, size_t want, size_t most) { return std::min(most, std::max(want, 2 * have)); }

@@ -1,7 +1,9 @@
-"""csrc/spare.cuh on the host, with a device that has so much room: what has to be had takes the room of scratch that can be done without, once, and only
-when it has to."""
+"""csrc/spare.cuh on the host.  With a device that has so much room, what has to be had takes the room of scratch that can be done without, once, and only
+when it has to; scratch that grows a little with every portion of a conversation is allocated a few times in all."""
 import os
 import subprocess
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "llama-gguf_b200", "csrc")
 
@@ -23,8 +25,31 @@ int main() {
 """
 
 
-def test_scratch_goes_before_an_allocation_fails(tmp_path):
-    (tmp_path / "t.cpp").write_text(PROGRAM)
+GROWTH = r"""
+#include <cstdio>
+#include "spare.cuh"
+int main() {
+    const size_t most = (size_t)1 << 30;
+    for (size_t portion : {(size_t)4096, (size_t)100000, (size_t)7777777}) {       // portions that see a little more each time, up to the limit
+        size_t have = 0;
+        int times = 0;
+        for (size_t want = portion; want <= most; want += portion)
+            if (want > have) {
+                const size_t n = grown(have, want, most);
+                if (n < want || n > most) return printf("%zu -> %zu\n", want, n), 1;
+                have = n;
+                times++;
+            }
+        if (times > 20) return printf("%d allocations\n", times), 1;               // log2(1 GB / 4096) = 18, the first and the limit
+    }
+    return 0;
+}
+"""
+
+
+@pytest.mark.parametrize("program", [PROGRAM, GROWTH], ids=["gives_back", "grows"])
+def test_on_the_host(tmp_path, program):
+    (tmp_path / "t.cpp").write_text(program)
     exe = str(tmp_path / "t")
     subprocess.run(["g++", "-std=c++17", "-I", CSRC, "-o", exe, str(tmp_path / "t.cpp")], check=True)
     r = subprocess.run([exe], capture_output=True, text=True)
