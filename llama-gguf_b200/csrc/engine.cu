@@ -1980,7 +1980,9 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         return gemm_dispatch(p, c->n_sm, st, &c->launches);
     };
     // Two-pass products (prompt_f16.cuh): the rows of `ws` one after the other -> fp16, at most pf_w16_elems at a time, then the product of those
-    // rows.  glu: ws = {gate, up}, the unit silu(gate) up -> fp16 y.
+    // rows.  glu: ws = {gate, up}, the unit silu(gate) up -> fp16 y.  cudaErrorNotSupported: the driver refused a tensor map (B200_PROMPT_F16_MAPS=0: as
+    // if it did), nothing has been computed, and the caller takes the fused products.
+    const bool f16_maps = env_int("B200_PROMPT_F16_MAPS", 1) != 0;
     auto gemm16 = [&](std::initializer_list<const DevTensor*> ws, int K, const __half* x, int ldx, int T, void* y, int ldy, const float* bias, int epi) -> cudaError_t {
         const bool glu = epi == tc16::EPI_SILU_GLU;
         long long total = 0;
@@ -2003,8 +2005,8 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 if (!glu) first += (long long)w->ne[1];
             }
             void* yt = glu ? (void*)((__half*)y + at) : (void*)((float*)y + at);
-            const cudaError_t e = tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, st);
-            if (e != cudaSuccess) return e;
+            const cudaError_t e = f16_maps ? tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, st) : cudaErrorNotSupported;
+            if (e != cudaSuccess) return e == cudaErrorNotSupported && at > 0 ? cudaErrorInvalidValue : e;
             c->launches++;
         }
         return cudaSuccess;
@@ -2024,10 +2026,18 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             c->pf_w16 = nullptr;
         }
     }
+    bool f16 = false;             // (of the chunk)
+    auto product = [&](const DevTensor& w, int K, const __half* x, int ldx, int T, float* y, int ldy, const DevTensor* bias, int acc) -> cudaError_t {
+        if (f16) {
+            const cudaError_t e = gemm16({&w}, K, x, ldx, T, y, ldy, bias && bias->present() ? bias->f32() : nullptr, acc ? tc16::EPI_ADD : tc16::EPI_STORE);
+            if (e != cudaErrorNotSupported) return e;
+        }
+        return gemm(w, K, x, ldx, T, y, ldy, bias, acc);
+    };
     int last_T = 0;
     for (int done = 0; done < n; done += cap) {
         const int T = std::min(cap, n - done);
-        const bool f16 = f16_able && c->pf_w16 && T >= f16_min;
+        f16 = f16_able && c->pf_w16 && T >= f16_min;
         const int pos0 = (int)sl.host_pos + done;
         last_T = T;
         if (!use_graph) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -2037,17 +2047,12 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             float* kc = sl.kv + (size_t)l * kv_layer;
             float* vc = kc + kv_layer / 2;
             CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.attn_norm.f32(), d.norm_eps, XNh, H));
-            if (f16 && !(L.bq.present() || L.bk.present() || L.bv.present())) {
-                CU(gemm16({&L.wq, &L.wk, &L.wv}, H, XNh, H, T, Q, QKV, nullptr, tc16::EPI_STORE));
-            } else if (f16) {
-                CU(gemm16({&L.wq}, H, XNh, H, T, Q, QKV, L.bq.present() ? L.bq.f32() : nullptr, tc16::EPI_STORE));
-                CU(gemm16({&L.wk}, H, XNh, H, T, Q + A, QKV, L.bk.present() ? L.bk.f32() : nullptr, tc16::EPI_STORE));
-                CU(gemm16({&L.wv}, H, XNh, H, T, Q + A + nkv * hd, QKV, L.bv.present() ? L.bv.f32() : nullptr, tc16::EPI_STORE));
-            } else {
-                CU(gemm(L.wq, H, XNh, H, T, Q, QKV, &L.bq, 0));
-                CU(gemm(L.wk, H, XNh, H, T, Q + A, QKV, &L.bk, 0));
-                CU(gemm(L.wv, H, XNh, H, T, Q + A + nkv * hd, QKV, &L.bv, 0));
-            }
+            cudaError_t e16 = f16 && !(L.bq.present() || L.bk.present() || L.bv.present()) ? gemm16({&L.wq, &L.wk, &L.wv}, H, XNh, H, T, Q, QKV, nullptr, tc16::EPI_STORE) : cudaErrorNotSupported;
+            if (e16 == cudaErrorNotSupported) {
+                CU(product(L.wq, H, XNh, H, T, Q, QKV, &L.bq, 0));
+                CU(product(L.wk, H, XNh, H, T, Q + A, QKV, &L.bk, 0));
+                CU(product(L.wv, H, XNh, H, T, Q + A + nkv * hd, QKV, &L.bv, 0));
+            } else CU(e16);
             PrefillRopeParams rp{};
             rp.qkv = Q; rp.ld = QKV; rp.k_cache = kc; rp.v_cache = vc; rp.freq = c->rope_freq; rp.pos0 = pos0;
             rp.n_heads = nh; rp.n_kv = nkv; rp.hd = hd; rp.max_seq = d.max_seq_len; rp.neox = d.rope_neox; rp.rope_scale = d.rope_scale;
@@ -2096,20 +2101,17 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                     CU(launch_on(st, pdl, Gq <= 4 ? prefill_attn_kernel<64, 4> : prefill_attn_kernel<64, 8>, dim3(ablocks), dim3(128), 0, ap));
                 }
             }
-            if (f16) CU(gemm16({&L.wo}, A, ATh, A, T, X, H, nullptr, tc16::EPI_ADD));
-            else CU(gemm(L.wo, A, ATh, A, T, X, H, nullptr, 1));                  // X += Wo attn
+            CU(product(L.wo, A, ATh, A, T, X, H, nullptr, 1));                    // X += Wo attn
             CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.ffn_norm.f32(), d.norm_eps, XNh, H));
-            if (f16) {
-                CU(gemm16({&L.gate, &L.up}, H, XNh, H, T, Hh, I, nullptr, tc16::EPI_SILU_GLU));
-                CU(gemm16({&L.down}, I, Hh, I, T, X, H, nullptr, tc16::EPI_ADD));
-                c->launches += 4;
-                continue;
-            }
-            CU(gemm(L.gate, H, XNh, H, T, G, I, nullptr, 0));
-            CU(gemm(L.up, H, XNh, H, T, U, I, nullptr, 0));
-            CU(launch_on(st, pdl, prefill_swiglu_kernel, dim3(std::min(148 * 8, (int)(((long long)T * I + 255) / 256))), dim3(256), 0, (const float*)G, (const float*)U, Hh, (long long)T * I));
-            CU(gemm(L.down, I, Hh, I, T, X, H, nullptr, 1));                      // X += Wd act
-            c->launches += 5;
+            e16 = f16 ? gemm16({&L.gate, &L.up}, H, XNh, H, T, Hh, I, nullptr, tc16::EPI_SILU_GLU) : cudaErrorNotSupported;
+            if (e16 == cudaErrorNotSupported) {
+                CU(product(L.gate, H, XNh, H, T, G, I, nullptr, 0));
+                CU(product(L.up, H, XNh, H, T, U, I, nullptr, 0));
+                CU(launch_on(st, pdl, prefill_swiglu_kernel, dim3(std::min(148 * 8, (int)(((long long)T * I + 255) / 256))), dim3(256), 0, (const float*)G, (const float*)U, Hh, (long long)T * I));
+                c->launches += 1;
+            } else CU(e16);
+            CU(product(L.down, I, Hh, I, T, X, H, nullptr, 1));                   // X += Wd act
+            c->launches += 4;
         }
         c->launches += 1;
         CU(cudaGetLastError());

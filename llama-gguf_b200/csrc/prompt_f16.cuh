@@ -115,13 +115,14 @@ template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& x
     const dim3 grid(n_mt * pl.splits, n_nt);
     return pl.tn == 128 ? launch_as<128, false, EPI>(xm, wm, a, grid, st) : launch_as<64, false, EPI>(xm, wm, a, grid, st);
 }
-// Y[t][n] = epi(sum_k x[t][k] w[n][k] + bias[n]), T rows, N outputs (EPI_SILU_GLU: N units from the 2 N rows [gate | up] of w, fp16 Y)
+// Y[t][n] = epi(sum_k x[t][k] w[n][k] + bias[n]), T rows, N outputs (EPI_SILU_GLU: N units from the 2 N rows [gate | up] of w, fp16 Y).
+// cudaErrorNotSupported: a tensor map was refused, nothing was launched
 inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, cudaStream_t st) {
     const bool glu = epi_is_glu(epi);
     const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu, true);
     const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     CUtensorMap xm, wm;
-    if (!tc_map(&xm, x, K, T, ldx, 1, 1, 0, pl.tn, kh) || !tc_map(&wm, w, K, N, K, glu ? 2 : 1, 1, 0, glu ? TC_M / 2 : TC_M, kh)) return cudaErrorInvalidValue;
+    if (!tc_map(&xm, x, K, T, ldx, 1, 1, 0, pl.tn, kh) || !tc_map(&wm, w, K, N, K, glu ? 2 : 1, 1, 0, glu ? TC_M / 2 : TC_M, kh)) return cudaErrorNotSupported;
     const TcArgs a{y, ldy, T, N, K, 1.0f, err, nullptr, 1, 0, 0, bias, float2{0.0f, 0.0f}, pl.splits, K % TC_K == 0 ? 1 : 0};
     return epi == EPI_STORE ? launch_epi<EPI_STORE>(pl, xm, wm, a, st) : epi == EPI_ADD ? launch_epi<EPI_ADD>(pl, xm, wm, a, st) : launch_epi<EPI_SILU_GLU>(pl, xm, wm, a, st);
 }

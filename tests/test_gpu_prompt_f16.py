@@ -35,3 +35,13 @@ def test_two_passes_against_the_fused_product(b200, monkeypatch, preset, mix, n)
     assert rel_err(two, fused) < TOL
     few = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="1", B200_PROMPT_F16_KROWS="1")     # portions of the least size
     assert rel_err(few, two) < TOL
+
+
+@pytest.mark.parametrize("preset,mix", [("llama-tiny", "Q4_K_M"), ("qwen-tiny", "Q8_0")])
+def test_a_refused_tensor_map_takes_the_fused_products(b200, monkeypatch, preset, mix):
+    """Bit for bit what the fused kernels give; the refusal is the host's (B200_PROMPT_F16_MAPS=0)."""
+    arch, desc, tensors = synth.synth_model(preset, mix, 160)
+    prompt = synth.prompt_tokens(129, desc["vocab"])
+    fused = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="100000")
+    refused = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="1", B200_PROMPT_F16_MAPS="0")
+    assert (refused == fused).all()
