@@ -1448,6 +1448,7 @@ struct LpModel {
     // activations behind them, which after a few layers has changed every activation by its bf16 rounding, and a token whose second and third expert are that
     // close then takes the other one -- a different row, not a rounding of it.
     bool tc_split = true;
+    bool tc_maps = true;                    // B200_LP_TC_MAPS=0: as if the driver refused the tensor maps of the products
     size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
     size_t chunk_scan_bytes = 0;
@@ -1665,16 +1666,27 @@ bool tc_takes(const LpModel* m, const void* X, int ldx, const void* W, int ldw, 
     if (m->f32 || !m->use_tc || R < m->tc_min_rows) return false;
     return !(K % 8 || ldx % 8 || ldw % 8 || wz % 8 || zs.x % 8 || ((uintptr_t)X & 15) || ((uintptr_t)W & 15));
 }
-// xrows: rows of X in all groups of `seg` together
+// A product's plan and tensor maps; false: not taken, or the driver refused a map (B200_LP_TC_MAPS=0: as if it did).  xrows: rows of X in all groups of `seg`
+// together
+struct TcProduct {
+    TcPlan pl;
+    CUtensorMap xm, wm;
+};
+bool tc_prepare(const LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, int R, bool glu, bool seg, int xrows, int groups, size_t wz, ZStride zs, TcProduct& t) {
+    if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs) || !m->tc_maps) return false;
+    const bool x_z = !seg && groups > 1 && zs.x > 0;
+    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->tc_split);
+    const int kh = t.pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
+    return tc_map(&t.xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, t.pl.tn, kh) &&
+           tc_map(&t.wm, W, K, N, ldw, glu ? 2 : 1, groups, wz, glu ? TC_M / 2 : TC_M, kh);
+}
 bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, void* Y, int ldy, int R, float alpha, int epi, const int* seg,
              int xrows, int groups, size_t wz, ZStride zs, const float* bias, float2 act) {
-    if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs)) return false;
     const bool glu = epi_is_glu(epi), x_z = !seg && groups > 1 && zs.x > 0;
-    const TcPlan pl = tc_plan(R, N, K, groups, xrows, seg != nullptr, glu, m->tc_split);
-    CUtensorMap xm, wm;
-    const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
-    if (!tc_map(&xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, pl.tn, kh) ||
-        !tc_map(&wm, W, K, N, ldw, glu ? 2 : 1, groups, wz, glu ? TC_M / 2 : TC_M, kh)) return false;
+    TcProduct t;
+    if (!tc_prepare(m, X, ldx, W, ldw, N, K, R, glu, seg != nullptr, xrows, groups, wz, zs, t)) return false;
+    const TcPlan& pl = t.pl;
+    const CUtensorMap &xm = t.xm, &wm = t.wm;
     const TcArgs a{Y, ldy, R, N, K, alpha, m->tc_err, seg, groups, x_z ? 1 : 0, zs.y, bias, act, pl.splits, K % TC_K == 0 ? 1 : 0};
     const int per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per, n_nt = (R + pl.tn - 1) / pl.tn;
     if (pl.persistent) {
@@ -1686,12 +1698,14 @@ bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, 
     return pl.tn == 128 ? tc_launch<128, false>(m, xm, wm, a, grid, epi) : tc_launch<64, false>(m, xm, wm, a, grid, epi);
 }
 
-// Whether gemm / project_in can end with a gated epilogue for these rows (K: the products' length; few: the input is made by the projection)
-bool glu_takes(const LpModel* m, const void* X, const void* W, int K, int R) {
+// Whether gemm / project_in can end with a gated epilogue for these rows (N units, K: the products' length; few: the input is made by the projection).  The
+// CUDA-core product has no such epilogue, so the tensor maps are tried here
+bool glu_takes(const LpModel* m, const void* X, const void* W, int N, int K, int R) {
     if (!m->use_fuse || m->f32) return false;
     if (R <= 2 || (!m->use_gemv_mma && R <= 2 * GV_ROWS)) return false;
     if (R <= 2 * GV_ROWS) return K % 32 == 0 && ((uintptr_t)X % 16) == 0 && ((uintptr_t)W % 16) == 0;
-    return tc_takes(m, X, K, W, K, K, R, 0, ZStride{0, 0});
+    TcProduct t;
+    return tc_prepare(m, X, K, W, K, N, K, R, true, false, 0, 1, 0, ZStride{0, 0}, t);
 }
 // Y = epi(alpha X W^T): rows of the step against a [N][K] matrix in the compute type.  Without `seg`, groups > 1 batches the product
 // over heads: head z multiplies columns [z zs.x, z zs.x + K) of X with rows [z N, (z + 1) N) of W (wz = N ldw) into columns
@@ -1757,6 +1771,10 @@ void gemm_t(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, i
         return;
     }
     if (tc_gemm(m, X, ldx, W, ldw, N, K, Y, ldy, R, alpha, epi, seg, xrows, groups, wz, zs, bias, act)) return;
+    if (epi_is_glu(epi)) {        // (glu_takes said yes, and the launch was refused since: an error of the step, never another epilogue)
+        if (m->launch_fail.empty()) m->launch_fail = "a gated product could not be launched";
+        return;
+    }
     dim3 grid((N + GB - 1) / GB, (R + GB - 1) / GB, groups), block(256);
 #define LP_GM(E) launch(m, lp_gemm_kernel<T, E>, grid, block, 0, x, ldx, w, ldw, Y, ldy, R, N, K, alpha, seg, wz, zs, bias, act)
     if (epi == EPI_STORE) LP_GM(EPI_STORE);
@@ -2007,6 +2025,8 @@ int lp_create(const b200_program_desc* prog, const b200_layer_desc* layers, int 
         if (e && *e) m->use_fuse = atoi(e) != 0;
         e = getenv("B200_LP_ATTN_TILE");
         if (e && *e) m->use_attn_tile = atoi(e) != 0;
+        e = getenv("B200_LP_TC_MAPS");
+        if (e && *e) m->tc_maps = atoi(e) != 0;
         e = getenv("B200_LP_KEYS16_MB");
         if (e && *e) m->keys16_most = (size_t)std::max(0, atoi(e)) << 20;
         e = getenv("B200_LP_PDL");
@@ -3551,8 +3571,10 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
             const int act_epi = e.act == B200_ACT_GELU ? EPI_GELU : e.act == B200_ACT_SILU_GLU ? EPI_SILU_GLU : e.act == B200_ACT_RELU_GLU ? EPI_RELU_GLU : EPI_RELU2;
             const int per = act_gated(e.act) ? 2 * e.expert_ff : e.expert_ff;                // rows of one expert's up matrix
             // gated experts whose weights go onto their outputs: the units in the grouped product's epilogue
+            TcProduct tried;
             const bool glu_epi = (e.act == B200_ACT_SILU_GLU || e.act == B200_ACT_RELU_GLU) && !e.weight_input && m->use_fuse &&
-                                 tc_takes(m, m->moe_xp, W, (const uint8_t*)L.w_up + (size_t)L.up_router_rows * W * es, W, W, R, (size_t)per * W, ZStride{0, 0});
+                                 tc_prepare(m, m->moe_xp, W, (const uint8_t*)L.w_up + (size_t)L.up_router_rows * W * es, W, e.expert_ff, W, R, true, true, R * e.top,
+                                            e.experts, (size_t)per * W, ZStride{0, 0}, tried);
             const bool own_act = (act_gated(e.act) && !glu_epi) || e.weight_input != 0;        // the hidden units need a kernel of their own
             const ExpertAct ea{e.act, e.weight_input, e.limit, e.shared_limit, e.slope};
             const int outs = e.experts + e.identity;                                            // what the router chooses among
@@ -3678,7 +3700,7 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
             const float* ffP = m->P;
             int ff_ld = L.n_up;
             if (par) { ffP = m->P + L.ff_off; ff_ld = L.n_in; }
-            const bool gated_epi = L.d.ff_kind == B200_FF_GATED_RELU && !par && out_norm && (few_in(L.w_up) || glu_takes(m, m->hn, L.w_up, W, R));
+            const bool gated_epi = L.d.ff_kind == B200_FF_GATED_RELU && !par && out_norm && (few_in(L.w_up) || glu_takes(m, m->hn, L.w_up, L.d.ff, W, R));
             if (gated_epi) project_in(nullptr, L.norm2, L.w_up, L.d.ff, m->act_a, L.d.ff, EPI_RELU_GLU);       // (the units in the product's epilogue)
             else if (!par) project_in(nullptr, L.norm2, L.w_up, L.n_up, m->P, L.n_up, EPI_STORE);
             const unsigned nb = (unsigned)(((size_t)R * L.d.ff + 255) / 256);

@@ -34,6 +34,23 @@ def test_products_at_tile_edges(b200, monkeypatch, rows, width, ff):
     assert np.median(d) < 1e-2 and (d < 4e-2).mean() > 0.9, (np.median(d), d.max())
 
 
+def test_refused_tensor_maps_take_the_cuda_core_products(b200, monkeypatch):
+    """Gated layers and experts included, whose units the tensor-core products make in their epilogues.  The refusal is the host's (B200_LP_TC_MAPS=0)."""
+    cfg = S.config([S.attn(heads=4, kv_heads=2, dim=16, mlp=S.dense(136)), S.latent(heads=3, dim=16, vdim=24, kv_rank=32, mlp=S.moe(ff=72))], width=72, vocab=264)
+    w = S.random_weights(cfg, 7)
+    toks = [int(t) for t in np.random.default_rng(1).integers(0, cfg["vocab"], 90)]
+    out = {}
+    for env in ("B200_LP_TC", "B200_LP_TC_MAPS"):
+        monkeypatch.setenv(env, "0")
+        gpu = S.gpu_model(cfg, w, "bfloat16", max_seq_len=96)
+        try:
+            out[env] = gpu.step([(0, toks)], list(range(90)))
+        finally:
+            gpu.close()
+            monkeypatch.delenv(env)
+    assert (out["B200_LP_TC"] == out["B200_LP_TC_MAPS"]).all()
+
+
 @pytest.mark.parametrize("kind", list(LAYERS))
 def test_programs_with_experts_add_in_the_order_of_k(b200, monkeypatch, kind):
     """32 rows at a width where K would be cut over clusters (B200_LP_TC_SPLIT=1): not in a program with experts, whose choices another order of the sums would turn in
