@@ -2011,13 +2011,14 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         }
         return cudaSuccess;
     };
-    // Which chunks: above 64 tokens all (two 8B layers, 80 / 333 / 2048 tokens: Q4_K_M 1160 -> 725, 1517 -> 993, 3635 -> 2635 us, Q6_K 1865 -> 822,
+    // Which chunks, layer by layer: above 64 tokens all (two 8B layers, 80 / 333 / 2048 tokens: Q4_K_M 1160 -> 725, 1517 -> 993, 3635 -> 2635 us, Q6_K 1865 -> 822,
     // 2420 -> 1092, 5873 -> 2730 us; two 2048-wide layers in Q8_0 699 -> 366, 931 -> 470, 1662 -> 1082 us), where the fused kernel's token tile
-    // doubles; down to 32 tokens too unless the wide matrices are Q4_K, whose fused unpacking costs less than the pass over fp16 rows (32 tokens:
+    // doubles; down to 32 tokens too unless the layer's wide matrices are Q4_K, whose fused unpacking costs less than the pass over fp16 rows (32 tokens:
     // Q4_K_M 551 against 674 us, Q6_K 783 against 772, Q8_0 380 against 331).  256 MB of rows at a time at most; a device without room for them
     // keeps the fused kernel.
-    const int f16_min = c->prompt_f16_min > 0 ? c->prompt_f16_min : c->layers[0].gate.type == T_Q4_K ? 65 : 32;
-    const bool f16_able = !rows && gemm_encode_fn() && std::min(cap, n) >= f16_min;
+    auto f16_min = [&](const Layer& L) { return c->prompt_f16_min > 0 ? c->prompt_f16_min : L.gate.type == T_Q4_K ? 65 : 32; };
+    bool f16_able = false;
+    for (const Layer& L : c->layers) f16_able |= !rows && gemm_encode_fn() && std::min(cap, n) >= f16_min(L);
     if (f16_able && !c->pf_w16) {
         const size_t want = std::max(std::min<size_t>((size_t)env_int("B200_PROMPT_F16_KROWS", 128 << 10) << 10, std::max((size_t)2 * I * H, (size_t)QKV * H)), (size_t)256 * std::max(std::max(I, H), A));
         if (cudaMalloc((void**)&c->pf_w16, want * sizeof(__half)) == cudaSuccess) c->pf_w16_elems = want;
@@ -2026,7 +2027,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             c->pf_w16 = nullptr;
         }
     }
-    bool f16 = false;             // (of the chunk)
+    bool f16 = false;             // (of the chunk and layer)
     auto product = [&](const DevTensor& w, int K, const __half* x, int ldx, int T, float* y, int ldy, const DevTensor* bias, int acc) -> cudaError_t {
         if (f16) {
             const cudaError_t e = gemm16({&w}, K, x, ldx, T, y, ldy, bias && bias->present() ? bias->f32() : nullptr, acc ? tc16::EPI_ADD : tc16::EPI_STORE);
@@ -2037,13 +2038,13 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     int last_T = 0;
     for (int done = 0; done < n; done += cap) {
         const int T = std::min(cap, n - done);
-        f16 = f16_able && c->pf_w16 && T >= f16_min;
         const int pos0 = (int)sl.host_pos + done;
         last_T = T;
         if (!use_graph) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
         CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T), dim3(256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)c->pf_tok, d.vocab, X));
         for (int l = 0; l < d.n_layers; l++) {
             Layer& L = c->layers[l];
+            f16 = f16_able && c->pf_w16 && T >= f16_min(L);
             float* kc = sl.kv + (size_t)l * kv_layer;
             float* vc = kc + kv_layer / 2;
             CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.attn_norm.f32(), d.norm_eps, XNh, H));

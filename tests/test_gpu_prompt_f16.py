@@ -45,3 +45,26 @@ def test_a_refused_tensor_map_takes_the_fused_products(b200, monkeypatch, preset
     fused = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="100000")
     refused = logits(b200, monkeypatch, desc, tensors, prompt, B200_PROMPT_F16_MIN="1", B200_PROMPT_F16_MAPS="0")
     assert (refused == fused).all()
+
+
+@pytest.mark.parametrize("first,second", [("Q4_K_M", "Q6_K"), ("Q6_K", "Q4_K_M")])
+def test_each_layer_goes_by_its_own_types(b200, monkeypatch, first, second):
+    """40 tokens through two layers, one of Q4_K (fused products up to 64 tokens) and one of Q6_K (two passes from 32 on), in either order: another number of
+    kernels than with either way for both layers."""
+    arch, desc, a = synth.synth_model("llama-tiny", first, 48, n_layers=2)
+    _, _, b = synth.synth_model("llama-tiny", second, 48, n_layers=2)
+    tensors = dict(a, **{k: v for k, v in b.items() if k.startswith("blk.1.")})
+    prompt = synth.prompt_tokens(40, desc["vocab"])
+    count = {}
+    for rule in ("0", "1", "100000"):
+        monkeypatch.setenv("B200_PROMPT_F16_MIN", rule)
+        gpu = b200.GpuOnlyInference(desc, tensors)
+        try:
+            gpu.prefill(prompt)
+            before = gpu.stats()["kernel_launches"]
+            gpu.reset()
+            gpu.prefill(prompt)
+            count[rule] = gpu.stats()["kernel_launches"] - before
+        finally:
+            gpu.close()
+    assert count["0"] not in (count["1"], count["100000"]), count
