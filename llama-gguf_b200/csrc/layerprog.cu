@@ -11,6 +11,7 @@
 // B200_COMPUTE_F32 keeps them in f32 and multiplies with FMA on the CUDA cores (no reduced-precision matrix mode).
 #include "layerprog.h"
 #include "ring.cuh"
+#include "soft_cap.cuh"
 #include "spare.cuh"
 
 #include <cuda.h>

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
         if (lane == 0) tc_arrive(q_full);
         const float L2E = 1.4426950408889634f;
         const bool capped = a.softcap > 0.0f;
-        const float sl = a.scale * L2E, cap_in = capped ? 2.0f * L2E / a.softcap * a.scale : 0.0f, cap_out = a.softcap * L2E, slope = attn_slope(a, h) * L2E;
+        const float sl = a.scale * L2E, cap_in = capped ? a.scale / a.softcap : 0.0f, cap_out = a.softcap * L2E, slope = attn_slope(a, h) * L2E;
         const int lo_i = attn_lo(a, i);
         float m = -INFINITY, l = 0.0f;
         {   // the extra term of the denominator
@@ -281,8 +281,19 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
                 }
             }
             if (capped) {
+                float big = 0.0f;
 #pragma unroll
-                for (int e = 0; e < KA_K; e++) s[e] = soft_cap_exp(s[e], cap_in, cap_out);
+                for (int e = 0; e < KA_K; e++) {
+                    s[e] *= cap_in;
+                    big = fmaxf(big, fabsf(s[e]));
+                }
+                if (!__any_sync(0xffffffffu, big >= SOFT_CAP_SMALL)) {
+#pragma unroll
+                    for (int e = 0; e < KA_K; e++) s[e] = cap_out * tanh_small(s[e]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < KA_K; e++) s[e] = fabsf(s[e]) < SOFT_CAP_SMALL ? cap_out * tanh_small(s[e]) : soft_cap_exp(s[e], 2.0f * L2E, cap_out);
+                }
             } else {
 #pragma unroll
                 for (int e = 0; e < KA_K; e++) s[e] *= sl;
