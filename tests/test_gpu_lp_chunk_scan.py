@@ -16,7 +16,7 @@ def both(monkeypatch, S, cfg, lens, more):
     rng = np.random.default_rng(sum(lens))
     runs = [(i, [int(t) for t in rng.integers(0, cfg["vocab"], n)]) for i, n in enumerate(lens)]
     cont = [int(t) for t in rng.integers(0, cfg["vocab"], more)]
-    outs = {}
+    outs, launches = {}, {}
     for on in ("1", "0"):
         monkeypatch.setenv("B200_LP_CHUNK_SCAN", on)
         gpu = S.gpu_model(cfg, w, "float32", max_seq_len=max(lens) + more + 8)
@@ -25,8 +25,10 @@ def both(monkeypatch, S, cfg, lens, more):
             second = gpu.step([(0, cont)], list(range(more)))
             last = gpu.step([(0, cont[:1])], [0])
             outs[on] = np.concatenate([first, second, last])
+            launches[on] = gpu.stats()["kernel_launches"]
         finally:
             gpu.close()
+    assert launches["1"] == launches["0"] + 2, launches        # both prompts went in chunks: two kernels for one, in the only scan of the model
     assert S.rel_err(outs["1"], outs["0"]) < 2e-4
 
 
@@ -40,7 +42,7 @@ def test_delta_rule_and_matrix_memory(b200, monkeypatch, layer, lens, more):
     both(monkeypatch, LS, LS.config([layer], width=64, vocab=80), lens, more)
 
 
-@pytest.mark.parametrize("lens,more", [((48, 1, 33), 65), ((129, 96, 32), 50), ((300,), 61)])
+@pytest.mark.parametrize("lens,more", [((129, 1, 96), 160), ((128, 31), 129), ((300,), 133)])
 @pytest.mark.parametrize("sizes", [dict(heads=4, vdim=8, state=16, groups=2, conv=4), dict(heads=2, vdim=128, state=128, groups=1, conv=4), dict(heads=4, vdim=20, state=72, groups=1, conv=3)])
 def test_state_space(b200, monkeypatch, sizes, lens, more):
     both(monkeypatch, MS, MS.config([MS.scan(**sizes)]), lens, more)

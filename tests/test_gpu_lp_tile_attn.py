@@ -9,6 +9,8 @@ import pytest
 
 import gefovik_synth as GS
 import lazilorn_synth as S
+import marosun_synth as MA
+import mefurax_synth as ME
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +76,42 @@ def test_one_tile_of_keys_per_run_keeps_the_mma_kernels(b200, monkeypatch, lens,
         finally:
             gpu.close()
     assert (outs["1024"] == outs["0"]).all() == same
+
+
+FORMS = {   # (synth module, layer, added to the learned extra terms of the denominator)
+    "slope_window": (ME, ME.layer_a(heads=4, kv_heads=2, dim=64, vdim=72, window=200, scale=0.125), 0.0),
+    "softcap_chunks_head_gate": (ME, ME.layer_b(heads=4, kv_heads=2, dim=64, vdim=64, chunk=100, softcap=5.0, scale=0.125), 0.0),
+    "softcap_bites": (ME, ME.layer_b(heads=4, kv_heads=1, dim=128, vdim=128, chunk=300, softcap=1.5, scale=0.2), 0.0),
+    "turned_values_sink": (MA, MA.layer_a(heads=4, kv_heads=2, dim=64, vdim=64), 0.0),
+    "sink_above_all": (MA, MA.layer_a(heads=4, kv_heads=2, dim=64, vdim=64), 25.0),
+    "sink_below_all": (MA, MA.layer_a(heads=3, kv_heads=1, dim=48, vdim=80), -60.0),
+    "channel_gate_chunks_sink": (MA, MA.layer_p(heads=4, kv_heads=2, dim=64, vdim=40, chunk=100, right_scale=0.0), 0.0),
+    "one_in_the_denominator": (MA, MA.layer_q(heads=4, kv_heads=2, dim=32, vdim=64), 0.0),
+    "values_from_unit_keys": (GS, GS.attn(heads=6, kv_heads=2, dim=128, scale=0.25, softcap=50.0), 0.0),
+    "values_from_unit_keys_capped": (GS, GS.attn(heads=4, kv_heads=4, dim=64, scale=0.25, softcap=2.0), 0.0),
+    "latent_sink_above": (GS, GS.latent(heads=3, dim=16, vdim=24, kv_rank=128), 20.0),
+    "latent_sink_below": (GS, GS.latent(heads=5, dim=48, vdim=64, kv_rank=64), -60.0),
+}
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+def test_every_form_against_the_warp_kernel(b200, monkeypatch, form):
+    """What a score goes through besides the products, over several tiles of keys and a portion that continues them: row by row, the bound of bf16 queries, keys and
+    probabilities (scores of a few units: 2^-8 of them in a probability, halved by the average over the keys; four times that)."""
+    M, layer, shift = FORMS[form]
+    cfg = M.config([layer], width=64, vocab=80)
+    w = M.random_weights(cfg, 5)
+    for k in w:
+        if k.endswith("sink"):
+            w[k] = (w[k] + shift).astype(np.float32)
+    rng = np.random.default_rng(3)
+    a, b, more = ([int(t) for t in rng.integers(0, cfg["vocab"], n)] for n in (300, 131, 97))
+    outs = {}
+    for tile in ("1", "0"):
+        monkeypatch.setenv("B200_LP_ATTN_TILE", tile)
+        gpu = M.gpu_model(cfg, w, "bfloat16", max_seq_len=512)
+        try:
+            outs[tile] = np.concatenate([gpu.step([(0, a), (1, b)], list(range(len(a) + len(b)))), gpu.step([(1, more[:1]), (0, more)], list(range(1 + len(more))))])
+        finally:
+            gpu.close()
+    assert GS.rel_err(outs["1"], outs["0"]) < 2e-2
