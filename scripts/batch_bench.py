@@ -1,4 +1,4 @@
-"""Batched decode (BASELINE configs[2]: Llama-3-8B Q4_K_M, batch 32): tokens/s of b200_decode_batch through the tcgen05
+"""Batched decode (Llama-3-8B Q4_K_M, batch 32): tokens/s of b200_decode_batch through the tcgen05
 dequant-GEMM pass against the same 32 sequences decoded one after the other.  usage: python scripts/batch_bench.py [B] [steps]"""
 import os, sys, time, json
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))

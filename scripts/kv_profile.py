@@ -1,11 +1,11 @@
-"""Decode attention at depth, f32 KV cache vs INT8 KV cache (SURVEY §8f row 4), same per-op decode path for both
+"""Decode attention at depth, f32 KV cache vs INT8 KV cache, same per-op decode path for both
 (B200_MEGA=0 for the f32 context so that the two attention kernels are the only difference):
 
     python scripts/kv_profile.py --kv-format int8 --depth 8000 --tokens 3
 
 The KV cache is taken as valid up to --depth as it is (b200_debug_set_position: zero rows -- the kernels' work does not depend on
 the values), then --tokens greedy tokens are decoded; prints one JSON line with ms/token (CUDA events).  Run it under
-`ncu -k regex:attn --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum` for the per-kernel numbers."""
+`ncu --clock-control none -k regex:attn --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum` for the per-kernel numbers."""
 import argparse
 import json
 import os

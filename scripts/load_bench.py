@@ -1,14 +1,14 @@
-"""GGUF -> HBM load time (SURVEY §8f row 2): a random-init GGUF of a named architecture is written to local disk, then loaded
+"""GGUF -> HBM load time: a random-init GGUF of a named architecture is written to local disk, then loaded
 into a finalized context by every path the package has, wall clock from the path to a context that can decode:
 
   native            b200_ctx_create_from_gguf: mmap + parse + pinned double-buffered upload inside the library (csrc/gguf_load.cuh)
   native_1thread    the same with one host thread filling the staging buffers
   native_8threads   ... with eight
   native_unstaged   cudaMemcpy straight from the mapping (pageable memory: the driver stages it itself)
-  python_shim       round 1's path: gguf-py reader -> numpy arrays -> b200_ctx_upload_tensor per tensor (gguf_io.load_gguf)
+  python_shim       the path through Python: gguf-py reader -> numpy arrays -> b200_ctx_upload_tensor per tensor (gguf_io.load_gguf)
 
 Every context decodes the same 4-token prompt and the logits must agree bit for bit.  One JSON line on stdout.
-Usage (GPU box): python scripts/load_bench.py [--model llama-3-8b] [--mix Q4_K_M] [--dir /tmp]
+Usage: python scripts/load_bench.py [--model llama-3-8b] [--mix Q4_K_M] [--dir /tmp]
 """
 import argparse
 import json

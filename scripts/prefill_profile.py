@@ -1,5 +1,5 @@
 """One GEMM prefill of N tokens on a 2-layer model with Llama-3-8B shapes (random GGUF blocks): run under
-`ncu --metrics gpu__time_duration.sum` for the per-kernel times.  usage: python scripts/prefill_profile.py [N] [mix]"""
+`ncu --clock-control none --metrics gpu__time_duration.sum` for the per-kernel times.  usage: python scripts/prefill_profile.py [N] [mix]"""
 import os, sys
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)

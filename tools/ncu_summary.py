@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Summarise an .ncu-rep: headline metrics per launch (raw page only).
-usage: python tools/ncu_summary.py gpurun_out/x.ncu-rep"""
+usage: python tools/ncu_summary.py x.ncu-rep"""
 import csv, subprocess, sys, io
 
 rep = sys.argv[1]
