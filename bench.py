@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py — decode tok/s of the quantized-forward hot path (BASELINE.json metric).
+"""bench.py — decode tok/s of the quantized-forward hot path.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
 
@@ -53,7 +53,7 @@ def measured_peaks():
 
 
 class ClockSampler:
-    """Samples nvidia-smi clocks / throttle reasons during the timed region (B200_PROFILING.md)."""
+    """Samples nvidia-smi clocks / throttle reasons during the timed region."""
 
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
@@ -191,7 +191,7 @@ def main():
     ap.add_argument("--seed", type=int, default=1236)
     ap.add_argument("--no-speculation", action="store_true", help="e2e: only the plain b200_forward loop (no greedy continuation)")
     ap.add_argument("--kv-format", default=os.environ.get("B200_KV_FORMAT", "f32"), choices=["f32", "int8"],
-                    help="KV cache storage (SURVEY 8f row 4): int8 = QuantizedKVCache Int8 rows + one scale per row (per-op decode path)")
+                    help="KV cache storage: int8 = QuantizedKVCache Int8 rows + one scale per row (per-op decode path)")
     ap.add_argument("--design", default=None, choices=["lazilorn", "mefurax", "madudra", "marosun", "fizesun", "gefovik"],
                     help="instead of the default workload: prefill / decode throughput of this layer-program design at a few sizes, "
                          "beside a llama-architecture model of the same size (bench_layers.py)")
@@ -358,7 +358,7 @@ def main():
                     "whole_token_frac": token_bytes / (ms_per_step * 1e-3) / 1e9 / peaks["hbm_gbs"],
                     "frac_of_nominal_8TBs": achieved / 8000.0}
 
-    # ---- extras: BASELINE configs[2] also names an 8K context and batch 32 ----
+    # ---- extras: an 8K context and batch 32 ----
     extras = {}
     if args.depth > 0 and args.depth + args.steps + args.warmup + 8 <= args.ctx:
         try:
@@ -436,7 +436,7 @@ def main():
             extras.setdefault("decode_batch", {"error": str(e)})
             extras["batch_error"] = str(e)
 
-    # ---- prefill: the whole prompt through the batch entry point (tcgen05 dequant-GEMM, csrc/gemm_umma.cuh) ----
+    # ---- prefill: the whole prompt through the batch entry point (weights to fp16 rows once per chunk, tcgen05 products: csrc/prompt_f16.cuh) ----
     prefill = None
     if args.prefill_len > 0 and args.prefill_len <= args.ctx:
         try:
@@ -456,7 +456,7 @@ def main():
             prefill = {"tokens": args.prefill_len, "seconds": pf_s, "tok_per_s": args.prefill_len / pf_s,
                        "gemm_tflops": tfl, "tensor_peak_tflops": peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops")),
                        "tensor_frac": tfl / peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops")),
-                       "path": "b200_prefill: 2048-token chunks, tcgen05.mma kind::f16 dequant-GEMM + batched RoPE/attention/SwiGLU, "
+                       "path": "b200_prefill: 2048-token chunks, weights to fp16 rows, tcgen05.mma kind::f16 products (SwiGLU in the epilogue), batched RoPE, tcgen05 attention, "
                                "host tokens in, logits of the last token out (wall clock)",
                        "token_by_token_tok_per_s": 1000.0 / ms_per_step}
         except Exception as e:

@@ -1,6 +1,6 @@
 /* llama_b200.h — C ABI of the `cuda-b200` backend for Lexmata/llama-gguf.
  *
- * This is the drop-in boundary: a Rust shim (INTEGRATION.md) binds these symbols
+ * This is the drop-in boundary: a Rust shim binds these symbols
  * with `extern "C"` and implements the crate's `GpuInference` trait
  * (src/backend/mod.rs:283-296) and `Backend` trait (src/backend/mod.rs:29-265)
  * on top of them.  Plain pointers and sizes only; every host pointer is read or
@@ -103,7 +103,7 @@ B200_API int b200_ctx_upload_tensor(b200_ctx* ctx, const char* gguf_name, uint32
 B200_API int b200_ctx_finalize(b200_ctx* ctx);
 B200_API void b200_ctx_destroy(b200_ctx* ctx);
 
-/* KV cache storage format (SURVEY 8f row 4; KVCacheFormat, src/model/kv_quantized.rs:11-20), chosen between b200_ctx_create and
+/* KV cache storage format (KVCacheFormat, src/model/kv_quantized.rs:11-20), chosen between b200_ctx_create and
  * b200_ctx_finalize (or with B200_KV_FORMAT=int8 in the environment): 0 = F32 (the KVCache of src/model/mod.rs:83-108, default),
  * 1 = Int8 -- QuantizedKVCache::write_kv / read_k_range semantics (kv_quantized.rs:143-216, 230-270, 366-392): one symmetric
  * scale = max|x| / 127 per (kv head, position) row, q = round(x / scale), attention over q * scale.  A quarter of the KV bytes; the
@@ -112,7 +112,7 @@ B200_API void b200_ctx_destroy(b200_ctx* ctx);
 B200_API int b200_ctx_set_kv_format(b200_ctx* ctx, int format);
 B200_API int b200_ctx_kv_format(b200_ctx* ctx, int* out);
 
-/* GGUF -> HBM direct load (SURVEY 8f row 2).  Replaces GgufFile::open (src/gguf/mod.rs:23-40, mmap), GgufReader::read
+/* GGUF -> HBM direct load.  Replaces GgufFile::open (src/gguf/mod.rs:23-40, mmap), GgufReader::read
  * (src/gguf/reader.rs:28-110: header, metadata, tensor infos, aligned data offset; versions 1-3), ModelLoader::parse_config
  * (src/model/loader.rs:62-300: the {arch}.* keys with the same defaults and the same strict typed getters, gguf/types.rs:78-97)
  * and the per-tensor Vec copy + upload of loader.rs:1341-1365 / cuda/gpu_only.rs:426-520: the file is mapped once, parsed in
@@ -146,7 +146,7 @@ B200_API int b200_ctx_load_gguf(b200_ctx* ctx, b200_gguf* file, b200_load_stats*
 B200_API int b200_ctx_create_from_gguf(const char* path, const b200_parallel_desc* par /* NULL = 1 GPU, device 0 */, int max_seq_len,
                                        int max_batch, int kv_format, b200_ctx** out, b200_load_stats* stats /* may be NULL */);
 
-/* Tensor parallel (SURVEY 8e; replaces the gRPC all-reduce-via-rank-0 of
+/* Tensor parallel (replaces the gRPC all-reduce-via-rank-0 of
  * src/distributed/tensor_parallel_distributed.rs:135-187): one context per rank/GPU, created with
  * world_size/rank in b200_parallel_desc.  Between b200_ctx_create and b200_ctx_finalize every rank calls
  * b200_ctx_tp_handle (a 64-byte CUDA IPC handle of its exchange region), the host passes the handles around
@@ -156,7 +156,7 @@ B200_API int b200_ctx_create_from_gguf(const char* path, const b200_parallel_des
 B200_API int b200_ctx_tp_handle(b200_ctx* ctx, void* handle_out64);
 B200_API int b200_ctx_tp_set_peer(b200_ctx* ctx, int peer_rank, const void* handle64);
 
-/* Single-process tensor / expert parallelism (SURVEY 8b: "TP ranks are threads inside the library; callers never see ranks";
+/* Single-process tensor / expert parallelism ("TP ranks are threads inside the library; callers never see ranks";
  * TensorParallel trait, src/backend/tensor_parallel.rs:13-32).  A group owns one context per device and one host thread per context;
  * peers are connected with cudaDeviceEnablePeerAccess (no IPC handles, no other process).  Dense models are tensor parallel
  * (ShardingPlan::from_config, tensor_parallel.rs:69-106), MoE models expert parallel.  Every call below fans out to the ranks and
@@ -187,7 +187,7 @@ B200_API int b200_prefill_token(b200_ctx* ctx, int seq, uint32_t token);
 /* GpuOnlyInference::forward_batch (gpu_only.rs:776-790): n tokens of ONE
  * sequence; logits of the last one (logits_out may be NULL). */
 B200_API int b200_prefill(b200_ctx* ctx, int seq, const uint32_t* tokens, int n, float* logits_out);
-/* One token for each of n DISTINCT sequence slots (SURVEY §8f row 1);
+/* One token for each of n DISTINCT sequence slots;
  * logits_out is n x vocab. */
 B200_API int b200_decode_batch(b200_ctx* ctx, const int* seqs, const uint32_t* tokens, int n, float* logits_out);
 /* Greedy continuation behind b200_forward (opt-in, after finalize; one GPU, megakernel paths).  When on, b200_forward also picks
@@ -204,7 +204,7 @@ B200_API int b200_ctx_speculation_stats(b200_ctx* ctx, int* enabled, uint64_t* h
  * ids instead of n x vocab logits. */
 B200_API int b200_decode_batch_greedy(b200_ctx* ctx, const int* seqs, const uint32_t* tokens, int n, uint32_t* next_out);
 
-/* Continuous batching (SURVEY 8f row 1): the peer of BatchedEngine (src/engine_batched.rs) below the tokenizer and the channels.
+/* Continuous batching: the peer of BatchedEngine (src/engine_batched.rs) below the tokenizer and the channels.
  * Requests become sequences that each own one KV slot of the context; b200_batch_step is one iteration of the reference's
  * background loop (engine_batched.rs:199-320) with step_sequence's rules (:366-411) -- the whole prompt on a sequence's first
  * step, one token per step after that, finished when the last token is EOS or max_tokens were generated, EOS itself is not
@@ -490,7 +490,7 @@ B200_API int b200_ctx_pool_counts(b200_ctx* ctx, int* live, int* pooled);
 B200_API int b200_reset(b200_ctx* ctx, int seq);
 B200_API int b200_position(b200_ctx* ctx, int seq, uint64_t* out);
 
-/* Device-resident greedy decode (SURVEY §8f row 3: sampling on device).
+/* Device-resident greedy decode (sampling on device).
  * Runs n_steps tokens starting from `first_token`, argmax (last max wins,
  * src/main.rs:1816-1821) on the GPU, no host round trip between tokens.
  * tokens_out (n_steps, may be NULL) receives the generated ids; elapsed_ms

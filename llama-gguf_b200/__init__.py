@@ -2,7 +2,7 @@
 
 The product is `libllama_b200.so` (C ABI: include/llama_b200.h, sources in csrc/).
 The reference's host language is Rust, which this image cannot compile, so the
-classes below play the role of the Rust shim of INTEGRATION.md: same names,
+classes below play the role of a Rust shim: same names,
 argument meaning and error behaviour as
 
   * `Backend`            -> CudaB200Backend   (src/backend/mod.rs:29-265)
@@ -992,7 +992,7 @@ class LayerProgramInference(GpuOnlyInference):
 
 class GroupInference:
     """GpuInference over the GPUs of ONE process (b200_group_*): tensor parallel for dense models, expert parallel for MoE models,
-    one host thread per device inside the library -- the caller never sees ranks (SURVEY §8b; TensorParallel trait,
+    one host thread per device inside the library -- the caller never sees ranks (TensorParallel trait,
     src/backend/tensor_parallel.rs:13-32).  Same surface as GpuOnlyInference: forward() returns the full logits row."""
 
     @classmethod

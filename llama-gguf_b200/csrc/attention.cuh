@@ -16,7 +16,7 @@
 // CTA to arrive for a kv head (atomic ticket) does the final merge in a fixed order, so
 // results are run-to-run deterministic.
 //
-// Deviation (documented in DESIGN.md): the reference skips value rows whose probability
+// Deviation: the reference skips value rows whose probability
 // is <= 1e-8 (cpu/ops.rs:1529); this kernel includes them.  The dropped mass is at most
 // kv_len * 1e-8 of the output — far below the 1e-3 parity tolerance.
 #pragma once

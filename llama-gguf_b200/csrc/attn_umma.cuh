@@ -16,9 +16,10 @@
 // average with heavy cancellation, so single-fp16 operands put 2^-12 of relative noise on it — measured: the logits of a 300-token prompt
 // moved from 6e-4 to 1.1e-3 of the oracle's.
 // Roles: 8 softmax warps, a loader thread (two stages of K and of V^T), an MMA thread that issues the next tile's scores before it waits for this
-// tile's probabilities.  What bounds it: 6 x 256 clocks of tensor pipe per tile (M = 128, N = 64, K = hd and back), under which the exponentials run;
-// the kernel before made two passes over the keys (maximum and sum, then values) with copy, product and exponentials one after the other: 12000
-// clocks per tile, 358 us per layer of 2048 tokens (32 heads over 8) against 157 us now (one tile at a time through load, maximum, exponentials and store: 5300 clocks).
+// tile's probabilities.  What bounds it: the serial chain of a tile -- TMEM load, the two halves' maximum, exponentials, store of P (one buffer, which the products of the tile
+// before must have left) -- with one CTA per SM to hide it: 5300 clocks per tile, 1536 of them tensor pipe (6 x 256: M = 128, N = 64, K = hd and back, 29 %
+// busy).  The kernel before made two passes over the keys (maximum and sum, then values): 12000 clocks per tile, 358 us per layer of 2048 tokens (32 heads
+// over 8) against 157 us now.
 // f32 scores / softmax / accumulation.  Every wait is bounded and reports through p.err.
 #pragma once
 #include <cuda.h>

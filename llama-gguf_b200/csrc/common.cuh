@@ -89,7 +89,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // x-vector layout in shared memory: 4 floats of padding after every 64, which makes the
-// float4 reads of the Q4_K/Q5_K lane mapping conflict-free (DESIGN.md §gemv).
+// float4 reads of the Q4_K/Q5_K lane mapping conflict-free.
 __host__ __device__ __forceinline__ int xidx(int e) { return e + ((e >> 6) << 2); }
 __host__ __device__ __forceinline__ int xpad_floats(int k) { return k + ((k + 63) >> 6) * 4 + 4; }
 

@@ -321,7 +321,7 @@ extern "C" int b200_ctx_create(const b200_model_desc* desc, const b200_parallel_
         if (P != 2 && P != 4 && P != 8) return bad("tensor-parallel world size must be 2, 4 or 8");
         if (d.n_experts > 0) {
             // MoE: EXPERT parallel -- attention, norms, router and the vocab head replicated, expert e on rank e / (E / P); at batch 1 the
-            // dispatch is free (every rank routes), the combine is the only exchange (SURVEY 8e; replaces moe.rs:352-361 on one host)
+            // dispatch is free (every rank routes), the combine is the only exchange (replaces moe.rs:352-361 on one host)
             if (d.n_experts % P) return bad("n_experts must be divisible by the world size");
             c->ep = true;
             c->ep_local = d.n_experts / P;
@@ -1773,7 +1773,7 @@ static cudaError_t gemm_dispatch(UmmaParams& p, int n_sm, cudaStream_t st, uint6
         if (launches) *launches += (p.k_split && !p.tile_cnt) ? 2 : 1;
         return umma2_launch(gemm_encode_fn(), p, n_sm, 227 * 1024 - 2048, st, ng);
     }
-    if (p.T > env_int("B200_GEMM_TMA_MAX_T", 64)) p.tmap = nullptr;   // first kernel: large tiles keep the direct reads (measured, round 1)
+    if (p.T > env_int("B200_GEMM_TMA_MAX_T", 64)) p.tmap = nullptr;   // first kernel: large tiles keep the direct reads (measured)
     p.tile_cnt = nullptr;                                             // first kernel: separate reduce kernel
     if (launches) *launches += p.k_split ? 2 : 1;
     return umma_launch(p, st);
@@ -3043,7 +3043,7 @@ extern "C" int b200_op_vec_mat(const float* a, const float* w, float* out, size_
 // Backend extension for prefill / batched decode: T input rows at once through the tcgen05 dequant-GEMM
 // (csrc/gemm_umma.cuh).  out[t][j] = sum_k a[t][k] * deq(W)[j][k]: the same contraction as T calls of vec_mat_q, fp16
 // operands with f32 accumulation (documented tolerance 2e-3 of the largest output).
-// Backend::matmul / matvec / matvec_q (src/backend/mod.rs:90, 93, 107): required trait methods that the model code never calls (SURVEY 8b)
+// Backend::matmul / matvec / matvec_q (src/backend/mod.rs:90, 93, 107): required trait methods that the model code never calls
 extern "C" int b200_op_matmul(const float* a, const float* b, float* out, size_t m, size_t k, size_t n) {
     int rc;
     if ((rc = op_ready())) return rc;
@@ -3275,7 +3275,7 @@ extern "C" int b200_op_attention(const float* q, const float* k, const float* v,
     return B200_OK;
 }
 
-// ------------------------------------------------------------------ GGUF -> HBM direct load (gguf_load.cuh; SURVEY 8f row 2)
+// ------------------------------------------------------------------ GGUF -> HBM direct load (gguf_load.cuh)
 extern "C" int b200_gguf_open(const char* path, b200_gguf** out) {
     if (!path || !out) return fail(B200_ERR_INVALID_ARGUMENT, "b200_gguf_open: null argument");
     *out = nullptr;
@@ -3929,7 +3929,7 @@ extern "C" int b200_debug_set_position(b200_ctx* c, int seq, uint64_t pos) {
 }
 
 // Host logic of the split-K planners, callable without a device (tests): K range per split (0 = unsplit) for an n_rows x K matrix at
-// T token rows on n_sm SMs; persistent = the cost model of gemm_umma2.cuh's kernel, else round 1's rule.
+// T token rows on n_sm SMs; persistent = the cost model of gemm_umma2.cuh's kernel, else that of gemm_umma.cuh.
 extern "C" int b200_debug_plan_split(int n_rows, int K, int T, int n_sm, int persistent, int* k_split_out) {
     if (!k_split_out || n_rows <= 0 || K <= 0 || K % 256 || T <= 0 || n_sm <= 0) return fail(B200_ERR_INVALID_ARGUMENT, "b200_debug_plan_split: bad argument");
     UmmaParams p{};

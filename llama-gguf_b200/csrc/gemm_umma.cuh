@@ -20,9 +20,9 @@
 //   * epilogue: warp w reads TMEM lanes 32w..32w+31 with tcgen05.ld.32x32b.x32, thread = weight row, 32
 //     tokens per load, and stores Y so that a warp writes 32 consecutive floats of one token's row.
 // fp16 operands, f32 accumulation: measured 3e-4 of the largest output against a double-precision dequant-then-dot
-// (tools/umma_lab.cu); the exact token-by-token path stays the default where bit-level greedy parity matters.
+// (N(0, 1) blocks of every type); the exact token-by-token path stays the default where bit-level greedy parity matters.
 // Two stages: the MMAs of step k overlap the dequant of step k + 1; the dequant (CUDA cores), not the tensor pipe, is the
-// limit (see DESIGN.md §3.6).
+// limit.
 #pragma once
 #include "common.cuh"
 #include "quant.cuh"

@@ -1,9 +1,9 @@
-// gemm_umma2.cuh — warp-specialised, persistent tcgen05 / TMEM dequant-GEMM (round 2): same contract as gemm_umma.cuh
+// gemm_umma2.cuh — warp-specialised, persistent tcgen05 / TMEM dequant-GEMM: same contract as gemm_umma.cuh
 //
 //   Y[t][j] (+)= sum_k deq(W)[j][k] * X[t][k] (+ bias[j]),   W = N rows of GGUF blocks (Q4_K / Q5_K / Q6_K / Q8_0), X fp16,
 //
 // (the contraction the reference runs as T GEMVs per matrix: src/model/llama.rs:327-345, src/backend/cuda/gpu_only.rs:776-790;
-// block arithmetic: src/tensor/quant/dequant.rs:103-109, 205-356), rebuilt around round 1's measurement that the first kernel
+// block arithmetic: src/tensor/quant/dequant.rs:103-109, 205-356), rebuilt around the measurement that the first kernel
 // (128 threads that all dequantise, then all wait for one thread's MMAs) keeps the tensor pipe 10 % busy and streams the
 // weights of a 32-row pass at 370 GB/s.  One persistent CTA per SM walks a list of (128 weight rows, TN tokens, K range)
 // items; its warps have fixed roles and meet only through mbarriers — there is no CTA-wide barrier in the loop:
@@ -40,7 +40,7 @@ struct Umma2Plan {
     int raw_stage;           // bytes per raw stage (128 rows x raw_pitch, rounded up to 128)
     int off_b, off_raw;      // byte offsets of the B and raw rings from the 1024-aligned base (A ring at 0)
     int x3d;                 // activations through the 3-D tensor map (1) or the 2-D fallback {K, T} (0: one load per 64-element slab)
-    int dbg;                 // lab only (tools/gemm_lab): 1 = no dequant math, 2 = no raw loads, 4 = no activation loads, 8 = no MMAs,
+    int dbg;                 // measurements only: 1 = no dequant math, 2 = no raw loads, 4 = no activation loads, 8 = no MMAs,
                              // 64 = no tcgen05.fence in the MMA loop, 128 = plain mbarrier arrives instead of tcgen05.commit (timing only)
     long long* prof;         // lab only: per CTA and role {clocks in the role loop, clocks spent waiting}
 };

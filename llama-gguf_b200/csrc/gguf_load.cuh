@@ -1,4 +1,4 @@
-// gguf_load.cuh — GGUF -> HBM direct load (SURVEY §8f row 2), host code only.
+// gguf_load.cuh — GGUF -> HBM direct load, host code only.
 //
 // What it replaces: GgufFile::open (src/gguf/mod.rs:23-40: mmap), GgufReader::read (src/gguf/reader.rs:28-110: header, metadata,
 // tensor infos, aligned data offset), ModelLoader::parse_config (src/model/loader.rs:62-300: the {arch}.* keys and their defaults)

@@ -1,4 +1,4 @@
-// kv_int8.cuh — INT8 KV cache (SURVEY §8f row 4): the reference's QuantizedKVCache in its Int8 format
+// kv_int8.cuh — INT8 KV cache: the reference's QuantizedKVCache in its Int8 format
 // (src/model/kv_quantized.rs:11-20, 143-216 write_kv, 230-270 read_k_range, 366-392 quantize_int8 / dequantize_int8) kept in
 // HBM as the bytes + one f32 scale per (kv head, position), and a GQA decode attention that reads it.
 //

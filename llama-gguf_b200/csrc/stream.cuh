@@ -1,7 +1,7 @@
 // stream.cuh — the streamed per-token megakernel: one persistent CTA per SM whose PRODUCER warp never stops pulling
 // weights from HBM while the consumer warps walk the phases of the token.
 //
-// Why (profiles/v1_mega_ncu_full.md, per-phase timeline): in the first megakernel (mega.cuh) every GEMV phase
+// Why (per-phase timeline): in the first megakernel (mega.cuh) every GEMV phase
 // pays ~5 us of fixed cost (grid barrier, x staging, ring ramp-up, stragglers) against 1.5-10 us of streaming, and
 // HBM idles during all of it: 29 % of the copy roofline for a whole token.  Weights never depend on the token, so
 // here they are fetched by a warp that is not part of any phase:
@@ -53,7 +53,7 @@ struct StreamParams {
 // Chunks (256 elements) per ring entry a type would like; a phase uses the minimum over its matrices.
 inline int stream_pref_chunks(int type) { return type == T_Q4_K ? 2 : 1; }
 // Inner box of the tensor map = row pitch of a ring entry.  The box must start on a 16-byte boundary of the row
-// (tools/tma_lab.cu: an unaligned start is an illegal instruction), so an entry that starts at byte b of its row is
+// (an unaligned start is an illegal instruction), so an entry that starts at byte b of its row is
 // fetched from b & ~15 and the consumer skips b & 15 bytes: the pitch covers the largest such residue.
 // Q4_K 288 (C = 2) / 144, Q5_K 176, Q6_K 210 + 14 = 224, Q8_0 272.
 inline int stream_pitch(int type, int C) {

@@ -1,7 +1,7 @@
-// stream2.cuh — second streamed per-token megakernel: the round-2 decode path.
+// stream2.cuh — second streamed per-token megakernel: the decode path.
 //
-// Round 1 (stream.cuh) moved exactly the algorithmic bytes but left HBM idle two thirds of the time
-// (profiles/v1_stream_ncu_full.md): ~4 us of fixed cost per phase (CTA-wide barriers around the grid
+// The first one (stream.cuh) moves exactly the algorithmic bytes but leaves HBM idle two thirds of the time
+// (ncu and per-phase timelines): ~4 us of fixed cost per phase (CTA-wide barriers around the grid
 // barrier, the staged-x copy, merge + epilogue), whole 32-row tiles per CTA (448 gate/up tiles on 148 CTAs: the four heavy
 // CTAs finish 4.4 us late; 128 O / down tiles leave 20 CTAs idle), 7 consumer warps at 255 registers (1.75 warps per
 // scheduler) and 15.6 us of attention per layer behind six dependent global round trips.  This kernel keeps the idea
@@ -46,7 +46,7 @@ namespace b200 {
 constexpr int kS2Cons = B200_S2_CONS;             // consumer warps (14 at 128 registers; 12: warpgroups 0-2 take kS2ConsRegs registers with setmaxnreg)
 constexpr int kS2NT = kS2Cons * 32;               // consumer threads
 // + the service warpgroup: loader warp, producer warp, two idle warps.  8 consumers: 256 x 200 + 128 x 96 = 63488 registers
-// (round 1's fully unrolled unit kernels: few fat warps); 12: 384 x 144 + 128 x 72 = 64512; 14: no setmaxnreg, 128 each
+// (fully unrolled unit kernels: few fat warps); 12: 384 x 144 + 128 x 72 = 64512; 14: no setmaxnreg, 128 each
 constexpr int kS2Threads = kS2Cons == 8 ? 384 : 512;
 // producer warps (the rest of the service warpgroup).  n_slots must be a multiple of it as well: a slot is then always filled by the
 // same producer, in order, so its wait on `empty` by phase parity can never see a stale phase
@@ -103,7 +103,7 @@ __device__ __forceinline__ void pdesc2_load(PDesc2& d, const MegaPhase* P) {
 
 // One issuing thread is latency-bound: a try_wait that succeeds at once, expect_tx, the operand moves to uniform registers and the
 // TMA issue take ~400 clocks per entry (measured: producer stamps of b200_debug_mega_phase), i.e. 23 B/clk for a 9 KB entry --
-// the HBM rate per SM with no slack, and the reason round 1's gate/up phase never went below 19 us.  So the ring is fed by
+// the HBM rate per SM with no slack, and the reason the gate/up phase of stream.cuh never went below 19 us.  So the ring is fed by
 // kS2Prods producer warps; producer `pidx` issues the entries whose global sequence number is pidx modulo kS2Prods (the slot of
 // an entry is its sequence number modulo n_slots, whoever issues it).
 __device__ __forceinline__ void s2_producer(const Stream2Params& sp, const SRing& rg, volatile int* s_dead, int pidx) {

@@ -80,7 +80,7 @@ def load_gguf(path, max_batch=1):
 
 
 def write_gguf(path, arch, desc, tensors):
-    """Synthetic-model writer (SURVEY.md §A.2 recipe, tests/embedded_model_test.rs:107-304)."""
+    """Synthetic-model writer (tests/embedded_model_test.rs:107-304)."""
     import gguf
 
     w = gguf.GGUFWriter(path, arch)

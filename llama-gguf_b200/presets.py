@@ -1,4 +1,4 @@
-"""Shapes of the architectures BASELINE.json names and the GGUF tensor
+"""Shapes of the architectures of the benchmark and the tests and the GGUF tensor
 inventory / quant-type mix of a Q4_K_M / Q5_K_M / uniform file for them."""
 
 F32, F16, Q4_0, Q5_0, Q8_0, Q4_K, Q5_K, Q6_K = 0, 1, 2, 6, 8, 12, 13, 14
@@ -39,7 +39,7 @@ def use_more_bits(i, n_layers):
 
 
 def _fit(t, k):
-    """K-quants need ne[0] % 256 == 0; real files fall back Q4_K/Q5_K -> Q5_0 and Q6_K -> Q8_0 (SURVEY §8 a5)."""
+    """K-quants need ne[0] % 256 == 0; real files fall back Q4_K/Q5_K -> Q5_0 and Q6_K -> Q8_0."""
     if t in (Q4_K, Q5_K, Q6_K) and k % 256:
         return Q8_0 if t == Q6_K else Q5_0
     return t

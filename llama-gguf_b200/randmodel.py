@@ -2,7 +2,7 @@
 
 Used by bench.py for the full-size models: pure-bandwidth work needs valid blocks with
 sane magnitudes, not a quantiser.  f16 scale fields are set so that dequantised weights
-have zero mean and standard deviation ~sigma (SURVEY.md §8d "direct random finite
+have zero mean and standard deviation ~sigma ("direct random finite
 blocks").  Parity tests do NOT use this module: they quantise N(0, sigma^2) weights with
 the restated reference quantisers (tests/synth.py).
 """

@@ -5,8 +5,8 @@
 // bench.py's cpu_baseline / --impl reference leg), never the product.
 //
 // The reference (Lexmata/llama-gguf v0.14.0) is pure Rust and no Rust toolchain
-// exists in the build image, so the reference cannot be compiled here
-// (DESIGN.md §oracle).  Every function below follows one reference function,
+// exists in the build image, so the reference cannot be compiled here.
+// Every function below follows one reference function,
 // cited as file:line relative to the reference root, and reproduces its
 // operation ORDER (Rust never contracts a*b+c into an FMA: build with
 // -ffp-contract=off; FMAs appear only where the reference calls _mm*_fmadd_ps).
@@ -15,7 +15,7 @@
 // gguf-py's numpy dequantize (tests/golden/, tests/test_oracle_golden.py) and
 // against the reference's own known-answer tests restated in
 // tests/test_oracle_kat.py.  The K-quant fused dots and the end-to-end forward
-// have NO golden vectors in the reference (SURVEY.md §8c "not pinned"), so for
+// have NO golden vectors in the reference, so for
 // those this restatement is the authority: "parity unpinned" beyond dequant.
 
 #include <cmath>
