@@ -19,8 +19,8 @@
 //     (TN columns x 128 lanes); tcgen05.commit -> mbarrier tells the CTA that the tiles may be overwritten;
 //   * epilogue: warp w reads TMEM lanes 32w..32w+31 with tcgen05.ld.32x32b.x32, thread = weight row, 32
 //     tokens per load, and stores Y so that a warp writes 32 consecutive floats of one token's row.
-// fp16 operands, f32 accumulation: measured 3e-4 of the largest output against a double-precision dequant-then-dot
-// (N(0, 1) blocks of every type); the exact token-by-token path stays the default where bit-level greedy parity matters.
+// fp16 operands, f32 accumulation: measured 3e-4 of the largest output against a double-precision dequant-then-dot;
+// the exact token-by-token path stays the default where bit-level greedy parity matters.
 // Two stages: the MMAs of step k overlap the dequant of step k + 1; the dequant (CUDA cores), not the tensor pipe, is the
 // limit.
 #pragma once

@@ -1,6 +1,6 @@
 """Generates tests/golden/dequant_golden.npz with gguf-py (gguf==0.19.0), an implementation
 independent of both the reference and this repo whose numpy dequantize uses the same
-operation order as the reference's dequant.rs (SURVEY.md §8c).  For every block format on
+operation order as the reference's dequant.rs.  For every block format on
 the hot path: 24 random blocks (random bytes, finite f16 scales incl. one subnormal and
 one negative scale) and their dequantised f32 values.
 

@@ -1,4 +1,4 @@
-"""Synthetic random-init models for the parity tests (SURVEY.md §8d recipe).
+"""Synthetic random-init models for the parity tests.
 
 Weights are drawn N(0, sigma^2) and quantised PER TENSOR TYPE with the restated reference
 quantisers (oracle.quantize -> src/tensor/quant/dequant.rs:374-999), norm weights are
@@ -68,7 +68,7 @@ def synth_model(preset_name, mix, max_seq_len, seed=1234, sigma=0.02, max_batch=
 
 
 def prompt_tokens(n, vocab):
-    """SURVEY.md §8d: prompt = (i*7919+1) % vocab"""
+    """prompt = (i*7919+1) % vocab"""
     return [(i * 7919 + 1) % vocab for i in range(n)]
 
 

@@ -1,4 +1,4 @@
-"""GGUF -> HBM direct load (SURVEY §8f row 2): the library's own GGUF reader and model-description rules (csrc/gguf_load.cuh,
+"""GGUF -> HBM direct load: the library's own GGUF reader and model-description rules (csrc/gguf_load.cuh,
 b200_gguf_* / b200_ctx_create_from_gguf) against
 
   * gguf-py (the format's reference implementation) on synthetic files of every model family: same header fields, same tensor

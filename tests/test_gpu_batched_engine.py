@@ -1,4 +1,4 @@
-"""Continuous batching (SURVEY §8f row 1): b200_batch_* against a restatement of the reference's BatchedEngine loop
+"""Continuous batching: b200_batch_* against a restatement of the reference's BatchedEngine loop
 (src/engine_batched.rs:199-411) that steps the ORACLE model one sequence at a time, exactly as the reference does
 (step_sequence, :366-411: whole prompt on the first step, then one token per step through Model::forward; greedy pick, last
 maximum wins).  The event streams -- token ids, their order across sequences, finish reasons, prompt / completion counts, the

@@ -1,4 +1,4 @@
-"""Parity at the shapes BASELINE.json names, not miniatures (VERDICT r1 "parity at real config shapes"), plus the tie rules of
+"""Parity at the shapes of the benchmark's models, not miniatures, plus the tie rules of
 the greedy pick (src/main.rs:1816-1821: LAST maximal index) and of the MoE router (src/model/moe.rs:168: stable sort, lowest
 index first) exercised on the device, the exported Backend methods and the opt-in prefill queue.
 Tolerance: logits within 1e-3 relative (max|a-b| / max|b|), greedy token sequences identical (north star)."""
@@ -15,7 +15,7 @@ TOL = 1e-3
 
 
 def test_config0_qwen25_05b_q4km_128_prompt_64_greedy(b200, oracle):
-    """BASELINE configs[0] verbatim: Qwen2.5-0.5B architecture (H = 896: Q4_K -> Q5_0 and Q6_K -> Q8_0 fallback types, NeoX RoPE,
+    """Qwen2.5-0.5B architecture (H = 896: Q4_K -> Q5_0 and Q6_K -> Q8_0 fallback types, NeoX RoPE,
     q/k/v biases, tied 151 936-row head), Q4_K_M mix, 128-token prompt + 64 greedy tokens, batch 1."""
     arch, desc, tensors = synth.synth_model("qwen2.5-0.5b", "Q4_K_M", 256)
     gpu = b200.GpuOnlyInference(desc, tensors)
@@ -166,7 +166,7 @@ def test_prefill_queue_reaches_the_gemm_prefill_through_prefill_token(b200, orac
 
 
 def test_llama3_8b_shape_int8_kv_from_a_gguf_file_and_the_batched_engine(b200, oracle, tmp_path):
-    """The rows added last at Llama-3-8B shapes, 2 layers, full 128 256-row head: the model is written to a
+    """Loading, batches and the int8 cache at Llama-3-8B shapes, 2 layers, full 128 256-row head: the model is written to a
     GGUF file, loaded by the library's own reader (b200_ctx_create_from_gguf) with the INT8 KV cache, decoded against the oracle's
     int8-cache model; then an f32 context of the same file runs four requests through the continuous-batching engine against the
     reference loop's restatement (exact path: < 8 rows)."""

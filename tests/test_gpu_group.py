@@ -1,6 +1,6 @@
 """The single-process group (b200_group_*: one context and one host thread per device INSIDE the library, peers connected with
 cudaDeviceEnablePeerAccess) against the oracle and the single-GPU context: what a Rust GpuOnlyInference would call when B200_TP is
-set -- no ranks, no other process (SURVEY §8b; TensorParallel trait, src/backend/tensor_parallel.rs:13-32; ShardingPlan :69-106;
+set -- no ranks, no other process (TensorParallel trait, src/backend/tensor_parallel.rs:13-32; ShardingPlan :69-106;
 MoE models: experts spread over the devices, src/model/moe.rs:321-413 on one host in the reference).
 Tolerance: logits within 1e-3 relative of the oracle, greedy tokens identical."""
 import numpy as np
@@ -40,7 +40,7 @@ def test_group_of_one_is_the_single_gpu_context(b200, oracle):
 @pytest.mark.parametrize("preset,mix", [("llama-stream-tiny", "Q4_K_M"), ("llama-tiny", "Q8_0"), ("mixtral-tiny", "Q4_K_M")])
 def test_group_of_two_devices_in_one_process(b200, oracle, preset, mix):
     if b200.device_count() < 2:
-        pytest.skip("needs 2 GPUs (run with gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     arch, desc, tensors = synth.synth_model(preset, mix, 64, vocab=1024 if preset == "llama-stream-tiny" else None)
     prompt = synth.prompt_tokens(6, desc["vocab"])
     g = b200.GroupInference(desc, tensors, n_devices=2)

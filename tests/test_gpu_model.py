@@ -104,7 +104,7 @@ def test_context_length_exceeded(b200, oracle):
 
 
 def test_independent_sequence_slots(b200, oracle):
-    """b200_decode_batch: slots do not clobber each other's KV cache (SURVEY §8f row 1)."""
+    """b200_decode_batch: slots do not clobber each other's KV cache."""
     arch, desc, tensors = synth.synth_model("llama-tiny", "Q4_K_M", 48, max_batch=3)
     gpu = b200.GpuOnlyInference(desc, tensors)
     refs = [oracle.OracleModel(desc, tensors) for _ in range(3)]

@@ -1,7 +1,7 @@
 """GEMM prefill (csrc/gemm_umma.cuh tcgen05/TMEM dequant-GEMM + csrc/prefill.cuh) through the batch entry point
 b200_prefill, against the oracle's token-by-token LlamaModel::forward (src/model/llama.rs:275-362).
 
-Tolerance: north_star's 1e-3 relative (max|a-b| / max|b|) on the logits.  This path rounds both GEMM operands to fp16 (f32
+Tolerance: 1e-3 relative (max|a-b| / max|b|) on the logits.  This path rounds both GEMM operands to fp16 (f32
 accumulation in TMEM); measured on these cases (scripts/gemm_err.py on a B200): 0.9e-4 ... 5.3e-4, so it holds the same
 bound as the exact token-by-token entry points (which measure ~2e-6).  The KV cache it leaves must let the exact decode
 path continue within the same bound."""
@@ -67,7 +67,7 @@ def test_short_prompts_and_disabled_gemm_stay_exact(b200, oracle):
 @pytest.mark.parametrize("preset,mix", [("llama-tiny", "Q4_K_M"), ("qwen-kq-tiny", "Q5_K_M")])
 def test_batched_decode_through_the_gemm(b200, oracle, preset, mix):
     """b200_decode_batch with >= 8 sequences: one pass of the dequant-GEMMs for all rows, each row at ITS slot's position
-    and on ITS slot's KV cache (SURVEY §8f rank 1).  Same 1e-3 bound as the GEMM prefill."""
+    and on ITS slot's KV cache.  Same 1e-3 bound as the GEMM prefill."""
     nseq = 12
     arch, desc, tensors = synth.synth_model(preset, mix, 64, max_batch=nseq)
     gpu = b200.GpuOnlyInference(desc, tensors)

@@ -70,7 +70,7 @@ def _run(rank, world, mix, q, torch, dist, B, synth, TensorParallelInference, np
 @pytest.mark.parametrize("mix,preset", [("Q4_K_M", "llama-tiny"), ("Q8_0", "llama-tiny"), ("Q4_K_M", "llama-stream-tiny")])
 def test_tp2_matches_single_gpu_and_oracle(b200, mix, preset):
     if b200.device_count() < 2:
-        pytest.skip("needs 2 GPUs (run with gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     import torch.multiprocessing as mp
 
     import synth
@@ -93,7 +93,7 @@ def test_tp2_matches_single_gpu_and_oracle(b200, mix, preset):
     # shards whose rows are 16-byte multiples run the streamed megakernel under TP too, the rest the first megakernel
     assert r0["path"] == r1["path"] == ("stream2" if preset == "llama-stream-tiny" or mix == "Q8_0" else "mega")
     assert np.array_equal(r0["logits"], r1["logits"])                      # every rank sees the same gathered logits
-    assert synth.rel_err(r0["logits"], r0["want"]) < 1e-3                   # north_star tolerance vs the CPU reference path
+    assert synth.rel_err(r0["logits"], r0["want"]) < 1e-3                   # tolerance vs the CPU reference path
     assert synth.rel_err(r0["logits"], r0["single_logits"]) < 1e-4          # summation order differs, nothing else
     assert r0["tokens"] == r1["tokens"] == r0["single_tokens"]              # identical greedy tokens on every rank
 
@@ -103,7 +103,7 @@ def test_expert_parallel_2_gpus_matches_single_gpu_and_oracle(b200, mix):
     """Mixtral-style MoE (4 experts, top-2) with the experts spread over 2 GPUs (src/model/moe.rs:321-413 on one host in the
     reference): every rank holds the full logits; the combine adds the weighted expert outputs in selection order, then the residual (moe.rs:363-368)."""
     if b200.device_count() < 2:
-        pytest.skip("needs 2 GPUs (run with gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     import torch.multiprocessing as mp
 
     import synth

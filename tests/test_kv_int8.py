@@ -1,4 +1,4 @@
-"""INT8 KV cache (SURVEY §8f row 4): the reference's QuantizedKVCache in its Int8 format (src/model/kv_quantized.rs).
+"""INT8 KV cache: the reference's QuantizedKVCache in its Int8 format (src/model/kv_quantized.rs).
 
 CPU part: the oracle's restatement of quantize_int8 / dequantize_int8 against the reference's own tests
 (kv_quantized.rs:547-561 test_int8_roundtrip, :613-670 test_quantized_kv_cache_basic — same inputs, same bounds) and against an
@@ -99,7 +99,7 @@ def test_int8_kv_rejects_what_it_does_not_cover(b200):
 @pytest.mark.gpu
 @pytest.mark.parametrize("preset,mix,n", [("llama-stream-tiny", "Q4_K_M", 130), ("tinyllama-stream-tiny", "Q8_0", 70), ("llama-tiny", "Q4_K_M", 48)])
 def test_int8_kv_prompt_through_the_tensor_core_path_is_opt_in(b200, oracle, preset, mix, n, monkeypatch):
-    """OPT-IN (B200_KV_INT8_GEMM=1), and NOT inside north_star's 1e-3: a prompt of >= 32 tokens takes ONE pass of the dequant-GEMMs
+    """OPT-IN (B200_KV_INT8_GEMM=1), and NOT inside the 1e-3 of the other paths: a prompt of >= 32 tokens takes ONE pass of the dequant-GEMMs
     -- RoPE + quantised cache write for all rows (prefill_rope_kv_q8_kernel), tcgen05 attention over fp16 tiles of the DEQUANTISED
     rows (prefill_kv16_q8_kernel) -- but its K / V rows differ from the exact path's by the fp16 operand rounding before they are
     quantised, and rounding to int8 codes is discontinuous (the neighbouring code is 1/127 of the row maximum away).  Measured

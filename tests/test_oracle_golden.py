@@ -1,6 +1,6 @@
 """Pins the oracle's block dequantisation bit-for-bit against the gguf-py golden vectors
 (tests/golden/make_golden.py) — the only byte->float authority available for K-quants,
-since the reference's own tests hold no exact K-quant vectors (SURVEY.md §8c)."""
+since the reference's own tests hold no exact K-quant vectors."""
 import os
 
 import numpy as np

@@ -1,5 +1,5 @@
-"""The reference's own known-answer tests for this path, restated against the oracle
-(SURVEY.md §4 rows 1-2, §8c).  Each test cites the reference test it restates."""
+"""The reference's own known-answer tests for this path, restated against the oracle.
+Each test cites the reference test it restates."""
 import numpy as np
 import pytest
 
