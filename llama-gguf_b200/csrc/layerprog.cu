@@ -1445,10 +1445,12 @@ struct LpModel {
     std::vector<int> step_p0, step_len; // the step's runs: first position, tokens
     uint8_t* keys16 = nullptr;          // lp_tile_attn.cuh: the keys and values of one layer in bf16, kept from call to call
     size_t keys16_bytes = 0;
-    // Whether the products may cut K over a cluster (B200_LP_TC_SPLIT=0 / 1).  Not in programs with experts: another order of the sums is another rounding of the
-    // activations behind them, which after a few layers has changed every activation by its bf16 rounding, and a token whose second and third expert are that
-    // close then takes the other one -- a different row, not a rounding of it.
-    bool tc_split = true;
+    // Whether steps may add in another order than the kernels of one row tile and one key tile do (B200_LP_ANY_ORDER=0 / 1): products that cut K over a cluster,
+    // tcgen05 attention where every run sees one tile of keys.  Not in programs with experts: another order of the sums is another rounding of the activations
+    // behind them, which after a few layers has changed every activation by its bf16 rounding, and a token whose second and third expert are that
+    // close then takes the other one -- a different row, not a rounding of it.  32 sequences through two layers of width 2048, a step's products of 32 rows 10.2 -> 14.9 us,
+    // prompts of 48 tokens 26 -> 44 us of attention per layer.
+    bool any_order = true;
     bool tc_maps = true;                    // B200_LP_TC_MAPS=0: as if the driver refused the tensor maps of the products
     size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
@@ -1676,7 +1678,7 @@ struct TcProduct {
 bool tc_prepare(const LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, int R, bool glu, bool seg, int xrows, int groups, size_t wz, ZStride zs, TcProduct& t) {
     if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs) || !m->tc_maps) return false;
     const bool x_z = !seg && groups > 1 && zs.x > 0;
-    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->tc_split);
+    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->any_order);
     const int kh = t.pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     return tc_map(&t.xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, t.pl.tn, kh) &&
            tc_map(&t.wm, W, K, N, ldw, glu ? 2 : 1, groups, wz, glu ? TC_M / 2 : TC_M, kh);
@@ -2758,8 +2760,8 @@ int lp_finalize(LpModel* m, std::string* err) {
         }
     }
     {
-        const char* e = getenv("B200_LP_TC_SPLIT");
-        m->tc_split = e && *e ? atoi(e) != 0 : m->max_experts == 0;
+        const char* e = getenv("B200_LP_ANY_ORDER");
+        m->any_order = e && *e ? atoi(e) != 0 : m->max_experts == 0;
     }
     LCU_ALLOC(cudaMalloc((void**)&m->tc_err, 256));
     LCU(cudaMemset(m->tc_err, 0, 256));
@@ -2974,7 +2976,7 @@ bool attn_tc(LpModel* m, const StepMeta& sm, const AttnGeom& ag, int ldp, int n_
         tiles += t;
     }
     if (tiles > (1 << 20)) return false;
-    if (tiles == n_runs) return false;      // (one tile of keys per run: the copies would cost what the mma.sync kernels take for all of it)
+    if (!m->any_order && tiles == n_runs) return false;      // (one tile of keys per run)
     if (ag.dim <= 64 && ag.vdim <= 64) return attn_tc_launch<64, 64>(m, sm, ag, ldp, n_runs, max_len, (int)tiles, out_ld, out_scale);
     return attn_tc_launch<128, 128>(m, sm, ag, ldp, n_runs, max_len, (int)tiles, out_ld, out_scale);
 }

@@ -54,14 +54,14 @@ def test_refused_tensor_maps_take_the_cuda_core_products(b200, monkeypatch):
 
 @pytest.mark.parametrize("kind", list(LAYERS))
 def test_programs_with_experts_add_in_the_order_of_k(b200, monkeypatch, kind):
-    """32 rows at a width where K would be cut over clusters (B200_LP_TC_SPLIT=1): not in a program with experts, whose choices another order of the sums would turn in
+    """32 rows at a width where K would be cut over clusters (B200_LP_ANY_ORDER=1): not in a program with experts, whose choices another order of the sums would turn in
     close calls."""
     cfg = S.config(LAYERS[kind](1024, 2048), width=1024, vocab=264)
     w = S.random_weights(cfg, 7)
     toks = [int(t) for t in np.random.default_rng(1).integers(0, cfg["vocab"], 32)]
     out = {}
     for split in ("", "0", "1"):
-        monkeypatch.setenv("B200_LP_TC_SPLIT", split)
+        monkeypatch.setenv("B200_LP_ANY_ORDER", split)
         gpu = S.gpu_model(cfg, w, "bfloat16", max_seq_len=40)
         try:
             out[split] = gpu.step([(0, toks)], list(range(32)))

@@ -60,10 +60,12 @@ def test_rounds_what_the_mma_kernels_round(b200, monkeypatch, layer, n):
     assert GS.rel_err(outs["1024"], outs["0"]) < 4e-3
 
 
-@pytest.mark.parametrize("lens,same", [((48, 64, 17), True), ((48, 65, 17), False)])
-def test_one_tile_of_keys_per_run_keeps_the_mma_kernels(b200, monkeypatch, lens, same):
-    """Steps whose runs see one tile of keys each: bit for bit the mma.sync kernels (B200_LP_KEYS16_MB=0); with one run of 65 keys the other kernel takes the step."""
-    cfg = GS.config([GS.attn(heads=4, kv_heads=2, dim=128, softcap=50.0), GS.latent(heads=3, dim=16, vdim=24, kv_rank=128)], width=256, vocab=80)
+@pytest.mark.parametrize("lens,mlp,same", [((48, 64, 17), "moe", True), ((48, 64, 17), "dense", False), ((48, 65, 17), "moe", False)])
+def test_one_tile_of_keys_per_run_in_programs_with_experts(b200, monkeypatch, lens, mlp, same):
+    """Steps of programs with experts whose runs see one tile of keys each: bit for bit the mma.sync kernels (B200_LP_KEYS16_MB=0).  Without experts, or with one run of
+    65 keys, the other kernel takes the step."""
+    cfg = GS.config([GS.attn(heads=4, kv_heads=2, dim=128, softcap=50.0), GS.latent(heads=3, dim=16, vdim=24, kv_rank=128, mlp=GS.moe() if mlp == "moe" else GS.dense())],
+                    width=256, vocab=80)
     w = GS.random_weights(cfg, 5)
     rng = np.random.default_rng(1)
     runs = [(i, [int(t) for t in rng.integers(0, cfg["vocab"], n)]) for i, n in enumerate(lens)]
