@@ -2013,10 +2013,20 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     };
     // Which chunks, layer by layer: above 64 tokens all (two 8B layers, 80 / 333 / 2048 tokens: Q4_K_M 1160 -> 725, 1517 -> 993, 3635 -> 2635 us, Q6_K 1865 -> 822,
     // 2420 -> 1092, 5873 -> 2730 us; two 2048-wide layers in Q8_0 699 -> 366, 931 -> 470, 1662 -> 1082 us), where the fused kernel's token tile
-    // doubles; down to 32 tokens too unless the layer's wide matrices are Q4_K, whose fused unpacking costs less than the pass over fp16 rows (32 tokens:
-    // Q4_K_M 551 against 674 us, Q6_K 783 against 772, Q8_0 380 against 331).  256 MB of rows at a time at most; a device without room for them
-    // keeps the fused kernel.
-    auto f16_min = [&](const Layer& L) { return c->prompt_f16_min > 0 ? c->prompt_f16_min : L.gate.type == T_Q4_K ? 65 : 32; };
+    // doubles.  Up to 64 tokens the fused kernel reads a matrix once, so what the pass over fp16 rows costs decides: 4 bytes of traffic per weight once gate and up are past
+    // the L2 cache, next to none before (fused / two-pass time of two layers, 32 and 64 tokens; hidden x ffn 2048 x 5632: Q8_0 1.14, 1.28, Q5_K_M 1.17, 1.32; 3072 x
+    // 8192: 0.97, 1.11, 1.01, 1.14; 4096 x 8192: 0.91, 1.05, 0.89, 1.04; 4096 x 14336: 0.78, 0.92, 0.80, 0.94).  Q6_K, whose fused unpacking is the dearest, takes it
+    // for wider layers too (4096 x 14336: 1.02, 1.14; 8192 x 28672: 0.83, 0.92), as do layers with Q6_K rows of no whole 16 bytes, which the TMA unit cannot fetch
+    // (3584 x 9728 Q5_K_M: 1.30, 1.47); Q4_K, the cheapest, not.  256 MB of rows at a time at most; a device without room for them keeps the fused kernel.
+    auto f16_min = [&](const Layer& L) {
+        if (c->prompt_f16_min > 0) return c->prompt_f16_min;
+        if (L.gate.type == T_Q4_K) return 65;
+        const size_t mb = (size_t)4 * I * H / 1000000;      // gate and up as fp16 rows
+        bool raw = false;
+        for (const DevTensor* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down}) raw |= w->type == T_Q6_K && w->row_bytes % 16;
+        if (raw || L.gate.type == T_Q6_K) return raw || mb <= 512 ? 32 : 65;
+        return mb <= 96 ? 32 : mb <= 136 ? 48 : 65;
+    };
     bool f16_able = false;
     for (const Layer& L : c->layers) f16_able |= !rows && gemm_encode_fn() && std::min(cap, n) >= f16_min(L);
     if (f16_able && !c->pf_w16) {

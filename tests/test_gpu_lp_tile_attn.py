@@ -42,10 +42,9 @@ def test_against_the_warp_kernel(b200, monkeypatch, heads, kv_heads, dim, vdim, 
                                    GS.latent(heads=3, dim=16, vdim=24, kv_rank=128, scale=1.0), GS.latent(heads=4, dim=48, vdim=64, kv_rank=64, scale=1.0)])
 @pytest.mark.parametrize("n", [65, 130, 300])
 def test_rounds_what_the_mma_kernels_round(b200, monkeypatch, layer, n):
-    """Queries, keys as they are stored and probabilities against the running maximum of tiles of 64 keys are rounded to bf16, and nothing else: a key row's factor meets
-    the f32 score.  The mma.sync kernels (B200_LP_KEYS16_MB=0) round the same numbers, so both differ by the order of f32 sums: here and there a probability
-    of a row falls on the other side of a bf16 boundary, 2^-8 of itself and at most 4e-3 of the row where it is nearly all of it.  A product of key and factor
-    that is rounded moves scores of some tens (scale 1) by 2^-9 of themselves, the row by 1e-2 and more."""
+    """Queries, keys as they are stored and probabilities are rounded to bf16, and nothing else: a key row's factor meets the f32 score.  The mma.sync kernels
+    (B200_LP_KEYS16_MB=0) round the same numbers, probabilities against another maximum: each is 2^-8 of itself apart at most, a row 4e-3 where one of them is nearly
+    all of it (measured 2.3e-3).  A product of key and factor that is rounded moves scores of some tens (scale 1) by 2^-9 of themselves, the row by 7e-3 to 1.4e-2."""
     cfg = GS.config([layer], width=256, vocab=80)
     w = GS.random_weights(cfg, 5)
     toks = [int(t) for t in np.random.default_rng(n).integers(0, cfg["vocab"], n)]

@@ -68,3 +68,26 @@ def test_each_layer_goes_by_its_own_types(b200, monkeypatch, first, second):
         finally:
             gpu.close()
     assert count["0"] not in (count["1"], count["100000"]), count
+
+
+@pytest.mark.parametrize("mix,ffn,n,two_pass", [("Q8_0", 16384, 40, True), ("Q8_0", 49152, 40, False), ("Q8_0", 49152, 50, True), ("Q8_0", 73728, 50, False),
+                                                ("Q8_0", 73728, 65, True), ("Q6_K", 73728, 40, True), ("Q4_K", 16384, 64, False)])
+def test_short_prompts_go_by_the_size_of_the_layer(b200, monkeypatch, mix, ffn, n, two_pass):
+    """Up to 64 tokens the two passes are taken while gate and up as fp16 rows fit in L2 (512 wide: 16384 units 34 MB, 49152 101 MB, 73728 151 MB); the number of
+    kernels shows which way a prompt went."""
+    monkeypatch.setitem(synth.TINY, "wide", dict(synth.TINY["tinyllama-tiny"], n_layers=1, ffn=ffn))
+    arch, desc, tensors = synth.synth_model("wide", mix, 80)
+    prompt = synth.prompt_tokens(n, desc["vocab"])
+    count = {}
+    for rule in ("0", "1", "100000"):
+        monkeypatch.setenv("B200_PROMPT_F16_MIN", rule)
+        gpu = b200.GpuOnlyInference(desc, tensors)
+        try:
+            gpu.prefill(prompt)
+            before = gpu.stats()["kernel_launches"]
+            gpu.reset()
+            gpu.prefill(prompt)
+            count[rule] = gpu.stats()["kernel_launches"] - before
+        finally:
+            gpu.close()
+    assert count["1"] != count["100000"] and count["0"] == count["1" if two_pass else "100000"], count
