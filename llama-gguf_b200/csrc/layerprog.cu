@@ -1455,8 +1455,9 @@ struct LpModel {
     size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
     size_t chunk_scan_bytes = 0;
-    // Programmatic launches for steps of more than 16 rows (B200_LP_PDL=0: none): three ragged prompts 702 -> 605 us, prompt of 2048 910 -> 863, 32 prompts
-    // and 8 steps of 32 sequences 2717 -> 2530; one row, whose kernels fill the chip with blocks that would only wait, 6275 -> 6404 (24 steps)
+    // Programmatic launches for bf16 steps of more than 16 rows (B200_LP_PDL=0: none): three ragged prompts 702 -> 605 us, prompt of 2048 910 -> 863, 32 prompts
+    // and 8 steps of 32 sequences 2717 -> 2530.  Not for one row, whose kernels fill the chip with blocks that would only wait, 6275 -> 6404 (24 steps), and not in f32, whose
+    // CUDA-core products do so with every prompt: 24 tokens through two layers of width 2048 2295 -> 4152 us, 251 through two of 1024 1739 -> 2581
     bool use_pdl = true, pdl_now = false;
     bool use_chunk_scan = true;         // B200_LP_CHUNK_SCAN=0: prompts go token by token
     std::vector<int> run_pass;          // pass number t when the run is the first of a pass (step vector t is added), else -1
@@ -3120,7 +3121,7 @@ void row_combine(LpModel* m, const AttnGeom& ag, int R, int splits) {
 // Every kernel of one step, in order, on the model's stream: eagerly, or while the stream is being captured into a CUDA graph (a
 // decode step: one row per run, nothing allocated).  head: 0 = no logits, 1 = logits of the wanted rows, 2 = their greedy picks.
 void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want, int head, int taps_len, int max_len) {
-    m->pdl_now = m->use_pdl && R > 2 * GV_ROWS;
+    m->pdl_now = m->use_pdl && !m->f32 && R > 2 * GV_ROWS;
     const b200_program_desc& p = m->p;
     const int W = p.width;
     const float* loop_step = p.loop_stop > p.loop_start ? (const float*)find(m, "loop.step")->d : nullptr;

@@ -8,9 +8,9 @@
 //   maximum has grown by more than 2^8 since the last time (probabilities up to 2^8 lose nothing in bf16; rescaling at every growth: 45 -> 53 us for 2048 queries of
 //   16 latent heads); the division comes last.
 // Both B operands have the contracted index contiguous, so the cached f32 rows are rounded to bf16 once per layer (lp_keys16_kernel): K16[g]
-// [key][DKP], as they are stored (their factors, if they have any, go into F[g][key] and meet the f32 score: rounding key x factor moves every score by another
-// 2^-9 of itself and, through the layers behind, the logits), and the transpose Vt16[g][channel][key], the keys of every run from the first one that a query of the step sees, in tiles of 64
-// whose missing keys are zeros; TMA brings the tiles.  Roles: 4 softmax warps, a loader thread, an MMA thread; two CTAs share an SM (112 KB
+// [key][DKP] as they are stored (their factors, if they have any, go into F[g][key] and meet the f32 score, as in the mma.sync kernel: 5 us of 70 for 2048 queries of
+// 16 heads), and the transpose Vt16[g][channel][key], the keys of every run from the first one that a query of the step sees, in tiles of 64 whose
+// missing keys are zeros; TMA brings the tiles.  Roles: 4 softmax warps, a loader thread, an MMA thread; two CTAs share an SM (112 KB
 // of shared memory and 256 TMEM columns each), so one CTA's products run under the other's exponentials.
 // What bounded the mma.sync kernels (each block converting its own tiles, one tile after the other): 12.5 us per 64-key tile of
 // lp_window_attn_tile_kernel, 5 us of lp_row_tile_kernel, where a tile's products need 0.3 us of this pipe and its exponentials 0.5.  Measured:
