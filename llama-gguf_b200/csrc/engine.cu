@@ -33,6 +33,7 @@
 #include "gemv.cuh"
 #include "gemm_umma.cuh"
 #include "gemm_umma2.cuh"
+#include "few_rows.cuh"
 #include "prompt_f16.cuh"
 #include "spare.cuh"
 #include "attn_umma.cuh"
@@ -236,6 +237,10 @@ struct b200_ctx {
     int* pf_tile_cnt = nullptr;      // split-K tile counters of the persistent dequant-GEMM (zeroed once; the kernel re-zeroes them)
     void* pf_tmaps = nullptr;        // TMA tensor maps (128-row boxes) of the GEMM weights
     std::map<const void*, int> pf_tmap_of;
+    std::map<const void*, int> few_tmap_of;   // ... of the products of few rows (gemm_few.cuh); Q6_K blocks with another pitch
+    bool few_able = false;           // every product of a layer can take that path
+    uint8_t* few_img[3] = {};        // images of the activations: normed rows, attention, gated units
+    float* few_part = nullptr;       // pieces of cut tiles
     bool pf_tmaps_built = false;
     size_t pf_split_floats = 0;
     int pf_logits_rows = 0;
@@ -911,6 +916,8 @@ extern "C" void b200_ctx_destroy(b200_ctx* c) {
     cudaFree(c->pf_split);
     cudaFree(c->pf_w16);
     cudaFree(c->pf_tmaps);
+    for (uint8_t* p : c->few_img) cudaFree(p);
+    cudaFree(c->few_part);
     cudaFree(c->pf_tile_cnt);
     cudaFree(c->attn_q8_part);
     cudaFree(c->pf_k16);
@@ -1806,12 +1813,26 @@ static int umma_tmaps_build(b200_ctx* c) {
             return;
         c->pf_tmap_of[w.d] = (int)maps.size();
         maps.push_back(tm);
+        const int fp = few_pitch(w.type);
+        if (fp != pitch) {
+            const cuuint32_t fbox[2] = {(cuuint32_t)(fp / 4), (cuuint32_t)kUmmaM};
+            if (encode(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)w.d, dims, strides, fbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return;
+            maps.push_back(tm);
+        }
+        c->few_tmap_of[w.d] = (int)maps.size() - 1;
     };
     for (const Layer& L : c->layers) { add(L.wq); add(L.wk); add(L.wv); add(L.wo); add(L.gate); add(L.up); add(L.down); }
     add(c->output.present() ? c->output : c->token_embd);
     if (maps.empty()) return B200_OK;
     CU_ALLOC(late_malloc(c, (void**)&c->pf_tmaps, maps.size() * sizeof(CUtensorMap)));
     CU(cudaMemcpy(c->pf_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+    const b200_model_desc& d = c->d;
+    // whole blocks of 256 in every row; narrower than 1024, a layer's products are a microsecond of work either way and keep the kernels they had (tests pin their count)
+    c->few_able = env_int("B200_FEW_GEMM", 1) != 0 && d.hidden % 256 == 0 && d.hidden >= 1024 && d.hidden <= kFewNormMax && d.n_heads * d.head_dim % 256 == 0 && d.ffn % 256 == 0;
+    for (const Layer& L : c->layers)
+        for (const DevTensor* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down}) c->few_able = c->few_able && c->few_tmap_of.count(w->d);
     return B200_OK;
 }
 static void umma_set_tmap(b200_ctx* c, UmmaParams& p) {
@@ -1882,6 +1903,21 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         CU_ALLOC(late_malloc(c, (void**)&c->pf_split, c->pf_split_floats * sizeof(float)));
         CU_ALLOC(late_malloc(c, (void**)&c->pf_tile_cnt, 8192 * sizeof(int)));
         CU(cudaMemset(c->pf_tile_cnt, 0, 8192 * sizeof(int)));
+    }
+    // products of few rows (gemm_few.cuh): images of the activations and pieces of cut tiles; a device without room for them keeps the other products
+    const int few_max = kFewTokens, last_chunk = n % cap ? n % cap : cap;
+    if (c->few_able && c->kv_format == 0 && !c->few_part && last_chunk <= few_max) {
+        const size_t bytes[4] = {few_image_bytes(few_max, 64, H), few_image_bytes(few_max, 64, A), few_image_bytes(few_max, 64, I), (size_t)2 * c->n_sm * 64 * 128 * sizeof(float)};
+        void* got[4] = {};
+        bool ok = true;
+        for (int i = 0; i < 4 && ok; i++) ok = cudaMalloc(&got[i], bytes[i]) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            for (void* q : got) cudaFree(q);
+        } else {
+            for (int i = 0; i < 3; i++) c->few_img[i] = (uint8_t*)got[i];
+            c->few_part = (float*)got[3];
+        }
     }
     // batched decode: per-row (position, KV base of the slot, SeqState of the slot)
     const bool rows = seqs != nullptr;
@@ -2011,7 +2047,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         }
         return cudaSuccess;
     };
-    // Which chunks, layer by layer: above 64 tokens all (two 8B layers, 80 / 333 / 2048 tokens: Q4_K_M 1160 -> 725, 1517 -> 993, 3635 -> 2635 us, Q6_K 1865 -> 822,
+    // Which chunks, layer by layer, of the models that the products of few rows do not take (few_able; up to 256 tokens), and longer ones: above 64 tokens all (two 8B layers, 80 / 333 / 2048 tokens: Q4_K_M 1160 -> 725, 1517 -> 993, 3635 -> 2635 us, Q6_K 1865 -> 822,
     // 2420 -> 1092, 5873 -> 2730 us; two 2048-wide layers in Q8_0 699 -> 366, 931 -> 470, 1662 -> 1082 us), where the fused kernel's token tile
     // doubles.  Up to 64 tokens the fused kernel reads a matrix once, so what the pass over fp16 rows costs decides: 4 bytes of traffic per weight once gate and up are past
     // the L2 cache, next to none before (fused / two-pass time of two layers, 32 and 64 tokens; hidden x ffn 2048 x 5632: Q8_0 1.14, 1.28, Q5_K_M 1.17, 1.32; 3072 x
@@ -2045,6 +2081,8 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         }
         return gemm(w, K, x, ldx, T, y, ldy, bias, acc);
     };
+    bool few = false, head_done = false;
+    const bool few_pdl = rows && c->batch_pdl;
     int last_T = 0;
     for (int done = 0; done < n; done += cap) {
         const int T = std::min(cap, n - done);
@@ -2052,7 +2090,110 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         last_T = T;
         if (!use_graph) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
         CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T), dim3(256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)c->pf_tok, d.vocab, X));
-        for (int l = 0; l < d.n_layers; l++) {
+        // Few rows: products straight from the blocks (gemm_few.cuh), their pieces added by the kernel behind them
+        few = c->few_part && !q8 && T <= few_max && (rows || c->prompt_f16_min == 0);
+        FewOut sum{};                                   // product that X still lacks (of the layer before)
+        bool has_sum = false;
+        auto few_norm = [&](const float* w, uint8_t* img) {
+            const cudaError_t e = launch_on(st, few_pdl, few_norm_kernel, dim3(T), dim3(H / 8), 0, X, sum, has_sum ? 1 : 0, w, d.norm_eps, img, few_n(T), H);
+            has_sum = false;
+            c->launches++;
+            return e;
+        };
+        auto few_product = [&](std::initializer_list<const DevTensor*> ws, int K, const uint8_t* img, std::initializer_list<float*> ys, int ldy, FewOut& out) {
+            FewArgs a{};
+            int rows_of[kFewMaxSeg] = {}, cost[kFewMaxSeg] = {}, n_seg = 0;
+            for (const DevTensor* w : ws) {
+                FewSeg& sg = a.seg[n_seg];
+                sg.map = (const CUtensorMap*)c->pf_tmaps + c->few_tmap_of.at(w->d);
+                sg.type = w->type;
+                sg.n_rows = rows_of[n_seg] = (int)w->ne[1];
+                sg.pitch = few_pitch(w->type);
+                cost[n_seg] = sg.pitch / 16;
+                sg.block_bytes = 256 / type_block_elems(w->type) * type_block_bytes(w->type);
+                sg.y = ys.begin()[n_seg];
+                sg.ldy = ldy;
+                n_seg++;
+            }
+            if (!few_plan(a.plan, n_seg, rows_of, cost, K, T, c->n_sm)) return cudaErrorInvalidValue;
+            a.image = img; a.part = c->few_part; a.err = c->mma_err;
+            out = FewOut{};
+            out.plan = a.plan; out.part = a.part; out.N = few_n(T);
+            for (int s = 0; s < n_seg; s++) { out.y[s] = a.seg[s].y; out.ldy[s] = ldy; }
+            c->launches++;
+            return few_launch(a, few_pdl, st);
+        };
+        for (int l = 0; few && l < d.n_layers; l++) {
+            Layer& L = c->layers[l];
+            float* kc = sl.kv + (size_t)l * kv_layer;
+            float* vc = kc + kv_layer / 2;
+            CU(few_norm(L.attn_norm.f32(), c->few_img[0]));
+            FewRopeArgs ra{};
+            CU(few_product({&L.wq, &L.wk, &L.wv}, H, c->few_img[0], {Q, Q + A, Q + A + nkv * hd}, QKV, ra.qkv));
+            const DevTensor* bias[3] = {&L.bq, &L.bk, &L.bv};
+            for (int s = 0; s < 3; s++) ra.bias[s] = bias[s]->present() ? bias[s]->f32() : nullptr;
+            const float scale = 1.0f / sqrtf((float)hd);
+            const int Gq = nh / nkv;
+            if (rows) {
+                FewAttnArgs fa{};
+                fa.qkv = ra.qkv; fa.freq = c->rope_freq; fa.n_heads = nh; fa.n_kv = nkv; fa.max_seq = d.max_seq_len; fa.neox = d.rope_neox; fa.A = A;
+                for (int s = 0; s < 3; s++) fa.bias[s] = ra.bias[s];
+                fa.rope_scale = d.rope_scale; fa.scale = scale; fa.row_pos = d_pos; fa.row_kv = d_kv;
+                fa.k_off = (long long)((size_t)l * kv_layer); fa.v_off = fa.k_off + (long long)(kv_layer / 2); fa.img = c->few_img[1];
+                CU(launch_on(st, few_pdl, hd == 128 ? (Gq <= 4 ? few_attn_kernel<128, 4> : few_attn_kernel<128, 8>) : (Gq <= 4 ? few_attn_kernel<64, 4> : few_attn_kernel<64, 8>),
+                             dim3(nkv, T), dim3(256), 0, fa));
+            } else {
+                PrefillRopeParams& rp = ra.p;
+                rp.qkv = Q; rp.ld = QKV; rp.k_cache = kc; rp.v_cache = vc; rp.freq = c->rope_freq; rp.pos0 = pos0;
+                rp.n_heads = nh; rp.n_kv = nkv; rp.hd = hd; rp.max_seq = d.max_seq_len; rp.neox = d.rope_neox; rp.rope_scale = d.rope_scale;
+                few_rope_kv_kernel<<<dim3(T, 4), 256, 0, st>>>(ra);
+                if (attn_tc) {
+                    const int kv_end = pos0 + T, kv_pad = (kv_end + 127) & ~127;
+                    AttnUmmaParams up{};
+                    up.qkv = Q; up.ld = QKV; up.out = ATh; up.ldo = A; up.pos0 = pos0; up.T = T; up.n_heads = nh; up.n_kv = nkv; up.G = Gq;
+                    up.P = c->pf_kv16_P; up.scale = scale; up.err = c->mma_err;
+                    const dim3 kgrid(kv_pad / 64, nkv);
+                    if (hd == 128) {
+                        prefill_kv16_kernel<128><<<kgrid, 256, 0, st>>>(kc, vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
+                        CU(attn_umma_launch_hd<128>(c->pf_kmap, c->pf_vmap, up, st));
+                    } else {
+                        prefill_kv16_kernel<64><<<kgrid, 256, 0, st>>>(kc, vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
+                        CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, st));
+                    }
+                    c->launches += 2;
+                } else {
+                    PrefillAttnParams ap{};
+                    ap.qkv = Q; ap.ld = QKV; ap.k_cache = kc; ap.v_cache = vc; ap.out = ATh; ap.ldo = A; ap.pos0 = pos0; ap.T = T;
+                    ap.n_heads = nh; ap.n_kv = nkv; ap.max_seq = d.max_seq_len; ap.scale = scale;
+                    const int ablocks = (int)(((long long)T * nkv * 32 + 127) / 128);
+                    CU(launch_on(st, false, hd == 128 ? (Gq <= 4 ? prefill_attn_kernel<128, 4> : prefill_attn_kernel<128, 8>) : (Gq <= 4 ? prefill_attn_kernel<64, 4> : prefill_attn_kernel<64, 8>),
+                                 dim3(ablocks), dim3(128), 0, ap));
+                    c->launches++;
+                }
+                few_image_kernel<<<dim3((A / 8 + 255) / 256, T), 256, 0, st>>>(ATh, A, c->few_img[1], few_n(T), A);
+                c->launches++;
+            }
+            CU(few_product({&L.wo}, A, c->few_img[1], {G}, H, sum));
+            has_sum = true;
+            CU(few_norm(L.ffn_norm.f32(), c->few_img[0]));
+            FewOut gu{};
+            CU(few_product({&L.gate, &L.up}, H, c->few_img[0], {G, U}, I, gu));
+            CU(launch_on(st, few_pdl, few_swiglu_kernel, dim3((I / 8 + 255) / 256, T), dim3(256), 0, gu, c->few_img[2], I));
+            CU(few_product({&L.down}, I, c->few_img[2], {G}, H, sum));
+            has_sum = true;
+            c->launches += 2;
+        }
+        if (few) {      // the last product -> X, and in batched decoding the head of all rows
+            const DevTensor& head = c->output.present() ? c->output : c->token_embd;
+            head_done = rows && c->few_tmap_of.count(head.d);
+            CU(few_norm(head_done ? c->output_norm.f32() : nullptr, head_done ? c->few_img[0] : nullptr));
+            if (head_done) {
+                FewOut lg{};
+                CU(few_product({&head}, H, c->few_img[0], {c->pf_logits}, d.vocab, lg));
+                CU(launch_on(st, few_pdl, few_finish_kernel, dim3((d.vocab + 127) / 128, (T + 7) / 8), dim3(128), 0, lg, c->pf_logits, d.vocab));
+            }
+        }
+        for (int l = 0; !few && l < d.n_layers; l++) {
             Layer& L = c->layers[l];
             f16 = f16_able && c->pf_w16 && T >= f16_min(L);
             float* kc = sl.kv + (size_t)l * kv_layer;
@@ -2130,12 +2271,14 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     if (rows) {   // every row's slot advances by one; final RMSNorm + vocab head of ALL rows through the GEMM
         CU(launch_on(st, pdl, prefill_advance_rows_kernel, dim3((n + 127) / 128), dim3(128), 0, (SeqState* const*)d_st, n));
         const DevTensor& head = c->output.present() ? c->output : c->token_embd;
-        CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(n), dim3(256), 0, (const float*)X, c->output_norm.f32(), d.norm_eps, XNh, H));
-        UmmaParams hp{};
-        hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = d.vocab; hp.K = H;
-        hp.x = XNh; hp.ldx = H; hp.T = n; hp.y = c->pf_logits; hp.ldy = d.vocab; hp.err = c->mma_err; hp.pdl = pdl ? 1 : 0;
-        umma_set_tmap(c, hp);
-        CU(gemm_dispatch(hp, c->n_sm, st));
+        if (!head_done) {
+            CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(n), dim3(256), 0, (const float*)X, c->output_norm.f32(), d.norm_eps, XNh, H));
+            UmmaParams hp{};
+            hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = d.vocab; hp.K = H;
+            hp.x = XNh; hp.ldx = H; hp.T = n; hp.y = c->pf_logits; hp.ldy = d.vocab; hp.err = c->mma_err; hp.pdl = pdl ? 1 : 0;
+            umma_set_tmap(c, hp);
+            CU(gemm_dispatch(hp, c->n_sm, st));
+        }
         c->launches += 3;
         if (capg.on) {
             capg.on = false;
