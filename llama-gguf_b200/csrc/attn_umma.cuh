@@ -150,24 +150,32 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
     long long waited = 0;
 
     if (warp == kAttnLoader) {
-        if (lane == 0) {
+        {
             int asked_k = 0, asked_v = 0;
             for (int j = 0; j < nt; j++) {
                 const uint32_t b = j & 1, ph = ((j >> 1) & 1) ^ 1;
                 u2_wait(k_empty + 8u * b, ph, alive, p.err, 21, waited);
+                alive = __all_sync(0xffffffffu, alive);
                 if (!alive) break;
-                u2_expect_tx(k_full + 8u * b, (uint32_t)(2 * SM::K));
+                if (u2_elect()) {
+                    u2_expect_tx(k_full + 8u * b, (uint32_t)(2 * SM::K));
 #pragma unroll
-                for (int h = 0; h < 2; h++)
+                    for (int h = 0; h < 2; h++)
 #pragma unroll
-                    for (int s = 0; s < NS; s++)
-                        u2_tma_2d(base + SM::K_AT + (2 * b + h) * SM::K + s * (kAttnTK * 128), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, k_full + 8u * b);
+                        for (int s = 0; s < NS; s++)
+                            u2_tma_2d(base + SM::K_AT + (2 * b + h) * SM::K + s * (kAttnTK * 128), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, k_full + 8u * b);
+                }
+                __syncwarp();
                 asked_k = j + 1;
                 u2_wait(v_empty + 8u * b, ph, alive, p.err, 22, waited);
+                alive = __all_sync(0xffffffffu, alive);
                 if (!alive) break;
-                u2_expect_tx(v_full + 8u * b, (uint32_t)(2 * SM::V));
+                if (u2_elect()) {
+                    u2_expect_tx(v_full + 8u * b, (uint32_t)(2 * SM::V));
 #pragma unroll
-                for (int h = 0; h < 2; h++) u2_tma_2d(base + SM::V_AT + (2 * b + h) * SM::V, &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, v_full + 8u * b);
+                    for (int h = 0; h < 2; h++) u2_tma_2d(base + SM::V_AT + (2 * b + h) * SM::V, &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, v_full + 8u * b);
+                }
+                __syncwarp();
                 asked_v = j + 1;
             }
             if (!alive) {                           // gave up: what has been asked for lands first (bounded)
@@ -182,7 +190,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
             }
         }
     } else if (warp == kAttnMma) {
-        if (lane == 0) {
+        {
             const uint32_t idS = umma_idesc(128, kAttnTK), idO = umma_idesc(128, HD);
             const uint64_t dQ = umma_desc(base), dP = umma_desc(base + SM::P_AT);
             auto scores = [&](int j) {              // S = Q_hi K_hi^T + Q_lo K_hi^T + Q_hi K_lo^T
@@ -191,7 +199,9 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
                 u2_wait(s_empty + 8u * b, ph ^ 1u, alive, p.err, 24, waited);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t dK = umma_desc(base + SM::K_AT + 2 * b * SM::K);
-                if (alive) {
+                alive = __all_sync(0xffffffffu, alive);
+                const bool lead = u2_elect();
+                if (lead && alive) {
 #pragma unroll
                     for (int t = 0; t < 3; t++) {
                         const uint64_t da = dQ + (t == 1 ? SM::Q / 16 : 0), db = dK + (t == 2 ? SM::K / 16 : 0);
@@ -203,8 +213,11 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
                                          (t > 0 || s > 0 || kk > 0) ? 1u : 0u);
                     }
                 }
-                umma_commit(k_empty + 8u * b);
-                umma_commit(s_full + 8u * b);
+                if (lead) {
+                    umma_commit(k_empty + 8u * b);
+                    umma_commit(s_full + 8u * b);
+                }
+                __syncwarp();
             };
             u2_wait(q_full, 0, alive, p.err, 25, waited);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -216,7 +229,9 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
                 u2_wait(p_full, j & 1, alive, p.err, 27, waited);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t dV = umma_desc(base + SM::V_AT + 2 * b * SM::V);
-                if (alive) {                        // O += P_hi V_hi + P_lo V_hi + P_hi V_lo
+                alive = __all_sync(0xffffffffu, alive);
+                const bool lead = u2_elect();
+                if (lead && alive) {                // O += P_hi V_hi + P_lo V_hi + P_hi V_lo
 #pragma unroll
                     for (int t = 0; t < 3; t++) {
                         const uint64_t da = dP + (t == 1 ? SM::P / 16 : 0), db = dV + (t == 2 ? SM::V / 16 : 0);
@@ -224,8 +239,11 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
                         for (int kk = 0; kk < kAttnTK / 16; kk++) umma_f16(tO, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), idO, (j > 0 || t > 0 || kk > 0) ? 1u : 0u);
                     }
                 }
-                umma_commit(v_empty + 8u * b);
-                umma_commit(pv_done);
+                if (lead) {
+                    umma_commit(v_empty + 8u * b);
+                    umma_commit(pv_done);
+                }
+                __syncwarp();
             }
         }
     } else {

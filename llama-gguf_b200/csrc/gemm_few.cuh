@@ -320,11 +320,6 @@ __device__ __forceinline__ void few_mma_tf32(uint32_t acc, uint32_t a, uint64_t 
                  "r"(accumulate)
                  : "memory");
 }
-__device__ __forceinline__ bool few_elect() {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
-    return ok != 0;
-}
 __device__ __forceinline__ void few_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
@@ -433,7 +428,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) few_gemm_kernel(const __grid_c
                 few_wait(b_re + 8u * rr.i, rr.ph ^ 1u, alive, p.err, 31);
                 alive = __all_sync(0xffffffffu, alive);
                 if (!alive) return;
-                if (few_elect()) {
+                if (u2_elect()) {
                     u2_expect_tx(b_rf + 8u * rr.i, (uint32_t)(sg.pitch * 128));
                     u2_tma_2d(umma_smem_u32(sR) + rr.i * (uint32_t)p.raw_stage, sg.map, (((int)cr.blk * sg.block_bytes) & ~15) >> 2, (cr.m - pl.tile0[cr.s]) * 128, b_rf + 8u * rr.i);
                 }
@@ -448,7 +443,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) few_gemm_kernel(const __grid_c
                 few_wait(b_be + 8u * rb.i, rb.ph ^ 1u, alive, p.err, 32);
                 alive = __all_sync(0xffffffffu, alive);
                 if (!alive) break;
-                if (few_elect()) {
+                if (u2_elect()) {
                     u2_expect_tx(b_bf + 8u * rb.i, kStageB);
                     few_bulk(umma_smem_u32(sB) + rb.i * kStageB, p.image + ((size_t)cb.nt * nblk + cb.blk) * kStageB, kStageB, b_bf + 8u * rb.i);
                 }
@@ -483,7 +478,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) few_gemm_kernel(const __grid_c
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a = tmem + g * kA, acc = tmem + kS + g * N;
                 const uint64_t db = db0 + (uint64_t)(rb.i * (kStageB / 16));
-                if (few_elect()) {
+                if (u2_elect()) {
     #pragma unroll
                     for (int kk = 0; kk < 16; kk++)
                         few_mma_f16(acc, a + 8u * kk, db + (uint64_t)((kk >> 2) * (kSlab / 16) + 2 * (kk & 3)), idesc, kk > 0 ? 1u : 0u);

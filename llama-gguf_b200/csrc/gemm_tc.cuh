@@ -56,6 +56,13 @@ __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, bool& ali
         }
     }
 }
+// One lane of a converged warp.  The warps that issue copies and MMAs run their loops whole and elect a lane at the issue: the operands are uniform registers, and
+// with a branch on the lane around the loop each of them was moved there by itself (an MMA every 45 clocks at best, whatever its size; 14 like this).
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
 __device__ __forceinline__ void tc_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -209,34 +216,38 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     TcWalk<TN> walk;
     TcTile t;
     if (warp == TC_LOAD_W || warp == TC_LOAD_X) {
-        if (lane == 0) {
-            uint32_t s = 0, ph = 1;
-            for (int item = blockIdx.x; alive && walk.find(a, n_mt, item, t); item += gridDim.x)
-                for (int k = 0; k < steps; k++) {
-                    tc_wait(empty + 8u * s, ph, alive, a.err, 1);
-                    if (!alive) break;
+        uint32_t s = 0, ph = 1;
+        for (int item = blockIdx.x; alive && walk.find(a, n_mt, item, t); item += gridDim.x)
+            for (int k = 0; k < steps; k++) {
+                tc_wait(empty + 8u * s, ph, alive, a.err, 1);
+                alive = __all_sync(0xffffffffu, alive);
+                if (!alive) break;
+                if (tc_elect()) {
                     if (warp == TC_LOAD_W) tc_load<TN, GLU, true>(ring + s * STAGE, &wmap, a, t, k * KS, full + 8u * s);
                     else tc_load<TN, GLU, false>(ring + s * STAGE, &xmap, a, t, k * KS, full + 8u * s);
-                    if (++s == NS) { s = 0; ph ^= 1u; }
                 }
-            if (!alive) tc_drain<NS>(full, s, ph);
-        }
+                __syncwarp();
+                if (++s == NS) { s = 0; ph ^= 1u; }
+            }
+        if (!alive) tc_drain<NS>(full, s, ph);
     } else if (warp == TC_MMA) {
-        if (lane == 0) {
-            const uint32_t idesc = tc_idesc(TC_M, TN);
-            uint32_t s = 0, ph = 0, it = 0;
-            for (int item = blockIdx.x; walk.find(a, n_mt, item, t); item += gridDim.x, it++) {
-                const uint32_t buf = it & 1u;
-                tc_wait(acc_empty + 8u * buf, ((it >> 1) & 1u) ^ 1u, alive, a.err, 2);
+        const uint32_t idesc = tc_idesc(TC_M, TN);
+        uint32_t s = 0, ph = 0, it = 0;
+        for (int item = blockIdx.x; walk.find(a, n_mt, item, t); item += gridDim.x, it++) {
+            const uint32_t buf = it & 1u;
+            tc_wait(acc_empty + 8u * buf, ((it >> 1) & 1u) ^ 1u, alive, a.err, 2);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int k = 0; k < steps; k++) {
+                tc_wait(full + 8u * s, ph, alive, a.err, 3);
+                alive = __all_sync(0xffffffffu, alive);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int k = 0; k < steps; k++) {
-                    tc_wait(full + 8u * s, ph, alive, a.err, 3);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (tc_elect()) {
                     if (alive) tc_mma_stage<TN>(tmem + buf * TN, ring + s * STAGE, idesc, k == 0);
                     tc_commit(empty + 8u * s);
-                    if (++s == NS) { s = 0; ph ^= 1u; }
+                    if (k == steps - 1) tc_commit(acc_full + 8u * buf);
                 }
-                tc_commit(acc_full + 8u * buf);
+                __syncwarp();
+                if (++s == NS) { s = 0; ph ^= 1u; }
             }
         }
     } else {
@@ -358,29 +369,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int all = (a.K + KS - 1) / KS, k_beg = rank * all / S, k_end = (rank + 1) * all / S;      // (S <= all)
     bool alive = true;
     if (warp == TC_LOAD_W || warp == TC_LOAD_X) {
-        if (lane == 0) {
-            uint32_t s = 0, ph = 1;
-            for (int k = k_beg; k < k_end; k++) {
-                tc_wait(empty + 8u * s, ph, alive, a.err, 1);
-                if (!alive) break;
+        uint32_t s = 0, ph = 1;
+        for (int k = k_beg; k < k_end; k++) {
+            tc_wait(empty + 8u * s, ph, alive, a.err, 1);
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            if (tc_elect()) {
                 if (warp == TC_LOAD_W) tc_load<TN, GLU, true>(ring + s * STAGE, &wmap, a, t, k * KS, full + 8u * s);
                 else tc_load<TN, GLU, false>(ring + s * STAGE, &xmap, a, t, k * KS, full + 8u * s);
-                if (++s == NS) { s = 0; ph ^= 1u; }
             }
-            if (!alive) tc_drain<NS>(full, s, ph);
+            __syncwarp();
+            if (++s == NS) { s = 0; ph ^= 1u; }
         }
+        if (!alive) tc_drain<NS>(full, s, ph);
     } else if (warp == TC_MMA) {
-        if (lane == 0) {
-            const uint32_t idesc = tc_idesc(TC_M, TN);
-            uint32_t s = 0, ph = 0;
-            for (int k = k_beg; k < k_end; k++) {
-                tc_wait(full + 8u * s, ph, alive, a.err, 3);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t idesc = tc_idesc(TC_M, TN);
+        uint32_t s = 0, ph = 0;
+        for (int k = k_beg; k < k_end; k++) {
+            tc_wait(full + 8u * s, ph, alive, a.err, 3);
+            alive = __all_sync(0xffffffffu, alive);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (tc_elect()) {
                 if (alive) tc_mma_stage<TN>(tmem, ring + s * STAGE, idesc, k == k_beg);
                 tc_commit(empty + 8u * s);
-                if (++s == NS) { s = 0; ph ^= 1u; }
+                if (k == k_end - 1) tc_commit(acc_full);
             }
-            tc_commit(acc_full);
+            __syncwarp();
+            if (++s == NS) { s = 0; ph ^= 1u; }
         }
     }
     __syncwarp();

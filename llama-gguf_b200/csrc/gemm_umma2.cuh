@@ -55,6 +55,12 @@ __device__ __forceinline__ void u2_mbar_arrive(uint32_t bar) { asm volatile("mba
 __device__ __forceinline__ void u2_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// one lane of a converged warp
+__device__ __forceinline__ bool u2_elect() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
 __device__ __forceinline__ void u2_tma_2d(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(tmap), "r"(c0), "r"(c1), "r"(bar)
