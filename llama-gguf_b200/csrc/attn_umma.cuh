@@ -45,6 +45,8 @@ struct AttnUmmaParams {
 template <int HD>
 __global__ void __launch_bounds__(256) prefill_kv16_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int max_seq, int kv_end, int P,
                                                            __half* __restrict__ k16, __half* __restrict__ vt16) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ __half tile[64][HD + 2], tile_lo[64][HD + 2];
     const int kh = blockIdx.y, n_kv = gridDim.y, p0 = blockIdx.x * 64;
     const float* ks = kc + (size_t)kh * max_seq * HD;
@@ -108,6 +110,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
     extern __shared__ __align__(1024) uint8_t au_smem[];
     using SM = AttnUmmaSmem<HD>;
     constexpr int NS = HD / 64;                     // 64-element slabs along hd
+    pdl_launch_dependents();
     const uint32_t base = umma_smem_u32(au_smem);
     if (base & 1023u) {                             // the swizzle is on absolute address bits (there is no static shared memory in front)
         if (threadIdx.x == 0 && p.err) atomicExch(p.err, 20);
@@ -146,6 +149,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(s_tmem));
     const uint32_t tO = tmem + 128u;                // S: columns 0..63 and 64..127, O: 128..128+HD-1
     const int nt = (p.pos0 + min(t0 + TQ, p.T) + kAttnTK - 1) / kAttnTK;     // key tiles that the block's queries see
+    pdl_wait();
     bool alive = true;
     long long waited = 0;
 
@@ -407,7 +411,7 @@ inline bool attn_umma_ok(int hd, int n_heads, int n_kv) {
 }
 
 template <int HD>
-inline cudaError_t attn_umma_launch_hd(const CUtensorMap& kmap, const CUtensorMap& vmap, const AttnUmmaParams& p, cudaStream_t st) {
+inline cudaError_t attn_umma_launch_hd(const CUtensorMap& kmap, const CUtensorMap& vmap, const AttnUmmaParams& p, bool pdl, cudaStream_t st) {
     static bool once[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -418,8 +422,14 @@ inline cudaError_t attn_umma_launch_hd(const CUtensorMap& kmap, const CUtensorMa
     }
     const int TQ = 128 / p.G;
     dim3 grid((p.T + TQ - 1) / TQ, p.n_kv);
-    prefill_attn_umma_kernel<HD><<<grid, kAttnTcThreads, AttnUmmaSmem<HD>::BYTES, st>>>(kmap, vmap, p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = dim3(kAttnTcThreads); cfg.dynamicSmemBytes = AttnUmmaSmem<HD>::BYTES; cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, prefill_attn_umma_kernel<HD>, kmap, vmap, p);
 }
 
 }  // namespace b200

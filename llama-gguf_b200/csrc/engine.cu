@@ -249,6 +249,7 @@ struct b200_ctx {
     struct BatchGraph { cudaGraphExec_t exec = nullptr; uint64_t launches = 0; bool warm = false; };
     std::vector<BatchGraph> batch_graphs;
     bool batch_graph = true;
+    bool prompt_pdl = true;           // prompts: programmatic launches between the kernels of a chunk (B200_PROMPT_PDL=0: plain)
     bool batch_pdl = true;            // ... with programmatic dependent launches between its kernels (B200_BATCH_PDL=0: plain edges)
     float* h_batch_logits = nullptr; // pinned staging of b200_decode_batch's n x vocab logits
     size_t h_batch_logits_bytes = 0;
@@ -366,6 +367,7 @@ extern "C" int b200_ctx_create(const b200_model_desc* desc, const b200_parallel_
     c->batch_gemm_min = std::max(2, env_int("B200_BATCH_GEMM_MIN", 8));
     c->batch_graph = env_int("B200_BATCH_GRAPH", 1) != 0;
     c->batch_pdl = env_int("B200_BATCH_PDL", 1) != 0;
+    c->prompt_pdl = env_int("B200_PROMPT_PDL", 1) != 0;
     c->mma_warps = std::max(4, std::min(kMmaMaxWarps, env_int("B200_MMA_WARPS", 16)));
     c->mma_stages = std::max(2, std::min(kMmaMaxStages, env_int("B200_MMA_STAGES", 3)));
     c->smem_optin = (size_t)prop.sharedMemPerBlockOptin;
@@ -2002,7 +2004,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     __half* Hh = ATh + (size_t)cap * A;                 // [T][I] silu(gate) * up, fp16
     const size_t kv_layer = (size_t)2 * nkv * d.max_seq_len * hd;
     cudaStream_t st = c->stream;
-    const bool pdl = rows && c->batch_pdl;   // batched decode: programmatic dependent launches along the whole chain
+    const bool pdl = rows ? c->batch_pdl : c->prompt_pdl;   // programmatic dependent launches along the whole chain
     auto gemm = [&](const DevTensor& w, int K, const __half* x, int ldx, int T, float* y, int ldy, const DevTensor* bias, int acc) -> cudaError_t {
         UmmaParams p{};
         p.w = w.d; p.row_bytes = w.row_bytes; p.type = w.type; p.n_rows = (int)w.ne[1]; p.K = K;
@@ -2033,15 +2035,16 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 const long long lo = glu ? at : std::max(at, first), hi = glu ? at + rows_n : std::min(at + rows_n, first + (long long)w->ne[1]);
                 if (lo < hi) {
                     const int nr = (int)(hi - lo);
-                    rows_to_f16_kernel<<<dim3((K / 8 + 255) / 256, (nr + F16_ROWS - 1) / F16_ROWS), 256, 0, st>>>(w->type, (const uint8_t*)w->d + (lo - (glu ? 0 : first)) * w->row_bytes,
-                                                                                                                w->row_bytes, nr, K, c->pf_w16 + put);
+                    const cudaError_t e = launch_on(st, pdl, rows_to_f16_kernel, dim3((K / 8 + 255) / 256, (nr + F16_ROWS - 1) / F16_ROWS), dim3(256), 0, w->type,
+                                                    (const uint8_t*)w->d + (lo - (glu ? 0 : first)) * w->row_bytes, (long long)w->row_bytes, nr, K, c->pf_w16 + put);
+                    if (e != cudaSuccess) return e;
                     c->launches++;
                     put += (size_t)nr * K;
                 }
                 if (!glu) first += (long long)w->ne[1];
             }
             void* yt = glu ? (void*)((__half*)y + at) : (void*)((float*)y + at);
-            const cudaError_t e = f16_maps ? tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, st) : cudaErrorNotSupported;
+            const cudaError_t e = f16_maps ? tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, pdl, st) : cudaErrorNotSupported;
             if (e != cudaSuccess) return e == cudaErrorNotSupported && at > 0 ? cudaErrorInvalidValue : e;
             c->launches++;
         }
@@ -2082,7 +2085,6 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         return gemm(w, K, x, ldx, T, y, ldy, bias, acc);
     };
     bool few = false, head_done = false;
-    const bool few_pdl = rows && c->batch_pdl;
     int last_T = 0;
     for (int done = 0; done < n; done += cap) {
         const int T = std::min(cap, n - done);
@@ -2095,7 +2097,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         FewOut sum{};                                   // product that X still lacks (of the layer before)
         bool has_sum = false;
         auto few_norm = [&](const float* w, uint8_t* img) {
-            const cudaError_t e = launch_on(st, few_pdl, few_norm_kernel, dim3(T), dim3(H / 8), 0, X, sum, has_sum ? 1 : 0, w, d.norm_eps, img, few_n(T), H);
+            const cudaError_t e = launch_on(st, pdl, few_norm_kernel, dim3(T), dim3(H / 8), 0, X, sum, has_sum ? 1 : 0, w, d.norm_eps, img, few_n(T), H);
             has_sum = false;
             c->launches++;
             return e;
@@ -2121,7 +2123,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             out.plan = a.plan; out.part = a.part; out.N = few_n(T);
             for (int s = 0; s < n_seg; s++) { out.y[s] = a.seg[s].y; out.ldy[s] = ldy; }
             c->launches++;
-            return few_launch(a, few_pdl, st);
+            return few_launch(a, pdl, st);
         };
         for (int l = 0; few && l < d.n_layers; l++) {
             Layer& L = c->layers[l];
@@ -2140,13 +2142,13 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 for (int s = 0; s < 3; s++) fa.bias[s] = ra.bias[s];
                 fa.rope_scale = d.rope_scale; fa.scale = scale; fa.row_pos = d_pos; fa.row_kv = d_kv;
                 fa.k_off = (long long)((size_t)l * kv_layer); fa.v_off = fa.k_off + (long long)(kv_layer / 2); fa.img = c->few_img[1];
-                CU(launch_on(st, few_pdl, hd == 128 ? (Gq <= 4 ? few_attn_kernel<128, 4> : few_attn_kernel<128, 8>) : (Gq <= 4 ? few_attn_kernel<64, 4> : few_attn_kernel<64, 8>),
+                CU(launch_on(st, pdl, hd == 128 ? (Gq <= 4 ? few_attn_kernel<128, 4> : few_attn_kernel<128, 8>) : (Gq <= 4 ? few_attn_kernel<64, 4> : few_attn_kernel<64, 8>),
                              dim3(nkv, T), dim3(256), 0, fa));
             } else {
                 PrefillRopeParams& rp = ra.p;
                 rp.qkv = Q; rp.ld = QKV; rp.k_cache = kc; rp.v_cache = vc; rp.freq = c->rope_freq; rp.pos0 = pos0;
                 rp.n_heads = nh; rp.n_kv = nkv; rp.hd = hd; rp.max_seq = d.max_seq_len; rp.neox = d.rope_neox; rp.rope_scale = d.rope_scale;
-                few_rope_kv_kernel<<<dim3(T, 4), 256, 0, st>>>(ra);
+                CU(launch_on(st, pdl, few_rope_kv_kernel, dim3(T, 4), dim3(256), 0, ra));
                 if (attn_tc) {
                     const int kv_end = pos0 + T, kv_pad = (kv_end + 127) & ~127;
                     AttnUmmaParams up{};
@@ -2154,11 +2156,11 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                     up.P = c->pf_kv16_P; up.scale = scale; up.err = c->mma_err;
                     const dim3 kgrid(kv_pad / 64, nkv);
                     if (hd == 128) {
-                        prefill_kv16_kernel<128><<<kgrid, 256, 0, st>>>(kc, vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
-                        CU(attn_umma_launch_hd<128>(c->pf_kmap, c->pf_vmap, up, st));
+                        CU(launch_on(st, pdl, prefill_kv16_kernel<128>, kgrid, dim3(256), 0, (const float*)kc, (const float*)vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16));
+                        CU(attn_umma_launch_hd<128>(c->pf_kmap, c->pf_vmap, up, pdl, st));
                     } else {
-                        prefill_kv16_kernel<64><<<kgrid, 256, 0, st>>>(kc, vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
-                        CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, st));
+                        CU(launch_on(st, pdl, prefill_kv16_kernel<64>, kgrid, dim3(256), 0, (const float*)kc, (const float*)vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16));
+                        CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, pdl, st));
                     }
                     c->launches += 2;
                 } else {
@@ -2166,11 +2168,11 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                     ap.qkv = Q; ap.ld = QKV; ap.k_cache = kc; ap.v_cache = vc; ap.out = ATh; ap.ldo = A; ap.pos0 = pos0; ap.T = T;
                     ap.n_heads = nh; ap.n_kv = nkv; ap.max_seq = d.max_seq_len; ap.scale = scale;
                     const int ablocks = (int)(((long long)T * nkv * 32 + 127) / 128);
-                    CU(launch_on(st, false, hd == 128 ? (Gq <= 4 ? prefill_attn_kernel<128, 4> : prefill_attn_kernel<128, 8>) : (Gq <= 4 ? prefill_attn_kernel<64, 4> : prefill_attn_kernel<64, 8>),
+                    CU(launch_on(st, pdl, hd == 128 ? (Gq <= 4 ? prefill_attn_kernel<128, 4> : prefill_attn_kernel<128, 8>) : (Gq <= 4 ? prefill_attn_kernel<64, 4> : prefill_attn_kernel<64, 8>),
                                  dim3(ablocks), dim3(128), 0, ap));
                     c->launches++;
                 }
-                few_image_kernel<<<dim3((A / 8 + 255) / 256, T), 256, 0, st>>>(ATh, A, c->few_img[1], few_n(T), A);
+                CU(launch_on(st, pdl, few_image_kernel, dim3((A / 8 + 255) / 256, T), dim3(256), 0, (const __half*)ATh, A, c->few_img[1], few_n(T), A));
                 c->launches++;
             }
             CU(few_product({&L.wo}, A, c->few_img[1], {G}, H, sum));
@@ -2178,7 +2180,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             CU(few_norm(L.ffn_norm.f32(), c->few_img[0]));
             FewOut gu{};
             CU(few_product({&L.gate, &L.up}, H, c->few_img[0], {G, U}, I, gu));
-            CU(launch_on(st, few_pdl, few_swiglu_kernel, dim3((I / 8 + 255) / 256, T), dim3(256), 0, gu, c->few_img[2], I));
+            CU(launch_on(st, pdl, few_swiglu_kernel, dim3((I / 8 + 255) / 256, T), dim3(256), 0, gu, c->few_img[2], I));
             CU(few_product({&L.down}, I, c->few_img[2], {G}, H, sum));
             has_sum = true;
             c->launches += 2;
@@ -2190,7 +2192,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             if (head_done) {
                 FewOut lg{};
                 CU(few_product({&head}, H, c->few_img[0], {c->pf_logits}, d.vocab, lg));
-                CU(launch_on(st, few_pdl, few_finish_kernel, dim3((d.vocab + 127) / 128, (T + 7) / 8), dim3(128), 0, lg, c->pf_logits, d.vocab));
+                CU(launch_on(st, pdl, few_finish_kernel, dim3((d.vocab + 127) / 128, (T + 7) / 8), dim3(128), 0, lg, c->pf_logits, d.vocab));
             }
         }
         for (int l = 0; !few && l < d.n_layers; l++) {
@@ -2236,12 +2238,12 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 const dim3 kgrid(kv_pad / 64, nkv);
                 if (hd == 128) {
                     if (q8) prefill_kv16_q8_kernel<128><<<kgrid, 256, 0, st>>>(k8, v8, k8s, v8s, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
-                    else prefill_kv16_kernel<128><<<kgrid, 256, 0, st>>>(kc, vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
-                    CU(attn_umma_launch_hd<128>(c->pf_kmap, c->pf_vmap, up, st));
+                    else CU(launch_on(st, pdl, prefill_kv16_kernel<128>, kgrid, dim3(256), 0, (const float*)kc, (const float*)vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16));
+                    CU(attn_umma_launch_hd<128>(c->pf_kmap, c->pf_vmap, up, pdl, st));
                 } else {
                     if (q8) prefill_kv16_q8_kernel<64><<<kgrid, 256, 0, st>>>(k8, v8, k8s, v8s, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
-                    else prefill_kv16_kernel<64><<<kgrid, 256, 0, st>>>(kc, vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16);
-                    CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, st));
+                    else CU(launch_on(st, pdl, prefill_kv16_kernel<64>, kgrid, dim3(256), 0, (const float*)kc, (const float*)vc, d.max_seq_len, kv_end, c->pf_kv16_P, c->pf_k16, c->pf_vt16));
+                    CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, pdl, st));
                 }
                 c->launches += 1;
             } else {
@@ -2301,7 +2303,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         }
         return B200_OK;
     }
-    prefill_advance_kernel<<<1, 32, 0, st>>>(sl.d_state, n);
+    CU(launch_on(st, pdl, prefill_advance_kernel, dim3(1), dim3(32), 0, sl.d_state, n));
     if (want_logits) {   // final RMSNorm + vocab head of the last token, through the exact GEMV path
         CU(cudaMemcpyAsync(c->xa, X + (size_t)(last_T - 1) * H, (size_t)H * sizeof(float), cudaMemcpyDeviceToDevice, st));
         GemvParams p{};

@@ -1,5 +1,5 @@
 // gemm_tc.cuh — 16-bit products of many rows on the 5th-generation tensor cores.  Included by layerprog.cu (bf16) and engine.cu (fp16), each
-// inside a namespace that has defined: next_grid / wait_grid (programmatic launches; empty where there are none), tc_t (the operand type), TC_BF16 (whether it is bfloat16), the epilogues EPI_STORE, EPI_ADD, ... with
+// inside a namespace that has defined: next_grid / wait_grid (programmatic launches; empty where there are none), tc_t (the operand type), TC_BF16 (whether it is bfloat16), TC_W_WAITS (whether the kernel before writes the weight rows), the epilogues EPI_STORE, EPI_ADD, ... with
 // epi_is_glu, epi_is_act, seg_rows<T, EPI>, epi_store<T, EPI> and glu_fast<EPI>, and from_f<T>.
 //
 // Y[t][n] = epi(alpha * sum_k X[t][k] W[n][k] + bias[n]).  A tile is TC_M = 128 weight rows (the M of tcgen05.mma) by TN tokens (its N); its
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * NS, acc_full = bar + 16u * NS, acc_empty = acc_full + 16u;
     tc_setup(tid, warp, bar, NS, &s_tmem, 2, 2 * TN);
-    if (a.seg || warp != TC_LOAD_W) wait_grid();          // (weights do not depend on the kernel before)
+    if (TC_W_WAITS || a.seg || warp != TC_LOAD_W) wait_grid();      // (other weights do not depend on the kernel before)
     const uint32_t tmem = s_tmem, ring = smem_u32(base);
     const int steps = (a.K + KS - 1) / KS, n_mt = (a.N + (GLU ? TC_M / 2 : TC_M) - 1) / (GLU ? TC_M / 2 : TC_M);
     bool alive = true;
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * NS, acc_full = bar + 16u * NS;
     tc_setup(tid, warp, bar, NS, &s_tmem, 1, TN);
-    if (!a.seg && warp != TC_LOAD_W) wait_grid();         // (weights do not depend on the kernel before)
+    if (!a.seg && (TC_W_WAITS || warp != TC_LOAD_W)) wait_grid();   // (other weights do not depend on the kernel before)
     const uint32_t tmem = s_tmem, ring = smem_u32(base);
     const int all = (a.K + KS - 1) / KS, k_beg = rank * all / S, k_end = (rank + 1) * all / S;      // (S <= all)
     bool alive = true;

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(256) lp_gemm_kernel(const T* __restrict__ X, i
 
 // ------------------------------------------------------------------------------------------------ GEMM (tcgen05 / TMEM, bf16)
 using tc_t = bf16;
-constexpr bool TC_BF16 = true;
+constexpr bool TC_BF16 = true, TC_W_WAITS = false;
 #include "gemm_tc.cuh"
 
 // Few rows (decoding): one warp per output column, the weight row is read once with 16-byte loads and meets up to GV_ROWS

@@ -272,6 +272,8 @@ __global__ void prefill_swiglu_kernel(const float* __restrict__ g, const float* 
 
 // the slot's position after T more tokens
 __global__ void prefill_advance_kernel(SeqState* st, int T) {
+    pdl_launch_dependents();
+    pdl_wait();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         st->pos_cur = st->pos_next + T - 1;
         st->pos_next = st->pos_next + T;

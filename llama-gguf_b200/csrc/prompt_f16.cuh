@@ -41,9 +41,10 @@ __device__ __forceinline__ uint4 f16_deq8_q4k(const uint8_t* row, int k0, int c)
 }
 
 // rows x K elements -> fp16 [rows][K].  A thread unpacks one chunk of 8 in F16_ROWS rows (independent loads in flight); bound by DRAM: 0.56 to
-// 1.06 bytes in, 2 out per element.
+// 1.06 bytes in, 2 out per element.  The blocks are read and unpacked before the wait for the kernel before (a product that may still read the scratch rows).
 constexpr int F16_ROWS = 4;
 __global__ void __launch_bounds__(256) rows_to_f16_kernel(int type, const uint8_t* __restrict__ w, long long row_bytes, int rows, int K, __half* __restrict__ out) {
+    pdl_launch_dependents();
     const int ch = blockIdx.x * 256 + threadIdx.x;
     if (ch * 8 >= K) return;
     const int k0 = (ch * 8) & ~63, c = ch & 7, r0 = blockIdx.y * F16_ROWS;
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(int type, const uint8_
 #pragma unroll
         for (int u = 0; u < F16_ROWS; u++) v[u] = umma_deq8<false>(type, w + (long long)min(r0 + u, rows - 1) * row_bytes, k0, c);
     }
+    pdl_wait();
 #pragma unroll
     for (int u = 0; u < F16_ROWS; u++)
         if (r0 + u < rows) *reinterpret_cast<uint4*>(out + (size_t)(r0 + u) * K + ch * 8) = v[u];
@@ -62,9 +64,9 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(int type, const uint8_
 
 namespace tc16 {
 using tc_t = __half;
-constexpr bool TC_BF16 = false;
-__device__ __forceinline__ void next_grid() {}      // (plain launches)
-__device__ __forceinline__ void wait_grid() {}
+constexpr bool TC_BF16 = false, TC_W_WAITS = true;
+__device__ __forceinline__ void next_grid() { pdl_launch_dependents(); }
+__device__ __forceinline__ void wait_grid() { pdl_wait(); }
 enum { EPI_STORE = 0, EPI_ADD = 1, EPI_SILU_GLU = 2 };
 constexpr bool epi_is_glu(int epi) { return epi == EPI_SILU_GLU; }
 constexpr bool epi_is_act(int epi) { return epi == EPI_SILU_GLU; }
@@ -82,7 +84,7 @@ template <typename T, int EPI> __device__ __forceinline__ void* seg_rows(void* Y
 #include "gemm_tc.cuh"
 
 template <int TN, bool PERSISTENT, int EPI>
-cudaError_t launch_as(const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid, cudaStream_t st) {
+cudaError_t launch_as(const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid, bool pdl, cudaStream_t st) {
     constexpr size_t smem = tc_smem_bytes<TN, PERSISTENT>(epi_is_glu(EPI));
     auto kern = PERSISTENT ? lp_gemm_tc_kernel<TN, EPI> : lp_gemm_tc_split_kernel<(TN > 128 ? 128 : TN), EPI>;
     static bool once[64] = {};
@@ -98,33 +100,41 @@ cudaError_t launch_as(const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)a.splits;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (pdl) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (!PERSISTENT && a.splits > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)a.splits;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        n++;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = !PERSISTENT && a.splits > 1 ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kern, xm, wm, a);
 }
-template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, cudaStream_t st) {
+template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, bool pdl, cudaStream_t st) {
     const int per = epi_is_glu(EPI) ? TC_M / 2 : TC_M, n_mt = (a.N + per - 1) / per, n_nt = (a.R + pl.tn - 1) / pl.tn;
     if (pl.persistent) {
         const dim3 grid(n_mt * n_nt < 148 ? n_mt * n_nt : 148);
-        return pl.tn == 256 ? launch_as<256, true, EPI>(xm, wm, a, grid, st) : launch_as<128, true, EPI>(xm, wm, a, grid, st);
+        return pl.tn == 256 ? launch_as<256, true, EPI>(xm, wm, a, grid, pdl, st) : launch_as<128, true, EPI>(xm, wm, a, grid, pdl, st);
     }
     const dim3 grid(n_mt * pl.splits, n_nt);
-    return pl.tn == 128 ? launch_as<128, false, EPI>(xm, wm, a, grid, st) : launch_as<64, false, EPI>(xm, wm, a, grid, st);
+    return pl.tn == 128 ? launch_as<128, false, EPI>(xm, wm, a, grid, pdl, st) : launch_as<64, false, EPI>(xm, wm, a, grid, pdl, st);
 }
 // Y[t][n] = epi(sum_k x[t][k] w[n][k] + bias[n]), T rows, N outputs (EPI_SILU_GLU: N units from the 2 N rows [gate | up] of w, fp16 Y).
 // cudaErrorNotSupported: a tensor map was refused, nothing was launched
-inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, cudaStream_t st) {
+inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, bool pdl, cudaStream_t st) {
     const bool glu = epi_is_glu(epi);
     const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu, true);
     const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     CUtensorMap xm, wm;
     if (!tc_map(&xm, x, K, T, ldx, 1, 1, 0, pl.tn, kh) || !tc_map(&wm, w, K, N, K, glu ? 2 : 1, 1, 0, glu ? TC_M / 2 : TC_M, kh)) return cudaErrorNotSupported;
     const TcArgs a{y, ldy, T, N, K, 1.0f, err, nullptr, 1, 0, 0, bias, float2{0.0f, 0.0f}, pl.splits, K % TC_K == 0 ? 1 : 0};
-    return epi == EPI_STORE ? launch_epi<EPI_STORE>(pl, xm, wm, a, st) : epi == EPI_ADD ? launch_epi<EPI_ADD>(pl, xm, wm, a, st) : launch_epi<EPI_SILU_GLU>(pl, xm, wm, a, st);
+    return epi == EPI_STORE ? launch_epi<EPI_STORE>(pl, xm, wm, a, pdl, st) : epi == EPI_ADD ? launch_epi<EPI_ADD>(pl, xm, wm, a, pdl, st) : launch_epi<EPI_SILU_GLU>(pl, xm, wm, a, pdl, st);
 }
 }  // namespace tc16
 }  // namespace b200
