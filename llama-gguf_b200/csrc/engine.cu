@@ -803,7 +803,7 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         CU_ALLOC(cudaMalloc((void**)&c->attn_q8_part, (size_t)nkv * c->attn_q8_splits * (nh / nkv) * (hd + 2) * sizeof(float)));
     }
     // kernels that may need more than 48 KB of dynamic shared memory
-    CU(cudaFuncSetAttribute(gemv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    for (auto k : {gemv_kernel<1>, gemv_kernel<2>, gemv_kernel<4>}) CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     CU(mma_set_smem_limit((int)c->smem_optin - 8192));
     {
         const int lim_attn = (int)c->smem_optin - 1024;
@@ -977,23 +977,23 @@ static cudaError_t launch_gemv(b200_ctx* c, GemvParams& p) {
     if (c->use_mma) {
         MParams m;
         MPlan plan;
-        if (to_mma_params(c, p, m, plan)) {
+        // Below 8 MB of weights a launch is too short for the tensor-pipe kernel's ring to fill and its cut tiles to be merged; above, its arithmetic wins.  One token
+        // after the other, int8 cache, per-op kernels: two 896-wide layers (down: 3.6 MB) 1038 -> 995 us, two 2048-wide ones in Q5_K_M / Q6_K / Q8_0 2400 / 2566 / 2617 ->
+        // 2194 / 2385 / 2512; with the line at 16 MB 2264 / 2438 / 2592
+        double mb = 0;
+        for (int s = 0; s < p.n_seg; s++) mb += (double)p.seg[s].n_rows * p.seg[s].row_bytes / 1e6;
+        const bool small = mb < 8 && (size_t)xpad_floats(p.K) * sizeof(float) <= 160 * 1024;
+        if (!small && to_mma_params(c, p, m, plan)) {
             c->mma_launches++;
             return launch_k(c, mma_kernel_for(plan.stages), dim3(plan.grid), dim3(plan.warps * 32), plan.smem, m);
         }
     }
     c->v1_launches++;
-    int n_tasks;
-    if (p.epi == EPI_SWIGLU) {
-        n_tasks = (p.seg[0].n_rows + 1) / 2;
-    } else {
-        n_tasks = 0;
-        for (int s = 0; s < p.n_seg; s++) n_tasks += (p.seg[s].n_rows + kGemvR - 1) / kGemvR;
-    }
+    const int R = gemv_rows(p, c->n_sm), n_tasks = gemv_tasks(p, R);
     int grid = (n_tasks + kGemvWarps - 1) / kGemvWarps;
-    grid = std::max(1, std::min(grid, 2 * c->n_sm));
+    grid = std::max(1, std::min(grid, (R == 4 ? 2 : 4) * c->n_sm));
     size_t smem = (size_t)xpad_floats(p.K) * sizeof(float);
-    return launch_k(c, gemv_kernel, dim3(grid), dim3(kGemvThreads), smem, p);
+    return launch_k(c, R == 4 ? gemv_kernel<4> : R == 2 ? gemv_kernel<2> : gemv_kernel<1>, dim3(grid), dim3(kGemvThreads), smem, p);
 }
 
 static cudaError_t launch_attn(b200_ctx* c, const AttnParams& ap, int hd, int G) {
@@ -3300,16 +3300,16 @@ extern "C" int b200_op_vec_mat_q(const float* a, const void* w, uint32_t ggml_ty
             return B200_OK;
         }
     }
-    CU(cudaFuncSetAttribute(gemv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    for (auto k : {gemv_kernel<1>, gemv_kernel<2>, gemv_kernel<4>}) CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     GemvParams p{};
     p.seg[0].w = dw.as<uint8_t>(); p.seg[0].out = dout.as<float>(); p.seg[0].row_bytes = (long long)row_bytes;
     p.seg[0].type = t; p.seg[0].n_rows = (int)n;
     p.n_seg = 1; p.K = (int)k; p.x = da.as<float>(); p.epi = EPI_STORE;
-    int n_tasks = (int)((n + kGemvR - 1) / kGemvR);
+    const int n_tasks = gemv_tasks(p, kGemvR);
     int grid = std::max(1, std::min((n_tasks + kGemvWarps - 1) / kGemvWarps, 296));
     size_t smem = (size_t)xpad_floats((int)k) * sizeof(float);
     if (smem > 160 * 1024) return fail(B200_ERR_UNSUPPORTED, "vec_mat_q: k too large for the shared-memory x staging");
-    gemv_kernel<<<grid, kGemvThreads, smem>>>(p);
+    gemv_kernel<kGemvR><<<grid, kGemvThreads, smem>>>(p);
     if ((rc = op_finish("vec_mat_q"))) return rc;
     CU(cudaMemcpy(out, dout.p, n * 4, cudaMemcpyDeviceToHost));
     return B200_OK;

@@ -25,7 +25,9 @@ namespace b200 {
 
 constexpr int kGemvWarps = 8;
 constexpr int kGemvThreads = kGemvWarps * kWarp;
-constexpr int kGemvR = 4;  // rows per warp task
+// rows per warp task: 4, or fewer where 4 would leave warps idle (gemv_rows).  Every row's sum is its own, whatever R is.  896 x 896 in Q5_0: 28 blocks of
+// eight warps with 4 rows each, 112 with one.
+constexpr int kGemvR = 4;
 
 enum : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU = 2, EPI_SCALED_ACC = 3 };
 
@@ -58,12 +60,17 @@ struct GemvParams {
     int expert_base, expert_count;
 };
 
-__device__ __forceinline__ float u8f(uint32_t w, int k) { return (float)((w >> (8 * k)) & 0xFFu); }
+// byte k of w, less `off`, as a float: PRMT drops it into the mantissa of 2^23, one subtraction removes 2^23 + off (exact; an integer conversion runs at a quarter of
+// the rate and needs the byte cut out first)
+template <int OFF = 0>
+__device__ __forceinline__ float u8f(uint32_t w, int k) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | k)) - (8388608.0f + (float)OFF);
+}
 
 // ---- Q4_K / Q5_K: 8 lanes per 256-element block, 16 qs bytes (32 elements) per lane ----
-template <bool Q5>
-__device__ __forceinline__ void rows_dot_k45(const uint8_t* const (&rp)[kGemvR], int nb, const float* xs, int lane,
-                                             float (&acc)[kGemvR]) {
+template <bool Q5, int R>
+__device__ __forceinline__ void rows_dot_k45(const uint8_t* const (&rp)[R], int nb, const float* xs, int lane,
+                                             float (&acc)[R]) {
     constexpr int BB = Q5 ? 176 : 144;
     constexpr int QS = Q5 ? 48 : 16;
     const int bl = lane >> 3, p = lane & 7, g = p >> 1, h = p & 1, gg = g & 1;
@@ -71,9 +78,9 @@ __device__ __forceinline__ void rows_dot_k45(const uint8_t* const (&rp)[kGemvR],
         const int b = b0 + bl;
         const bool ok = b < nb;
         const int bc = ok ? b : nb - 1;
-        uint4 hd[kGemvR], q[kGemvR], qh[kGemvR];
+        uint4 hd[R], q[R], qh[R];
 #pragma unroll
-        for (int r = 0; r < kGemvR; r++) {
+        for (int r = 0; r < R; r++) {
             const uint8_t* bp = rp[r] + (size_t)bc * BB;
             hd[r] = ldg_stream_u4(bp);
             q[r] = ldg_stream_u4(bp + QS + 16 * p);
@@ -92,7 +99,7 @@ __device__ __forceinline__ void rows_dot_k45(const uint8_t* const (&rp)[kGemvR],
 #pragma unroll
         for (int i = 0; i < 16; i++) { sl += xl[i]; sh += xh[i]; }
 #pragma unroll
-        for (int r = 0; r < kGemvR; r++) {
+        for (int r = 0; r < R; r++) {
             const float d = half_bits_to_float(hd[r].x);
             const float dmin = half_bits_to_float(hd[r].x >> 16);
             const uint32_t A = (hd[r].y >> (16 * gg)) & 0xFFFFu;
@@ -132,17 +139,18 @@ __device__ __forceinline__ void rows_dot_k45(const uint8_t* const (&rp)[kGemvR],
 }
 
 // ---- Q6_K: 8 lanes per 210-byte block (2-byte aligned: 16-bit loads), 32 elements per lane ----
-__device__ __forceinline__ void rows_dot_q6k(const uint8_t* const (&rp)[kGemvR], int nb, const float* xs, int lane,
-                                             float (&acc)[kGemvR]) {
+template <int R>
+__device__ __forceinline__ void rows_dot_q6k(const uint8_t* const (&rp)[R], int nb, const float* xs, int lane,
+                                             float (&acc)[R]) {
     const int bl = lane >> 3, t = lane & 7, n = t >> 2, j = t & 3, is = j >> 1;
     for (int b0 = 0; b0 < nb; b0 += 4) {
         const int b = b0 + bl;
         const bool ok = b < nb;
         const int bc = ok ? b : nb - 1;
-        uint32_t qa[kGemvR][2], qb[kGemvR][2], qhv[kGemvR][2], dd[kGemvR];
-        int sc[kGemvR][4];
+        uint32_t qa[R][2], qb[R][2], qhv[R][2], dd[R];
+        int sc[R][4];
 #pragma unroll
-        for (int r = 0; r < kGemvR; r++) {
+        for (int r = 0; r < R; r++) {
             const uint8_t* bp = rp[r] + (size_t)bc * 210;
             const uint8_t* pa = bp + 64 * n + 8 * j;
             const uint8_t* ph = bp + 128 + 32 * n + 8 * j;
@@ -168,7 +176,7 @@ __device__ __forceinline__ void rows_dot_q6k(const uint8_t* const (&rp)[kGemvR],
             xsum[c] = ((a.x + a.y) + (a.z + a.w)) + ((e.x + e.y) + (e.z + e.w));
         }
 #pragma unroll
-        for (int r = 0; r < kGemvR; r++) {
+        for (int r = 0; r < R; r++) {
             const float d = half_bits_to_float(dd[r]);
             float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -195,8 +203,9 @@ __device__ __forceinline__ void rows_dot_q6k(const uint8_t* const (&rp)[kGemvR],
 }
 
 // ---- 32-element block types (Q8_0, Q4_0, Q5_0) and F16/F32: one lane per 32 elements ----
-__device__ __forceinline__ void rows_dot_b32(int type, const uint8_t* const (&rp)[kGemvR], int K, const float* xs,
-                                             int lane, float (&acc)[kGemvR]) {
+template <int R>
+__device__ __forceinline__ void rows_dot_b32(int type, const uint8_t* const (&rp)[R], int K, const float* xs,
+                                             int lane, float (&acc)[R]) {
     const int nb = K >> 5;
     const int bb = (type == T_F32) ? 128 : (type == T_F16) ? 64 : type_block_bytes(type);
     for (int b = lane; b < nb; b += 32) {
@@ -208,19 +217,18 @@ __device__ __forceinline__ void rows_dot_b32(int type, const uint8_t* const (&rp
             xv[4 * i] = a.x; xv[4 * i + 1] = a.y; xv[4 * i + 2] = a.z; xv[4 * i + 3] = a.w;
         }
 #pragma unroll
-        for (int r = 0; r < kGemvR; r++) {
+        for (int r = 0; r < R; r++) {
             const uint8_t* bp = rp[r] + (size_t)b * bb;
             float s = 0.0f;
             if (type == T_Q8_0) {
                 const float d = half_bits_to_float(ldg_u16(bp));
-                uint32_t qv[16];
+                uint32_t qv[8];
 #pragma unroll
-                for (int i = 0; i < 16; i++) qv[i] = ldg_u16(bp + 2 + 2 * i);
+                for (int i = 0; i < 8; i++) qv[i] = (ldg_u16(bp + 2 + 4 * i) | (ldg_u16(bp + 4 + 4 * i) << 16)) ^ 0x80808080u;
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    s = fmaf((float)(int)(signed char)(qv[i] & 0xFFu), xv[2 * i], s);
-                    s = fmaf((float)(int)(signed char)(qv[i] >> 8), xv[2 * i + 1], s);
-                }
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) s = fmaf(u8f<128>(qv[i], k), xv[4 * i + k], s);
                 s *= d;
             } else if (type == T_Q4_0) {
                 const float d = half_bits_to_float(ldg_u16(bp));
@@ -238,16 +246,15 @@ __device__ __forceinline__ void rows_dot_b32(int type, const uint8_t* const (&rp
                 const float d = half_bits_to_float(ldg_u16(bp));
                 const uint32_t qh = ldg_u16(bp + 2) | (ldg_u16(bp + 4) << 16);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    uint32_t v = ldg_u16(bp + 6 + 2 * i);
+                for (int i = 0; i < 4; i++) {      // bytes 4i .. 4i + 3: elements 4i .. (low nibbles) and 16 + 4i .. (high); bit e of qh is the fifth bit of element e
+                    const uint32_t v = ldg_u16(bp + 6 + 4 * i) | (ldg_u16(bp + 8 + 4 * i) << 16);
+                    // four bits to bit 4 of four bytes: the products of one bit with 2^4, 2^11, 2^18, 2^25 that land elsewhere are masked off
+                    const uint32_t lo = (v & 0x0F0F0F0Fu) | ((((qh >> (4 * i)) & 15u) * 0x02040810u) & 0x10101010u);
+                    const uint32_t hi = ((v >> 4) & 0x0F0F0F0Fu) | ((((qh >> (16 + 4 * i)) & 15u) * 0x02040810u) & 0x10101010u);
 #pragma unroll
-                    for (int k = 0; k < 2; k++) {
-                        int e = 2 * i + k;
-                        int byte = (v >> (8 * k)) & 0xFF;
-                        int lo = ((byte & 0xF) | (((qh >> e) & 1) << 4)) - 16;
-                        int hi = ((byte >> 4) | (((qh >> (e + 16)) & 1) << 4)) - 16;
-                        s = fmaf((float)lo, xv[e], s);
-                        s = fmaf((float)hi, xv[e + 16], s);
+                    for (int k = 0; k < 4; k++) {
+                        s = fmaf(u8f<16>(lo, k), xv[4 * i + k], s);
+                        s = fmaf(u8f<16>(hi, k), xv[16 + 4 * i + k], s);
                     }
                 }
                 s *= d;
@@ -275,9 +282,56 @@ __device__ __forceinline__ void rows_dot_b32(int type, const uint8_t* const (&rp
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
 
-// Stage x (optionally RMS-normalised) into shared memory in the padded layout.
-__device__ __forceinline__ void stage_x(const GemvParams& p, float* xs, float* red) {
+// Stage x (optionally RMS-normalised) into shared memory in the padded layout.  Rows of up to 4 * kStageV * kGemvThreads elements are loaded once, and their
+// norm weights before the wait for the kernel before.
+constexpr int kStageV = 4;
+struct StageW {
+    float4 w[kStageV];
+};
+__device__ __forceinline__ void stage_w(const GemvParams& p, StageW& sw) {
+    if (!p.norm_w || p.K > 4 * kStageV * kGemvThreads) return;
+#pragma unroll
+    for (int i = 0; i < kStageV; i++) {
+        const int e = (threadIdx.x + i * kGemvThreads) * 4;
+        if (e < p.K) sw.w[i] = *reinterpret_cast<const float4*>(p.norm_w + e);
+    }
+}
+__device__ __forceinline__ void stage_x(const GemvParams& p, const StageW& sw, float* xs, float* red) {
     const int tid = threadIdx.x;
+    if (p.K <= 4 * kStageV * kGemvThreads) {
+        float4 v[kStageV];
+#pragma unroll
+        for (int i = 0; i < kStageV; i++) {
+            const int e = (tid + i * kGemvThreads) * 4;
+            if (e < p.K) v[i] = *reinterpret_cast<const float4*>(p.x + e);
+        }
+        float inv = 1.0f;
+        if (p.norm_w) {
+            float ss = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kStageV; i++)
+                if ((tid + i * kGemvThreads) * 4 < p.K) ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+            ss = warp_sum(ss);
+            if ((tid & 31) == 0) red[tid >> 5] = ss;
+            __syncthreads();
+            float tot = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kGemvWarps; w++) tot += red[w];
+            inv = 1.0f / sqrtf(tot / (float)p.K + p.eps);
+        }
+#pragma unroll
+        for (int i = 0; i < kStageV; i++) {
+            const int e = (tid + i * kGemvThreads) * 4;
+            if (e < p.K) {
+                if (p.norm_w) {
+                    v[i].x = (v[i].x * inv) * sw.w[i].x; v[i].y = (v[i].y * inv) * sw.w[i].y; v[i].z = (v[i].z * inv) * sw.w[i].z; v[i].w = (v[i].w * inv) * sw.w[i].w;
+                }
+                *reinterpret_cast<float4*>(xs + xidx(e)) = v[i];
+            }
+        }
+        __syncthreads();
+        return;
+    }
     float inv = 1.0f;
     if (p.norm_w) {
         float ss = 0.0f;
@@ -304,21 +358,23 @@ __device__ __forceinline__ void stage_x(const GemvParams& p, float* xs, float* r
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kGemvThreads) gemv_kernel(const GemvParams p) {
+template <int R>
+__global__ void __launch_bounds__(kGemvThreads) gemv_kernel(const __grid_constant__ GemvParams p) {
+    static_assert(R == 1 || R == 2 || R == 4, "rows per warp");
+    constexpr int G = R / 2 > 0 ? R / 2 : 1;      // (EPI_SWIGLU: R / 2 gate rows and their up rows; never with R = 1)
     extern __shared__ __align__(16) float xs[];
     __shared__ float red[kGemvWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    // task table: segment s owns tasks [t0[s], t0[s+1]); a task = kGemvR rows
-    // (EPI_SWIGLU: 2 gate rows + the 2 matching up rows).
+    // task table: segment s owns tasks [t0[s], t0[s+1]); a task = R rows
     int t0[4];
     t0[0] = 0;
     if (p.epi == EPI_SWIGLU) {
-        t0[1] = (p.seg[0].n_rows + 1) / 2;
+        t0[1] = (p.seg[0].n_rows + G - 1) / G;
         t0[2] = t0[3] = t0[1];
     } else {
 #pragma unroll
-        for (int s = 0; s < 3; s++) t0[s + 1] = t0[s] + (s < p.n_seg ? (p.seg[s].n_rows + kGemvR - 1) / kGemvR : 0);
+        for (int s = 0; s < 3; s++) t0[s + 1] = t0[s] + (s < p.n_seg ? (p.seg[s].n_rows + R - 1) / R : 0);
     }
     const int n_tasks = t0[3];
 
@@ -327,8 +383,8 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_kernel(const GemvParams p) 
         int task = blockIdx.x * kGemvWarps + warp;
         if (task < n_tasks) {
             if (p.epi == EPI_SWIGLU) {
-                const long long off = (long long)task * 2;
-                const long long bytes = 2 * p.seg[0].row_bytes;
+                const long long off = (long long)task * G;
+                const long long bytes = G * p.seg[0].row_bytes;
                 for (long long o = (long long)lane * 128; o < bytes; o += 32 * 128) {
                     prefetch_l2(p.seg[0].w + off * p.seg[0].row_bytes + o);
                     prefetch_l2(p.seg[1].w + off * p.seg[1].row_bytes + o);
@@ -336,14 +392,16 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_kernel(const GemvParams p) 
             } else {
                 int s = (task >= t0[2]) ? 2 : (task >= t0[1]) ? 1 : 0;
                 const GemvSeg& sg = p.seg[s];
-                int row0 = (task - t0[s]) * kGemvR;
-                int rows = min(kGemvR, sg.n_rows - row0);
+                int row0 = (task - t0[s]) * R;
+                int rows = min(R, sg.n_rows - row0);
                 const uint8_t* base = sg.w + (long long)row0 * sg.row_bytes;
                 long long bytes = (long long)rows * sg.row_bytes;
                 for (long long o = (long long)lane * 128; o < bytes; o += 32 * 128) prefetch_l2(base + o);
             }
         }
     }
+    StageW sw;
+    stage_w(p, sw);
     pdl_wait();
     // MoE: the selected expert is written by the routing kernel (a predecessor): read it only after the wait
     long long eoff = p.expert_sel ? (long long)p.expert_sel[p.expert_slot] : 0;
@@ -351,50 +409,53 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_kernel(const GemvParams p) 
         eoff -= p.expert_base;
         if (eoff < 0 || eoff >= p.expert_count) return;
     }
-    stage_x(p, xs, red);
+    stage_x(p, sw, xs, red);
 
     for (int task = blockIdx.x * kGemvWarps + warp; task < n_tasks; task += gridDim.x * kGemvWarps) {
-        const uint8_t* rp[kGemvR];
+        const uint8_t* rp[R];
         int type, s = 0, row0, rows;
         if (p.epi == EPI_SWIGLU) {
             const GemvSeg& ga = p.seg[0];
             const GemvSeg& up = p.seg[1];
-            row0 = task * 2;
-            rows = min(2, ga.n_rows - row0);
+            row0 = task * G;
+            rows = min(G, ga.n_rows - row0);
             type = ga.type;
-            const int r1 = row0 + (rows > 1 ? 1 : 0);
-            rp[0] = ga.w + eoff * ga.expert_stride + (long long)row0 * ga.row_bytes;
-            rp[1] = ga.w + eoff * ga.expert_stride + (long long)r1 * ga.row_bytes;
-            rp[2] = up.w + eoff * up.expert_stride + (long long)row0 * up.row_bytes;
-            rp[3] = up.w + eoff * up.expert_stride + (long long)r1 * up.row_bytes;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const GemvSeg& sg = r < G ? ga : up;
+                rp[r] = sg.w + eoff * sg.expert_stride + (long long)(row0 + min(r < G ? r : r - G, rows - 1)) * sg.row_bytes;
+            }
         } else {
             s = (task >= t0[2]) ? 2 : (task >= t0[1]) ? 1 : 0;
             const GemvSeg& sg = p.seg[s];
-            row0 = (task - t0[s]) * kGemvR;
-            rows = min(kGemvR, sg.n_rows - row0);
+            row0 = (task - t0[s]) * R;
+            rows = min(R, sg.n_rows - row0);
             type = sg.type;
 #pragma unroll
-            for (int r = 0; r < kGemvR; r++)
+            for (int r = 0; r < R; r++)
                 rp[r] = sg.w + eoff * sg.expert_stride + (long long)(row0 + min(r, rows - 1)) * sg.row_bytes;
         }
-        float acc[kGemvR] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = 0.0f;
         switch (type) {
-            case T_Q4_K: rows_dot_k45<false>(rp, p.K >> 8, xs, lane, acc); break;
-            case T_Q5_K: rows_dot_k45<true>(rp, p.K >> 8, xs, lane, acc); break;
+            case T_Q4_K: rows_dot_k45<false, R>(rp, p.K >> 8, xs, lane, acc); break;
+            case T_Q5_K: rows_dot_k45<true, R>(rp, p.K >> 8, xs, lane, acc); break;
             case T_Q6_K: rows_dot_q6k(rp, p.K >> 8, xs, lane, acc); break;
             default: rows_dot_b32(type, rp, p.K, xs, lane, acc); break;
         }
 #pragma unroll
-        for (int r = 0; r < kGemvR; r++) acc[r] = warp_sum(acc[r]);
+        for (int r = 0; r < R; r++) acc[r] = warp_sum(acc[r]);
         if (lane == 0) {
             if (p.epi == EPI_SWIGLU) {
                 float* out = p.seg[0].out;
-                out[row0] = silu_f(acc[0]) * acc[2];
-                if (rows > 1) out[row0 + 1] = silu_f(acc[1]) * acc[3];
+#pragma unroll
+                for (int r = 0; r < G; r++)
+                    if (r < rows) out[row0 + r] = silu_f(acc[r]) * acc[R > 1 ? r + G : r];
             } else {
                 const GemvSeg& sg = p.seg[s];
 #pragma unroll
-                for (int r = 0; r < kGemvR; r++) {
+                for (int r = 0; r < R; r++) {
                     if (r < rows) {
                         const int jrow = row0 + r;
                         float v = acc[r];
@@ -411,6 +472,19 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_kernel(const GemvParams p) 
             }
         }
     }
+}
+
+// Rows per task: as many as still give every one of the chip's warps (two blocks per SM) a task
+inline int gemv_tasks(const GemvParams& p, int R) {
+    if (p.epi == EPI_SWIGLU) return (p.seg[0].n_rows + R / 2 - 1) / (R / 2);
+    int n = 0;
+    for (int s = 0; s < p.n_seg; s++) n += (p.seg[s].n_rows + R - 1) / R;
+    return n;
+}
+inline int gemv_rows(const GemvParams& p, int n_sm) {
+    for (int R = kGemvR; R > (p.epi == EPI_SWIGLU ? 2 : 1); R /= 2)
+        if (gemv_tasks(p, R) >= 2 * n_sm * kGemvWarps) return R;
+    return p.epi == EPI_SWIGLU ? 2 : 1;
 }
 
 }  // namespace b200
