@@ -124,6 +124,7 @@ struct Slot {
 };
 
 constexpr int kMaxGenerated = 1 << 16;
+constexpr int kTokenRing = 64;
 
 struct b200_ctx {
     b200_model_desc d{};
@@ -149,7 +150,7 @@ struct b200_ctx {
     // tensor-pipe GEMV (gemv_mma.cuh): stream-K scratch, watchdog flag, launch knobs
     float* mma_part = nullptr;
     unsigned int* mma_tickets = nullptr;
-    int* mma_err = nullptr;
+    int* mma_err = nullptr;      // watchdog words: the eight in front of the logits (one copy fetches both)
     int mma_tickets_n = 0;
     bool use_mma = true;
     int mma_warps = 16, mma_stages = 3;
@@ -258,7 +259,10 @@ struct b200_ctx {
     int batch_gemm_min = 8;    // measured crossover on Llama-3-8B: a GEMM pass costs ~12 ms up to 32 rows, a sequence alone 2 ms
     uint64_t prefill_gemm_tokens = 0;
     int* h_err = nullptr;   // pinned copy of the first watchdog word, fetched with every synchronising call
-    int* h_token = nullptr;
+    int* h_token = nullptr;          // [kTokenRing]: tokens on their way to the device
+    int h_token_at = 0;
+    uint8_t* h_rows = nullptr;       // pinned: tables of a batched decode step
+    size_t h_rows_bytes = 0;
     std::vector<Slot> slots;
     // layer-program model (layerprog.cu): when set, every entry point below runs through lp_run(); the slots keep the host positions
     LpModel* lp = nullptr;
@@ -736,7 +740,9 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
     CU_ALLOC(cudaMalloc((void**)&c->attn, nh * hd * 4));
     CU_ALLOC(cudaMalloc((void**)&c->hbuf, ffn_w * 4));
     c->out_scratch_elems = std::max<uint64_t>(std::max<uint64_t>(V, ffn_w), std::max<uint64_t>(H, nh * hd));
-    CU_ALLOC(cudaMalloc((void**)&c->logits, c->out_scratch_elems * 4));
+    CU_ALLOC(cudaMalloc((void**)&c->mma_err, (8 + c->out_scratch_elems) * 4));
+    CU(cudaMemset(c->mma_err, 0, 8 * sizeof(int)));
+    c->logits = (float*)c->mma_err + 8;
     c->n_splits = (int)std::min<uint64_t>(64, std::max<uint64_t>(1, (2 * (uint64_t)c->n_sm + nkv - 1) / nkv));
     {   // the split merge stages n_splits * G * (hd + 2) floats in shared memory: it must fit the opt-in limit (G = 7..8 with hd = 128
         // and 64 splits would need 233-266 KB: Qwen2.5-3B / Qwen2-7B shapes)
@@ -750,8 +756,6 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
     c->mma_tickets_n = (int)((std::max<uint64_t>(std::max<uint64_t>(V, 2 * ffn_w), (nh + 2 * nkv) * hd) + 15) / 16 + 8);
     CU_ALLOC(cudaMalloc((void**)&c->mma_tickets, (size_t)c->mma_tickets_n * sizeof(unsigned int)));
     CU(cudaMemset(c->mma_tickets, 0, (size_t)c->mma_tickets_n * sizeof(unsigned int)));
-    CU_ALLOC(cudaMalloc((void**)&c->mma_err, 8 * sizeof(int)));
-    CU(cudaMemset(c->mma_err, 0, 8 * sizeof(int)));
     if (c->ep) {
         CU_ALLOC(cudaMalloc((void**)&c->ep_y, (size_t)8 * H * sizeof(float)));
         CU(cudaMemset(c->ep_y, 0, (size_t)8 * H * sizeof(float)));
@@ -772,10 +776,10 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         CU_ALLOC(cudaMalloc((void**)&c->rope_freq, f.size() * 4));
         CU(cudaMemcpy(c->rope_freq, f.data(), f.size() * 4, cudaMemcpyHostToDevice));
     }
-    CU_ALLOC(cudaHostAlloc((void**)&c->h_logits, V * 4, cudaHostAllocDefault));
-    CU_ALLOC(cudaHostAlloc((void**)&c->h_err, 8 * sizeof(int), cudaHostAllocDefault));
+    CU_ALLOC(cudaHostAlloc((void**)&c->h_err, (8 + V) * 4, cudaHostAllocDefault));
+    c->h_logits = (float*)c->h_err + 8;
     memset(c->h_err, 0, 8 * sizeof(int));
-    CU_ALLOC(cudaHostAlloc((void**)&c->h_token, sizeof(int), cudaHostAllocDefault));
+    CU_ALLOC(cudaHostAlloc((void**)&c->h_token, kTokenRing * sizeof(int), cudaHostAllocDefault));
     c->slots.resize(d.max_batch);
     const uint64_t kv_elems = (uint64_t)d.n_layers * 2 * nkv * d.max_seq_len * hd;
     for (Slot& s : c->slots) {
@@ -925,13 +929,13 @@ extern "C" void b200_ctx_destroy(b200_ctx* c) {
     cudaFree(c->pf_k16);
     cudaFree(c->pf_vt16);
     for (uint8_t* p : c->mega_stage) cudaFree(p);
-    for (void* p : {(void*)c->xa, (void*)c->xb, (void*)c->qkv, (void*)c->attn, (void*)c->hbuf, (void*)c->logits,
+    for (void* p : {(void*)c->xa, (void*)c->xb, (void*)c->qkv, (void*)c->attn, (void*)c->hbuf,
                     (void*)c->attn_part, (void*)c->tickets, (void*)c->moe_sel, (void*)c->moe_wt, (void*)c->taps,
                     (void*)c->rope_freq, c->flush_buf, (void*)c->mma_part, (void*)c->mma_tickets, (void*)c->mma_err})
         cudaFree(p);
-    if (c->h_logits) cudaFreeHost(c->h_logits);
     if (c->h_err) cudaFreeHost(c->h_err);
     if (c->h_token) cudaFreeHost(c->h_token);
+    if (c->h_rows) cudaFreeHost(c->h_rows);
     for (int b = 0; b < 2; b++) {
         if (c->h_spec_logits[b]) cudaFreeHost(c->h_spec_logits[b]);
         if (c->spec_ev[b]) cudaEventDestroy(c->spec_ev[b]);
@@ -1937,22 +1941,29 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     }
     const bool q8 = c->kv_format == 1;
     if (q8 && (rows || !attn_tc)) return fail(B200_ERR_UNSUPPORTED, "int8 KV cache: the GEMM pass needs the tensor-core prompt attention");
-    int* d_pos = reinterpret_cast<int*>(c->pf_rows);
-    float** d_kv = reinterpret_cast<float**>(c->pf_rows + (size_t)cap * 8);
-    SeqState** d_st = reinterpret_cast<SeqState**>(c->pf_rows + (size_t)cap * 16);
+    // tables of a batched decode step, one copy: per row token, position, KV base of the slot, SeqState of the slot
+    int* d_tok = rows ? reinterpret_cast<int*>(c->pf_rows) : c->pf_tok;
+    int* d_pos = reinterpret_cast<int*>(c->pf_rows + (size_t)n * 4);
+    float** d_kv = reinterpret_cast<float**>(c->pf_rows + (size_t)n * 8);
+    SeqState** d_st = reinterpret_cast<SeqState**>(c->pf_rows + (size_t)n * 16);
     if (rows) {
         if (n > cap) return fail(B200_ERR_INVALID_ARGUMENT, "batched decode: more rows than the activation buffers hold");
-        std::vector<int> hp(n);
-        std::vector<float*> hk(n);
-        std::vector<SeqState*> hs(n);
+        if (c->h_rows_bytes < (size_t)n * 24) {
+            if (c->h_rows) cudaFreeHost(c->h_rows);
+            c->h_rows = nullptr;
+            c->h_rows_bytes = 0;
+            CU_ALLOC(cudaHostAlloc((void**)&c->h_rows, (size_t)cap * 24, cudaHostAllocDefault));
+            c->h_rows_bytes = (size_t)cap * 24;
+        }
+        int* h_tok = reinterpret_cast<int*>(c->h_rows);
+        int* h_pos = h_tok + n;
+        float** h_kv = reinterpret_cast<float**>(c->h_rows + (size_t)n * 8);
+        SeqState** h_st = reinterpret_cast<SeqState**>(c->h_rows + (size_t)n * 16);
         for (int i = 0; i < n; i++) {
             Slot& s = c->slots[seqs[i]];
-            hp[i] = (int)s.host_pos; hk[i] = s.kv; hs[i] = s.d_state;
+            h_tok[i] = (int)tokens[i]; h_pos[i] = (int)s.host_pos; h_kv[i] = s.kv; h_st[i] = s.d_state;
         }
-        CU(cudaMemcpyAsync(d_pos, hp.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
-        CU(cudaMemcpyAsync(d_kv, hk.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
-        CU(cudaMemcpyAsync(d_st, hs.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
-        CU(cudaStreamSynchronize(c->stream));   // the host vectors go out of scope
+        CU(cudaMemcpyAsync(c->pf_rows, c->h_rows, (size_t)n * 24, cudaMemcpyHostToDevice, c->stream));      // (the callers wait for the step before they return)
         if (c->pf_logits_rows < n) {
             cudaFree(c->pf_logits);
             c->pf_logits = nullptr;
@@ -1981,7 +1992,6 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     const uint64_t launches0 = c->launches;
     if (use_graph) {
         if ((int)c->batch_graphs.size() <= n) c->batch_graphs.resize((size_t)n + 1);
-        CU(cudaMemcpyAsync(c->pf_tok, tokens, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, c->stream));   // the caller's buffer: not part of the graph
         b200_ctx::BatchGraph& bg = c->batch_graphs[n];
         if (bg.exec) {
             CU(cudaGraphLaunch(bg.exec, c->stream));
@@ -2090,8 +2100,8 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         const int T = std::min(cap, n - done);
         const int pos0 = (int)sl.host_pos + done;
         last_T = T;
-        if (!use_graph) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
-        CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T), dim3(256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)c->pf_tok, d.vocab, X));
+        if (!rows) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
+        CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T), dim3(256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)d_tok, d.vocab, X));
         // Few rows: products straight from the blocks (gemm_few.cuh), their pieces added by the kernel behind them
         few = c->few_part && !q8 && T <= few_max && (rows || c->prompt_f16_min == 0);
         FewOut sum{};                                   // product that X still lacks (of the layer before)
@@ -2389,8 +2399,13 @@ static int check_token(b200_ctx* c, int seq, uint32_t token, const char* fn) {
 }
 
 static int set_token(b200_ctx* c, Slot& sl, uint32_t token) {
-    *c->h_token = (int)token;
-    CU(cudaMemcpyAsync(&sl.d_state->token, c->h_token, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    if (++c->h_token_at == kTokenRing) {      // every place of the ring may hold a token that has not been copied yet
+        CU(cudaStreamSynchronize(c->stream));
+        c->h_token_at = 0;
+    }
+    int* at = c->h_token + c->h_token_at;
+    *at = (int)token;
+    CU(cudaMemcpyAsync(&sl.d_state->token, at, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     return B200_OK;
 }
 
@@ -2502,8 +2517,7 @@ extern "C" int b200_forward(b200_ctx* c, int seq, uint32_t token, float* logits_
         return B200_OK;
     }
     // tensor parallel: this rank's slice [rank * vocab/P, (rank+1) * vocab/P) of the logits (the caller gathers)
-    CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t)c->vocab_l * 4, cudaMemcpyDeviceToHost, c->stream));
-    WATCHDOG_FETCH(c);
+    CU(cudaMemcpyAsync(c->h_err, c->mma_err, (8 + (size_t)c->vocab_l) * 4, cudaMemcpyDeviceToHost, c->stream));      // watchdog words and logits
     CU(cudaStreamSynchronize(c->stream));
     if ((rc = watchdog_check(c, "b200_forward"))) return rc;
     memcpy(logits_out, c->h_logits, (size_t)c->vocab_l * 4);
@@ -2530,7 +2544,7 @@ extern "C" int b200_prefill_token(b200_ctx* c, int seq, uint32_t token) {
     if ((rc = set_token(c, sl, token))) return rc;
     if ((rc = run_token(c, seq, MODE_PREFILL))) return rc;
     WATCHDOG_FETCH(c);
-    CU(cudaStreamSynchronize(c->stream));  // h_token is reused by the next call
+    CU(cudaStreamSynchronize(c->stream));
     if ((rc = watchdog_check(c, "b200_prefill_token"))) return rc;
     sl.host_pos++;
     return B200_OK;
@@ -2553,15 +2567,30 @@ extern "C" int b200_prefill(b200_ctx* c, int seq, const uint32_t* tokens, int n,
         if (sl.host_pos + (uint64_t)n > (uint64_t)c->d.max_seq_len) return fail(B200_ERR_INVALID_ARGUMENT, "b200_prefill: context length exceeded");
         CU(cudaSetDevice(c->par.device));
         if ((rc = prefill_gemm(c, seq, tokens, n, logits_out != nullptr))) return rc;
-        if (logits_out) CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t)c->vocab_l * 4, cudaMemcpyDeviceToHost, c->stream));
-        WATCHDOG_FETCH(c);
+        CU(cudaMemcpyAsync(c->h_err, c->mma_err, (8 + (logits_out ? (size_t)c->vocab_l : 0)) * 4, cudaMemcpyDeviceToHost, c->stream));      // watchdog words (and logits)
         CU(cudaStreamSynchronize(c->stream));
         if ((rc = watchdog_check(c, "b200_prefill"))) return rc;
         if (logits_out) memcpy(logits_out, c->h_logits, (size_t)c->vocab_l * 4);
         sl.host_pos += (uint64_t)n;
         return B200_OK;
     }
-    for (int i = 0; i < n; i++) {
+    // token by token: the launches follow one another without a wait between (unless b200_prefill_token would queue the tokens)
+    const bool queued = c->prefill_queue && !c->queue_bypass && prefill_gemm_ok(c);
+    const int ahead = queued ? 0 : logits_out ? n - 1 : n;
+    CU(cudaSetDevice(c->par.device));
+    rc = B200_OK;
+    int done = 0;
+    for (; done < ahead && rc == B200_OK; done++) {
+        if ((rc = check_token(c, seq, tokens[done], "b200_prefill_token"))) break;
+        if ((rc = set_token(c, c->slots[seq], tokens[done])) == B200_OK && (rc = run_token(c, seq, MODE_PREFILL)) == B200_OK) c->slots[seq].host_pos++;
+    }
+    if (done > 0 && (rc || !logits_out)) {
+        WATCHDOG_FETCH(c);
+        CU(cudaStreamSynchronize(c->stream));
+        if (const int wrc = watchdog_check(c, "b200_prefill_token")) return wrc;
+    }
+    if (rc) return rc;
+    for (int i = done; i < n; i++) {
         if (i == n - 1 && logits_out) return b200_forward(c, seq, tokens[i], logits_out);
         if ((rc = b200_prefill_token(c, seq, tokens[i]))) return rc;
     }
@@ -2597,26 +2626,22 @@ extern "C" int b200_decode_batch(b200_ctx* c, const int* seqs, const uint32_t* t
             }
             CU(cudaSetDevice(c->par.device));
             if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs))) return rc;
+            // n x vocab logits (16.4 MB at batch 32 on Llama-3) to the caller's pageable buffer: DMA into a pinned buffer, rows copied
+            // out by a few host threads (a pageable cudaMemcpy stages the same bytes through the driver on one thread)
+            const size_t bytes = (size_t)n * c->d.vocab * sizeof(float);
+            if (c->h_batch_logits_bytes < bytes) {
+                if (c->h_batch_logits) cudaFreeHost(c->h_batch_logits);
+                c->h_batch_logits = nullptr;
+                c->h_batch_logits_bytes = 0;
+                if (cudaHostAlloc((void**)&c->h_batch_logits, bytes, cudaHostAllocDefault) == cudaSuccess) c->h_batch_logits_bytes = bytes;
+                else cudaGetLastError();
+            }
+            if (c->h_batch_logits) CU(cudaMemcpyAsync(c->h_batch_logits, c->pf_logits, bytes, cudaMemcpyDeviceToHost, c->stream));
             WATCHDOG_FETCH(c);
             CU(cudaStreamSynchronize(c->stream));
             if ((rc = watchdog_check(c, "b200_decode_batch"))) return rc;
-            {   // n x vocab logits (16.4 MB at batch 32 on Llama-3) to the caller's pageable buffer: DMA into a pinned buffer, rows copied
-                // out by a few host threads (a pageable cudaMemcpy stages the same bytes through the driver on one thread)
-                const size_t bytes = (size_t)n * c->d.vocab * sizeof(float);
-                if (c->h_batch_logits_bytes < bytes) {
-                    if (c->h_batch_logits) cudaFreeHost(c->h_batch_logits);
-                    c->h_batch_logits = nullptr;
-                    c->h_batch_logits_bytes = 0;
-                    if (cudaHostAlloc((void**)&c->h_batch_logits, bytes, cudaHostAllocDefault) == cudaSuccess) c->h_batch_logits_bytes = bytes;
-                    else cudaGetLastError();
-                }
-                if (c->h_batch_logits) {
-                    CU(cudaMemcpy(c->h_batch_logits, c->pf_logits, bytes, cudaMemcpyDeviceToHost));
-                    gguf_parallel_copy((uint8_t*)logits_out, (const uint8_t*)c->h_batch_logits, bytes, 4);
-                } else {
-                    CU(cudaMemcpy(logits_out, c->pf_logits, bytes, cudaMemcpyDeviceToHost));
-                }
-            }
+            if (c->h_batch_logits) gguf_parallel_copy((uint8_t*)logits_out, (const uint8_t*)c->h_batch_logits, bytes, 4);
+            else CU(cudaMemcpy(logits_out, c->pf_logits, bytes, cudaMemcpyDeviceToHost));
             for (int i = 0; i < n; i++) c->slots[seqs[i]].host_pos++;
             return B200_OK;
         }
@@ -2638,8 +2663,7 @@ extern "C" int b200_reset(b200_ctx* c, int seq) {
     CU(cudaSetDevice(c->par.device));
     Slot& sl = c->slots[seq];
     sl.pending.clear();
-    CU(cudaMemsetAsync(sl.d_state, 0, sizeof(SeqState), c->stream));
-    CU(cudaStreamSynchronize(c->stream));
+    CU(cudaMemsetAsync(sl.d_state, 0, sizeof(SeqState), c->stream));      // (what reads it next is on the same stream)
     sl.host_pos = 0;
     return B200_OK;
 }
@@ -4078,6 +4102,7 @@ extern "C" int b200_debug_set_position(b200_ctx* c, int seq, uint64_t pos) {
     CU(cudaSetDevice(c->par.device));
     CU(cudaStreamSynchronize(c->stream));
     const int p = (int)pos;
+    CU(cudaStreamSynchronize(c->stream));
     CU(cudaMemcpy(&c->slots[seq].d_state->pos_next, &p, sizeof(int), cudaMemcpyHostToDevice));
     c->slots[seq].host_pos = pos;
     return B200_OK;
