@@ -3059,7 +3059,7 @@ bool chunk_scan_launch(LpModel* m, const StepMeta& sm, const ChunkScan& g, int n
     }
     const int cols = MODE == CS_MEM ? CS_COLS - 1 : CS_COLS;
     launch(m, lp_chunk_prep_kernel<MODE, DM>, dim3((max_len + CS - 1) / CS, g.H, n_runs), dim3(CS_THREADS), prep, sm, g);
-    launch(m, lp_chunk_scan_kernel<MODE, DM>, dim3((g.vdim + cols - 1) / cols, g.H, n_runs), dim3(CS_THREADS), scan, sm, g);
+    launch(m, lp_chunk_scan_kernel<MODE, DM>, dim3((g.vdim + cols - 1) / cols, g.H, n_runs), dim3(CS_SCAN_THREADS), scan, sm, g);
     return true;
 }
 template <int MODE>

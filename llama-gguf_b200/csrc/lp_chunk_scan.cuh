@@ -11,13 +11,13 @@
 // lp_chunk_prep_kernel does what does not need S0, a block per (chunk, head, run); lp_chunk_scan_kernel walks a run's chunks, a block per (8 state
 // columns, head, run) with the columns in shared memory and the next chunk's rows on their way.
 // What bounded the token-by-token form: a chain of two reductions per token (1370 clocks for the delta rule at 128 x 128), SMs mostly waiting.
-// Here a chunk's reductions are products of 64 x 128 by 8; the chain is per chunk.  1500 tokens, 8 heads of 128 x 128: delta rule 1044 -> 33 + 118 us;
-// 4 heads of 64 x 128: memory 656 -> 21 + 90 us.  The decay from s to t is multiplied up (MEM: its logarithm
+// Here a chunk's reductions are products of 64 x 128 by 8; the chain is per chunk.  1500 tokens, 8 heads of 128 x 128: delta rule 1044 -> 26 + 109 us;
+// 4 heads of 64 x 128: memory 656 -> 8 + 73 us.  The decay from s to t is multiplied up (MEM: its logarithm
 // added up) from s on for every s, never a quotient or difference of running products, so it is as exact as one token after the other and a
 // decay of 0 stays 0.
 #pragma once
 
-constexpr int CS = 32, CS_COLS = 8, CS_THREADS = 256;
+constexpr int CS = 32, CS_COLS = 8, CS_THREADS = 256, CS_SCAN_THREADS = 512, CS_STAGES = 3;
 enum { CS_MEM = 0, CS_SSD = 1, CS_DELTA = 2 };
 struct ChunkScan {
     int H, G, dim, vdim, R;             // heads, heads of q and k, sizes, rows of the step
@@ -205,23 +205,62 @@ __global__ void __launch_bounds__(CS_THREADS) lp_chunk_prep_kernel(StepMeta sm, 
 template <int MODE, int DM> struct CsSmem {
     static constexpr int PI = DM + 4, ROWS = MODE == CS_DELTA ? 3 : 2;                       // staged row blocks: q, k (, W)
     static constexpr int STAGE = ROWS * CS * PI + CS * CS_COLS + CS * 36 + 3 * CS;          // + U0, M (pitch 36), scalars
-    static constexpr size_t BYTES = (size_t)(2 * STAGE + DM * CS_COLS + 2 * CS * CS_COLS + 2 * CS * CS_COLS + 4 * CS) * 4;
+    static constexpr size_t BYTES = (size_t)(CS_STAGES * STAGE + 2 * DM * CS_COLS + 4 * CS * CS_COLS + 8 * CS) * 4;
 };
 template <int DM> constexpr size_t cp_smem_bytes() { return (size_t)(2 * CS * (DM + 4) + 3 * CS * 33) * 4; }
-// blockIdx.x: 8 columns of the state (MEM: 7 and the column of ones, whose state is n)
+__device__ __forceinline__ void cs_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void cs_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// RT rows of A (from `a`, pitch PI) times the state S0 [DM][8] (two halves [DM][4]), the key channels d = sl + SL i dealt to SL neighbouring lanes; their partial sums
+// are added in a tree that keeps half of the values per step.  out: [RT][8] of this tile.
+template <int DM, int PI, int SL, int RT> __device__ __forceinline__ void cs_rows_state(const float* a, const float* S0, int sl, float* out) {
+    float acc[8 * RT];
+#pragma unroll
+    for (int e = 0; e < 8 * RT; e++) acc[e] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < DM / SL; i++) {
+        const int d = i * SL + sl;
+        const float4 x = *reinterpret_cast<const float4*>(S0 + d * 4), y = *reinterpret_cast<const float4*>(S0 + DM * 4 + d * 4);
+#pragma unroll
+        for (int r = 0; r < RT; r++) {
+            const float v = a[r * PI + d];
+            acc[8 * r] = fmaf(v, x.x, acc[8 * r]); acc[8 * r + 1] = fmaf(v, x.y, acc[8 * r + 1]);
+            acc[8 * r + 2] = fmaf(v, x.z, acc[8 * r + 2]); acc[8 * r + 3] = fmaf(v, x.w, acc[8 * r + 3]);
+            acc[8 * r + 4] = fmaf(v, y.x, acc[8 * r + 4]); acc[8 * r + 5] = fmaf(v, y.y, acc[8 * r + 5]);
+            acc[8 * r + 6] = fmaf(v, y.z, acc[8 * r + 6]); acc[8 * r + 7] = fmaf(v, y.w, acc[8 * r + 7]);
+        }
+    }
+#pragma unroll
+    for (int o = SL / 2, n = 4 * RT; o > 0; o >>= 1, n >>= 1) {
+        const bool up = (sl & o) != 0;
+#pragma unroll
+        for (int e = 0; e < n; e++) {
+            const float give = up ? acc[e] : acc[e + n], keep = up ? acc[e + n] : acc[e];
+            acc[e] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    const int e0 = sl * (8 * RT / SL);
+#pragma unroll
+    for (int e = 0; e < 8 * RT / SL; e++) out[e0 + e] = acc[e];
+}
+// blockIdx.x: 8 columns of the state (MEM: 7 and the column of ones, whose state is n).
+// Two groups of eight warps.  The chain (threads 0 .. 255): W S0, U, the state after the chunk; the others: q S0 and the chunk's outputs, from the state before it, beside
+// the chain (the state has two buffers), and the copies of the rows two chunks ahead.  1500 tokens: delta rule 115 -> 109 us, memory 88 -> 73 us against one group of eight
+// warps for all of it with the rows one chunk ahead; bound by the chain's shared-memory loads (delta: W S0, U, the update, 2.3 us per chunk).
 template <int MODE, int DM>
-__global__ void __launch_bounds__(CS_THREADS) lp_chunk_scan_kernel(StepMeta sm, ChunkScan g) {
+__global__ void __launch_bounds__(CS_SCAN_THREADS) lp_chunk_scan_kernel(StepMeta sm, ChunkScan g) {
     prev_grid();
     using L = CsSmem<MODE, DM>;
-    constexpr int PI = L::PI, VC = MODE == CS_MEM ? CS_COLS - 1 : CS_COLS;
-    constexpr int TILES = MODE == CS_DELTA ? 16 : 8, SL = CS_THREADS / TILES;                // row tiles of 4 of [W; q] (or q), slices of the key channels
+    constexpr int PI = L::PI, VC = MODE == CS_MEM ? CS_COLS - 1 : CS_COLS, SL = MODE == CS_DELTA ? 16 : 32, RT = MODE == CS_DELTA ? 2 : 4;
     extern __shared__ __align__(16) float cs_sm[];
-    float* S0 = cs_sm + 2 * L::STAGE;           // [DM][8]
-    float* YZ = S0 + DM * CS_COLS;              // [64][8]: W S0, q S0
-    float* U = YZ + 2 * CS * CS_COLS;           // [32][8]
+    float* S0 = cs_sm + CS_STAGES * L::STAGE;   // [2 buffers][2 halves][DM][4]
+    float* Y = S0 + 2 * DM * CS_COLS;           // [32][8]: W S0
+    float* Z = Y + CS * CS_COLS;                // [32][8]: q S0
+    float* U = Z + CS * CS_COLS;                // [32][8]
     float* Us = U + CS * CS_COLS;               // [32][8]: u_s U_s
-    float* scl = Us + CS * CS_COLS;             // [4][32]: z, p, u, e^-m
+    float* scl = Us + CS * CS_COLS;             // [2 buffers][4][32]: z, p, u, e^-m
     const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, run = blockIdx.z, j0 = blockIdx.x * VC;
+    const bool chain = tid < 256;
+    const int ct = tid & 255;                   // thread of its group
     const int r0 = sm.run_start[run], r1 = sm.run_start[run + 1], hk = h * g.G / g.H;
     float* rec = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off);
     float* Sg = rec + (size_t)h * g.dim * g.vdim;
@@ -237,7 +276,8 @@ __global__ void __launch_bounds__(CS_THREADS) lp_chunk_scan_kernel(StepMeta sm, 
         float* s = m + CS * 36;
         const int nt = min(CS, r1 - c0);
         const size_t hr = (size_t)h * g.R + c0;
-        for (int i = tid; i < CS * (DM / 4); i += CS_THREADS) {
+        if (chain) return;                      // (the chain is the longer way)
+        for (int i = ct; i < CS * (DM / 4); i += 256) {
             const int t = i / (DM / 4), d = (i - t * (DM / 4)) * 4;
             const bool in = t < nt && d < g.dim;
             const size_t at = in ? (size_t)(c0 + t) * g.ldq + hk * g.dim + d : 0;
@@ -246,139 +286,114 @@ __global__ void __launch_bounds__(CS_THREADS) lp_chunk_scan_kernel(StepMeta sm, 
             if (MODE == CS_DELTA) cp_async16(smem_u32(w + t * PI + d), in ? g.W + (hr + t) * g.dim + d : g.W, in ? 16u : 0u);
         }
         {
-            const int t = tid >> 3, c = tid & 7, j = j0 + c;
+            const int t = ct >> 3, c = ct & 7, j = j0 + c;
             float* dst = u0 + t * CS_COLS + c;
             if (t >= nt || (c < VC && j >= g.vdim)) *dst = 0.0f;
             else if (c >= VC) *dst = 1.0f;
             else cp_async4(dst, MODE == CS_DELTA ? g.U0 + (hr + t) * g.vdim + j : g.V + (size_t)(c0 + t) * g.ldv + h * g.vdim + j);
             cp_async16(smem_u32(m + t * 36 + c * 4), t < nt ? g.M + (hr + t) * CS + c * 4 : g.M, t < nt ? 16u : 0u);
         }
-        if (tid < 3 * CS) {
-            const int t = tid & 31, row = min(t, nt - 1);                 // (the last row's scalars stand for what is past the end: F and mu of the chunk, D)
-            cp_async4(s + tid, g.sc + (size_t)(tid >> 5) * g.H * g.R + hr + row);
+        if (ct < 3 * CS) {
+            const int t = ct & 31, row = min(t, nt - 1);                 // (the last row's scalars stand for what is past the end: F and mu of the chunk, D)
+            cp_async4(s + ct, g.sc + (size_t)(ct >> 5) * g.H * g.R + hr + row);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // state: row k, columns c4 .. c4 + 3 of the block's 8
-    const int kr = tid >> 1, c4 = (tid & 1) * 4;
+    // the chain's threads: state row kr, columns c4 .. c4 + 3 of the block's 8
+    const int kr = ct >> 1, half = ct & 1, c4 = half * 4;
+    const bool mine = chain && kr < DM;
     float st[4] = {0.f, 0.f, 0.f, 0.f};
-    if (kr < DM) {
+    if (mine) {
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int c = c4 + e, j = j0 + c;
             if (kr < g.dim) st[e] = c >= VC ? nm[kr] : j < g.vdim ? Sg[(size_t)kr * g.vdim + j] : 0.0f;
-            S0[kr * CS_COLS + c] = st[e];
         }
+        *reinterpret_cast<float4*>(S0 + half * DM * 4 + kr * 4) = make_float4(st[0], st[1], st[2], st[3]);
     }
     float m_run = MODE == CS_MEM ? nm[g.dim] : 0.0f;
     const float dskip = MODE == CS_SSD ? g.skip[h] : 0.0f;
     const float qsc = MODE == CS_MEM ? 1.0f / sqrtf((float)g.dim) : 1.0f;
+    // (a chunk's rows are asked for two chunks ahead: one is less than their way from L2 takes)
     stage(r0, 0);
-    for (int c0 = r0, buf = 0; c0 < r1; c0 += CS, buf ^= 1) {
+    if (r0 + CS < r1) stage(r0 + CS, 1);
+    for (int c0 = r0, buf = 0, st3 = 0; c0 < r1; c0 += CS, buf ^= 1, st3 = st3 == CS_STAGES - 1 ? 0 : st3 + 1) {
         const int nt = min(CS, r1 - c0);
-        if (c0 + CS < r1) {
-            stage(c0 + CS, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const float* q = cs_sm + buf * L::STAGE;
+        if (c0 + CS < r1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                        // this chunk's rows are here, and both groups are done with the chunk before
+        if (c0 + 2 * CS < r1) stage(c0 + 2 * CS, st3 == 0 ? 2 : st3 - 1);
+        const float* q = cs_sm + st3 * L::STAGE;
         const float* k = q + CS * PI;
         const float* w = k + CS * PI;
         const float* u0 = q + L::ROWS * CS * PI;
         const float* M = u0 + CS * CS_COLS;
         const float* s = M + CS * 36;
-        float D, m_end = 0.0f;
+        const float* Sb = S0 + buf * DM * CS_COLS;
+        float* sc = scl + buf * 4 * CS;
+        const int t = ct >> 3, c = ct & 7;
+        float D;
         if (MODE == CS_MEM) {
-            const float fe = s[CS - 1];
-            m_end = fmaxf(m_run + fe, s[3 * CS - 1]);
+            const float fe = s[CS - 1], m_end = fmaxf(m_run + fe, s[3 * CS - 1]);
             D = expf(m_run + fe - m_end);
-            if (tid < CS) {
-                const float f = s[tid], mt = fmaxf(m_run + f, s[2 * CS + tid]);
-                scl[tid] = expf(m_run + f - mt) * qsc;
-                scl[CS + tid] = expf(s[2 * CS + tid] - mt);
-                scl[2 * CS + tid] = tid < nt ? expf(s[CS + tid] - m_end) : 0.0f;
-                scl[3 * CS + tid] = expf(-mt);
+            if (!chain && ct < CS) {
+                const float f = s[ct], mt = fmaxf(m_run + f, s[2 * CS + ct]);
+                sc[ct] = expf(m_run + f - mt) * qsc;
+                sc[CS + ct] = expf(s[2 * CS + ct] - mt);
+                sc[3 * CS + ct] = expf(-mt);
             }
+            if (chain) Us[t * CS_COLS + c] = (t < nt ? expf(s[CS + t] - m_end) : 0.0f) * u0[t * CS_COLS + c];
             m_run = m_end;
         } else {
             D = s[3 * CS - 1];
-            if (tid < CS) {
-                scl[tid] = s[tid];
-                scl[2 * CS + tid] = tid < nt ? s[CS + tid] : 0.0f;
-            }
+            if (MODE == CS_SSD && chain) Us[t * CS_COLS + c] = (t < nt ? s[CS + t] : 0.0f) * u0[t * CS_COLS + c];
         }
-        {   // [W; q] S0: row tile `tile`, key channels d = sl + SL i
-            const int tile = tid / SL, sl = tid % SL;
-            const float* a = MODE == CS_DELTA && tile < 8 ? w + tile * 4 * PI : q + (tile & 7) * 4 * PI;
-            float acc[32];
-#pragma unroll
-            for (int e = 0; e < 32; e++) acc[e] = 0.0f;
-#pragma unroll
-            for (int i = 0; i < DM / SL; i++) {
-                const int d = i * SL + sl;
-                const float4 x = *reinterpret_cast<const float4*>(S0 + d * CS_COLS), y = *reinterpret_cast<const float4*>(S0 + d * CS_COLS + 4);
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const float v = a[r * PI + d];
-                    acc[8 * r] = fmaf(v, x.x, acc[8 * r]); acc[8 * r + 1] = fmaf(v, x.y, acc[8 * r + 1]);
-                    acc[8 * r + 2] = fmaf(v, x.z, acc[8 * r + 2]); acc[8 * r + 3] = fmaf(v, x.w, acc[8 * r + 3]);
-                    acc[8 * r + 4] = fmaf(v, y.x, acc[8 * r + 4]); acc[8 * r + 5] = fmaf(v, y.y, acc[8 * r + 5]);
-                    acc[8 * r + 6] = fmaf(v, y.z, acc[8 * r + 6]); acc[8 * r + 7] = fmaf(v, y.w, acc[8 * r + 7]);
-                }
+        if (chain) {
+            if (MODE == CS_DELTA) {
+                cs_rows_state<DM, PI, SL, RT>(w + (ct / SL) * RT * PI, Sb, ct % SL, Y + (ct / SL) * RT * CS_COLS);
+                cs_sync(1, 256);
+                const float ut = u0[t * CS_COLS + c] - Y[t * CS_COLS + c];
+                U[t * CS_COLS + c] = ut;
+                Us[t * CS_COLS + c] = (t < nt ? s[CS + t] : 0.0f) * ut;
+                cs_arrive(2, 512);              // (U is there for the outputs)
             }
-            // sums over the SL neighbouring lanes: each step keeps half of the values, so lane sl ends with the 32 / SL values from sl * 32 / SL on
+            cs_sync(1, 256);
+            if (mine) {
 #pragma unroll
-            for (int o = SL / 2, n = 16; o > 0; o >>= 1, n >>= 1) {
-                const bool up = (sl & o) != 0;
-#pragma unroll
-                for (int e = 0; e < n; e++) {
-                    const float give = up ? acc[e] : acc[e + n], keep = up ? acc[e + n] : acc[e];
-                    acc[e] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                for (int e = 0; e < 4; e++) st[e] *= D;
+#pragma unroll 8
+                for (int i = 0; i < CS; i++) {
+                    const float kv = k[i * PI + kr];
+                    const float4 u = *reinterpret_cast<const float4*>(Us + i * CS_COLS + c4);
+                    st[0] = fmaf(kv, u.x, st[0]); st[1] = fmaf(kv, u.y, st[1]); st[2] = fmaf(kv, u.z, st[2]); st[3] = fmaf(kv, u.w, st[3]);
                 }
+                *reinterpret_cast<float4*>(S0 + (buf ^ 1) * DM * CS_COLS + half * DM * 4 + kr * 4) = make_float4(st[0], st[1], st[2], st[3]);
             }
-            const int e0 = sl * (32 / SL);
-#pragma unroll
-            for (int e = 0; e < 32 / SL; e++) YZ[tile * 32 + e0 + e] = acc[e];
-        }
-        __syncthreads();
-        const int t = tid >> 3, c = tid & 7;
-        const float ut = u0[t * CS_COLS + c] - (MODE == CS_DELTA ? YZ[t * CS_COLS + c] : 0.0f);
-        U[t * CS_COLS + c] = ut;
-        Us[t * CS_COLS + c] = scl[2 * CS + t] * ut;
-        __syncthreads();
-        {   // output of (t, c)
-            float a0 = 0.0f, a1 = 0.0f;
+        } else {
+            cs_rows_state<DM, PI, SL, RT>(q + (ct / SL) * RT * PI, Sb, ct % SL, Z + (ct / SL) * RT * CS_COLS);
+            if (MODE == CS_DELTA) cs_sync(2, 512);
+            else cs_sync(2, 256);
+            const float* Uc = MODE == CS_DELTA ? U : u0;
+            float a0 = 0.0f, a1 = 0.0f;         // output of (t, c)
 #pragma unroll
             for (int i = 0; i < CS; i += 4) {
                 const float4 m = *reinterpret_cast<const float4*>(M + t * 36 + i);
-                a0 = fmaf(m.x, U[i * CS_COLS + c], a0);
-                a1 = fmaf(m.y, U[(i + 1) * CS_COLS + c], a1);
-                a0 = fmaf(m.z, U[(i + 2) * CS_COLS + c], a0);
-                a1 = fmaf(m.w, U[(i + 3) * CS_COLS + c], a1);
+                a0 = fmaf(m.x, Uc[i * CS_COLS + c], a0);
+                a1 = fmaf(m.y, Uc[(i + 1) * CS_COLS + c], a1);
+                a0 = fmaf(m.z, Uc[(i + 2) * CS_COLS + c], a0);
+                a1 = fmaf(m.w, Uc[(i + 3) * CS_COLS + c], a1);
             }
-            const float z = YZ[(MODE == CS_DELTA ? CS * CS_COLS : 0) + t * CS_COLS + c];
-            float o = MODE == CS_MEM ? fmaf(scl[t], z, scl[CS + t] * (a0 + a1)) : fmaf(scl[t], z, a0 + a1);
-            if (MODE == CS_SSD) o = fmaf(dskip, ut, o);
+            const float z = Z[t * CS_COLS + c], zt = MODE == CS_MEM ? sc[t] : s[t];
+            float o = MODE == CS_MEM ? fmaf(zt, z, sc[CS + t] * (a0 + a1)) : fmaf(zt, z, a0 + a1);
+            if (MODE == CS_SSD) o = fmaf(dskip, Uc[t * CS_COLS + c], o);
             if (MODE == CS_MEM) {
                 const float nq = __shfl_sync(0xffffffffu, o, lane | 7);
-                o /= fmaxf(fabsf(nq), scl[3 * CS + t]) + 1e-6f;
+                o /= fmaxf(fabsf(nq), sc[3 * CS + t]) + 1e-6f;
             }
             if (t < nt && c < VC && j0 + c < g.vdim) g.O[(size_t)(c0 + t) * g.ldo + h * g.vdim + j0 + c] = o;
         }
-        if (kr < DM) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) st[e] *= D;
-#pragma unroll 8
-            for (int i = 0; i < CS; i++) {
-                const float kv = k[i * PI + kr];
-                const float4 u = *reinterpret_cast<const float4*>(Us + i * CS_COLS + c4);
-                st[0] = fmaf(kv, u.x, st[0]); st[1] = fmaf(kv, u.y, st[1]); st[2] = fmaf(kv, u.z, st[2]); st[3] = fmaf(kv, u.w, st[3]);
-            }
-            *reinterpret_cast<float4*>(S0 + kr * CS_COLS + c4) = make_float4(st[0], st[1], st[2], st[3]);
-        }
-        __syncthreads();
     }
-    if (kr < g.dim) {
+    if (mine && kr < g.dim) {
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int c = c4 + e, j = j0 + c;
