@@ -54,6 +54,22 @@ __global__ void lp_gated_gelu_kernel(const float* __restrict__ P, int ldp, OutT*
     out[i] = from_f<OutT>(gelu_tanh_f(p[n]) * p[ff + n]);
 }
 
+// the same, four units per thread (ff, ldp and the addresses' multiples of 16 bytes; 948 x 4096: 17 -> 9 us)
+template <typename OutT>
+__global__ void lp_gated_gelu4_kernel(const float* __restrict__ P, int ldp, OutT* __restrict__ out, int ff, int R) {
+    prev_grid();
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i >= (size_t)R * ff) return;
+    const int r = (int)(i / ff), n = (int)(i - (size_t)r * ff);
+    const float4 g = *reinterpret_cast<const float4*>(P + (size_t)r * ldp + n), u = *reinterpret_cast<const float4*>(P + (size_t)r * ldp + ff + n);
+    struct alignas(4 * sizeof(OutT)) { OutT v[4]; } o;
+    o.v[0] = from_f<OutT>(gelu_tanh_f(g.x) * u.x);
+    o.v[1] = from_f<OutT>(gelu_tanh_f(g.y) * u.y);
+    o.v[2] = from_f<OutT>(gelu_tanh_f(g.z) * u.z);
+    o.v[3] = from_f<OutT>(gelu_tanh_f(g.w) * u.w);
+    *reinterpret_cast<decltype(o)*>(out + i) = o;
+}
+
 // out[r][n] = relu(P[r][n])^2 (the relu^2 layer when its up projection is part of a wider product)
 template <typename OutT>
 __global__ void lp_relu2_kernel(const float* __restrict__ P, int ldp, OutT* __restrict__ out, int ff, int R) {
