@@ -2045,8 +2045,11 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 const long long lo = glu ? at : std::max(at, first), hi = glu ? at + rows_n : std::min(at + rows_n, first + (long long)w->ne[1]);
                 if (lo < hi) {
                     const int nr = (int)(hi - lo);
-                    const cudaError_t e = launch_on(st, pdl, rows_to_f16_kernel, dim3((K / 8 + 255) / 256, (nr + F16_ROWS - 1) / F16_ROWS), dim3(256), 0, w->type,
-                                                    (const uint8_t*)w->d + (lo - (glu ? 0 : first)) * w->row_bytes, (long long)w->row_bytes, nr, K, c->pf_w16 + put);
+                    const long long elems = (long long)nr * K;
+                    const int run = f16_run_of(elems, c->n_sm);
+                    const long long per = 256LL * run * F16_WARPS;
+                    const cudaError_t e = launch_on(st, pdl, rows_to_f16_for(w->type), dim3((unsigned)((elems + per - 1) / per)), dim3(F16_WARPS * 32), 0,
+                                                    (const uint8_t*)w->d + (lo - (glu ? 0 : first)) * w->row_bytes, elems, run, c->pf_w16 + put);
                     if (e != cudaSuccess) return e;
                     c->launches++;
                     put += (size_t)nr * K;

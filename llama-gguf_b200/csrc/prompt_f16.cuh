@@ -13,22 +13,17 @@
 
 namespace b200 {
 
-// eight consecutive elements k0 + 8c .. of a Q4_K row (k0 % 64 == 0), as u2_deq64_q4k computes them
-__device__ __forceinline__ uint4 f16_deq8_q4k(const uint8_t* row, int k0, int c) {
-    const uint8_t* blk = row + (long long)(k0 >> 8) * 144;
-    const int gp = (k0 & 255) >> 6, hi = c >> 2, b = 16 * (gp & 1) + 8 * hi;
-    const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(blk));
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(blk + 16 + 32 * gp + 8 * (c & 3)));
-    const float d = half_bits_to_float(hdr.x), dmin = half_bits_to_float(hdr.x >> 16);
-    int s, m;
-    if (gp < 2) {
-        s = (hdr.y >> b) & 63;
-        m = (hdr.z >> b) & 63;
-    } else {
-        s = ((hdr.w >> b) & 15) | (((hdr.y >> (b + 6)) & 3) << 4);
-        m = ((hdr.w >> (b + 4)) & 15) | (((hdr.z >> (b + 6)) & 3) << 4);
-    }
-    const float ds = __fmul_rn(d, (float)s) * 16777216.0f, cm = -__fmul_rn(dmin, (float)m);      // nibbles as subnormal fp16: q 2^-24
+// One warp unpacks `run` consecutive units of 256 elements: a matrix's rows follow one another without gaps, in blocks and in fp16, so units are counted through
+// the matrix and a unit may cross rows of block types of 32.  The run's bytes come in by whole 16-byte words (all in flight), lie in shared memory at their own
+// offset, and a lane takes eight (Q8_0) or two times eight elements (K-quants: the low and the high halves of the same bytes) of a unit at a time.  The blocks
+// are read before the wait for the kernel before (a product that may still read the scratch rows).
+// Bound by DRAM: 0.56 to 1.06 bytes in, 2 out per element.  Runs of eight units, or of two where eight would leave SMs without a block (f16_run_of).  Against a thread per
+// eight elements of four rows with 16-bit loads from global memory, whole prompts: 300 tokens through two 8B layers in Q4_K_M 1053 -> 997 us, 700 tokens in Q6_K / Q5_K_M
+// 1455 / 1525 -> 1366 / 1372 us, 333 through four 2048-wide ones in Q8_0 624 -> 593 us.
+constexpr int F16_RUN = 8, F16_WARPS = 8;
+constexpr int F16_BYTES = F16_RUN * 272 + 32;      // of a run, widest type, at any offset of 16
+// eight values d sc q - dmin m, each one f32 FMA on a nibble held as subnormal fp16 (q 2^-24), as u2_deq64_q4k computes them
+__device__ __forceinline__ uint4 f16_nibbles(uint2 q, int hi, float ds, float cm) {
     uint32_t out[4];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -39,27 +34,89 @@ __device__ __forceinline__ uint4 f16_deq8_q4k(const uint8_t* row, int k0, int c)
     }
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
-
-// rows x K elements -> fp16 [rows][K].  A thread unpacks one chunk of 8 in F16_ROWS rows (independent loads in flight); bound by DRAM: 0.56 to
-// 1.06 bytes in, 2 out per element.  The blocks are read and unpacked before the wait for the kernel before (a product that may still read the scratch rows).
-constexpr int F16_ROWS = 4;
-__global__ void __launch_bounds__(256) rows_to_f16_kernel(int type, const uint8_t* __restrict__ w, long long row_bytes, int rows, int K, __half* __restrict__ out) {
-    pdl_launch_dependents();
-    const int ch = blockIdx.x * 256 + threadIdx.x;
-    if (ch * 8 >= K) return;
-    const int k0 = (ch * 8) & ~63, c = ch & 7, r0 = blockIdx.y * F16_ROWS;
-    uint4 v[F16_ROWS];
-    if (type == T_Q4_K && (((uintptr_t)w | (uintptr_t)row_bytes) & 15) == 0) {
-#pragma unroll
-        for (int u = 0; u < F16_ROWS; u++) v[u] = f16_deq8_q4k(w + (long long)min(r0 + u, rows - 1) * row_bytes, k0, c);
+template <int TYPE> struct F16Unit {
+    static constexpr int BYTES = TYPE == T_Q4_K ? 144 : TYPE == T_Q5_K ? 176 : TYPE == T_Q6_K ? 210 : 272;
+    static constexpr int LANES = TYPE == T_Q8_0 ? 32 : 16;      // lanes per unit
+};
+// lane i (< LANES) of a unit whose blocks start at blk (shared memory): its elements -> out (the unit's 256 fp16 values); live: elements that exist
+template <int TYPE>
+__device__ __forceinline__ void f16_unit(const uint8_t* blk, int i, __half* out, int live) {
+    if constexpr (TYPE == T_Q4_K) {
+        const int gp = i >> 2, c = i & 3, b = 16 * (gp & 1);
+        const uint2 h0 = *reinterpret_cast<const uint2*>(blk), h1 = *reinterpret_cast<const uint2*>(blk + 8);      // (blocks are 8-byte aligned at least: umma_eligible)
+        const uint4 hdr = make_uint4(h0.x, h0.y, h1.x, h1.y);
+        const uint2 q = *reinterpret_cast<const uint2*>(blk + 16 + 32 * gp + 8 * c);
+        const float d = half_bits_to_float(hdr.x), dmin = half_bits_to_float(hdr.x >> 16);
+        int s0, m0, s1, m1;
+        if (gp < 2) {
+            s0 = (hdr.y >> b) & 63; m0 = (hdr.z >> b) & 63;
+            s1 = (hdr.y >> (b + 8)) & 63; m1 = (hdr.z >> (b + 8)) & 63;
+        } else {
+            s0 = ((hdr.w >> b) & 15) | (((hdr.y >> (b + 6)) & 3) << 4);
+            m0 = ((hdr.w >> (b + 4)) & 15) | (((hdr.z >> (b + 6)) & 3) << 4);
+            s1 = ((hdr.w >> (b + 8)) & 15) | (((hdr.y >> (b + 14)) & 3) << 4);
+            m1 = ((hdr.w >> (b + 12)) & 15) | (((hdr.z >> (b + 14)) & 3) << 4);
+        }
+        const uint4 lo = f16_nibbles(q, 0, __fmul_rn(d, (float)s0) * 16777216.0f, -__fmul_rn(dmin, (float)m0));
+        const uint4 hi = f16_nibbles(q, 1, __fmul_rn(d, (float)s1) * 16777216.0f, -__fmul_rn(dmin, (float)m1));
+        *reinterpret_cast<uint4*>(out + 64 * gp + 8 * c) = lo;
+        *reinterpret_cast<uint4*>(out + 64 * gp + 32 + 8 * c) = hi;
+    } else if constexpr (TYPE == T_Q8_0) {
+        if (8 * i < live) *reinterpret_cast<uint4*>(out + 8 * i) = umma_deq8<true>(TYPE, blk, 64 * (i >> 3), i & 7);
     } else {
-#pragma unroll
-        for (int u = 0; u < F16_ROWS; u++) v[u] = umma_deq8<false>(type, w + (long long)min(r0 + u, rows - 1) * row_bytes, k0, c);
+        const int gp = i >> 2, c = i & 3;
+        const uint4 lo = umma_deq8<true>(TYPE, blk, 64 * gp, c), hi = umma_deq8<true>(TYPE, blk, 64 * gp, c + 4);
+        *reinterpret_cast<uint4*>(out + 64 * gp + 8 * c) = lo;
+        *reinterpret_cast<uint4*>(out + 64 * gp + 32 + 8 * c) = hi;
     }
-    pdl_wait();
+}
+template <int TYPE>
+__global__ void __launch_bounds__(F16_WARPS * 32) rows_to_f16_kernel(const uint8_t* __restrict__ w, long long elems, int run, __half* __restrict__ out) {
+    pdl_launch_dependents();
+    using U = F16Unit<TYPE>;
+    __shared__ __align__(16) uint8_t s_raw[F16_WARPS][(F16_BYTES + 15) & ~15];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long unit0 = ((long long)blockIdx.x * F16_WARPS + warp) * run, units = (elems + 255) / 256;
+    const int n = (int)(units - unit0 < run ? units - unit0 : run);
+    int off = 0;
+    if (n > 0) {
+        const long long beg = unit0 * U::BYTES;
+        const long long all = (elems / type_block_elems(TYPE)) * type_block_bytes(TYPE);      // bytes of the matrix
+        const long long end = beg + (long long)n * U::BYTES < all ? beg + (long long)n * U::BYTES : all;
+        const uintptr_t a = (uintptr_t)(w + beg);
+        off = (int)(a & 15);
+        const int words = (int)((off + (end - beg) + 15) / 16);
+        const uint8_t* p = (const uint8_t*)(a & ~(uintptr_t)15);
+        constexpr int WORDS = ((F16_RUN * U::BYTES + 30) / 16 + 31) / 32;      // of 16 bytes, per lane
+        uint4 raw[WORDS];
 #pragma unroll
-    for (int u = 0; u < F16_ROWS; u++)
-        if (r0 + u < rows) *reinterpret_cast<uint4*>(out + (size_t)(r0 + u) * K + ch * 8) = v[u];
+        for (int k = 0; k < WORDS; k++) {
+            const int i = lane + 32 * k;
+            if (i >= words) continue;
+            const uint8_t* q = p + 16 * i;
+            if (q >= w && q + 16 <= w + all) raw[k] = __ldg(reinterpret_cast<const uint4*>(q));
+            else {                                          // a word that begins before the matrix or ends behind it
+                uint32_t v[4] = {0u, 0u, 0u, 0u};
+                for (int j = 0; j < 16; j++)
+                    if (q + j >= w && q + j < w + all) v[j >> 2] |= (uint32_t)__ldg(q + j) << (8 * (j & 3));
+                raw[k] = make_uint4(v[0], v[1], v[2], v[3]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < WORDS; k++)
+            if (lane + 32 * k < words) *reinterpret_cast<uint4*>(&s_raw[warp][16 * (lane + 32 * k)]) = raw[k];
+    }
+    __syncwarp();
+    pdl_wait();
+    constexpr int PER = 32 / U::LANES;
+    for (int u = lane / U::LANES; u < n; u += PER) {
+        const long long left = elems - (unit0 + u) * 256;
+        f16_unit<TYPE>(&s_raw[warp][off + u * U::BYTES], lane % U::LANES, out + (unit0 + u) * 256, left < 256 ? (int)left : 256);
+    }
+}
+inline int f16_run_of(long long elems, int n_sm) { return elems >= 2LL * n_sm * F16_WARPS * F16_RUN * 256 ? F16_RUN : 2; }
+inline void (*rows_to_f16_for(int type))(const uint8_t*, long long, int, __half*) {
+    return type == T_Q4_K ? rows_to_f16_kernel<T_Q4_K> : type == T_Q5_K ? rows_to_f16_kernel<T_Q5_K> : type == T_Q6_K ? rows_to_f16_kernel<T_Q6_K> : rows_to_f16_kernel<T_Q8_0>;
 }
 
 namespace tc16 {
