@@ -2104,7 +2104,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         const int pos0 = (int)sl.host_pos + done;
         last_T = T;
         if (!rows) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
-        CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T), dim3(256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)d_tok, d.vocab, X));
+        CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T, T <= 256 ? 4 : 1), dim3(T <= 256 ? 128 : 256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)d_tok, d.vocab, X));
         // Few rows: products straight from the blocks (gemm_few.cuh), their pieces added by the kernel behind them
         few = c->few_part && !q8 && T <= few_max && (rows || c->prompt_f16_min == 0);
         FewOut sum{};                                   // product that X still lacks (of the layer before)

@@ -101,4 +101,30 @@ __global__ void dequantize_kernel(int type, const uint8_t* __restrict__ src, lon
     }
 }
 
+// Eight consecutive elements e0 .. (e0 % 8 == 0) of the block at `b`: the values dequant_elem gives, with scales, minima and factors read once.
+__device__ __forceinline__ void dequant_elem8(int type, const uint8_t* b, int e0, float (&v)[8]) {
+    if (type == T_Q4_K || type == T_Q5_K) {
+        const float d = half_bits_to_float(rd_u16(b)), dmin = half_bits_to_float(rd_u16(b + 2));
+        const int j = e0 >> 5, l = e0 & 31;
+        int sc, mn;
+        scale_min_k4(b + 4, j, sc, mn);
+        const float d1 = __fmul_rn(d, (float)sc), m1 = __fmul_rn(dmin, (float)mn);
+        const uint8_t* qs = b + (type == T_Q5_K ? 48 : 16) + (j >> 1) * 32 + l;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint8_t byte = qs[i];
+            float q = (float)((j & 1) ? (byte >> 4) : (byte & 0x0F));
+            if (type == T_Q5_K) q = __fadd_rn(q, ((b[16 + l + i] >> j) & 1) ? 16.0f : 0.0f);
+            v[i] = __fsub_rn(__fmul_rn(d1, q), m1);
+        }
+    } else if (type == T_Q8_0) {
+        const float d = half_bits_to_float(rd_u16(b));
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __fmul_rn((float)(int)(signed char)b[2 + e0 + i], d);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = dequant_elem(type, b, e0 + i);
+    }
+}
+
 }  // namespace b200
