@@ -1011,16 +1011,30 @@ static cudaError_t launch_attn(b200_ctx* c, const AttnParams& ap, int hd, int G)
 }
 
 // Enqueue every kernel of one token for `slot` on c->stream (captured into a graph by the caller).
-// Device memory that a call after loading has to have: the prompts' fp16 weight rows, which the fused products can do without, go first when there is no room
+// Device memory that a call after loading has to have: the prompts' fp16 weight rows and the buffers of the products of few rows, which the fused products can do
+// without, go first when there is no room (and with the latter the captured steps that name them).  Never called inside a capture
 static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
     return (cudaError_t)alloc_or_give_back(
         [&] { return (int)cudaMalloc(p, bytes); },
         [&] {
             cudaGetLastError();
-            if (!c->pf_w16) return false;
+            if (!c->pf_w16 && !c->few_part) return false;
             cudaFree(c->pf_w16);
             c->pf_w16 = nullptr;
             c->pf_w16_elems = 0;
+            if (c->few_part) {
+                cudaStreamSynchronize(c->stream);
+                for (auto& bg : c->batch_graphs) {
+                    if (bg.exec) cudaGraphExecDestroy(bg.exec);
+                    bg = b200_ctx::BatchGraph();
+                }
+                for (uint8_t*& q : c->few_img) {
+                    cudaFree(q);
+                    q = nullptr;
+                }
+                cudaFree(c->few_part);
+                c->few_part = nullptr;
+            }
             return true;
         });
 }
