@@ -401,13 +401,38 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __syncwarp();
     float* part = reinterpret_cast<float*>(base);           // [TN tokens][128 rows] over the drained ring
     const int rows = min(TN, t.rows - t.t0);
+    // K in one piece: nothing to exchange, so the sums go from tensor memory straight to Y, neighbouring lanes to neighbouring columns.  Through shared memory
+    // with two cluster barriers this end cost 1 to 4 us of a launch: 32 sequences through two layers of 2048 2943 -> 2867 us, prompts of 777, 130 and 41 rows
+    // through three of 1024 626 -> 586 (<64, 0>: 14.1 -> 10.2 us a launch).  Gated units keep the exchange, which pairs two rows of a tile.
+    const bool alone = !GLU && S == 1;
     if (warp < TC_EPI_WARPS) {
+        const int n = t.m * (GLU ? TC_M / 2 : TC_M) + (tid & (TC_M - 1));
+        const bool live = n < a.N;
+        const float bn = (alone && a.bias && live) ? a.bias[n] : 0.0f;
+        void* Yt = seg_rows<tc_t, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
         tc_wait(acc_full, 0, alive, a.err, 4);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
         for (int c0 = 32 * (warp >> 2); c0 < rows; c0 += 64) {
             uint32_t v[32];
             tc_ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0);
+            if (alone) {
+                if constexpr (!GLU) {
+                    if (EPI == EPI_ADD) {                   // (the old sums first: no load behind a store to the same array)
+                        float old[32];
+#pragma unroll
+                        for (int c = 0; c < 32; c++) old[c] = (live && c0 + c < rows) ? reinterpret_cast<const float*>(Yt)[(size_t)(c0 + c) * a.ldy + n] : 0.0f;
+#pragma unroll
+                        for (int c = 0; c < 32; c++)
+                            if (live && c0 + c < rows) reinterpret_cast<float*>(Yt)[(size_t)(c0 + c) * a.ldy + n] = old[c] + (a.alpha * __uint_as_float(v[c]) + bn);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 32; c++)
+                            if (live && c0 + c < rows) epi_store<tc_t, EPI>(Yt, (size_t)(c0 + c) * a.ldy + n, a.alpha * __uint_as_float(v[c]) + bn, a.act);
+                    }
+                }
+                continue;
+            }
 #pragma unroll
             for (int c = 0; c < 32; c++) part[(c0 + c) * TC_M + (tid & (TC_M - 1))] = __uint_as_float(v[c]);
         }
@@ -415,7 +440,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-    if (warp < TC_EPI_WARPS) {
+    if (warp < TC_EPI_WARPS && !alone) {
         const int c_beg = rank * rows / S, c_end = (rank + 1) * rows / S, n0 = t.m * (GLU ? TC_M / 2 : TC_M);
         const uint32_t part_s = smem_u32(part);
         void* Yt = seg_rows<tc_t, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
@@ -456,8 +481,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             }
         }
     }
-    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");      // nobody leaves while its partial sums are read
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (!alone) {                                           // nobody leaves while its partial sums are read
+        asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    }
     if (warp == TC_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN) : "memory");
 }
 
