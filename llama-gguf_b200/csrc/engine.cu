@@ -35,6 +35,7 @@
 #include "gemm_umma2.cuh"
 #include "few_rows.cuh"
 #include "prompt_f16.cuh"
+#include "prompt_rows.cuh"
 #include "spare.cuh"
 #include "attn_umma.cuh"
 #include "kv_int8.cuh"
@@ -1910,10 +1911,10 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     Slot& sl = c->slots[seq];
     const int H = d.hidden, hd = d.head_dim, nh = d.n_heads, nkv = d.n_kv_heads, A = nh * hd, I = (int)d.ffn;
     const int QKV = (nh + 2 * nkv) * hd;
-    const size_t per_tok = (size_t)H + QKV + 2 * (size_t)I + ((size_t)H + A + I + 1) / 2;   // floats (the fp16 rows count half)
     const int cap = std::min(prefill_chunk(), d.max_seq_len);
+    const PromptRows place = prompt_rows(cap, kFewTokens, H, QKV, A, I);
     if (!c->pf_buf) {
-        CU_ALLOC(late_malloc(c, (void**)&c->pf_buf, per_tok * cap * sizeof(float)));
+        CU_ALLOC(late_malloc(c, (void**)&c->pf_buf, place.floats * sizeof(float)));
         CU_ALLOC(late_malloc(c, (void**)&c->pf_tok, cap * sizeof(int)));
         CU_ALLOC(late_malloc(c, (void**)&c->pf_rows, (size_t)cap * 24));
     }
@@ -2019,13 +2020,13 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             bg.warm = true;
         }
     }
-    float* X = c->pf_buf;                               // [T][H] residual stream (f32)
-    float* Q = X + (size_t)cap * H;                     // [T][QKV] f32
-    float* G = Q + (size_t)cap * QKV;                   // [T][I] gate
-    float* U = G + (size_t)cap * I;                     // [T][I] up
-    __half* XNh = reinterpret_cast<__half*>(U + (size_t)cap * I);   // [T][H] normed rows, fp16 (GEMM input)
-    __half* ATh = XNh + (size_t)cap * H;                // [T][A] attention output, fp16
-    __half* Hh = ATh + (size_t)cap * A;                 // [T][I] silu(gate) * up, fp16
+    float* X = c->pf_buf + place.x;                     // [T][H] residual stream (f32)
+    float* Q = c->pf_buf + place.qkv;                   // [T][QKV] f32
+    float* G = c->pf_buf + place.gate;                  // [T][I] gate; few rows also [T][H], what X still lacks
+    float* U = c->pf_buf + place.up;                    // [T][I] up
+    __half* XNh = reinterpret_cast<__half*>(c->pf_buf + place.xn);   // [T][H] normed rows, fp16 (GEMM input)
+    __half* ATh = reinterpret_cast<__half*>(c->pf_buf + place.at);   // [T][A] attention output, fp16
+    __half* Hh = reinterpret_cast<__half*>(c->pf_buf + place.act);   // [T][I] silu(gate) * up, fp16
     const size_t kv_layer = (size_t)2 * nkv * d.max_seq_len * hd;
     cudaStream_t st = c->stream;
     const bool pdl = rows ? c->batch_pdl : c->prompt_pdl;   // programmatic dependent launches along the whole chain

@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-3
 synth.TINY["few-128"] = dict(synth.TINY["llama-tiny"], hidden=2048, n_layers=2, n_heads=16, n_kv_heads=4, ffn=4096, vocab=700)
 synth.TINY["few-64"] = dict(synth.TINY["qwen-tiny"], hidden=1024, n_layers=2, n_heads=16, n_kv_heads=2, ffn=2048, vocab=1000)
-MODELS = [("few-128", "Q4_K_M"), ("few-128", "Q5_K_M"), ("few-128", "Q6_K"), ("few-64", "Q8_0")]
+# hidden above ffn: the sums that the residual stream still lacks are wider than the gate rows in whose place they lie
+synth.TINY["few-wide"] = dict(synth.TINY["llama-tiny"], hidden=2048, n_layers=2, n_heads=2, n_kv_heads=1, ffn=256, vocab=300)
+MODELS = [("few-wide", "Q4_K"), ("few-128", "Q4_K_M"), ("few-128", "Q5_K_M"), ("few-128", "Q6_K"), ("few-64", "Q8_0")]
 
 
 def launches(gpu, call):
