@@ -36,6 +36,7 @@
 #include "few_rows.cuh"
 #include "prompt_f16.cuh"
 #include "prompt_rows.cuh"
+#include "ahead.cuh"
 #include "spare.cuh"
 #include "attn_umma.cuh"
 #include "kv_int8.cuh"
@@ -262,6 +263,8 @@ struct b200_ctx {
     int* h_err = nullptr;   // pinned copy of the first watchdog word, fetched with every synchronising call
     int* h_token = nullptr;          // [kTokenRing]: tokens on their way to the device
     int h_token_at = 0;
+    int* h_ahead = nullptr;          // [2][8]: watchdog words behind a group of queued tokens (ahead.cuh)
+    cudaEvent_t ahead_ev[2] = {nullptr, nullptr};
     uint8_t* h_rows = nullptr;       // pinned: tables of a batched decode step
     size_t h_rows_bytes = 0;
     std::vector<Slot> slots;
@@ -780,7 +783,9 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
     CU_ALLOC(cudaHostAlloc((void**)&c->h_err, (8 + V) * 4, cudaHostAllocDefault));
     c->h_logits = (float*)c->h_err + 8;
     memset(c->h_err, 0, 8 * sizeof(int));
-    CU_ALLOC(cudaHostAlloc((void**)&c->h_token, kTokenRing * sizeof(int), cudaHostAllocDefault));
+    CU_ALLOC(cudaHostAlloc((void**)&c->h_token, (kTokenRing + 16) * sizeof(int), cudaHostAllocDefault));
+    c->h_ahead = c->h_token + kTokenRing;
+    for (cudaEvent_t& e : c->ahead_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     c->slots.resize(d.max_batch);
     const uint64_t kv_elems = (uint64_t)d.n_layers * 2 * nkv * d.max_seq_len * hd;
     for (Slot& s : c->slots) {
@@ -936,6 +941,8 @@ extern "C" void b200_ctx_destroy(b200_ctx* c) {
         cudaFree(p);
     if (c->h_err) cudaFreeHost(c->h_err);
     if (c->h_token) cudaFreeHost(c->h_token);
+    for (cudaEvent_t e : c->ahead_ev)
+        if (e) cudaEventDestroy(e);
     if (c->h_rows) cudaFreeHost(c->h_rows);
     for (int b = 0; b < 2; b++) {
         if (c->h_spec_logits[b]) cudaFreeHost(c->h_spec_logits[b]);
@@ -2592,16 +2599,30 @@ extern "C" int b200_prefill(b200_ctx* c, int seq, const uint32_t* tokens, int n,
         sl.host_pos += (uint64_t)n;
         return B200_OK;
     }
-    // token by token: the launches follow one another without a wait between (unless b200_prefill_token would queue the tokens)
+    // token by token: the launches follow one another without a wait between, and the watchdog words are looked at some tokens later (unless b200_prefill_token
+    // would queue the tokens)
     const bool queued = c->prefill_queue && !c->queue_bypass && prefill_gemm_ok(c);
-    const int ahead = queued ? 0 : logits_out ? n - 1 : n;
     CU(cudaSetDevice(c->par.device));
-    rc = B200_OK;
     int done = 0;
-    for (; done < ahead && rc == B200_OK; done++) {
-        if ((rc = check_token(c, seq, tokens[done], "b200_prefill_token"))) break;
-        if ((rc = set_token(c, c->slots[seq], tokens[done])) == B200_OK && (rc = run_token(c, seq, MODE_PREFILL)) == B200_OK) c->slots[seq].host_pos++;
-    }
+    rc = run_ahead(
+        queued ? 0 : logits_out ? n - 1 : n,
+        [&](int i) {
+            if (const int e = check_token(c, seq, tokens[i], "b200_prefill_token")) return e;
+            if (const int e = set_token(c, c->slots[seq], tokens[i])) return e;
+            if (const int e = run_token(c, seq, MODE_PREFILL)) return e;
+            c->slots[seq].host_pos++;
+            done++;
+            return (int)B200_OK;
+        },
+        [&](int j) {
+            CU(cudaMemcpyAsync(c->h_ahead + 8 * j, c->mma_err, 8 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            CU(cudaEventRecord(c->ahead_ev[j], c->stream));
+            return (int)B200_OK;
+        },
+        [&](int j) {
+            CU(cudaEventSynchronize(c->ahead_ev[j]));
+            return c->h_ahead[8 * j] ? (int)B200_ERR_OPERATION_FAILED : (int)B200_OK;      // (watchdog_check below says which)
+        });
     if (done > 0 && (rc || !logits_out)) {
         WATCHDOG_FETCH(c);
         CU(cudaStreamSynchronize(c->stream));
