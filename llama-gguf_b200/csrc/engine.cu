@@ -2101,8 +2101,11 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (raw || L.gate.type == T_Q6_K) return raw || mb <= 512 ? 32 : 65;
         return mb <= 96 ? 32 : mb <= 136 ? 48 : 65;
     };
+    // chunks of T rows that the products of few rows take whole
+    auto few_takes = [&](int T) { return c->few_part && !q8 && T <= few_max && (rows || c->prompt_f16_min == 0); };
     bool f16_able = false;
-    for (const Layer& L : c->layers) f16_able |= !rows && gemm_encode_fn() && std::min(cap, n) >= f16_min(L);
+    if (!rows && gemm_encode_fn() && !few_takes(std::min(cap, n)))
+        for (const Layer& L : c->layers) f16_able |= std::min(cap, n) >= f16_min(L);
     if (f16_able && !c->pf_w16) {
         const size_t want = std::max(std::min<size_t>((size_t)env_int("B200_PROMPT_F16_KROWS", 128 << 10) << 10, std::max((size_t)2 * I * H, (size_t)QKV * H)), (size_t)256 * std::max(std::max(I, H), A));
         if (cudaMalloc((void**)&c->pf_w16, want * sizeof(__half)) == cudaSuccess) c->pf_w16_elems = want;
@@ -2128,7 +2131,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (!rows) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
         CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T, T <= 256 ? 4 : 1), dim3(T <= 256 ? 128 : 256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)d_tok, d.vocab, X));
         // Few rows: products straight from the blocks (gemm_few.cuh), their pieces added by the kernel behind them
-        few = c->few_part && !q8 && T <= few_max && (rows || c->prompt_f16_min == 0);
+        few = few_takes(T);
         FewOut sum{};                                   // product that X still lacks (of the layer before)
         bool has_sum = false;
         auto few_norm = [&](const float* w, uint8_t* img) {

@@ -5,6 +5,7 @@ Tolerance: activations are rounded to fp16 at four places per layer; with weight
 logit, within the bound of 1e-3 that every path of rows holds; here the weights are exact.  A wrong row, block or piece is off by the size of the logits."""
 import numpy as np
 import pytest
+import torch
 
 import synth
 from synth import rel_err
@@ -76,3 +77,18 @@ def test_switched_off(b200, monkeypatch):
         finally:
             gpu.close()
     assert n[0] != n[1]
+
+
+def test_no_fp16_rows_for_prompts_that_need_none(b200):
+    """The fp16 weight rows of the two-pass products are allocated by the first prompt that uses them, not by one of up to 256 tokens."""
+    arch, desc, tensors = synth.synth_model("few-128", "Q4_K_M", 320)
+    gpu = b200.GpuOnlyInference(desc, tensors)
+    try:
+        gpu.prefill(synth.prompt_tokens(256, desc["vocab"]))
+        before = torch.cuda.mem_get_info()[0]
+        gpu.reset()
+        gpu.prefill(synth.prompt_tokens(300, desc["vocab"]))
+        rows = 2 * 2 * desc["ffn"] * desc["hidden"]      # gate and up in fp16
+        assert before - torch.cuda.mem_get_info()[0] >= rows
+    finally:
+        gpu.close()
