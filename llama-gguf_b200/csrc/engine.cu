@@ -242,6 +242,7 @@ struct b200_ctx {
     std::map<const void*, int> pf_tmap_of;
     std::map<const void*, int> few_tmap_of;   // ... of the products of few rows (gemm_few.cuh); Q6_K blocks with another pitch
     bool few_able = false;           // every product of a layer can take that path
+    bool few_head = false;           // ... and the head of batched decoding
     uint8_t* few_img[3] = {};        // images of the activations: normed rows, attention, gated units
     float* few_part = nullptr;       // pieces of cut tiles
     bool pf_tmaps_built = false;
@@ -1814,6 +1815,16 @@ static cudaError_t gemm_dispatch(UmmaParams& p, int n_sm, cudaStream_t st, uint6
     return umma_launch(p, st);
 }
 
+// The deal of a product of few rows; false: its numbers do not fit.
+static bool few_deal(FewPlan& pl, std::initializer_list<const DevTensor*> ws, int K, int T, int n_sm) {
+    int rows[kFewMaxSeg] = {}, cost[kFewMaxSeg] = {}, n = 0;
+    for (const DevTensor* w : ws) {
+        rows[n] = (int)w->ne[1];
+        cost[n++] = few_pitch(w->type) / 16;
+    }
+    return few_plan(pl, n, rows, cost, K, T, n_sm);
+}
+
 // TMA tensor maps for the dequant-GEMM's weight tiles: box = 128 rows x one 256-element block (stream_pitch(type, 1) bytes).
 // Matrices whose rows are not 16-byte multiples keep the direct global reads.
 static int umma_tmaps_build(b200_ctx* c) {
@@ -1859,8 +1870,14 @@ static int umma_tmaps_build(b200_ctx* c) {
     const b200_model_desc& d = c->d;
     // whole blocks of 256 in every row; narrower than 1024, a layer's products are a microsecond of work either way and keep the kernels they had (tests pin their count)
     c->few_able = env_int("B200_FEW_GEMM", 1) != 0 && d.hidden % 256 == 0 && d.hidden >= 1024 && d.hidden <= kFewNormMax && d.n_heads * d.head_dim % 256 == 0 && d.ffn % 256 == 0;
-    for (const Layer& L : c->layers)
-        for (const DevTensor* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down}) c->few_able = c->few_able && c->few_tmap_of.count(w->d);
+    auto fits = [&](std::initializer_list<const DevTensor*> ws) {      // in the 32-bit arithmetic of the deal, at any number of rows
+        FewPlan pl;
+        for (const DevTensor* w : ws)
+            if (!c->few_tmap_of.count(w->d)) return false;
+        return few_deal(pl, ws, (int)(*ws.begin())->ne[0], kFewTokens, c->n_sm);
+    };
+    for (const Layer& L : c->layers) c->few_able = c->few_able && fits({&L.wq, &L.wk, &L.wv}) && fits({&L.wo}) && fits({&L.gate, &L.up}) && fits({&L.down});
+    c->few_head = fits({c->output.present() ? &c->output : &c->token_embd});
     return B200_OK;
 }
 static void umma_set_tmap(b200_ctx* c, UmmaParams& p) {
@@ -2142,20 +2159,19 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         };
         auto few_product = [&](std::initializer_list<const DevTensor*> ws, int K, const uint8_t* img, std::initializer_list<float*> ys, int ldy, FewOut& out) {
             FewArgs a{};
-            int rows_of[kFewMaxSeg] = {}, cost[kFewMaxSeg] = {}, n_seg = 0;
+            int n_seg = 0;
             for (const DevTensor* w : ws) {
                 FewSeg& sg = a.seg[n_seg];
                 sg.map = (const CUtensorMap*)c->pf_tmaps + c->few_tmap_of.at(w->d);
                 sg.type = w->type;
-                sg.n_rows = rows_of[n_seg] = (int)w->ne[1];
+                sg.n_rows = (int)w->ne[1];
                 sg.pitch = few_pitch(w->type);
-                cost[n_seg] = sg.pitch / 16;
                 sg.block_bytes = 256 / type_block_elems(w->type) * type_block_bytes(w->type);
                 sg.y = ys.begin()[n_seg];
                 sg.ldy = ldy;
                 n_seg++;
             }
-            if (!few_plan(a.plan, n_seg, rows_of, cost, K, T, c->n_sm)) return cudaErrorInvalidValue;
+            if (!few_deal(a.plan, ws, K, T, c->n_sm)) return cudaErrorInvalidValue;
             a.image = img; a.part = c->few_part; a.err = c->mma_err;
             out = FewOut{};
             out.plan = a.plan; out.part = a.part; out.N = few_n(T);
@@ -2225,7 +2241,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         }
         if (few) {      // the last product -> X, and in batched decoding the head of all rows
             const DevTensor& head = c->output.present() ? c->output : c->token_embd;
-            head_done = rows && c->few_tmap_of.count(head.d);
+            head_done = rows && c->few_head;
             CU(few_norm(head_done ? c->output_norm.f32() : nullptr, head_done ? c->few_img[0] : nullptr));
             if (head_done) {
                 FewOut lg{};

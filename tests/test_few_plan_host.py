@@ -1,4 +1,5 @@
-"""csrc/few_plan.cuh on the host: the deal of units to blocks is a partition, readers find every piece of a cut tile in its slot and in the order of K."""
+"""csrc/few_plan.cuh on the host: the deal of units to blocks is a partition, readers find every piece of a cut tile in its slot and in the order of K.  A matrix that
+can be dealt at 256 rows can be at any smaller number: what the engine asks once, before it lets a model take these products."""
 import os
 import subprocess
 
@@ -60,6 +61,15 @@ int main() {
         const int K = 256 * (1 + (rnd(4) ? rnd(60) : rnd(4))), T = 1 + rnd(256);
         if (int r = check(n, rows, cost, K, T)) return printf("%d: %d segments, rows %d, K %d, T %d\n", r, n, rows[0], K, T), 1;
     }
+    for (int rows : {128256, 1 << 20, 1 << 21, 3 << 20})
+        for (int K : {4096, 8192, 28672}) {
+            FewPlan p;
+            const int cost = 17;
+            const bool most = few_plan(p, 1, &rows, &cost, K, 256, 148);
+            if (most != ((rows + 127) / 128 * 4ull * (K / 256) * 17 * 148 < 1ull << 32)) return printf("bound: rows %d, K %d\n", rows, K), 1;
+            for (int T = 1; T <= 256; T++)
+                if (most && !few_plan(p, 1, &rows, &cost, K, T, 148)) return printf("rows %d, K %d: %d tokens\n", rows, K, T), 1;
+        }
     return 0;
 }
 """
