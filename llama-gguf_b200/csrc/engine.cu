@@ -2006,6 +2006,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (c->pf_logits_rows < n) {
             cudaFree(c->pf_logits);
             c->pf_logits = nullptr;
+            c->pf_logits_rows = 0;      // (until there is one again)
             CU_ALLOC(late_malloc(c, (void**)&c->pf_logits, (size_t)n * d.vocab * sizeof(float)));
             c->pf_logits_rows = n;
             for (auto& bg : c->batch_graphs) {   // (the captured head GEMMs write the old buffer)
@@ -3879,6 +3880,7 @@ extern "C" int b200_decode_batch_greedy(b200_ctx* c, const int* seqs, const uint
         if (c->pf_argmax_rows < n) {
             cudaFree(c->pf_argmax);
             c->pf_argmax = nullptr;
+            c->pf_argmax_rows = 0;
             CU_ALLOC(late_malloc(c, (void**)&c->pf_argmax, (size_t)n * sizeof(int)));
             c->pf_argmax_rows = n;
         }
