@@ -8,15 +8,17 @@ import synth
 from synth import rel_err
 
 pytestmark = pytest.mark.gpu
-# rows of a product: 448 and 64 (one row per warp), 2368 x 2 of gate and up (two), 9600 (four); 2, 4 and 8 MB K-quants around the line; ragged row counts
+# rows of a product: 448 and 64 (one row per warp), 2368 x 2 of gate and up and 5001 of the head (two), 9600 (four); K-quants below the line (2 to 7 MB) and above it (9.4);
+# ragged row counts
 synth.TINY["rows-1"] = dict(synth.TINY["qwen-tiny"], n_layers=1, ffn=768)
-synth.TINY["rows-2"] = dict(synth.TINY["qwen-tiny"], n_layers=1, ffn=2368)
+synth.TINY["rows-2"] = dict(synth.TINY["qwen-tiny"], n_layers=1, ffn=2368, vocab=5001)
 synth.TINY["rows-4"] = dict(synth.TINY["qwen-tiny"], n_layers=1, ffn=9600, vocab=9601)
 synth.TINY["line"] = dict(synth.TINY["tinyllama-tiny"], n_layers=1, ffn=8192)
+synth.TINY["line-above"] = dict(synth.TINY["tinyllama-tiny"], n_layers=1, ffn=16384)
 
 
 @pytest.mark.parametrize("preset,mix", [("rows-1", "Q4_K_M"), ("rows-1", "Q8_0"), ("rows-2", "Q4_K_M"), ("rows-4", "Q8_0"), ("rows-4", "Q4_K_M"), ("line", "Q4_K_M"),
-                                        ("line", "Q6_K")])
+                                        ("line", "Q6_K"), ("line-above", "Q4_K_M")])
 def test_tokens(b200, oracle, monkeypatch, preset, mix):
     monkeypatch.setenv("B200_MEGA", "0")
     arch, desc, tensors = synth.synth_model(preset, mix, 16)
