@@ -48,3 +48,35 @@ def test_a_step_that_failed_leaves_a_context_that_works(b200, monkeypatch):
             gpu.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_buffers_of_few_rows_are_given_back(b200, monkeypatch):
+    """Captured steps of eight rows; then 256 rows whose logits fit only where the images and pieces of the products of few rows were, eight rows on the full device, and
+    eight with room again.  The steps captured before name buffers that are gone: they must not be replayed."""
+    arch, desc, tensors = model()
+    calls = [(8, 0), (8, 1), (8, 2), (ROWS, 3), (8, 4), (8, 5), (8, 6)]
+    out, launches = {}, {}
+    for few in ("0", "1"):      # (the first also loads the kernels that the full device needs)
+        monkeypatch.setenv("B200_FEW_GEMM", few)
+        gpu = b200.GpuOnlyInference(desc, tensors)
+        block = None
+        try:
+            out[few], launches[few] = [], []
+            for k, (n, seed) in enumerate(calls):
+                if few == "1" and k == 3:
+                    block = fill(3 << 20)
+                if few == "1" and k == 4:        # what was given back is taken as well
+                    more = fill(1 << 20)
+                if few == "1" and k == 5:
+                    del block, more
+                    torch.cuda.empty_cache()
+                before = gpu.stats()["kernel_launches"]
+                out[few].append(gpu.decode_batch(list(range(n)), tokens(n, seed)))
+                launches[few].append(gpu.stats()["kernel_launches"] - before)
+        finally:
+            gpu.close()
+    few_path = 8 * desc["n_layers"] + 6
+    assert [x == few_path for x in launches["1"]] == [True] * 3 + [False] * 2 + [True] * 2, launches
+    assert few_path not in launches["0"]
+    for a, b in zip(out["1"], out["0"]):
+        assert max(rel_err(x, y) for x, y in zip(a, b)) < TOL
