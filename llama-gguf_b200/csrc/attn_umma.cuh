@@ -154,101 +154,97 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
     long long waited = 0;
 
     if (warp == kAttnLoader) {
-        {
-            int asked_k = 0, asked_v = 0;
-            for (int j = 0; j < nt; j++) {
-                const uint32_t b = j & 1, ph = ((j >> 1) & 1) ^ 1;
-                u2_wait(k_empty + 8u * b, ph, alive, p.err, 21, waited);
-                alive = __all_sync(0xffffffffu, alive);
-                if (!alive) break;
-                if (u2_elect()) {
-                    u2_expect_tx(k_full + 8u * b, (uint32_t)(2 * SM::K));
+        int asked_k = 0, asked_v = 0;
+        for (int j = 0; j < nt; j++) {
+            const uint32_t b = j & 1, ph = ((j >> 1) & 1) ^ 1;
+            u2_wait(k_empty + 8u * b, ph, alive, p.err, 21, waited);
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            if (u2_elect()) {
+                u2_expect_tx(k_full + 8u * b, (uint32_t)(2 * SM::K));
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
+                for (int h = 0; h < 2; h++)
 #pragma unroll
-                        for (int s = 0; s < NS; s++)
-                            u2_tma_2d(base + SM::K_AT + (2 * b + h) * SM::K + s * (kAttnTK * 128), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, k_full + 8u * b);
-                }
-                __syncwarp();
-                asked_k = j + 1;
-                u2_wait(v_empty + 8u * b, ph, alive, p.err, 22, waited);
-                alive = __all_sync(0xffffffffu, alive);
-                if (!alive) break;
-                if (u2_elect()) {
-                    u2_expect_tx(v_full + 8u * b, (uint32_t)(2 * SM::V));
-#pragma unroll
-                    for (int h = 0; h < 2; h++) u2_tma_2d(base + SM::V_AT + (2 * b + h) * SM::V, &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, v_full + 8u * b);
-                }
-                __syncwarp();
-                asked_v = j + 1;
+                    for (int s = 0; s < NS; s++)
+                        u2_tma_2d(base + SM::K_AT + (2 * b + h) * SM::K + s * (kAttnTK * 128), &kmap, s * 64, (h * p.n_kv + kh) * p.P + j * kAttnTK, k_full + 8u * b);
             }
-            if (!alive) {                           // gave up: what has been asked for lands first (bounded)
-                auto land = [&](uint32_t full, int asked) {
-                    ring_in_flight<2>(asked, [&](int stage, unsigned parity) {
-                        bool w = true;
-                        u2_wait(full + 8u * stage, parity, w, nullptr, 0, waited);
-                    });
-                };
-                land(k_full, asked_k);
-                land(v_full, asked_v);
+            __syncwarp();
+            asked_k = j + 1;
+            u2_wait(v_empty + 8u * b, ph, alive, p.err, 22, waited);
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            if (u2_elect()) {
+                u2_expect_tx(v_full + 8u * b, (uint32_t)(2 * SM::V));
+#pragma unroll
+                for (int h = 0; h < 2; h++) u2_tma_2d(base + SM::V_AT + (2 * b + h) * SM::V, &vmap, j * kAttnTK, (h * p.n_kv + kh) * HD, v_full + 8u * b);
             }
+            __syncwarp();
+            asked_v = j + 1;
+        }
+        if (!alive) {                           // gave up: what has been asked for lands first (bounded)
+            auto land = [&](uint32_t full, int asked) {
+                ring_in_flight<2>(asked, [&](int stage, unsigned parity) {
+                    bool w = true;
+                    u2_wait(full + 8u * stage, parity, w, nullptr, 0, waited);
+                });
+            };
+            land(k_full, asked_k);
+            land(v_full, asked_v);
         }
     } else if (warp == kAttnMma) {
-        {
-            const uint32_t idS = umma_idesc(128, kAttnTK), idO = umma_idesc(128, HD);
-            const uint64_t dQ = umma_desc(base), dP = umma_desc(base + SM::P_AT);
-            auto scores = [&](int j) {              // S = Q_hi K_hi^T + Q_lo K_hi^T + Q_hi K_lo^T
-                const uint32_t b = j & 1, ph = (j >> 1) & 1;
-                u2_wait(k_full + 8u * b, ph, alive, p.err, 23, waited);
-                u2_wait(s_empty + 8u * b, ph ^ 1u, alive, p.err, 24, waited);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dK = umma_desc(base + SM::K_AT + 2 * b * SM::K);
-                alive = __all_sync(0xffffffffu, alive);
-                const bool lead = u2_elect();
-                if (lead && alive) {
-#pragma unroll
-                    for (int t = 0; t < 3; t++) {
-                        const uint64_t da = dQ + (t == 1 ? SM::Q / 16 : 0), db = dK + (t == 2 ? SM::K / 16 : 0);
-#pragma unroll
-                        for (int s = 0; s < NS; s++)
-#pragma unroll
-                            for (int kk = 0; kk < 4; kk++)
-                                umma_f16(tmem + b * kAttnTK, da + (uint64_t)(s * (128 * 128 / 16) + 2 * kk), db + (uint64_t)(s * (kAttnTK * 128 / 16) + 2 * kk), idS,
-                                         (t > 0 || s > 0 || kk > 0) ? 1u : 0u);
-                    }
-                }
-                if (lead) {
-                    umma_commit(k_empty + 8u * b);
-                    umma_commit(s_full + 8u * b);
-                }
-                __syncwarp();
-            };
-            u2_wait(q_full, 0, alive, p.err, 25, waited);
+        const uint32_t idS = umma_idesc(128, kAttnTK), idO = umma_idesc(128, HD);
+        const uint64_t dQ = umma_desc(base), dP = umma_desc(base + SM::P_AT);
+        auto scores = [&](int j) {              // S = Q_hi K_hi^T + Q_lo K_hi^T + Q_hi K_lo^T
+            const uint32_t b = j & 1, ph = (j >> 1) & 1;
+            u2_wait(k_full + 8u * b, ph, alive, p.err, 23, waited);
+            u2_wait(s_empty + 8u * b, ph ^ 1u, alive, p.err, 24, waited);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            scores(0);
-            for (int j = 0; j < nt; j++) {
-                const uint32_t b = j & 1;
-                if (j + 1 < nt) scores(j + 1);
-                u2_wait(v_full + 8u * b, (j >> 1) & 1, alive, p.err, 26, waited);
-                u2_wait(p_full, j & 1, alive, p.err, 27, waited);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dV = umma_desc(base + SM::V_AT + 2 * b * SM::V);
-                alive = __all_sync(0xffffffffu, alive);
-                const bool lead = u2_elect();
-                if (lead && alive) {                // O += P_hi V_hi + P_lo V_hi + P_hi V_lo
+            const uint64_t dK = umma_desc(base + SM::K_AT + 2 * b * SM::K);
+            alive = __all_sync(0xffffffffu, alive);
+            const bool lead = u2_elect();
+            if (lead && alive) {
 #pragma unroll
-                    for (int t = 0; t < 3; t++) {
-                        const uint64_t da = dP + (t == 1 ? SM::P / 16 : 0), db = dV + (t == 2 ? SM::V / 16 : 0);
+                for (int t = 0; t < 3; t++) {
+                    const uint64_t da = dQ + (t == 1 ? SM::Q / 16 : 0), db = dK + (t == 2 ? SM::K / 16 : 0);
 #pragma unroll
-                        for (int kk = 0; kk < kAttnTK / 16; kk++) umma_f16(tO, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), idO, (j > 0 || t > 0 || kk > 0) ? 1u : 0u);
-                    }
+                    for (int s = 0; s < NS; s++)
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++)
+                            umma_f16(tmem + b * kAttnTK, da + (uint64_t)(s * (128 * 128 / 16) + 2 * kk), db + (uint64_t)(s * (kAttnTK * 128 / 16) + 2 * kk), idS,
+                                     (t > 0 || s > 0 || kk > 0) ? 1u : 0u);
                 }
-                if (lead) {
-                    umma_commit(v_empty + 8u * b);
-                    umma_commit(pv_done);
-                }
-                __syncwarp();
             }
+            if (lead) {
+                umma_commit(k_empty + 8u * b);
+                umma_commit(s_full + 8u * b);
+            }
+            __syncwarp();
+        };
+        u2_wait(q_full, 0, alive, p.err, 25, waited);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        scores(0);
+        for (int j = 0; j < nt; j++) {
+            const uint32_t b = j & 1;
+            if (j + 1 < nt) scores(j + 1);
+            u2_wait(v_full + 8u * b, (j >> 1) & 1, alive, p.err, 26, waited);
+            u2_wait(p_full, j & 1, alive, p.err, 27, waited);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t dV = umma_desc(base + SM::V_AT + 2 * b * SM::V);
+            alive = __all_sync(0xffffffffu, alive);
+            const bool lead = u2_elect();
+            if (lead && alive) {                // O += P_hi V_hi + P_lo V_hi + P_hi V_lo
+#pragma unroll
+                for (int t = 0; t < 3; t++) {
+                    const uint64_t da = dP + (t == 1 ? SM::P / 16 : 0), db = dV + (t == 2 ? SM::V / 16 : 0);
+#pragma unroll
+                    for (int kk = 0; kk < kAttnTK / 16; kk++) umma_f16(tO, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), idO, (j > 0 || t > 0 || kk > 0) ? 1u : 0u);
+                }
+            }
+            if (lead) {
+                umma_commit(v_empty + 8u * b);
+                umma_commit(pv_done);
+            }
+            __syncwarp();
         }
     } else {
         // threads t and t + 128 share query row t & 127 (TMEM lane t & 127): row r = (token t0 + r / G, head kh * G + r % G); they split every tile's 64

@@ -4162,7 +4162,6 @@ extern "C" int b200_debug_set_position(b200_ctx* c, int seq, uint64_t pos) {
     CU(cudaSetDevice(c->par.device));
     CU(cudaStreamSynchronize(c->stream));
     const int p = (int)pos;
-    CU(cudaStreamSynchronize(c->stream));
     CU(cudaMemcpy(&c->slots[seq].d_state->pos_next, &p, sizeof(int), cudaMemcpyHostToDevice));
     c->slots[seq].host_pos = pos;
     return B200_OK;

@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     t.rows = a.seg ? a.seg[2 * t.z + 1] : a.R;
     if (t.t0 >= t.rows) return;             // (the whole cluster)
     uint8_t* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * NS, acc_full = bar + 16u * NS;
     tc_setup(tid, warp, bar, NS, &s_tmem, 1, TN);
     if (!a.seg && (TC_W_WAITS || warp != TC_LOAD_W)) wait_grid();   // (other weights do not depend on the kernel before)

@@ -172,81 +172,77 @@ __global__ void __launch_bounds__(192, 2) lp_tile_attn_kernel(const __grid_const
     auto place = [&](int t) { return t < nA ? t : t + t_lo; };
     auto position = [&](int t) { return t < nA ? t * KA_K : start + (t - nA + t_lo) * KA_K; };
     if (warp == 4) {
-        {
-            int asked_k = 0, asked_v = 0;
-            for (int t = 0; t < n_tiles; t++) {
-                const uint32_t b = t & 1, ph = ((t >> 1) & 1) ^ 1;
-                const int col = (before + place(t)) * KA_K;
-                tc_wait(k_empty + 8u * b, ph, alive, err, 21);
-                alive = __all_sync(0xffffffffu, alive);
-                if (!alive) break;
-                if (tc_elect()) {
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(k_full + 8u * b), "r"((uint32_t)SM::K) : "memory");
-                    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(base + SM::K_AT + b * SM::K),
-                                 "l"(&kmap), "r"(0), "r"(g * cols + col), "r"(0), "r"(k_full + 8u * b)
-                                 : "memory");
-                }
-                __syncwarp();
-                asked_k = t + 1;
-                tc_wait(v_empty + 8u * b, ph, alive, err, 22);
-                alive = __all_sync(0xffffffffu, alive);
-                if (!alive) break;
-                if (tc_elect()) {
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(v_full + 8u * b), "r"((uint32_t)SM::V) : "memory");
-                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(base + SM::V_AT + b * SM::V),
-                                 "l"(&vmap), "r"(col), "r"(g * DVP), "r"(v_full + 8u * b)
-                                 : "memory");
-                }
-                __syncwarp();
-                asked_v = t + 1;
+        int asked_k = 0, asked_v = 0;
+        for (int t = 0; t < n_tiles; t++) {
+            const uint32_t b = t & 1, ph = ((t >> 1) & 1) ^ 1;
+            const int col = (before + place(t)) * KA_K;
+            tc_wait(k_empty + 8u * b, ph, alive, err, 21);
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            if (tc_elect()) {
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(k_full + 8u * b), "r"((uint32_t)SM::K) : "memory");
+                asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(base + SM::K_AT + b * SM::K),
+                             "l"(&kmap), "r"(0), "r"(g * cols + col), "r"(0), "r"(k_full + 8u * b)
+                             : "memory");
             }
-            if (!alive) {               // gave up: what has been asked for lands first (bounded)
-                auto land = [&](uint32_t full, int asked) {
-                    ring_in_flight<2>(asked, [&](int stage, unsigned parity) {
-                        bool w = true;
-                        tc_wait(full + 8u * stage, parity, w, nullptr, 0);
-                    });
-                };
-                land(k_full, asked_k);
-                land(v_full, asked_v);
+            __syncwarp();
+            asked_k = t + 1;
+            tc_wait(v_empty + 8u * b, ph, alive, err, 22);
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            if (tc_elect()) {
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(v_full + 8u * b), "r"((uint32_t)SM::V) : "memory");
+                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(base + SM::V_AT + b * SM::V),
+                             "l"(&vmap), "r"(col), "r"(g * DVP), "r"(v_full + 8u * b)
+                             : "memory");
             }
+            __syncwarp();
+            asked_v = t + 1;
+        }
+        if (!alive) {               // gave up: what has been asked for lands first (bounded)
+            auto land = [&](uint32_t full, int asked) {
+                ring_in_flight<2>(asked, [&](int stage, unsigned parity) {
+                    bool w = true;
+                    tc_wait(full + 8u * stage, parity, w, nullptr, 0);
+                });
+            };
+            land(k_full, asked_k);
+            land(v_full, asked_v);
         }
     } else if (warp == 5) {
-        {
-            const uint32_t id_s = tc_idesc(KA_Q, KA_K), id_o = tc_idesc(KA_Q, DVP);
-            const uint64_t dq = tc_desc(base), dp = tc_desc(base + SM::P_AT);
-            auto scores = [&](int t) {
-                const uint32_t b = t & 1, ph = (t >> 1) & 1;
-                tc_wait(k_full + 8u * b, ph, alive, err, 23);
-                tc_wait(s_empty + 8u * b, ph ^ 1, alive, err, 24);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                alive = __all_sync(0xffffffffu, alive);
-                const bool lead = tc_elect();
-                if (lead && alive) ka_mma(tmem + b * KA_K, dq, tc_desc(base + SM::K_AT + b * SM::K), id_s, DKP / 64, KA_Q * 8, KA_K * 8, true);
-                if (lead) {
-                    tc_commit(k_empty + 8u * b);
-                    tc_commit(s_full + 8u * b);
-                }
-                __syncwarp();
-            };
-            tc_wait(q_full, 0, alive, err, 25);
+        const uint32_t id_s = tc_idesc(KA_Q, KA_K), id_o = tc_idesc(KA_Q, DVP);
+        const uint64_t dq = tc_desc(base), dp = tc_desc(base + SM::P_AT);
+        auto scores = [&](int t) {
+            const uint32_t b = t & 1, ph = (t >> 1) & 1;
+            tc_wait(k_full + 8u * b, ph, alive, err, 23);
+            tc_wait(s_empty + 8u * b, ph ^ 1, alive, err, 24);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            scores(0);
-            for (int t = 0; t < n_tiles; t++) {
-                const uint32_t b = t & 1, ph = (t >> 1) & 1;
-                if (t + 1 < n_tiles) scores(t + 1);
-                tc_wait(v_full + 8u * b, ph, alive, err, 26);
-                tc_wait(p_full, t & 1, alive, err, 27);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                alive = __all_sync(0xffffffffu, alive);
-                const bool lead = tc_elect();
-                if (lead && alive) ka_mma(tO, dp, tc_desc(base + SM::V_AT + b * SM::V), id_o, 1, 0, 0, t == 0);
-                if (lead) {
-                    tc_commit(v_empty + 8u * b);
-                    tc_commit(pv_done);
-                }
-                __syncwarp();
+            alive = __all_sync(0xffffffffu, alive);
+            const bool lead = tc_elect();
+            if (lead && alive) ka_mma(tmem + b * KA_K, dq, tc_desc(base + SM::K_AT + b * SM::K), id_s, DKP / 64, KA_Q * 8, KA_K * 8, true);
+            if (lead) {
+                tc_commit(k_empty + 8u * b);
+                tc_commit(s_full + 8u * b);
             }
+            __syncwarp();
+        };
+        tc_wait(q_full, 0, alive, err, 25);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        scores(0);
+        for (int t = 0; t < n_tiles; t++) {
+            const uint32_t b = t & 1, ph = (t >> 1) & 1;
+            if (t + 1 < n_tiles) scores(t + 1);
+            tc_wait(v_full + 8u * b, ph, alive, err, 26);
+            tc_wait(p_full, t & 1, alive, err, 27);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            alive = __all_sync(0xffffffffu, alive);
+            const bool lead = tc_elect();
+            if (lead && alive) ka_mma(tO, dp, tc_desc(base + SM::V_AT + b * SM::V), id_o, 1, 0, 0, t == 0);
+            if (lead) {
+                tc_commit(v_empty + 8u * b);
+                tc_commit(pv_done);
+            }
+            __syncwarp();
         }
     } else {
         const int f = min(f0 + tid, rows - 1), tok = f / hpg, h = g * hpg + f - tok * hpg, i = p0 + tok;
