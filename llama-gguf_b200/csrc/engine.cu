@@ -259,7 +259,9 @@ struct b200_ctx {
     size_t h_batch_logits_bytes = 0;
     int* pf_argmax = nullptr;        // batched decode with the pick on the device: [rows]
     int pf_argmax_rows = 0;
-    int batch_gemm_min = 8;    // measured crossover on Llama-3-8B: a GEMM pass costs ~12 ms up to 32 rows, a sequence alone 2 ms
+    // Sequences that a batched step takes as rows.  For time alone it could be two: a pass of Llama-3-8B costs 2.7 ms for 2 rows and 2.8 for 8 with the pick on the device,
+    // a sequence alone 2.0 ms.  But rows round their activations to fp16 (5e-4 of the logits), a sequence alone is within 2e-6: fewer than eight keep that.
+    int batch_gemm_min = 8;
     uint64_t prefill_gemm_tokens = 0;
     int* h_err = nullptr;   // pinned copy of the first watchdog word, fetched with every synchronising call
     int* h_token = nullptr;          // [kTokenRing]: tokens on their way to the device
@@ -1868,7 +1870,9 @@ static int umma_tmaps_build(b200_ctx* c) {
     CU_ALLOC(late_malloc(c, (void**)&c->pf_tmaps, maps.size() * sizeof(CUtensorMap)));
     CU(cudaMemcpy(c->pf_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     const b200_model_desc& d = c->d;
-    // whole blocks of 256 in every row; narrower than 1024, a layer's products are a microsecond of work either way and keep the kernels they had (tests pin their count)
+    // Whole blocks of 256 in every row, and 1024 wide at least: narrower models gain as well, but not at every length (two-pass or fused products -> these, prompts of 33 /
+    // 64 / 128 / 256 tokens through four layers: 512 wide, ffn 2048, Q4_K 389 / 431 / 291 / 315 -> 218 / 231 / 243 / 251 us; 768 wide 442 / 521 / 399 / 732 -> 226 / 265 /
+    // 436 / 517), and tests pin the launches of the kernels they have
     c->few_able = env_int("B200_FEW_GEMM", 1) != 0 && d.hidden % 256 == 0 && d.hidden >= 1024 && d.hidden <= kFewNormMax && d.n_heads * d.head_dim % 256 == 0 && d.ffn % 256 == 0;
     auto fits = [&](std::initializer_list<const DevTensor*> ws) {      // in the 32-bit arithmetic of the deal, at any number of rows
         FewPlan pl;

@@ -5,11 +5,12 @@
 // (the contraction the reference runs as T GEMVs per matrix: src/model/llama.rs:327-345; block arithmetic src/tensor/quant/dequant.rs:103-109,
 // 205-356).  Up to 64 tokens a weight byte meets too few products to matter to the tensor pipe; what counts is unpacking at the rate DRAM delivers.
 //
-//  * Weights enter the tensor core as INTEGERS: q * sc (6-bit scale times a 4- or 5-bit quant, at most 1953; int8 scale times 6 bits for Q6_K) is an
-//    fp16 number, one LOP3 and one HFMA2 for two weights.  The block's f32 factor d multiplies the sum of its 256 products instead of every
+//  * Weights enter the tensor core as INTEGERS: q * sc (6-bit scale times a 4- or 5-bit quant, at most 1953: an fp16 number; int8 scale times 6 bits for Q6_K, which
+//    fp16 rounds to even numbers above 2048), one LOP3 and one HFMA2 for two weights.  The block's f32 factor d multiplies the sum of its 256 products instead of every
 //    weight, when the block's accumulator is drained (T / 2 FMAs per 256 weights and thread).  The minimum term -dmin sum_s m_s X_s (X_s = sum of the 32
-//    activations of sub-block s) is two more K steps of a tf32 product: dmin m_s has 17 bits, X_s is carried as two tf32 numbers.  So the weights are exact,
-//    and only the activations are rounded (to fp16, as in gemm_umma2.cuh, which rounds each dequantised weight to fp16 too).
+//    activations of sub-block s) is two more K steps of a tf32 product: dmin m_s has 17 bits, X_s is carried as two tf32 numbers.  So Q4_K and
+//    Q5_K weights are exact; Q6_K ones are rounded where |q sc| > 2048 (2^-12 of themselves), and Q8_0 ones once, since no factor is common to 256 of them.  Activations
+//    are rounded to fp16 (as in gemm_umma2.cuh, which rounds each dequantised weight to fp16 too).
 //  * The unpacked operand goes to TENSOR MEMORY (tcgen05.st, thread = weight row) and never through shared memory: 128 x 256 weights written and
 //    read back there would cost 1024 clocks of its bandwidth, where DRAM delivers the block in 790.
 //  * Activations come as an image of the shared-memory tiles (few_put8): one bulk copy per block of 256, no tensor map.
@@ -19,8 +20,9 @@
 // Roles: 2 groups of 128 threads that unpack every other unit each and add up what its products gave (the sums of the two meet at a piece's end, through
 // tensor memory); a warp that loads; a warp that issues the MMAs.  They meet through mbarriers only; every wait is bounded and reports through `err`.
 //
-// What bounds it: unpacking, about 700 instructions per unit and warp (LOP3 and shifts at half rate), 1450 clocks per unit of Q4_K where DRAM needs 790;
-// and 5 us of launch, fill and drain.  Measured back to back (weights from DRAM), 32 tokens, the seven products of an 8B layer: gate and up 23.4 us (2.8 TB/s; the
+// What bounds it: unpacking, about 700 instructions per unit and warp (LOP3 and shifts at half rate), 1450 clocks per unit of Q4_K where DRAM needs 790.  No unit of the
+// SM is full meanwhile (counters of gate and up, 32 tokens: issue slots 37 %, tensor pipe 13 %, DRAM 27 % of a cold launch): a scheduler has two unpacking warps, and what
+// they wait for is their own chains.  And 5 us of launch, fill and drain.  Measured back to back (weights from DRAM), 32 tokens, the seven products of an 8B layer: gate and up 23.4 us (2.8 TB/s; the
 // fused kernel 86), down Q4_K 14.8 (35), Q6_K 18.1, q / k / v 9.3, o 7.5; gate and up in Q8_0 26.4 us (4.7 TB/s), at 64 tokens 27.9 us.
 #pragma once
 #include <cuda.h>
@@ -32,8 +34,10 @@ namespace b200 {
 
 // Up to 256 tokens, in token tiles of 64 (the weights of a second tile come from L2).  Prompts through two 8B layers, against the two passes of prompt_f16.cuh or
 // the fused kernel, Q4_K_M / Q6_K / Q8_0 / Q5_K_M: 33 tokens 794 / 1005 / 876 / 1025 -> 585 / 645 / 621 / 627 us, 128 tokens 929 / 1060 / 1018 / 1139 -> 695 / 766 /
-// 730 / 741, 256 tokens 1024 / 1154 / 1108 / 1238 -> 887 / 1013 / 923 / 957; 2048-wide layers in Q8_0, 256 tokens: 561 -> 536.  Every token tile unpacks again, so
-// the gain is gone a tile or two above.
+// 730 / 741, 256 tokens 1024 / 1154 / 1108 / 1238 -> 887 / 1013 / 923 / 957; four 2048-wide layers (ffn 8192), 64 / 128 / 192 / 256 tokens: Q4_K_M 622 / 506 / 561 / 603 -> 390 / 459 / 529 /
+// 589; 1024-wide ones (ffn 4096) Q4_K 549 / 362 / 369 / 382 -> 278 / 312 / 349 / 378, Q8_0 324 / 360 / 388 / 380 -> 283 / 317 / 359 / 387.  Every token tile unpacks again,
+// so the gain is gone at 256 in the last of these, and a tile or two above in the others.  Batched decoding gains more, since what it replaces is the fused kernel (8 /
+// 33 / 128 / 256 sequences, two 8B layers: 439 / 538 / 1284 / 2040 -> 231 / 293 / 581 / 1363).
 constexpr int kFewTokens = 256;
 constexpr int kFewThreads = 384, kFewLoader = 8, kFewMma = 9;      // (warps 10 and 11 are there for the register split: it goes by warpgroups)
 constexpr int kFewRegsWork = 224, kFewRegsServe = 56;              // 256 x 224 + 128 x 56 = 384 x 168, what the block is launched with

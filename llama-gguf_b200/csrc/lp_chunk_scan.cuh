@@ -11,8 +11,8 @@
 // lp_chunk_prep_kernel does what does not need S0, a block per (chunk, head, run); lp_chunk_scan_kernel walks a run's chunks, a block per (8 state
 // columns, head, run) with the columns in shared memory and the next chunk's rows on their way.
 // What bounded the token-by-token form: a chain of two reductions per token (1370 clocks for the delta rule at 128 x 128), SMs mostly waiting.
-// Here a chunk's reductions are products of 64 x 128 by 8; the chain is per chunk.  1500 tokens, 8 heads of 128 x 128: delta rule 1044 -> 26 + 109 us;
-// 4 heads of 64 x 128: memory 656 -> 8 + 73 us.  The decay from s to t is multiplied up (MEM: its logarithm
+// Here a chunk's reductions are products of 64 x 128 by 8; the chain is per chunk.  1500 tokens, 8 heads of 128 x 128: delta rule 1044 -> 33 + 112 us;
+// 4 heads of 64 x 128: memory 656 -> 11 + 75 us (preparation + scan, each launched cold).  The decay from s to t is multiplied up (MEM: its logarithm
 // added up) from s on for every s, never a quotient or difference of running products, so it is as exact as one token after the other and a
 // decay of 0 stays 0.
 #pragma once
@@ -244,7 +244,7 @@ template <int DM, int PI, int SL, int RT> __device__ __forceinline__ void cs_row
 }
 // blockIdx.x: 8 columns of the state (MEM: 7 and the column of ones, whose state is n).
 // Two groups of eight warps.  The chain (threads 0 .. 255): W S0, U, the state after the chunk; the others: q S0 and the chunk's outputs, from the state before it, beside
-// the chain (the state has two buffers), and the copies of the rows two chunks ahead.  1500 tokens: delta rule 115 -> 109 us, memory 88 -> 73 us against one group of eight
+// the chain (the state has two buffers), and the copies of the rows two chunks ahead.  1500 tokens, back to back: delta rule 115 -> 109 us, memory 88 -> 73 us against one group of eight
 // warps for all of it with the rows one chunk ahead; bound by the chain's shared-memory loads (delta: W S0, U, the update, 2.3 us per chunk).
 template <int MODE, int DM>
 __global__ void __launch_bounds__(CS_SCAN_THREADS) lp_chunk_scan_kernel(StepMeta sm, ChunkScan g) {
