@@ -2,7 +2,7 @@
 b200_prefill, against the oracle's token-by-token LlamaModel::forward (src/model/llama.rs:275-362).
 
 Tolerance: 1e-3 relative (max|a-b| / max|b|) on the logits.  This path rounds both GEMM operands to fp16 (f32
-accumulation in TMEM); measured on these cases (scripts/gemm_err.py on a B200): 0.9e-4 ... 5.3e-4, so it holds the same
+accumulation in TMEM); measured on these cases on a B200: 0.9e-4 ... 5.3e-4, so it holds the same
 bound as the exact token-by-token entry points (which measure ~2e-6).  The KV cache it leaves must let the exact decode
 path continue within the same bound."""
 import os
