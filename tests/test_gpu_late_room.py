@@ -1,6 +1,8 @@
 """Batched decode steps of a context that finds no room on the device for what it has to allocate after loading.
 
 Tolerance: that of test_gpu_few_rows.py for rows of fp16 activations, 1e-3 of the largest logit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -22,9 +24,22 @@ def tokens(n, k):
     return np.random.default_rng([n, k]).integers(0, 5000, n).astype(np.uint32)
 
 
-def fill(leave):
-    torch.cuda.empty_cache()
-    return torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+class Full:
+    """All device memory but less than 4 MB in one piece, taken straight from the driver (the caching allocator rounds, and what free memory there is may be in pieces)."""
+
+    def __init__(self):
+        torch.cuda.empty_cache()
+        self.rt, self.at = C.CDLL("libcudart.so.12"), []
+        for size in [(1 << 30) * 16, 1 << 30, 1 << 26, 1 << 24, 1 << 22]:
+            p = C.c_void_p()
+            while self.rt.cudaMalloc(C.byref(p), C.c_size_t(size)) == 0:
+                self.at.append(p)
+                p = C.c_void_p()
+            self.rt.cudaGetLastError()
+
+    def free(self):
+        for p in self.at:
+            assert self.rt.cudaFree(p) == 0
 
 
 def test_a_step_that_failed_leaves_a_context_that_works(b200, monkeypatch):
@@ -37,11 +52,12 @@ def test_a_step_that_failed_leaves_a_context_that_works(b200, monkeypatch):
         try:
             got = [gpu.decode_batch(list(range(8)), tokens(8, 0))]
             if full:
-                block = fill(3 << 20)
-                with pytest.raises(b200.AllocationFailed):
-                    gpu.decode_batch(list(range(ROWS)), tokens(ROWS, 1))
-                del block
-                torch.cuda.empty_cache()
+                block = Full()
+                try:
+                    with pytest.raises(b200.AllocationFailed):
+                        gpu.decode_batch(list(range(ROWS)), tokens(ROWS, 1))
+                finally:
+                    block.free()
             got += [gpu.decode_batch(list(range(8)), tokens(8, k)) for k in (2, 3, 4)]
             out.append(got)
         finally:
@@ -59,21 +75,21 @@ def test_buffers_of_few_rows_are_given_back(b200, monkeypatch):
     for few in ("0", "1"):      # (the first also loads the kernels that the full device needs)
         monkeypatch.setenv("B200_FEW_GEMM", few)
         gpu = b200.GpuOnlyInference(desc, tensors)
-        block = None
+        blocks = []
         try:
             out[few], launches[few] = [], []
             for k, (n, seed) in enumerate(calls):
-                if few == "1" and k == 3:
-                    block = fill(3 << 20)
-                if few == "1" and k == 4:        # what was given back is taken as well
-                    more = fill(1 << 20)
+                if few == "1" and k in (3, 4):        # (at 4: what was given back is taken as well)
+                    blocks.append(Full())
                 if few == "1" and k == 5:
-                    del block, more
-                    torch.cuda.empty_cache()
+                    while blocks:
+                        blocks.pop().free()
                 before = gpu.stats()["kernel_launches"]
                 out[few].append(gpu.decode_batch(list(range(n)), tokens(n, seed)))
                 launches[few].append(gpu.stats()["kernel_launches"] - before)
         finally:
+            for b in blocks:
+                b.free()
             gpu.close()
     few_path = 8 * desc["n_layers"] + 6
     assert [x == few_path for x in launches["1"]] == [True] * 3 + [False] * 2 + [True] * 2, launches
