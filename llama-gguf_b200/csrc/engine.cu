@@ -245,6 +245,7 @@ struct b200_ctx {
     bool few_head = false;           // ... and the head of batched decoding
     uint8_t* few_img[3] = {};        // images of the activations: normed rows, attention, gated units
     float* few_part = nullptr;       // pieces of cut tiles
+    SpareRetry few_retry;            // ... where there was no room for these
     bool pf_tmaps_built = false;
     size_t pf_split_floats = 0;
     int pf_logits_rows = 0;
@@ -1021,7 +1022,14 @@ static cudaError_t launch_attn(b200_ctx* c, const AttnParams& ap, int hd, int G)
     return launch_k(c, attn_decode_kernel<64, 8>, grid, dim3(kAttnThreads), attn_smem_bytes(64, 8, ap.n_splits, ap.G), ap);
 }
 
-// Enqueue every kernel of one token for `slot` on c->stream (captured into a graph by the caller).
+// Captured steps of batched decoding whose kernels or buffers are others from now on.
+static void drop_batch_graphs(b200_ctx* c) {
+    for (auto& bg : c->batch_graphs) {
+        if (bg.exec) cudaGraphExecDestroy(bg.exec);
+        bg = b200_ctx::BatchGraph();
+    }
+}
+
 // Device memory that a call after loading has to have: the prompts' fp16 weight rows and the buffers of the products of few rows, which the fused products can do
 // without, go first when there is no room (and with the latter the captured steps that name them).  Never called inside a capture
 static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
@@ -1035,10 +1043,7 @@ static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
             c->pf_w16_elems = 0;
             if (c->few_part) {
                 cudaStreamSynchronize(c->stream);
-                for (auto& bg : c->batch_graphs) {
-                    if (bg.exec) cudaGraphExecDestroy(bg.exec);
-                    bg = b200_ctx::BatchGraph();
-                }
+                drop_batch_graphs(c);
                 for (uint8_t*& q : c->few_img) {
                     cudaFree(q);
                     q = nullptr;
@@ -1049,6 +1054,7 @@ static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
             return true;
         });
 }
+// Enqueue every kernel of one token for `slot` on c->stream (captured into a graph by the caller).
 static cudaError_t enqueue_token(b200_ctx* c, int slot_i, Mode mode, bool only_gemv = false) {
     const b200_model_desc& d = c->d;
     Slot& sl = c->slots[slot_i];
@@ -1955,7 +1961,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     }
     // products of few rows (gemm_few.cuh): images of the activations and pieces of cut tiles; a device without room for them keeps the other products
     const int few_max = kFewTokens, last_chunk = n % cap ? n % cap : cap;
-    if (c->few_able && c->kv_format == 0 && !c->few_part && last_chunk <= few_max) {
+    if (c->few_able && c->kv_format == 0 && !c->few_part && last_chunk <= few_max && c->few_retry.due()) {
         const size_t bytes[4] = {few_image_bytes(few_max, 64, H), few_image_bytes(few_max, 64, A), few_image_bytes(few_max, 64, I), (size_t)2 * c->n_sm * 64 * 128 * sizeof(float)};
         void* got[4] = {};
         bool ok = true;
@@ -1963,9 +1969,12 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (!ok) {
             cudaGetLastError();
             for (void* q : got) cudaFree(q);
+            c->few_retry.failed();
         } else {
             for (int i = 0; i < 3; i++) c->few_img[i] = (uint8_t*)got[i];
             c->few_part = (float*)got[3];
+            c->few_retry.got();
+            drop_batch_graphs(c);      // (steps captured without them)
         }
     }
     // batched decode: per-row (position, KV base of the slot, SeqState of the slot)
@@ -2013,10 +2022,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             c->pf_logits_rows = 0;      // (until there is one again)
             CU_ALLOC(late_malloc(c, (void**)&c->pf_logits, (size_t)n * d.vocab * sizeof(float)));
             c->pf_logits_rows = n;
-            for (auto& bg : c->batch_graphs) {   // (the captured head GEMMs write the old buffer)
-                if (bg.exec) cudaGraphExecDestroy(bg.exec);
-                bg = b200_ctx::BatchGraph();
-            }
+            drop_batch_graphs(c);      // (the captured head GEMMs write the old buffer)
         }
     }
     // CUDA graph of the step (rows mode): replay if this row count has one, capture on its second step (the first runs eagerly:

@@ -1,5 +1,6 @@
 """csrc/spare.cuh on the host.  With a device that has so much room, what has to be had takes the room of scratch that can be done without, once, and only
-when it has to; scratch that grows a little with every portion of a conversation is allocated a few times in all."""
+when it has to; scratch that grows a little with every portion of a conversation is allocated a few times in all; scratch that finds no room is asked for seldom, and again
+soon after there was room once."""
 import os
 import subprocess
 
@@ -46,8 +47,31 @@ int main() {
 }
 """
 
+RETRY = r"""
+#include <cstdio>
+#include "spare.cuh"
+int main() {
+    SpareRetry r;
+    for (int round = 0; round < 2; round++) {
+        int asked = 0, last = -1, most = 0;
+        for (int call = 0; call < 1000; call++)
+            if (r.due()) {
+                if (last < 0 && call != 0) return printf("first asked at %d\n", call), 1;
+                if (last >= 0) most = std::max(most, call - last - 1);
+                last = call;
+                asked++;
+                r.failed();
+            }
+        if (asked < 1000 / 65 || asked > 1000 / 65 + 8 || most != 64) return printf("asked %d times, at most %d calls between\n", asked, most), 1;
+        while (!r.due()) {}
+        r.got();
+    }
+    return 0;
+}
+"""
 
-@pytest.mark.parametrize("program", [PROGRAM, GROWTH], ids=["gives_back", "grows"])
+
+@pytest.mark.parametrize("program", [PROGRAM, GROWTH, RETRY], ids=["gives_back", "grows", "asks_again"])
 def test_on_the_host(tmp_path, program):
     (tmp_path / "t.cpp").write_text(program)
     exe = str(tmp_path / "t")
