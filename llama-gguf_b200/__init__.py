@@ -814,7 +814,8 @@ class GpuOnlyInference:
 
     def forward_batch(self, token_ids, seq=0):
         """GpuOnlyInference::forward_batch (src/backend/cuda/gpu_only.rs:776-790): the whole prompt, logits of its last
-        token.  Prompts of >= 32 tokens of an eligible dense model run through the tcgen05 dequant-GEMM (fp16 operands)."""
+        token.  Prompts of >= 32 tokens of an eligible dense model run through the tcgen05 dequant-GEMM (fp16 operands),
+        shorter ones and those of block types it does not know as rows in f32."""
         toks = np.ascontiguousarray(token_ids, dtype=np.uint32)
         logits = np.empty(self.vocab, dtype=np.float32)
         _check(lib().b200_prefill(self._h, seq, toks.ctypes.data_as(C.POINTER(C.c_uint32)), toks.size, _fp(logits)))

@@ -435,6 +435,33 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(const AttnPar
     attn_decode_item<HD, GMAX, kAttnWarps>(p, blockIdx.x, blockIdx.y, kv_len, sm, &s_ticket);
 }
 
+// The same for several rows (blockIdx.z): consecutive positions of one sequence, or rows of their own sequences (row_pos, row_kv).  Queries rotated, caches written.
+struct AttnRows {
+    int ldq, ldo, pos0;
+    long long part_row;        // floats of p.part per row; tickets: p.n_kv per row
+    const int* row_pos;
+    float* const* row_kv;
+    long long k_off, v_off;
+};
+template <int HD, int GMAX>
+__global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnParams p0, const AttnRows r) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ unsigned int s_ticket;
+    pdl_launch_dependents();
+    pdl_wait();
+    AttnParams p = p0;
+    const int z = blockIdx.z;
+    p.q += (size_t)z * r.ldq;
+    p.out += (size_t)z * r.ldo;
+    p.part += (size_t)z * r.part_row;
+    p.tickets += (size_t)z * p.n_kv;
+    if (r.row_pos) {
+        p.k_cache = r.row_kv[z] + r.k_off;
+        p.v_cache = r.row_kv[z] + r.v_off;
+    }
+    attn_decode_item<HD, GMAX, kAttnWarps>(p, blockIdx.x, blockIdx.y, (r.row_pos ? r.row_pos[z] : r.pos0 + z) + 1, sm, &s_ticket);
+}
+
 // floats of shared memory attn_decode_item needs
 __host__ __device__ inline size_t attn_item_floats(int hd, int gmax, int nw, int n_splits, int G) {
     size_t a = (size_t)(2 * nw * gmax + nw * gmax * hd + gmax * hd), b = (size_t)n_splits * G * (hd + 2);

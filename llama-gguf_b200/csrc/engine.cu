@@ -34,6 +34,7 @@
 #include "gemm_umma.cuh"
 #include "gemm_umma2.cuh"
 #include "few_rows.cuh"
+#include "exact_rows.cuh"
 #include "prompt_f16.cuh"
 #include "prompt_rows.cuh"
 #include "ahead.cuh"
@@ -246,6 +247,12 @@ struct b200_ctx {
     uint8_t* few_img[3] = {};        // images of the activations: normed rows, attention, gated units
     float* few_part = nullptr;       // pieces of cut tiles
     SpareRetry few_retry;            // ... where there was no room for these
+    // products of several rows in f32 (exact_rows.cuh): activations, pieces of cut products, attention partials and tickets of up to er_rows rows
+    bool exact_rows = true;          // B200_EXACT_ROWS=0: such prompts and steps token by token
+    float* er_buf = nullptr;
+    unsigned int* er_tickets = nullptr;
+    int er_rows = 0;
+    SpareRetry er_retry;
     bool pf_tmaps_built = false;
     size_t pf_split_floats = 0;
     int pf_logits_rows = 0;
@@ -261,7 +268,7 @@ struct b200_ctx {
     int* pf_argmax = nullptr;        // batched decode with the pick on the device: [rows]
     int pf_argmax_rows = 0;
     // Sequences that a batched step takes as rows.  For time alone it could be two: a pass of Llama-3-8B costs 2.7 ms for 2 rows and 2.8 for 8 with the pick on the device,
-    // a sequence alone 2.0 ms.  But rows round their activations to fp16 (5e-4 of the logits), a sequence alone is within 2e-6: fewer than eight keep that.
+    // a sequence alone 2.0 ms.  But rows round their activations to fp16 (5e-4 of the logits), a sequence alone is within 2e-6: fewer than eight keep that (exact_rows.cuh).
     int batch_gemm_min = 8;
     uint64_t prefill_gemm_tokens = 0;
     int* h_err = nullptr;   // pinned copy of the first watchdog word, fetched with every synchronising call
@@ -373,6 +380,7 @@ extern "C" int b200_ctx_create(const b200_model_desc* desc, const b200_parallel_
         if (kf && (!strcmp(kf, "int8") || !strcmp(kf, "1"))) c->kv_format = 1;
         c->kv_int8_gemm = env_int("B200_KV_INT8_GEMM", 0) != 0;
     }
+    c->exact_rows = env_int("B200_EXACT_ROWS", 1) != 0;
     c->prefill_gemm_min = std::max(1, env_int("B200_PREFILL_GEMM_MIN", 32));
     c->prefill_queue = env_int("B200_PREFILL_QUEUE", 0) != 0;
     c->prompt_f16_min = std::max(0, env_int("B200_PROMPT_F16_MIN", 0));
@@ -825,6 +833,10 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         CU(cudaFuncSetAttribute(attn_decode_kernel<128, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
         CU(cudaFuncSetAttribute(attn_decode_kernel<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
         CU(cudaFuncSetAttribute(attn_decode_kernel<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
+        CU(cudaFuncSetAttribute(rows_tile_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsTileSmem<8>));
+        CU(cudaFuncSetAttribute(rows_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<128>));
+        CU(cudaFuncSetAttribute(rows_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<64>));
+        for (auto k : {attn_rows_kernel<128, 4>, attn_rows_kernel<128, 8>, attn_rows_kernel<64, 4>, attn_rows_kernel<64, 8>}) CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
     }
     c->finalized = true;
     if (c->par.world_size > 1) {
@@ -934,6 +946,8 @@ extern "C" void b200_ctx_destroy(b200_ctx* c) {
     cudaFree(c->pf_tmaps);
     for (uint8_t* p : c->few_img) cudaFree(p);
     cudaFree(c->few_part);
+    cudaFree(c->er_buf);
+    cudaFree(c->er_tickets);
     cudaFree(c->pf_tile_cnt);
     cudaFree(c->attn_q8_part);
     cudaFree(c->pf_k16);
@@ -1030,14 +1044,27 @@ static void drop_batch_graphs(b200_ctx* c) {
     }
 }
 
-// Device memory that a call after loading has to have: the prompts' fp16 weight rows and the buffers of the products of few rows, which the fused products can do
-// without, go first when there is no room (and with the latter the captured steps that name them).  Never called inside a capture
+static void exact_rows_free(b200_ctx* c) {
+    if (c->er_buf) {
+        cudaStreamSynchronize(c->stream);
+        drop_batch_graphs(c);
+    }
+    cudaFree(c->er_buf);
+    cudaFree(c->er_tickets);
+    c->er_buf = nullptr;
+    c->er_tickets = nullptr;
+    c->er_rows = 0;
+}
+
+// Device memory that a call after loading has to have: the prompts' fp16 weight rows, the buffers of the products of few rows and those of the f32 rows, which the
+// calls can do without, go first when there is no room (and with the latter two the captured steps that name them).  Never called inside a capture
 static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
     return (cudaError_t)alloc_or_give_back(
         [&] { return (int)cudaMalloc(p, bytes); },
         [&] {
             cudaGetLastError();
-            if (!c->pf_w16 && !c->few_part) return false;
+            if (!c->pf_w16 && !c->few_part && !c->er_buf) return false;
+            exact_rows_free(c);
             cudaFree(c->pf_w16);
             c->pf_w16 = nullptr;
             c->pf_w16_elems = 0;
@@ -1938,22 +1965,222 @@ static bool prefill_gemm_ok(const b200_ctx* c, bool prompt = false) {
     return true;
 }
 
+// ------------------------------------------------------------------ rows in f32 (exact_rows.cuh)
+// Up to kExactFew rows go through the kernel that shares a weight between the rows of a warp pass, eight at a time; more through tiles.
+constexpr int kExactFew = 32;
+constexpr int kNoRoom = -1000;      // (prefill_gemm: nothing has been computed for want of the buffers; the caller goes token by token)
+
+// What n rows may take this path: dense single-GPU models whose rows the f32 kernels read as they lie; with the int8 cache prompts of fewer than 32 tokens
+// (tests pin the launches of longer ones)
+static bool exact_rows_ok(const b200_ctx* c, int n, bool prompt) {
+    const b200_model_desc& d = c->d;
+    if (!c->exact_rows || !c->use_prefill_gemm || n < 2 || c->par.world_size > 1 || d.n_experts > 0 || c->use_taps) return false;
+    if (!prompt && n > kExactFew) return false;
+    if (c->kv_format == 1 && (!prompt || n >= 32)) return false;
+    const int H = d.hidden, A = d.n_heads * d.head_dim, I = (int)d.ffn;
+    if (H % 32 || A % 32 || I % 32) return false;
+    auto ok = [](const DevTensor& w, int K) {
+        if (!w.present() || (int)w.ne[0] != K) return false;
+        const int be = type_block_elems(w.type);
+        const bool words = w.type == T_Q4_K || w.type == T_Q5_K || w.type == T_F16 || w.type == T_F32;      // (read by 16 bytes; the others by 2)
+        return be > 0 && K % be == 0 && ((uintptr_t)w.d & (words ? 15 : 1)) == 0 && (words ? w.row_bytes % 16 : w.row_bytes % 2) == 0;
+    };
+    for (const Layer& L : c->layers)
+        if (!ok(L.wq, H) || !ok(L.wk, H) || !ok(L.wv, H) || !ok(L.wo, A) || !ok(L.gate, H) || !ok(L.up, H) || !ok(L.down, I) || L.gate.type != L.up.type) return false;
+    return ok(c->output.present() ? c->output : c->token_embd, H);
+}
+
+struct ExactRoom {      // offsets in floats, for up to `rows` rows
+    size_t x, xn, qkv, at, act, part, floats, part_floats, attn_row;
+};
+static ExactRoom exact_room(const b200_ctx* c, int rows) {
+    const b200_model_desc& d = c->d;
+    const size_t H = d.hidden, A = (size_t)d.n_heads * d.head_dim, I = (size_t)d.ffn, QKV = A + (size_t)2 * d.n_kv_heads * d.head_dim, n = rows;
+    const int G = d.n_heads / d.n_kv_heads;
+    ExactRoom r{};
+    auto up = [](size_t v) { return (v + 31) & ~(size_t)31; };
+    r.x = 0;
+    r.xn = r.x + up(n * H);
+    r.qkv = r.xn + up(n * H);
+    r.at = r.qkv + up(n * QKV);
+    r.act = r.at + up(n * A);
+    r.part = r.act + up(n * I);
+    // pieces of a product (two waves of 64 x 64 tiles, or one uncut), or the partial attention of few rows
+    const size_t widest = std::max({H, QKV, 2 * I});
+    r.attn_row = (size_t)d.n_kv_heads * std::max(c->n_splits, c->attn_q8_splits) * G * (d.head_dim + 2);
+    r.part_floats = up(std::max(rows > kExactFew ? n * widest + (size_t)4 * c->n_sm * 64 * 128 : 0, kExactFew * r.attn_row));
+    r.floats = r.part + r.part_floats;
+    return r;
+}
+static bool exact_rows_room(b200_ctx* c, int n) {
+    const int cap = std::max(kExactFew, std::min(prefill_chunk(), c->d.max_seq_len)), rows = n <= kExactFew ? kExactFew : cap;
+    if (c->er_rows >= rows) return true;
+    if (!c->er_retry.due()) return false;
+    exact_rows_free(c);
+    const size_t tickets = (size_t)kExactFew * c->d.n_kv_heads * sizeof(unsigned int);
+    if (cudaMalloc((void**)&c->er_buf, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess || cudaMalloc((void**)&c->er_tickets, tickets) != cudaSuccess ||
+        cudaMemset(c->er_tickets, 0, tickets) != cudaSuccess) {
+        cudaGetLastError();
+        exact_rows_free(c);
+        c->er_retry.failed();
+        return false;
+    }
+    c->er_rows = rows;
+    c->er_retry.got();
+    return true;
+}
+
+struct ExactPass {
+    int T, pos0;                  // rows; position of the first (prompts)
+    bool rows;                    // every row its own sequence: positions, caches
+    const int* d_pos;
+    float* const* d_kv;
+    cudaStream_t st;
+    bool pdl;
+};
+// The layers over T rows of X (embedding rows on entry, the residual stream on return)
+static int exact_layers(b200_ctx* c, Slot& sl, const ExactPass& e) {
+    const b200_model_desc& d = c->d;
+    const int H = d.hidden, hd = d.head_dim, nh = d.n_heads, nkv = d.n_kv_heads, A = nh * hd, I = (int)d.ffn, QKV = (nh + 2 * nkv) * hd, T = e.T, G = nh / nkv;
+    const ExactRoom room = exact_room(c, c->er_rows);
+    float *X = c->er_buf + room.x, *XN = c->er_buf + room.xn, *Q = c->er_buf + room.qkv, *AT = c->er_buf + room.at, *HB = c->er_buf + room.act, *PT = c->er_buf + room.part;
+    const size_t kv_layer = (size_t)2 * nkv * d.max_seq_len * hd, q8_rows = (size_t)2 * nkv * d.max_seq_len;
+    const bool q8 = c->kv_format == 1, few = T <= kExactFew;
+    const float scale = 1.0f / sqrtf((float)hd);
+    auto seg = [&](RowsSeg& s, const DevTensor& w, float* out, int ldo, const DevTensor* bias) {
+        s.w = (const uint8_t*)w.d; s.row_bytes = w.row_bytes; s.type = w.type; s.n_rows = (int)w.ne[1]; s.out = out; s.ldo = ldo;
+        s.bias = bias && bias->present() ? bias->f32() : nullptr;
+    };
+    auto go_few = [&](RowsParams& p) {
+        c->launches++;
+        return rows_few_launch(p, c->n_sm, e.pdl, e.st);
+    };
+    // Tiles of 64 weight rows x 128 rows of x, or 64 where that leaves less padding (a narrow tile reads shared memory twice for the same multiply-adds: taken at two
+    // thirds of the rows and below), K cut until two blocks are on every SM; `sum`: what the kernel behind adds
+    auto go_tile = [&](RowsParams& p, int ld, RowsSum& sum) {
+        int tiles = 0;
+        for (int s = 0; s < p.n_seg; s++) tiles += (p.seg[s].n_rows + kRowsBN - 1) / kRowsBN;
+        const int wide = (T + 127) / 128, slim = (T + 63) / 64;
+        const bool narrow = slim * 3 <= wide * 4;
+        const int all = tiles * (narrow ? slim : wide), steps = p.K / kRowsBK;
+        int z = std::max(1, std::min({(narrow ? 3 : 2) * c->n_sm / all, steps / 4, 16}));
+        while (z > 1 && (size_t)z * T * ld > room.part_floats) z--;
+        p.k_split = (steps + z - 1) / z * kRowsBK;
+        z = (p.K + p.k_split - 1) / p.k_split;
+        p.piece = (long long)T * ld;
+        sum = RowsSum{PT, z, ld, p.piece};
+        c->launches++;
+        return launch_on(e.st, e.pdl, narrow ? rows_tile_kernel<4> : rows_tile_kernel<8>, dim3((unsigned)tiles, (unsigned)(narrow ? slim : wide), (unsigned)z), dim3(128),
+                         narrow ? kRowsTileSmem<4> : kRowsTileSmem<8>, p);
+    };
+    RowsSum sum{};
+    for (int l = 0; l < d.n_layers; l++) {
+        Layer& L = c->layers[l];
+        float *kc = e.rows ? nullptr : sl.kv + (size_t)l * kv_layer, *vc = e.rows ? nullptr : kc + kv_layer / 2;
+        const long long k_off = (long long)((size_t)l * kv_layer), v_off = k_off + (long long)(kv_layer / 2);
+        signed char *k8 = q8 ? sl.kv8 + (size_t)l * q8_rows * hd : nullptr, *v8 = q8 ? k8 + q8_rows * hd / 2 : nullptr;
+        float *k8s = q8 ? sl.kv_scale + (size_t)l * q8_rows : nullptr, *v8s = q8 ? k8s + q8_rows / 2 : nullptr;
+        RowsParams p{};
+        p.T = T; p.eps = d.norm_eps; p.n_seg = 3; p.K = H;
+        if (few) {
+            seg(p.seg[0], L.wq, Q, QKV, &L.bq); seg(p.seg[1], L.wk, Q + A, QKV, &L.bk); seg(p.seg[2], L.wv, Q + A + nkv * hd, QKV, &L.bv);
+            p.x = X; p.ldx = H; p.norm_w = L.attn_norm.f32(); p.epi = EPI_STORE;
+            CU(go_few(p));
+        } else {
+            CU(launch_on(e.st, e.pdl, rows_norm_kernel, dim3(T), dim3(256), 0, X, sum, L.attn_norm.f32(), d.norm_eps, XN, H));
+            seg(p.seg[0], L.wq, PT, QKV, nullptr); seg(p.seg[1], L.wk, PT + A, QKV, nullptr); seg(p.seg[2], L.wv, PT + A + nkv * hd, QKV, nullptr);
+            p.x = XN; p.ldx = H;
+            CU(go_tile(p, QKV, sum));
+            CU(launch_on(e.st, e.pdl, rows_qkv_kernel, dim3((QKV + 255) / 256, T), dim3(256), 0, sum, L.bq.present() ? (const float*)L.bq.f32() : nullptr,
+                         L.bk.present() ? (const float*)L.bk.f32() : nullptr, L.bv.present() ? (const float*)L.bv.f32() : nullptr, A, nkv * hd, Q, QKV));
+            c->launches += 2;
+        }
+        if (q8) {
+            RopeKvQ8Params qp{};
+            qp.q = Q; qp.k8 = k8; qp.v8 = v8; qp.k_scale = k8s; qp.v_scale = v8s; qp.freq = c->rope_freq;
+            qp.n_heads = nh; qp.n_kv = nkv; qp.hd = hd; qp.max_seq = d.max_seq_len; qp.neox = d.rope_neox; qp.rope_scale = d.rope_scale;
+            CU(launch_on(e.st, e.pdl, hd == 128 ? prefill_rope_kv_q8_kernel<4> : prefill_rope_kv_q8_kernel<2>, dim3((nh + 2 * nkv + 3) / 4, T), dim3(128), 0, qp, QKV, e.pos0));
+            AttnQ8Params ap{};
+            ap.q = Q; ap.k8 = k8; ap.v8 = v8; ap.k_scale = k8s; ap.v_scale = v8s; ap.part = PT; ap.out = AT; ap.pos0 = e.pos0; ap.ldq = QKV; ap.ldo = A;
+            ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.scale = scale;
+            ap.n_splits = std::max(std::min(8, c->attn_q8_splits), std::min(c->attn_q8_splits, 2 * c->n_sm / (nkv * T)));      // (two blocks per SM)
+            ap.part_row = (long long)nkv * ap.n_splits * G * (hd + 2);
+            CU(launch_on(e.st, e.pdl, hd == 128 ? attn_q8_split_kernel<128, 4> : attn_q8_split_kernel<64, 4>, dim3(ap.n_splits, nkv, T), dim3(kAttnQ8Warps * 32), 0, ap));
+            CU(launch_on(e.st, e.pdl, attn_q8_merge_kernel, dim3(nh, 1, T), dim3(kAttnQ8MergeThreads), 0, ap, hd));
+            c->launches += 3;
+        } else {
+            PrefillRopeParams rp{};
+            rp.qkv = Q; rp.ld = QKV; rp.k_cache = kc; rp.v_cache = vc; rp.freq = c->rope_freq; rp.pos0 = e.pos0;
+            rp.n_heads = nh; rp.n_kv = nkv; rp.hd = hd; rp.max_seq = d.max_seq_len; rp.neox = d.rope_neox; rp.rope_scale = d.rope_scale;
+            if (e.rows) { rp.row_pos = e.d_pos; rp.row_kv = e.d_kv; rp.k_off = k_off; rp.v_off = v_off; }
+            CU(launch_on(e.st, e.pdl, prefill_rope_kv_kernel, dim3(T, T <= 64 ? 4 : 1), dim3(256), 0, rp));
+            if (few) {      // split over the keys as a single token's
+                AttnParams ap{};
+                ap.q = Q; ap.k_cache = kc; ap.v_cache = vc; ap.out = AT; ap.part = PT; ap.tickets = c->er_tickets;
+                ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.scale = scale;
+                ap.n_splits = std::max(1, std::min(c->n_splits, 2 * c->n_sm / (nkv * T)));
+                AttnRows ar{};
+                ar.ldq = QKV; ar.ldo = A; ar.pos0 = e.pos0; ar.part_row = (long long)nkv * ap.n_splits * G * (hd + 2);
+                if (e.rows) { ar.row_pos = e.d_pos; ar.row_kv = e.d_kv; ar.k_off = k_off; ar.v_off = v_off; }
+                CU(launch_on(e.st, e.pdl, hd == 128 ? (G <= 4 ? attn_rows_kernel<128, 4> : attn_rows_kernel<128, 8>) : (G <= 4 ? attn_rows_kernel<64, 4> : attn_rows_kernel<64, 8>),
+                             dim3(nkv, ap.n_splits, T), dim3(kAttnThreads), attn_smem_bytes(hd, G <= 4 ? 4 : 8, ap.n_splits, G), ap, ar));
+            } else {
+                RowsAttn ap{};
+                ap.qkv = Q; ap.ld = QKV; ap.k_cache = kc; ap.v_cache = vc; ap.out = AT; ap.ldo = A; ap.pos0 = e.pos0; ap.T = T;
+                ap.n_heads = nh; ap.n_kv = nkv; ap.max_seq = d.max_seq_len; ap.scale = scale;
+                CU(launch_on(e.st, e.pdl, hd == 128 ? rows_attn_kernel<128> : rows_attn_kernel<64>, dim3((unsigned)(((long long)T * G + 63) / 64), nkv), dim3(128),
+                             hd == 128 ? kRowsAttnSmem<128> : kRowsAttnSmem<64>, ap));
+            }
+            c->launches += 2;
+        }
+        RowsParams o{}, g{}, w{};
+        o.T = g.T = w.T = T; o.eps = g.eps = w.eps = d.norm_eps; o.K = A; g.K = H; w.K = I; o.n_seg = w.n_seg = 1; g.n_seg = 2;
+        o.x = AT; o.ldx = A; w.x = HB; w.ldx = I;
+        if (few) {
+            seg(o.seg[0], L.wo, X, H, nullptr);
+            o.epi = EPI_RESIDUAL; o.residual = X;      // (every element read and written by one thread)
+            CU(go_few(o));
+            seg(g.seg[0], L.gate, HB, I, nullptr); seg(g.seg[1], L.up, HB, I, nullptr);
+            g.x = X; g.ldx = H; g.norm_w = L.ffn_norm.f32(); g.epi = EPI_SWIGLU;
+            CU(go_few(g));
+            seg(w.seg[0], L.down, X, H, nullptr);
+            w.epi = EPI_RESIDUAL; w.residual = X;
+            CU(go_few(w));
+        } else {
+            seg(o.seg[0], L.wo, PT, H, nullptr);
+            CU(go_tile(o, H, sum));
+            CU(launch_on(e.st, e.pdl, rows_norm_kernel, dim3(T), dim3(256), 0, X, sum, L.ffn_norm.f32(), d.norm_eps, XN, H));
+            seg(g.seg[0], L.gate, PT, 2 * I, nullptr); seg(g.seg[1], L.up, PT + I, 2 * I, nullptr);
+            g.x = XN; g.ldx = H;
+            CU(go_tile(g, 2 * I, sum));
+            CU(launch_on(e.st, e.pdl, rows_swiglu_kernel, dim3((I + 255) / 256, T), dim3(256), 0, sum, HB, I));
+            seg(w.seg[0], L.down, PT, H, nullptr);
+            CU(go_tile(w, H, sum));
+            c->launches += 2;
+        }
+    }
+    if (!few) {
+        CU(launch_on(e.st, e.pdl, rows_norm_kernel, dim3(T), dim3(256), 0, X, sum, (const float*)nullptr, d.norm_eps, (float*)nullptr, H));
+        c->launches++;
+    }
+    return B200_OK;
+}
+
 // seqs == nullptr: the n tokens are consecutive positions of slot `seq` (prefill).  seqs != nullptr: batched decode, token i
 // is the next token of slot seqs[i] (distinct slots); the logits of all n rows are left in c->pf_logits ([n][vocab]).
-static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, bool want_logits, const int* seqs = nullptr) {
+// exact: rows in f32 (exact_rows_ok), kNoRoom where there is no room for their buffers.
+static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, bool want_logits, const int* seqs = nullptr, bool exact = false) {
     const b200_model_desc& d = c->d;
     Slot& sl = c->slots[seq];
     const int H = d.hidden, hd = d.head_dim, nh = d.n_heads, nkv = d.n_kv_heads, A = nh * hd, I = (int)d.ffn;
     const int QKV = (nh + 2 * nkv) * hd;
     const int cap = std::min(prefill_chunk(), d.max_seq_len);
     const PromptRows place = prompt_rows(cap, kFewTokens, H, QKV, A, I);
-    if (!c->pf_buf) {
-        CU_ALLOC(late_malloc(c, (void**)&c->pf_buf, place.floats * sizeof(float)));
-        CU_ALLOC(late_malloc(c, (void**)&c->pf_tok, cap * sizeof(int)));
-        CU_ALLOC(late_malloc(c, (void**)&c->pf_rows, (size_t)cap * 24));
-    }
-    { int rc_t = umma_tmaps_build(c); if (rc_t) return rc_t; }
-    if (!c->pf_split) {   // split-K scratch for passes of <= 64 rows: 8 partial tiles of the widest projection
+    if (!c->pf_buf && !exact) CU_ALLOC(late_malloc(c, (void**)&c->pf_buf, place.floats * sizeof(float)));
+    if (!c->pf_tok) CU_ALLOC(late_malloc(c, (void**)&c->pf_tok, cap * sizeof(int)));
+    if (!c->pf_rows) CU_ALLOC(late_malloc(c, (void**)&c->pf_rows, (size_t)cap * 24));
+    if (!exact) { int rc_t = umma_tmaps_build(c); if (rc_t) return rc_t; }
+    if (!c->pf_split && !exact) {   // split-K scratch for passes of <= 64 rows: 8 partial tiles of the widest projection
         c->pf_split_floats = (size_t)8 * 64 * std::max(std::max(I, QKV), H);
         CU_ALLOC(late_malloc(c, (void**)&c->pf_split, c->pf_split_floats * sizeof(float)));
         CU_ALLOC(late_malloc(c, (void**)&c->pf_tile_cnt, 8192 * sizeof(int)));
@@ -1961,7 +2188,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     }
     // products of few rows (gemm_few.cuh): images of the activations and pieces of cut tiles; a device without room for them keeps the other products
     const int few_max = kFewTokens, last_chunk = n % cap ? n % cap : cap;
-    if (c->few_able && c->kv_format == 0 && !c->few_part && last_chunk <= few_max && c->few_retry.due()) {
+    if (!exact && c->few_able && c->kv_format == 0 && !c->few_part && last_chunk <= few_max && c->few_retry.due()) {
         const size_t bytes[4] = {few_image_bytes(few_max, 64, H), few_image_bytes(few_max, 64, A), few_image_bytes(few_max, 64, I), (size_t)2 * c->n_sm * 64 * 128 * sizeof(float)};
         void* got[4] = {};
         bool ok = true;
@@ -1980,7 +2207,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     // batched decode: per-row (position, KV base of the slot, SeqState of the slot)
     const bool rows = seqs != nullptr;
     // tensor-core attention of a prompt chunk (attn_umma.cuh): fp16 K / V^T copies of ONE layer (rewritten per layer and chunk)
-    bool attn_tc = !rows && c->pf_attn_tc && gemm_encode_fn() && attn_umma_ok(hd, nh, nkv);
+    bool attn_tc = !rows && !exact && c->pf_attn_tc && gemm_encode_fn() && attn_umma_ok(hd, nh, nkv);
     if (attn_tc && !c->pf_k16) {
         const int P = (d.max_seq_len + 127) & ~127;
         CU_ALLOC(late_malloc(c, (void**)&c->pf_k16, (size_t)2 * nkv * P * hd * sizeof(__half)));    // hi rows, then lo rows
@@ -1992,7 +2219,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         }
     }
     const bool q8 = c->kv_format == 1;
-    if (q8 && (rows || !attn_tc)) return fail(B200_ERR_UNSUPPORTED, "int8 KV cache: the GEMM pass needs the tensor-core prompt attention");
+    if (q8 && !exact && (rows || !attn_tc)) return fail(B200_ERR_UNSUPPORTED, "int8 KV cache: the GEMM pass needs the tensor-core prompt attention");
     // tables of a batched decode step, one copy: per row token, position, KV base of the slot, SeqState of the slot
     int* d_tok = rows ? reinterpret_cast<int*>(c->pf_rows) : c->pf_tok;
     int* d_pos = reinterpret_cast<int*>(c->pf_rows + (size_t)n * 4);
@@ -2025,6 +2252,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             drop_batch_graphs(c);      // (the captured head GEMMs write the old buffer)
         }
     }
+    if (exact && !exact_rows_room(c, std::min(n, cap))) return kNoRoom;
     // CUDA graph of the step (rows mode): replay if this row count has one, capture on its second step (the first runs eagerly:
     // function attributes and lazy allocations happen there), and run the capture's graph to do the step itself
     struct CaptureGuard {
@@ -2055,7 +2283,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             bg.warm = true;
         }
     }
-    float* X = c->pf_buf + place.x;                     // [T][H] residual stream (f32)
+    float* X = exact ? c->er_buf : c->pf_buf + place.x; // [T][H] residual stream (f32)
     float* Q = c->pf_buf + place.qkv;                   // [T][QKV] f32
     float* G = c->pf_buf + place.gate;                  // [T][I] gate; few rows also [T][H], what X still lacks
     float* U = c->pf_buf + place.up;                    // [T][I] up
@@ -2158,6 +2386,12 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         last_T = T;
         if (!rows) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
         CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T, T <= 256 ? 4 : 1), dim3(T <= 256 ? 128 : 256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)d_tok, d.vocab, X));
+        if (exact) {
+            ExactPass ep{T, pos0, rows, d_pos, d_kv, st, pdl};
+            if (const int rc_x = exact_layers(c, sl, ep)) return rc_x;
+            c->launches++;
+            continue;
+        }
         // Few rows: products straight from the blocks (gemm_few.cuh), their pieces added by the kernel behind them
         few = few_takes(T);
         FewOut sum{};                                   // product that X still lacks (of the layer before)
@@ -2338,7 +2572,12 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     if (rows) {   // every row's slot advances by one; final RMSNorm + vocab head of ALL rows through the GEMM
         CU(launch_on(st, pdl, prefill_advance_rows_kernel, dim3((n + 127) / 128), dim3(128), 0, (SeqState* const*)d_st, n));
         const DevTensor& head = c->output.present() ? c->output : c->token_embd;
-        if (!head_done) {
+        if (exact) {
+            RowsParams p{};
+            p.seg[0].w = (const uint8_t*)head.d; p.seg[0].row_bytes = head.row_bytes; p.seg[0].type = head.type; p.seg[0].n_rows = d.vocab; p.seg[0].out = c->pf_logits; p.seg[0].ldo = d.vocab;
+            p.n_seg = 1; p.K = H; p.T = n; p.x = X; p.ldx = H; p.norm_w = c->output_norm.f32(); p.eps = d.norm_eps; p.epi = EPI_STORE;
+            CU(rows_few_launch(p, c->n_sm, pdl, st));
+        } else if (!head_done) {
             CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(n), dim3(256), 0, (const float*)X, c->output_norm.f32(), d.norm_eps, XNh, H));
             UmmaParams hp{};
             hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = d.vocab; hp.K = H;
@@ -2359,7 +2598,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 if (c->batch_pdl) c->batch_pdl = false;
                 else c->batch_graph = false;
                 c->launches = launches0;
-                return prefill_gemm(c, seq, tokens, n, want_logits, seqs);
+                return prefill_gemm(c, seq, tokens, n, want_logits, seqs, exact);
             }
             b200_ctx::BatchGraph& bg = c->batch_graphs[n];
             bg.exec = ex;
@@ -2376,7 +2615,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         p.n_seg = 1; p.K = H; p.x = c->xa; p.norm_w = c->output_norm.f32(); p.eps = d.norm_eps; p.epi = EPI_STORE;
         CU(launch_gemv(c, p));
     }
-    c->prefill_gemm_tokens += (uint64_t)n;
+    if (!exact) c->prefill_gemm_tokens += (uint64_t)n;
     return B200_OK;
 }
 
@@ -2615,23 +2854,26 @@ extern "C" int b200_prefill(b200_ctx* c, int seq, const uint32_t* tokens, int n,
     if ((rc = check_slot(c, seq, "b200_prefill"))) return rc;
     if (!tokens || n <= 0) return fail(B200_ERR_INVALID_ARGUMENT, "b200_prefill: no tokens");
     if (!c->slots[seq].pending.empty() && (rc = flush_pending(c, seq))) return rc;
-    if (n >= c->prefill_gemm_min && prefill_gemm_ok(c, true)) {
+    const bool as_gemm = n >= c->prefill_gemm_min && prefill_gemm_ok(c, true);
+    const bool queued = !as_gemm && c->prefill_queue && !c->queue_bypass && prefill_gemm_ok(c);      // (b200_prefill_token would queue the tokens)
+    if (as_gemm || (!queued && exact_rows_ok(c, n, true))) {
         for (int i = 0; i < n; i++)
             if (tokens[i] >= (uint32_t)c->d.vocab) return fail(B200_ERR_INVALID_ARGUMENT, "b200_prefill: token id exceeds vocab size");
         Slot& sl = c->slots[seq];
         if (sl.host_pos + (uint64_t)n > (uint64_t)c->d.max_seq_len) return fail(B200_ERR_INVALID_ARGUMENT, "b200_prefill: context length exceeded");
         CU(cudaSetDevice(c->par.device));
-        if ((rc = prefill_gemm(c, seq, tokens, n, logits_out != nullptr))) return rc;
-        CU(cudaMemcpyAsync(c->h_err, c->mma_err, (8 + (logits_out ? (size_t)c->vocab_l : 0)) * 4, cudaMemcpyDeviceToHost, c->stream));      // watchdog words (and logits)
-        CU(cudaStreamSynchronize(c->stream));
-        if ((rc = watchdog_check(c, "b200_prefill"))) return rc;
-        if (logits_out) memcpy(logits_out, c->h_logits, (size_t)c->vocab_l * 4);
-        sl.host_pos += (uint64_t)n;
-        return B200_OK;
+        if ((rc = prefill_gemm(c, seq, tokens, n, logits_out != nullptr, nullptr, !as_gemm)) != kNoRoom) {
+            if (rc) return rc;
+            CU(cudaMemcpyAsync(c->h_err, c->mma_err, (8 + (logits_out ? (size_t)c->vocab_l : 0)) * 4, cudaMemcpyDeviceToHost, c->stream));      // watchdog words (and logits)
+            CU(cudaStreamSynchronize(c->stream));
+            if ((rc = watchdog_check(c, "b200_prefill"))) return rc;
+            if (logits_out) memcpy(logits_out, c->h_logits, (size_t)c->vocab_l * 4);
+            sl.host_pos += (uint64_t)n;
+            return B200_OK;
+        }
     }
     // token by token: the launches follow one another without a wait between, and the watchdog words are looked at some tokens later (unless b200_prefill_token
     // would queue the tokens)
-    const bool queued = c->prefill_queue && !c->queue_bypass && prefill_gemm_ok(c);
     CU(cudaSetDevice(c->par.device));
     int done = 0;
     rc = run_ahead(
@@ -2666,6 +2908,15 @@ extern "C" int b200_prefill(b200_ctx* c, int seq, const uint32_t* tokens, int n,
     return B200_OK;
 }
 
+static bool batch_gemm_eligible(b200_ctx* c, int n) {
+    if (n < c->batch_gemm_min || !prefill_gemm_ok(c)) return false;
+    const DevTensor& head = c->output.present() ? c->output : c->token_embd;
+    UmmaParams hp{};
+    hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = c->d.vocab; hp.K = c->d.hidden; hp.T = 1;
+    hp.x = reinterpret_cast<const __half*>(c->xa); hp.ldx = c->d.hidden;
+    return umma_eligible(hp) && n <= std::min(prefill_chunk(), c->d.max_seq_len);
+}
+
 extern "C" int b200_decode_batch(b200_ctx* c, const int* seqs, const uint32_t* tokens, int n, float* logits_out) {
     if (!c || !seqs || !tokens || !logits_out || n <= 0) return fail(B200_ERR_INVALID_ARGUMENT, "b200_decode_batch: bad argument");
     if (c->lp) {
@@ -2683,18 +2934,15 @@ extern "C" int b200_decode_batch(b200_ctx* c, const int* seqs, const uint32_t* t
         if (seqs[i] >= 0 && seqs[i] < (int)c->slots.size() && (rc = flush_pending(c, seqs[i]))) return rc;
     // n >= batch_gemm_min rows of an eligible dense model: ONE pass of the tcgen05 dequant-GEMMs for all the sequences (the
     // weights are read once per step instead of once per sequence); fp16 tensor-core operands, see gemm_umma.cuh
-    if (n >= c->batch_gemm_min && prefill_gemm_ok(c)) {
-        const DevTensor& head = c->output.present() ? c->output : c->token_embd;
-        UmmaParams hp{};
-        hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = c->d.vocab; hp.K = c->d.hidden; hp.T = 1;
-        hp.x = reinterpret_cast<const __half*>(c->xa); hp.ldx = c->d.hidden;
-        if (umma_eligible(hp) && n <= std::min(prefill_chunk(), c->d.max_seq_len)) {
-            for (int i = 0; i < n; i++) {
-                if ((rc = check_slot(c, seqs[i], "b200_decode_batch"))) return rc;
-                if ((rc = check_token(c, seqs[i], tokens[i], "b200_decode_batch"))) return rc;
-            }
-            CU(cudaSetDevice(c->par.device));
-            if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs))) return rc;
+    const bool as_gemm = batch_gemm_eligible(c, n);
+    if (as_gemm || (n <= c->d.max_seq_len && exact_rows_ok(c, n, false))) {
+        for (int i = 0; i < n; i++) {
+            if ((rc = check_slot(c, seqs[i], "b200_decode_batch"))) return rc;
+            if ((rc = check_token(c, seqs[i], tokens[i], "b200_decode_batch"))) return rc;
+        }
+        CU(cudaSetDevice(c->par.device));
+        if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs, !as_gemm)) != kNoRoom) {
+            if (rc) return rc;
             // n x vocab logits (16.4 MB at batch 32 on Llama-3) to the caller's pageable buffer: DMA into a pinned buffer, rows copied
             // out by a few host threads (a pageable cudaMemcpy stages the same bytes through the driver on one thread)
             const size_t bytes = (size_t)n * c->d.vocab * sizeof(float);
@@ -3857,15 +4105,6 @@ extern "C" int b200_group_load_gguf(b200_group* g, b200_gguf* file, b200_load_st
 }
 
 // ------------------------------------------------------------------ batched decode with the pick on the device + continuous batching
-static bool batch_gemm_eligible(b200_ctx* c, int n) {
-    if (n < c->batch_gemm_min || !prefill_gemm_ok(c)) return false;
-    const DevTensor& head = c->output.present() ? c->output : c->token_embd;
-    UmmaParams hp{};
-    hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = c->d.vocab; hp.K = c->d.hidden; hp.T = 1;
-    hp.x = reinterpret_cast<const __half*>(c->xa); hp.ldx = c->d.hidden;
-    return umma_eligible(hp) && n <= std::min(prefill_chunk(), c->d.max_seq_len);
-}
-
 // b200_decode_batch with the greedy pick (last maximum wins, src/main.rs:1816-1821) on the device: n token ids come back instead
 // of n x vocab logits (16 MB per step at batch 32 on Llama-3).  Same two paths as b200_decode_batch.
 extern "C" int b200_decode_batch_greedy(b200_ctx* c, const int* seqs, const uint32_t* tokens, int n, uint32_t* next_out) {
@@ -3885,7 +4124,8 @@ extern "C" int b200_decode_batch_greedy(b200_ctx* c, const int* seqs, const uint
         if ((rc = check_token(c, seqs[i], tokens[i], "b200_decode_batch_greedy"))) return rc;
         if ((rc = flush_pending(c, seqs[i]))) return rc;
     }
-    if (batch_gemm_eligible(c, n)) {
+    const bool as_gemm = batch_gemm_eligible(c, n);
+    if (as_gemm || (n <= c->d.max_seq_len && exact_rows_ok(c, n, false))) {
         CU(cudaSetDevice(c->par.device));
         if (c->pf_argmax_rows < n) {
             cudaFree(c->pf_argmax);
@@ -3894,15 +4134,17 @@ extern "C" int b200_decode_batch_greedy(b200_ctx* c, const int* seqs, const uint
             CU_ALLOC(late_malloc(c, (void**)&c->pf_argmax, (size_t)n * sizeof(int)));
             c->pf_argmax_rows = n;
         }
-        if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs))) return rc;
-        argmax_rows_kernel<<<n, 1024, 0, c->stream>>>(c->pf_logits, c->d.vocab, c->pf_argmax);
-        c->launches++;
-        CU(cudaMemcpyAsync(next_out, c->pf_argmax, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        WATCHDOG_FETCH(c);
-        CU(cudaStreamSynchronize(c->stream));
-        if ((rc = watchdog_check(c, "b200_decode_batch_greedy"))) return rc;
-        for (int i = 0; i < n; i++) c->slots[seqs[i]].host_pos++;
-        return B200_OK;
+        if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs, !as_gemm)) != kNoRoom) {
+            if (rc) return rc;
+            argmax_rows_kernel<<<n, 1024, 0, c->stream>>>(c->pf_logits, c->d.vocab, c->pf_argmax);
+            c->launches++;
+            CU(cudaMemcpyAsync(next_out, c->pf_argmax, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            WATCHDOG_FETCH(c);
+            CU(cudaStreamSynchronize(c->stream));
+            if ((rc = watchdog_check(c, "b200_decode_batch_greedy"))) return rc;
+            for (int i = 0; i < n; i++) c->slots[seqs[i]].host_pos++;
+            return B200_OK;
+        }
     }
     for (int i = 0; i < n; i++)
         if ((rc = b200_decode_greedy(c, seqs[i], tokens[i], 1, next_out + i, nullptr))) return rc;

@@ -108,6 +108,8 @@ __global__ void rope_kv_q8_kernel(const RopeKvQ8Params p) {
 // floats apart (p.q = the first row; p.k / p.v / p.pos unused).  grid (ceil(units / 4), T), 128 threads.
 template <int VEC>
 __global__ void prefill_rope_kv_q8_kernel(const RopeKvQ8Params p, int ld, int pos0) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int lane = threadIdx.x & 31, unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, t = blockIdx.y;
     if (unit >= p.n_heads + 2 * p.n_kv) return;
     const int hd = 32 * VEC;
@@ -158,10 +160,21 @@ struct AttnQ8Params {
     const float* v_scale;
     float* part;               // [n_kv][n_splits][G][hd + 2]: unnormalised accumulator, running max, running sum
     float* out;                // [n_heads][hd]
-    const int* pos;            // device scalar: kv_len = *pos + 1
+    const int* pos;            // device scalar: kv_len = *pos + 1; nullptr: blockIdx.z is the row of a prompt, at position pos0 + z
     int n_kv, G, max_seq, n_splits;
     float scale;
+    int pos0, ldq, ldo;        // (rows)
+    long long part_row;
 };
+// the row of a block
+__device__ __forceinline__ int attn_q8_row(AttnQ8Params& p) {
+    if (p.pos) return *p.pos + 1;
+    const int z = blockIdx.z;
+    p.q += (size_t)z * p.ldq;
+    p.out += (size_t)z * p.ldo;
+    p.part += (size_t)z * p.part_row;
+    return p.pos0 + z + 1;
+}
 
 // 16 int8 values (one 16-byte load) -> 16 floats without I2F (quarter rate): x ^ 0x80 is the unsigned byte x + 128, PRMT drops it
 // into the mantissa of 2^23 (0x4B000000 | u = 2^23 + u exactly), one FADD removes 2^23 + 128.
@@ -187,15 +200,16 @@ constexpr int kAttnQ8Unroll = 4;
 // (both read the same rows; the second read hits L1 / L2).  The row scale is applied once per score (K) and folded into the
 // softmax weight (V).  grid (n_splits, n_kv), 128 threads.
 template <int HD, int HG>
-__global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(const AttnQ8Params p) {
+__global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(const AttnQ8Params p_in) {
     constexpr int LPR = HD / 16, RPW = 32 / LPR, U = kAttnQ8Unroll;
     __shared__ float sm[kAttnQ8Warps][HG][HD + 2];
     pdl_launch_dependents();
     pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, split = blockIdx.x, kh = blockIdx.y, G = p.G;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, split = blockIdx.x, kh = blockIdx.y, G = p_in.G;
     const int NHG = (G + HG - 1) / HG, WPG = kAttnQ8Warps / NHG;   // head groups (1 or 2), warps per head group
     const int hgp = warp % NHG, wsub = warp / NHG, sub = lane % LPR, rg = lane / LPR;
-    const int kv_len = *p.pos + 1;
+    AttnQ8Params p = p_in;
+    const int kv_len = attn_q8_row(p);
     const int chunk = (kv_len + p.n_splits - 1) / p.n_splits;
     const int p_begin = split * chunk, p_end = min(kv_len, p_begin + chunk);
     const int stride = WPG * RPW;
@@ -308,12 +322,14 @@ __global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(con
 // (groups in order at the end).  9 positions in 128 splits, 14 heads of 64: 21 -> 5 us against one thread per channel that walked all splits after two
 // serial passes of one thread over the maxima and sums.
 constexpr int kAttnQ8MaxSplits = 128, kAttnQ8MergeThreads = 256;
-__global__ void __launch_bounds__(kAttnQ8MergeThreads) attn_q8_merge_kernel(const AttnQ8Params p, int hd) {
+__global__ void __launch_bounds__(kAttnQ8MergeThreads) attn_q8_merge_kernel(const AttnQ8Params p_in, int hd) {
     __shared__ float sc[kAttnQ8MaxSplits], sums[kAttnQ8MergeThreads], s_l;
     pdl_launch_dependents();
     pdl_wait();
+    AttnQ8Params p = p_in;
+    const int kv_len = attn_q8_row(p);
     const int head = blockIdx.x, kh = head / p.G, g = head - kh * p.G, lane = threadIdx.x & 31;
-    const int kv_len = *p.pos + 1, chunk = (kv_len + p.n_splits - 1) / p.n_splits, live = (kv_len + chunk - 1) / chunk;      // (<= n_splits)
+    const int chunk = (kv_len + p.n_splits - 1) / p.n_splits, live = (kv_len + chunk - 1) / chunk;      // (<= n_splits)
     const float* base = p.part + (((size_t)kh * p.n_splits) * p.G + g) * (hd + 2);
     const size_t stride = (size_t)p.G * (hd + 2);
     if (threadIdx.x < 32) {
