@@ -488,6 +488,142 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (warp == TC_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN) : "memory");
 }
 
+// Few token rows whose sums may not be cut along K: the token rows are the M of tcgen05.mma (MR = 64 or 128, those above R are whatever the shared memory holds;
+// their sums stay in tensor memory unread) and NT = 16 or 32 weight rows its N, so that 2048 outputs are 128 or 64 CTAs instead of the 16 that tiles of 128 weight rows
+// give, each with a quarter of the operand bytes.  Every sum adds its products in the order of K, by the same MMAs of 16: the bits of the other kernels.
+// Bound by the operands on their way into shared memory, 128 (R + NT) bytes per 64 elements of K at 64 per clock; the whole ring is asked for at once.
+// Warps 0 - 3: epilogue (tensor-memory lane = token row), 4 weight rows, 5 token rows, 6 MMAs.  One CTA per tile of NT outputs.
+enum { TR_LOAD_W = 4, TR_LOAD_X = 5, TR_MMA = 6, TR_THREADS = 224, TR_KH = 4, TR_STAGES = 8 };
+// stages of 4 slabs: R token rows (a multiple of 8), then NT weight rows; behind the ring what an MMA over MR rows reads beyond the last token rows
+__host__ __device__ inline uint32_t tr_stage_bytes(int rows8, int nt) { return (uint32_t)TR_KH * (rows8 + nt) * 128; }
+__host__ __device__ inline int tr_stages(int rows8, int nt, int K) {
+    const int fit = (int)(196608 / tr_stage_bytes(rows8, nt)), need = (K + TR_KH * TC_K - 1) / (TR_KH * TC_K), most = fit < TR_STAGES ? fit : (int)TR_STAGES;
+    return need < most ? need : most;
+}
+inline size_t tr_smem_bytes(int rows8, int nt, int K, int mr) { return (size_t)tr_stages(rows8, nt, K) * tr_stage_bytes(rows8, nt) + (size_t)mr * 128 + 1024; }
+
+template <int MR, int NT, int EPI>
+__global__ void __launch_bounds__(TR_THREADS, 1) lp_gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const TcArgs a) {
+    static_assert(!epi_is_glu(EPI), "gated units pair two weight rows");
+    next_grid();
+    extern __shared__ __align__(1024) uint8_t tc_smem[];
+    __shared__ __align__(8) unsigned long long s_bar[2 * TR_STAGES + 1];
+    __shared__ uint32_t s_tmem;
+    uint8_t* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rows8 = (a.R + 7) & ~7, NS = tr_stages(rows8, NT, a.K), all = (a.K + TC_K - 1) / TC_K, steps = (all + TR_KH - 1) / TR_KH;
+    const uint32_t stage_bytes = tr_stage_bytes(rows8, NT), x_bytes = (uint32_t)TR_KH * rows8 * 128, ring = smem_u32(base);
+    const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * TR_STAGES, done = bar + 16u * TR_STAGES;
+    constexpr uint32_t COLS = 32;
+    if (tid == 0) {
+        for (int i = 0; i < TR_STAGES; i++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(full + 8u * i) : "memory");      // both loaders
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty + 8u * i) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == TR_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (TC_W_WAITS || warp != TR_LOAD_W) wait_grid();       // (other weights do not depend on the kernel before)
+    const uint32_t tmem = s_tmem;
+    const int n0 = blockIdx.x * NT;
+    bool alive = true;
+    if (warp == TR_LOAD_W || warp == TR_LOAD_X) {
+        const bool is_w = warp == TR_LOAD_W;
+        const int rows = is_w ? NT : rows8;
+        uint32_t s = 0, ph = 1;
+        for (int k = 0; k < steps; k++) {
+            tc_wait(empty + 8u * s, ph, alive, a.err, 1);
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            if (tc_elect()) {
+                const uint32_t dst = ring + s * stage_bytes + (is_w ? x_bytes : 0u);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8u * s), "r"((uint32_t)TR_KH * rows * 128u) : "memory");
+                if (a.slabs) {
+                    tc_tma(dst, is_w ? &wmap : &xmap, 0, is_w ? n0 : 0, k * TR_KH, 0, full + 8u * s);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < TR_KH; h++) tc_tma(dst + (uint32_t)h * rows * 128u, is_w ? &wmap : &xmap, (k * TR_KH + h) * TC_K, is_w ? n0 : 0, 0, 0, full + 8u * s);
+                }
+            }
+            __syncwarp();
+            if (++s == (uint32_t)NS) { s = 0; ph ^= 1u; }
+        }
+        if (!alive)      // what has been asked for lands first (bounded)
+            for (uint32_t i = 0; i < (uint32_t)NS; i++) {
+                bool wait = true;
+                tc_wait(full + 8u * i, i < s ? ph ^ 1u : ph, wait, nullptr, 0);
+            }
+    } else if (warp == TR_MMA) {
+        const uint32_t idesc = tc_idesc(MR, NT);
+        uint32_t s = 0, ph = 0;
+        for (int k = 0; k < steps; k++) {
+            tc_wait(full + 8u * s, ph, alive, a.err, 3);
+            alive = __all_sync(0xffffffffu, alive);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (tc_elect()) {
+                if (alive) {
+                    const uint64_t da = tc_desc(ring + s * stage_bytes), db = tc_desc(ring + s * stage_bytes + x_bytes);
+#pragma unroll
+                    for (int h = 0; h < TR_KH; h++)
+                        if (k * TR_KH + h < all) {
+#pragma unroll
+                            for (int kk = 0; kk < TC_K / 16; kk++) {
+                                const uint32_t accum = (k > 0 || h > 0 || kk > 0) ? 1u : 0u;
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                                    "l"(da + (uint64_t)(h * rows8 * 8 + 2 * kk)), "l"(db + (uint64_t)(h * NT * 8 + 2 * kk)), "r"(idesc), "r"(accum)
+                                    : "memory");
+                            }
+                        }
+                }
+                tc_commit(empty + 8u * s);
+                if (k == steps - 1) tc_commit(done);
+            }
+            __syncwarp();
+            if (++s == (uint32_t)NS) { s = 0; ph ^= 1u; }
+        }
+    } else {
+        // M = 128: row = lane of tensor memory; M = 64: rows 16 w .. 16 w + 15 in the first half of warp w's lanes
+        const int t = MR == 128 ? tid : 16 * warp + lane;
+        const bool live = t < a.R && (MR == 128 || lane < 16);
+        tc_wait(done, 0, alive, a.err, 4);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t v[32];
+        tc_ld32(v, tmem + ((uint32_t)(warp * 32) << 16));
+        if (live) {
+            const size_t at = (size_t)t * a.ldy + n0;
+            if (!epi_is_act(EPI) && n0 + NT <= a.N && a.ldy % 4 == 0 && ((uintptr_t)a.Y & 15) == 0 && !a.bias) {
+                float4* y = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.Y) + at);
+#pragma unroll
+                for (int c = 0; c < NT / 4; c++) {
+                    const float4 old = EPI == EPI_ADD ? y[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    float f[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) f[u] = a.alpha * __uint_as_float(v[4 * c + u]) + 0.0f;
+                    y[c] = EPI == EPI_ADD ? make_float4(old.x + f[0], old.y + f[1], old.z + f[2], old.w + f[3]) : make_float4(f[0], f[1], f[2], f[3]);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < NT; c++)
+                    if (n0 + c < a.N) epi_store<tc_t, EPI>(a.Y, at + c, a.alpha * __uint_as_float(v[c]) + (a.bias ? a.bias[n0 + c] : 0.0f), a.act);
+            }
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == TR_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+}
+
 // ------------------------------------------------------------------------------------------------ host
 using TcEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -522,18 +658,26 @@ bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts,
 // their CTAs already took two waves (12.4 us where 64 CTAs in clusters of 4 took 8.3: 32 x 2048 x 2048).
 // split: K may be cut over a cluster.  Without, every sum adds its products in the order of K, so that a row's result is the same bits whatever the number of
 // rows of the step.
+// rows: token rows as M (lp_gemm_tc_rows_kernel), tn weight rows per CTA: for sums that may not be cut (a cut over a cluster is as fast), up to 128 rows
 struct TcPlan {
     bool persistent;
     int tn, splits;
+    bool rows;
 };
-TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, bool split) {
+TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, bool split, bool tc_rows_able = false) {
     const int n_sm = 148, steps = (K + TC_K - 1) / TC_K, per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per;
     auto tiles = [&](int tn) { return (long long)n_mt * (seg ? xrows / tn + (groups + 1) / 2 : groups * ((R + tn - 1) / tn)); };
-    TcPlan best{true, 256, 1};
+    TcPlan best{true, 256, 1, false};
     long long least = -1;
     auto offer = [&](bool persistent, int tn, int s, long long cost) {
-        if (least < 0 || cost < least) { least = cost; best = TcPlan{persistent, tn, s}; }
+        if (least < 0 || cost < least) { least = cost; best = TcPlan{persistent, tn, s, false}; }
     };
+    if (tc_rows_able && !split && !seg && !glu && groups == 1 && R <= 128)
+        for (int nt : {16, 32}) {
+            const long long waves = ((N + nt - 1) / nt + n_sm - 1) / n_sm, step = std::max(2 * (((R + 7) & ~7) + nt), R <= 64 ? 64 + nt : 128 + nt);
+            const long long cost = waves * (steps * step + 4500) - 4500 + 18 * 64;
+            if (least < 0 || cost < least) { least = cost; best = TcPlan{false, nt, 1, true}; }
+        }
     for (int tn : {256, 128}) {
         if (tn == 256 && R <= 128) continue;
         const long long waves = (tiles(tn) + n_sm - 1) / n_sm;

@@ -1528,6 +1528,7 @@ struct LpModel {
     // close then takes the other one -- a different row, not a rounding of it.  32 sequences through two layers of width 2048, a step's products of 32 rows 10.2 -> 14.9 us,
     // prompts of 48 tokens 26 -> 44 us of attention per layer.
     bool any_order = true;
+    bool tc_rows = true;                    // B200_LP_TC_ROWS=0: no tiles of token rows as M
     bool tc_maps = true;                    // B200_LP_TC_MAPS=0: as if the driver refused the tensor maps of the products
     size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
     float* chunk_scan = nullptr;        // lp_chunk_scan.cuh: one layer's scratch, kept from call to call
@@ -1742,6 +1743,32 @@ bool tc_launch(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const T
         default: return tc_launch_as<TN, PERSISTENT, EPI_RELU2>(m, xm, wm, a, grid);
     }
 }
+template <int MR, int NT, int EPI>
+bool tc_rows_launch_as(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a) {
+    auto kern = lp_gemm_tc_rows_kernel<MR, NT, EPI>;
+    static bool once[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !once[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (dev >= 0 && dev < 64) once[dev] = true;
+    }
+    launch(m, kern, dim3((a.N + NT - 1) / NT), dim3(TR_THREADS), tr_smem_bytes((a.R + 7) & ~7, NT, a.K, MR), xm, wm, a);
+    return true;
+}
+template <int MR, int NT>
+bool tc_rows_launch(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, int epi) {
+    switch (epi) {
+        case EPI_STORE: return tc_rows_launch_as<MR, NT, EPI_STORE>(m, xm, wm, a);
+        case EPI_ADD: return tc_rows_launch_as<MR, NT, EPI_ADD>(m, xm, wm, a);
+        case EPI_GELU: return tc_rows_launch_as<MR, NT, EPI_GELU>(m, xm, wm, a);
+        case EPI_XIELU: return tc_rows_launch_as<MR, NT, EPI_XIELU>(m, xm, wm, a);
+        default: return tc_rows_launch_as<MR, NT, EPI_RELU2>(m, xm, wm, a);
+    }
+}
 // The tensor-core GEMM takes bf16 operands whose rows are 16-byte aligned (K and the row pitches multiples of 8).
 bool tc_takes(const LpModel* m, const void* X, int ldx, const void* W, int ldw, int K, int R, size_t wz, ZStride zs) {
     if (m->f32 || !m->use_tc || R < m->tc_min_rows) return false;
@@ -1756,7 +1783,8 @@ struct TcProduct {
 bool tc_prepare(const LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, int R, bool glu, bool seg, int xrows, int groups, size_t wz, ZStride zs, TcProduct& t) {
     if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs) || !m->tc_maps) return false;
     const bool x_z = !seg && groups > 1 && zs.x > 0;
-    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->any_order);
+    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->any_order, m->tc_rows);
+    if (t.pl.rows) return tc_map(&t.xm, X, K, R, ldx, 1, 1, 0, (R + 7) & ~7, TR_KH) && tc_map(&t.wm, W, K, N, ldw, 1, 1, 0, t.pl.tn, TR_KH);
     const int kh = t.pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     return tc_map(&t.xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, t.pl.tn, kh) &&
            tc_map(&t.wm, W, K, N, ldw, glu ? 2 : 1, groups, wz, glu ? TC_M / 2 : TC_M, kh);
@@ -1769,6 +1797,10 @@ bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, 
     const TcPlan& pl = t.pl;
     const CUtensorMap &xm = t.xm, &wm = t.wm;
     const TcArgs a{Y, ldy, R, N, K, alpha, m->tc_err, seg, groups, x_z ? 1 : 0, zs.y, bias, act, pl.splits, K % TC_K == 0 ? 1 : 0};
+    if (pl.rows) {
+        if (R <= 64) return pl.tn == 16 ? tc_rows_launch<64, 16>(m, xm, wm, a, epi) : tc_rows_launch<64, 32>(m, xm, wm, a, epi);
+        return pl.tn == 16 ? tc_rows_launch<128, 16>(m, xm, wm, a, epi) : tc_rows_launch<128, 32>(m, xm, wm, a, epi);
+    }
     const int per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per, n_nt = (R + pl.tn - 1) / pl.tn;
     if (pl.persistent) {
         const int most = seg ? n_mt * (xrows / pl.tn + groups) : n_mt * n_nt * groups;
@@ -2108,6 +2140,8 @@ int lp_create(const b200_program_desc* prog, const b200_layer_desc* layers, int 
         if (e && *e) m->use_attn_tile = atoi(e) != 0;
         e = getenv("B200_LP_TC_MAPS");
         if (e && *e) m->tc_maps = atoi(e) != 0;
+        e = getenv("B200_LP_TC_ROWS");
+        if (e && *e) m->tc_rows = atoi(e) != 0;
         e = getenv("B200_LP_KEYS16_MB");
         if (e && *e) m->keys16_most = (size_t)std::max(0, atoi(e)) << 20;
         e = getenv("B200_LP_PDL");
