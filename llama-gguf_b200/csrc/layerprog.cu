@@ -116,8 +116,9 @@ __global__ void lp_rmsnorm_kernel(float* __restrict__ x, const float* __restrict
     float* xr = x + (size_t)r * width;
     __shared__ float red[34];
     constexpr int NV = 32;
-    if (!center && width <= NV * 128 && blockDim.x == 128) {      // the row in registers: every load is in flight at once (2048 wide, 32 rows: 11 -> 5 us); same order of sums
-        float v[NV], wv[NV], ss = 0.0f;
+    // the row in registers: every load is in flight at once (2048 wide, 32 rows: 11 -> 5 us, the layer norm 17 -> 5); same order of sums
+    if (width <= NV * 128 && blockDim.x == 128) {
+        float v[NV], wv[NV], ss = 0.0f, mean = 0.0f;
 #pragma unroll
         for (int k = 0; k < NV; k++) {
             const int c = threadIdx.x + 128 * k;
@@ -134,9 +135,24 @@ __global__ void lp_rmsnorm_kernel(float* __restrict__ x, const float* __restrict
                 }
             }
         }
+        if (center) {
+            float t = 0.0f;
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                if (threadIdx.x + 128 * k < width) t += v[k];
+            t = wsum(t);
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                const float u = wsum(threadIdx.x < 4 ? red[threadIdx.x] : 0.0f);
+                if (threadIdx.x == 0) red[33] = u / (float)width;
+            }
+            __syncthreads();
+            mean = red[33];
+        }
 #pragma unroll
         for (int k = 0; k < NV; k++)
-            if (threadIdx.x + 128 * k < width) ss += v[k] * v[k];
+            if (threadIdx.x + 128 * k < width) ss += (v[k] - mean) * (v[k] - mean);
         ss = wsum(ss);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
         __syncthreads();
@@ -149,7 +165,7 @@ __global__ void lp_rmsnorm_kernel(float* __restrict__ x, const float* __restrict
 #pragma unroll
         for (int k = 0; k < NV; k++) {
             const int c = threadIdx.x + 128 * k;
-            if (c < width) out[(size_t)b * width + c] = from_f<OutT>(v[k] * inv * wv[k]);
+            if (c < width) out[(size_t)b * width + c] = from_f<OutT>((v[k] - mean) * inv * wv[k]);
         }
         return;
     }
