@@ -43,29 +43,71 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
     const int run = sm.row_run[r], pos = sm.row_pos[r], t = r - sm.run_start[run];
     float* tail = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off);
     const int nt = g.taps;
-    for (int c = threadIdx.x; c < g.C; c += blockDim.x) {
-        const float b = bias ? bias[c] : 0.0f;
-        float v;
-        if (nt == 0) v = P[(size_t)r * ldp + c] + b;
-        else {
-            v = 0.0f;
-            for (int i = 0; i < nt; i++) {
-                const int tt = t - (nt - 1) + i;
-                const float in = tt >= 0 ? P[(size_t)(r - t + tt) * ldp + c] + b : tail[(size_t)(nt - 1 + tt) * g.C + c];
-                v = fmaf(cw[(size_t)c * nt + i], in, v);
-            }
-            if (shift_tail && nt > 1) {   // every run has one row (decoding): the tail moves on by this input, channel by channel
-                for (int i = 0; i + 1 < nt - 1; i++) tail[(size_t)i * g.C + c] = tail[(size_t)(i + 1) * g.C + c];
-                tail[(size_t)(nt - 2) * g.C + c] = P[(size_t)r * ldp + c] + b;
-            }
-        }
-        y[c] = v;
-    }
-    for (int i = threadIdx.x; i < g.rot_dims / 2; i += blockDim.x) {
+    // the angles by the last threads, which have the fewest channels, while the others' loads are under way
+    for (int i = (int)(blockDim.x - 1 - threadIdx.x); i < g.rot_dims / 2; i += blockDim.x) {
         double s, c;
         sincos((double)pos * inv_freq[i], &s, &c);
         cs[i] = (float)c * g.rot_gain;
         sn[i] = (float)s * g.rot_gain;
+    }
+    // PV channels per thread at a time, every load of them before the first store (a store between makes the next channel's loads wait for it)
+    constexpr int PV = 4, PT = 4;
+    if (nt <= PT) {
+        for (int c0 = threadIdx.x; c0 < g.C; c0 += PV * blockDim.x) {
+            float in[PV][PT], wv[PV][PT], b[PV];
+#pragma unroll
+            for (int u = 0; u < PV; u++) {
+                const int c = c0 + u * blockDim.x;
+                const bool ok = c < g.C;
+                b[u] = ok && bias ? bias[c] : 0.0f;
+                if (nt == 0) in[u][0] = ok ? P[(size_t)r * ldp + c] : 0.0f;
+#pragma unroll
+                for (int i = 0; i < PT; i++)
+                    if (i < nt) {
+                        const int tt = t - (nt - 1) + i;
+                        in[u][i] = !ok ? 0.0f : tt >= 0 ? P[(size_t)(r - t + tt) * ldp + c] : tail[(size_t)(nt - 1 + tt) * g.C + c];
+                        wv[u][i] = ok ? cw[(size_t)c * nt + i] : 0.0f;
+                    }
+            }
+#pragma unroll
+            for (int u = 0; u < PV; u++) {
+                const int c = c0 + u * blockDim.x;
+                if (c >= g.C) continue;
+                float v = 0.0f;
+                if (nt == 0) v = in[u][0] + b[u];
+#pragma unroll
+                for (int i = 0; i < PT; i++)
+                    if (i < nt) {
+                        if (t - (nt - 1) + i >= 0) in[u][i] += b[u];
+                        v = fmaf(wv[u][i], in[u][i], v);
+                    }
+                if (shift_tail && nt > 1) {   // every run has one row (decoding): the tail moves on by this input, channel by channel
+#pragma unroll
+                    for (int i = 0; i + 1 < PT; i++)
+                        if (i + 1 < nt) tail[(size_t)i * g.C + c] = in[u][i + 1];
+                }
+                y[c] = v;
+            }
+        }
+    } else {
+        for (int c = threadIdx.x; c < g.C; c += blockDim.x) {
+            const float b = bias ? bias[c] : 0.0f;
+            float v;
+            if (nt == 0) v = P[(size_t)r * ldp + c] + b;
+            else {
+                v = 0.0f;
+                for (int i = 0; i < nt; i++) {
+                    const int tt = t - (nt - 1) + i;
+                    const float in = tt >= 0 ? P[(size_t)(r - t + tt) * ldp + c] + b : tail[(size_t)(nt - 1 + tt) * g.C + c];
+                    v = fmaf(cw[(size_t)c * nt + i], in, v);
+                }
+                if (shift_tail && nt > 1) {   // every run has one row (decoding): the tail moves on by this input, channel by channel
+                    for (int i = 0; i + 1 < nt - 1; i++) tail[(size_t)i * g.C + c] = tail[(size_t)(i + 1) * g.C + c];
+                    tail[(size_t)(nt - 2) * g.C + c] = P[(size_t)r * ldp + c] + b;
+                }
+            }
+            y[c] = v;
+        }
     }
     if (g.v_rot) {
         for (int i = threadIdx.x; i < a.vdim / 2; i += blockDim.x) {
