@@ -24,60 +24,11 @@
 
 namespace b200 {
 
-struct RopeKvParams {
-    float* q;              // [n_heads * hd] in place
-    const float* k;        // [n_kv * hd] raw projection (+bias)
-    const float* v;        // [n_kv * hd]
-    float* k_cache;        // [n_kv][max_seq][hd]
-    float* v_cache;
-    const float* freq;     // [hd/2] = 1 / base^(2i/hd), computed on the host with libm powf
-    const int* pos;        // device scalar: position of the current token
-    int n_heads, n_kv, hd, max_seq, neox;
-    float rope_scale;
-    long long kv_head_stride, kv_pos_stride;   // floats; 0 = the reference layout [n_kv][max_seq][hd]
-};
 // offset (floats) of row (kv head, position) in a K or V cache
 template <class P>
 __device__ __forceinline__ size_t kv_row(const P& p, int kh, int pos, int hd) {
     return p.kv_pos_stride ? (size_t)kh * (size_t)p.kv_head_stride + (size_t)pos * (size_t)p.kv_pos_stride
                            : ((size_t)kh * p.max_seq + pos) * hd;
-}
-
-// Backend::rope + cache write.  One thread per rotated pair, then one per v element.
-__global__ void rope_kv_kernel(const RopeKvParams p) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int pos = *p.pos;
-    const int half = p.hd >> 1;
-    const int n_pairs = (p.n_heads + p.n_kv) * half;
-    const int n_v = p.n_kv * p.hd;
-    const float position = (float)pos / p.rope_scale;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pairs + n_v; i += gridDim.x * blockDim.x) {
-        if (i < n_pairs) {
-            const int head = i / half, pi = i - head * half;
-            const float theta = position * p.freq[pi];
-            const float c = cosf(theta), s = sinf(theta);
-            const int i0 = p.neox ? pi : 2 * pi;
-            const int i1 = p.neox ? pi + half : 2 * pi + 1;
-            if (head < p.n_heads) {
-                float* d = p.q + (size_t)head * p.hd;
-                const float x0 = d[i0], x1 = d[i1];
-                d[i0] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-                d[i1] = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
-            } else {
-                const int kh = head - p.n_heads;
-                const float* d = p.k + (size_t)kh * p.hd;
-                float* o = p.k_cache + kv_row(p, kh, pos, p.hd);
-                const float x0 = d[i0], x1 = d[i1];
-                o[i0] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-                o[i1] = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
-            }
-        } else {
-            const int j = i - n_pairs;
-            const int kh = j / p.hd, d = j - kh * p.hd;
-            p.v_cache[kv_row(p, kh, pos, p.hd) + d] = p.v[j];
-        }
-    }
 }
 
 constexpr int kAttnWarps = 8;
@@ -96,7 +47,7 @@ struct AttnParams {
     int min_chunk;         // KV positions per split below which a context is not split further (0: kAttnMinChunk)
     float scale;
     // optional fused RoPE + KV-cache write (per-token megakernel): q | k | v raw from the QKV GEMV (+bias), rotated
-    // here exactly as rope_kv_kernel does; the split that owns position `pos` also writes the cache rows
+    // here as Backend::rope does (cpu/ops.rs:1216-1337); the split that owns position `pos` also writes the cache rows
     const float* qkv_raw;  // nullptr: q is already rotated, the cache already holds position pos
     const float* freq;     // [hd/2]
     float rope_scale;

@@ -58,6 +58,8 @@ struct GemvParams {
     // expert lives on another GPU returns at once; EPI_SCALED_ACC writes out[j] = wt * acc (no accumulate, no residual): the
     // weighted output of ONE expert, combined across GPUs by ep_combine_kernel (misc.cuh).  expert_count == 0: off.
     int expert_base, expert_count;
+    // n_slots > 1: all selected experts in one launch (the tensor-pipe kernel only, gemv_mma.cuh): slot s reads x + s x_slot and writes out + s out_slot
+    int n_slots, x_slot, out_slot;
 };
 
 // byte k of w, less `off`, as a float: PRMT drops it into the mantissa of 2^23, one subtraction removes 2^23 + off (exact; an integer conversion runs at a quarter of

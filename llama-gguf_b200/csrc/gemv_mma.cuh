@@ -107,6 +107,9 @@ struct MParams {
     const float* expert_wt;
     int expert_slot;
     int expert_base, expert_count;   // expert parallel: see GemvParams (gemv.cuh)
+    // n_slots > 1: the selected experts share the launch, n_ctas / n_slots CTAs each (cbase, crem and total_units are one slot's).  A launch for itself fills its
+    // rings, stages x and merges its cut tiles for 17 us beside the bytes of an expert of an 8 x 7B layer (12 and 7 us)
+    int n_slots, x_slot, out_slot;
     // tensor parallel (megakernel only).  Input side: x = sum_r xsum[r * sum_stride + e] (+ x_res[e]) -- the
     // all-reduce of a row-parallel GEMV is finished by its consumer, in rank order on every rank; CTA 0 also
     // stores the summed vector to x_full_out (it is the residual of a later phase).  Output side: the finished
@@ -778,10 +781,12 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
     // units are dealt in contiguous runs, CTA after CTA, warp after warp: the pieces of a tile meet inside one CTA
     // (merged through shared memory); only tiles that straddle CTAs (tile_mode 0) go through global memory
     const int upt = p.units_per_tile;
-    const int cta = blockIdx.x;
+    const int per_slot = p.n_slots > 1 ? p.n_ctas / p.n_slots : 0;
+    const int slot_cta0 = p.n_slots > 1 ? (int)blockIdx.x / per_slot * per_slot : 0, ex_slot = p.n_slots > 1 ? min((int)blockIdx.x / per_slot, p.n_slots - 1) : p.expert_slot;
+    const int cta = blockIdx.x - slot_cta0;      // (among its slot's)
     const long long gw = (long long)blockIdx.x * nw + warp;  // debug stamps only
     int cu0 = 0, cu1 = 0;
-    if (cta < p.n_ctas) {
+    if ((int)blockIdx.x < p.n_ctas) {
         const int first = cta * p.cbase + min(cta, p.crem), cnt = p.cbase + (cta < p.crem ? 1 : 0);
         cu0 = p.tile_mode ? first * upt : first;
         cu1 = p.tile_mode ? (first + cnt) * upt : first + cnt;
@@ -921,7 +926,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
     MMA_STAMP(1);
 
     if (p.expert_sel) {
-        eoff = (long long)p.expert_sel[p.expert_slot];
+        eoff = (long long)p.expert_sel[ex_slot];
         if (p.expert_count > 0) {   // expert parallel: not this GPU's expert -> nothing to do (uniform over the grid)
             eoff -= p.expert_base;
             if (eoff < 0 || eoff >= p.expert_count) return;
@@ -955,7 +960,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
     } else {
         // x: the loads are issued BEFORE the weight copies, the split after them
         XStage xst;
-        const XSource xsrc{p.x, p.xsum, p.n_sum, p.sum_stride, p.x_res, p.x_full_out};
+        const XSource xsrc{p.n_slots > 1 ? p.x + (size_t)ex_slot * p.x_slot : p.x, p.xsum, p.n_sum, p.sum_stride, p.x_res, p.x_full_out};
         stage_x_load(xst, xsrc, p.norm_w, K, (int)blockDim.x);
         if (!issued_early) {
             for (int k = 0; k < STAGES - 1; k++) {
@@ -1001,7 +1006,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
             if (p.n_peer > 0) {
                 for (int r = 0; r < p.n_peer; r++) p.peer_out[r][j] = val;  // partial of a row-parallel GEMV, to every rank
             } else {
-                sg.out[j] = val;
+                sg.out[(p.n_slots > 1 ? (size_t)ex_slot * p.out_slot : 0) + j] = val;
             }
         }
         if (p.stage_out) stage_out32(val, e_w, j, p.stage_K, p.stage_out);   // the next GEMV's input, ready to copy
@@ -1146,9 +1151,9 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
             vu += s_part[w][ws][1][lane];
         }
         if (tu0 < cu0 || tu0 + upt > cu1) {  // the tile straddles CTAs (tile_mode 0 only)
-            const int tile_id = (s == 0 ? 0 : (s == 1 ? p.seg[0].n_tiles : p.seg[0].n_tiles + p.seg[1].n_tiles)) + tile;
+            const int tile_id = (p.n_slots > 1 ? ex_slot * (p.total_units / upt) : 0) + (s == 0 ? 0 : (s == 1 ? p.seg[0].n_tiles : p.seg[0].n_tiles + p.seg[1].n_tiles)) + tile;
             const int c_first = cta_of(tu0), c_last = cta_of(tu0 + upt - 1);
-            float* mine = p.part + ((size_t)cta * 2 + ((cu0 >= tu0) ? 0 : 1)) * 64;
+            float* mine = p.part + ((size_t)(slot_cta0 + cta) * 2 + ((cu0 >= tu0) ? 0 : 1)) * 64;
             mine[lane] = v;
             mine[32 + lane] = vu;
             __syncwarp();
@@ -1159,7 +1164,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
             v = 0.f;
             vu = 0.f;
             for (int c = c_first; c <= c_last; c++) {
-                const float* theirs = p.part + ((size_t)c * 2 + ((cta_first(c) >= tu0) ? 0 : 1)) * 64;
+                const float* theirs = p.part + ((size_t)(slot_cta0 + c) * 2 + ((cta_first(c) >= tu0) ? 0 : 1)) * 64;
                 v += ld_relaxed_gpu(theirs + lane);
                 vu += ld_relaxed_gpu(theirs + 32 + lane);
             }
@@ -1301,6 +1306,13 @@ inline bool mma_plan(MParams& p, int n_sm, int want_warps, int want_stages, size
     plan.smem = need(warps, stages);
     plan.grid = (int)std::min<long long>(n_sm, (p.total_units + warps - 1) / warps);
     if (plan.grid < 1) plan.grid = 1;
+    if (p.n_slots > 1) {
+        if (p.epi == ME_SCALED_ACC || p.expert_count > 0 || p.n_slots > n_sm) return false;
+        mma_deal(p, std::min(plan.grid, n_sm / p.n_slots));
+        p.n_ctas *= p.n_slots;
+        plan.grid = p.n_ctas;
+        return true;
+    }
     mma_deal(p, plan.grid);
     return true;
 }

@@ -45,7 +45,7 @@ __device__ __forceinline__ float kv_q8_row(const float (&x)[VEC], signed char (&
 }
 
 // One warp per head unit: n_heads query heads (rotated in place), n_kv key heads (rotated, quantised, stored), n_kv value heads
-// (quantised, stored).  Rotation arithmetic as rope_kv_kernel (ops.rs:1216-1337).  HD = 32 * VEC.  `q`, `k`, `v` are the rows of ONE
+// (quantised, stored).  Rotation arithmetic as attn_decode_item (ops.rs:1216-1337).  HD = 32 * VEC.  `q`, `k`, `v` are the rows of ONE
 // token, `pos` its position.
 template <int VEC>
 __device__ __forceinline__ void rope_kv_q8_unit(const RopeKvQ8Params& p, float* q, const float* k, const float* v, int pos, int unit, int lane) {

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float* __restri
 
 // MoeRouter::route (src/model/moe.rs:128-198) with normalize=false: logits = W_r h (f32),
 // stable descending top-k (ties -> lowest expert index), softmax over the k selected.
-// One CTA; warp e computes logit e.  h is the (already RMS-normalised) FFN input.
+// h is the (already RMS-normalised) FFN input.
 struct RouteParams {
     const float* x;        // [hidden] un-normalised hidden state
     const float* norm_w;   // ffn_norm weight (fused RMSNorm, same as the GEMV prologue)
@@ -122,68 +122,67 @@ struct RouteParams {
     int hidden, n_experts, top_k;
     int* sel;              // out [top_k]
     float* wt;             // out [top_k]
+    float* logits;         // scratch [n_experts]
+    unsigned int* ticket;  // zero on entry, left zero on exit
     unsigned int* epoch;   // optional (expert parallel): bumped once per call -- the layer's exchange epoch, the same on every GPU
 };
-// One CTA: bound by latency, so every load of the row is in flight at once.  The 32 warps are dealt over (expert, segment of the row); a warp adds
-// x norm_w w_router over its segment (1 / rms comes out of the sum), beside the sum of squares.  4096 wide, 8 experts: 44 -> 11 us against
-// one warp per expert that walked the row with one element per lane after a pass of its own for the sum of squares.
-constexpr int kRouteThreads = 1024;
+// A block per expert: x norm_w w_router and the sum of squares of x over the row (1 / rms comes out of the sum), every load in flight at once; the last block to
+// arrive takes the choice.  Bound by latency (4096 wide, 8 experts: one block of 1024 threads, which read 131 KB of router rows alone, took 11 us).
+constexpr int kRouteThreads = 256;
 __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const RouteParams p) {
     pdl_launch_dependents();
-    pdl_wait();
-    __shared__ float red[32], part[64];
-    __shared__ float logits[64];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* wr = p.w_router + (size_t)e * p.hidden;
     const bool v4 = (p.hidden & 3) == 0 && (((uintptr_t)p.x | (uintptr_t)p.norm_w | (uintptr_t)p.w_router) & 15) == 0;
-    const int V = v4 ? 4 : 1, n = p.hidden / V, S = p.n_experts <= 16 ? 32 / p.n_experts : 1;
-    float ss = 0.0f;
-    for (int i = threadIdx.x; i < n; i += kRouteThreads) {
-        if (v4) {
-            const float4 v = reinterpret_cast<const float4*>(p.x)[i];
-            ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
-        } else ss = fmaf(p.x[i], p.x[i], ss);
-    }
-    for (int u = warp; u < p.n_experts * S; u += 32) {
-        const int e = u / S, sg = u - e * S, beg = (int)((long long)n * sg / S), end = (int)((long long)n * (sg + 1) / S);
-        const float* wr = p.w_router + (size_t)e * p.hidden;
-        float d = 0.0f;
-        if (v4) {
-#pragma unroll 8
-            for (int i = beg + lane; i < end; i += 32) {
-                const float4 x = reinterpret_cast<const float4*>(p.x)[i], w = reinterpret_cast<const float4*>(p.norm_w)[i], r = reinterpret_cast<const float4*>(wr)[i];
-                d = fmaf(x.x * w.x, r.x, d);
-                d = fmaf(x.y * w.y, r.y, d);
-                d = fmaf(x.z * w.z, r.z, d);
-                d = fmaf(x.w * w.w, r.w, d);
-            }
-        } else {
-            for (int i = beg + lane; i < end; i += 32) d = fmaf(p.x[i] * p.norm_w[i], wr[i], d);
+    if (v4 && threadIdx.x * 32 < p.hidden) prefetch_l2(wr + threadIdx.x * 32);
+    pdl_wait();
+    __shared__ float red[2][kRouteThreads / 32];
+    __shared__ float logits[64];
+    __shared__ int is_last;
+    float ss = 0.0f, d = 0.0f;
+    if (v4) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < p.hidden / 4; i += kRouteThreads) {
+            const float4 x = reinterpret_cast<const float4*>(p.x)[i], w = reinterpret_cast<const float4*>(p.norm_w)[i], r = reinterpret_cast<const float4*>(wr)[i];
+            ss += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
+            d = fmaf(x.x * w.x, r.x, d);
+            d = fmaf(x.y * w.y, r.y, d);
+            d = fmaf(x.z * w.z, r.z, d);
+            d = fmaf(x.w * w.w, r.w, d);
         }
-        d = warp_sum(d);
-        if (lane == 0) part[u] = d;
+    } else {
+        for (int i = threadIdx.x; i < p.hidden; i += kRouteThreads) {
+            ss = fmaf(p.x[i], p.x[i], ss);
+            d = fmaf(p.x[i] * p.norm_w[i], wr[i], d);
+        }
     }
     ss = warp_sum(ss);
-    if (lane == 0) red[warp] = ss;
-    __syncthreads();
-    if (warp == 0) {
-        const float inv = 1.0f / sqrtf(warp_sum(red[lane]) / (float)p.hidden + p.eps);
-        for (int e = lane; e < p.n_experts; e += 32) {
-            float d = 0.0f;
-            for (int sg = 0; sg < S; sg++) d += part[e * S + sg];
-            logits[e] = d * inv;
-        }
-    }
+    d = warp_sum(d);
+    if (lane == 0) { red[0][warp] = ss; red[1][warp] = d; }
     __syncthreads();
     if (threadIdx.x == 0) {
+        float s = 0.0f, t = 0.0f;
+        for (int i = 0; i < kRouteThreads / 32; i++) { s += red[0][i]; t += red[1][i]; }
+        p.logits[e] = t / sqrtf(s / (float)p.hidden + p.eps);
+        unsigned int n;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(n) : "l"(p.ticket) : "memory");
+        is_last = n == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    if ((int)threadIdx.x < p.n_experts) logits[threadIdx.x] = __ldcg(p.logits + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *p.ticket = 0u;
         if (p.epoch) *p.epoch += 1u;
         unsigned long long taken = 0ull;
         float sel_l[8];
         float mx = -INFINITY;
         for (int k = 0; k < p.top_k; k++) {
             int best = -1;
-            for (int e = 0; e < p.n_experts; e++) {
-                if ((taken >> e) & 1ull) continue;
-                if (best < 0 || logits[e] > logits[best]) best = e;  // strict >: lowest index wins ties
+            for (int e2 = 0; e2 < p.n_experts; e2++) {
+                if ((taken >> e2) & 1ull) continue;
+                if (best < 0 || logits[e2] > logits[best]) best = e2;  // strict >: lowest index wins ties
             }
             taken |= 1ull << best;
             p.sel[k] = best;
@@ -194,6 +193,18 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const RoutePar
         for (int k = 0; k < p.top_k; k++) sum += expf(sel_l[k] - mx);
         for (int k = 0; k < p.top_k; k++) p.wt[k] = expf(sel_l[k] - mx) / sum;
     }
+}
+
+// out = ((0 + w_0 y_0) + w_1 y_1 ..) + residual: the selected experts' outputs in selection order (moe.rs:363-368, layers.rs:1235-1241)
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, int n_slots, const float* __restrict__ wt, const float* __restrict__ residual,
+                                                          float* __restrict__ out, int hidden) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    if (j >= hidden) return;
+    float v = 0.0f;
+    for (int s = 0; s < n_slots; s++) v = fmaf(wt[s], y[(size_t)s * hidden + j], v);
+    out[j] = v + residual[j];
 }
 
 // ---- Backend element-wise surface (kernels.rs:48-95 equivalents; cpu/ops.rs) ----
@@ -273,7 +284,7 @@ __global__ void vec_mat_f32_kernel(const float* a, const float* w, float* out, i
     if (lane == 0) out[row] = s;
 }
 
-// Backend::rope on host-provided q/k (per-op surface): same math as rope_kv_kernel.
+// Backend::rope on host-provided q/k (per-op surface): same math as attn_decode_item (attention.cuh).
 __global__ void rope_inplace_kernel(float* q, float* k, const float* freq, int n_heads, int n_kv, int hd, int pos,
                                     float rope_scale, int neox) {
     const int half = hd >> 1;

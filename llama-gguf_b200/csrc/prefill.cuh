@@ -1,6 +1,6 @@
 // prefill.cuh — the memory-bound kernels around the tcgen05 dequant-GEMM (gemm_umma.cuh) when a prompt is processed T
 // tokens at a time: embedding rows, RoPE + KV-cache write, causal GQA attention over the cache, SwiGLU.
-// Same arithmetic as the per-token kernels (embed_kernel, rope_kv_kernel, attn_decode_item) and as the reference
+// Same arithmetic as the per-token kernels (embed_kernel, attn_decode_item) and as the reference
 // (LlamaModel::forward src/model/llama.rs:275-362; ops::rope cpu/ops.rs:1216-1337; attention_cached :1479-1537;
 // silu_mul_inplace cpu/simd.rs:598-649), applied to T rows.
 #pragma once
