@@ -671,13 +671,29 @@ __global__ void lp_attn_prep_kernel(StepMeta sm, AttnGeom a, const float* __rest
 // scores (q from shared memory), online softmax in f32 per warp, then the block's 32 value rows are added lane-per-channel; the
 // warps' partial (max, sum, output) triples are merged through shared memory.  Visible keys of position i: [0, min(keep_first, lo))
 // and [lo, i], lo = max(0, i - window + 1).  The output is multiplied by sigmoid(gate) when the layer has an output gate.
+// Short rows (dim and vdim up to 128): every warp brings its blocks' rows through a ring of 4 KB chunks in shared memory (eight rows of keys or values,
+// 16-byte cp.async), as many in flight as the ring has room for: a block of 32 keys is eight of them.  With loads into registers a block of 32 keys was
+// eight trips to memory one after the other (110 keys, one row of 16 heads: 24 -> 7 us).  The same sums in the same order.
+constexpr int ATT_RING = 48, ATT_CHUNK = 8 * 128;   // chunks of 8 rows x 128 floats: 192 KB
+__device__ __forceinline__ void att_wait(int n) {    // at most n newest groups still in flight
+    switch (n) {
+        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+        case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+        case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+    }
+}
 constexpr int ATT_ACC = 16;   // value channels per lane at most: vdim <= 512 (the kernel is instantiated for 4, 8 and 16)
 constexpr int ATT_WARPS = 16;
 constexpr int ATT_QCH = 2;    // 16-byte query chunks per lane in the split-channel score loop: dim <= 256 (wider: one key per lane)
 template <typename OutT, int VCH>
 __global__ void __launch_bounds__(32 * ATT_WARPS) lp_window_attn_kernel(StepMeta sm, AttnGeom a, const float* __restrict__ qbuf,
                                                                         const float* __restrict__ P, int ldp, const float* __restrict__ qw,
-                                                                        const float* __restrict__ kw, OutT* __restrict__ out) {
+                                                                        const float* __restrict__ kw, OutT* __restrict__ out, int ring_at) {
     prev_grid();
     extern __shared__ __align__(16) float smem[];
     float* qs = smem;                                  // [dim]
@@ -737,6 +753,87 @@ __global__ void __launch_bounds__(32 * ATT_WARPS) lp_window_attn_kernel(StepMeta
         const int d = (lane + 32 * c) * 4;
         qr[c] = (v4 && d < a.dim) ? *reinterpret_cast<const float4*>(qs + d) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    if (VCH == 4 && ring_at > 0) {      // (dim and vdim multiples of 4, up to 128)
+        const int nb = nb0 + nb1, depth = min(8, ATT_RING / min(ATT_WARPS, nb)), total = warp < nb ? 8 * ((nb - warp + ATT_WARPS - 1) / ATT_WARPS) : 0;
+        float* ring = smem + ring_at + (size_t)warp * depth * ATT_CHUNK;      // (warps without a block use none)
+        const int d = lane * 4;
+        auto at = [&](int q, int& j0, int& end) {      // chunk q: keys (4) and then values (4) of one block
+            const int b = warp + ATT_WARPS * (q >> 3);
+            j0 = b < nb0 ? b * 32 : lo + (b - nb0) * 32;
+            end = b < nb0 ? a_end : i + 1;
+        };
+        auto issue = [&](int q, int slot) {
+            if (q < total) {
+                int j0, end;
+                at(q, j0, end);
+                const bool val = q & 4;
+                const int first = j0 + 8 * (q & 3);
+                const float* src = val ? vc + gv : kc + g * a.dim;
+                const size_t ld = val ? ldv : ldk;
+                if (d < (val ? a.vdim : a.dim)) {
+#pragma unroll
+                    for (int u = 0; u < 8; u++)
+                        if (first + u < end) cp_async16(smem_u32(ring + (size_t)slot * ATT_CHUNK + u * 128 + d), src + (size_t)(first + u) * ld + d, 16u);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (int q = 0; q < (total ? depth : 0); q++) issue(q, q);
+        float s = -INFINITY, p = 0.0f;
+        int slot = 0;
+        for (int q = 0; q < total; q++) {
+            int j0, end;
+            at(q, j0, end);
+            const int cnt = min(32, end - j0), jb = 8 * (q & 3);
+            att_wait(depth - 1);
+            __syncwarp();
+            const float* ch = ring + (size_t)slot * ATT_CHUNK;
+            if (!(q & 4)) {
+                if (jb == 0) s = -INFINITY;
+                float part[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    part[u] = 0.0f;
+                    if (jb + u < cnt && d < a.dim) {
+                        const float4 kv = *reinterpret_cast<const float4*>(ch + u * 128 + d);
+                        part[u] = fmaf(qr[0].x, kv.x, part[u]);
+                        part[u] = fmaf(qr[0].y, kv.y, part[u]);
+                        part[u] = fmaf(qr[0].z, kv.z, part[u]);
+                        part[u] = fmaf(qr[0].w, kv.w, part[u]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const float tot = wsum(part[u]);
+                    if (lane == jb + u && jb + u < cnt) s = tot * a.scale;
+                }
+            } else {
+                if (jb == 0) {
+                    const int j = j0 + lane;
+                    if (kinv && j < end) s *= kinv[(size_t)j * a.G];
+                    if (j < end) s = attn_score(a, s, slope, i, j);
+                    const float m_new = fmaxf(m, wmax(s));
+                    p = j < end ? expf(s - m_new) : 0.0f;
+                    const float corr = expf(m - m_new);      // (m = -inf on the warp's first block: 0)
+                    l = l * corr + wsum(p);
+                    m = m_new;
+#pragma unroll
+                    for (int c = 0; c < VCH; c++) acc[c] *= corr;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const float pj = __shfl_sync(0xffffffffu, p, jb + u);
+                    if (jb + u < cnt) {
+#pragma unroll
+                        for (int c = 0; c < VCH; c++) acc[c] = fmaf(pj, c * 32 + lane < a.vdim ? ch[u * 128 + c * 32 + lane] : 0.0f, acc[c]);
+                    }
+                }
+            }
+            __syncwarp();
+            issue(q + depth, slot);
+            slot = slot + 1 == depth ? 0 : slot + 1;
+        }
+    } else
     for (int b = warp; b < nb0 + nb1; b += ATT_WARPS) {
         const int j0 = b < nb0 ? b * 32 : lo + (b - nb0) * 32;
         const int end = b < nb0 ? a_end : i + 1;
@@ -2812,6 +2909,8 @@ int lp_finalize(LpModel* m, std::string* err) {
         if (need > 200 * 1024) return lp_fail(err, B200_ERR_UNSUPPORTED, "softmax mixer: q, k and v of one token exceed 200 KB of shared memory");
         if (need > 32 * 1024) LCU(cudaFuncSetAttribute(lp_attn_prep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     }
+    LCU(cudaFuncSetAttribute(lp_window_attn_kernel<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+    LCU(cudaFuncSetAttribute(lp_window_attn_kernel<bf16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
     if (m->lat_o_floats > 0) {
         LCU_ALLOC(cudaMalloc((void**)&m->lat_o, up16(m->lat_o_floats * 4)));
         LCU_ALLOC(cudaMalloc((void**)&m->lat_ml, up16(m->lat_ml_floats * 4)));
@@ -3218,9 +3317,14 @@ int glin_segments(const LpModel* m, int H, int dim, int vdim, int n_runs, int ma
 // The warp kernel: any row count, both compute modes.
 void attn_rows(LpModel* m, const StepMeta& sm, const AttnGeom& ag, const LayerPlan& L, int R) {
     dim3 agrid(R, ag.H);
-    const size_t asmem = (size_t)(((ag.dim + 3) & ~3) + ATT_WARPS * ag.vdim + 2 * ATT_WARPS + (ag.vrot ? ag.vdim : 0)) * 4;
+    size_t asmem = (size_t)(((ag.dim + 3) & ~3) + ATT_WARPS * ag.vdim + 2 * ATT_WARPS + (ag.vrot ? ag.vdim : 0)) * 4;
+    int ring_at = 0;
+    if (ag.dim % 4 == 0 && ag.vdim % 4 == 0 && ag.dim <= 128 && ag.vdim <= 128 && ag.kv_off % 16 == 0) {
+        ring_at = (int)((asmem + 15) / 16 * 4);
+        asmem = (size_t)(ring_at + ATT_RING * ATT_CHUNK) * 4;
+    }
     const int vch = ag.vdim <= 128 ? 4 : ag.vdim <= 256 ? 8 : 16;
-#define LP_ATTN(T, V) launch(m, lp_window_attn_kernel<T, V>, agrid, dim3(32 * ATT_WARPS), asmem, sm, ag, (const float*)m->qbuf, (const float*)m->P, L.n_in, L.qn, L.kn, (T*)m->act_a)
+#define LP_ATTN(T, V) launch(m, lp_window_attn_kernel<T, V>, agrid, dim3(32 * ATT_WARPS), asmem, sm, ag, (const float*)m->qbuf, (const float*)m->P, L.n_in, L.qn, L.kn, (T*)m->act_a, ring_at)
     if (m->f32) {
         if (vch == 4) LP_ATTN(float, 4); else if (vch == 8) LP_ATTN(float, 8); else LP_ATTN(float, 16);
     } else {
