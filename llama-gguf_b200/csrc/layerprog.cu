@@ -2907,7 +2907,8 @@ int lp_finalize(LpModel* m, std::string* err) {
             if ((L.d.mixer == B200_MIX_SOFTMAX_ATTN || L.d.mixer == B200_MIX_ATTN_RECURRENT) && !L.d.sattn.v_from_k)
                 need = std::max(need, (size_t)(((L.pg.C + 3) & ~3) + L.pg.rot_dims + (L.pg.v_rot ? L.ag.vdim : 0)) * 4);
         if (need > 200 * 1024) return lp_fail(err, B200_ERR_UNSUPPORTED, "softmax mixer: q, k and v of one token exceed 200 KB of shared memory");
-        if (need > 32 * 1024) LCU(cudaFuncSetAttribute(lp_attn_prep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+        if (need > 32 * 1024)
+            for (auto k : {lp_attn_prep2_kernel<true>, lp_attn_prep2_kernel<false>}) LCU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     }
     LCU(cudaFuncSetAttribute(lp_window_attn_kernel<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
     LCU(cudaFuncSetAttribute(lp_window_attn_kernel<bf16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
@@ -3618,8 +3619,8 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
             pg.rec_off = m->run_rec_off[run];
             const size_t psmem = (size_t)(((pg.C + 3) & ~3) + pg.rot_dims + (pg.v_rot ? ag.vdim : 0)) * 4;
             const int shift = (m->use_fuse && max_len == 1) ? 1 : 0;   // one row per run: the row's block moves the run's tail on itself
-            launch(m, lp_attn_prep2_kernel, dim3(R), dim3(256), psmem, sm, ag, pg, (const float*)m->P, L.n_in, L.qkv_bias, L.conv_w, L.qn, L.kn, L.rot_freq,
-                   L.vmix, m->vsrc, m->qbuf, shift, L.v_freq, m->vrot);
+            launch(m, shift ? lp_attn_prep2_kernel<true> : lp_attn_prep2_kernel<false>, dim3(R), dim3(256), psmem, sm, ag, pg, (const float*)m->P, L.n_in, L.qkv_bias, L.conv_w, L.qn, L.kn, L.rot_freq,
+                   L.vmix, m->vsrc, m->qbuf, L.v_freq, m->vrot);
             if (pg.taps > 1 && !shift) launch(m, lp_attn_conv_tail_kernel, dim3(n_runs), dim3(256), 0, sm, pg, (const float*)m->P, L.n_in, L.qkv_bias);
             if (!attn_tile(m, sm, ag, L.n_in, n_runs, max_len)) attn_rows(m, sm, ag, L, R);
             if (!dual) {

@@ -22,15 +22,17 @@ struct PrepGeom {
 // One block per row.  Step 1: u = P + bias, y = causal convolution of u over time (inputs before the run's first row come from the
 // run's tail, zeros at the start of a sequence) into shared memory.  Step 2: per head of q and k (a warp each): rotate the first
 // rot_dims channels (channel 2i with 2i + 1).  Step 3: the norm (over the whole of q and of k, or a warp per head).  Step 4: q to
-// qbuf, k to the cache row, v (blended) to the cache row.  shift_tail: the step has one row per run and the block also moves the
+// qbuf, k to the cache row, v (blended) to the cache row.  STEP: the step has one row per run and the block also moves the
 // run's tail on by this row (else lp_attn_conv_tail_kernel does it for the whole run afterwards).  rot_after_norm swaps steps 2 and 3.
 // v_rot: the pairs (2m, 2m + 1) of every value head are turned by pos * v_freq[m]; cos | sin of these angles also go to
 // vrot_out[r][vdim], where the attention kernels find them to turn the summed values back.
+// STEP (shift_tail): one row per run.  There are few blocks then, each bound by its own loads; prompts have a block per token and want them small
+template <bool STEP>
 __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeom a, PrepGeom g, const float* __restrict__ P, int ldp,
                                                             const float* __restrict__ bias, const float* __restrict__ cw,
                                                             const float* __restrict__ qw, const float* __restrict__ kw,
                                                             const double* __restrict__ inv_freq, const float* __restrict__ lam_p,
-                                                            float* __restrict__ vsrc, float* __restrict__ qbuf, int shift_tail,
+                                                            float* __restrict__ vsrc, float* __restrict__ qbuf,
                                                             const double* __restrict__ v_freq, float* __restrict__ vrot_out) {
     prev_grid();
     extern __shared__ __align__(16) float ps[];
@@ -43,16 +45,17 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
     const int run = sm.row_run[r], pos = sm.row_pos[r], t = r - sm.run_start[run];
     float* tail = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off);
     const int nt = g.taps;
-    // the angles by the last threads, which have the fewest channels, while the others' loads are under way
-    for (int i = (int)(blockDim.x - 1 - threadIdx.x); i < g.rot_dims / 2; i += blockDim.x) {
-        double s, c;
-        sincos((double)pos * inv_freq[i], &s, &c);
-        cs[i] = (float)c * g.rot_gain;
-        sn[i] = (float)s * g.rot_gain;
-    }
+    // the angles first (by the last threads, which have the fewest channels): the others' loads are under way meanwhile
+    if (STEP)
+        for (int i = (int)(blockDim.x - 1 - threadIdx.x); i < g.rot_dims / 2; i += blockDim.x) {
+            double s, c;
+            sincos((double)pos * inv_freq[i], &s, &c);
+            cs[i] = (float)c * g.rot_gain;
+            sn[i] = (float)s * g.rot_gain;
+        }
     // PV channels per thread at a time, every load of them before the first store (a store between makes the next channel's loads wait for it)
     constexpr int PV = 4, PT = 4;
-    if (nt <= PT) {
+    if (STEP && nt <= PT) {
         for (int c0 = threadIdx.x; c0 < g.C; c0 += PV * blockDim.x) {
             float in[PV][PT], wv[PV][PT], b[PV];
 #pragma unroll
@@ -81,7 +84,7 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
                         if (t - (nt - 1) + i >= 0) in[u][i] += b[u];
                         v = fmaf(wv[u][i], in[u][i], v);
                     }
-                if (shift_tail && nt > 1) {   // every run has one row (decoding): the tail moves on by this input, channel by channel
+                if (nt > 1) {   // the tail moves on by this input, channel by channel
 #pragma unroll
                     for (int i = 0; i + 1 < PT; i++)
                         if (i + 1 < nt) tail[(size_t)i * g.C + c] = in[u][i + 1];
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
                     const float in = tt >= 0 ? P[(size_t)(r - t + tt) * ldp + c] + b : tail[(size_t)(nt - 1 + tt) * g.C + c];
                     v = fmaf(cw[(size_t)c * nt + i], in, v);
                 }
-                if (shift_tail && nt > 1) {   // every run has one row (decoding): the tail moves on by this input, channel by channel
+                if (STEP && nt > 1) {   // the tail moves on by this input, channel by channel
                     for (int i = 0; i + 1 < nt - 1; i++) tail[(size_t)i * g.C + c] = tail[(size_t)(i + 1) * g.C + c];
                     tail[(size_t)(nt - 2) * g.C + c] = P[(size_t)r * ldp + c] + b;
                 }
@@ -109,6 +112,13 @@ __global__ void __launch_bounds__(256) lp_attn_prep2_kernel(StepMeta sm, AttnGeo
             y[c] = v;
         }
     }
+    if (!STEP)
+        for (int i = threadIdx.x; i < g.rot_dims / 2; i += blockDim.x) {
+            double s, c;
+            sincos((double)pos * inv_freq[i], &s, &c);
+            cs[i] = (float)c * g.rot_gain;
+            sn[i] = (float)s * g.rot_gain;
+        }
     if (g.v_rot) {
         for (int i = threadIdx.x; i < a.vdim / 2; i += blockDim.x) {
             double s, c;
