@@ -16,6 +16,9 @@
 // x 2048 195 -> 112 us (1220 TFLOP/s), 32 x 2048 x 2048 20 -> 8.3 us.
 //   lp_gemm_tc_kernel        persistent: a CTA per SM walks tiles; two accumulators in TMEM, so the epilogue of a tile runs under the
 //                            next tile's products, and the ring never drains between tiles.
+//                            With PAIR two CTAs share a tile of 256 x 256: gate and up of an 8B layer, 2048 rows, 357 -> 327 us (1.47 PFLOP/s, 0.91 of
+//                            cuBLAS's burst rate), its output and down products 132 -> 118 on average.
+//   lp_gemm_tc_rows_kernel   few token rows as M, below.
 //   lp_gemm_tc_split_kernel  few tiles: S = 1, 2, 4 or 8 CTAs of a cluster share a tile's K steps; each leaves its partial sums in its own
 //                            shared memory and every CTA adds one S-th of the tokens out of all of them (distributed shared memory, always
 //                            in CTA order).
@@ -63,6 +66,33 @@ __device__ __forceinline__ bool tc_elect() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
     return ok != 0;
 }
+// Pairs (cta_group::2): the barrier at `bar` of the cluster's CTA 0
+__device__ __forceinline__ uint32_t tc_leader(uint32_t bar) {
+    uint32_t p;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(p) : "r"(bar));
+    return p;
+}
+__device__ __forceinline__ uint32_t tc_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void tc_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc_arrive_leader(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tc_leader(bar)) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {      // the barrier at this place in both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// into this CTA's shared memory, counted by the leader's barrier
+__device__ __forceinline__ void tc_tma_pair(uint32_t dst, const CUtensorMap* map, int k, int row, int slab, int z, uint32_t leader_bar) {
+    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst), "l"(map),
+                 "r"(k), "r"(row), "r"(0), "r"(slab), "r"(z), "r"(leader_bar)
+                 : "memory");
+}
 __device__ __forceinline__ void tc_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -91,6 +121,10 @@ __device__ __forceinline__ void tc_ld32(uint32_t* v, uint32_t taddr) {
 // the ring: 192 KB of the 227; a stage = KH slabs of 128 weight rows, then KH slabs of TN token rows
 template <int TN> struct TcRing {
     static constexpr int KH = TN == 256 ? 1 : 2, W_BYTES = KH * TC_M * 128, X_BYTES = KH * TN * 128, STAGE = W_BYTES + X_BYTES, N = 196608 / STAGE, K = KH * TC_K;
+};
+// ... of a pair of CTAs: each has its 128 weight rows and half of the 256 token rows
+struct TcPairRing {
+    static constexpr int W_BYTES = TC_M * 128, X_BYTES = 128 * 128, STAGE = W_BYTES + X_BYTES, N = 196608 / STAGE, K = TC_K;
 };
 constexpr int TC_EX_BYTES = 32768;      // gated epilogue of the persistent kernel, for each half of its warps: exchanged sums [2][16][64] f32, units [2][32][64] of tc_t
 template <int TN, bool PERSISTENT> constexpr size_t tc_smem_bytes(bool glu) {
@@ -135,6 +169,7 @@ template <int TN> struct TcWalk {
     }
 };
 
+template <bool PAIR = false>
 __device__ __forceinline__ void tc_setup(uint32_t tid, uint32_t warp, uint32_t bar, int stages, uint32_t* s_tmem, int n_acc, uint32_t cols) {
     if (tid == 0) {
         for (int i = 0; i < stages; i++) {
@@ -143,17 +178,23 @@ __device__ __forceinline__ void tc_setup(uint32_t tid, uint32_t warp, uint32_t b
         }
         for (int i = 0; i < n_acc; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8u * (2 * stages + i)) : "memory");                             // accumulator done
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8u * (2 * stages + n_acc + i)), "r"((uint32_t)TC_EPI_WARPS) : "memory");   // accumulator read
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8u * (2 * stages + n_acc + i)), "r"((uint32_t)(PAIR ? 2 * TC_EPI_WARPS : TC_EPI_WARPS)) : "memory");   // accumulator read (by both CTAs of a pair)
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == TC_MMA) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) tc_cluster_sync();      // (the other CTA's barriers are there)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // a producer that gave up at stage s (its empty parity: ph): the copies that it has asked for land before it goes on (bounded)
@@ -196,55 +237,90 @@ __device__ __forceinline__ void tc_mma_stage(uint32_t acc, uint32_t stage, uint3
     }
 }
 
-template <int TN, int EPI>
+// PAIR: two CTAs of a cluster share a tile of 256 weight rows x 256 tokens (tcgen05.mma.cta_group::2, issued by CTA 0): each brings its own 128 weight rows and half of the
+// tokens' rows, 32 KB per 64 elements of K instead of 48, and ends with its own 128 rows.  The sums and their order are the single CTA's.
+template <int TN, int EPI, bool PAIR = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     lp_gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const TcArgs a) {
     next_grid();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
-    constexpr int NS = TcRing<TN>::N, STAGE = TcRing<TN>::STAGE, KS = TcRing<TN>::K;
+    static_assert(!PAIR || TN == 256, "pairs share 256 tokens");
+    constexpr int NS = PAIR ? TcPairRing::N : TcRing<TN>::N, STAGE = PAIR ? TcPairRing::STAGE : TcRing<TN>::STAGE, KS = PAIR ? TcPairRing::K : TcRing<TN>::K;
     constexpr bool GLU = epi_is_glu(EPI);
     __shared__ __align__(8) unsigned long long s_bar[2 * NS + 4];
     __shared__ uint32_t s_tmem;
     uint8_t* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);   // the swizzle is on absolute address bits
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = smem_u32(&s_bar[0]), full = bar, empty = bar + 8u * NS, acc_full = bar + 16u * NS, acc_empty = acc_full + 16u;
-    tc_setup(tid, warp, bar, NS, &s_tmem, 2, 2 * TN);
+    tc_setup<PAIR>(tid, warp, bar, NS, &s_tmem, 2, 2 * TN);
+    const uint32_t rank = PAIR ? tc_cluster_rank() : 0u;
     if (TC_W_WAITS || a.seg || warp != TC_LOAD_W) wait_grid();      // (other weights do not depend on the kernel before)
     const uint32_t tmem = s_tmem, ring = smem_u32(base);
-    const int steps = (a.K + KS - 1) / KS, n_mt = (a.N + (GLU ? TC_M / 2 : TC_M) - 1) / (GLU ? TC_M / 2 : TC_M);
+    const int steps = (a.K + KS - 1) / KS, n_own = (a.N + (GLU ? TC_M / 2 : TC_M) - 1) / (GLU ? TC_M / 2 : TC_M), n_mt = PAIR ? (n_own + 1) / 2 : n_own;
     bool alive = true;
     TcWalk<TN> walk;
     TcTile t;
+    const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, stride = PAIR ? gridDim.x >> 1 : gridDim.x;
+    auto find = [&](int item) {
+        if (!walk.find(a, n_mt, item, t)) return false;
+        if (PAIR) t.m = 2 * t.m + rank;      // (one past the last row tile: zeros in, nothing out)
+        return true;
+    };
     if (warp == TC_LOAD_W || warp == TC_LOAD_X) {
         uint32_t s = 0, ph = 1;
-        for (int item = blockIdx.x; alive && walk.find(a, n_mt, item, t); item += gridDim.x)
+        for (int item = first; alive && find(item); item += stride)
             for (int k = 0; k < steps; k++) {
                 tc_wait(empty + 8u * s, ph, alive, a.err, 1);
                 alive = __all_sync(0xffffffffu, alive);
                 if (!alive) break;
                 if (tc_elect()) {
-                    if (warp == TC_LOAD_W) tc_load<TN, GLU, true>(ring + s * STAGE, &wmap, a, t, k * KS, full + 8u * s);
+                    if constexpr (PAIR) {
+                        const bool is_w = warp == TC_LOAD_W;
+                        const int row = is_w ? t.m * (GLU ? TC_M / 2 : TC_M) : t.row0 + t.t0 + (int)rank * 128, z = is_w || a.x_z ? t.z : 0;
+                        if (rank == 0)      // both CTAs' bytes
+                            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8u * s), "r"((uint32_t)(2 * (is_w ? TcPairRing::W_BYTES : TcPairRing::X_BYTES))) : "memory");
+                        tc_tma_pair(ring + s * STAGE + (is_w ? 0u : (uint32_t)TcPairRing::W_BYTES), is_w ? &wmap : &xmap, a.slabs ? 0 : k * KS, row, a.slabs ? k : 0, z, tc_leader(full + 8u * s));
+                    } else if (warp == TC_LOAD_W) tc_load<TN, GLU, true>(ring + s * STAGE, &wmap, a, t, k * KS, full + 8u * s);
                     else tc_load<TN, GLU, false>(ring + s * STAGE, &xmap, a, t, k * KS, full + 8u * s);
                 }
                 __syncwarp();
                 if (++s == NS) { s = 0; ph ^= 1u; }
             }
-        if (!alive) tc_drain<NS>(full, s, ph);
+        if (!alive && rank == 0) tc_drain<NS>(full, s, ph);
     } else if (warp == TC_MMA) {
-        const uint32_t idesc = tc_idesc(TC_M, TN);
+        const uint32_t idesc = tc_idesc(PAIR ? 2 * TC_M : TC_M, TN);
         uint32_t s = 0, ph = 0, it = 0;
-        for (int item = blockIdx.x; walk.find(a, n_mt, item, t); item += gridDim.x, it++) {
+        if (!PAIR || rank == 0)
+        for (int item = first; find(item); item += stride, it++) {
             const uint32_t buf = it & 1u;
             tc_wait(acc_empty + 8u * buf, ((it >> 1) & 1u) ^ 1u, alive, a.err, 2);
+            if (PAIR) asm volatile("fence.acq_rel.cluster;" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int k = 0; k < steps; k++) {
                 tc_wait(full + 8u * s, ph, alive, a.err, 3);
                 alive = __all_sync(0xffffffffu, alive);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (tc_elect()) {
-                    if (alive) tc_mma_stage<TN>(tmem + buf * TN, ring + s * STAGE, idesc, k == 0);
-                    tc_commit(empty + 8u * s);
-                    if (k == steps - 1) tc_commit(acc_full + 8u * buf);
+                    if constexpr (PAIR) {
+                        if (alive) {
+                            const uint64_t da = tc_desc(ring + s * STAGE), db = tc_desc(ring + s * STAGE + TcPairRing::W_BYTES);
+#pragma unroll
+                            for (int kk = 0; kk < TC_K / 16; kk++) {
+                                const uint32_t accum = (k > 0 || kk > 0) ? 1u : 0u;
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + buf * TN),
+                                    "l"(da + (uint64_t)(2 * kk)), "l"(db + (uint64_t)(2 * kk)), "r"(idesc), "r"(accum)
+                                    : "memory");
+                            }
+                        }
+                        tc_commit_pair(empty + 8u * s);
+                        if (k == steps - 1) tc_commit_pair(acc_full + 8u * buf);
+                    } else {
+                        if (alive) tc_mma_stage<TN>(tmem + buf * TN, ring + s * STAGE, idesc, k == 0);
+                        tc_commit(empty + 8u * s);
+                        if (k == steps - 1) tc_commit(acc_full + 8u * buf);
+                    }
                 }
                 __syncwarp();
                 if (++s == NS) { s = 0; ph ^= 1u; }
@@ -254,7 +330,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         // warps w and w + 4 read TMEM lanes 32 (w & 3) .. + 31 (= weight rows), every second batch of 32 tokens each
         const int half = warp >> 2, row = tid & (TC_M - 1);
         uint32_t it = 0;
-        for (int item = blockIdx.x; walk.find(a, n_mt, item, t); item += gridDim.x, it++) {
+        for (int item = first; find(item); item += stride, it++) {
             const uint32_t buf = it & 1u, acc = tmem + buf * TN + ((uint32_t)((warp & 3) * 32) << 16);
             const int n0 = t.m * (GLU ? TC_M / 2 : TC_M), n = n0 + row, rows = t.rows - t.t0;        // rows: tokens of the tile that exist
             void* Yt = seg_rows<tc_t, EPI>(a.Y, (size_t)(t.row0 + t.t0) * a.ldy + (a.seg ? 0 : t.z * a.yz));
@@ -326,13 +402,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) tc_arrive(acc_empty + 8u * buf);
+            if (lane == 0) {
+                if (PAIR) tc_arrive_leader(acc_empty + 8u * buf);
+                else tc_arrive(acc_empty + 8u * buf);
+            }
         }
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == TC_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
+    if (PAIR) {                                             // nobody leaves while the other's copies, commits or arrivals may still come here
+        tc_cluster_sync();
+        if (warp == TC_MMA) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
+    } else if (warp == TC_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
 }
 
 __device__ __forceinline__ float tc_peer_f32(uint32_t addr, uint32_t rank) {
@@ -654,34 +736,42 @@ bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts,
 
 // Which kernel a product of R rows (of every group; xrows in all groups together when the rows come from `seg`) takes: the least clocks by
 // what each one measured, of a step of 64 elements per CTA (operand bytes at 64 per clock) and of what a CTA adds when it is not overlapped
-// (filling the ring, epilogue, the exchange of a split), on 148 SMs.  Clusters of 8 do not tile the chip's SM groups: 128 of
+// (filling the ring, epilogue, the exchange of a split), on 148 SMs (74 pairs: a step of 801 clocks where the single CTA's took 875, gate and up of an 8B layer; starting and
+// ending together 3000: 1500 rows x 2568 x 1024 lost 2 % of a prompt to pairs that the steps alone spoke for).  Clusters of 8 do not tile the chip's SM groups: 128 of
 // their CTAs already took two waves (12.4 us where 64 CTAs in clusters of 4 took 8.3: 32 x 2048 x 2048).
 // split: K may be cut over a cluster.  Without, every sum adds its products in the order of K, so that a row's result is the same bits whatever the number of
 // rows of the step.
 // rows: token rows as M (lp_gemm_tc_rows_kernel), tn weight rows per CTA: for sums that may not be cut (a cut over a cluster is as fast), up to 128 rows
+// pair: two CTAs per tile (lp_gemm_tc_kernel)
 struct TcPlan {
     bool persistent;
     int tn, splits;
-    bool rows;
+    bool rows, pair;
 };
-TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, bool split, bool tc_rows_able = false) {
+TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, bool split, bool tc_rows_able = false, int pairs = 1) {
     const int n_sm = 148, steps = (K + TC_K - 1) / TC_K, per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per;
     auto tiles = [&](int tn) { return (long long)n_mt * (seg ? xrows / tn + (groups + 1) / 2 : groups * ((R + tn - 1) / tn)); };
-    TcPlan best{true, 256, 1, false};
+    TcPlan best{true, 256, 1, false, false};
     long long least = -1;
     auto offer = [&](bool persistent, int tn, int s, long long cost) {
-        if (least < 0 || cost < least) { least = cost; best = TcPlan{persistent, tn, s, false}; }
+        if (least < 0 || cost < least) { least = cost; best = TcPlan{persistent, tn, s, false, false}; }
     };
     if (tc_rows_able && !split && !seg && !glu && groups == 1 && R <= 128)
         for (int nt : {16, 32}) {
             const long long waves = ((N + nt - 1) / nt + n_sm - 1) / n_sm, step = std::max(2 * (((R + 7) & ~7) + nt), R <= 64 ? 64 + nt : 128 + nt);
             const long long cost = waves * (steps * step + 4500) - 4500 + 18 * 64;
-            if (least < 0 || cost < least) { least = cost; best = TcPlan{false, nt, 1, true}; }
+            if (least < 0 || cost < least) { least = cost; best = TcPlan{false, nt, 1, true, false}; }
         }
     for (int tn : {256, 128}) {
         if (tn == 256 && R <= 128) continue;
         const long long waves = (tiles(tn) + n_sm - 1) / n_sm;
         offer(true, tn, 1, waves * steps * (tn == 256 ? 750 : 470) + 17 * tn);
+    }
+    if (pairs && R > 128) {
+        const long long two = (long long)((n_mt + 1) / 2) * (seg ? xrows / 256 + (groups + 1) / 2 : groups * ((R + 255) / 256)), waves = (two + n_sm / 2 - 1) / (n_sm / 2);
+        const long long cost = waves * steps * 680 + 17 * 256 + 3000;
+        if (cost < least || pairs == 2) { least = cost; best = TcPlan{true, 256, 1, false, true}; }
+        if (pairs == 2) return best;
     }
     for (int tn : {128, 64}) {
         if (tn == 128 && R <= 64) continue;

@@ -1641,6 +1641,7 @@ struct LpModel {
     // close then takes the other one -- a different row, not a rounding of it.  32 sequences through two layers of width 2048, a step's products of 32 rows 10.2 -> 14.9 us,
     // prompts of 48 tokens 26 -> 44 us of attention per layer.
     bool any_order = true;
+    int tc_pair = 1;                        // B200_TC_PAIR=0: no pairs of CTAs in the products, 2: for all of more than 128 rows
     bool tc_rows = true;                    // B200_LP_TC_ROWS=0: no tiles of token rows as M
     bool tc_maps = true;                    // B200_LP_TC_MAPS=0: as if the driver refused the tensor maps of the products
     size_t keys16_most = (size_t)1 << 30;   // B200_LP_KEYS16_MB: a layer that needs more takes the mma.sync kernels (0: always)
@@ -1827,10 +1828,10 @@ void launch(LpModel* m, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sm
 }
 
 // One launch of a tensor-core product: the tensor maps are made for the call (about a microsecond of host time each) and travel with it.
-template <int TN, bool PERSISTENT, int EPI>
+template <int TN, bool PERSISTENT, int EPI, bool PAIR>
 bool tc_launch_as(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid) {
     constexpr size_t smem = tc_smem_bytes<TN, PERSISTENT>(epi_is_glu(EPI));
-    auto kern = PERSISTENT ? lp_gemm_tc_kernel<TN, EPI> : lp_gemm_tc_split_kernel<(TN > 128 ? 128 : TN), EPI>;
+    auto kern = PERSISTENT ? lp_gemm_tc_kernel<TN, EPI, PAIR> : lp_gemm_tc_split_kernel<(TN > 128 ? 128 : TN), EPI>;
     static bool once[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1841,19 +1842,19 @@ bool tc_launch_as(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, cons
         }
         if (dev >= 0 && dev < 64) once[dev] = true;
     }
-    launch_cluster(m, kern, grid, dim3(TC_THREADS), smem, PERSISTENT ? 1 : a.splits, xm, wm, a);
+    launch_cluster(m, kern, grid, dim3(TC_THREADS), smem, PAIR ? 2 : PERSISTENT ? 1 : a.splits, xm, wm, a);
     return true;
 }
-template <int TN, bool PERSISTENT>
+template <int TN, bool PERSISTENT, bool PAIR = false>
 bool tc_launch(LpModel* m, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid, int epi) {
     switch (epi) {
-        case EPI_STORE: return tc_launch_as<TN, PERSISTENT, EPI_STORE>(m, xm, wm, a, grid);
-        case EPI_ADD: return tc_launch_as<TN, PERSISTENT, EPI_ADD>(m, xm, wm, a, grid);
-        case EPI_GELU: return tc_launch_as<TN, PERSISTENT, EPI_GELU>(m, xm, wm, a, grid);
-        case EPI_XIELU: return tc_launch_as<TN, PERSISTENT, EPI_XIELU>(m, xm, wm, a, grid);
-        case EPI_RELU_GLU: return tc_launch_as<TN, PERSISTENT, EPI_RELU_GLU>(m, xm, wm, a, grid);
-        case EPI_SILU_GLU: return tc_launch_as<TN, PERSISTENT, EPI_SILU_GLU>(m, xm, wm, a, grid);
-        default: return tc_launch_as<TN, PERSISTENT, EPI_RELU2>(m, xm, wm, a, grid);
+        case EPI_STORE: return tc_launch_as<TN, PERSISTENT, EPI_STORE, PAIR>(m, xm, wm, a, grid);
+        case EPI_ADD: return tc_launch_as<TN, PERSISTENT, EPI_ADD, PAIR>(m, xm, wm, a, grid);
+        case EPI_GELU: return tc_launch_as<TN, PERSISTENT, EPI_GELU, PAIR>(m, xm, wm, a, grid);
+        case EPI_XIELU: return tc_launch_as<TN, PERSISTENT, EPI_XIELU, PAIR>(m, xm, wm, a, grid);
+        case EPI_RELU_GLU: return tc_launch_as<TN, PERSISTENT, EPI_RELU_GLU, PAIR>(m, xm, wm, a, grid);
+        case EPI_SILU_GLU: return tc_launch_as<TN, PERSISTENT, EPI_SILU_GLU, PAIR>(m, xm, wm, a, grid);
+        default: return tc_launch_as<TN, PERSISTENT, EPI_RELU2, PAIR>(m, xm, wm, a, grid);
     }
 }
 template <int MR, int NT, int EPI>
@@ -1896,10 +1897,10 @@ struct TcProduct {
 bool tc_prepare(const LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, int R, bool glu, bool seg, int xrows, int groups, size_t wz, ZStride zs, TcProduct& t) {
     if (!tc_takes(m, X, ldx, W, ldw, K, R, wz, zs) || !m->tc_maps) return false;
     const bool x_z = !seg && groups > 1 && zs.x > 0;
-    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->any_order, m->tc_rows);
+    t.pl = tc_plan(R, N, K, groups, xrows, seg, glu, m->any_order, m->tc_rows, m->tc_pair);
     if (t.pl.rows) return tc_map(&t.xm, X, K, R, ldx, 1, 1, 0, (R + 7) & ~7, TR_KH) && tc_map(&t.wm, W, K, N, ldw, 1, 1, 0, t.pl.tn, TR_KH);
     const int kh = t.pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
-    return tc_map(&t.xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, t.pl.tn, kh) &&
+    return tc_map(&t.xm, X, K, seg ? xrows : R, ldx, 1, x_z ? groups : 1, zs.x, t.pl.pair ? 128 : t.pl.tn, kh) &&
            tc_map(&t.wm, W, K, N, ldw, glu ? 2 : 1, groups, wz, glu ? TC_M / 2 : TC_M, kh);
 }
 bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, int K, void* Y, int ldy, int R, float alpha, int epi, const int* seg,
@@ -1915,6 +1916,10 @@ bool tc_gemm(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, 
         return pl.tn == 16 ? tc_rows_launch<128, 16>(m, xm, wm, a, epi) : tc_rows_launch<128, 32>(m, xm, wm, a, epi);
     }
     const int per = glu ? TC_M / 2 : TC_M, n_mt = (N + per - 1) / per, n_nt = (R + pl.tn - 1) / pl.tn;
+    if (pl.pair) {
+        const int two = (n_mt + 1) / 2, most = seg ? two * (xrows / 256 + groups) : two * n_nt * groups;
+        return tc_launch<256, true, true>(m, xm, wm, a, dim3(2 * std::min(most, 74)), epi);
+    }
     if (pl.persistent) {
         const int most = seg ? n_mt * (xrows / pl.tn + groups) : n_mt * n_nt * groups;
         const dim3 grid(std::min(most, 148));
@@ -2253,6 +2258,8 @@ int lp_create(const b200_program_desc* prog, const b200_layer_desc* layers, int 
         if (e && *e) m->use_attn_tile = atoi(e) != 0;
         e = getenv("B200_LP_TC_MAPS");
         if (e && *e) m->tc_maps = atoi(e) != 0;
+        e = getenv("B200_TC_PAIR");
+        if (e && *e) m->tc_pair = atoi(e);
         e = getenv("B200_LP_TC_ROWS");
         if (e && *e) m->tc_rows = atoi(e) != 0;
         e = getenv("B200_LP_KEYS16_MB");

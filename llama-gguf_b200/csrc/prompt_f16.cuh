@@ -140,10 +140,10 @@ template <typename T, int EPI> __device__ __forceinline__ void* seg_rows(void* Y
 }
 #include "gemm_tc.cuh"
 
-template <int TN, bool PERSISTENT, int EPI>
+template <int TN, bool PERSISTENT, int EPI, bool PAIR = false>
 cudaError_t launch_as(const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, dim3 grid, bool pdl, cudaStream_t st) {
     constexpr size_t smem = tc_smem_bytes<TN, PERSISTENT>(epi_is_glu(EPI));
-    auto kern = PERSISTENT ? lp_gemm_tc_kernel<TN, EPI> : lp_gemm_tc_split_kernel<(TN > 128 ? 128 : TN), EPI>;
+    auto kern = PERSISTENT ? lp_gemm_tc_kernel<TN, EPI, PAIR> : lp_gemm_tc_split_kernel<(TN > 128 ? 128 : TN), EPI>;
     static bool once[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -163,9 +163,9 @@ cudaError_t launch_as(const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs
         at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[n++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (!PERSISTENT && a.splits > 1) {
+    if (PAIR || (!PERSISTENT && a.splits > 1)) {
         at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = (unsigned)a.splits;
+        at[n].val.clusterDim.x = PAIR ? 2u : (unsigned)a.splits;
         at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
         n++;
     }
@@ -175,6 +175,10 @@ cudaError_t launch_as(const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs
 }
 template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& xm, const CUtensorMap& wm, const TcArgs& a, bool pdl, cudaStream_t st) {
     const int per = epi_is_glu(EPI) ? TC_M / 2 : TC_M, n_mt = (a.N + per - 1) / per, n_nt = (a.R + pl.tn - 1) / pl.tn;
+    if (pl.pair) {
+        const int two = (n_mt + 1) / 2 * n_nt;
+        return launch_as<256, true, EPI, true>(xm, wm, a, dim3(2 * (two < 74 ? two : 74)), pdl, st);
+    }
     if (pl.persistent) {
         const dim3 grid(n_mt * n_nt < 148 ? n_mt * n_nt : 148);
         return pl.tn == 256 ? launch_as<256, true, EPI>(xm, wm, a, grid, pdl, st) : launch_as<128, true, EPI>(xm, wm, a, grid, pdl, st);
@@ -186,10 +190,12 @@ template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& x
 // cudaErrorNotSupported: a tensor map was refused, nothing was launched
 inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, bool pdl, cudaStream_t st) {
     const bool glu = epi_is_glu(epi);
-    const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu, true);
+    const char* pe = getenv("B200_TC_PAIR");
+    const int pairs = pe && *pe ? atoi(pe) : 1;      // B200_TC_PAIR=0: no pairs of CTAs, 2: pairs for all products of more than 128 rows
+    const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu, true, false, pairs);
     const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     CUtensorMap xm, wm;
-    if (!tc_map(&xm, x, K, T, ldx, 1, 1, 0, pl.tn, kh) || !tc_map(&wm, w, K, N, K, glu ? 2 : 1, 1, 0, glu ? TC_M / 2 : TC_M, kh)) return cudaErrorNotSupported;
+    if (!tc_map(&xm, x, K, T, ldx, 1, 1, 0, pl.pair ? 128 : pl.tn, kh) || !tc_map(&wm, w, K, N, K, glu ? 2 : 1, 1, 0, glu ? TC_M / 2 : TC_M, kh)) return cudaErrorNotSupported;
     const TcArgs a{y, ldy, T, N, K, 1.0f, err, nullptr, 1, 0, 0, bias, float2{0.0f, 0.0f}, pl.splits, K % TC_K == 0 ? 1 : 0};
     return epi == EPI_STORE ? launch_epi<EPI_STORE>(pl, xm, wm, a, pdl, st) : epi == EPI_ADD ? launch_epi<EPI_ADD>(pl, xm, wm, a, pdl, st) : launch_epi<EPI_SILU_GLU>(pl, xm, wm, a, pdl, st);
 }
