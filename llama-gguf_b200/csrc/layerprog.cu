@@ -107,9 +107,10 @@ __global__ void lp_embed_kernel(StepMeta sm, const T* __restrict__ table, const 
 // out[b] = x[src] / sqrt(mean(x[src]^2) + eps) * w, src = gather ? gather[b] : b.  add != null: x[src] += add first (stored back):
 // the per-pass step vector of a repeated layer range.  center = 1: the layer norm, (x - mean) / sqrt(mean((x - mean)^2) + eps) * w
 // (the mean in a pass of its own).  One block per row.
-template <typename OutT>
+template <typename OutT, bool CENTER>
 __global__ void lp_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ add, const float* __restrict__ w, OutT* __restrict__ out,
-                                  const int* __restrict__ gather, int width, float eps, int center) {
+                                  const int* __restrict__ gather, int width, float eps) {
+    constexpr bool center = CENTER;
     prev_grid();
     const int b = blockIdx.x;
     const int r = gather ? gather[b] : b;
@@ -2044,8 +2045,9 @@ void gemm_ld(LpModel* m, const void* X, int ldx, const void* Wm, int ldw, int N,
 int norm_center(const LpModel* m) { return m->p.norm_kind == B200_NORM_LAYER ? 1 : 0; }
 
 void rmsnorm(LpModel* m, float* x, const float* add, const float* w, void* out, const int* gather, int rows) {
-    if (m->f32) launch(m, lp_rmsnorm_kernel<float>, dim3(rows), dim3(128), 0, x, add, w, (float*)out, gather, m->p.width, m->p.norm_eps, norm_center(m));
-    else launch(m, lp_rmsnorm_kernel<bf16>, dim3(rows), dim3(128), 0, x, add, w, (bf16*)out, gather, m->p.width, m->p.norm_eps, norm_center(m));
+    const bool ln = norm_center(m);
+    if (m->f32) launch(m, ln ? lp_rmsnorm_kernel<float, true> : lp_rmsnorm_kernel<float, false>, dim3(rows), dim3(128), 0, x, add, w, (float*)out, gather, m->p.width, m->p.norm_eps);
+    else launch(m, ln ? lp_rmsnorm_kernel<bf16, true> : lp_rmsnorm_kernel<bf16, false>, dim3(rows), dim3(128), 0, x, add, w, (bf16*)out, gather, m->p.width, m->p.norm_eps);
 }
 
 // norm + projection of the step's rows: one fused kernel for a few rows (decoding) when the normed rows fit in shared memory,
