@@ -54,22 +54,52 @@ __global__ void __launch_bounds__(256) prefill_kv16_kernel(const float* __restri
     const int kh = blockIdx.y, n_kv = gridDim.y, p0 = blockIdx.x * 64;
     const float* ks = kc + (size_t)kh * max_seq * HD;
     const float* vs = vc + (size_t)kh * max_seq * HD;
-    for (int i = threadIdx.x; i < 64 * HD; i += 256) {
-        const int pr = i / HD, d = i - pr * HD, pos = p0 + pr;
-        const bool ok = pos < kv_end;
-        const float k = ok ? fminf(fmaxf(ks[(size_t)pos * HD + d], -65504.0f), 65504.0f) : 0.0f;
-        const float v = ok ? fminf(fmaxf(vs[(size_t)pos * HD + d], -65504.0f), 65504.0f) : 0.0f;
-        const __half khi = __float2half_rn(k), vhi = __float2half_rn(v);
-        k16[((size_t)kh * P + pos) * HD + d] = khi;
-        k16[((size_t)(n_kv + kh) * P + pos) * HD + d] = __float2half_rn(k - __half2float(khi));
-        tile[pr][d] = vhi;
-        tile_lo[pr][d] = __float2half_rn(v - __half2float(vhi));
+    auto half4 = [](float4 f, uint2& hi, uint2& lo) {
+        const float v[4] = {fminf(fmaxf(f.x, -65504.0f), 65504.0f), fminf(fmaxf(f.y, -65504.0f), 65504.0f), fminf(fmaxf(f.z, -65504.0f), 65504.0f), fminf(fmaxf(f.w, -65504.0f), 65504.0f)};
+        const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
+        const float2 af = __half22float2(a), bf = __half22float2(b);
+        const __half2 c = __floats2half2_rn(v[0] - af.x, v[1] - af.y), d = __floats2half2_rn(v[2] - bf.x, v[3] - bf.y);
+        hi = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        lo = make_uint2(*reinterpret_cast<const uint32_t*>(&c), *reinterpret_cast<const uint32_t*>(&d));
+    };
+    // four channels per thread in (NB times, all loads first), eight positions of a channel out (2048 positions of 8 heads: 20 -> 9 us against one by one)
+    constexpr int NB = HD / 32;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        float4 k[NB], v[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int i = 4 * (threadIdx.x + 256 * (h * NB + u)), pr = i / HD, d = i - pr * HD, pos = p0 + pr;
+            const bool ok = pos < kv_end;
+            k[u] = ok ? *reinterpret_cast<const float4*>(ks + (size_t)pos * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = ok ? *reinterpret_cast<const float4*>(vs + (size_t)pos * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int i = 4 * (threadIdx.x + 256 * (h * NB + u)), pr = i / HD, d = i - pr * HD, pos = p0 + pr;
+            uint2 hi, lo;
+            half4(k[u], hi, lo);
+            *reinterpret_cast<uint2*>(k16 + ((size_t)kh * P + pos) * HD + d) = hi;
+            *reinterpret_cast<uint2*>(k16 + ((size_t)(n_kv + kh) * P + pos) * HD + d) = lo;
+            half4(v[u], hi, lo);
+            *reinterpret_cast<uint32_t*>(&tile[pr][d]) = hi.x;
+            *reinterpret_cast<uint32_t*>(&tile[pr][d + 2]) = hi.y;
+            *reinterpret_cast<uint32_t*>(&tile_lo[pr][d]) = lo.x;
+            *reinterpret_cast<uint32_t*>(&tile_lo[pr][d + 2]) = lo.y;
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 64 * HD; i += 256) {
-        const int d = i >> 6, pr = i & 63;
-        vt16[((size_t)kh * HD + d) * P + p0 + pr] = tile[pr][d];
-        vt16[((size_t)(n_kv + kh) * HD + d) * P + p0 + pr] = tile_lo[pr][d];
+    for (int i = threadIdx.x; i < 8 * HD; i += 256) {      // eight lanes: the 64 positions of a channel
+        const int d = i >> 3, pr = 8 * (i & 7);
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const __half2 x = __halves2half2(tile[pr + 2 * u][d], tile[pr + 2 * u + 1][d]), y = __halves2half2(tile_lo[pr + 2 * u][d], tile_lo[pr + 2 * u + 1][d]);
+            a[u] = *reinterpret_cast<const uint32_t*>(&x);
+            b[u] = *reinterpret_cast<const uint32_t*>(&y);
+        }
+        *reinterpret_cast<uint4*>(vt16 + ((size_t)kh * HD + d) * P + p0 + pr) = make_uint4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<uint4*>(vt16 + ((size_t)(n_kv + kh) * HD + d) * P + p0 + pr) = make_uint4(b[0], b[1], b[2], b[3]);
     }
 }
 

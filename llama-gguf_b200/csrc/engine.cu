@@ -2528,7 +2528,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             f16 = f16_able && c->pf_w16 && T >= f16_min(L);
             float* kc = sl.kv + (size_t)l * kv_layer;
             float* vc = kc + kv_layer / 2;
-            CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.attn_norm.f32(), d.norm_eps, XNh, H));
+            CU(launch_on(st, pdl, prefill_rms_norm_for(H), dim3(T), dim3(256), 0, (const float*)X, L.attn_norm.f32(), d.norm_eps, XNh, H));
             cudaError_t e16 = f16 && !(L.bq.present() || L.bk.present() || L.bv.present()) ? gemm16({&L.wq, &L.wk, &L.wv}, H, XNh, H, T, Q, QKV, nullptr, tc16::EPI_STORE) : cudaErrorNotSupported;
             if (e16 == cudaErrorNotSupported) {
                 CU(product(L.wq, H, XNh, H, T, Q, QKV, &L.bq, 0));
@@ -2584,7 +2584,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 }
             }
             CU(product(L.wo, A, ATh, A, T, X, H, nullptr, 1));                    // X += Wo attn
-            CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(T), dim3(256), 0, (const float*)X, L.ffn_norm.f32(), d.norm_eps, XNh, H));
+            CU(launch_on(st, pdl, prefill_rms_norm_for(H), dim3(T), dim3(256), 0, (const float*)X, L.ffn_norm.f32(), d.norm_eps, XNh, H));
             e16 = f16 ? gemm16({&L.gate, &L.up}, H, XNh, H, T, Hh, I, nullptr, tc16::EPI_SILU_GLU) : cudaErrorNotSupported;
             if (e16 == cudaErrorNotSupported) {
                 CU(product(L.gate, H, XNh, H, T, G, I, nullptr, 0));
@@ -2607,7 +2607,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             p.n_seg = 1; p.K = H; p.T = n; p.x = X; p.ldx = H; p.norm_w = c->output_norm.f32(); p.eps = d.norm_eps; p.epi = EPI_STORE;
             CU(rows_few_launch(p, c->n_sm, pdl, st));
         } else if (!head_done) {
-            CU(launch_on(st, pdl, prefill_rms_norm_kernel, dim3(n), dim3(256), 0, (const float*)X, c->output_norm.f32(), d.norm_eps, XNh, H));
+            CU(launch_on(st, pdl, prefill_rms_norm_for(H), dim3(n), dim3(256), 0, (const float*)X, c->output_norm.f32(), d.norm_eps, XNh, H));
             UmmaParams hp{};
             hp.w = head.d; hp.row_bytes = head.row_bytes; hp.type = head.type; hp.n_rows = d.vocab; hp.K = H;
             hp.x = XNh; hp.ldx = H; hp.T = n; hp.y = c->pf_logits; hp.ldy = d.vocab; hp.err = c->mma_err; hp.pdl = pdl ? 1 : 0;

@@ -63,42 +63,53 @@ __global__ void prefill_rope_kv_kernel(const PrefillRopeParams p) {
     const int n_pairs = (p.n_heads + p.n_kv) * half, n_v = p.n_kv * p.hd;
     const float position = (float)pos / p.rope_scale;
     float* row = p.qkv + (size_t)t * p.ld;
-    const float* kraw = row + (size_t)p.n_heads * p.hd;
-    const float* vraw = kraw + (size_t)p.n_kv * p.hd;
+    const float* vraw = row + (size_t)(p.n_heads + p.n_kv) * p.hd;
     // a token's hd / 2 angles once per CTA (every head turns by the same ones; four 2048-wide layers, 333 tokens: 806 -> 798 us)
-    __shared__ float cs_s[64], sn_s[64];
-    const bool once = half <= 64;
-    if (once && (int)threadIdx.x < half) {
+    __shared__ __align__(16) float cs_s[64], sn_s[64];      // (hd is 64 or 128)
+    if ((int)threadIdx.x < half) {
         const float theta = position * p.freq[threadIdx.x];
         cs_s[threadIdx.x] = cosf(theta);
         sn_s[threadIdx.x] = sinf(theta);
     }
     __syncthreads();
-    // gridDim.y CTAs share a token's items (each item is independent: same arithmetic whoever computes it)
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n_pairs + n_v; i += blockDim.x * gridDim.y) {
-        if (i < n_pairs) {
-            const int head = i / half, pi = i - head * half;
-            const float theta = once ? 0.0f : position * p.freq[pi];
-            const float c = once ? cs_s[pi] : cosf(theta), s = once ? sn_s[pi] : sinf(theta);
-            const int i0 = p.neox ? pi : 2 * pi, i1 = p.neox ? pi + half : 2 * pi + 1;
-            if (head < p.n_heads) {
-                float* d = row + (size_t)head * p.hd;
-                const float x0 = d[i0], x1 = d[i1];
-                d[i0] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-                d[i1] = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
-            } else {
-                const int kh = head - p.n_heads;
-                const float* d = kraw + (size_t)kh * p.hd;
-                float* o = k_cache + ((size_t)kh * p.max_seq + pos) * p.hd;
-                const float x0 = d[i0], x1 = d[i1];
-                o[i0] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-                o[i1] = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
-            }
-        } else {
-            const int j = i - n_pairs;
-            const int kh = j / p.hd, d = j - kh * p.hd;
-            v_cache[((size_t)kh * p.max_seq + pos) * p.hd + d] = vraw[j];
+    // gridDim.y CTAs share a token's items (each item is independent: same arithmetic whoever computes it): four pairs by two 16-byte loads, three items' loads before the
+    // first store.  A pair per thread and iteration was bound by its index arithmetic and by loads that waited
+    // for stores (2048 tokens of an 8B layer: 28 -> 18 us, 83 MB).
+    const int stride = blockDim.x * gridDim.y, at0 = blockIdx.y * blockDim.x + threadIdx.x, sh = half == 64 ? 4 : 3, n_items = n_pairs >> 2;
+    constexpr int NB = 3;
+    for (int b0 = at0; b0 < n_items; b0 += NB * stride) {
+        float4 a[NB], b[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int i = b0 + u * stride;
+            if (i >= n_items) continue;
+            const int head = i >> sh, pi = (i & ((1 << sh) - 1)) * 4;
+            const float* d = row + (size_t)head * p.hd;      // (k heads follow q heads)
+            a[u] = *reinterpret_cast<const float4*>(d + (p.neox ? pi : 2 * pi));
+            b[u] = *reinterpret_cast<const float4*>(d + (p.neox ? pi + half : 2 * pi + 4));
         }
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int i = b0 + u * stride;
+            if (i >= n_items) continue;
+            const int head = i >> sh, pi = (i & ((1 << sh) - 1)) * 4;
+            const float4 c = *reinterpret_cast<const float4*>(cs_s + pi), s = *reinterpret_cast<const float4*>(sn_s + pi);
+            float* o = head < p.n_heads ? row + (size_t)head * p.hd : k_cache + ((size_t)(head - p.n_heads) * p.max_seq + pos) * p.hd;
+            auto lo = [](float x0, float x1, float cc, float ss) { return __fsub_rn(__fmul_rn(x0, cc), __fmul_rn(x1, ss)); };
+            auto hi = [](float x0, float x1, float cc, float ss) { return __fadd_rn(__fmul_rn(x0, ss), __fmul_rn(x1, cc)); };
+            const float4 x = a[u], y = b[u];
+            if (p.neox) {
+                *reinterpret_cast<float4*>(o + pi) = make_float4(lo(x.x, y.x, c.x, s.x), lo(x.y, y.y, c.y, s.y), lo(x.z, y.z, c.z, s.z), lo(x.w, y.w, c.w, s.w));
+                *reinterpret_cast<float4*>(o + pi + half) = make_float4(hi(x.x, y.x, c.x, s.x), hi(x.y, y.y, c.y, s.y), hi(x.z, y.z, c.z, s.z), hi(x.w, y.w, c.w, s.w));
+            } else {
+                *reinterpret_cast<float4*>(o + 2 * pi) = make_float4(lo(x.x, x.y, c.x, s.x), hi(x.x, x.y, c.x, s.x), lo(x.z, x.w, c.y, s.y), hi(x.z, x.w, c.y, s.y));
+                *reinterpret_cast<float4*>(o + 2 * pi + 4) = make_float4(lo(y.x, y.y, c.z, s.z), hi(y.x, y.y, c.z, s.z), lo(y.z, y.w, c.w, s.w), hi(y.z, y.w, c.w, s.w));
+            }
+        }
+    }
+    for (int i = at0; i < n_v / 4; i += stride) {      // (hd is a multiple of 4)
+        const int j = 4 * i, kh = j / p.hd, d = j - kh * p.hd;
+        *reinterpret_cast<float4*>(v_cache + ((size_t)kh * p.max_seq + pos) * p.hd + d) = *reinterpret_cast<const float4*>(vraw + j);
     }
 }
 
@@ -226,7 +237,9 @@ __global__ void __launch_bounds__(128) prefill_attn_kernel(const PrefillAttnPara
 // rms_norm_rows_kernel: ss = sum x^2, inv = 1/sqrt(ss/n + eps), (x*inv)*w; simd.rs:847-899)
 // Rows of up to 256 * kRmsMaxV elements are held in registers: all loads of a thread are issued before the first is used (a row is
 // 16 dependent-latency trips otherwise: 15 us per launch at 32 rows), the sums run in the SAME order as before (bit-identical).
+// NV4 > 0: rows of up to 1024 NV4 elements (a multiple of 4, as the buffers' rows are aligned) by float4 (2048 rows of 4096: 17 -> 10 us; few registers, many blocks).
 constexpr int kRmsMaxV = 32;
+template <int NV4>
 __global__ void __launch_bounds__(256) prefill_rms_norm_kernel(const float* x, const float* w, float eps, __half* out, int n) {
     pdl_launch_dependents();
     pdl_wait();
@@ -235,6 +248,32 @@ __global__ void __launch_bounds__(256) prefill_rms_norm_kernel(const float* x, c
     __half* orow = out + (size_t)blockIdx.x * n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float ss = 0.0f;
+    if (NV4 > 0) {
+        float4 v[NV4 > 0 ? NV4 : 1], wv[NV4 > 0 ? NV4 : 1];
+#pragma unroll
+        for (int k = 0; k < NV4; k++) {
+            const int i = 4 * (threadIdx.x + 256 * k);
+            v[k] = i < n ? *reinterpret_cast<const float4*>(xr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            wv[k] = i < n ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < NV4; k++) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+        ss = warp_sum(ss);
+        if (lane == 0) red[warp] = ss;
+        __syncthreads();
+        float tot = 0.0f;
+        for (int k = 0; k < 8; k++) tot += red[k];
+        const float inv = 1.0f / sqrtf(tot / (float)n + eps);
+#pragma unroll
+        for (int k = 0; k < NV4; k++) {
+            const int i = 4 * (threadIdx.x + 256 * k);
+            if (i >= n) continue;
+            const __half2 a = __halves2half2(f2h_sat(__fmul_rn(__fmul_rn(v[k].x, inv), wv[k].x)), f2h_sat(__fmul_rn(__fmul_rn(v[k].y, inv), wv[k].y)));
+            const __half2 b = __halves2half2(f2h_sat(__fmul_rn(__fmul_rn(v[k].z, inv), wv[k].z)), f2h_sat(__fmul_rn(__fmul_rn(v[k].w, inv), wv[k].w)));
+            *reinterpret_cast<uint2*>(orow + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        }
+        return;
+    }
     if (n <= 256 * kRmsMaxV) {
         float v[kRmsMaxV], wv[kRmsMaxV];
 #pragma unroll
@@ -271,6 +310,10 @@ __global__ void __launch_bounds__(256) prefill_rms_norm_kernel(const float* x, c
     for (int k = 0; k < 8; k++) tot += red[k];
     const float inv = 1.0f / sqrtf(tot / (float)n + eps);
     for (int i = threadIdx.x; i < n; i += blockDim.x) orow[i] = f2h_sat(__fmul_rn(__fmul_rn(xr[i], inv), w[i]));
+}
+
+inline void (*prefill_rms_norm_for(int n))(const float*, const float*, float, __half*, int) {
+    return n % 4 || n > 8192 ? prefill_rms_norm_kernel<0> : n <= 1024 ? prefill_rms_norm_kernel<1> : n <= 2048 ? prefill_rms_norm_kernel<2> : n <= 4096 ? prefill_rms_norm_kernel<4> : prefill_rms_norm_kernel<8>;
 }
 
 // g[i] = silu(g[i]) * u[i]  (silu rounded to f32 first, then the product: simd.rs:598-649)
