@@ -89,6 +89,62 @@ __device__ __forceinline__ void softmax_merge_scale(float m, float m2, float& ca
     cb = (m2 == -INFINITY) ? 0.0f : expf(m2 - mo);
 }
 
+// NV sums over the warp's lanes (NV a power of two up to 32), one per lane: lane l gets sum l / (32 / NV).  Halves of what is left go to the lanes that differ in the next bit, in
+// the pairs of a butterfly: its bits, with NV - 1 + log2(32 / NV) shuffles for its 5 NV.
+template <int NV>
+__device__ __forceinline__ float warp_sums(float (&v)[NV]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16, n = NV; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < NV / 2; i++)
+                if (i < n) {
+                    const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+        } else v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+    return v[0];
+}
+
+// Online softmax over the UB positions of a batch and the G <= GMAX heads that share their rows: lane l keeps the maximum m and sum l of head (l / (32 / NV)) % GMAX, NV = UB
+// GMAX, and has the score of that head and position l / (32 / UB) (warp_sums), so an exponential is taken once and not by every lane; weights and factors then go to
+// all lanes, which hold the channels.
+template <int UB, int GMAX, int VEC>
+__device__ __forceinline__ void attn_batch(float (&sv)[UB * GMAX], float scale, bool mine_valid, int G, float& m, float& l, const float (&vr)[UB][VEC], float (&acc)[GMAX][VEC]) {
+    constexpr int NV = UB * GMAX, LPV = 32 / NV;
+    const int lane = threadIdx.x & 31, g = (lane / LPV) % GMAX;
+    float s = warp_sums<NV>(sv) * scale;
+    if (!mine_valid) s = -INFINITY;
+    float mb = s;
+#pragma unroll
+    for (int o = 16; o >= 32 / UB; o >>= 1) mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+    const float mn = fmaxf(m, mb);            // finite: the first position of a batch is always valid
+    const float corr = m == -INFINITY ? 0.0f : expf(m - mn), w = s == -INFINITY || g >= G ? 0.0f : expf(s - mn);
+    float ws = w;
+#pragma unroll
+    for (int o = 16; o >= 32 / UB; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    l = l * corr + ws;
+    m = mn;
+#pragma unroll
+    for (int k = 0; k < GMAX; k++) {
+        const float c = __shfl_sync(0xffffffffu, corr, k * LPV);
+        float wk[UB];
+#pragma unroll
+        for (int u = 0; u < UB; u++) wk[u] = __shfl_sync(0xffffffffu, w, (u * GMAX + k) * LPV);
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+            float a = acc[k][v] * c;
+#pragma unroll
+            for (int u = 0; u < UB; u++) a = fmaf(wk[u], vr[u][v], a);
+            acc[k][v] = a;
+        }
+    }
+}
+
 // Barrier of the NT threads that execute an item: named barrier 1, so that the streamed megakernel (stream.cuh) can
 // run an extra producer warp that never joins (in the stand-alone kernels NT is the whole CTA).
 template <int NT>
@@ -151,11 +207,9 @@ __device__ __forceinline__ void attn_decode_item(const AttnParams& p, int kh, in
     }
     attn_stamp(p, 2);
 
-    float q[GMAX][VEC], acc[GMAX][VEC], m[GMAX], l[GMAX];
+    float q[GMAX][VEC], acc[GMAX][VEC], m = -INFINITY, l = 0.0f;      // (m, l: of this lane's head, attn_batch)
 #pragma unroll
     for (int g = 0; g < GMAX; g++) {
-        m[g] = -INFINITY;
-        l[g] = 0.0f;
 #pragma unroll
         for (int v = 0; v < VEC; v++) {
             acc[g][v] = 0.0f;
@@ -201,7 +255,7 @@ __device__ __forceinline__ void attn_decode_item(const AttnParams& p, int kh, in
         pr_n++;
         if (pr_n == 1) pr_t0 = clock64();
 #endif
-        float s[UB][GMAX];
+        float sv[UB * GMAX];
 #pragma unroll
         for (int u = 0; u < UB; u++)
 #pragma unroll
@@ -209,44 +263,10 @@ __device__ __forceinline__ void attn_decode_item(const AttnParams& p, int kh, in
                 float d = 0.0f;
 #pragma unroll
                 for (int v = 0; v < VEC; v++) d = fmaf(q[g][v], kr[u][v], d);
-                s[u][g] = d;
+                sv[u * GMAX + g] = d;
             }
         ATTN_PROBE(4);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int u = 0; u < UB; u++)
-#pragma unroll
-                for (int g = 0; g < GMAX; g++) s[u][g] += __shfl_xor_sync(0xffffffffu, s[u][g], o);
-        ATTN_PROBE(5);
-#pragma unroll
-        for (int g = 0; g < GMAX; g++) {
-            if (g < G) {
-                float mb = -INFINITY;
-#pragma unroll
-                for (int u = 0; u < UB; u++) {
-                    s[u][g] = (pos0 + u * NW < end) ? s[u][g] * p.scale : -INFINITY;   // warp-uniform
-                    mb = fmaxf(mb, s[u][g]);
-                }
-                const float mn = fmaxf(m[g], mb);   // finite: the first position of a batch is always valid
-                const float corr = (m[g] == -INFINITY) ? 0.0f : expf(m[g] - mn);
-                float w[UB], ws = 0.0f;
-#pragma unroll
-                for (int u = 0; u < UB; u++) {
-                    w[u] = (s[u][g] == -INFINITY) ? 0.0f : expf(s[u][g] - mn);
-                    ws += w[u];
-                }
-                l[g] = l[g] * corr + ws;
-#pragma unroll
-                for (int v = 0; v < VEC; v++) {
-                    float a = acc[g][v] * corr;
-#pragma unroll
-                    for (int u = 0; u < UB; u++) a = fmaf(w[u], vr[u][v], a);
-                    acc[g][v] = a;
-                }
-                m[g] = mn;
-            }
-        }
+        attn_batch<UB, GMAX, VEC>(sv, p.scale, pos0 + lane / (32 / UB) * NW < end, G, m, l, vr, acc);
         ATTN_PROBE(6);
     };
     {
@@ -269,9 +289,9 @@ __device__ __forceinline__ void attn_decode_item(const AttnParams& p, int kh, in
 #pragma unroll
     for (int g = 0; g < GMAX; g++) {
         if (g < G) {
-            if (lane == 0) {
-                s_m[warp * GMAX + g] = m[g];
-                s_l[warp * GMAX + g] = l[g];
+            if (lane == g * (32 / (UB * GMAX))) {
+                s_m[warp * GMAX + g] = m;
+                s_l[warp * GMAX + g] = l;
             }
 #pragma unroll
             for (int v = 0; v < VEC; v++) s_acc[(warp * GMAX + g) * HD + lane * VEC + v] = acc[g][v];

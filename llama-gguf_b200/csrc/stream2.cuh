@@ -749,11 +749,9 @@ __device__ __forceinline__ void attn2_phase(const AttnParams& p, int kv_len, flo
     }
     s2_cons_sync();
 
-    float q[GMAX][VEC], acc[GMAX][VEC], m[GMAX], l[GMAX];
+    float q[GMAX][VEC], acc[GMAX][VEC], m = -INFINITY, l = 0.0f;      // (m, l: of this lane's head, attn_batch)
 #pragma unroll
     for (int gq = 0; gq < GMAX; gq++) {
-        m[gq] = -INFINITY;
-        l[gq] = 0.0f;
 #pragma unroll
         for (int v = 0; v < VEC; v++) {
             acc[gq][v] = 0.0f;
@@ -761,7 +759,7 @@ __device__ __forceinline__ void attn2_phase(const AttnParams& p, int kv_len, flo
         }
     }
     auto compute = [&](int p0, int lim, const float (&kr)[UB][VEC], const float (&vr)[UB][VEC]) {
-        float s[UB][GMAX];
+        float sv[UB * GMAX];
 #pragma unroll
         for (int u = 0; u < UB; u++)
 #pragma unroll
@@ -769,42 +767,9 @@ __device__ __forceinline__ void attn2_phase(const AttnParams& p, int kv_len, flo
                 float d = 0.0f;
 #pragma unroll
                 for (int v = 0; v < VEC; v++) d = fmaf(q[gq][v], kr[u][v], d);
-                s[u][gq] = d;
+                sv[u * GMAX + gq] = d;
             }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int u = 0; u < UB; u++)
-#pragma unroll
-                for (int gq = 0; gq < GMAX; gq++) s[u][gq] += __shfl_xor_sync(0xffffffffu, s[u][gq], o);
-#pragma unroll
-        for (int gq = 0; gq < GMAX; gq++) {
-            if (gq < G) {
-                float mb = -INFINITY;
-#pragma unroll
-                for (int u = 0; u < UB; u++) {
-                    s[u][gq] = (p0 + u * NW < lim) ? s[u][gq] * p.scale : -INFINITY;   // warp-uniform
-                    mb = fmaxf(mb, s[u][gq]);
-                }
-                const float mn = fmaxf(m[gq], mb);   // finite: the first position of a batch is always valid
-                const float corr = (m[gq] == -INFINITY) ? 0.0f : expf(m[gq] - mn);
-                float w[UB], ws = 0.0f;
-#pragma unroll
-                for (int u = 0; u < UB; u++) {
-                    w[u] = (s[u][gq] == -INFINITY) ? 0.0f : expf(s[u][gq] - mn);
-                    ws += w[u];
-                }
-                l[gq] = l[gq] * corr + ws;
-#pragma unroll
-                for (int v = 0; v < VEC; v++) {
-                    float a = acc[gq][v] * corr;
-#pragma unroll
-                    for (int u = 0; u < UB; u++) a = fmaf(w[u], vr[u][v], a);
-                    acc[gq][v] = a;
-                }
-                m[gq] = mn;
-            }
-        }
+        attn_batch<UB, GMAX, VEC>(sv, p.scale, p0 + lane / (32 / UB) * NW < lim, G, m, l, vr, acc);
     };
 #ifdef B200_NO_ATTN_PRE2
     if (pos0 + STEP < end_g) load(pos0 + STEP, kB, vB);
@@ -834,9 +799,9 @@ __device__ __forceinline__ void attn2_phase(const AttnParams& p, int kv_len, flo
 #pragma unroll
     for (int gq = 0; gq < GMAX; gq++) {
         if (gq < G) {
-            if (lane == 0) {
-                s_m[warp * GMAX + gq] = m[gq];
-                s_l[warp * GMAX + gq] = l[gq];
+            if (lane == gq * (32 / (UB * GMAX))) {
+                s_m[warp * GMAX + gq] = m;
+                s_l[warp * GMAX + gq] = l;
             }
 #pragma unroll
             for (int v = 0; v < VEC; v++) s_acc[(warp * GMAX + gq) * HD + lane * VEC + v] = acc[gq][v];
