@@ -836,7 +836,6 @@ __global__ void __launch_bounds__(256) rows_swiglu_kernel(const RowsSum sum, flo
 }
 
 // ---------------------------------------------------------------- host
-// Weight rows per warp of rows_few_kernel: as many as still give every warp a task
 inline int rows_few_tasks(const RowsParams& p, int R) {
     if (p.epi == EPI_SWIGLU) return (p.seg[0].n_rows + R / 2 - 1) / (R / 2);
     int n = 0;
@@ -873,9 +872,13 @@ inline cudaError_t rows_few_go(RowsParams& p, int n_sm, bool pdl, cudaStream_t s
     return cudaLaunchKernelEx(&cfg, rows_few_kernel<R, TT>, p);
 }
 inline cudaError_t rows_few_launch(RowsParams& p, int n_sm, bool pdl, cudaStream_t st) {
-    const int full = 2 * n_sm * kRowsWarps;
+    // rounds of the chip's warps times a round's instructions: R weight columns to unpack and multiply, and the rows' x to load whatever R is.  4096 x 14336 with 3 rows: one
+    // weight row per warp takes two rounds, 40 us, two take one
+    const int full = 2 * n_sm * kRowsWarps, tt = p.T <= 2 ? 2 : p.T <= 4 ? 4 : 8;
     const bool glu = p.epi == EPI_SWIGLU;
-    const bool four = rows_few_tasks(p, 4) >= full, two = glu || rows_few_tasks(p, 2) >= full;
+    auto cost = [&](int R) { return (rows_few_tasks(p, R) + full - 1) / full * (R * (4 + tt / 2) + (tt == 8 ? 16 : 6)); };
+    const int c4 = cost(4), c2 = cost(2), c1 = glu ? c2 + 1 : cost(1);
+    const bool four = c4 <= c2 && c4 <= c1, two = c2 <= c1;
     if (p.T <= 2) return four ? rows_few_go<4, 2>(p, n_sm, pdl, st) : two ? rows_few_go<2, 2>(p, n_sm, pdl, st) : rows_few_go<1, 2>(p, n_sm, pdl, st);
     if (p.T <= 4) return four ? rows_few_go<4, 4>(p, n_sm, pdl, st) : two ? rows_few_go<2, 4>(p, n_sm, pdl, st) : rows_few_go<1, 4>(p, n_sm, pdl, st);
     return four ? rows_few_go<4, 8>(p, n_sm, pdl, st) : two ? rows_few_go<2, 8>(p, n_sm, pdl, st) : rows_few_go<1, 8>(p, n_sm, pdl, st);
