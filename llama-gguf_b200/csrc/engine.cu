@@ -117,6 +117,7 @@ struct Slot {
     signed char* kv8 = nullptr;   // int8 KV format (kv_int8.cuh): [L][2][n_kv][max_seq][hd] bytes ...
     float* kv_scale = nullptr;    // ... and [L][2][n_kv][max_seq] scales; kv stays null
     uint64_t host_pos = 0;
+    bool stale = false;            // reset since: d_state is zeroed before the next token that starts from it (prompts and batched steps write it whole)
     bool spec = false;            // greedy continuation (b200_ctx_set_speculation): the NEXT token is already in flight ...
     int spec_buf = 0;             // ... its logits land in h_spec_logits[spec_buf], the token it consumed in h_spec_pick[spec_buf]
     cudaGraphExec_t graph[MODE_COUNT] = {nullptr, nullptr, nullptr};
@@ -2303,6 +2304,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         if (bg.exec) {
             CU(cudaGraphLaunch(bg.exec, c->stream));
             c->launches += bg.launches;
+            for (int i = 0; i < n; i++) c->slots[seqs[i]].stale = false;
             return B200_OK;
         }
         if (bg.warm) {
@@ -2599,7 +2601,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         CU(cudaGetLastError());
     }
     if (rows) {   // every row's slot advances by one; final RMSNorm + vocab head of ALL rows through the GEMM
-        CU(launch_on(st, pdl, prefill_advance_rows_kernel, dim3((n + 127) / 128), dim3(128), 0, (SeqState* const*)d_st, n));
+        CU(launch_on(st, pdl, prefill_advance_rows_kernel, dim3((n + 127) / 128), dim3(128), 0, (SeqState* const*)d_st, (const int*)d_pos, n));
         const DevTensor& head = c->output.present() ? c->output : c->token_embd;
         if (exact) {
             RowsParams p{};
@@ -2634,9 +2636,11 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             bg.launches = c->launches - launches0;
             CU(cudaGraphLaunch(ex, st));
         }
+        for (int i = 0; i < n; i++) c->slots[seqs[i]].stale = false;
         return B200_OK;
     }
-    CU(launch_on(st, pdl, prefill_advance_kernel, dim3(1), dim3(32), 0, sl.d_state, n));
+    CU(launch_on(st, pdl, prefill_advance_kernel, dim3(1), dim3(32), 0, sl.d_state, (int)sl.host_pos + n));
+    sl.stale = false;
     if (want_logits) {   // final RMSNorm + vocab head of the last token, through the exact GEMV path
         CU(cudaMemcpyAsync(c->xa, X + (size_t)(last_T - 1) * H, (size_t)H * sizeof(float), cudaMemcpyDeviceToDevice, st));
         GemvParams p{};
@@ -2721,7 +2725,14 @@ static int check_token(b200_ctx* c, int seq, uint32_t token, const char* fn) {
     return B200_OK;
 }
 
+static int settle_state(b200_ctx* c, Slot& sl) {
+    if (!sl.stale) return B200_OK;
+    CU(cudaMemsetAsync(sl.d_state, 0, sizeof(SeqState), c->stream));
+    sl.stale = false;
+    return B200_OK;
+}
 static int set_token(b200_ctx* c, Slot& sl, uint32_t token) {
+    if (const int rc = settle_state(c, sl)) return rc;
     if (++c->h_token_at == kTokenRing) {      // every place of the ring may hold a token that has not been copied yet
         CU(cudaStreamSynchronize(c->stream));
         c->h_token_at = 0;
@@ -2746,6 +2757,7 @@ static int watchdog_check(b200_ctx* c, const char* who) {
     memset(c->h_err, 0, 8 * sizeof(int));
     for (Slot& sl : c->slots) {
         SeqState st{};
+        if (sl.stale) continue;      // (host_pos is 0)
         if (cudaMemcpy(&st, sl.d_state, sizeof st, cudaMemcpyDeviceToHost) == cudaSuccess) sl.host_pos = (uint64_t)std::max(st.pos_next, 0);
     }
     return fail(B200_ERR_OPERATION_FAILED, msg);
@@ -3009,7 +3021,7 @@ extern "C" int b200_reset(b200_ctx* c, int seq) {
     CU(cudaSetDevice(c->par.device));
     Slot& sl = c->slots[seq];
     sl.pending.clear();
-    CU(cudaMemsetAsync(sl.d_state, 0, sizeof(SeqState), c->stream));      // (what reads it next is on the same stream)
+    sl.stale = true;
     sl.host_pos = 0;
     return B200_OK;
 }
@@ -4441,6 +4453,7 @@ extern "C" int b200_debug_set_position(b200_ctx* c, int seq, uint64_t pos) {
     if (pos >= (uint64_t)c->d.max_seq_len) return fail(B200_ERR_INVALID_ARGUMENT, "b200_debug_set_position: beyond the context");
     if ((rc = flush_pending(c, seq))) return rc;
     CU(cudaSetDevice(c->par.device));
+    if ((rc = settle_state(c, c->slots[seq]))) return rc;
     CU(cudaStreamSynchronize(c->stream));
     const int p = (int)pos;
     CU(cudaMemcpy(&c->slots[seq].d_state->pos_next, &p, sizeof(int), cudaMemcpyHostToDevice));

@@ -1624,6 +1624,7 @@ struct SlotMem {
 
 }  // namespace
 
+constexpr int HEAD_WORDS = 64;
 struct LpModel {
     b200_program_desc p{};
     std::vector<b200_layer_desc> layers;
@@ -1656,6 +1657,7 @@ struct LpModel {
     std::vector<int> run_pass;          // pass number t when the run is the first of a pass (step vector t is added), else -1
     std::vector<size_t> run_kv_off, run_rec_off;
     size_t slot_kv_bytes = 0, slot_rec_bytes = 0;
+    bool slot_state = false;            // the program keeps a state beside the cache
     std::vector<SlotMem> slot;          // per sequence slot; null = holds nothing
     std::vector<SlotMem> pool;
     double* inv_freq = nullptr;
@@ -1686,7 +1688,6 @@ struct LpModel {
     bool need_y2 = false;               // m->y holds two sublayer outputs per row (branches that are normed before they are summed)
     void *hn = nullptr, *act_a = nullptr, *hw = nullptr;
     int* pick = nullptr;
-    float* h_logits = nullptr;          // pinned
     size_t h_logits_bytes = 0;
     int max_in = 0, max_act = 0, max_o = 0, max_conv = 0, max_q = 0;
     float* taps = nullptr;
@@ -1712,8 +1713,8 @@ struct LpModel {
     bool use_gemv_mma = true;    // B200_LP_GEMV_MMA=0: small decode batches multiply on the CUDA cores
     int conv_fuse_rows = 1;      // B200_LP_CONV_FUSE_ROWS: decode steps of so many rows norm and convolve inside the projection
     bool use_lat_split = true;   // B200_LP_LAT_SPLIT=0: decoding attention over shared rows in the many-row kernels
-    int* tc_err = nullptr;
-    int* h_tc_err = nullptr;
+    int* tc_err = nullptr;              // [HEAD_WORDS], the tail's counter among them, and behind them the logits
+    int* h_tc_err = nullptr;            // pinned: the same
     unsigned* tail_counter = nullptr;   // arrival counter of rows_tail (zero between kernels)
 };
 
@@ -2973,7 +2974,8 @@ int lp_finalize(LpModel* m, std::string* err) {
         m->n_convs = (int)offs.size();
     }
     m->slot_kv_bytes = std::max<size_t>(kv, 256);
-    m->slot_rec_bytes = std::max<size_t>(rec, 256);
+    m->slot_state = rec > 0;
+    m->slot_rec_bytes = up16(std::max<size_t>(rec, 256));
     // frequencies of the sinusoidal position vector, in double
     {
         const int nf = (p.width + 1) / 2;
@@ -3000,10 +3002,10 @@ int lp_finalize(LpModel* m, std::string* err) {
         const char* e = getenv("B200_LP_ANY_ORDER");
         m->any_order = e && *e ? atoi(e) != 0 : m->max_experts == 0;
     }
-    LCU_ALLOC(cudaMalloc((void**)&m->tc_err, 256));
-    LCU(cudaMemset(m->tc_err, 0, 256));
+    LCU_ALLOC(cudaMalloc((void**)&m->tc_err, HEAD_WORDS * 4));
+    LCU(cudaMemset(m->tc_err, 0, HEAD_WORDS * 4));
     m->tail_counter = (unsigned*)(m->tc_err + 16);
-    LCU_ALLOC(cudaHostAlloc((void**)&m->h_tc_err, 64, cudaHostAllocDefault));
+    LCU_ALLOC(cudaHostAlloc((void**)&m->h_tc_err, HEAD_WORDS * 4, cudaHostAllocDefault));
     *m->h_tc_err = 0;
     m->finalized = true;
     return B200_OK;
@@ -3022,13 +3024,12 @@ void lp_destroy(LpModel* m) {
     }
     for (SlotMem& s : m->slot) { cudaFree(s.kv); cudaFree(s.rec); }
     for (SlotMem& s : m->pool) { cudaFree(s.kv); cudaFree(s.rec); }
-    for (void* ptr : {(void*)m->inv_freq, (void*)m->d_meta, (void*)m->x, (void*)m->P, (void*)m->qbuf, (void*)m->O, (void*)m->conv, (void*)m->logits,
+    for (void* ptr : {(void*)m->inv_freq, (void*)m->d_meta, (void*)m->x, (void*)m->P, (void*)m->qbuf, (void*)m->O, (void*)m->conv,
                       m->hn, m->act_a, m->hw, (void*)m->pick, (void*)m->taps, (void*)m->glin_carry, (void*)m->y, (void*)m->vsrc, (void*)m->moe_w, (void*)m->moe_selw,
                       (void*)m->moe_sel, (void*)m->moe_pos, (void*)m->moe_seg, m->moe_xp, (void*)m->moe_yp, (void*)m->xs, (void*)m->x2, m->cq, (void*)m->vrot, m->xcat,
                       (void*)m->lat_o, (void*)m->lat_ml, (void*)m->moe_shw, (void*)m->ring_offs, (void*)m->conv_pend})
         cudaFree(ptr);
     if (m->h_meta) cudaFreeHost(m->h_meta);
-    if (m->h_logits) cudaFreeHost(m->h_logits);
     if (m->h_tc_err) cudaFreeHost(m->h_tc_err);
     cudaFree(m->tc_err);
     cudaFree(m->keys16);
@@ -3095,6 +3096,34 @@ int grow(LpModel* m, P** ptr, size_t bytes, std::string* err) {
     return B200_OK;
 }
 
+// The logits lie behind the error word and the tail's counter, so that a step brings both back in one copy.
+int grow_logits(LpModel* m, size_t bytes, std::string* err) {
+    auto take = [&](size_t n) {
+        int* b = nullptr;
+        if (step_malloc(m, (void**)&b, HEAD_WORDS * 4 + up16(n)) != cudaSuccess || cudaMemsetAsync(b, 0, HEAD_WORDS * 4, m->stream) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(b);
+            return false;
+        }
+        cudaFree(m->tc_err);
+        m->tc_err = b;
+        m->tail_counter = (unsigned*)(b + 16);
+        m->logits = n ? (float*)(b + HEAD_WORDS) : nullptr;
+        return true;
+    };
+    if (take(bytes)) return B200_OK;
+    take(0);                              // (no room beside the old ones: they go first)
+    if (take(bytes)) return B200_OK;
+    return lp_fail(err, B200_ERR_ALLOCATION_FAILED, "logits: out of memory");
+}
+// A step's new sequences start from zeroed states: one launch for all of them.  grid (16, runs)
+__global__ void __launch_bounds__(256) lp_zero_states_kernel(StepMeta sm, size_t words) {
+    const int run = blockIdx.y;
+    if (sm.run_pos0[run] != 0) return;
+    uint4* r = reinterpret_cast<uint4*>(sm.run_rec[run]);
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (size_t)gridDim.x * 256) r[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) {
     int rc;
     if (R > m->cap_rows || n_want > m->cap_want || n_runs > m->cap_runs) m->scratch_epoch++;   // buffers or table offsets move: graphs are void
@@ -3130,7 +3159,7 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     }
     if (n_want > m->cap_want) {
         const int cap = std::max(n_want, 2 * m->cap_want);
-        if ((rc = grow(m, &m->logits, (size_t)cap * m->p.vocab * 4, err))) return rc;
+        if ((rc = grow_logits(m, (size_t)cap * m->p.vocab * 4, err))) return rc;
         if ((rc = grow(m, &m->hw, (size_t)cap * W * es, err))) return rc;
         if ((rc = grow(m, &m->pick, (size_t)cap * 4, err))) return rc;
         m->cap_want = cap;
@@ -4041,6 +4070,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
     m->step_p0.assign(pos0, pos0 + n_runs);
     m->step_len.assign(lens, lens + n_runs);
     if ((rc = ensure_scratch(m, R, n_runs, n_want, err))) return rc;
+    bool fresh = false;
     // slot memory: a slot at position 0 starts from a zeroed state block (out of the pool when one is waiting there)
     for (int i = 0; i < n_runs; i++) {
         SlotMem& s = m->slot[seqs[i]];
@@ -4062,7 +4092,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
                     return lp_fail(err, B200_ERR_ALLOCATION_FAILED, std::string("slot state: ") + cudaGetErrorString(e));
                 }
             }
-            LCU(cudaMemsetAsync(s.rec, 0, m->slot_rec_bytes, m->stream));
+            fresh = true;
         }
     }
     // tables of the step
@@ -4102,6 +4132,10 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         sm.want = sm.run_pos0 + m->cap_runs + 1;
         sm.run_kv = (uint8_t* const*)(d + ints);
         sm.run_rec = sm.run_kv + m->cap_runs;
+    }
+    if (fresh && m->slot_state) {      // (exactly the runs at position 0 have new slots)
+        lp_zero_states_kernel<<<dim3(16, n_runs), 256, 0, m->stream>>>(sm, up16(m->slot_rec_bytes) / 16);
+        m->launches++;
     }
     const int W = p.width;
     if (m->taps_on) {
@@ -4186,15 +4220,15 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
     } else if (head == 1) {
         const size_t bytes = (size_t)n_want * p.vocab * 4;
         if (bytes > m->h_logits_bytes) {
-            if (m->h_logits) cudaFreeHost(m->h_logits);
-            m->h_logits = nullptr;
-            m->h_logits_bytes = 0;
-            LCU_ALLOC(cudaHostAlloc((void**)&m->h_logits, bytes, cudaHostAllocDefault));
+            int* b = nullptr;
+            LCU_ALLOC(cudaHostAlloc((void**)&b, HEAD_WORDS * 4 + bytes, cudaHostAllocDefault));
+            *b = 0;
+            cudaFreeHost(m->h_tc_err);
+            m->h_tc_err = b;
             m->h_logits_bytes = bytes;
         }
-        LCU(cudaMemcpyAsync(m->h_logits, m->logits, bytes, cudaMemcpyDeviceToHost, m->stream));
-    }
-    LCU(cudaMemcpyAsync(m->h_tc_err, m->tc_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+        LCU(cudaMemcpyAsync(m->h_tc_err, m->tc_err, HEAD_WORDS * 4 + bytes, cudaMemcpyDeviceToHost, m->stream));      // (logits behind the error word)
+    } else LCU(cudaMemcpyAsync(m->h_tc_err, m->tc_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     LCU(cudaStreamSynchronize(m->stream));
     {
         const cudaError_t e_ = cudaGetLastError();
@@ -4210,6 +4244,6 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         cudaMemset(m->tc_err, 0, sizeof(int));
         return lp_fail(err, B200_ERR_OPERATION_FAILED, "b200_step: tensor-core GEMM wait gave up (code " + std::to_string(code) + "): results discarded");
     }
-    if (n_want > 0 && logits_out) memcpy(logits_out, m->h_logits, (size_t)n_want * p.vocab * 4);
+    if (n_want > 0 && logits_out) memcpy(logits_out, m->h_tc_err + HEAD_WORDS, (size_t)n_want * p.vocab * 4);
     return B200_OK;
 }

@@ -326,25 +326,25 @@ __global__ void prefill_swiglu_kernel(const float* __restrict__ g, const float* 
     }
 }
 
-// the slot's position after T more tokens
-__global__ void prefill_advance_kernel(SeqState* st, int T) {
+// the slot's position after a prompt whose last token was at `next` - 1
+__global__ void prefill_advance_kernel(SeqState* st, int next) {
     pdl_launch_dependents();
     pdl_wait();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
-        st->pos_cur = st->pos_next + T - 1;
-        st->pos_next = st->pos_next + T;
+        st->pos_cur = next - 1;
+        st->pos_next = next;
     }
 }
 
-// batched decode: every row's slot advances by one token
-__global__ void prefill_advance_rows_kernel(SeqState* const* st, int n) {
+// batched decode: every row's slot stands behind the token at row_pos
+__global__ void prefill_advance_rows_kernel(SeqState* const* st, const int* __restrict__ row_pos, int n) {
     pdl_launch_dependents();
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         SeqState* s = st[i];
-        s->pos_cur = s->pos_next;
-        s->pos_next = s->pos_next + 1;
+        s->pos_cur = row_pos[i];
+        s->pos_next = row_pos[i] + 1;
     }
 }
 
