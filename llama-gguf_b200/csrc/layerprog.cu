@@ -360,15 +360,38 @@ template <typename T, int NR> __device__ __forceinline__ void gemv_dot(const T* 
         acc[i] = 0.0f;
         xr[i] = X + (size_t)min(i, nr - 1) * ldx;
     }
-#pragma unroll(NR <= 2 ? 8 : 4)
-    for (int k = lane * VN; k < K; k += 32 * VN) {
-        float wv[VN], xv[VN];
-        Vec8<T>::load(w + k, wv);
+    if constexpr (NR <= 2) {
+        // Bound by DRAM latency: U weight loads of 16 bytes per lane, then their products (unrolled alone, fewer were in flight).
+        // Four rows and more keep the plain loop: with explicit loads there, six rows through three layers took 1742 -> 2095 us.
+        constexpr int U = 8, STEP = 32 * VN;
+        for (int k0 = lane * VN; k0 < K; k0 += U * STEP) {
+            uint4 raw[U];
 #pragma unroll
-        for (int i = 0; i < NR; i++) {
-            Vec8<T>::load(xr[i] + k, xv);
+            for (int u = 0; u < U; u++) raw[u] = k0 + u * STEP < K ? *reinterpret_cast<const uint4*>(w + k0 + u * STEP) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-            for (int e = 0; e < VN; e++) acc[i] = fmaf(wv[e], xv[e], acc[i]);
+            for (int u = 0; u < U; u++) {
+                if (k0 + u * STEP >= K) break;
+                float wv[VN], xv[VN];
+                Vec8<T>::load(reinterpret_cast<const T*>(&raw[u]), wv);
+#pragma unroll
+                for (int i = 0; i < NR; i++) {
+                    Vec8<T>::load(xr[i] + k0 + u * STEP, xv);
+#pragma unroll
+                    for (int e = 0; e < VN; e++) acc[i] = fmaf(wv[e], xv[e], acc[i]);
+                }
+            }
+        }
+    } else {
+#pragma unroll 4
+        for (int k = lane * VN; k < K; k += 32 * VN) {
+            float wv[VN], xv[VN];
+            Vec8<T>::load(w + k, wv);
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                Vec8<T>::load(xr[i] + k, xv);
+#pragma unroll
+                for (int e = 0; e < VN; e++) acc[i] = fmaf(wv[e], xv[e], acc[i]);
+            }
         }
     }
 }
@@ -381,7 +404,10 @@ template <typename T, int NR> __device__ __forceinline__ void gemv_dot(const T* 
         if ((R) <= 1) { CALL(1); } else if ((R) <= 2) { CALL(2); } else if ((R) <= 4) { CALL(4); } else { CALL(GV_ROWS); } \
     } while (0)
 
-template <typename T, int EPI, int NR>
+// TAIL: the grid's last blocks may norm the rows (rows_tail).  An instance of its own, because the tail's registers cost the launches
+// that have none their loads in flight.  With gemv_dot's explicit loads: 300 tokens and 24 steps of one row through four 1024-wide
+// layers 5940 -> 5660 us, 12 rows through two layers with a window 1090 -> 1029.
+template <typename T, int EPI, int NR, bool TAIL>
 __global__ void __launch_bounds__(256) lp_gemv_kernel(const T* __restrict__ X, int ldx, const T* __restrict__ W, int ldw, void* __restrict__ Y,
                                                       int ldy, int R, int N, int K, float alpha, int vec_ok, int stage, RowsTail tail, int nh,
                                                       ZStride zs, const float* __restrict__ bias, float2 act) {
@@ -439,7 +465,7 @@ __global__ void __launch_bounds__(256) lp_gemv_kernel(const T* __restrict__ X, i
         }
     }
     }
-    if (tail.on) rows_tail<T>(tail);
+    if constexpr (TAIL) rows_tail<T>(tail);
 }
 
 __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
@@ -1983,7 +2009,7 @@ void gemm_t(LpModel* m, const void* X, int ldx, const void* W, int ldw, int N, i
         const RowsTail tl = tail ? *tail : RowsTail{};
         const int nh = heads ? N : 0;
 #define LP_GV(E) LP_NR_DISPATCH(R, LP_GV_##E)
-#define LP_GV_N(E, NR) launch(m, lp_gemv_kernel<T, E, NR>, grid, block, smem, x, ldx, w, ldw, Y, ldy, R, Nall, K, alpha, vec_ok, stage, tl, nh, zs, bias, act)
+#define LP_GV_N(E, NR) launch(m, tl.on ? lp_gemv_kernel<T, E, NR, E == EPI_STORE> : lp_gemv_kernel<T, E, NR, false>, grid, block, smem, x, ldx, w, ldw, Y, ldy, R, Nall, K, alpha, vec_ok, stage, tl, nh, zs, bias, act)
 #define LP_GV_EPI_STORE(NR) LP_GV_N(EPI_STORE, NR)
 #define LP_GV_EPI_ADD(NR) LP_GV_N(EPI_ADD, NR)
 #define LP_GV_EPI_GELU(NR) LP_GV_N(EPI_GELU, NR)
@@ -3903,10 +3929,10 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
                 if (sfew) pre_done = true;
                 if (m->f32) {
                     launch(m, lp_moe_up_sel_kernel<float>, ugrid, dim3(256), hbytes, (const float*)m->hn, (const float*)up_experts, (const int*)m->moe_sel, (const float*)m->moe_selw, (const float*)shw, e.experts, e.top, e.expert_ff, e.shared_ff, W, R, (float*)m->act_a, ea);
-                    launch(m, lp_moe_down_sel_kernel<float>, dgrid, dim3(256), 0, (const float*)m->act_a, (const float*)L.w_down, (const int*)m->moe_sel, e.experts, e.top, e.expert_ff, e.shared_ff, W, R, ydst, t, direct ? 1 : 0, (const float*)m->moe_selw, (const float*)m->hn, hf, e.identity);
+                    launch(m, t.on ? lp_moe_down_sel_kernel<float, true> : lp_moe_down_sel_kernel<float, false>, dgrid, dim3(256), 0, (const float*)m->act_a, (const float*)L.w_down, (const int*)m->moe_sel, e.experts, e.top, e.expert_ff, e.shared_ff, W, R, ydst, t, direct ? 1 : 0, (const float*)m->moe_selw, (const float*)m->hn, hf, e.identity);
                 } else {
                     launch(m, lp_moe_up_sel_kernel<bf16>, ugrid, dim3(256), hbytes, (const bf16*)m->hn, (const bf16*)up_experts, (const int*)m->moe_sel, (const float*)m->moe_selw, (const float*)shw, e.experts, e.top, e.expert_ff, e.shared_ff, W, R, (bf16*)m->act_a, ea);
-                    launch(m, lp_moe_down_sel_kernel<bf16>, dgrid, dim3(256), 0, (const bf16*)m->act_a, (const bf16*)L.w_down, (const int*)m->moe_sel, e.experts, e.top, e.expert_ff, e.shared_ff, W, R, ydst, t, direct ? 1 : 0, (const float*)m->moe_selw, (const bf16*)m->hn, hf, e.identity);
+                    launch(m, t.on ? lp_moe_down_sel_kernel<bf16, true> : lp_moe_down_sel_kernel<bf16, false>, dgrid, dim3(256), 0, (const bf16*)m->act_a, (const bf16*)L.w_down, (const int*)m->moe_sel, e.experts, e.top, e.expert_ff, e.shared_ff, W, R, ydst, t, direct ? 1 : 0, (const float*)m->moe_selw, (const bf16*)m->hn, hf, e.identity);
                 }
             } else if (m->use_fuse && R > 2 * GV_ROWS) {
                 // many rows: the (token, choice) pairs in expert order, one product pair per expert over its block of rows (the row

@@ -237,8 +237,9 @@ __global__ void __launch_bounds__(256) lp_moe_up_sel_kernel(const T* __restrict_
 // each takes every MD_SPLIT-th 16-byte group of every segment (more loads in flight per output: a decode step has only `width` of
 // them), the partial sums meet in shared memory and are added in warp order.  accum = 1: y += (y is the residual stream).  Identity experts
 // (choices e >= E) have no segment: they add their weight times what the feed-forward reads, hf in f32 or, when that is null, h.
+// TAIL: the last blocks may norm the rows; the instance without keeps the registers for loads (as lp_gemv_kernel's).
 constexpr int MD_SPLIT = 4, MD_BATCH = 6;
-template <typename T>
+template <typename T, bool TAIL>
 __global__ void __launch_bounds__(256) lp_moe_down_sel_kernel(const T* __restrict__ act, const T* __restrict__ down_cat, const int* __restrict__ sel,
                                                               int E, int top, int eff, int sff, int width, int R, float* __restrict__ y, RowsTail tail, int accum,
                                                               const float* __restrict__ selw, const T* __restrict__ h, const float* hf, int identity) {
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(256) lp_moe_down_sel_kernel(const T* __restric
         }
         __syncthreads();
     }
-    if (tail.on) rows_tail<T>(tail);
+    if constexpr (TAIL) rows_tail<T>(tail);
 }
 
 // Many rows: the (token, choice) pairs are put in expert order, so that every expert multiplies a contiguous block of rows.
