@@ -1140,8 +1140,8 @@ static cudaError_t enqueue_token(b200_ctx* c, int slot_i, Mode mode, bool only_g
             ap.q = q; ap.k8 = k8; ap.v8 = v8; ap.k_scale = ks; ap.v_scale = vs; ap.part = c->attn_q8_part; ap.out = c->attn; ap.pos = pos_ptr;
             ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.n_splits = c->attn_q8_splits; ap.scale = 1.0f / sqrtf((float)hd);
             const dim3 grid(ap.n_splits, nkv);
-            CK(launch_k(c, hd == 128 ? attn_q8_split_kernel<128, 4> : attn_q8_split_kernel<64, 4>, grid, dim3(kAttnQ8Warps * 32), 0, ap));
-            CK(launch_k(c, attn_q8_merge_kernel, dim3(nh), dim3(kAttnQ8MergeThreads), 0, ap, hd));
+            CK(launch_k(c, hd == 128 ? attn_q8_split_kernel<128, 4, false> : attn_q8_split_kernel<64, 4, false>, grid, dim3(kAttnQ8Warps * 32), 0, ap));
+            CK(launch_k(c, attn_q8_merge_kernel<false>, dim3(nh), dim3(kAttnQ8MergeThreads), 0, ap, hd));
         }
         if (!only_gemv && c->kv_format == 0) {   // RoPE, KV write and GQA decode attention over [0, pos]
             AttnParams ap{};
@@ -2135,8 +2135,8 @@ static int exact_layers(b200_ctx* c, Slot& sl, const ExactPass& e) {
             ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.scale = scale;
             ap.n_splits = std::max(std::min(8, c->attn_q8_splits), std::min(c->attn_q8_splits, 2 * c->n_sm / (nkv * T)));      // (two blocks per SM)
             ap.part_row = (long long)nkv * ap.n_splits * G * (hd + 2);
-            CU(launch_on(e.st, e.pdl, hd == 128 ? attn_q8_split_kernel<128, 4> : attn_q8_split_kernel<64, 4>, dim3(ap.n_splits, nkv, T), dim3(kAttnQ8Warps * 32), 0, ap));
-            CU(launch_on(e.st, e.pdl, attn_q8_merge_kernel, dim3(nh, 1, T), dim3(kAttnQ8MergeThreads), 0, ap, hd));
+            CU(launch_on(e.st, e.pdl, hd == 128 ? attn_q8_split_kernel<128, 4, true> : attn_q8_split_kernel<64, 4, true>, dim3(ap.n_splits, nkv, T), dim3(kAttnQ8Warps * 32), 0, ap));
+            CU(launch_on(e.st, e.pdl, attn_q8_merge_kernel<true>, dim3(nh, 1, T), dim3(kAttnQ8MergeThreads), 0, ap, hd));
             c->launches += 3;
         } else {
             PrefillRopeParams rp{};

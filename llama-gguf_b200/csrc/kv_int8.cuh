@@ -160,15 +160,18 @@ struct AttnQ8Params {
     const float* v_scale;
     float* part;               // [n_kv][n_splits][G][hd + 2]: unnormalised accumulator, running max, running sum
     float* out;                // [n_heads][hd]
-    const int* pos;            // device scalar: kv_len = *pos + 1; nullptr: blockIdx.z is the row of a prompt, at position pos0 + z
+    const int* pos;            // device scalar: kv_len = *pos + 1; rows (ROWS): blockIdx.z is the row of a prompt, at position pos0 + z
     int n_kv, G, max_seq, n_splits;
     float scale;
     int pos0, ldq, ldo;        // (rows)
     long long part_row;
 };
-// the row of a block
+// The row of a block.  Decoding reads the parameters where they are: a copy with the row's pointers costs its launches 1 us each (20 tokens through one 8B layer
+// 2981 -> 3033 us).
+template <bool ROWS> struct AttnQ8Row { using P = const AttnQ8Params&; };
+template <> struct AttnQ8Row<true> { using P = AttnQ8Params; };
+__device__ __forceinline__ int attn_q8_row(const AttnQ8Params& p) { return *p.pos + 1; }
 __device__ __forceinline__ int attn_q8_row(AttnQ8Params& p) {
-    if (p.pos) return *p.pos + 1;
     const int z = blockIdx.z;
     p.q += (size_t)z * p.ldq;
     p.out += (size_t)z * p.ldo;
@@ -199,7 +202,7 @@ constexpr int kAttnQ8Unroll = 4;
 // across the warps through shared memory.  HG <= 4 query heads per warp: a group of 8 heads is two head groups on two warp pairs
 // (both read the same rows; the second read hits L1 / L2).  The row scale is applied once per score (K) and folded into the
 // softmax weight (V).  grid (n_splits, n_kv), 128 threads.
-template <int HD, int HG>
+template <int HD, int HG, bool ROWS>
 __global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(const AttnQ8Params p_in) {
     constexpr int LPR = HD / 16, RPW = 32 / LPR, U = kAttnQ8Unroll;
     __shared__ float sm[kAttnQ8Warps][HG][HD + 2];
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(con
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, split = blockIdx.x, kh = blockIdx.y, G = p_in.G;
     const int NHG = (G + HG - 1) / HG, WPG = kAttnQ8Warps / NHG;   // head groups (1 or 2), warps per head group
     const int hgp = warp % NHG, wsub = warp / NHG, sub = lane % LPR, rg = lane / LPR;
-    AttnQ8Params p = p_in;
+    typename AttnQ8Row<ROWS>::P p = p_in;
     const int kv_len = attn_q8_row(p);
     const int chunk = (kv_len + p.n_splits - 1) / p.n_splits;
     const int p_begin = split * chunk, p_end = min(kv_len, p_begin + chunk);
@@ -322,11 +325,12 @@ __global__ void __launch_bounds__(kAttnQ8Warps * 32, 2) attn_q8_split_kernel(con
 // (groups in order at the end).  9 positions in 128 splits, 14 heads of 64: 21 -> 5 us against one thread per channel that walked all splits after two
 // serial passes of one thread over the maxima and sums.
 constexpr int kAttnQ8MaxSplits = 128, kAttnQ8MergeThreads = 256;
+template <bool ROWS>
 __global__ void __launch_bounds__(kAttnQ8MergeThreads) attn_q8_merge_kernel(const AttnQ8Params p_in, int hd) {
     __shared__ float sc[kAttnQ8MaxSplits], sums[kAttnQ8MergeThreads], s_l;
     pdl_launch_dependents();
     pdl_wait();
-    AttnQ8Params p = p_in;
+    typename AttnQ8Row<ROWS>::P p = p_in;
     const int kv_len = attn_q8_row(p);
     const int head = blockIdx.x, kh = head / p.G, g = head - kh * p.G, lane = threadIdx.x & 31;
     const int chunk = (kv_len + p.n_splits - 1) / p.n_splits, live = (kv_len + chunk - 1) / chunk;      // (<= n_splits)
