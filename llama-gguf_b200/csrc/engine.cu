@@ -1027,7 +1027,7 @@ static cudaError_t launch_gemv(b200_ctx* c, GemvParams& p) {
         const bool small = mb < 8 && (size_t)xpad_floats(p.K) * sizeof(float) <= 160 * 1024;
         if (!small && to_mma_params(c, p, m, plan)) {
             c->mma_launches++;
-            return launch_k(c, mma_kernel_for(plan.stages), dim3(plan.grid), dim3(plan.warps * 32), plan.smem, m);
+            return launch_k(c, mma_kernel_for(c->d.n_experts > 0), dim3(plan.grid), dim3(plan.warps * 32), plan.smem, m);
         }
     }
     c->v1_launches++;
@@ -1183,8 +1183,8 @@ static cudaError_t enqueue_token(b200_ctx* c, int slot_i, Mode mode, bool only_g
                 if (mb >= 8 && mb2 >= 8 && to_mma_params(c, p, m, plan) && to_mma_params(c, q2, m2, plan2)) {
                     together = true;
                     c->mma_launches += 2;
-                    CK(launch_k(c, mma_kernel_for(plan.stages), dim3(plan.grid), dim3(plan.warps * 32), plan.smem, m));
-                    CK(launch_k(c, mma_kernel_for(plan2.stages), dim3(plan2.grid), dim3(plan2.warps * 32), plan2.smem, m2));
+                    CK(launch_k(c, mma_kernel_for(true), dim3(plan.grid), dim3(plan.warps * 32), plan.smem, m));
+                    CK(launch_k(c, mma_kernel_for(true), dim3(plan2.grid), dim3(plan2.warps * 32), plan2.smem, m2));
                     if (!only_gemv) CK(launch_k(c, moe_combine_kernel, dim3((H + 255) / 256), dim3(256), 0, (const float*)c->moe_y(), d.n_experts_used, (const float*)c->moe_wt, (const float*)c->xb, c->xa, H));
                 }
             }
@@ -3676,7 +3676,7 @@ extern "C" int b200_op_vec_mat_q(const float* a, const void* w, uint32_t ggml_ty
             CU(cudaMemset(dtick.p, 0, tiles * 4));
             m.part = dpart.as<float>(); m.tickets = dtick.as<unsigned int>();
             CU(mma_set_smem_limit((int)lim));
-            mma_kernel_for(plan.stages)<<<plan.grid, plan.warps * 32, plan.smem>>>(m);
+            mma_kernel_for(false)<<<plan.grid, plan.warps * 32, plan.smem>>>(m);
             if ((rc = op_finish("vec_mat_q"))) return rc;
             CU(cudaMemcpy(out, dout.p, n * 4, cudaMemcpyDeviceToHost));
             return B200_OK;

@@ -766,10 +766,12 @@ struct MCursor {
 //   early  : issue the first ring stages with cp.async BEFORE post() (weights never depend on a predecessor), so
 //            they land while the barrier is being waited for; otherwise they are issued after the x loads
 //   warm_l2: (not early) pull the first stages towards L2 before post()
-template <class Pre, class Post>
+//   SLOTS  : p.n_slots may be above 1
+template <bool SLOTS, class Pre, class Post>
 __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, float* s_red, float (*s_part)[2][2][32], Pre pre_fn,
                                              Post post_fn, bool early, bool warm_l2) {
     pre_fn();
+    const bool slots = SLOTS && p.n_slots > 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int nw = blockDim.x >> 5;
     const int K = p.K;
@@ -781,8 +783,8 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
     // units are dealt in contiguous runs, CTA after CTA, warp after warp: the pieces of a tile meet inside one CTA
     // (merged through shared memory); only tiles that straddle CTAs (tile_mode 0) go through global memory
     const int upt = p.units_per_tile;
-    const int per_slot = p.n_slots > 1 ? p.n_ctas / p.n_slots : 0;
-    const int slot_cta0 = p.n_slots > 1 ? (int)blockIdx.x / per_slot * per_slot : 0, ex_slot = p.n_slots > 1 ? min((int)blockIdx.x / per_slot, p.n_slots - 1) : p.expert_slot;
+    const int per_slot = slots ? p.n_ctas / p.n_slots : 0;
+    const int slot_cta0 = slots ? (int)blockIdx.x / per_slot * per_slot : 0, ex_slot = slots ? min((int)blockIdx.x / per_slot, p.n_slots - 1) : p.expert_slot;
     const int cta = blockIdx.x - slot_cta0;      // (among its slot's)
     const long long gw = (long long)blockIdx.x * nw + warp;  // debug stamps only
     int cu0 = 0, cu1 = 0;
@@ -960,7 +962,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
     } else {
         // x: the loads are issued BEFORE the weight copies, the split after them
         XStage xst;
-        const XSource xsrc{p.n_slots > 1 ? p.x + (size_t)ex_slot * p.x_slot : p.x, p.xsum, p.n_sum, p.sum_stride, p.x_res, p.x_full_out};
+        const XSource xsrc{slots ? p.x + (size_t)ex_slot * p.x_slot : p.x, p.xsum, p.n_sum, p.sum_stride, p.x_res, p.x_full_out};
         stage_x_load(xst, xsrc, p.norm_w, K, (int)blockDim.x);
         if (!issued_early) {
             for (int k = 0; k < STAGES - 1; k++) {
@@ -1006,7 +1008,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
             if (p.n_peer > 0) {
                 for (int r = 0; r < p.n_peer; r++) p.peer_out[r][j] = val;  // partial of a row-parallel GEMV, to every rank
             } else {
-                sg.out[(p.n_slots > 1 ? (size_t)ex_slot * p.out_slot : 0) + j] = val;
+                sg.out[(slots ? (size_t)ex_slot * p.out_slot : 0) + j] = val;
             }
         }
         if (p.stage_out) stage_out32(val, e_w, j, p.stage_K, p.stage_out);   // the next GEMV's input, ready to copy
@@ -1151,7 +1153,7 @@ __device__ __forceinline__ void mma_gemv_cta(const MParams& p, uint8_t* smem, fl
             vu += s_part[w][ws][1][lane];
         }
         if (tu0 < cu0 || tu0 + upt > cu1) {  // the tile straddles CTAs (tile_mode 0 only)
-            const int tile_id = (p.n_slots > 1 ? ex_slot * (p.total_units / upt) : 0) + (s == 0 ? 0 : (s == 1 ? p.seg[0].n_tiles : p.seg[0].n_tiles + p.seg[1].n_tiles)) + tile;
+            const int tile_id = (slots ? ex_slot * (p.total_units / upt) : 0) + (s == 0 ? 0 : (s == 1 ? p.seg[0].n_tiles : p.seg[0].n_tiles + p.seg[1].n_tiles)) + tile;
             const int c_first = cta_of(tu0), c_last = cta_of(tu0 + upt - 1);
             float* mine = p.part + ((size_t)(slot_cta0 + cta) * 2 + ((cu0 >= tu0) ? 0 : 1)) * 64;
             mine[lane] = v;
@@ -1205,11 +1207,12 @@ __device__ __forceinline__ void mma_warm_l2(const MParams& p, int depth) {
     }
 }
 
+template <bool SLOTS>
 __global__ void __launch_bounds__(kMmaMaxWarps * 32, 1) gemv_mma_kernel(const __grid_constant__ MParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float s_red[2 * kMmaMaxWarps];
     __shared__ float s_part[kMmaMaxWarps][2][2][32];   // pieces of tiles shared between warps of this CTA
-    mma_gemv_cta(p, smem, s_red, s_part, [] {}, [](auto&&) { pdl_launch_dependents(); pdl_wait(); }, false, true);
+    mma_gemv_cta<SLOTS>(p, smem, s_red, s_part, [] {}, [](auto&&) { pdl_launch_dependents(); pdl_wait(); }, false, true);
 }
 
 // ---------------------------------------------------------------- host-side launch planning
@@ -1318,9 +1321,12 @@ inline bool mma_plan(MParams& p, int n_sm, int want_warps, int want_stages, size
 }
 
 using MmaKernel = void (*)(const MParams);
-inline MmaKernel mma_kernel_for(int) { return gemv_mma_kernel; }
+// Models with experts take the instance with slots for every launch (their steps would fetch two kernels' instructions: 1334 -> 1434 us for eight tokens
+// through one layer of 8 experts of 7B), others the one without (its index arithmetic: 20 tokens through one 8B layer, int8 cache, 2985 -> 2943).
+inline MmaKernel mma_kernel_for(bool experts) { return experts ? gemv_mma_kernel<true> : gemv_mma_kernel<false>; }
 inline cudaError_t mma_set_smem_limit(int bytes) {
-    return cudaFuncSetAttribute(gemv_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemv_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(gemv_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 }  // namespace b200

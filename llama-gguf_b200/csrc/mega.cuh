@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kMmaMaxWarps * 32, 1) mega_decode_kernel(const
                         return busy();
                     });
                 };
-                mma_gemv_cta(cur.gemv, smem, s_red, s_part, bar_arrive, wait_kv, mp.early != 0, false);
+                mma_gemv_cta<false>(cur.gemv, smem, s_red, s_part, bar_arrive, wait_kv, mp.early != 0, false);
                 if (!ok) return;
             } else {
                 attn_stamp(cur.attn, 0);
