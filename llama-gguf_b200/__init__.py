@@ -226,6 +226,7 @@ def lib():
     L.b200_ctx_speculation_stats.argtypes = [vp, i32p, u64p, u64p]
     L.b200_debug_set_position.argtypes = [vp, C.c_int, C.c_uint64]
     L.b200_debug_plan_split.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, i32p]
+    L.b200_debug_prompt_norm.argtypes = [fp, fp, C.c_float, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_uint16)]
     L.b200_decode_batch_greedy.argtypes = [vp, C.POINTER(C.c_int), C.POINTER(C.c_uint32), C.c_int, C.POINTER(C.c_uint32)]
     L.b200_batch_create.argtypes = [vp, C.POINTER(BatchConfig), C.POINTER(vp)]
     L.b200_batch_destroy.argtypes = [vp]
@@ -548,6 +549,14 @@ def plan_split(n_rows, K, T, n_sm=148, persistent=True):
     v = C.c_int(0)
     _check(lib().b200_debug_plan_split(int(n_rows), int(K), int(T), int(n_sm), 1 if persistent else 0, C.byref(v)))
     return v.value
+
+
+def prompt_norm(x, w, eps, any_length=False):
+    """RMS norm of a prompt's rows to fp16: the kernel that rows of this length take, or the one for any length."""
+    x, w = (np.ascontiguousarray(v, dtype=np.float32) for v in (x, w))
+    out = np.empty(x.shape, dtype=np.float16)
+    _check(lib().b200_debug_prompt_norm(_fp(x), _fp(w), float(eps), x.shape[0], x.shape[1], 1 if any_length else 0, out.ctypes.data_as(C.POINTER(C.c_uint16))))
+    return out
 
 
 class BatchedEngine:

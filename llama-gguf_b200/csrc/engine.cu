@@ -4473,3 +4473,19 @@ extern "C" int b200_debug_plan_split(int n_rows, int K, int T, int n_sm, int per
     *k_split_out = p.k_split;
     return B200_OK;
 }
+
+// The norm of a prompt's rows before its fp16 products (tests): the kernel that rows of n elements take, or the one for rows of any length; out: fp16 [rows][n].
+extern "C" int b200_debug_prompt_norm(const float* x, const float* w, float eps, int rows, int n, int any_length, uint16_t* out) {
+    int rc;
+    if ((rc = op_ready())) return rc;
+    if (!x || !w || !out || rows <= 0 || n <= 0) return fail(B200_ERR_INVALID_ARGUMENT, "b200_debug_prompt_norm: bad argument");
+    const size_t all = (size_t)rows * n;
+    DevBuf dx, dw, dout;
+    if (dx.alloc(all * 4) || dw.alloc((size_t)n * 4) || dout.alloc(all * 2)) return fail(B200_ERR_ALLOCATION_FAILED, "b200_debug_prompt_norm");
+    CU(cudaMemcpy(dx.p, x, all * 4, cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(dw.p, w, (size_t)n * 4, cudaMemcpyHostToDevice));
+    (any_length ? prefill_rms_norm_kernel<0> : prefill_rms_norm_for(n))<<<rows, 256>>>(dx.as<float>(), dw.as<float>(), eps, dout.as<__half>(), n);
+    if ((rc = op_finish("b200_debug_prompt_norm"))) return rc;
+    CU(cudaMemcpy(out, dout.p, all * 2, cudaMemcpyDeviceToHost));
+    return B200_OK;
+}

@@ -235,81 +235,57 @@ __global__ void __launch_bounds__(128) prefill_attn_kernel(const PrefillAttnPara
 
 // RMSNorm of T rows, output rounded to fp16 for the tensor-core GEMM that consumes it (same f32 arithmetic as
 // rms_norm_rows_kernel: ss = sum x^2, inv = 1/sqrt(ss/n + eps), (x*inv)*w; simd.rs:847-899)
-// Rows of up to 256 * kRmsMaxV elements are held in registers: all loads of a thread are issued before the first is used (a row is
-// 16 dependent-latency trips otherwise: 15 us per launch at 32 rows), the sums run in the SAME order as before (bit-identical).
-// NV4 > 0: rows of up to 1024 NV4 elements (a multiple of 4, as the buffers' rows are aligned) by float4 (2048 rows of 4096: 17 -> 10 us; few registers, many blocks).
-constexpr int kRmsMaxV = 32;
+// Sums in the order of a block that walks the row: thread t adds the squares of elements t, t + 256, .., then lanes, then warps.
+// NV4 > 0: rows of up to 1024 NV4 elements (a multiple of 4, as the buffers' rows are aligned) by float4, all loads of a thread before the first use; the row goes
+// through shared memory, where thread t finds the elements of its sum (two 8B layers, 2048 rows: 1905 us by wall clock, as with squares added word by word, whose results differed; few registers, many blocks).  NV4 = 0: any row.
 template <int NV4>
 __global__ void __launch_bounds__(256) prefill_rms_norm_kernel(const float* x, const float* w, float eps, __half* out, int n) {
     pdl_launch_dependents();
     pdl_wait();
+    constexpr int NV = NV4 > 0 ? NV4 : 1;
     __shared__ float red[8];
     const float* xr = x + (size_t)blockIdx.x * n;
     __half* orow = out + (size_t)blockIdx.x * n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float ss = 0.0f;
+    float4 v[NV], wv[NV];
     if (NV4 > 0) {
-        float4 v[NV4 > 0 ? NV4 : 1], wv[NV4 > 0 ? NV4 : 1];
+        __shared__ __align__(16) float row[1024 * NV];
 #pragma unroll
-        for (int k = 0; k < NV4; k++) {
+        for (int k = 0; k < NV; k++) {
             const int i = 4 * (threadIdx.x + 256 * k);
             v[k] = i < n ? *reinterpret_cast<const float4*>(xr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             wv[k] = i < n ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-        for (int k = 0; k < NV4; k++) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-        ss = warp_sum(ss);
-        if (lane == 0) red[warp] = ss;
+        for (int k = 0; k < NV; k++) *reinterpret_cast<float4*>(row + 4 * (threadIdx.x + 256 * k)) = v[k];
         __syncthreads();
-        float tot = 0.0f;
-        for (int k = 0; k < 8; k++) tot += red[k];
-        const float inv = 1.0f / sqrtf(tot / (float)n + eps);
 #pragma unroll
-        for (int k = 0; k < NV4; k++) {
-            const int i = 4 * (threadIdx.x + 256 * k);
-            if (i >= n) continue;
-            const __half2 a = __halves2half2(f2h_sat(__fmul_rn(__fmul_rn(v[k].x, inv), wv[k].x)), f2h_sat(__fmul_rn(__fmul_rn(v[k].y, inv), wv[k].y)));
-            const __half2 b = __halves2half2(f2h_sat(__fmul_rn(__fmul_rn(v[k].z, inv), wv[k].z)), f2h_sat(__fmul_rn(__fmul_rn(v[k].w, inv), wv[k].w)));
-            *reinterpret_cast<uint2*>(orow + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        for (int k = 0; k < 4 * NV; k++) {      // (zeros behind the row)
+            const float f = row[threadIdx.x + 256 * k];
+            ss = fmaf(f, f, ss);
         }
-        return;
+    } else {
+        for (int i = threadIdx.x; i < n; i += 256) ss = fmaf(xr[i], xr[i], ss);
     }
-    if (n <= 256 * kRmsMaxV) {
-        float v[kRmsMaxV], wv[kRmsMaxV];
-#pragma unroll
-        for (int k = 0; k < kRmsMaxV; k++) {
-            const int i = threadIdx.x + 256 * k;
-            v[k] = i < n ? xr[i] : 0.0f;
-        }
-#pragma unroll
-        for (int k = 0; k < kRmsMaxV; k++) {
-            const int i = threadIdx.x + 256 * k;
-            wv[k] = i < n ? w[i] : 0.0f;
-        }
-#pragma unroll
-        for (int k = 0; k < kRmsMaxV; k++)
-            if (threadIdx.x + 256 * k < n) ss = fmaf(v[k], v[k], ss);
-        ss = warp_sum(ss);
-        if (lane == 0) red[warp] = ss;
-        __syncthreads();
-        float tot = 0.0f;
-        for (int k = 0; k < 8; k++) tot += red[k];
-        const float inv = 1.0f / sqrtf(tot / (float)n + eps);
-#pragma unroll
-        for (int k = 0; k < kRmsMaxV; k++) {
-            const int i = threadIdx.x + 256 * k;
-            if (i < n) orow[i] = f2h_sat(__fmul_rn(__fmul_rn(v[k], inv), wv[k]));
-        }
-        return;
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ss = fmaf(xr[i], xr[i], ss);
     ss = warp_sum(ss);
     if (lane == 0) red[warp] = ss;
     __syncthreads();
     float tot = 0.0f;
     for (int k = 0; k < 8; k++) tot += red[k];
     const float inv = 1.0f / sqrtf(tot / (float)n + eps);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) orow[i] = f2h_sat(__fmul_rn(__fmul_rn(xr[i], inv), w[i]));
+    if (NV4 > 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int i = 4 * (threadIdx.x + 256 * k);
+            if (i >= n) continue;
+            const __half2 a = __halves2half2(f2h_sat(__fmul_rn(__fmul_rn(v[k].x, inv), wv[k].x)), f2h_sat(__fmul_rn(__fmul_rn(v[k].y, inv), wv[k].y)));
+            const __half2 b = __halves2half2(f2h_sat(__fmul_rn(__fmul_rn(v[k].z, inv), wv[k].z)), f2h_sat(__fmul_rn(__fmul_rn(v[k].w, inv), wv[k].w)));
+            *reinterpret_cast<uint2*>(orow + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        }
+    } else {
+        for (int i = threadIdx.x; i < n; i += 256) orow[i] = f2h_sat(__fmul_rn(__fmul_rn(xr[i], inv), w[i]));
+    }
 }
 
 inline void (*prefill_rms_norm_for(int n))(const float*, const float*, float, __half*, int) {
