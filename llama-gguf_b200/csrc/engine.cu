@@ -862,6 +862,9 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         c->finalized = false;
         return fail(B200_ERR_UNSUPPORTED, "tensor parallelism needs the megakernel path (dense model, K-quant / Q8_0 weights with 256-aligned shards)");
     }
+    // What was cleared and copied above went through the legacy stream, which orders nothing on c->stream (non-blocking); with work of the process before it there (torch's
+    // default stream) none of it may have happened yet.  Later calls clear and copy on c->stream
+    CU(cudaStreamSynchronize(cudaStreamLegacy));
     return B200_OK;
 }
 
@@ -1931,7 +1934,7 @@ static int umma_tmaps_build(b200_ctx* c) {
     add(c->output.present() ? c->output : c->token_embd);
     if (maps.empty()) return B200_OK;
     CU_ALLOC(late_malloc(c, (void**)&c->pf_tmaps, maps.size() * sizeof(CUtensorMap)));
-    CU(cudaMemcpy(c->pf_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(c->pf_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, c->stream));      // (from pageable memory: staged before the call returns)
     const b200_model_desc& d = c->d;
     // Whole blocks of 256 in every row, and 1024 wide at least: narrower models gain as well, but not at every length (two-pass or fused products -> these, prompts of 33 /
     // 64 / 128 / 256 tokens through four layers: 512 wide, ffn 2048, Q4_K 389 / 431 / 291 / 315 -> 218 / 231 / 243 / 251 us; 768 wide 442 / 521 / 399 / 732 -> 226 / 265 /
@@ -2049,7 +2052,7 @@ static bool exact_rows_room(b200_ctx* c, int n) {
     exact_rows_free(c);
     const size_t tickets = (size_t)kExactFew * c->d.n_kv_heads * sizeof(unsigned int);
     if (cudaMalloc((void**)&c->er_buf, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess || cudaMalloc((void**)&c->er_tickets, tickets) != cudaSuccess ||
-        cudaMemset(c->er_tickets, 0, tickets) != cudaSuccess) {
+        cudaMemsetAsync(c->er_tickets, 0, tickets, c->stream) != cudaSuccess) {
         cudaGetLastError();
         exact_rows_free(c);
         c->er_retry.failed();
@@ -2214,7 +2217,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         c->pf_split_floats = (size_t)8 * 64 * std::max(std::max(I, QKV), H);
         CU_ALLOC(late_malloc(c, (void**)&c->pf_split, c->pf_split_floats * sizeof(float)));
         CU_ALLOC(late_malloc(c, (void**)&c->pf_tile_cnt, 8192 * sizeof(int)));
-        CU(cudaMemset(c->pf_tile_cnt, 0, 8192 * sizeof(int)));
+        CU(cudaMemsetAsync(c->pf_tile_cnt, 0, 8192 * sizeof(int), c->stream));
     }
     // products of few rows (gemm_few.cuh): images of the activations and pieces of cut tiles; a device without room for them keeps the other products
     const int few_max = kFewTokens, last_chunk = n % cap ? n % cap : cap;
@@ -2708,7 +2711,7 @@ static int spec_drain(b200_ctx* c, int seq) {
     CU(cudaSetDevice(c->par.device));
     CU(cudaStreamSynchronize(c->stream));
     const int pos = (int)sl.host_pos;
-    CU(cudaMemcpy(&sl.d_state->pos_next, &pos, sizeof(int), cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(&sl.d_state->pos_next, &pos, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     return B200_OK;
 }
 static int check_slot(b200_ctx* c, int seq, const char* fn) {
@@ -2753,7 +2756,7 @@ static int watchdog_check(b200_ctx* c, const char* who) {
              c->h_err[1], c->h_err[2], c->h_err[3]);
     // reported once: clear the words (a later call starts clean) and resynchronise every slot's host position with the device's
     // (the launch may have advanced pos_next before it gave up)
-    cudaMemset(c->mma_err, 0, 8 * sizeof(int));
+    cudaMemsetAsync(c->mma_err, 0, 8 * sizeof(int), c->stream);
     memset(c->h_err, 0, 8 * sizeof(int));
     for (Slot& sl : c->slots) {
         SeqState st{};
@@ -3367,7 +3370,7 @@ extern "C" int b200_debug_err(b200_ctx* c, int* out8) {
     CU(cudaSetDevice(c->par.device));
     CU(cudaStreamSynchronize(c->stream));
     CU(cudaMemcpy(out8, c->mma_err, 8 * sizeof(int), cudaMemcpyDeviceToHost));
-    CU(cudaMemset(c->mma_err, 0, 8 * sizeof(int)));
+    CU(cudaMemsetAsync(c->mma_err, 0, 8 * sizeof(int), c->stream));
     memset(c->h_err, 0, 8 * sizeof(int));
     return B200_OK;
 }
@@ -4456,7 +4459,7 @@ extern "C" int b200_debug_set_position(b200_ctx* c, int seq, uint64_t pos) {
     if ((rc = settle_state(c, c->slots[seq]))) return rc;
     CU(cudaStreamSynchronize(c->stream));
     const int p = (int)pos;
-    CU(cudaMemcpy(&c->slots[seq].d_state->pos_next, &p, sizeof(int), cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(&c->slots[seq].d_state->pos_next, &p, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     c->slots[seq].host_pos = pos;
     return B200_OK;
 }

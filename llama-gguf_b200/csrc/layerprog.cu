@@ -3033,6 +3033,7 @@ int lp_finalize(LpModel* m, std::string* err) {
     m->tail_counter = (unsigned*)(m->tc_err + 16);
     LCU_ALLOC(cudaHostAlloc((void**)&m->h_tc_err, HEAD_WORDS * 4, cudaHostAllocDefault));
     *m->h_tc_err = 0;
+    LCU(cudaStreamSynchronize(cudaStreamLegacy));      // (what was cleared and copied there: the model's stream is non-blocking and does not wait for it)
     m->finalized = true;
     return B200_OK;
 }
@@ -4267,7 +4268,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
     if (*m->h_tc_err) {   // a bounded wait of the tensor-core GEMM gave up: the step's results are void
         const int code = *m->h_tc_err;
         *m->h_tc_err = 0;
-        cudaMemset(m->tc_err, 0, sizeof(int));
+        cudaMemsetAsync(m->tc_err, 0, sizeof(int), m->stream);
         return lp_fail(err, B200_ERR_OPERATION_FAILED, "b200_step: tensor-core GEMM wait gave up (code " + std::to_string(code) + "): results discarded");
     }
     if (n_want > 0 && logits_out) memcpy(logits_out, m->h_tc_err + HEAD_WORDS, (size_t)n_want * p.vocab * 4);
