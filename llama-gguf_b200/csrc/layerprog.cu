@@ -701,6 +701,8 @@ __global__ void lp_attn_prep_kernel(StepMeta sm, AttnGeom a, const float* __rest
 // Short rows (dim and vdim up to 128): every warp brings its blocks' rows through a ring of 4 KB chunks in shared memory (eight rows of keys or values,
 // 16-byte cp.async), as many in flight as the ring has room for: a block of 32 keys is eight of them.  With loads into registers a block of 32 keys was
 // eight trips to memory one after the other (110 keys, one row of 16 heads: 24 -> 7 us).  The same sums in the same order.
+// With fused_prep the position's own key and value go into the ring from shared memory: a copy past L1 does not wait for the block's
+// stores to the cache row, and read what the row held before.
 constexpr int ATT_RING = 48, ATT_CHUNK = 8 * 128;   // chunks of 8 rows x 128 floats: 192 KB
 __device__ __forceinline__ void att_wait(int n) {    // at most n newest groups still in flight
     switch (n) {
@@ -734,6 +736,9 @@ __global__ void __launch_bounds__(32 * ATT_WARPS) lp_window_attn_kernel(StepMeta
     const float* vc = a.v_in_k ? kc : kc + (size_t)a.cap * a.G * a.dim;
     const int ldk = a.G * a.dim, ldv = a.v_in_k ? ldk : a.G * a.vdim, gv = g * (a.v_in_k ? a.dim : a.vdim);
     const float* kinv = a.k_inv ? kc + (size_t)a.cap * ldk + g : nullptr;
+    float* own_k = smem + ring_at + ATT_RING * ATT_CHUNK;      // [dim], then the value [vdim] (ring and fused_prep only)
+    float* own_v = own_k + a.dim;
+    const bool ring_own = VCH == 4 && ring_at > 0 && a.fused_prep;
     if (a.fused_prep) {
         // what lp_attn_prep_kernel does, for this head and its K/V group only: warp 0 norms q into shared memory, warp 1 norms k
         // into the cache row of this position, the other warps copy v there.  Every head of a group writes the same values; a
@@ -750,10 +755,18 @@ __global__ void __launch_bounds__(32 * ATT_WARPS) lp_window_attn_kernel(StepMeta
                 ss = wsum(ss);
                 inv = 1.0f / sqrtf(ss / (float)a.dim + a.eps);
             }
-            for (int d = lane; d < a.dim; d += 32) dst[d] = a.qk_norm ? src[d] * inv * w[d] : src[d];
+            for (int d = lane; d < a.dim; d += 32) {
+                const float y = a.qk_norm ? src[d] * inv * w[d] : src[d];
+                dst[d] = y;
+                if (ring_own && warp) own_k[d] = y;
+            }
         } else {
             float* dst = const_cast<float*>(vc) + (size_t)i * ldv + g * a.vdim;
-            for (int c = threadIdx.x - 64; c < a.vdim; c += blockDim.x - 64) dst[c] = p[a.v_off + g * a.vdim + c];
+            for (int c = threadIdx.x - 64; c < a.vdim; c += blockDim.x - 64) {
+                const float y = p[a.v_off + g * a.vdim + c];
+                dst[c] = y;
+                if (ring_own) own_v[c] = y;
+            }
         }
         __threadfence_block();
     } else {
@@ -799,8 +812,11 @@ __global__ void __launch_bounds__(32 * ATT_WARPS) lp_window_attn_kernel(StepMeta
                 const size_t ld = val ? ldv : ldk;
                 if (d < (val ? a.vdim : a.dim)) {
 #pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        if (first + u < end) cp_async16(smem_u32(ring + (size_t)slot * ATT_CHUNK + u * 128 + d), src + (size_t)(first + u) * ld + d, 16u);
+                    for (int u = 0; u < 8; u++) {
+                        float* to = ring + (size_t)slot * ATT_CHUNK + u * 128 + d;
+                        if (ring_own && first + u == i) *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>((val ? own_v : own_k) + d);
+                        else if (first + u < end) cp_async16(smem_u32(to), src + (size_t)(first + u) * ld + d, 16u);
+                    }
                 }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
@@ -3387,7 +3403,7 @@ void attn_rows(LpModel* m, const StepMeta& sm, const AttnGeom& ag, const LayerPl
     int ring_at = 0;
     if (ag.dim % 4 == 0 && ag.vdim % 4 == 0 && ag.dim <= 128 && ag.vdim <= 128 && ag.kv_off % 16 == 0) {
         ring_at = (int)((asmem + 15) / 16 * 4);
-        asmem = (size_t)(ring_at + ATT_RING * ATT_CHUNK) * 4;
+        asmem = (size_t)(ring_at + ATT_RING * ATT_CHUNK + ag.dim + ag.vdim) * 4;
     }
     const int vch = ag.vdim <= 128 ? 4 : ag.vdim <= 256 ? 8 : 16;
 #define LP_ATTN(T, V) launch(m, lp_window_attn_kernel<T, V>, agrid, dim3(32 * ATT_WARPS), asmem, sm, ag, (const float*)m->qbuf, (const float*)m->P, L.n_in, L.qn, L.kn, (T*)m->act_a, ring_at)
