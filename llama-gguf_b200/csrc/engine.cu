@@ -2045,20 +2045,46 @@ static ExactRoom exact_room(const b200_ctx* c, int rows) {
     r.floats = r.part + r.part_floats;
     return r;
 }
-static bool exact_rows_room(b200_ctx* c, int n) {
-    const int cap = std::max(kExactFew, std::min(prefill_chunk(), c->d.max_seq_len)), rows = n <= kExactFew ? kExactFew : cap;
-    if (c->er_rows >= rows) return true;
+// What n rows (of a prompt, or of a step of n sequences) need beside the model; false: some of it finds no room, and the caller goes token by token
+static bool exact_rows_room(b200_ctx* c, int n, bool step) {
+    const int most = std::min(prefill_chunk(), c->d.max_seq_len), cap = std::max(kExactFew, most), rows = n <= kExactFew ? kExactFew : cap;
+    const bool logits = step && c->pf_logits_rows < n, tables = step && c->h_rows_bytes < (size_t)n * 24;
+    if (c->er_rows >= rows && c->pf_tok && c->pf_rows && !logits && !tables) return true;
     if (!c->er_retry.due()) return false;
-    exact_rows_free(c);
     const size_t tickets = (size_t)kExactFew * c->d.n_kv_heads * sizeof(unsigned int);
-    if (cudaMalloc((void**)&c->er_buf, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess || cudaMalloc((void**)&c->er_tickets, tickets) != cudaSuccess ||
-        cudaMemsetAsync(c->er_tickets, 0, tickets, c->stream) != cudaSuccess) {
-        cudaGetLastError();
+    auto take = [&] {
+        if (!c->pf_tok && cudaMalloc((void**)&c->pf_tok, most * sizeof(int)) != cudaSuccess) return false;
+        if (!c->pf_rows && cudaMalloc((void**)&c->pf_rows, (size_t)most * 24) != cudaSuccess) return false;
+        if (tables) {
+            uint8_t* h = nullptr;
+            if (cudaHostAlloc((void**)&h, (size_t)most * 24, cudaHostAllocDefault) != cudaSuccess) return false;
+            if (c->h_rows) cudaFreeHost(c->h_rows);
+            c->h_rows = h;
+            c->h_rows_bytes = (size_t)most * 24;
+        }
+        if (logits) {
+            float* l = nullptr;
+            if (cudaMalloc((void**)&l, (size_t)n * c->d.vocab * sizeof(float)) != cudaSuccess) return false;
+            cudaFree(c->pf_logits);
+            c->pf_logits = l;
+            c->pf_logits_rows = n;
+            drop_batch_graphs(c);      // (captured steps write the old ones)
+        }
+        if (c->er_rows >= rows) return true;
         exact_rows_free(c);
+        if (cudaMalloc((void**)&c->er_buf, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess || cudaMalloc((void**)&c->er_tickets, tickets) != cudaSuccess ||
+            cudaMemsetAsync(c->er_tickets, 0, tickets, c->stream) != cudaSuccess) {
+            exact_rows_free(c);
+            return false;
+        }
+        c->er_rows = rows;
+        return true;
+    };
+    if (!take()) {
+        cudaGetLastError();
         c->er_retry.failed();
         return false;
     }
-    c->er_rows = rows;
     c->er_retry.got();
     return true;
 }
@@ -2209,6 +2235,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     const int QKV = (nh + 2 * nkv) * hd;
     const int cap = std::min(prefill_chunk(), d.max_seq_len);
     const PromptRows place = prompt_rows(cap, kFewTokens, H, QKV, A, I);
+    if (exact && !exact_rows_room(c, std::min(n, cap), seqs != nullptr)) return kNoRoom;      // (all that it allocates)
     if (!c->pf_buf && !exact) CU_ALLOC(late_malloc(c, (void**)&c->pf_buf, place.floats * sizeof(float)));
     if (!c->pf_tok) CU_ALLOC(late_malloc(c, (void**)&c->pf_tok, cap * sizeof(int)));
     if (!c->pf_rows) CU_ALLOC(late_malloc(c, (void**)&c->pf_rows, (size_t)cap * 24));
@@ -2285,7 +2312,6 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             drop_batch_graphs(c);      // (the captured head GEMMs write the old buffer)
         }
     }
-    if (exact && !exact_rows_room(c, std::min(n, cap))) return kNoRoom;
     // CUDA graph of the step (rows mode): replay if this row count has one, capture on its second step (the first runs eagerly:
     // function attributes and lazy allocations happen there), and run the capture's graph to do the step itself
     struct CaptureGuard {
@@ -4175,10 +4201,12 @@ extern "C" int b200_decode_batch_greedy(b200_ctx* c, const int* seqs, const uint
             cudaFree(c->pf_argmax);
             c->pf_argmax = nullptr;
             c->pf_argmax_rows = 0;
-            CU_ALLOC(late_malloc(c, (void**)&c->pf_argmax, (size_t)n * sizeof(int)));
-            c->pf_argmax_rows = n;
+            const cudaError_t e = late_malloc(c, (void**)&c->pf_argmax, (size_t)n * sizeof(int));
+            if (e != cudaSuccess && as_gemm) CU_ALLOC(e);
+            if (e == cudaSuccess) c->pf_argmax_rows = n;
+            else cudaGetLastError();
         }
-        if ((rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs, !as_gemm)) != kNoRoom) {
+        if (c->pf_argmax && (rc = prefill_gemm(c, seqs[0], tokens, n, false, seqs, !as_gemm)) != kNoRoom) {
             if (rc) return rc;
             argmax_rows_kernel<<<n, 1024, 0, c->stream>>>(c->pf_logits, c->d.vocab, c->pf_argmax);
             c->launches++;

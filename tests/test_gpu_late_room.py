@@ -1,6 +1,7 @@
 """Batched decode steps of a context that finds no room on the device for what it has to allocate after loading.
 
-Tolerance: that of test_gpu_few_rows.py for rows of fp16 activations, 1e-3 of the largest logit."""
+Tolerance: that of test_gpu_few_rows.py for rows of fp16 activations, 1e-3 of the largest logit; rows in f32 (csrc/exact_rows.cuh) against token by token that of
+test_gpu_exact_rows.py, 1e-5, and without room for their buffers the bits of token by token."""
 import ctypes as C
 
 import numpy as np
@@ -14,6 +15,9 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-3
 synth.TINY["room"] = dict(synth.TINY["llama-tiny"], hidden=2048, n_layers=2, n_heads=16, n_kv_heads=4, ffn=4096, vocab=5000)
 ROWS = 256       # their logits are 5.1 MB
+# rows in f32 up to 32 sequences (no fp16 products of these blocks): the logits of 32 are 5.1 MB
+synth.TINY["room-f32"] = dict(synth.TINY["llama-tiny"], hidden=256, n_layers=2, n_heads=4, n_kv_heads=2, head_dim=64, ffn=352, vocab=40000)
+EXACT_TOL = 1e-5
 
 
 def model():
@@ -97,3 +101,76 @@ def test_buffers_of_few_rows_are_given_back(b200, monkeypatch):
     assert few_path not in launches["0"]
     for a, b in zip(out["1"], out["0"]):
         assert max(rel_err(x, y) for x, y in zip(a, b)) < TOL
+
+
+def exact_calls(b200, monkeypatch, desc, tensors, calls, fill=None):
+    """The calls with and without rows in f32; fill(k, blocks): before call k of the run with them."""
+    out, launches = {}, {}
+    for exact in ("0", "1"):
+        monkeypatch.setenv("B200_EXACT_ROWS", exact)
+        gpu = b200.GpuOnlyInference(desc, tensors)
+        blocks = []
+        try:
+            out[exact], launches[exact] = [], []
+            for k, call in enumerate(calls):
+                if exact == "1" and fill:
+                    fill(k, blocks)
+                before = gpu.stats()["kernel_launches"]
+                out[exact].append(call(gpu))
+                launches[exact].append(gpu.stats()["kernel_launches"] - before)
+        finally:
+            while blocks:
+                blocks.pop().free()
+            gpu.close()
+    return out, [a != b for a, b in zip(launches["1"], launches["0"])]      # (which calls took the rows)
+
+
+def step(n, k, vocab=5000, greedy=False):
+    t = np.random.default_rng([n, k]).integers(0, vocab, n).astype(np.uint32)
+    return lambda gpu: (gpu.decode_batch_greedy if greedy else gpu.decode_batch)(list(range(n)), t)
+
+
+def test_rows_in_f32_on_a_full_device(b200, monkeypatch):
+    """The first steps and prompts of several rows find no room: none for their logits.  They go sequence by sequence and token by token, with those bits; the rows come
+    when there is room."""
+    arch, desc, tensors = synth.synth_model("room-f32", "Q4_0", 96, max_batch=32)
+    prompt = lambda gpu: gpu.prefill(synth.prompt_tokens(9, desc["vocab"]), 31)  # noqa: E731
+
+    def alone(gpu):      # (graphs of single tokens, one per slot and kind, are made while there is room)
+        for s in range(32):
+            gpu.prefill_token(1, s)
+            gpu.decode_greedy(2, 1, s)
+        return np.array([gpu.forward(3, s) for s in range(32)])
+    calls = [alone, step(32, 0, 40000), step(32, 1, 40000, True), step(3, 2, 40000), prompt] + [step(32, 3 + k, 40000) for k in range(8)]
+
+    def fill(k, blocks):
+        if k == 1:
+            blocks.append(Full())
+        if k == 6:
+            blocks.pop().free()
+    out, rows = exact_calls(b200, monkeypatch, desc, tensors, calls, fill)
+    assert not any(rows[:3]) and all(rows[-4:]), rows      # (three rows may fit what is left)
+    for took, a, b in zip(rows, out["1"], out["0"]):
+        if took:
+            assert max(rel_err(x, y) for x, y in zip(np.atleast_2d(a), np.atleast_2d(b))) < EXACT_TOL
+        else:
+            assert np.array_equal(a, b)
+
+
+def test_buffers_of_rows_in_f32_are_given_back(b200, monkeypatch):
+    """Captured steps of seven sequences in f32; then 256 rows whose logits fit only where the buffers of the f32 rows were, seven on the full device, and seven with room again: a
+    step captured before names buffers that are gone and may not be replayed."""
+    monkeypatch.setenv("B200_FEW_GEMM", "0")          # (nothing else to give back)
+    arch, desc, tensors = model()
+    calls = [step(8, 0)] + [step(7, k) for k in (1, 2, 3)] + [step(ROWS, 4)] + [step(7, k) for k in range(5, 16)]
+
+    def fill(k, blocks):
+        if k in (4, 5):
+            blocks.append(Full())
+        if k == 6:
+            while blocks:
+                blocks.pop().free()
+    out, rows = exact_calls(b200, monkeypatch, desc, tensors, calls, fill)
+    assert all(rows[1:4]) and not any(rows[4:6]) and all(rows[-4:]), rows
+    for k, (a, b) in enumerate(zip(out["1"], out["0"])):
+        assert max(rel_err(x, y) for x, y in zip(a, b)) < (EXACT_TOL if 0 < k < 4 else TOL)      # (from 4 on they read cache rows of fp16 activations)
