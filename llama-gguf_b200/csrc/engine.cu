@@ -257,7 +257,7 @@ struct b200_ctx {
     float* er_buf = nullptr;
     unsigned int* er_tickets = nullptr;
     int er_rows = 0;
-    SpareRetry er_retry;
+    SpareRetry er_retry, er_tiles_retry;      // where there was no room for those of kExactFew rows, of more
     bool pf_tmaps_built = false;
     size_t pf_split_floats = 0;
     int pf_logits_rows = 0;
@@ -2050,7 +2050,8 @@ static bool exact_rows_room(b200_ctx* c, int n, bool step) {
     const int most = std::min(prefill_chunk(), c->d.max_seq_len), cap = std::max(kExactFew, most), rows = n <= kExactFew ? kExactFew : cap;
     const bool logits = step && c->pf_logits_rows < n, tables = step && c->h_rows_bytes < (size_t)n * 24;
     if (c->er_rows >= rows && c->pf_tok && c->pf_rows && !logits && !tables) return true;
-    if (!c->er_retry.due()) return false;
+    SpareRetry& retry = rows > kExactFew ? c->er_tiles_retry : c->er_retry;      // (a long prompt that finds no room says nothing of the short calls)
+    if (!retry.due()) return false;
     const size_t tickets = (size_t)kExactFew * c->d.n_kv_heads * sizeof(unsigned int);
     auto take = [&] {
         if (!c->pf_tok && cudaMalloc((void**)&c->pf_tok, most * sizeof(int)) != cudaSuccess) return false;
@@ -2071,21 +2072,32 @@ static bool exact_rows_room(b200_ctx* c, int n, bool step) {
             drop_batch_graphs(c);      // (captured steps write the old ones)
         }
         if (c->er_rows >= rows) return true;
-        exact_rows_free(c);
-        if (cudaMalloc((void**)&c->er_buf, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess || cudaMalloc((void**)&c->er_tickets, tickets) != cudaSuccess ||
-            cudaMemsetAsync(c->er_tickets, 0, tickets, c->stream) != cudaSuccess) {
-            exact_rows_free(c);
-            return false;
+        if (!c->er_tickets) {
+            unsigned int* t = nullptr;
+            if (cudaMalloc((void**)&t, tickets) != cudaSuccess) return false;
+            c->er_tickets = t;
+            if (cudaMemsetAsync(t, 0, tickets, c->stream) != cudaSuccess) {
+                exact_rows_free(c);
+                return false;
+            }
         }
+        float* b = nullptr;      // beside what there is, which short prompts and small steps keep when the larger one finds no room
+        if (cudaMalloc((void**)&b, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess) return false;
+        if (c->er_buf) {
+            cudaStreamSynchronize(c->stream);
+            drop_batch_graphs(c);
+            cudaFree(c->er_buf);
+        }
+        c->er_buf = b;
         c->er_rows = rows;
         return true;
     };
     if (!take()) {
         cudaGetLastError();
-        c->er_retry.failed();
+        retry.failed();
         return false;
     }
-    c->er_retry.got();
+    retry.got();
     return true;
 }
 

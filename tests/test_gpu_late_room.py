@@ -174,3 +174,18 @@ def test_buffers_of_rows_in_f32_are_given_back(b200, monkeypatch):
     assert all(rows[1:4]) and not any(rows[4:6]) and all(rows[-4:]), rows
     for k, (a, b) in enumerate(zip(out["1"], out["0"])):
         assert max(rel_err(x, y) for x, y in zip(a, b)) < (EXACT_TOL if 0 < k < 4 else TOL)      # (from 4 on they read cache rows of fp16 activations)
+
+
+def test_short_calls_keep_their_rows_when_a_long_prompt_finds_no_room(b200, monkeypatch):
+    arch, desc, tensors = synth.synth_model("room-f32", "Q4_0", 160, max_batch=32)
+    prompt = lambda n: lambda gpu: gpu.prefill(synth.prompt_tokens(n, desc["vocab"]), 30)  # noqa: E731
+    alone = lambda gpu: (gpu.prefill_token(1, 30), gpu.forward(2, 30))[1]  # noqa: E731
+    calls = [alone, step(3, 0, 40000), prompt(5), prompt(100), step(3, 1, 40000), prompt(7), step(3, 2, 40000), step(3, 3, 40000)]
+
+    def fill(k, blocks):
+        if k == 3:
+            blocks.append(Full())
+    out, rows = exact_calls(b200, monkeypatch, desc, tensors, calls, fill)
+    assert rows == [False, True, True, False, True, True, True, True]
+    for a, b in zip(out["1"], out["0"]):
+        assert max(rel_err(x, y) for x, y in zip(np.atleast_2d(a), np.atleast_2d(b))) < EXACT_TOL
