@@ -3172,8 +3172,10 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     if (R > m->cap_rows || n_want > m->cap_want || n_runs > m->cap_runs) m->scratch_epoch++;   // buffers or table offsets move: graphs are void
     const size_t es = elt(m);
     const int W = m->p.width;
+    // (a capacity is 0 while its buffers are replaced: when one finds no room, a smaller step after it grows them again and does not take them as they are)
     if (R > m->cap_rows) {
         const int cap = std::max(R, std::min(2 * m->cap_rows, 1 << 20));
+        m->cap_rows = 0;
         if ((rc = grow(m, &m->x, (size_t)cap * W * 4, err))) return rc;
         if (m->p.post_norm == B200_FORM_NORM_OUTPUT && (rc = grow(m, &m->x2, (size_t)cap * W * 4, err))) return rc;
         if ((rc = grow(m, &m->P, (size_t)cap * m->max_in * 4, err))) return rc;
@@ -3202,6 +3204,7 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     }
     if (n_want > m->cap_want) {
         const int cap = std::max(n_want, 2 * m->cap_want);
+        m->cap_want = 0;
         if ((rc = grow_logits(m, (size_t)cap * m->p.vocab * 4, err))) return rc;
         if ((rc = grow(m, &m->hw, (size_t)cap * W * es, err))) return rc;
         if ((rc = grow(m, &m->pick, (size_t)cap * 4, err))) return rc;
@@ -3212,6 +3215,7 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
     if (meta > m->meta_bytes) {
         if (m->h_meta) cudaFreeHost(m->h_meta);
         m->h_meta = nullptr;
+        m->meta_bytes = 0;
         LCU_ALLOC(cudaHostAlloc((void**)&m->h_meta, meta, cudaHostAllocDefault));
         if ((rc = grow(m, &m->d_meta, meta, err))) return rc;
         m->meta_bytes = meta;
@@ -4184,6 +4188,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
     if (m->taps_on) {
         const size_t need = (size_t)m->runs.size() * lens[0] * W;
         if (need > m->taps_floats) {
+            m->taps_floats = 0;
             if ((rc = grow(m, &m->taps, need * 4, err))) return rc;
             m->taps_floats = need;
         }

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 import torch
 
+import lazilorn_synth
 import synth
 from synth import rel_err
 
@@ -189,3 +190,32 @@ def test_short_calls_keep_their_rows_when_a_long_prompt_finds_no_room(b200, monk
     assert rows == [False, True, True, False, True, True, True, True]
     for a, b in zip(out["1"], out["0"]):
         assert max(rel_err(x, y) for x, y in zip(np.atleast_2d(a), np.atleast_2d(b))) < EXACT_TOL
+
+
+def test_a_layer_program_after_a_step_that_found_no_room(b200):
+    """300 rows' logits (24 MB) find no room: the step fails, and smaller ones after it, on the full device and with room again, give what they give without it."""
+    cfg = lazilorn_synth.config([lazilorn_synth.parallel_layer(), lazilorn_synth.delta_layer(ff=80)], vocab=20000)
+    w = lazilorn_synth.random_weights(cfg, 1)
+    toks = [int(t) for t in np.random.default_rng(1).integers(0, cfg["vocab"], 310)]
+    out = []
+    for full in (False, True):
+        gpu = lazilorn_synth.gpu_model(cfg, w, "float32", max_seq_len=320)
+        try:
+            got = [gpu.step([(0, toks[:300])], [299]), gpu.step([(0, [toks[300]])], [0])]
+            if full:
+                gpu.step([(1, toks[:3])], [2])
+                block = Full()
+                try:
+                    with pytest.raises(b200.AllocationFailed):
+                        gpu.step([(1, toks[:300])], list(range(300)))
+                    got.append(gpu.step([(0, [toks[301]])], [0]))
+                finally:
+                    block.free()
+            else:
+                got.append(gpu.step([(0, [toks[301]])], [0]))
+            got += [gpu.step([(0, toks[302:306])], [0, 1, 2, 3]), gpu.step([(0, [toks[306]])], [0])]
+            out.append(got)
+        finally:
+            gpu.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
