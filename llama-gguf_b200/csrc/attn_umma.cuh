@@ -39,9 +39,6 @@ struct AttnUmmaParams {
     int* err;
 };
 
-// query rows per token of a block's 128: the heads of a kv head, up to the next power of two
-__host__ __device__ __forceinline__ int attn_umma_slots(int G) { return G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8; }
-
 // fp16 hi / lo pairs of one layer's cache rows 0 .. kv_end-1 (zero up to kv_pad): K16[kv][pos][hd] and the transpose
 // Vt16[kv][hd][pos]; hi = fp16(x), lo = fp16(x - hi); the lo halves follow the hi halves (rows n_kv * P ... / n_kv * hd ...).
 // grid (kv_pad / 64, n_kv), 256 threads; HD = 64 or 128.
@@ -150,7 +147,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
         return;
     }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int G = p.G, GS = attn_umma_slots(G), TQ = 128 / GS;
+    const int G = p.G, TQ = 128 / G;
     const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;   // heavy (late) query tiles first
     const int kh = blockIdx.y, t0 = qt * TQ;
     const uint32_t bars = base + SM::BAR_AT, s_tmem = bars + 120u;
@@ -280,10 +277,9 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
             __syncwarp();
         }
     } else {
-        // threads t and t + 128 share query row t & 127 (TMEM lane t & 127): row r = (token t0 + r / GS, head kh * G + r % GS); they split every tile's 64
-        // keys and the head dimension.  Rows of slots above G repeat the last head and store nothing
-        const int r = tid & 127, half = tid >> 7, tq = t0 + r / GS, g = min(r % GS, G - 1);
-        const bool live = tq < p.T && r % GS < G;
+        // threads t and t + 128 share query row t & 127 (TMEM lane t & 127): row r = (token t0 + r / G, head kh * G + r % G); they split every tile's 64
+        // keys and the head dimension
+        const int r = tid & 127, half = tid >> 7, tq = t0 + r / G, g = r % G;
         {   // Q row, f32 -> fp16 hi / lo, swizzled K-major; each thread of the pair converts half of the row's 16-byte chunks
             const float* qrow = p.qkv + (size_t)min(tq, p.T - 1) * p.ld + (size_t)(kh * G + g) * HD;
 #pragma unroll
@@ -393,7 +389,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 1) prefill_attn_umma_kernel(co
         for (int c0 = 0; c0 < HD / 2; c0 += 32) {
             uint32_t v[32];
             au_ld32(v, tO + lanes + (uint32_t)(half * (HD / 2) + c0));
-            if (live) {
+            if (tq < p.T) {
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     uint32_t w[4];
@@ -435,9 +431,11 @@ inline bool attn_umma_encode(Umma2EncodeFn encode, const __half* k16, const __ha
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Other numbers of heads per kv head keep an f32 attention (rows_attn_kernel): padded to the next power of two they would run here too, but with probabilities and values as
+// pairs of fp16 in one accumulator over all keys, 2.8e-6 of the logits at 1000 keys for its 4e-7.
 inline bool attn_umma_ok(int hd, int n_heads, int n_kv) {
     const int G = n_kv > 0 ? n_heads / n_kv : 0;
-    return (hd == 64 || hd == 128) && n_kv > 0 && n_heads % n_kv == 0 && G >= 1 && G <= 8;
+    return (hd == 64 || hd == 128) && n_kv > 0 && n_heads % n_kv == 0 && (G == 1 || G == 2 || G == 4 || G == 8);
 }
 
 template <int HD>
@@ -450,7 +448,7 @@ inline cudaError_t attn_umma_launch_hd(const CUtensorMap& kmap, const CUtensorMa
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) once[dev] = true;
     }
-    const int TQ = 128 / attn_umma_slots(p.G);
+    const int TQ = 128 / p.G;
     dim3 grid((p.T + TQ - 1) / TQ, p.n_kv);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = dim3(kAttnTcThreads); cfg.dynamicSmemBytes = AttnUmmaSmem<HD>::BYTES; cfg.stream = st;

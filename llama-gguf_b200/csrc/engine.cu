@@ -847,6 +847,8 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         CU(cudaFuncSetAttribute(rows_tile_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsTileSmem<8>));
         CU(cudaFuncSetAttribute(rows_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<128>));
         CU(cudaFuncSetAttribute(rows_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<64>));
+        CU(cudaFuncSetAttribute(rows_attn_kernel<128, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<128>));
+        CU(cudaFuncSetAttribute(rows_attn_kernel<64, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<64>));
         for (auto k : {attn_rows_kernel<128, 4>, attn_rows_kernel<128, 8>, attn_rows_kernel<64, 4>, attn_rows_kernel<64, 8>}) CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
     }
     c->finalized = true;
@@ -2381,6 +2383,15 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
     // rows.  glu: ws = {gate, up}, the unit silu(gate) up -> fp16 y.  cudaErrorNotSupported: the driver refused a tensor map (B200_PROMPT_F16_MAPS=0: as
     // if it did), nothing has been computed, and the caller takes the fused products.
     const bool f16_maps = env_int("B200_PROMPT_F16_MAPS", 1) != 0;
+    // prompts whose heads per kv head the tensor-core attention does not take: f32 tiles of 64 rows and keys (B200_PREFILL_ATTN_TC=0: a warp per token and kv head)
+    const bool attn_f32 = !rows && !exact && c->pf_attn_tc && !attn_umma_ok(hd, nh, nkv);
+    auto rows_attn = [&](const float* kc, const float* vc, int pos0, int T) -> cudaError_t {
+        RowsAttn ra{};
+        ra.qkv = Q; ra.ld = QKV; ra.k_cache = kc; ra.v_cache = vc; ra.out = ATh; ra.ldo = A; ra.pos0 = pos0; ra.T = T;
+        ra.n_heads = nh; ra.n_kv = nkv; ra.max_seq = d.max_seq_len; ra.scale = 1.0f / sqrtf((float)hd);
+        return launch_on(st, pdl, hd == 128 ? rows_attn_kernel<128, __half> : rows_attn_kernel<64, __half>, dim3((unsigned)(((long long)T * (nh / nkv) + 63) / 64), nkv), dim3(128),
+                         hd == 128 ? kRowsAttnSmem<128> : kRowsAttnSmem<64>, ra);
+    };
     auto gemm16 = [&](std::initializer_list<const DevTensor*> ws, int K, const __half* x, int ldx, int T, void* y, int ldy, const float* bias, int epi) -> cudaError_t {
         const bool glu = epi == tc16::EPI_SILU_GLU;
         long long total = 0;
@@ -2534,6 +2545,9 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                         CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, pdl, st));
                     }
                     c->launches += 2;
+                } else if (attn_f32) {
+                    CU(rows_attn(kc, vc, pos0, T));
+                    c->launches++;
                 } else {
                     PrefillAttnParams ap{};
                     ap.qkv = Q; ap.ld = QKV; ap.k_cache = kc; ap.v_cache = vc; ap.out = ATh; ap.ldo = A; ap.pos0 = pos0; ap.T = T;
@@ -2617,6 +2631,8 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                     CU(attn_umma_launch_hd<64>(c->pf_kmap, c->pf_vmap, up, pdl, st));
                 }
                 c->launches += 1;
+            } else if (attn_f32) {
+                CU(rows_attn(kc, vc, pos0, T));
             } else {
                 const int ablocks = (int)(((long long)T * nkv * 32 + 127) / 128);
                 const int Gq = nh / nkv;

@@ -624,7 +624,7 @@ struct RowsAttn {
     const float* qkv;      // [T][ld], q rotated
     const float* k_cache;  // [n_kv][max_seq][HD], positions 0 .. pos0 + T - 1 valid
     const float* v_cache;
-    float* out;            // [T][ldo]
+    void* out;             // [T][ldo] of OutT
     int ld, ldo, pos0, T, n_heads, n_kv, max_seq;
     float scale;
 };
@@ -633,8 +633,10 @@ template <int HD> constexpr int kRowsAttnSmem = (3 * 64 * HD + 64 * 64) * 4;
 // Causal GQA attention in f32 (attention_cached, cpu/ops.rs:1479-1537, over the rows of a prompt): a block owns 64 query rows (token, head of one kv head), walks
 // the keys 64 at a time with an online softmax; scores and sums as rows_tile_kernel's tiles, 8 keys (HD / 8 channels) x 4 rows per thread.  The tensor-core
 // attention of fp16 pairs adds all keys into one accumulator that cuts its sums off: 2.8e-6 of the logits at 1000 keys, against 4e-7 here (sums of 64 keys, then of tiles).
+// OutT = __half: prompts with fp16 products whose heads per kv head are no power of two (attn_umma_ok); prompts of 33, 333, 900, 4000 tokens through
+// two layers of 14 heads of 64 over 2: 200, 353, 574, 3080 us, with a warp per token and kv head (prefill_attn_kernel) 215, 600, 1358, 16475, with the padded pairs of fp16 186, 236, 298, 913.
 // grid (ceil(T G / 64), n_kv), the blocks with the most keys first.
-template <int HD>
+template <int HD, typename OutT = float>
 __global__ void __launch_bounds__(128) rows_attn_kernel(const RowsAttn p) {
     extern __shared__ __align__(16) float rows_attn_smem[];
     float *qs = rows_attn_smem, *ks = qs + 64 * HD, *vs = ks + 64 * HD, *ps = vs + 64 * HD;      // [HD][64 rows], [HD][64 keys], [64 keys][HD], [64 keys][64 rows]
@@ -769,12 +771,16 @@ __global__ void __launch_bounds__(128) rows_attn_kernel(const RowsAttn p) {
         for (int w = 1; w < 8; w <<= 1) l[t] += __shfl_xor_sync(0xffffffffu, l[t], w);
         const int r = r0 + 4 * ty + t;
         if (r >= n_rows) continue;
-        float* out = p.out + (size_t)(r / G) * p.ldo + (size_t)(kh * G + r % G) * HD;
+        OutT* out = reinterpret_cast<OutT*>(p.out) + (size_t)(r / G) * p.ldo + (size_t)(kh * G + r % G) * HD;
         const float inv = 1.0f / l[t];
 #pragma unroll
         for (int i = 0; i < HD / 32; i++) {
             const float2 a = f2_unpack(o[2 * i][t]), b = f2_unpack(o[2 * i + 1][t]);
-            *reinterpret_cast<float4*>(out + 32 * i + 4 * tx) = make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+            if constexpr (sizeof(OutT) == 4) *reinterpret_cast<float4*>(out + 32 * i + 4 * tx) = make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+            else {
+                const __half2 lo = __halves2half2(f2h_sat(a.x * inv), f2h_sat(a.y * inv)), hi = __halves2half2(f2h_sat(b.x * inv), f2h_sat(b.y * inv));
+                *reinterpret_cast<uint2*>(out + 32 * i + 4 * tx) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
         }
     }
 }

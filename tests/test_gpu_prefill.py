@@ -121,3 +121,43 @@ def test_tensor_core_prefill_attention_with_peaked_softmax(b200, oracle, preset,
     # wider weights also widen the fp16 GEMMs' own error (it can pass 1e-3 here with either attention kernel): the claims are that the
     # two attention kernels agree within the bound and that the tensor-core one is no further from the oracle than the CUDA-core one
     assert e_ab < TOL and e_tc < max(TOL, 1.25 * e_simt)
+
+
+@pytest.mark.parametrize("heads,kv,hd,lens", [(6, 2, 128, (45, 100)), (10, 2, 128, (64, 33)), (12, 2, 64, (333,)), (14, 2, 128, (130, 37)), (12, 4, 64, (200,))])
+def test_heads_per_kv_head_beside_the_powers_of_two(b200, oracle, monkeypatch, heads, kv, hd, lens):
+    """Three, five, six and seven query heads per kv head: prompts keep f32 attention (csrc/exact_rows.cuh, rows_attn_kernel<HD, __half>), no fp16 copies of keys and values: as many
+    launches as with a warp per token (B200_PREFILL_ATTN_TC=0).  Peaked softmax, ragged last tiles of rows, a second portion.  Bounds as above: the two f32 attentions differ in
+    the last place, which moves fp16 operands behind them."""
+    n = sum(lens)
+    monkeypatch.setitem(synth.TINY, "heads-odd", dict(synth.TINY["llama-tiny"], hidden=512, n_layers=2, n_heads=heads, n_kv_heads=kv, head_dim=hd, ffn=768, vocab=300))
+    arch, desc, tensors = synth.synth_model("heads-odd", "Q4_K_M", n + 8, sigma=0.05)
+    prompt = synth.prompt_tokens(n, desc["vocab"])
+    want = oracle.OracleModel(desc, tensors).forward(prompt)
+    got, launches = {}, {}
+    for tc in ("1", "0"):
+        monkeypatch.setenv("B200_PREFILL_ATTN_TC", tc)
+        gpu = b200.GpuOnlyInference(desc, tensors)
+        at = 0
+        for k in lens:
+            got[tc] = gpu.prefill(prompt[at:at + k])
+            at += k
+        launches[tc] = gpu.stats()["kernel_launches"]
+        gpu.close()
+    e, e_warp, e_ab = rel_err(got["1"], want), rel_err(got["0"], want), rel_err(got["1"], got["0"])
+    print(f"{heads} heads over {kv}: tiles vs oracle {e:.2e}, a warp per token {e_warp:.2e}, tiles vs warps {e_ab:.2e}")
+    assert launches["1"] == launches["0"], launches
+    assert e_ab < TOL and e < max(TOL, 1.25 * e_warp)
+
+
+@pytest.mark.parametrize("heads", [6, 14])
+def test_int8_prompts_of_such_heads_go_token_by_token(b200, monkeypatch, heads):
+    """B200_KV_INT8_GEMM=1 asks for the pass with the tensor-core attention; these heads have none."""
+    monkeypatch.setitem(synth.TINY, "heads-odd", dict(synth.TINY["llama-tiny"], hidden=512, n_layers=2, n_heads=heads, n_kv_heads=2, head_dim=128, ffn=768, vocab=300))
+    arch, desc, tensors = synth.synth_model("heads-odd", "Q4_K_M", 64)
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("B200_KV_INT8_GEMM", on)
+        gpu = b200.GpuOnlyInference(desc, tensors, kv_format="int8")
+        out.append(gpu.prefill(synth.prompt_tokens(40, desc["vocab"])))
+        gpu.close()
+    assert np.array_equal(*out)
