@@ -510,6 +510,8 @@ B200_API int b200_debug_mega_phase(b200_ctx* ctx, int phase, unsigned long long*
 B200_API int b200_debug_err(b200_ctx* ctx, int* out8);
 /* Host logic of the dequant-GEMM's split-K planners (no device needed): K range per split, 0 = unsplit. */
 B200_API int b200_debug_plan_split(int n_rows, int K, int T, int n_sm, int persistent, int* k_split_out);
+/* Host logic of the fp16 products' plan (no device needed): out4 = persistent, tokens per tile, cuts of K, pairs of CTAs. */
+B200_API int b200_debug_tc_plan(int rows, int n, int k, int glu, int may_cut, int pairs, int* out4);
 /* The RMS norm of a prompt's rows to fp16 [rows][n] (tests): the kernel that rows of n elements take, or the one for any length. */
 B200_API int b200_debug_prompt_norm(const float* x, const float* w, float eps, int rows, int n, int any_length, uint16_t* out);
 /* Lab: take the first `pos` positions of the slot's KV cache as valid as they are (attention at depth without a prompt). */

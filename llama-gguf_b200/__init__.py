@@ -226,6 +226,7 @@ def lib():
     L.b200_ctx_speculation_stats.argtypes = [vp, i32p, u64p, u64p]
     L.b200_debug_set_position.argtypes = [vp, C.c_int, C.c_uint64]
     L.b200_debug_plan_split.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, i32p]
+    L.b200_debug_tc_plan.argtypes = [C.c_int] * 6 + [i32p]
     L.b200_debug_prompt_norm.argtypes = [fp, fp, C.c_float, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_uint16)]
     L.b200_decode_batch_greedy.argtypes = [vp, C.POINTER(C.c_int), C.POINTER(C.c_uint32), C.c_int, C.POINTER(C.c_uint32)]
     L.b200_batch_create.argtypes = [vp, C.POINTER(BatchConfig), C.POINTER(vp)]
@@ -549,6 +550,13 @@ def plan_split(n_rows, K, T, n_sm=148, persistent=True):
     v = C.c_int(0)
     _check(lib().b200_debug_plan_split(int(n_rows), int(K), int(T), int(n_sm), 1 if persistent else 0, C.byref(v)))
     return v.value
+
+
+def tc_plan(rows, n, k, glu=False, may_cut=True, pairs=1):
+    """(persistent, tokens per tile, cuts of K, pairs of CTAs) of the fp16 product rows x n x k: host logic, no device needed."""
+    v = (C.c_int * 4)()
+    _check(lib().b200_debug_tc_plan(int(rows), int(n), int(k), 1 if glu else 0, 1 if may_cut else 0, int(pairs), v))
+    return tuple(v)
 
 
 def prompt_norm(x, w, eps, any_length=False):

@@ -4533,6 +4533,14 @@ extern "C" int b200_debug_plan_split(int n_rows, int K, int T, int n_sm, int per
     return B200_OK;
 }
 
+// Host logic of the fp16 products' plan (gemm_tc.cuh), callable without a device (tests): out = persistent, tokens per tile, cuts of K, pairs of CTAs.
+extern "C" int b200_debug_tc_plan(int rows, int n, int k, int glu, int may_cut, int pairs, int* out4) {
+    if (!out4 || rows <= 0 || n <= 0 || k <= 0) return fail(B200_ERR_INVALID_ARGUMENT, "b200_debug_tc_plan: bad argument");
+    const tc16::TcPlan p = tc16::tc_plan(rows, n, k, 1, 0, false, glu != 0, may_cut != 0, false, pairs);
+    out4[0] = p.persistent; out4[1] = p.tn; out4[2] = p.splits; out4[3] = p.pair;
+    return B200_OK;
+}
+
 // The norm of a prompt's rows before its fp16 products (tests): the kernel that rows of n elements take, or the one for rows of any length; out: fp16 [rows][n].
 extern "C" int b200_debug_prompt_norm(const float* x, const float* w, float eps, int rows, int n, int any_length, uint16_t* out) {
     int rc;

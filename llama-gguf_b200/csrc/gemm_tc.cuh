@@ -742,7 +742,9 @@ bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts,
 // split: K may be cut over a cluster.  Without, every sum adds its products in the order of K, so that a row's result is the same bits whatever the number of
 // rows of the step.
 // rows: token rows as M (lp_gemm_tc_rows_kernel), tn weight rows per CTA: for sums that may not be cut (a cut over a cluster is as fast), up to 128 rows
-// pair: two CTAs per tile (lp_gemm_tc_kernel)
+// pair: two CTAs per tile (lp_gemm_tc_kernel), where the single CTAs would not cut K either: a pair adds all of K in one accumulator of tensor memory, which cuts its sums off,
+// so in place of a cut it gives other bits and a larger error: 4096 x 700 x 14336 in two cuts, one 8B layer over 24 inputs, 1.0002 +- 0.0001 (Q4_K_M) and 1.0009 +- 0.0001 (Q8_0, 645
+// rows) times the distance to float64.  (Time: two 8B layers of 700 rows 910 us with pairs there, 1024 without.)
 struct TcPlan {
     bool persistent;
     int tn, splits;
@@ -767,11 +769,11 @@ TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, b
         const long long waves = (tiles(tn) + n_sm - 1) / n_sm;
         offer(true, tn, 1, waves * steps * (tn == 256 ? 750 : 470) + 17 * tn);
     }
+    long long pair_cost = -1;
     if (pairs && R > 128) {
         const long long two = (long long)((n_mt + 1) / 2) * (seg ? xrows / 256 + (groups + 1) / 2 : groups * ((R + 255) / 256)), waves = (two + n_sm / 2 - 1) / (n_sm / 2);
-        const long long cost = waves * steps * 680 + 17 * 256 + 3000;
-        if (cost < least || pairs == 2) { least = cost; best = TcPlan{true, 256, 1, false, true}; }
-        if (pairs == 2) return best;
+        pair_cost = waves * steps * 680 + 17 * 256 + 3000;
+        if (pairs == 2) return TcPlan{true, 256, 1, false, true};
     }
     for (int tn : {128, 64}) {
         if (tn == 128 && R <= 64) continue;
@@ -781,5 +783,6 @@ TcPlan tc_plan(int R, int N, int K, int groups, int xrows, bool seg, bool glu, b
             offer(false, tn, s, waves * ((steps + s - 1) / s * (tn == 128 ? 470 : 375) + 4500) - 4500 + 18 * tn + (s > 1 ? 1000 : 0));
         }
     }
+    if (pair_cost >= 0 && best.splits == 1 && pair_cost < least) return TcPlan{true, 256, 1, false, true};
     return best;
 }
