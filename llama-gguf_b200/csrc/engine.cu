@@ -252,12 +252,12 @@ struct b200_ctx {
     uint8_t* few_img[3] = {};        // images of the activations: normed rows, attention, gated units
     float* few_part = nullptr;       // pieces of cut tiles
     SpareRetry few_retry;            // ... where there was no room for these
-    // products of several rows in f32 (exact_rows.cuh): activations, pieces of cut products, attention partials and tickets of up to er_rows rows
+    // products of several rows in f32 (exact_rows.cuh): activations, pieces of cut products, attention partials
     bool exact_rows = true;          // B200_EXACT_ROWS=0: such prompts and steps token by token
-    float* er_buf = nullptr;
+    float* er_few = nullptr;         // of up to kExactFew rows: made with the context, kept
+    float* er_tiles = nullptr;       // of a chunk's rows: made by the first longer prompt, given back (late_malloc)
     unsigned int* er_tickets = nullptr;
-    int er_rows = 0;
-    SpareRetry er_retry, er_tiles_retry;      // where there was no room for those of kExactFew rows, of more
+    SpareRetry er_retry, er_tiles_retry;      // where there was no room for them
     bool pf_tmaps_built = false;
     size_t pf_split_floats = 0;
     int pf_logits_rows = 0;
@@ -693,6 +693,7 @@ static int check_f32_vec(const DevTensor& t, const char* what, uint64_t n, int l
     return B200_OK;
 }
 
+static void exact_rows_at_load(b200_ctx* c);
 extern "C" int b200_ctx_finalize(b200_ctx* c) {
     if (!c) return fail(B200_ERR_INVALID_ARGUMENT, "b200_ctx_finalize: null ctx");
     if (c->finalized) return B200_OK;
@@ -864,6 +865,7 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         c->finalized = false;
         return fail(B200_ERR_UNSUPPORTED, "tensor parallelism needs the megakernel path (dense model, K-quant / Q8_0 weights with 256-aligned shards)");
     }
+    exact_rows_at_load(c);
     // What was cleared and copied above went through the legacy stream, which orders nothing on c->stream (non-blocking); with work of the process before it there (torch's
     // default stream) none of it may have happened yet.  Later calls clear and copy on c->stream
     CU(cudaStreamSynchronize(cudaStreamLegacy));
@@ -962,7 +964,8 @@ extern "C" void b200_ctx_destroy(b200_ctx* c) {
     cudaFree(c->pf_tmaps);
     for (uint8_t* p : c->few_img) cudaFree(p);
     cudaFree(c->few_part);
-    cudaFree(c->er_buf);
+    cudaFree(c->er_few);
+    cudaFree(c->er_tiles);
     cudaFree(c->er_tickets);
     cudaFree(c->pf_tile_cnt);
     cudaFree(c->attn_q8_part);
@@ -1061,27 +1064,16 @@ static void drop_batch_graphs(b200_ctx* c) {
     }
 }
 
-static void exact_rows_free(b200_ctx* c) {
-    if (c->er_buf) {
-        cudaStreamSynchronize(c->stream);
-        drop_batch_graphs(c);
-    }
-    cudaFree(c->er_buf);
-    cudaFree(c->er_tickets);
-    c->er_buf = nullptr;
-    c->er_tickets = nullptr;
-    c->er_rows = 0;
-}
-
-// Device memory that a call after loading has to have: the prompts' fp16 weight rows, the buffers of the products of few rows and those of the f32 rows, which the
-// calls can do without, go first when there is no room (and with the latter two the captured steps that name them).  Never called inside a capture
+// Device memory that a call after loading has to have: the prompts' fp16 weight rows, the buffers of the products of few rows and those of long prompts in f32, which the
+// calls can do without, go first when there is no room (and with the second the captured steps that name them).  Never called inside a capture
 static cudaError_t late_malloc(b200_ctx* c, void** p, size_t bytes) {
     return (cudaError_t)alloc_or_give_back(
         [&] { return (int)cudaMalloc(p, bytes); },
         [&] {
             cudaGetLastError();
-            if (!c->pf_w16 && !c->few_part && !c->er_buf) return false;
-            exact_rows_free(c);
+            if (!c->pf_w16 && !c->few_part && !c->er_tiles) return false;
+            cudaFree(c->er_tiles);      // (waits for what runs)
+            c->er_tiles = nullptr;
             cudaFree(c->pf_w16);
             c->pf_w16 = nullptr;
             c->pf_w16_elems = 0;
@@ -2026,12 +2018,11 @@ static bool exact_rows_ok(const b200_ctx* c, int n, bool prompt) {
 }
 
 struct ExactRoom {      // offsets in floats, for up to `rows` rows
-    size_t x, xn, qkv, at, act, part, floats, part_floats, attn_row;
+    size_t x, xn, qkv, at, act, part, floats, part_floats;
 };
 static ExactRoom exact_room(const b200_ctx* c, int rows) {
     const b200_model_desc& d = c->d;
     const size_t H = d.hidden, A = (size_t)d.n_heads * d.head_dim, I = (size_t)d.ffn, QKV = A + (size_t)2 * d.n_kv_heads * d.head_dim, n = rows;
-    const int G = d.n_heads / d.n_kv_heads;
     ExactRoom r{};
     auto up = [](size_t v) { return (v + 31) & ~(size_t)31; };
     r.x = 0;
@@ -2040,21 +2031,26 @@ static ExactRoom exact_room(const b200_ctx* c, int rows) {
     r.at = r.qkv + up(n * QKV);
     r.act = r.at + up(n * A);
     r.part = r.act + up(n * I);
-    // pieces of a product (two waves of 64 x 64 tiles, or one uncut), or the partial attention of few rows
-    const size_t widest = std::max({H, QKV, 2 * I});
-    r.attn_row = (size_t)d.n_kv_heads * std::max(c->n_splits, c->attn_q8_splits) * G * (d.head_dim + 2);
-    r.part_floats = up(std::max(rows > kExactFew ? n * widest + (size_t)4 * c->n_sm * 64 * 128 : 0, kExactFew * r.attn_row));
+    // pieces of a product (two waves of 64 x 64 tiles, or one uncut), or the partial attention of few rows: rows times splits (exact_splits) at most 8 (int8) or one per row, or two
+    // blocks per SM and kv head
+    const size_t widest = std::max({H, QKV, 2 * I}), splits = std::max((size_t)kExactFew * (c->kv_format == 1 ? 8 : 1), (size_t)2 * c->n_sm / d.n_kv_heads);
+    r.part_floats = up(rows > kExactFew ? n * widest + (size_t)4 * c->n_sm * 64 * 128 : splits * d.n_heads * (d.head_dim + 2));
     r.floats = r.part + r.part_floats;
     return r;
 }
+// splits of the keys for T rows at once: two blocks per SM
+static int exact_splits(const b200_ctx* c, int T) {
+    const int two = 2 * c->n_sm / (c->d.n_kv_heads * T);
+    if (c->kv_format == 1) return std::max(std::min(8, c->attn_q8_splits), std::min(c->attn_q8_splits, two));
+    return std::max(1, std::min(c->n_splits, two));
+}
 // What n rows (of a prompt, or of a step of n sequences) need beside the model; false: some of it finds no room, and the caller goes token by token
 static bool exact_rows_room(b200_ctx* c, int n, bool step) {
-    const int most = std::min(prefill_chunk(), c->d.max_seq_len), cap = std::max(kExactFew, most), rows = n <= kExactFew ? kExactFew : cap;
-    const bool logits = step && c->pf_logits_rows < n, tables = step && c->h_rows_bytes < (size_t)n * 24;
-    if (c->er_rows >= rows && c->pf_tok && c->pf_rows && !logits && !tables) return true;
-    SpareRetry& retry = rows > kExactFew ? c->er_tiles_retry : c->er_retry;      // (a long prompt that finds no room says nothing of the short calls)
+    const int most = std::min(prefill_chunk(), c->d.max_seq_len);
+    const bool tiles = n > kExactFew, logits = step && c->pf_logits_rows < n, tables = step && c->h_rows_bytes < (size_t)n * 24;
+    if (c->er_few && c->er_tickets && (!tiles || c->er_tiles) && c->pf_tok && c->pf_rows && !logits && !tables) return true;
+    SpareRetry& retry = tiles ? c->er_tiles_retry : c->er_retry;      // (a long prompt that finds no room says nothing of the short calls)
     if (!retry.due()) return false;
-    const size_t tickets = (size_t)kExactFew * c->d.n_kv_heads * sizeof(unsigned int);
     auto take = [&] {
         if (!c->pf_tok && cudaMalloc((void**)&c->pf_tok, most * sizeof(int)) != cudaSuccess) return false;
         if (!c->pf_rows && cudaMalloc((void**)&c->pf_rows, (size_t)most * 24) != cudaSuccess) return false;
@@ -2073,26 +2069,18 @@ static bool exact_rows_room(b200_ctx* c, int n, bool step) {
             c->pf_logits_rows = n;
             drop_batch_graphs(c);      // (captured steps write the old ones)
         }
-        if (c->er_rows >= rows) return true;
         if (!c->er_tickets) {
+            const size_t bytes = (size_t)kExactFew * c->d.n_kv_heads * sizeof(unsigned int);
             unsigned int* t = nullptr;
-            if (cudaMalloc((void**)&t, tickets) != cudaSuccess) return false;
-            c->er_tickets = t;
-            if (cudaMemsetAsync(t, 0, tickets, c->stream) != cudaSuccess) {
-                exact_rows_free(c);
+            if (cudaMalloc((void**)&t, bytes) != cudaSuccess) return false;
+            if (cudaMemsetAsync(t, 0, bytes, c->stream) != cudaSuccess) {
+                cudaFree(t);
                 return false;
             }
+            c->er_tickets = t;
         }
-        float* b = nullptr;      // beside what there is, which short prompts and small steps keep when the larger one finds no room
-        if (cudaMalloc((void**)&b, exact_room(c, rows).floats * sizeof(float)) != cudaSuccess) return false;
-        if (c->er_buf) {
-            cudaStreamSynchronize(c->stream);
-            drop_batch_graphs(c);
-            cudaFree(c->er_buf);
-        }
-        c->er_buf = b;
-        c->er_rows = rows;
-        return true;
+        if (!c->er_few && cudaMalloc((void**)&c->er_few, exact_room(c, kExactFew).floats * sizeof(float)) != cudaSuccess) return false;
+        return !tiles || c->er_tiles || cudaMalloc((void**)&c->er_tiles, exact_room(c, most).floats * sizeof(float)) == cudaSuccess;
     };
     if (!take()) {
         cudaGetLastError();
@@ -2101,6 +2089,21 @@ static bool exact_rows_room(b200_ctx* c, int n, bool step) {
     }
     retry.got();
     return true;
+}
+// X of T rows
+static float* exact_x(const b200_ctx* c, int T) { return T <= kExactFew ? c->er_few : c->er_tiles; }
+
+// The buffers of up to kExactFew rows, a few MB, and the code of the kernels: a context's first short prompt pays for neither, and finds both when the device has filled up
+// since (steps still bring their logits).  Without room here, they are asked for again when they are needed
+static void exact_rows_at_load(b200_ctx* c) {
+    if (!exact_rows_ok(c, 2, true)) return;
+    cudaError_t e = rows_load();
+    cudaFuncAttributes a;
+    for (const void* f : {(const void*)prefill_embed_kernel, (const void*)prefill_rope_kv_kernel, (const void*)prefill_rope_kv_q8_kernel<4>, (const void*)prefill_rope_kv_q8_kernel<2>,
+                          (const void*)attn_q8_split_kernel<128, 4, true>, (const void*)attn_q8_split_kernel<64, 4, true>, (const void*)attn_q8_merge_kernel<true>,
+                          (const void*)prefill_advance_kernel, (const void*)prefill_advance_rows_kernel, (const void*)argmax_rows_kernel})
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, f);
+    if (e != cudaSuccess || !exact_rows_room(c, 2, false)) cudaGetLastError();
 }
 
 struct ExactPass {
@@ -2115,8 +2118,8 @@ struct ExactPass {
 static int exact_layers(b200_ctx* c, Slot& sl, const ExactPass& e) {
     const b200_model_desc& d = c->d;
     const int H = d.hidden, hd = d.head_dim, nh = d.n_heads, nkv = d.n_kv_heads, A = nh * hd, I = (int)d.ffn, QKV = (nh + 2 * nkv) * hd, T = e.T, G = nh / nkv;
-    const ExactRoom room = exact_room(c, c->er_rows);
-    float *X = c->er_buf + room.x, *XN = c->er_buf + room.xn, *Q = c->er_buf + room.qkv, *AT = c->er_buf + room.at, *HB = c->er_buf + room.act, *PT = c->er_buf + room.part;
+    const ExactRoom room = exact_room(c, T <= kExactFew ? kExactFew : std::min(prefill_chunk(), d.max_seq_len));
+    float *X = exact_x(c, T), *XN = X + room.xn, *Q = X + room.qkv, *AT = X + room.at, *HB = X + room.act, *PT = X + room.part;
     const size_t kv_layer = (size_t)2 * nkv * d.max_seq_len * hd, q8_rows = (size_t)2 * nkv * d.max_seq_len;
     const bool q8 = c->kv_format == 1, few = T <= kExactFew;
     const float scale = 1.0f / sqrtf((float)hd);
@@ -2176,7 +2179,7 @@ static int exact_layers(b200_ctx* c, Slot& sl, const ExactPass& e) {
             AttnQ8Params ap{};
             ap.q = Q; ap.k8 = k8; ap.v8 = v8; ap.k_scale = k8s; ap.v_scale = v8s; ap.part = PT; ap.out = AT; ap.pos0 = e.pos0; ap.ldq = QKV; ap.ldo = A;
             ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.scale = scale;
-            ap.n_splits = std::max(std::min(8, c->attn_q8_splits), std::min(c->attn_q8_splits, 2 * c->n_sm / (nkv * T)));      // (two blocks per SM)
+            ap.n_splits = exact_splits(c, T);
             ap.part_row = (long long)nkv * ap.n_splits * G * (hd + 2);
             CU(launch_on(e.st, e.pdl, hd == 128 ? attn_q8_split_kernel<128, 4, true> : attn_q8_split_kernel<64, 4, true>, dim3(ap.n_splits, nkv, T), dim3(kAttnQ8Warps * 32), 0, ap));
             CU(launch_on(e.st, e.pdl, attn_q8_merge_kernel<true>, dim3(nh, 1, T), dim3(kAttnQ8MergeThreads), 0, ap, hd));
@@ -2191,7 +2194,7 @@ static int exact_layers(b200_ctx* c, Slot& sl, const ExactPass& e) {
                 AttnParams ap{};
                 ap.q = Q; ap.k_cache = kc; ap.v_cache = vc; ap.out = AT; ap.part = PT; ap.tickets = c->er_tickets;
                 ap.n_kv = nkv; ap.G = G; ap.max_seq = d.max_seq_len; ap.scale = scale;
-                ap.n_splits = std::max(1, std::min(c->n_splits, 2 * c->n_sm / (nkv * T)));
+                ap.n_splits = exact_splits(c, T);
                 AttnRows ar{};
                 ar.ldq = QKV; ar.ldo = A; ar.pos0 = e.pos0; ar.part_row = (long long)nkv * ap.n_splits * G * (hd + 2);
                 if (e.rows) { ar.row_pos = e.d_pos; ar.row_kv = e.d_kv; ar.k_off = k_off; ar.v_off = v_off; }
@@ -2357,7 +2360,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
             bg.warm = true;
         }
     }
-    float* X = exact ? c->er_buf : c->pf_buf + place.x; // [T][H] residual stream (f32)
+    float* X = c->pf_buf + place.x;                     // [T][H] residual stream (f32); rows in f32: exact_x of the chunk's
     float* Q = c->pf_buf + place.qkv;                   // [T][QKV] f32
     float* G = c->pf_buf + place.gate;                  // [T][I] gate; few rows also [T][H], what X still lacks
     float* U = c->pf_buf + place.up;                    // [T][I] up
@@ -2467,6 +2470,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
         const int T = std::min(cap, n - done);
         const int pos0 = (int)sl.host_pos + done;
         last_T = T;
+        if (exact) X = exact_x(c, T);
         if (!rows) CU(cudaMemcpyAsync(c->pf_tok, tokens + done, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, st));
         CU(launch_on(st, pdl, prefill_embed_kernel, dim3(T, T <= 256 ? 4 : 1), dim3(T <= 256 ? 128 : 256), 0, c->token_embd.type, (const uint8_t*)c->token_embd.d, c->token_embd.row_bytes, H, (const int*)d_tok, d.vocab, X));
         if (exact) {

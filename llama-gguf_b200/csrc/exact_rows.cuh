@@ -848,21 +848,24 @@ inline int rows_few_tasks(const RowsParams& p, int R) {
     for (int s = 0; s < p.n_seg; s++) n += (p.seg[s].n_rows + R - 1) / R;
     return n;
 }
+template <int R, int TT> constexpr size_t kRowsFewSmem = (R * TT <= 16 ? 110 : 220) << 10;
 template <int R, int TT>
-inline cudaError_t rows_few_go(RowsParams& p, int n_sm, bool pdl, cudaStream_t st) {
-    // shared memory: all of K where two blocks' rows fit an SM (one block's from 32 sums per warp on), else 256s of it
-    constexpr size_t most = (R * TT <= 16 ? 110 : 220) << 10;
-    const int fit = (int)(most / (TT * sizeof(float)));
-    p.chunk = xpad_floats(p.K) <= fit ? p.K : (fit - 8) * 16 / 17 / 256 * 256;
-    const size_t smem = (size_t)TT * xpad_floats(p.chunk) * sizeof(float);
+inline cudaError_t rows_few_ready() {
     static bool once[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !once[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(rows_few_kernel<R, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) once[dev] = true;
-    }
+    if (dev >= 0 && dev < 64 && once[dev]) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(rows_few_kernel<R, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsFewSmem<R, TT>);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) once[dev] = true;
+    return e;
+}
+template <int R, int TT>
+inline cudaError_t rows_few_go(RowsParams& p, int n_sm, bool pdl, cudaStream_t st) {
+    // shared memory: all of K where two blocks' rows fit an SM (one block's from 32 sums per warp on), else 256s of it
+    const int fit = (int)(kRowsFewSmem<R, TT> / (TT * sizeof(float)));
+    p.chunk = xpad_floats(p.K) <= fit ? p.K : (fit - 8) * 16 / 17 / 256 * 256;
+    const size_t smem = (size_t)TT * xpad_floats(p.chunk) * sizeof(float);
+    if (const cudaError_t e = rows_few_ready<R, TT>()) return e;
     const int want = (rows_few_tasks(p, R) + kRowsWarps - 1) / kRowsWarps, groups = (p.T + TT - 1) / TT;
     const int per_sm = R * TT <= 16 && smem <= (size_t)(110 << 10) ? 2 : 1;
     cudaLaunchConfig_t cfg{};
@@ -876,6 +879,16 @@ inline cudaError_t rows_few_go(RowsParams& p, int n_sm, bool pdl, cudaStream_t s
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, rows_few_kernel<R, TT>, p);
+}
+// The kernels' code on the device (it is loaded at a kernel's first use, and a device that has filled up since has no room for it)
+inline cudaError_t rows_load() {
+    for (cudaError_t e : {rows_few_ready<4, 2>(), rows_few_ready<2, 2>(), rows_few_ready<1, 2>(), rows_few_ready<4, 4>(), rows_few_ready<2, 4>(), rows_few_ready<1, 4>(), rows_few_ready<4, 8>(),
+                          rows_few_ready<2, 8>(), rows_few_ready<1, 8>()})
+        if (e != cudaSuccess) return e;
+    cudaFuncAttributes a;
+    for (const void* f : {(const void*)rows_norm_kernel, (const void*)rows_qkv_kernel, (const void*)rows_swiglu_kernel})
+        if (const cudaError_t e = cudaFuncGetAttributes(&a, f)) return e;
+    return cudaSuccess;
 }
 inline cudaError_t rows_few_launch(RowsParams& p, int n_sm, bool pdl, cudaStream_t st) {
     // rounds of the chip's warps times a round's instructions: R weight columns to unpack and multiply, and the rows' x to load whatever R is.  4096 x 14336 with 3 rows: one

@@ -89,3 +89,20 @@ def test_steps_of_sequences(b200, monkeypatch, preset, mix, n):
         assert len(gpu.decode_batch_greedy(list(range(n)), steps[0])) == n
         return out
     assert max(both(b200, monkeypatch, desc, tensors, call)) < TOL
+
+
+@pytest.mark.parametrize("preset,mix,kv", [("qwen-tiny", "Q4_K_M", "int8"), ("llama-tiny", "Q4_K_M", "f32")])
+def test_first_short_prompt_allocates_nothing(b200, preset, mix, kv):
+    """The buffers of up to 32 rows come with the context."""
+    import torch
+    arch, desc, tensors = synth.synth_model(preset, mix, 64)
+    for _ in range(2):      # (kernels loaded)
+        gpu = b200.GpuOnlyInference(desc, tensors, kv_format=kv)
+        try:
+            before = gpu.stats()["kernel_launches"], torch.cuda.mem_get_info()[0]
+            gpu.prefill(synth.prompt_tokens(31, desc["vocab"]))
+            launches, free = gpu.stats()["kernel_launches"] - before[0], torch.cuda.mem_get_info()[0]
+        finally:
+            gpu.close()
+    assert launches < 31 * desc["n_layers"]      # (as rows)
+    assert free == before[1]

@@ -151,30 +151,32 @@ def test_rows_in_f32_on_a_full_device(b200, monkeypatch):
             blocks.pop().free()
     out, rows = exact_calls(b200, monkeypatch, desc, tensors, calls, fill)
     assert not any(rows[:3]) and all(rows[-4:]), rows      # (three rows may fit what is left)
-    for took, a, b in zip(rows, out["1"], out["0"]):
-        if took:
-            assert max(rel_err(x, y) for x, y in zip(np.atleast_2d(a), np.atleast_2d(b))) < EXACT_TOL
-        else:
+    for k, (a, b) in enumerate(zip(out["1"], out["0"])):
+        if not any(rows[:k + 1]):
             assert np.array_equal(a, b)
+        assert max(rel_err(x, y) for x, y in zip(np.atleast_2d(a), np.atleast_2d(b))) < EXACT_TOL
 
 
-def test_buffers_of_rows_in_f32_are_given_back(b200, monkeypatch):
-    """Captured steps of seven sequences in f32; then 256 rows whose logits fit only where the buffers of the f32 rows were, seven on the full device, and seven with room again: a
-    step captured before names buffers that are gone and may not be replayed."""
+def test_rows_in_f32_beside_calls_that_need_all_room(b200, monkeypatch):
+    """Captured steps of seven sequences and a long prompt in f32; then, on a full device, 256 rows whose logits fit only where the long prompt's buffers were.  The steps keep theirs and
+    replay; the next long prompt goes token by token until there is room."""
     monkeypatch.setenv("B200_FEW_GEMM", "0")          # (nothing else to give back)
+    monkeypatch.setenv("B200_PREFILL_GEMM_MIN", "1000")
     arch, desc, tensors = model()
-    calls = [step(8, 0)] + [step(7, k) for k in (1, 2, 3)] + [step(ROWS, 4)] + [step(7, k) for k in range(5, 16)]
+    prompt = lambda n: lambda gpu: gpu.prefill(synth.prompt_tokens(n, desc["vocab"]), 250)  # noqa: E731
+    alone = lambda gpu: (gpu.prefill_token(1, 250), gpu.forward(2, 250))[1]  # noqa: E731
+    calls = [alone, step(8, 0)] + [step(7, k) for k in (1, 2, 3)] + [prompt(50), step(ROWS, 4), step(7, 5), prompt(40), step(7, 6), prompt(9), prompt(36), prompt(35), prompt(34)]
 
     def fill(k, blocks):
-        if k in (4, 5):
+        if k in (6, 7):
             blocks.append(Full())
-        if k == 6:
+        if k == 10:
             while blocks:
                 blocks.pop().free()
     out, rows = exact_calls(b200, monkeypatch, desc, tensors, calls, fill)
-    assert all(rows[1:4]) and not any(rows[4:6]) and all(rows[-4:]), rows
+    assert rows[2:6] == [True] * 4 and rows[7:11] == [True, False, True, True] and rows[-1], rows
     for k, (a, b) in enumerate(zip(out["1"], out["0"])):
-        assert max(rel_err(x, y) for x, y in zip(a, b)) < (EXACT_TOL if 0 < k < 4 else TOL)      # (from 4 on they read cache rows of fp16 activations)
+        assert max(rel_err(x, y) for x, y in zip(np.atleast_2d(a), np.atleast_2d(b))) < (EXACT_TOL if k < 6 and k != 1 else TOL)      # (from 6 on they read cache rows of fp16 activations)
 
 
 def test_short_calls_keep_their_rows_when_a_long_prompt_finds_no_room(b200, monkeypatch):
