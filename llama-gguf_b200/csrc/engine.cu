@@ -258,6 +258,7 @@ struct b200_ctx {
     float* er_tiles = nullptr;       // of a chunk's rows: made by the first longer prompt, given back (late_malloc)
     unsigned int* er_tickets = nullptr;
     SpareRetry er_retry, er_tiles_retry;      // where there was no room for them
+    int tc_pair = 1;                 // B200_TC_PAIR=0: no pairs of CTAs in the two-pass products, 2: for all of more than 128 rows
     bool pf_tmaps_built = false;
     size_t pf_split_floats = 0;
     int pf_logits_rows = 0;
@@ -386,6 +387,7 @@ extern "C" int b200_ctx_create(const b200_model_desc* desc, const b200_parallel_
         c->kv_int8_gemm = env_int("B200_KV_INT8_GEMM", 0) != 0;
     }
     c->exact_rows = env_int("B200_EXACT_ROWS", 1) != 0;
+    c->tc_pair = env_int("B200_TC_PAIR", 1);
     c->prefill_gemm_min = std::max(1, env_int("B200_PREFILL_GEMM_MIN", 32));
     c->prefill_queue = env_int("B200_PREFILL_QUEUE", 0) != 0;
     c->prompt_f16_min = std::max(0, env_int("B200_PROMPT_F16_MIN", 0));
@@ -2421,7 +2423,7 @@ static int prefill_gemm(b200_ctx* c, int seq, const uint32_t* tokens, int n, boo
                 if (!glu) first += (long long)w->ne[1];
             }
             void* yt = glu ? (void*)((__half*)y + at) : (void*)((float*)y + at);
-            const cudaError_t e = f16_maps ? tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, pdl, st) : cudaErrorNotSupported;
+            const cudaError_t e = f16_maps ? tc16::product(epi, x, ldx, c->pf_w16, rows_n, K, yt, ldy, T, bias ? bias + at : nullptr, c->mma_err, c->tc_pair, pdl, st) : cudaErrorNotSupported;
             if (e != cudaSuccess) return e == cudaErrorNotSupported && at > 0 ? cudaErrorInvalidValue : e;
             c->launches++;
         }

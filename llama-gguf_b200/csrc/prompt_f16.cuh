@@ -188,10 +188,8 @@ template <int EPI> cudaError_t launch_epi(const TcPlan& pl, const CUtensorMap& x
 }
 // Y[t][n] = epi(sum_k x[t][k] w[n][k] + bias[n]), T rows, N outputs (EPI_SILU_GLU: N units from the 2 N rows [gate | up] of w, fp16 Y).
 // cudaErrorNotSupported: a tensor map was refused, nothing was launched
-inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, bool pdl, cudaStream_t st) {
+inline cudaError_t product(int epi, const __half* x, int ldx, const __half* w, int N, int K, void* y, int ldy, int T, const float* bias, int* err, int pairs, bool pdl, cudaStream_t st) {
     const bool glu = epi_is_glu(epi);
-    const char* pe = getenv("B200_TC_PAIR");
-    const int pairs = pe && *pe ? atoi(pe) : 1;      // B200_TC_PAIR=0: no pairs of CTAs, 2: pairs for all products of more than 128 rows
     const TcPlan pl = tc_plan(T, N, K, 1, 0, false, glu, true, false, pairs);
     const int kh = pl.tn == 256 ? TcRing<256>::KH : TcRing<128>::KH;
     CUtensorMap xm, wm;

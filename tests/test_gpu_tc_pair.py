@@ -44,3 +44,19 @@ def test_the_same_bits_in_programs_with_experts(b200, monkeypatch, rows, width, 
         finally:
             gpu.close()
     assert (out["2"] == out["0"]).all()
+
+
+def test_the_switch_is_read_when_the_context_is_made(b200, monkeypatch):
+    """Products whose K is cut without pairs show by their bits which of the two ran."""
+    monkeypatch.setenv("B200_FEW_GEMM", "0")
+    arch, desc, tensors = synth.synth_model("pair-128", "Q8_0", 304)
+    out = []
+    for made, called in (("0", "0"), ("0", "2"), ("2", "2"), ("2", "0")):
+        monkeypatch.setenv("B200_TC_PAIR", made)
+        gpu = b200.GpuOnlyInference(desc, tensors)
+        try:
+            monkeypatch.setenv("B200_TC_PAIR", called)
+            out.append(gpu.prefill(synth.prompt_tokens(300, desc["vocab"])))
+        finally:
+            gpu.close()
+    assert (out[0] == out[1]).all() and (out[2] == out[3]).all() and (out[0] != out[2]).any()
