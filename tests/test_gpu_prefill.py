@@ -87,7 +87,7 @@ def test_batched_decode_through_the_gemm(b200, oracle, preset, mix):
             want = refs[s].forward([toks[s]])
             assert rel_err(got[s], want) < TOL, f"step {step} slot {s}"
             assert gpu.position(s) == refs[s].position()
-    # a small batch takes the per-sequence path (one launch sequence per row) on the caches the GEMM steps wrote
+    # a small batch takes rows in f32 (csrc/exact_rows.cuh) on the caches the GEMM steps wrote
     l0 = gpu.stats()["kernel_launches"]
     got = gpu.decode_batch([0, 1, 2], [3, 4, 5])
     assert gpu.stats()["kernel_launches"] - l0 >= 3
