@@ -848,6 +848,7 @@ extern "C" int b200_ctx_finalize(b200_ctx* c) {
         CU(cudaFuncSetAttribute(attn_decode_kernel<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
         CU(cudaFuncSetAttribute(attn_decode_kernel<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim_attn));
         CU(cudaFuncSetAttribute(rows_tile_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsTileSmem<8>));
+        CU(cudaFuncSetAttribute(rows_tile_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsTileSmem<4>));
         CU(cudaFuncSetAttribute(rows_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<128>));
         CU(cudaFuncSetAttribute(rows_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<64>));
         CU(cudaFuncSetAttribute(rows_attn_kernel<128, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsAttnSmem<128>));

@@ -12,7 +12,7 @@
 // The multiply-adds are packed pairs (fma.rn.f32x2): two along K in the first kernel, two weight rows in the second.
 // Measured, token by token -> here: prompts through two layers of a 0.5B model (896 wide, Q5_0 / Q8_0) of 5, 16, 31 tokens 428, 1318, 2545 -> 176, 205, 301 us; of 33, 100, 333,
 // 1000, 4000 tokens 2696, 8666, 29785, 94147, 453403 -> 374, 586, 1054, 2596, 10730; two 8B layers in Q4_K_M, 2, 8, 31 tokens 321, 1194, 4628 -> 300, 617, 1874, steps of 2, 4, 7
-// sequences 345, 678, 1187 -> 299, 418, 652.  Distance to float64 of 0.5B prompts of 100, 333, 1000 tokens: 3.0e-7, 3.5e-7, 4.3e-7 -> 2.8e-7, 4.1e-7, 4.6e-7.
+// sequences 345, 678, 1187 -> 299, 418, 652.  Distance to float64 of 0.5B prompts of 100, 333, 1000 tokens: 2.7e-7, 3.5e-7, 4.1e-7 -> 2.5e-7, 3.3e-7, 4.0e-7 (16 inputs).
 #pragma once
 #include "attention.cuh"
 #include "gemv.cuh"
@@ -245,8 +245,8 @@ __device__ __forceinline__ void rows_few_b32(int type, const uint8_t* const (&rp
     }
 }
 
-// What bounds it: instructions, 6.6 per weight at two rows (unpacking three, T / 2 packed multiply-adds), issued in 45 % of the slots by 16 warps per SM of 128 registers: gate and up
-// of an 8B layer take 47 us where DRAM would take 10.  grid (CTAs, ceil(T / TT)).
+// What bounds it: instructions, 6.8 per weight at two rows (unpacking three, T / 2 packed multiply-adds), issued in 58 % of the slots by 16 warps per SM of 128 registers (o, q / k / v and
+// down, with fewer warps: 39 - 45 %): gate and up of an 8B layer take 47 us where DRAM would take 10.  grid (CTAs, ceil(T / TT)).
 template <int R, int TT>
 __global__ void __launch_bounds__(kRowsWarps * 32, R * TT <= 16 ? 2 : 1) rows_few_kernel(const __grid_constant__ RowsParams p) {
     constexpr int G = R / 2 > 0 ? R / 2 : 1, NV = R * TT;
@@ -513,18 +513,20 @@ __device__ __forceinline__ void rows_values(int type, const uint8_t* row, int k0
 }
 
 // Y[z][t][n] = sum over piece z of K.  128 threads: 8 weight rows x TPT rows of x each (weight rows 4 tx .. and 32 + 4 tx .., so that a warp's loads of four
-// are 128 bytes in a row); 16 TPT rows of x per CTA, four by four.  Sums run over 64 elements of K and are then added to the piece's: the error of one long chain of f32
-// additions grows with the root of its length (K = 4864: 1.7e-6 of the result, this way 3e-7, what a warp's 32 chains of gemv_kernel give).
-// Bound by the FMA pipe: 45 - 53 % of it busy (8 x 8 sums per thread; 29 % with 8 x 4, which waits for shared memory: 129 -> 72 us for 1152 x 1000 x 896).
+// are 128 bytes in a row); 16 TPT rows of x per CTA, four by four.  Sums run over 16 elements of K, eight of those make a sum of 128, and these are added to the piece's (in shared
+// memory): the error of a chain of f32 additions grows with the root of its length (one chain of 4864: 1.7e-6 of the result).  Distance to float64 of prompts of 40, 100, 333, 1000 tokens through two
+// layers of a 0.5B model, times that of token by token (16 inputs, +- 0.02): 0.95, 0.94, 0.95, 0.98; with sums of 64 that went straight to the piece's 1.16, 1.14, 1.06, 1.02, in the same time.
+// Bound by the FMA pipe: 43 - 52 % of it busy (8 x 8 sums per thread; 29 % with 8 x 4, which waits for shared memory: 129 -> 72 us for 1152 x 1000 x 896).
 // grid (tiles of all segments, ceil(T / (16 TPT)), pieces).
-template <int TPT> constexpr int kRowsTileSmem = 2 * 32 * (64 + 16 * TPT) * 4;
-constexpr int kRowsBN = 64, kRowsBK = 32, kRowsFlush = 2;
+template <int TPT> constexpr int kRowsTileSmem = 2 * 32 * (64 + 16 * TPT) * 4 + 128 * 4 * TPT * 8;
+constexpr int kRowsBN = 64, kRowsBK = 32, kRowsSum = 4;      // kRowsSum: steps of a sum that goes to the piece's
 template <int TPT>
 __global__ void __launch_bounds__(128, TPT == 8 ? 2 : 3) rows_tile_kernel(const __grid_constant__ RowsParams p) {
     constexpr int BT = 16 * TPT, XV = BT / 16;      // XV: float4 of x per thread and step
     extern __shared__ __align__(16) float rows_tile_smem[];
     auto ws = reinterpret_cast<float (*)[kRowsBK][kRowsBN]>(rows_tile_smem);
     auto xt = reinterpret_cast<float (*)[kRowsBK][BT]>(rows_tile_smem + 2 * kRowsBK * kRowsBN);
+    uint64_t* top = reinterpret_cast<uint64_t*>(rows_tile_smem + 2 * kRowsBK * (kRowsBN + BT)) + threadIdx.x;      // this thread's sums of the piece, 128 apart
     const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
     int s = 0, tile = blockIdx.x;
     while (s < p.n_seg - 1 && tile >= (p.seg[s].n_rows + kRowsBN - 1) / kRowsBN) {
@@ -574,31 +576,45 @@ __global__ void __launch_bounds__(128, TPT == 8 ? 2 : 3) rows_tile_kernel(const 
             rows_raw(type, row, k + kRowsBK + wk, raw);
             load_x(k + kRowsBK);
         }
+#pragma unroll 1
+        for (int half = 0; half < kRowsBK; half += 16) {
 #pragma unroll 4
-        for (int kk = 0; kk < kRowsBK; kk++) {
-            const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][4 * tx]), w1 = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][32 + 4 * tx]);
-            float xs[TPT];
+            for (int kk = half; kk < half + 16; kk++) {
+                const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][4 * tx]), w1 = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][32 + 4 * tx]);
+                float xs[TPT];
 #pragma unroll
-            for (int i = 0; i < TPT / 4; i++) {
-                const float4 f = *reinterpret_cast<const float4*>(&xt[buf][kk][64 * i + 4 * ty]);
-                xs[4 * i] = f.x; xs[4 * i + 1] = f.y; xs[4 * i + 2] = f.z; xs[4 * i + 3] = f.w;
-            }
+                for (int i = 0; i < TPT / 4; i++) {
+                    const float4 f = *reinterpret_cast<const float4*>(&xt[buf][kk][64 * i + 4 * ty]);
+                    xs[4 * i] = f.x; xs[4 * i + 1] = f.y; xs[4 * i + 2] = f.z; xs[4 * i + 3] = f.w;
+                }
 #pragma unroll
-            for (int t = 0; t < TPT; t++) {
-                const uint64_t x2 = f2_pack(xs[t], xs[t]);
-                f2_fma(acc[0][t], w0.x, x2);
-                f2_fma(acc[1][t], w0.y, x2);
-                f2_fma(acc[2][t], w1.x, x2);
-                f2_fma(acc[3][t], w1.y, x2);
+                for (int t = 0; t < TPT; t++) {
+                    const uint64_t x2 = f2_pack(xs[t], xs[t]);
+                    f2_fma(acc[0][t], w0.x, x2);
+                    f2_fma(acc[1][t], w0.y, x2);
+                    f2_fma(acc[2][t], w1.x, x2);
+                    f2_fma(acc[3][t], w1.y, x2);
+                }
             }
-        }
-        if ((step & (kRowsFlush - 1)) == kRowsFlush - 1 || !more) {
 #pragma unroll
             for (int n = 0; n < 4; n++)
 #pragma unroll
                 for (int t = 0; t < TPT; t++) {
                     f2_add(tot[n][t], acc[n][t]);
                     acc[n][t] = 0;
+                }
+        }
+        if (more ? step % kRowsSum == kRowsSum - 1 : step >= kRowsSum) {
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int t = 0; t < TPT; t++) {
+                    uint64_t* at = top + (n * TPT + t) * 128;
+                    if (step >= kRowsSum) f2_add(tot[n][t], *at);
+                    if (more) {
+                        *at = tot[n][t];
+                        tot[n][t] = 0;
+                    }
                 }
         }
         if (more) put(buf ^ 1, k + kRowsBK);

@@ -106,3 +106,22 @@ def test_first_short_prompt_allocates_nothing(b200, preset, mix, kv):
             gpu.close()
     assert launches < 31 * desc["n_layers"]      # (as rows)
     assert free == before[1]
+
+
+@pytest.mark.parametrize("n", [40, 100])
+def test_rows_are_no_further_from_float64_than_token_by_token(b200, monkeypatch, n):
+    """Prompts in tiles: root mean square of the distances over eight inputs, which spreads by 3 %."""
+    from perf import cases
+    case = dict(family="gguf", preset="qwen2.5-0.5b", layers=2, vocab=4096, mix="Q4_K_M", kv="f32", batch=1, prompt=n, decode=0)
+    err = {"1": [], "0": []}
+    for seed in range(201, 209):
+        want = cases.exact(case, seed)[0].cpu().numpy()
+        for on in err:
+            monkeypatch.setenv("B200_EXACT_ROWS", on)
+            state = cases.prepare(case, seed)
+            got = np.asarray(cases.run(state)[0], dtype=np.float64)
+            state["gpu"].close()
+            err[on].append(np.linalg.norm(got - want) / np.linalg.norm(want))
+    rows, tokens = (float(np.sqrt(np.mean(np.square(err[on])))) for on in ("1", "0"))
+    print(f"{n} tokens: rows {rows:.3e}, token by token {tokens:.3e}")
+    assert rows < 1.05 * tokens
