@@ -67,6 +67,7 @@ struct StepMeta {
     const int* row_pos;
     const int* run_start;
     const int* run_pos0;
+    const int* run_flip;       // which of its two copies of n and m (matrix memory) a run reads; it writes the other
     uint8_t* const* run_kv;
     uint8_t* const* run_rec;
     const int* want;
@@ -1201,7 +1202,8 @@ __global__ void __launch_bounds__(128) lp_window_attn_tile_kernel(StepMeta sm, A
 // Per (run, head): S [dim][vdim], n [dim], m; thread = value channel j, its column S[:, j] lives in registers for the whole run.
 //   i = cap tanh((zi + bi) / cap),  f = logsigmoid(cap tanh((zf + bf) / cap)),  m' = max(f + m, i)
 //   S <- e^(f + m - m') S + e^(i - m') k v^T,  n likewise with k,  o = S^T q / (max(|n . q|, e^(-m')) + 1e-6),  q = (W_q h) dim^(-1/2)
-// State block of a run: S [H][dim][vdim] | n [H][dim] | m [H], f32.
+// State block of a run: S [H][dim][vdim] | n [2][H][dim] | m [2][H], f32.  All column blocks of a head read n and m and one of them writes them: into the copy that no
+// step in flight reads (a block placed late would otherwise find them moved on already: 27 sequences, one of ten steps), and the next step reads that one.
 struct MemGeom {
     int H, dim, vdim;
     float cap;
@@ -1239,8 +1241,10 @@ __global__ void __launch_bounds__(SCAN_BD) lp_matrix_memory_kernel(StepMeta sm, 
     const int j = blockIdx.x * COLS + col, h = blockIdx.y, run = blockIdx.z;
     const int r0 = sm.run_start[run], r1 = sm.run_start[run + 1];
     float* Sg = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off) + (size_t)h * g.dim * g.vdim;
-    float* ng = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off) + (size_t)g.H * g.dim * g.vdim + (size_t)h * g.dim;
-    float* mg = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off) + (size_t)g.H * g.dim * g.vdim + (size_t)g.H * g.dim + h;
+    const int flip = sm.run_flip[run];
+    float* n0 = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off) + (size_t)g.H * g.dim * g.vdim;
+    const float* ng = n0 + ((size_t)flip * g.H + h) * g.dim;
+    float* mg = n0 + (size_t)2 * g.H * g.dim;      // [2][H]
     const bool live = j < g.vdim;
     float s[SCAN_DREG];
 #pragma unroll
@@ -1255,7 +1259,7 @@ __global__ void __launch_bounds__(SCAN_BD) lp_matrix_memory_kernel(StepMeta sm, 
         (&qs[0][0])[i] = 0.0f;
         (&ks[0][0])[i] = 0.0f;
     }
-    float m = *mg;
+    float m = mg[flip * g.H + h];
     const float qscale = 1.0f / sqrtf((float)g.dim);
     const float bi = ib[h], bf_ = fb[h];
     const int jc = blockIdx.x * COLS + (tid % COLS);   // the column this thread stages
@@ -1318,10 +1322,11 @@ __global__ void __launch_bounds__(SCAN_BD) lp_matrix_memory_kernel(StepMeta sm, 
             if (d < g.dim) Sg[(size_t)d * g.vdim + j] = s[i];
         }
     if (blockIdx.x == 0 && tid < 32) {
+        float* nn = n0 + ((size_t)(flip ^ 1) * g.H + h) * g.dim;
 #pragma unroll
         for (int i = 0; i < DMAX / 32; i++)
-            if (lane + 32 * i < g.dim) ng[lane + 32 * i] = nreg[i];
-        if (tid == 0) *mg = m;
+            if (lane + 32 * i < g.dim) nn[lane + 32 * i] = nreg[i];
+        if (tid == 0) mg[(flip ^ 1) * g.H + h] = m;
     }
 }
 
@@ -1662,6 +1667,7 @@ struct LayerPlan {
 struct SlotMem {
     uint8_t* kv = nullptr;
     uint8_t* rec = nullptr;
+    int flip = 0;            // (StepMeta)
 };
 
 }  // namespace
@@ -2554,7 +2560,7 @@ int lp_finalize(LpModel* m, std::string* err) {
             if ((rc = need_vec(m, r + "i.b", mm.heads, &L.ib, err))) return rc;
             if ((rc = need_vec(m, r + "f.b", mm.heads, &L.fb, err))) return rc;
             L.kv_bytes = up16((size_t)p.max_seq_len * a.kv_heads * (a.dim + a.vdim) * 4);
-            L.rec_bytes = up16(((size_t)mm.heads * mm.dim * mm.vdim + (size_t)mm.heads * mm.dim + mm.heads) * 4);
+            L.rec_bytes = up16(((size_t)mm.heads * mm.dim * mm.vdim + 2 * ((size_t)mm.heads * mm.dim + mm.heads)) * 4);
             m->max_act = std::max(m->max_act, L.k_cat);
             m->max_o = std::max(m->max_o, mm.heads * mm.vdim);
             m->max_q = std::max(m->max_q, a.heads * a.dim);
@@ -3211,7 +3217,7 @@ int ensure_scratch(LpModel* m, int R, int n_runs, int n_want, std::string* err) 
         m->cap_want = cap;
     }
     m->cap_runs = std::max(m->cap_runs, n_runs);
-    const size_t meta = up16((size_t)(3 * m->cap_rows + 2 * m->cap_runs + 2 + m->cap_want) * 4) + (size_t)2 * m->cap_runs * 8 + 64;
+    const size_t meta = up16((size_t)(3 * m->cap_rows + 3 * m->cap_runs + 2 + m->cap_want) * 4) + (size_t)2 * m->cap_runs * 8 + 64;
     if (meta > m->meta_bytes) {
         if (m->h_meta) cudaFreeHost(m->h_meta);
         m->h_meta = nullptr;
@@ -3378,14 +3384,13 @@ template <int MODE>
 bool chunk_scan(LpModel* m, const StepMeta& sm, ChunkScan g, int n_runs, int max_len) {
     if (!m->use_chunk_scan || max_len < (MODE == CS_SSD ? 128 : 48)) return false;
     if (g.dim % 4 || g.vdim % 4 || g.dim > 128 || g.ldq % 4 || g.ldv % 4 || (((uintptr_t)g.Q | (uintptr_t)g.K | (uintptr_t)g.V) & 15)) return false;
-    const size_t hr = (size_t)g.H * g.R, nm = MODE == CS_MEM ? (size_t)n_runs * g.H * (g.dim + 1) : 0;
-    const size_t want = (hr * (3 + CS) + 8 + (MODE == CS_DELTA ? hr * (g.dim + g.vdim) : 0) + nm) * 4;
+    const size_t hr = (size_t)g.H * g.R;
+    const size_t want = (hr * (3 + CS) + 8 + (MODE == CS_DELTA ? hr * (g.dim + g.vdim) : 0)) * 4;
     if (!keep_scratch(m->chunk_scan, m->chunk_scan_bytes, want, (size_t)512 << 20)) return false;
     g.M = m->chunk_scan;                               // (16-byte rows first)
     g.W = g.M + hr * CS;
     g.U0 = g.W + (MODE == CS_DELTA ? hr * g.dim : 0);
     g.sc = g.U0 + (MODE == CS_DELTA ? hr * g.vdim : 0);
-    g.nm = g.sc + 3 * hr;
     return g.dim <= 64 ? chunk_scan_launch<MODE, 64>(m, sm, g, n_runs, max_len) : chunk_scan_launch<MODE, 128>(m, sm, g, n_runs, max_len);
 }
 
@@ -3777,7 +3782,7 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
             const int mcols = SCAN_BD / (pick_dmax(mg.dim) / SCAN_DREG);
             dim3 sgrid((mg.vdim + mcols - 1) / mcols, mg.H, n_runs);
             const ChunkScan cm{mg.H, mg.H, mg.dim, mg.vdim, R, m->P + mg.q_off, m->P + mg.k_off, m->P + mg.v_off, L.n_in, L.n_in, m->P + mg.i_off, m->P + mg.f_off, L.n_in,
-                               L.ib, L.fb, nullptr, mg.cap, mg.rec_off, nullptr, nullptr, nullptr, nullptr, nullptr, m->O, ldo};
+                               L.ib, L.fb, nullptr, mg.cap, mg.rec_off, nullptr, nullptr, nullptr, nullptr, m->O, ldo};
             if (!chunk_scan<CS_MEM>(m, sm, cm, n_runs, max_len)) switch (pick_dmax(mg.dim)) {
                 case 32: launch(m, lp_matrix_memory_kernel<32>, sgrid, dim3(SCAN_BD), 0, sm, mg, (const float*)m->P, L.n_in, L.ib, L.fb, m->O, ldo); break;
                 case 64: launch(m, lp_matrix_memory_kernel<64>, sgrid, dim3(SCAN_BD), 0, sm, mg, (const float*)m->P, L.n_in, L.ib, L.fb, m->O, ldo); break;
@@ -3856,7 +3861,7 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
             dim3 sgrid((g.vdim + dcols - 1) / dcols, g.heads, n_runs);
 #define LP_SSD(DM) launch(m, lp_ssd_scan_kernel<DM>, sgrid, dim3(SCAN_BD), 0, sm, sg, (const float*)m->conv, dg.C, (const float*)m->P, L.n_in, L.A_log, L.dt_bias, L.ssd_D, m->O, inner)
             const ChunkScan cs{sg.H, sg.G, sg.N, sg.vdim, R, m->conv + inner + sg.G * sg.N, m->conv + inner, m->conv, dg.C, dg.C, m->P + sg.dt_off, m->P + sg.dt_off, L.n_in,
-                               L.A_log, L.dt_bias, L.ssd_D, 0.0f, sg.rec_off, nullptr, nullptr, nullptr, nullptr, nullptr, m->O, inner};
+                               L.A_log, L.dt_bias, L.ssd_D, 0.0f, sg.rec_off, nullptr, nullptr, nullptr, nullptr, m->O, inner};
             if (!chunk_scan<CS_SSD>(m, sm, cs, n_runs, max_len)) switch (pick_dmax(g.state)) {
                 case 32: LP_SSD(32); break;
                 case 64: LP_SSD(64); break;
@@ -3877,7 +3882,7 @@ void enqueue_step(LpModel* m, const StepMeta& sm, int R, int n_runs, int n_want,
             const int dcols = SCAN_BD / (pick_dmax(dg.dim) / SCAN_DREG);
             dim3 sgrid((dg.vdim + dcols - 1) / dcols, dg.H, n_runs);
             const ChunkScan cd{dg.H, dg.G, dg.dim, dg.vdim, R, m->conv, m->conv + dg.G * dg.dim, m->conv + 2 * dg.G * dg.dim, dg.C, dg.C, m->P + dg.b_off, m->P + dg.a_off,
-                               L.n_in, L.A_log, L.dt_bias, nullptr, 0.0f, dg.rec_off, nullptr, nullptr, nullptr, nullptr, nullptr, m->O, ldo};
+                               L.n_in, L.A_log, L.dt_bias, nullptr, 0.0f, dg.rec_off, nullptr, nullptr, nullptr, nullptr, m->O, ldo};
             if (!chunk_scan<CS_DELTA>(m, sm, cd, n_runs, max_len)) switch (pick_dmax(dg.dim)) {
                 case 32: launch(m, lp_gated_delta_kernel<32>, sgrid, dim3(SCAN_BD), 0, sm, dg, (const float*)m->conv, (const float*)m->P, L.n_in, L.A_log, L.dt_bias, m->O, ldo); break;
                 case 64: launch(m, lp_gated_delta_kernel<64>, sgrid, dim3(SCAN_BD), 0, sm, dg, (const float*)m->conv, (const float*)m->P, L.n_in, L.A_log, L.dt_bias, m->O, ldo); break;
@@ -4130,6 +4135,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
             if (!m->pool.empty()) {
                 s = m->pool.back();
                 m->pool.pop_back();
+                s.flip = 0;
             } else {
                 LCU_ALLOC(step_malloc(m, (void**)&s.kv, m->slot_kv_bytes));
                 cudaError_t e = step_malloc(m, (void**)&s.rec, m->slot_rec_bytes);
@@ -4151,14 +4157,16 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         int* row_pos = row_run + m->cap_rows;
         int* run_start = row_pos + m->cap_rows;
         int* run_p0 = run_start + m->cap_runs + 1;
-        int* want = run_p0 + m->cap_runs + 1;
-        const size_t ints = up16((size_t)(3 * m->cap_rows + 2 * m->cap_runs + 2 + m->cap_want) * 4);
+        int* run_flip = run_p0 + m->cap_runs + 1;
+        int* want = run_flip + m->cap_runs;
+        const size_t ints = up16((size_t)(3 * m->cap_rows + 3 * m->cap_runs + 2 + m->cap_want) * 4);
         uint8_t** kvp = (uint8_t**)(m->h_meta + ints);
         uint8_t** recp = kvp + m->cap_runs;
         int r = 0;
         for (int i = 0; i < n_runs; i++) {
             run_start[i] = r;
             run_p0[i] = pos0[i];
+            run_flip[i] = m->slot[seqs[i]].flip;
             kvp[i] = m->slot[seqs[i]].kv;
             recp[i] = m->slot[seqs[i]].rec;
             for (int t = 0; t < lens[i]; t++, r++) {
@@ -4176,7 +4184,8 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         sm.row_pos = sm.row_run + m->cap_rows;
         sm.run_start = sm.row_pos + m->cap_rows;
         sm.run_pos0 = sm.run_start + m->cap_runs + 1;
-        sm.want = sm.run_pos0 + m->cap_runs + 1;
+        sm.run_flip = sm.run_pos0 + m->cap_runs + 1;
+        sm.want = sm.run_flip + m->cap_runs;
         sm.run_kv = (uint8_t* const*)(d + ints);
         sm.run_rec = sm.run_kv + m->cap_runs;
     }
@@ -4292,6 +4301,7 @@ int lp_step(LpModel* m, int n_runs, const int* seqs, const int* pos0, const int*
         cudaMemsetAsync(m->tc_err, 0, sizeof(int), m->stream);
         return lp_fail(err, B200_ERR_OPERATION_FAILED, "b200_step: tensor-core GEMM wait gave up (code " + std::to_string(code) + "): results discarded");
     }
+    for (int i = 0; i < n_runs; i++) m->slot[seqs[i]].flip ^= 1;
     if (n_want > 0 && logits_out) memcpy(logits_out, m->h_tc_err + HEAD_WORDS, (size_t)n_want * p.vocab * 4);
     return B200_OK;
 }

@@ -29,7 +29,7 @@ struct ChunkScan {
     const float* skip;                  // SSD: D
     float cap;
     size_t rec_off;
-    float *sc, *M, *W, *U0, *nm;        // scratch: [3][H][R] scalars, [H][R][32], DELTA: [H][R][dim], [H][R][vdim], MEM: [runs][H][dim + 1] n and m as they were
+    float *sc, *M, *W, *U0;             // scratch: [3][H][R] scalars, [H][R][32], DELTA: [H][R][dim], [H][R][vdim]
     float* O;
     int ldo;
 };
@@ -55,12 +55,6 @@ __global__ void __launch_bounds__(CS_THREADS) lp_chunk_prep_kernel(StepMeta sm, 
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         *reinterpret_cast<float4*>(qs + t * PI + d) = in ? *reinterpret_cast<const float4*>(g.Q + (size_t)(r0 + t) * g.ldq + hk * g.dim + d) : z;
         *reinterpret_cast<float4*>(ks + t * PI + d) = in ? *reinterpret_cast<const float4*>(g.K + (size_t)(r0 + t) * g.ldq + hk * g.dim + d) : z;
-    }
-    if (MODE == CS_MEM && blockIdx.x == 0) {    // the scan's first block writes n and m while others may still have to read them
-        const float* rec = reinterpret_cast<const float*>(sm.run_rec[run] + g.rec_off) + (size_t)g.H * g.dim * g.vdim;
-        float* nm = g.nm + ((size_t)run * g.H + h) * (g.dim + 1);
-        for (int d = tid; d < g.dim; d += CS_THREADS) nm[d] = rec[(size_t)h * g.dim + d];
-        if (tid == 0) nm[g.dim] = rec[(size_t)g.H * g.dim + h];
     }
     // gates: decay (MEM: its logarithm; none past the end), a / b: what else M and u need
     if (tid < CS) {
@@ -264,9 +258,11 @@ __global__ void __launch_bounds__(CS_SCAN_THREADS) lp_chunk_scan_kernel(StepMeta
     const int r0 = sm.run_start[run], r1 = sm.run_start[run + 1], hk = h * g.G / g.H;
     float* rec = reinterpret_cast<float*>(sm.run_rec[run] + g.rec_off);
     float* Sg = rec + (size_t)h * g.dim * g.vdim;
-    float* ng = rec + (size_t)g.H * g.dim * g.vdim + (size_t)h * g.dim;                       // MEM
-    float* mg = rec + (size_t)g.H * g.dim * g.vdim + (size_t)g.H * g.dim + h;
-    const float* nm = MODE == CS_MEM ? g.nm + ((size_t)run * g.H + h) * (g.dim + 1) : nullptr;
+    const int flip = MODE == CS_MEM ? sm.run_flip[run] : 0;                                   // MEM: n and m are read from one copy and written to the other (lp_matrix_memory_kernel)
+    float* n0 = rec + (size_t)g.H * g.dim * g.vdim;
+    const float* nm = n0 + ((size_t)flip * g.H + h) * g.dim;
+    float* ng = n0 + ((size_t)(flip ^ 1) * g.H + h) * g.dim;
+    float* mg = n0 + (size_t)2 * g.H * g.dim;                                                 // [2][H]
     auto stage = [&](int c0, int buf) {
         float* q = cs_sm + buf * L::STAGE;
         float* k = q + CS * PI;
@@ -311,7 +307,7 @@ __global__ void __launch_bounds__(CS_SCAN_THREADS) lp_chunk_scan_kernel(StepMeta
         }
         *reinterpret_cast<float4*>(S0 + half * DM * 4 + kr * 4) = make_float4(st[0], st[1], st[2], st[3]);
     }
-    float m_run = MODE == CS_MEM ? nm[g.dim] : 0.0f;
+    float m_run = MODE == CS_MEM ? mg[flip * g.H + h] : 0.0f;
     const float dskip = MODE == CS_SSD ? g.skip[h] : 0.0f;
     const float qsc = MODE == CS_MEM ? 1.0f / sqrtf((float)g.dim) : 1.0f;
     // (a chunk's rows are asked for two chunks ahead: one is less than their way from L2 takes)
@@ -402,5 +398,5 @@ __global__ void __launch_bounds__(CS_SCAN_THREADS) lp_chunk_scan_kernel(StepMeta
             } else if (j < g.vdim) Sg[(size_t)kr * g.vdim + j] = st[e];
         }
     }
-    if (MODE == CS_MEM && blockIdx.x == 0 && tid == 0) *mg = m_run;
+    if (MODE == CS_MEM && blockIdx.x == 0 && tid == 0) mg[(flip ^ 1) * g.H + h] = m_run;
 }
