@@ -107,8 +107,9 @@ B200_API void b200_ctx_destroy(b200_ctx* ctx);
  * b200_ctx_finalize (or with B200_KV_FORMAT=int8 in the environment): 0 = F32 (the KVCache of src/model/mod.rs:83-108, default),
  * 1 = Int8 -- QuantizedKVCache::write_kv / read_k_range semantics (kv_quantized.rs:143-216, 230-270, 366-392): one symmetric
  * scale = max|x| / 127 per (kv head, position) row, q = round(x / scale), attention over q * scale.  A quarter of the KV bytes; the
- * context then decodes on the per-op (graph) path and prefills token by token (B200_KV_INT8_GEMM=1: prompts of >= 32 tokens through
- * the tensor-core pass, outside the 1e-3 parity bound).  The FP8 formats are not built (UNSUPPORTED). */
+ * context then decodes on the per-op (graph) path and prefills in f32, prompts of fewer than 32 tokens as rows, longer ones token by
+ * token (B200_KV_INT8_GEMM=1: prompts of >= 32 tokens through the tensor-core pass, where its attention takes the model's heads;
+ * outside the 1e-3 parity bound).  The FP8 formats are not built (UNSUPPORTED). */
 B200_API int b200_ctx_set_kv_format(b200_ctx* ctx, int format);
 B200_API int b200_ctx_kv_format(b200_ctx* ctx, int* out);
 
@@ -188,7 +189,8 @@ B200_API int b200_prefill_token(b200_ctx* ctx, int seq, uint32_t token);
  * sequence; logits of the last one (logits_out may be NULL). */
 B200_API int b200_prefill(b200_ctx* ctx, int seq, const uint32_t* tokens, int n, float* logits_out);
 /* One token for each of n DISTINCT sequence slots;
- * logits_out is n x vocab. */
+ * logits_out is n x vocab.  Dense single-GPU models: two to seven sequences as rows in f32, eight and more with fp16 activations
+ * (where the products know the blocks); without room for a step's buffers the former go one by one. */
 B200_API int b200_decode_batch(b200_ctx* ctx, const int* seqs, const uint32_t* tokens, int n, float* logits_out);
 /* Greedy continuation behind b200_forward (opt-in, after finalize; one GPU, megakernel paths).  When on, b200_forward also picks
  * argmax (last maximum wins, src/main.rs:1816-1821) on the device and launches the NEXT token on that pick before it returns.  If
