@@ -11,8 +11,8 @@
 //                      rows_qkv_kernel, rows_swiglu_kernel).
 // The multiply-adds are packed pairs (fma.rn.f32x2): two along K in the first kernel, two weight rows in the second.
 // Measured, token by token -> here: prompts through two layers of a 0.5B model (896 wide, Q5_0 / Q8_0) of 5, 16, 31 tokens 428, 1318, 2545 -> 176, 205, 301 us; of 33, 100, 333,
-// 1000, 4000 tokens 2696, 8666, 29785, 94147, 453403 -> 374, 586, 1054, 2596, 10730; two 8B layers in Q4_K_M, 2, 8, 31 tokens 321, 1194, 4628 -> 300, 617, 1874, steps of 2, 4, 7
-// sequences 345, 678, 1187 -> 299, 418, 652.  Distance to float64 of 0.5B prompts of 100, 333, 1000 tokens: 2.7e-7, 3.5e-7, 4.1e-7 -> 2.5e-7, 3.3e-7, 4.0e-7 (16 inputs).
+// 1000, 4000 tokens 2696, 8666, 29785, 94147, 453403 -> 380, 598, 1082, 2597, 10840; two 8B layers in Q4_K_M, 2, 8, 31 tokens 321, 1194, 4628 -> 300, 617, 1874, steps of 2, 4, 7
+// sequences 350, 682, 1187 -> 265, 355, 513.  Distance to float64 of 0.5B prompts of 100, 333, 1000 tokens: 2.7e-7, 3.5e-7, 4.1e-7 -> 2.5e-7, 3.3e-7, 4.0e-7 (16 inputs).
 #pragma once
 #include "attention.cuh"
 #include "gemv.cuh"
@@ -245,8 +245,8 @@ __device__ __forceinline__ void rows_few_b32(int type, const uint8_t* const (&rp
     }
 }
 
-// What bounds it: instructions, 6.8 per weight at two rows (unpacking three, T / 2 packed multiply-adds), issued in 58 % of the slots by 16 warps per SM of 128 registers (o, q / k / v and
-// down, with fewer warps: 39 - 45 %): gate and up of an 8B layer take 47 us where DRAM would take 10.  grid (CTAs, ceil(T / TT)).
+// What bounds it: instructions, 6.6 per weight at two rows (unpacking three, T / 2 packed multiply-adds), issued in 57 % of the slots by 16 warps per SM of 128 registers (o, q / k / v and
+// down, with fewer warps: 39 - 47 %): gate and up of an 8B layer take 46 us where DRAM would take 10.  grid (CTAs, ceil(T / TT)).
 template <int R, int TT>
 __global__ void __launch_bounds__(kRowsWarps * 32, R * TT <= 16 ? 2 : 1) rows_few_kernel(const __grid_constant__ RowsParams p) {
     constexpr int G = R / 2 > 0 ? R / 2 : 1, NV = R * TT;
@@ -516,7 +516,7 @@ __device__ __forceinline__ void rows_values(int type, const uint8_t* row, int k0
 // are 128 bytes in a row); 16 TPT rows of x per CTA, four by four.  Sums run over 16 elements of K, eight of those make a sum of 128, and these are added to the piece's (in shared
 // memory): the error of a chain of f32 additions grows with the root of its length (one chain of 4864: 1.7e-6 of the result).  Distance to float64 of prompts of 40, 100, 333, 1000 tokens through two
 // layers of a 0.5B model, times that of token by token (16 inputs, +- 0.02): 0.95, 0.94, 0.95, 0.98; with sums of 64 that went straight to the piece's 1.16, 1.14, 1.06, 1.02, in the same time.
-// Bound by the FMA pipe: 43 - 52 % of it busy (8 x 8 sums per thread; 29 % with 8 x 4, which waits for shared memory: 129 -> 72 us for 1152 x 1000 x 896).
+// Bound by the FMA pipe: 50 - 54 % of it busy (8 x 8 sums per thread; 29 % with 8 x 4, which waits for shared memory: 129 -> 72 us for 1152 x 1000 x 896).
 // grid (tiles of all segments, ceil(T / (16 TPT)), pieces).
 template <int TPT> constexpr int kRowsTileSmem = 2 * 32 * (64 + 16 * TPT) * 4 + 128 * 4 * TPT * 8;
 constexpr int kRowsBN = 64, kRowsBK = 32, kRowsSum = 4;      // kRowsSum: steps of a sum that goes to the piece's
@@ -650,7 +650,7 @@ template <int HD> constexpr int kRowsAttnSmem = (3 * 64 * HD + 64 * 64) * 4;
 // the keys 64 at a time with an online softmax; scores and sums as rows_tile_kernel's tiles, 8 keys (HD / 8 channels) x 4 rows per thread.  The tensor-core
 // attention of fp16 pairs adds all keys into one accumulator that cuts its sums off: 2.8e-6 of the logits at 1000 keys, against 4e-7 here (sums of 64 keys, then of tiles).
 // OutT = __half: prompts with fp16 products whose heads per kv head are no power of two (attn_umma_ok); prompts of 33, 333, 900, 4000 tokens through
-// two layers of 14 heads of 64 over 2: 200, 353, 574, 3080 us, with a warp per token and kv head (prefill_attn_kernel) 215, 600, 1358, 16475, with the padded pairs of fp16 186, 236, 298, 913.
+// two layers of 14 heads of 64 over 2: 200, 358, 606, 3136 us, with a warp per token and kv head (prefill_attn_kernel) 222, 616, 1387, 16564, with the padded pairs of fp16 188, 241, 303, 924.
 // grid (ceil(T G / 64), n_kv), the blocks with the most keys first.
 template <int HD, typename OutT = float>
 __global__ void __launch_bounds__(128) rows_attn_kernel(const RowsAttn p) {

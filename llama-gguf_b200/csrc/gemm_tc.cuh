@@ -744,7 +744,7 @@ bool tc_map(CUtensorMap* map, const void* p, int K, int rows, int ld, int parts,
 // rows: token rows as M (lp_gemm_tc_rows_kernel), tn weight rows per CTA: for sums that may not be cut (a cut over a cluster is as fast), up to 128 rows
 // pair: two CTAs per tile (lp_gemm_tc_kernel), where the single CTAs would not cut K either: a pair adds all of K in one accumulator of tensor memory, which cuts its sums off,
 // so in place of a cut it gives other bits and a larger error: 4096 x 700 x 14336 in two cuts, one 8B layer over 24 inputs, 1.0002 +- 0.0001 (Q4_K_M) and 1.0009 +- 0.0001 (Q8_0, 645
-// rows) times the distance to float64.  (Time: two 8B layers of 700 rows 910 us with pairs there, 1024 without.)
+// rows) times the distance to float64.  (Time: two 8B layers of 700 rows 1065 us before pairs, 910 with pairs there, 1000 without.)
 struct TcPlan {
     bool persistent;
     int tn, splits;
